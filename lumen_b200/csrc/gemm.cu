@@ -17,7 +17,7 @@
 #include <map>
 #include <mutex>
 
-#include "device.h"
+#include "gemm.h"
 #include "sm100.cuh"
 
 namespace lb {
@@ -31,10 +31,6 @@ constexpr int kEpilogueWarps = 8;
 constexpr int kStageBytesA = BM * BK * 2, kStageBytesB = BN * BK * 2;
 constexpr int kEpilogueStageBytes = 8 * 4096;  // one 4 KB staging area per epilogue warp (store_rows_coalesced)
 constexpr int kSmemBytes = STAGES * (kStageBytesA + kStageBytesB) + 1024 /*alignment slack*/ + 256 /*barriers*/ + kEpilogueStageBytes;
-
-// EPI_ADD: out = round(round(acc) + aux); EPI_MASK: out = aux > 0 ? round(acc) : 0 - each exactly the two primitives
-// of the traced program (a rounded product followed by an add / a select), with `aux` a tensor shaped like the output
-enum Epilogue : int { EPI_NONE = 0, EPI_RELU = 1, EPI_ADD = 2, EPI_MASK = 3 };
 
 struct GemmArgs {
     int M, N, K, batch;
@@ -647,84 +643,6 @@ __global__ void splitk_reduce(const float* __restrict__ partial, GemmArgs p) {
     }
 }
 
-// ---- SIMT GEMM: exact fp32 accumulation in contracting order -------------------------------------------------
-template <class T>
-__device__ __forceinline__ float load_as_float(const T* p);
-template <>
-__device__ __forceinline__ float load_as_float<float>(const float* p) { return *p; }
-template <>
-__device__ __forceinline__ float load_as_float<__nv_bfloat16>(const __nv_bfloat16* p) { return __bfloat162float(*p); }
-template <>
-__device__ __forceinline__ float load_as_float<__half>(const __half* p) { return __half2float(*p); }
-
-struct SimtArgs {
-    int M, N, K, batch;
-    long long a_sm, a_sk, a_sb, b_sk, b_sn, b_sb, ldd, d_sb;
-    void* d;
-    int d_dtype;
-    int epilogue;
-    const void* aux;  // EPI_ADD / EPI_MASK operand (16-bit, the output's dtype), rows ld_aux apart, batches aux_sb apart
-    long long ld_aux, aux_sb;
-};
-
-constexpr int ST = 64, SK = 16;  // 64x64 output tile per 256 threads (4x4 each), 16-deep k slices
-
-template <class T>
-__global__ void __launch_bounds__(256) gemm_simt(const T* __restrict__ a, const T* __restrict__ b, const SimtArgs p) {
-    __shared__ float sa[SK][ST + 1], sb[SK][ST + 1];
-    const int bz = blockIdx.z, m0 = blockIdx.y * ST, n0 = blockIdx.x * ST;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const T* ab = a + (long long)bz * p.a_sb;
-    const T* bb = b + (long long)bz * p.b_sb;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < p.K; k0 += SK) {
-        for (int i = threadIdx.x; i < ST * SK; i += 256) {
-            // read along whichever of (row, k) is contiguous in memory
-            int r, k;
-            if (p.a_sk == 1) { k = i % SK; r = i / SK; } else { r = i % ST; k = i / ST; }
-            int gm = m0 + r, gk = k0 + k;
-            sa[k][r] = (gm < p.M && gk < p.K) ? load_as_float(ab + gm * p.a_sm + gk * p.a_sk) : 0.0f;
-            int c;
-            if (p.b_sn == 1) { c = i % ST; k = i / ST; } else { k = i % SK; c = i / SK; }
-            int gn = n0 + c;
-            gk = k0 + k;
-            sb[k][c] = (gn < p.N && gk < p.K) ? load_as_float(bb + gk * p.b_sk + gn * p.b_sn) : 0.0f;
-        }
-        __syncthreads();
-        const int kmax = min(SK, p.K - k0);
-        for (int k = 0; k < kmax; k++) {
-            float av[4], bv[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) av[i] = sa[k][ty * 4 + i], bv[i] = sb[k][tx * 4 + i];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = __fadd_rn(acc[i][j], __fmul_rn(av[i], bv[j]));
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            int gm = m0 + ty * 4 + i, gn = n0 + tx * 4 + j;
-            if (gm >= p.M || gn >= p.N) continue;
-            float x = acc[i][j];
-            if (p.epilogue == EPI_RELU) x = fmaxf(x, 0.0f);
-            if (p.epilogue >= EPI_ADD) {  // the rounded product, then the second primitive on it (as the tensor-core kernels do)
-                const uint16_t a16 = ((const uint16_t*)p.aux)[(long long)bz * p.aux_sb + (long long)gm * p.ld_aux + gn];
-                float prod, other;
-                if (p.d_dtype == LB_BF16) prod = __bfloat162float(__float2bfloat16_rn(x)), other = __uint_as_float((uint32_t)a16 << 16);
-                else prod = __half2float(__float2half_rn(x)), other = __half2float(__ushort_as_half(a16));
-                x = p.epilogue == EPI_ADD ? __fadd_rn(other, prod) : (other > 0.0f ? prod : 0.0f);
-            }
-            long long at = (long long)bz * p.d_sb + (long long)gm * p.ldd + gn;
-            if (p.d_dtype == LB_F32) ((float*)p.d)[at] = x;
-            else if (p.d_dtype == LB_BF16) ((__nv_bfloat16*)p.d)[at] = __float2bfloat16_rn(x);
-            else ((__half*)p.d)[at] = __float2half_rn(x);
-        }
-}
-
 // [batch, rows, cols] view of a rank-2/3 tensor
 struct View3 {
     void* ptr;
@@ -923,11 +841,13 @@ void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
     p.b_sk = b.sr, p.b_sn = b.sc, p.b_sb = b.batch > 1 ? b.sb : 0;
     p.ldd = d.sr, p.d_sb = d.batch > 1 ? d.sb : 0;
     p.d = d.ptr, p.d_dtype = d.dtype, p.epilogue = epilogue;
-    dim3 grid((unsigned)((N + ST - 1) / ST), (unsigned)((M + ST - 1) / ST), (unsigned)batch);
-    if (a.dtype == LB_F32) gemm_simt<float><<<grid, 256, 0, s>>>((const float*)a.ptr, (const float*)b.ptr, p);
-    else if (a.dtype == LB_BF16) gemm_simt<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)a.ptr, (const __nv_bfloat16*)b.ptr, p);
-    else gemm_simt<__half><<<grid, 256, 0, s>>>((const __half*)a.ptr, (const __half*)b.ptr, p);
-    LB_CUDA(cudaGetLastError());
+    auto vec = [](const View3& v, long long along, long long across) {  // the strides the kernel fetches along and across
+        const uintptr_t group = v.dtype == LB_F32 ? 16 : 8;
+        return along == 1 && across % 4 == 0 && (v.batch == 1 || v.sb % 4 == 0) && (uintptr_t)v.ptr % group == 0;
+    };
+    p.a_vec = p.a_sk == 1 ? vec(a, p.a_sk, p.a_sm) : vec(a, p.a_sm, p.a_sk);
+    p.b_vec = p.b_sn == 1 ? vec(b, p.b_sn, p.b_sk) : vec(b, p.b_sk, p.b_sn);
+    gemm_simt(a.ptr, b.ptr, a.dtype, p, device_info().sms, s);
 }
 
 }  // namespace lb

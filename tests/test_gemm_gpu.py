@@ -36,6 +36,19 @@ def test_float32_gemm_is_bit_exact(cuda, shape):
     np.testing.assert_array_equal(to_numpy(out), oracle_matmul(a, b, "float32", "float32"))
 
 
+@pytest.mark.parametrize("shape", [(16, 32, 64), (17, 33, 65), (400, 410, 70), (416, 384, 128), (1100, 1121, 33), (1152, 1152, 64)])
+@pytest.mark.parametrize("majors", ["nn", "nt", "tn", "tt"])
+def test_float32_gemm_tiles_and_majors_are_bit_exact(cuda, shape, majors):
+    """Each tile size the CUDA-core kernel picks (few, some, many output tiles), whole and ragged, with either operand
+    contiguous along either axis (aligned groups of four and element by element)."""
+    m, n, k = shape
+    a, b = operands(m, n, k, 5)
+    ta, tb = (to_torch(x if major == "n" else np.ascontiguousarray(x.T), cuda) for x, major in zip((a, b), majors))
+    out = torch.full((m, n), float("nan"), dtype=torch.float32, device=cuda)
+    gemm(ta if majors[0] == "n" else ta.t(), tb if majors[1] == "n" else tb.t(), out)
+    np.testing.assert_array_equal(to_numpy(out), oracle_matmul(a, b, "float32", "float32"))
+
+
 def test_simt_bf16_gemm_is_bit_exact(cuda):
     a, b = operands(96, 80, 72, 1)
     a, b = bf16(a), bf16(b)
