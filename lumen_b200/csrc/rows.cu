@@ -6,13 +6,14 @@
 //    every add exactly like the interpreter: bit-identical to it and from run to run. The ATOMIC form adds in float32
 //    atomics in arrival order and rounds once: results vary in the last bits when a row is hit more than once.
 //  * attention_simt_fwd / attention_simt_bwd: float32 or bfloat16, any head dim up to 256, one warp per query row,
-//    scores and sums in float32 in key order. Used for float32 graphs (no hidden narrowing to bf16 tensor cores)
+//    scores and sums in float32. Used for float32 graphs (no hidden narrowing to bf16 tensor cores)
 //    and head dims other than 64/128.
 #include "device.h"
 
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 namespace lb {
 namespace {
@@ -155,172 +156,213 @@ struct AttnShape {
     float scale;
 };
 
-// one warp per (b, n, i): online softmax over the visible keys; lane l owns head-dim elements l, l+32, ...
-template <class T>
-__global__ void attention_simt_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ o,
-                                          float* __restrict__ lse, AttnShape s) {
-    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= (long long)s.B * s.N * s.Sq) return;
-    const int i = (int)(w % s.Sq), n = (int)((w / s.Sq) % s.N), b = (int)(w / ((long long)s.Sq * s.N));
-    const int nk = n / (s.N / s.Nkv);
-    const T* qp = q + b * s.q_s[0] + (long long)i * s.q_s[1] + n * s.q_s[2];
-    float qv[8], acc[8];
+// CUDA-core attention: one warp per row (a query of the forward and dQ kernels, a key of the dK/dV kernel), eight
+// neighbouring rows of one head per CTA. The rows they attend to stream through shared memory 32 at a time, as float32.
+// Within a chunk a lane first owns one streamed row (its dot products run over the head dimension without any exchange
+// between lanes), then head-dim elements l, l + 32, ... (the weighted sum over the chunk). A warp-wide sum per streamed
+// row, as one row at a time would need, is a chain of five shuffles: at 64 keys of 32 elements those chains were nine
+// tenths of the 48 us that the forward took.
+constexpr int kAttnRows = 8, kChunk = 32;
+
+// DU: head-dim elements per lane. Row pitch: a multiple of four floats whose 16-byte groups fall in different banks for
+// eight neighbouring rows.
+template <int DU>
+struct AttnSmem {
+    static constexpr int kD = DU * 32, kPitch = kD + 4;
+    float tile[2][kChunk * kPitch];   // streamed rows
+    float own[2][kAttnRows * kD];     // the warps' rows
+    float weight[2][kAttnRows][kChunk];
+};
+
+template <class T, int DU>
+__device__ __forceinline__ void load_chunk(float* dst, const T* base, long long stride, long long row0, long long end, int D) {
+    constexpr int kD = AttnSmem<DU>::kD;
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-        int d = lane + 32 * u;
-        qv[u] = d < s.D ? to_f(qp[d]) : 0.0f;
-        acc[u] = 0.0f;
+    for (int i = threadIdx.x; i < kChunk * kD; i += kAttnRows * 32) {
+        const int r = i / kD, d = i % kD;
+        dst[r * AttnSmem<DU>::kPitch + d] = row0 + r < end && d < D ? to_f(base[(row0 + r) * stride + d]) : 0.0f;
     }
-    long long last = s.causal ? min((long long)s.Sk - 1, (long long)i + s.offset) : (long long)s.Sk - 1;
-    float m = -INFINITY, l = 0.0f;
-    for (long long j = 0; j <= last; j++) {
-        const T* kp = k + b * s.k_s[0] + j * s.k_s[1] + nk * s.k_s[2];
-        float dot = 0.0f;
+}
+template <class T, int DU>
+__device__ __forceinline__ void load_own(float* dst, const T* row, bool live, int D, int lane) {  // this warp's row
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            int d = lane + 32 * u;
-            if (d < s.D) dot = fmaf(qv[u], to_f(kp[d]), dot);
+    for (int u = 0; u < DU; u++) dst[lane + 32 * u] = live && lane + 32 * u < D ? to_f(row[lane + 32 * u]) : 0.0f;
+}
+// the warp's own row times the chunk row this lane owns
+template <int DU>
+__device__ __forceinline__ float dot_row(const float* own, const float* tile, int lane) {
+    const float4* a = (const float4*)own;
+    const float4* b = (const float4*)(tile + lane * AttnSmem<DU>::kPitch);
+    float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll 8
+    for (int d = 0; d < DU * 8; d++) {
+        const float4 x = a[d], y = b[d];
+        s0 = fmaf(x.x, y.x, s0), s1 = fmaf(x.y, y.y, s1);
+        s0 = fmaf(x.z, y.z, s0), s1 = fmaf(x.w, y.w, s1);
+    }
+    return s0 + s1;
+}
+// acc[u] += sum over the chunk of weight[row] * tile[row][lane + 32 u], in row order
+template <int DU>
+__device__ __forceinline__ void add_weighted(float* acc, const float* weight, const float* tile, int lane) {
+#pragma unroll (DU > 2 ? 2 : 8)
+    for (int j = 0; j < kChunk; j += 4) {
+        const float4 w = *(const float4*)(weight + j);
+#pragma unroll
+        for (int u = 0; u < DU; u++) {
+            const float* t = tile + j * AttnSmem<DU>::kPitch + lane + 32 * u;
+            acc[u] = fmaf(w.x, t[0], acc[u]);
+            acc[u] = fmaf(w.y, t[AttnSmem<DU>::kPitch], acc[u]);
+            acc[u] = fmaf(w.z, t[2 * AttnSmem<DU>::kPitch], acc[u]);
+            acc[u] = fmaf(w.w, t[3 * AttnSmem<DU>::kPitch], acc[u]);
         }
+    }
+}
+// the CTA's rows: kAttnRows neighbours of one (batch, head)
+__device__ __forceinline__ void block_rows(int rows, int heads, int& r0, int& n, int& b) {
+    const int per = (rows + kAttnRows - 1) / kAttnRows;
+    r0 = (int)(blockIdx.x % per) * kAttnRows, n = (int)(blockIdx.x / per % heads), b = (int)(blockIdx.x / per / heads);
+}
+
+template <class T, int DU>
+__global__ void __launch_bounds__(kAttnRows * 32)
+attention_simt_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ o,
+                          float* __restrict__ lse, AttnShape s) {
+    extern __shared__ __align__(16) uint8_t raw[];
+    AttnSmem<DU>& sm = *(AttnSmem<DU>*)raw;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int i0, n, b;
+    block_rows(s.Sq, s.N, i0, n, b);
+    const int i = i0 + warp, nk = n / (s.N / s.Nkv);
+    const bool live = i < s.Sq;
+    float* own = sm.own[0] + warp * AttnSmem<DU>::kD;
+    load_own<T, DU>(own, q + b * s.q_s[0] + (long long)i * s.q_s[1] + n * s.q_s[2], live, s.D, lane);
+    const long long last = !live ? -1 : s.causal ? min((long long)s.Sk - 1, (long long)i + s.offset) : (long long)s.Sk - 1;
+    const long long end = s.causal ? min((long long)s.Sk, (long long)i0 + kAttnRows + s.offset) : (long long)s.Sk;  // past the CTA's last key
+    float acc[DU] = {}, m = -INFINITY, l = 0.0f;
+    for (long long j0 = 0; j0 < end; j0 += kChunk) {
+        __syncthreads();
+        load_chunk<T, DU>(sm.tile[0], k + b * s.k_s[0] + nk * s.k_s[2], s.k_s[1], j0, end, s.D);
+        load_chunk<T, DU>(sm.tile[1], v + b * s.v_s[0] + nk * s.v_s[2], s.v_s[1], j0, end, s.D);
+        __syncthreads();
+        if (j0 > last) continue;  // warp-uniform: this row sees nothing of the chunk
+        const float sc = j0 + lane <= last ? dot_row<DU>(own, sm.tile[0], lane) * s.scale : -INFINITY;
+        float top = sc;
 #pragma unroll
-        for (int x = 16; x >= 1; x >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, x);
-        const float sc = dot * s.scale;
-        const float m_new = fmaxf(m, sc);
-        const float alpha = __expf(m - m_new), p = __expf(sc - m_new);
-        // the value product sees the probability in the operands' dtype; the normaliser is applied at the end
-        l = l * alpha + p;
-        const T* vp = v + b * s.v_s[0] + j * s.v_s[1] + nk * s.v_s[2];
+        for (int x = 16; x >= 1; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
+        const float m_new = fmaxf(m, top);
+        const float alpha = __expf(m - m_new), p = j0 + lane <= last ? __expf(sc - m_new) : 0.0f;
+        sm.weight[0][warp][lane] = p;
+        float sum = p;
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            int d = lane + 32 * u;
-            if (d < s.D) acc[u] = fmaf(acc[u], alpha, p * to_f(vp[d]));
-        }
+        for (int x = 16; x >= 1; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
+        l = l * alpha + sum;
+#pragma unroll
+        for (int u = 0; u < DU; u++) acc[u] *= alpha;
+        __syncwarp();
+        // the normaliser is applied at the end
+        add_weighted<DU>(acc, sm.weight[0][warp], sm.tile[1], lane);
+        __syncwarp();
         m = m_new;
     }
+    if (!live) return;
     T* op = o + b * s.o_s[0] + (long long)i * s.o_s[1] + n * s.o_s[2];
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-        int d = lane + 32 * u;
-        if (d < s.D) op[d] = from_f<T>(acc[u] / l);
-    }
+    for (int u = 0; u < DU; u++)
+        if (lane + 32 * u < s.D) op[lane + 32 * u] = from_f<T>(acc[u] / l);
     if (lse && lane == 0) lse[((long long)b * s.N + n) * s.Sq + i] = m + logf(l);
 }
 
-// dQ: one warp per query row. dK/dV: one warp per (b, kv head, key j), looping over the group's heads and the queries that see j.
-template <class T>
-__global__ void attention_simt_dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ g,
-                                         const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dq, AttnShape s) {
-    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= (long long)s.B * s.N * s.Sq) return;
-    const int i = (int)(w % s.Sq), n = (int)((w / s.Sq) % s.N), b = (int)(w / ((long long)s.Sq * s.N));
-    const int nk = n / (s.N / s.Nkv);
-    const T* qp = q + b * s.q_s[0] + (long long)i * s.q_s[1] + n * s.q_s[2];
-    const T* gp = g + b * s.g_s[0] + (long long)i * s.g_s[1] + n * s.g_s[2];
-    float qv[8], gv[8], acc[8];
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-        int d = lane + 32 * u;
-        qv[u] = d < s.D ? to_f(qp[d]) : 0.0f;
-        gv[u] = d < s.D ? to_f(gp[d]) : 0.0f;
-        acc[u] = 0.0f;
-    }
+// dQ: one warp per query row.
+template <class T, int DU>
+__global__ void __launch_bounds__(kAttnRows * 32)
+attention_simt_dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ g,
+                         const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dq, AttnShape s) {
+    extern __shared__ __align__(16) uint8_t raw[];
+    AttnSmem<DU>& sm = *(AttnSmem<DU>*)raw;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int i0, n, b;
+    block_rows(s.Sq, s.N, i0, n, b);
+    const int i = i0 + warp, nk = n / (s.N / s.Nkv);
+    const bool live = i < s.Sq;
+    float *own_q = sm.own[0] + warp * AttnSmem<DU>::kD, *own_g = sm.own[1] + warp * AttnSmem<DU>::kD;
+    load_own<T, DU>(own_q, q + b * s.q_s[0] + (long long)i * s.q_s[1] + n * s.q_s[2], live, s.D, lane);
+    load_own<T, DU>(own_g, g + b * s.g_s[0] + (long long)i * s.g_s[1] + n * s.g_s[2], live, s.D, lane);
     const long long at = ((long long)b * s.N + n) * s.Sq + i;
-    const float L = lse[at], dl = delta[at];
-    long long last = s.causal ? min((long long)s.Sk - 1, (long long)i + s.offset) : (long long)s.Sk - 1;
-    for (long long j = 0; j <= last; j++) {
-        const T* kp = k + b * s.k_s[0] + j * s.k_s[1] + nk * s.k_s[2];
-        const T* vp = v + b * s.v_s[0] + j * s.v_s[1] + nk * s.v_s[2];
-        float dot = 0.0f, dp = 0.0f;
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            int d = lane + 32 * u;
-            if (d < s.D) {
-                dot = fmaf(qv[u], to_f(kp[d]), dot);
-                dp = fmaf(gv[u], to_f(vp[d]), dp);
-            }
+    const float L = live ? lse[at] : 0.0f, dl = live ? delta[at] : 0.0f;
+    const long long last = !live ? -1 : s.causal ? min((long long)s.Sk - 1, (long long)i + s.offset) : (long long)s.Sk - 1;
+    const long long end = s.causal ? min((long long)s.Sk, (long long)i0 + kAttnRows + s.offset) : (long long)s.Sk;
+    float acc[DU] = {};
+    for (long long j0 = 0; j0 < end; j0 += kChunk) {
+        __syncthreads();
+        load_chunk<T, DU>(sm.tile[0], k + b * s.k_s[0] + nk * s.k_s[2], s.k_s[1], j0, end, s.D);
+        load_chunk<T, DU>(sm.tile[1], v + b * s.v_s[0] + nk * s.v_s[2], s.v_s[1], j0, end, s.D);
+        __syncthreads();
+        if (j0 > last) continue;
+        float ds = 0.0f;
+        if (j0 + lane <= last) {
+            const float p = __expf(dot_row<DU>(own_q, sm.tile[0], lane) * s.scale - L);
+            ds = to_f(from_f<T>(p * (dot_row<DU>(own_g, sm.tile[1], lane) - dl) * s.scale));  // dS is rounded to the operands' dtype (flash.py:71)
         }
-#pragma unroll
-        for (int x = 16; x >= 1; x >>= 1) {
-            dot += __shfl_xor_sync(0xffffffffu, dot, x);
-            dp += __shfl_xor_sync(0xffffffffu, dp, x);
-        }
-        const float p = __expf(dot * s.scale - L);
-        const float ds = to_f(from_f<T>(p * (dp - dl) * s.scale));  // dS is rounded to the operands' dtype (flash.py:71)
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            int d = lane + 32 * u;
-            if (d < s.D) acc[u] = fmaf(ds, to_f(kp[d]), acc[u]);
-        }
+        sm.weight[0][warp][lane] = ds;
+        __syncwarp();
+        add_weighted<DU>(acc, sm.weight[0][warp], sm.tile[0], lane);
+        __syncwarp();
     }
+    if (!live) return;
     T* out = dq + b * s.dq_s[0] + (long long)i * s.dq_s[1] + n * s.dq_s[2];
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-        int d = lane + 32 * u;
-        if (d < s.D) out[d] = from_f<T>(acc[u]);
-    }
+    for (int u = 0; u < DU; u++)
+        if (lane + 32 * u < s.D) out[lane + 32 * u] = from_f<T>(acc[u]);
 }
 
-template <class T>
-__global__ void attention_simt_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ g,
-                                           const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dk,
-                                           T* __restrict__ dv, AttnShape s) {
-    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= (long long)s.B * s.Nkv * s.Sk) return;
-    const int j = (int)(w % s.Sk), nk = (int)((w / s.Sk) % s.Nkv), b = (int)(w / ((long long)s.Sk * s.Nkv));
-    const int group = s.N / s.Nkv;
-    const T* kp = k + b * s.k_s[0] + (long long)j * s.k_s[1] + nk * s.k_s[2];
-    const T* vp = v + b * s.v_s[0] + (long long)j * s.v_s[1] + nk * s.v_s[2];
-    float kv[8], vv[8], ak[8], av[8];
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-        int d = lane + 32 * u;
-        kv[u] = d < s.D ? to_f(kp[d]) : 0.0f;
-        vv[u] = d < s.D ? to_f(vp[d]) : 0.0f;
-        ak[u] = av[u] = 0.0f;
-    }
-    long long first = s.causal ? max(0LL, (long long)j - s.offset) : 0LL;
+// dK/dV: one warp per (b, kv head, key j), looping over the group's heads and the queries that see j.
+template <class T, int DU>
+__global__ void __launch_bounds__(kAttnRows * 32)
+attention_simt_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ g,
+                           const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dk, T* __restrict__ dv, AttnShape s) {
+    extern __shared__ __align__(16) uint8_t raw[];
+    AttnSmem<DU>& sm = *(AttnSmem<DU>*)raw;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int k0, nk, b;
+    block_rows(s.Sk, s.Nkv, k0, nk, b);
+    const int j = k0 + warp, group = s.N / s.Nkv;
+    const bool live = j < s.Sk;
+    float *own_k = sm.own[0] + warp * AttnSmem<DU>::kD, *own_v = sm.own[1] + warp * AttnSmem<DU>::kD;
+    load_own<T, DU>(own_k, k + b * s.k_s[0] + (long long)j * s.k_s[1] + nk * s.k_s[2], live, s.D, lane);
+    load_own<T, DU>(own_v, v + b * s.v_s[0] + (long long)j * s.v_s[1] + nk * s.v_s[2], live, s.D, lane);
+    float ak[DU] = {}, av[DU] = {};
+    const long long first = s.causal ? max(0LL, (long long)j - s.offset) : 0LL;       // the first query that sees this key
+    const long long begin = s.causal ? max(0LL, (long long)k0 - s.offset) : 0LL;      // ... that sees the CTA's first key
     for (int h = 0; h < group; h++) {
         const int n = nk * group + h;
-        for (long long i = first; i < s.Sq; i++) {
-            const T* qp = q + b * s.q_s[0] + i * s.q_s[1] + n * s.q_s[2];
-            const T* gp = g + b * s.g_s[0] + i * s.g_s[1] + n * s.g_s[2];
-            float dot = 0.0f, dp = 0.0f;
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                int d = lane + 32 * u;
-                if (d < s.D) {
-                    dot = fmaf(kv[u], to_f(qp[d]), dot);
-                    dp = fmaf(vv[u], to_f(gp[d]), dp);
-                }
+        for (long long i0 = begin; i0 < s.Sq; i0 += kChunk) {
+            __syncthreads();
+            load_chunk<T, DU>(sm.tile[0], q + b * s.q_s[0] + n * s.q_s[2], s.q_s[1], i0, s.Sq, s.D);
+            load_chunk<T, DU>(sm.tile[1], g + b * s.g_s[0] + n * s.g_s[2], s.g_s[1], i0, s.Sq, s.D);
+            __syncthreads();
+            if (!live || i0 + kChunk <= first) continue;
+            const long long i = i0 + lane;
+            float ds = 0.0f, pr = 0.0f;
+            if (i >= first && i < s.Sq) {
+                const long long at = ((long long)b * s.N + n) * s.Sq + i;
+                const float p = __expf(dot_row<DU>(own_k, sm.tile[0], lane) * s.scale - lse[at]);
+                ds = to_f(from_f<T>(p * (dot_row<DU>(own_v, sm.tile[1], lane) - delta[at]) * s.scale));
+                pr = to_f(from_f<T>(p));
             }
-#pragma unroll
-            for (int x = 16; x >= 1; x >>= 1) {
-                dot += __shfl_xor_sync(0xffffffffu, dot, x);
-                dp += __shfl_xor_sync(0xffffffffu, dp, x);
-            }
-            const long long at = ((long long)b * s.N + n) * s.Sq + i;
-            const float p = __expf(dot * s.scale - lse[at]);
-            const float ds = to_f(from_f<T>(p * (dp - delta[at]) * s.scale));
-            const float pr = to_f(from_f<T>(p));
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                int d = lane + 32 * u;
-                if (d < s.D) {
-                    ak[u] = fmaf(ds, to_f(qp[d]), ak[u]);
-                    av[u] = fmaf(pr, to_f(gp[d]), av[u]);
-                }
-            }
+            sm.weight[0][warp][lane] = ds, sm.weight[1][warp][lane] = pr;
+            __syncwarp();
+            add_weighted<DU>(ak, sm.weight[0][warp], sm.tile[0], lane);
+            add_weighted<DU>(av, sm.weight[1][warp], sm.tile[1], lane);
+            __syncwarp();
         }
     }
+    if (!live) return;
     T* ok = dk + b * s.dk_s[0] + (long long)j * s.dk_s[1] + nk * s.dk_s[2];
     T* ov = dv + b * s.dv_s[0] + (long long)j * s.dv_s[1] + nk * s.dv_s[2];
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-        int d = lane + 32 * u;
-        if (d < s.D) ok[d] = from_f<T>(ak[u]), ov[d] = from_f<T>(av[u]);
-    }
+    for (int u = 0; u < DU; u++)
+        if (lane + 32 * u < s.D) ok[lane + 32 * u] = from_f<T>(ak[u]), ov[lane + 32 * u] = from_f<T>(av[u]);
 }
 
 template <class T>
@@ -580,17 +622,58 @@ void strided_copy(const lb_tensor& in, const lb_tensor& out, void* stream) {
     LB_CUDA(cudaGetLastError());
 }
 
+namespace {
+// CTAs of kAttnRows rows over `rows` rows of every (batch, head)
+unsigned attn_blocks(long long batch, long long heads, long long rows) {
+    const long long blocks = batch * heads * ((rows + kAttnRows - 1) / kAttnRows);
+    if (blocks > INT32_MAX) fail(LB_ERR_UNSUPPORTED, "attention: too many rows for the CUDA-core kernels' grid");
+    return (unsigned)blocks;
+}
+template <int DU, class Kernel, class... Args>
+void launch_attn(Kernel kernel, unsigned blocks, cudaStream_t st, Args... args) {
+    constexpr int bytes = (int)sizeof(AttnSmem<DU>);
+    if (bytes > 48 * 1024 && first_use_on_device((const void*)kernel))
+        LB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    kernel<<<blocks, kAttnRows * 32, bytes, st>>>(args...);
+}
+// calls `f` with the head-dim elements per lane as a compile-time number: 1, 2, 4 or 8
+template <class F>
+void with_dims_per_lane(int D, F&& f) {
+    if (D <= 32) f(std::integral_constant<int, 1>());
+    else if (D <= 64) f(std::integral_constant<int, 2>());
+    else if (D <= 128) f(std::integral_constant<int, 4>());
+    else f(std::integral_constant<int, 8>());
+}
+template <class T>
+void simt_fwd(const AttnShape& s, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o, float* lse, cudaStream_t st) {
+    with_dims_per_lane(s.D, [&](auto du) {
+        launch_attn<du>(attention_simt_fwd_kernel<T, du>, attn_blocks(s.B, s.N, s.Sq), st, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr, (T*)o.ptr, lse, s);
+    });
+}
+template <class T>
+void simt_bwd(const AttnShape& s, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o, const lb_tensor& g,
+              const float* lse, float* delta, const lb_tensor& dq, const lb_tensor& dk, const lb_tensor& dv, cudaStream_t st) {
+    const long long warps = (long long)s.B * s.N * s.Sq;
+    attention_delta_simt<T><<<(unsigned)((warps * 32 + 255) / 256), 256, 0, st>>>((const T*)o.ptr, (const T*)g.ptr, delta, s);
+    with_dims_per_lane(s.D, [&](auto du) {
+        launch_attn<du>(attention_simt_dq_kernel<T, du>, attn_blocks(s.B, s.N, s.Sq), st, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr,
+                        (const T*)g.ptr, lse, (const float*)delta, (T*)dq.ptr, s);
+        launch_attn<du>(attention_simt_dkdv_kernel<T, du>, attn_blocks(s.B, s.Nkv, s.Sk), st, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr,
+                        (const T*)g.ptr, lse, (const float*)delta, (T*)dk.ptr, (T*)dv.ptr, s);
+    });
+}
+}  // namespace
+
 void attention_simt_fwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o,
                         const lb_tensor* lse, void* stream) {
     AttnShape s = attn_shape(desc, q, k, v);
     fill_strides(s.o_s, o);
     driver();
-    const long long warps = (long long)s.B * s.N * s.Sq;
-    if (warps == 0) return;
-    const unsigned blocks = (unsigned)((warps * 32 + 255) / 256);
+    if ((long long)s.B * s.N * s.Sq == 0) return;
     cudaStream_t st = (cudaStream_t)stream;
-    if (q.dtype == LB_F32) attention_simt_fwd_kernel<float><<<blocks, 256, 0, st>>>((const float*)q.ptr, (const float*)k.ptr, (const float*)v.ptr, (float*)o.ptr, lse ? (float*)lse->ptr : nullptr, s);
-    else if (q.dtype == LB_BF16) attention_simt_fwd_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)q.ptr, (const __nv_bfloat16*)k.ptr, (const __nv_bfloat16*)v.ptr, (__nv_bfloat16*)o.ptr, lse ? (float*)lse->ptr : nullptr, s);
+    float* out_lse = lse ? (float*)lse->ptr : nullptr;
+    if (q.dtype == LB_F32) simt_fwd<float>(s, q, k, v, o, out_lse, st);
+    else if (q.dtype == LB_BF16) simt_fwd<__nv_bfloat16>(s, q, k, v, o, out_lse, st);
     else fail(LB_ERR_UNSUPPORTED, "attention: float32 or bfloat16 operands");
     LB_CUDA(cudaGetLastError());
 }
@@ -602,21 +685,10 @@ void attention_simt_bwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_t
     fill_strides(s.o_s, o), fill_strides(s.g_s, g), fill_strides(s.dq_s, dq), fill_strides(s.dk_s, dk), fill_strides(s.dv_s, dv);
     driver();
     cudaStream_t st = (cudaStream_t)stream;
-    const long long qw = (long long)s.B * s.N * s.Sq, kw = (long long)s.B * s.Nkv * s.Sk;
-    if (qw == 0 || kw == 0) return;
-    const unsigned qb = (unsigned)((qw * 32 + 255) / 256), kb = (unsigned)((kw * 32 + 255) / 256);
-    if (q.dtype == LB_F32) {
-        attention_delta_simt<float><<<qb, 256, 0, st>>>((const float*)o.ptr, (const float*)g.ptr, (float*)delta.ptr, s);
-        attention_simt_dq_kernel<float><<<qb, 256, 0, st>>>((const float*)q.ptr, (const float*)k.ptr, (const float*)v.ptr, (const float*)g.ptr, (const float*)lse.ptr, (const float*)delta.ptr, (float*)dq.ptr, s);
-        attention_simt_dkdv_kernel<float><<<kb, 256, 0, st>>>((const float*)q.ptr, (const float*)k.ptr, (const float*)v.ptr, (const float*)g.ptr, (const float*)lse.ptr, (const float*)delta.ptr, (float*)dk.ptr, (float*)dv.ptr, s);
-    } else if (q.dtype == LB_BF16) {
-        typedef __nv_bfloat16 H;
-        attention_delta_simt<H><<<qb, 256, 0, st>>>((const H*)o.ptr, (const H*)g.ptr, (float*)delta.ptr, s);
-        attention_simt_dq_kernel<H><<<qb, 256, 0, st>>>((const H*)q.ptr, (const H*)k.ptr, (const H*)v.ptr, (const H*)g.ptr, (const float*)lse.ptr, (const float*)delta.ptr, (H*)dq.ptr, s);
-        attention_simt_dkdv_kernel<H><<<kb, 256, 0, st>>>((const H*)q.ptr, (const H*)k.ptr, (const H*)v.ptr, (const H*)g.ptr, (const float*)lse.ptr, (const float*)delta.ptr, (H*)dk.ptr, (H*)dv.ptr, s);
-    } else {
-        fail(LB_ERR_UNSUPPORTED, "attention: float32 or bfloat16 operands");
-    }
+    if ((long long)s.B * s.N * s.Sq == 0 || (long long)s.B * s.Nkv * s.Sk == 0) return;
+    if (q.dtype == LB_F32) simt_bwd<float>(s, q, k, v, o, g, (const float*)lse.ptr, (float*)delta.ptr, dq, dk, dv, st);
+    else if (q.dtype == LB_BF16) simt_bwd<__nv_bfloat16>(s, q, k, v, o, g, (const float*)lse.ptr, (float*)delta.ptr, dq, dk, dv, st);
+    else fail(LB_ERR_UNSUPPORTED, "attention: float32 or bfloat16 operands");
     LB_CUDA(cudaGetLastError());
 }
 

@@ -277,3 +277,32 @@ def test_random_attention_shapes_against_float64(cuda, seed):
         for result in (a, s):
             np.testing.assert_allclose(to_numpy(result).astype(np.float64), w, rtol=TOL, atol=TOL * max(np.abs(w).max(), 2.0**-8), err_msg=name)
         assert torch.equal(a, a2), name
+
+
+# (B, Sq, Sk, N, Nkv, H): the CUDA-core kernels' edges - rows per CTA (8), streamed chunks (32), head-dim elements per lane
+SIMT_CASES = [((1, 8, 32, 1, 1, 32), True), ((2, 9, 33, 2, 1, 33), True), ((1, 7, 31, 3, 3, 1), False), ((1, 65, 64, 2, 2, 65), False),
+              ((1, 40, 40, 4, 2, 129), True), ((1, 33, 70, 1, 1, 256), True)]
+
+
+@pytest.mark.parametrize("case", SIMT_CASES)
+def test_cuda_core_attention_against_float64(cuda, case):
+    """float32 operands: every result within 2e-5 of its largest value. A score is a float32 sum of H <= 256 products of
+    size about 1 / sqrt(H) each (error under 256 * 2^-24 = 1.5e-5 of a score, typically its square root), and __expf is
+    accurate to 2 ulp + 2^-21 |x|."""
+    (b, sq, sk, n, nkv, h), causal = case
+    rng = np.random.default_rng(h)
+    q, k, v, do = (rng.standard_normal(s).astype(np.float32) for s in ((b, sq, n, h), (b, sk, nkv, h), (b, sk, nkv, h), (b, sq, n, h)))
+    tq, tk, tv, tdo = (to_torch(x, cuda) for x in (q, k, v, do))
+    o, lse = attention_forward(tq, tk, tv, causal=causal)
+    grads = attention_backward(tq, tk, tv, o, tdo, lse, causal=causal)
+    device_status()
+    x = [torch.from_numpy(a.astype(np.float64)).requires_grad_(True) for a in (q, k, v)]
+    qq, kk, vv = x[0].transpose(1, 2), x[1].repeat_interleave(n // nkv, 2).transpose(1, 2), x[2].repeat_interleave(n // nkv, 2).transpose(1, 2)
+    s = qq @ kk.transpose(-1, -2) * h**-0.5
+    if causal:
+        s = s.masked_fill(torch.arange(sk)[None, :] > torch.arange(sq)[:, None] + sk - sq, float("-inf"))
+    out = (torch.softmax(s, -1) @ vv).transpose(1, 2)
+    out.backward(torch.from_numpy(do.astype(np.float64)))
+    for name, got, want in zip(("o", "lse", "dq", "dk", "dv"), (o, lse, *grads), (out, torch.logsumexp(s, -1), *(t.grad for t in x))):
+        want = want.detach().numpy()
+        assert np.abs(to_numpy(got) - want).max() <= 2e-5 * max(np.abs(want).max(), 1.0), name
