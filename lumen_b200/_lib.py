@@ -48,6 +48,25 @@ class LumenError(RuntimeError):
 
 
 _lib = None
+_host = None
+
+
+def host():
+    """The native call path (`_host.so` beside the library), set up on first use."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            from lumen_b200 import _host as module
+        except ImportError as e:
+            raise ImportError("lumen_b200/_host.so is missing or does not load: build it with `make -C lumen_b200/csrc`") from e
+        from lumen_b200.runtime import current_stream, dtype_name
+
+        codes = dict(DTYPE_CODES)
+        module.setup(codes, lambda d: DTYPE_CODES[dtype_name(d)], check, current_stream, None)
+        module.for_torch = lambda raw: module.setup(codes, lambda d: DTYPE_CODES[dtype_name(d)], check, current_stream, raw)
+        _host = module
+    return _host
 
 
 def lib():
@@ -109,11 +128,4 @@ def dense(ptr: int, dtype: str, shape) -> LbTensor:
 
 
 def strided(ptr: int, dtype: str, shape, strides) -> LbTensor:
-    t = LbTensor()
-    t.ptr = ptr
-    t.dtype = DTYPE_CODES[dtype]
-    t.rank = len(shape)
-    for d in range(len(shape)):
-        t.shape[d] = shape[d]
-        t.stride[d] = strides[d]
-    return t
+    return LbTensor(ptr, DTYPE_CODES[dtype], len(shape), shape, strides)  # array fields take tuples of up to MAX_RANK numbers

@@ -11,7 +11,9 @@ Non-tensor arguments are static: they are part of the signature.
 
 from __future__ import annotations
 
-from lumen_b200 import tracer
+import sys
+
+from lumen_b200 import _lib, runtime, tracer
 from lumen_b200.compiler import compile_graph
 from lumen_b200.device import Tensor as DeviceTensor
 from lumen_b200.plan import Plan
@@ -24,6 +26,23 @@ def _is_torch(a) -> bool:
 
 def _is_tensor(a) -> bool:
     return isinstance(a, DeviceTensor) or _is_torch(a)
+
+
+def _on_current_gpu(a, device) -> bool:
+    """Whether `.to(device)` would return the torch tensor `a` itself."""
+    if not a.is_cuda:
+        return False
+    torch = sys.modules["torch"]
+    return device == "cuda" and (torch.cuda.device_count() == 1 or a.get_device() == torch.cuda.current_device())
+
+
+_tensor_types: dict = {}  # argument types met that are tensors -> whether they are torch's
+
+
+def _device_index() -> int:
+    """What `CallTable.call` checks torch arguments against: the current device, or -1 in a process with one GPU."""
+    torch = sys.modules.get("torch")
+    return -1 if torch is None or torch.cuda.device_count() <= 1 else torch.cuda.current_device()
 
 
 class _Signature:
@@ -57,6 +76,7 @@ class _Signature:
         self.results = [_empty_like_input(like, self.graph.types[v].shape, self.graph.types[v].dtype) for v in self.graph.outputs]
         self.recorded = None
         self.bound_to = None
+        self.returned = self.results[0] if len(self.results) == 1 else tuple(self.results)
 
 
 class Compiled:
@@ -68,23 +88,45 @@ class Compiled:
             raise ValueError("lumen_b200 compiles for device=\"cuda\" only (there is no CPU fallback)")
         self.fn, self.device, self.use_graphs, self.lowering = fn, device, use_graphs, lowering
         self.signatures: dict = {}
-        self.latest: _Signature | None = None
+        self.calls = _lib.host().CallTable()  # the signatures of tensors only, found and run natively
+
+    @property
+    def latest(self) -> _Signature | None:
+        return self.calls.latest
 
     def __call__(self, *args):
+        out = self.calls.call(args, runtime._current[0], _device_index())
+        return out if out is not None else self._general_call(args)
+
+    def _general_call(self, args):
         require_cuda()
         # any array that speaks DLPack (the reference's tensors import and export it, lumen/tensor/dlpack.rs) is taken
         # in place, without a copy when it already lives on this device
-        if any(not _is_tensor(a) and hasattr(a, "__dlpack__") for a in args):
-            import torch  # the DLPack importer of a harness that passes foreign arrays
+        key, inputs = [], []
+        for a in args:
+            kind = type(a)
+            if kind not in _tensor_types:
+                if not _is_tensor(a):
+                    if hasattr(a, "__dlpack__"):
+                        import torch  # the DLPack importer of a harness that passes foreign arrays
 
-            args = tuple(torch.from_dlpack(a) if not _is_tensor(a) and hasattr(a, "__dlpack__") else a for a in args)
-        key = tuple((dtype_name(a.dtype), tuple(a.shape)) if _is_tensor(a) else ("static", a) for a in args)
+                        return self._general_call([torch.from_dlpack(x) if not _is_tensor(x) and hasattr(x, "__dlpack__") else x for x in args])
+                    key.append(("static", a))
+                    continue
+                _tensor_types[kind] = not isinstance(a, DeviceTensor)
+            key.append((dtype_name(a.dtype), a.shape))
+            inputs.append(a)
+        key = tuple(key)
         sig = self.signatures.get(key)
         if sig is None:
             sig = self.signatures[key] = _Signature(self.fn, args, self.device, self.lowering)
-        self.latest = sig
-        inputs = [a.to(self.device).contiguous() if _is_torch(a) else a for a in args if _is_tensor(a)]
-        pointers = tuple(t.data_ptr() for t in inputs)
+            if not self.use_graphs and len(inputs) == len(args):
+                self._add(sig, inputs)
+        self.calls.latest = sig
+        for k, a in enumerate(inputs):
+            if _tensor_types[type(a)] and not (_on_current_gpu(a, self.device) and a.is_contiguous()):
+                inputs[k] = a.to(self.device).contiguous()
+        pointers = [t.data_ptr() for t in inputs]
         if self.use_graphs and sig.bound_to == pointers and sig.recorded is not None:
             sig.recorded.launch()  # the same argument memory as the recorded call: one graph launch
         else:
@@ -93,8 +135,18 @@ class Compiled:
             if self.use_graphs and sig.bound_to == pointers:
                 sig.recorded = sig.plan.record(bound)  # second call with these pointers: record for the next ones
             sig.bound_to, sig.keep = pointers, (inputs, bound)
-        outs = sig.results
-        return outs[0] if len(outs) == 1 else tuple(outs)
+        return sig.returned
+
+    def _add(self, sig, inputs):
+        """Calls with arguments like these from now on run natively."""
+        torches = tuple(_tensor_types[type(a)] for a in inputs)
+        if any(torches):
+            torch = sys.modules["torch"]
+            if self.device != "cuda" or (torch.cuda.device_count() > 1 and not all(torches)):
+                return
+            _lib.host().for_torch(getattr(torch._C, "_cuda_getCurrentRawStream", None))
+        self.calls.add(tuple(inputs), torches, sig.plan.handle.value, sig.plan.workspace_ptr, tuple(t.data_ptr() for t in sig.results),
+                       sig, sig.returned)
 
     def __str__(self) -> str:
         return self.latest.graph.to_text() if self.latest else "<not traced yet>"

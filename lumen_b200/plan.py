@@ -106,7 +106,7 @@ class Plan:
 
             self.region = region if region is not None else Region(max(self.workspace_bytes, 256) + 256)
             workspace = self.region.empty((max(self.workspace_bytes, 256),), "uint8")
-        self.workspace = workspace
+        self.workspace, self.workspace_ptr = workspace, workspace.data_ptr()
         if self.workspace.data_ptr() % self.lib.lb_plan_workspace_alignment(self.handle):
             raise ValueError("the workspace must be 256-byte aligned")
         self.num_steps = self.lib.lb_plan_num_steps(self.handle)
@@ -137,13 +137,9 @@ class Plan:
         return ins, len(inputs), outs, len(outputs)
 
     def run_bound(self, bound, first=0, last=-1, stream=None):
-        ins, n_in, outs, n_out = bound
-        _lib.check(
-            self.lib.lb_plan_run(
-                self.handle, self.workspace.data_ptr(), ins, n_in, outs, n_out, first, last,
-                current_stream() if stream is None else stream,
-            )
-        )  # fmt: skip
+        status = self.lib.lb_plan_run(self.handle, self.workspace_ptr, *bound, first, last, current_stream() if stream is None else stream)
+        if status:
+            _lib.check(status)
 
     def autotune(self, bound, stream=None) -> list:
         """Times the candidate configurations of the plan's large GEMM steps on its own buffers and keeps the fastest

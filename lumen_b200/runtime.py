@@ -30,26 +30,38 @@ class _TorchDtypes(dict):
 TORCH_DTYPES = _TorchDtypes()
 
 
+_names: dict = {}  # dtype object -> lumen dtype name, as they are met
+
+
 def dtype_name(dtype) -> str:
     """The lumen dtype name of a tensor's `dtype` attribute (a name already, or another framework's dtype object)."""
     if isinstance(dtype, str):
         return dtype
-    name = str(dtype).rsplit(".", 1)[-1]  # "torch.bfloat16" -> "bfloat16"
-    if name not in _lib.DTYPE_CODES:
-        raise TypeError(f"no lumen dtype for {dtype!r}")
+    name = _names.get(dtype)
+    if name is None:
+        name = str(dtype).rsplit(".", 1)[-1]  # "torch.bfloat16" -> "bfloat16"
+        if name not in _lib.DTYPE_CODES:
+            raise TypeError(f"no lumen dtype for {dtype!r}")
+        _names[dtype] = name
     return name
 
 
+_cuda_seen = False
+
+
 def require_cuda() -> None:
-    if _lib.lib().lb_device_count() <= 0:
-        raise RuntimeError("lumen_b200 runs on a B200 GPU only: no CUDA device is available and there is no CPU fallback")
+    global _cuda_seen
+    if not _cuda_seen:  # the devices of a process do not go away
+        if _lib.lib().lb_device_count() <= 0:
+            raise RuntimeError("lumen_b200 runs on a B200 GPU only: no CUDA device is available and there is no CPU fallback")
+        _cuda_seen = True
 
 
 def desc(t) -> _lib.LbTensor:
     """The lb_tensor descriptor of a device tensor (shape, element strides, data pointer)."""
     if not getattr(t, "is_cuda", True):
         raise ValueError("expected a CUDA tensor")
-    return _lib.strided(t.data_ptr(), dtype_name(t.dtype), tuple(t.shape), tuple(t.stride()))
+    return _lib.strided(t.data_ptr(), dtype_name(t.dtype), t.shape, t.stride())
 
 
 _current = [0]
@@ -63,10 +75,16 @@ def set_current_stream(stream) -> None:
 def current_stream() -> int:
     """The caller's current stream: torch's when the process uses torch (a harness), else the one set with
     `set_current_stream` (the legacy default stream by default)."""
-    torch = sys.modules.get("torch")
-    if torch is not None and _current[0] == 0 and torch.cuda.is_initialized():
-        return torch.cuda.current_stream().cuda_stream
+    if _current[0] == 0:
+        torch = sys.modules.get("torch")
+        if torch is not None and torch.cuda.is_initialized():
+            raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # the handle without a Stream object around it
+            return raw(torch.cuda.current_device()) if raw is not None else torch.cuda.current_stream().cuda_stream
     return _current[0]
+
+
+def _stream(stream) -> int:
+    return (current_stream() if stream is None else getattr(stream, "handle", stream)) or 0
 
 
 class Fusion:
@@ -118,9 +136,7 @@ def _empty_like_input(like, shape, dtype: str):
     """A new dense device tensor of `shape`/`dtype` in the framework `like` comes from: torch for a torch tensor (the
     harness's convenience), else the backend's own region (grown in 256 MiB reservations)."""
     if type(like).__module__.startswith("torch"):
-        import torch
-
-        return torch.empty(tuple(shape), dtype=TORCH_DTYPES[dtype], device=like.device)
+        return sys.modules["torch"].empty(shape, dtype=TORCH_DTYPES[dtype], device=like.device)
     from lumen_b200.device import ITEMSIZE, Region
 
     import math
@@ -145,22 +161,8 @@ def gemm(a, b, out, epilogue=None, kernel="auto", stream=None, scratch=None, aux
     uint8 tensor of `gemm_scratch_bytes` bytes) lets few-tile, long-K problems split K. Epilogues: "relu";
     "add" (`round(product) + aux`) and "mask_positive" (`aux > 0 ? round(product) : 0`) with `aux` shaped like `out`."""
     require_cuda()
-    o = _lib.LbGemmOut()
-    o.product = desc(out)
-    o.epilogue = EPILOGUES[epilogue]
-    if aux is not None:
-        o.aux = desc(aux)
-    cfg = _lib.LbGemmCfg()
-    cfg.kernel = GEMM_KERNELS[kernel]
-    if scratch is not None:
-        cfg.scratch, cfg.scratch_bytes = scratch.data_ptr(), scratch.numel() * scratch.element_size()
-    da, db = desc(a), desc(b)
-    _lib.check(
-        _lib.lib().lb_gemm(
-            ctypes.byref(da), ctypes.byref(db), ctypes.byref(o), ctypes.byref(cfg),
-            current_stream() if stream is None else stream,
-        )
-    )  # fmt: skip
+    scratch_ptr, scratch_bytes = (scratch.data_ptr(), scratch.numel() * scratch.element_size()) if scratch is not None else (0, 0)
+    _lib.host().gemm(a, b, out, aux, EPILOGUES[epilogue], GEMM_KERNELS[kernel], scratch_ptr, scratch_bytes, _stream(stream))
     return out
 
 
@@ -179,17 +181,7 @@ def attention_forward(q, k, v, scale=None, causal=False, out=None, lse=None, str
         out = _empty_like_input(q, (b, sq, n, h), dtype_name(q.dtype))
     if lse is None:
         lse = _empty_like_input(q, (b, n, sq), "float32")
-    d = _lib.LbAttnDesc()
-    d.scale = float(scale if scale is not None else h**-0.5)
-    d.causal = int(bool(causal))
-    d.causal_offset = sk - sq
-    dq, dk, dv, do, dl = desc(q), desc(k), desc(v), desc(out), desc(lse)
-    _lib.check(
-        _lib.lib().lb_attention_fwd(
-            ctypes.byref(d), ctypes.byref(dq), ctypes.byref(dk), ctypes.byref(dv), ctypes.byref(do), ctypes.byref(dl),
-            current_stream() if stream is None else stream,
-        )
-    )  # fmt: skip
+    _lib.host().attention_fwd(float(scale if scale is not None else h**-0.5), bool(causal), sk - sq, q, k, v, out, lse, _stream(stream))
     return out, lse
 
 
@@ -204,17 +196,9 @@ def attention_backward(q, k, v, o, d_o, lse, scale=None, causal=False, delta=Non
     dq, dk, dv = (_empty_like_input(t, tuple(t.shape), dtype_name(t.dtype)) for t in (q, k, v))
     if delta is None:
         delta = _empty_like_input(q, (b, n, sq), "float32")
-    d = _lib.LbAttnDesc()
-    d.scale = float(scale if scale is not None else h**-0.5)
-    d.causal = int(bool(causal))
-    d.causal_offset = sk - sq
-    tensors = [q, k, v, o, d_o, lse, delta, dq, dk, dv]
-    entry = _lib.lib().lb_attention_bwd
-    if not deterministic:
-        tensors.insert(7, _empty_like_input(q, (b, sq, n, h), "float32"))
-        entry = _lib.lib().lb_attention_bwd_atomic
-    descs = [desc(t) for t in tensors]
-    _lib.check(entry(ctypes.byref(d), *[ctypes.byref(x) for x in descs], current_stream() if stream is None else stream))
+    dq_accum = None if deterministic else _empty_like_input(q, (b, sq, n, h), "float32")
+    _lib.host().attention_bwd(float(scale if scale is not None else h**-0.5), bool(causal), sk - sq, q, k, v, o, d_o, lse, delta,
+                              dq_accum, dq, dk, dv, _stream(stream))
     return dq, dk, dv
 
 
