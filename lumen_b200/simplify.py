@@ -10,7 +10,8 @@ Every rewrite here leaves each remaining value bit-identical when the graph is e
   pass re-traces broadcasts, iotas and constants the forward already has);
 * `simplify`: `reshape` to the operand's own shape, `transpose` by the identity, `cast` to the operand's own dtype and
   `broadcast_in_dim` to the same shape are removed; a transpose of a transpose becomes one; a reshape of a reshape
-  becomes one; `cast(dot_general(..), t)` with the product used nowhere else becomes the product's `output_dtype`
+  becomes one; the transpose of a product used nowhere else becomes the product of the swapped operands;
+  `cast(dot_general(..), t)` with the product used nowhere else becomes the product's `output_dtype`
   (the accumulator is rounded once either way).
 """
 
@@ -115,6 +116,19 @@ def simplify(graph: G.Graph) -> G.Graph:
             first = tuple(inner.params["permutation"])
             second = tuple(n.params["permutation"])
             n = G.Node("transpose", (src(inner.inputs[0]),), n.output, {"permutation": tuple(first[p] for p in second)})
+        elif (n.op == "transpose" and tuple(n.params["permutation"]) == (1, 0) and inner is not None and inner.op == "dot_general"
+              and uses.get(inner.output, 0) == 1 and types[inner.inputs[0]].dtype in ("bfloat16", "float16") and inner in nodes):
+            # a transposed product (a weight gradient) is the product of the swapped operands: the same sums of the same
+            # products in the same order, without a pass over the result. 16-bit operands only: at 1024 x 4096 the pass
+            # took as long as half the tensor-core product; beside a CUDA-core product of float32 it does not show.
+            at = nodes.index(inner)
+            params = dict(inner.params)
+            for side in ("contracting", "batch"):
+                params["lhs_" + side], params["rhs_" + side] = inner.params["rhs_" + side], inner.params["lhs_" + side]
+            nodes[at] = G.Node("dot_general", inner.inputs[::-1], n.output, params)
+            producer[n.output] = nodes[at]
+            dropped.add(inner.output)
+            continue
         elif n.op == "reshape" and inner is not None and inner.op == "reshape" and inner.output not in dropped:
             n = G.Node("reshape", (src(inner.inputs[0]),), n.output, dict(n.params))
         elif (n.op == "cast" and inner is not None and inner.op == "dot_general" and uses.get(inner.output, 0) == 1
