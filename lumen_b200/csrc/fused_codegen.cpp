@@ -298,6 +298,10 @@ class Generator {
         std::vector<std::pair<int, int>> full_outputs, row_outputs;  // (output position, value)
         for (size_t k = 0; k < g_.outputs.size(); k++) {
             const TensorType& t = g_.type(g_.outputs[k]);
+            if (behind_columns_.count(g_.outputs[k])) {
+                column_outputs_.push_back((int)k);
+                continue;
+            }
             if (t.numel() == R_ * C_ && (C_ != 1 || !has_reduce_)) full_outputs.push_back({(int)k, g_.outputs[k]});
             else if (t.numel() == R_) row_outputs.push_back({(int)k, g_.outputs[k]});
             else
@@ -333,6 +337,21 @@ class Generator {
             home->post += format("if (active) stv<%s, VEC>((%s*)out%d + (r * (idx_t)NCOLS + c0), %s);\n", ct.memory,
                                  ct.memory, k, buf.c_str());
         }
+        // Column sums: a thread keeps its columns for all the rows its CTA walks, so the partial sums stay in registers.
+        for (size_t k = 0; k < col_reduces_.size(); k++) {
+            const Node& n = *g_.node_of(col_reduces_[k]);
+            Index idx = column_operand_index(g_.type(n.inputs[0]), n.ints("axes").size());
+            Phase* home = &main_phase;
+            for (Phase& ph : phases_)
+                if (ph.chunked && ph.memo.count(key_of(n.inputs[0], idx))) {
+                    home = &ph;
+                    break;
+                }
+            main_used |= home == &main_phase;
+            std::string val = gen(n.inputs[0], idx, *home), init, combine;
+            reduce_ops(n, g_.type(n.output), &init, &combine);
+            home->body += "if (active) {\n" + accumulate(format("cacc%d[ch][e]", (int)k), combine, val) + "}\n";
+        }
         if (main_used) phases_.push_back(main_phase);
         if (!row_outputs.empty()) phases_.push_back(epilogue);
         return emit();
@@ -356,16 +375,42 @@ class Generator {
     std::map<std::string, std::string> cached_loads_;
     int cached_regs_ = 0;
 
+    // Row and column reductions in one kernel: the values read from column totals (generated in fused_finalize), and the
+    // outputs among them by position.
+    std::set<int> behind_columns_;
+    std::vector<int> column_outputs_;
+    // Values of a phase that a later phase of the same row reads again and that cost more to compute than to keep: by
+    // key, the row-scope array they are kept in.
+    std::map<std::string, std::string> kept_;
+    int kept_regs_ = 0;
+    int resident_ = 1;  // CTAs per SM a kernel with column sums is built for and launched with
+
     std::string fresh(const char* prefix) { return format("%s%d", prefix, counter_++); }
 
     // ---- iteration space ----------------------------------------------------------------------------------
     void plan_space() {
         const TensorType* space = nullptr;
+        int64_t col_r = -1, col_c = -1;
         for (const Node& n : g_.nodes) {
+            for (int v : n.inputs)
+                if (behind_columns_.count(v)) behind_columns_.insert(n.output);
             if (n.op != "reduce_sum" && n.op != "reduce_max") continue;
             const TensorType& x = g_.type(n.inputs[0]);
             auto axes = n.ints("axes");
             std::sort(axes.begin(), axes.end());
+            int lead = 0;
+            if (mixed_ && leading_axes(n, x, &lead)) {
+                int64_t r = 1;
+                for (int d = 0; d < lead; d++) r *= x.shape[d];
+                const int64_t c = r ? x.numel() / r : 0;
+                if (!r || !c || (col_r >= 0 && (r != col_r || c != col_c)) || behind_columns_.count(n.inputs[0]))
+                    fail(LB_ERR_UNSUPPORTED, "column reductions over different shapes in one fusion");
+                col_r = r, col_c = c;
+                col_reduces_.push_back(n.output);
+                behind_columns_.insert(n.output);
+                continue;
+            }
+            if (behind_columns_.count(n.inputs[0])) fail(LB_ERR_UNSUPPORTED, "a row reduction of column totals in one fusion");
             for (size_t k = 0; k < axes.size(); k++)
                 if (axes[k] != (int64_t)(x.rank() - axes.size() + k))
                     fail(LB_ERR_UNSUPPORTED,
@@ -381,7 +426,10 @@ class Generator {
             R_ = c ? r : 0;
             space = &x;
         }
-        if (!has_reduce_) {
+        if (mixed_) {
+            if (has_reduce_ && (R_ != col_r || C_ != col_c)) fail(LB_ERR_UNSUPPORTED, "row and column reductions over different shapes in one fusion");
+            R_ = col_r, C_ = col_c, has_reduce_ = true;
+        } else if (!has_reduce_) {
             for (int v : g_.outputs)
                 if (!space || g_.type(v).numel() > space->numel()) space = &g_.type(v);
             if (!space) fail(LB_ERR_INVALID, "fusion without outputs");
@@ -424,6 +472,19 @@ class Generator {
         RPB_ = T_ >= 32 ? 1 : 256 / T_;
         if (T_ > 32) RPB_ = 1;
         else RPB_ = std::max(1, 256 / T_);
+        if (mixed_) {
+            // Column sums and kept values live in registers beside the row: eight elements of a row per thread where a
+            // block can be that wide. Residual + layer norm forward and backward of 8192 x 1024 bfloat16 in one such kernel:
+            // 31 us + 6 us for its totals, against 125 us for the nine kernels of one kind of reduction each; bound by
+            // instructions in flight (63 per element, issued 43 % of the time; with 16 elements it spills: 59 us; with four,
+            // or five blocks an SM, 30 - 32 us).
+            const int64_t chunks = std::max<int64_t>(1, 16 / VEC_ / 2);
+            want = std::min<int64_t>((nvec + chunks - 1) / chunks, 1024);
+            for (T_ = 1; T_ < want && T_ < 32;) T_ *= 2;
+            if (want > 32) T_ = (int)((want + 31) / 32 * 32);
+            RPB_ = T_ > 32 ? 1 : 128 / T_;
+            resident_ = std::max(1, 512 / (T_ * RPB_));  // 16 warps an SM, 128 registers a thread
+        }
         NCH_ = (int)((nvec + T_ - 1) / T_);
         if (NCH_ > 64) fail(LB_ERR_UNSUPPORTED, format("rows of %lld elements are too long for the fused row kernel", (long long)C_));
         wide_index_ = R_ * C_ >= (1LL << 31) - 4096;
@@ -747,6 +808,7 @@ class Generator {
     }
 
     bool multi_phase_hint_ = false;
+    bool mixed_ = false;         // row and column reductions (or full outputs beside column reductions) in one kernel
     bool column_mode_ = false;   // reductions over the leading axes: partial sums per row slice, then a finalize pass
     bool inplace_ = false;       // an output aliases an input: plain loads, no __restrict__
     bool multi_ = false;         // one launch serves a table of tensor groups: pointers and row count per group
@@ -758,9 +820,45 @@ class Generator {
         std::string key = key_of(v, idx);
         auto it = ph.memo.find(key);
         if (it != ph.memo.end()) return it->second;
-        std::string name = gen_uncached(v, idx, ph);
+        std::string name = kept(v, key, idx, ph);
+        if (name.empty()) name = gen_uncached(v, idx, ph);
         ph.memo[key] = name;
         return name;
+    }
+
+    // The value from an earlier phase's registers, or "" where it is computed (again): divisions and functions of float32
+    // elements, while they fit 64 registers per thread.
+    std::string kept(int v, const std::string& key, const Index& idx, Phase& ph) {
+        static const std::set<std::string> costly = {"div", "exp", "log", "sqrt", "rsqrt", "tanh", "logistic", "exp2", "log2", "sin", "cos", "pow"};
+        const Node* n = g_.node_of(v);
+        if (!n || column_mode_ || !ph.chunked || !e_dep(idx) || g_.type(v).dtype != LB_F32 || !costly.count(n->op)) return "";
+        if (n->op == "exp" && normaliser_term(*n)) return "";
+        for (Phase& before : phases_) {
+            if (!before.chunked || !before.memo.count(key)) continue;
+            auto it = kept_.find(key);
+            if (it == kept_.end()) {
+                if (kept_regs_ + NCH_ * VEC_ > 64) return "";
+                kept_regs_ += NCH_ * VEC_;
+                it = kept_.emplace(key, fresh("kept")).first;
+                row_decls_ += format("float %s[NCH][VEC];\n", it->second.c_str());
+                const std::string& name = before.memo[key];
+                before.body += pair_ ? both_lanes(format("%s[ch][e] = LX(%s);\n", it->second.c_str(), name.c_str()))
+                                     : format("%s[ch][e] = %s;\n", it->second.c_str(), name.c_str());
+            }
+            return define(ph, "float", it->second + "[ch][e]", true, nullptr, LB_F32);
+        }
+        return "";
+    }
+
+    // the index of a column reduction's operand at row r, column c0 + e
+    Index column_operand_index(const TensorType& x, size_t lead_rank) {
+        Comp flat_c;
+        flat_c.base = "c0", flat_c.expr = "(c0 + e)";
+        flat_c.lane = flat_c.e_dep = flat_c.c_dep = true;
+        Index idx = unravel(row_comp(), std::vector<int64_t>(x.shape.begin(), x.shape.begin() + lead_rank));
+        Index tail = unravel(flat_c, std::vector<int64_t>(x.shape.begin() + lead_rank, x.shape.end()));
+        idx.insert(idx.end(), tail.begin(), tail.end());
+        return idx;
     }
 
     // exp(a - m) with m a row maximum computed in this kernel (through reshapes / broadcasts), read by reduce_sum only
@@ -1001,6 +1099,8 @@ class Generator {
     }
 
     std::string gen_reduce(const Node& n, const Index& idx) {
+        if (mixed_ && !column_mode_ && behind_columns_.count(n.output))
+            fail(LB_ERR_UNSUPPORTED, n.op + ": a column total read inside the rows it sums");
         if (column_mode_) {
             auto it = std::find(col_reduces_.begin(), col_reduces_.end(), n.output);
             if (it == col_reduces_.end()) fail(LB_ERR_UNSUPPORTED, n.op + ": mixed row and column reductions in one fusion");
@@ -1082,11 +1182,16 @@ class Generator {
         s << "template <class A, class F> __device__ __forceinline__ A row_reduce(A v, F f, A identity, void* smem) {\n";
         s << "    #pragma unroll\n    for (int m = " << width / 2 << "; m >= 1; m >>= 1) v = f(v, shfl_xor_any<A>(v, m));\n";
         if (T_ > 32) {
+            // the caller alternates between two areas of shared memory, so the next reduction's writes cannot overtake
+            // this one's reads and one barrier is enough
             s << "    A* sm = (A*)smem; const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;\n";
             s << "    if (lane == 0) sm[warp] = v;\n    __syncthreads();\n";
-            s << "    v = lane < " << T_ / 32 << " ? sm[lane] : identity;\n";
-            s << "    #pragma unroll\n    for (int m = 16; m >= 1; m >>= 1) v = f(v, shfl_xor_any<A>(v, m));\n";
-            s << "    __syncthreads();\n";
+            if (T_ <= 256) {
+                s << "    v = sm[0];\n    #pragma unroll\n    for (int w = 1; w < " << T_ / 32 << "; w++) v = f(v, sm[w]);\n";
+            } else {
+                s << "    v = lane < " << T_ / 32 << " ? sm[lane] : identity;\n";
+                s << "    #pragma unroll\n    for (int m = 16; m >= 1; m >>= 1) v = f(v, shfl_xor_any<A>(v, m));\n";
+            }
         }
         s << "    return v;\n}\n";
         const char* restrict_kw = inplace_ ? "" : " __restrict__";
@@ -1113,16 +1218,26 @@ class Generator {
             for (size_t i = 0; i < g_.outputs.size(); i++)
                 s << "    void*" << restrict_kw << " out" << i << " = table.ptr[group][" << g_.inputs.size() + i << "];\n";
         } else {
-            s << "extern \"C\" __global__ void __launch_bounds__(" << T_ * RPB_ << ") fused_kernel(";
+            s << "extern \"C\" __global__ void __launch_bounds__(" << T_ * RPB_;
+            if (mixed_) s << ", " << resident_;
+            s << ") fused_kernel(";
             for (size_t i = 0; i < g_.inputs.size(); i++) s << (i ? ", " : "") << "const void*" << restrict_kw << " in" << i;
             for (size_t i = 0; i < g_.outputs.size(); i++)
                 s << ((i || !g_.inputs.empty()) ? ", " : "") << "void*" << restrict_kw << " out" << i;
+            if (mixed_) s << ", void* __restrict__ scratch";
             s << ") {\n";
         }
-        s << "    __shared__ unsigned long long red_smem[32];\n";
+        s << "    __shared__ unsigned long long red_smem[2][32];\n    int red_turn = 0;\n";
         s << "    const int lane_in_row = threadIdx.x % TPR, row_in_block = threadIdx.x / TPR;\n";
         s << "    const idx_t row_blocks = (idx_t)((NROWS + RPB - 1) / RPB);\n";
         s << indent(kernel_cache_, 4);
+        for (size_t i = 0; i < col_reduces_.size(); i++) {
+            const Node& n = *g_.node_of(col_reduces_[i]);
+            std::string init, combine;
+            reduce_ops(n, g_.type(n.output), &init, &combine);
+            s << "    " << ctype(g_.type(n.output).dtype).compute << " cacc" << i << "[NCH][VEC];\n";
+            s << "    _Pragma(\"unroll\") for (int ch = 0; ch < NCH; ch++) { _Pragma(\"unroll\") for (int e = 0; e < VEC; e++) cacc" << i << "[ch][e] = " << init << "; }\n";
+        }
         // Rows cached in registers are loaded one row block ahead (while the current block's phases compute), when that
         // costs at most 64 bytes of registers per thread: a block's phases are a serial chain behind its loads.
         int cached_bytes = 0;
@@ -1175,17 +1290,55 @@ class Generator {
             if (ph.reduces) {
                 s << "            " << ph.result << " = row_reduce<" << ph.acc_type << ">(" << ph.acc << ", [](" << ph.acc_type
                   << " a, " << ph.acc_type << " b) { return " << subst(ph.combine_a_b, "a", "b") << "; }, (" << ph.acc_type
-                  << ")" << ph.init << ", red_smem);\n";
+                  << ")" << ph.init << ", red_smem[red_turn ^= 1]);\n";
             }
             s << "        }\n";
         }
-        s << (multi_ ? "    }\n  }\n}\n" : "    }\n}\n");
+        s << (multi_ ? "    }\n  }\n" : "    }\n");
+        if (mixed_) {
+            // enough CTAs to keep several rows in flight on every SM; each leaves one slice of partial sums per column
+            const int64_t row_blocks = std::max<int64_t>((R_ + RPB_ - 1) / RPB_, 1);
+            k.two_pass = true;
+            k.col_blocks = std::min<int64_t>(row_blocks, 148LL * resident_);
+            k.slices = 1;
+            std::vector<size_t> offsets;
+            size_t scratch = 0;
+            for (size_t i = 0; i < col_reduces_.size(); i++) {
+                const Node& n = *g_.node_of(col_reduces_[i]);
+                const TensorType& t = g_.type(n.output);
+                const std::string type = ctype(t.dtype).compute;
+                const int width = type == "float" ? 4 : type == "double" ? 8 : dtype_size(t.dtype);
+                std::string init, combine;
+                reduce_ops(n, t, &init, &combine);
+                s << "    {\n        " << type << "* part = (" << type << "*)((char*)scratch + " << scratch << ") + (idx_t)blockIdx.x * NCOLS;\n";
+                if (RPB_ > 1) {  // the block's rows in order, through shared memory
+                    s << "        __shared__ " << type << " csum" << i << "[NCOLS];\n";
+                    s << "        for (int y = 0; y < RPB; y++) {\n            if (row_in_block == y) { CHUNK_LOOP_BEGIN _Pragma(\"unroll\") for (int e = 0; e < VEC; e++) csum"
+                      << i << "[c0 + e] = y ? " << subst(combine, format("csum%d[c0 + e]", (int)i), format("cacc%d[ch][e]", (int)i)) << " : cacc" << i
+                      << "[ch][e]; CHUNK_LOOP_END }\n            __syncthreads();\n        }\n";
+                    s << "        for (int c = threadIdx.x; c < NCOLS; c += TPR * RPB) part[c] = csum" << i << "[c];\n    }\n";
+                } else {
+                    s << "        CHUNK_LOOP_BEGIN _Pragma(\"unroll\") for (int e = 0; e < VEC; e++) part[c0 + e] = cacc" << i << "[ch][e]; CHUNK_LOOP_END\n    }\n";
+                }
+                offsets.push_back(scratch);
+                scratch = (scratch + (size_t)k.col_blocks * C_ * width + 255) & ~(size_t)255;
+            }
+            s << "}\n#define SLICES " << k.col_blocks << "\n";
+            std::string sig;
+            for (size_t i = 0; i < g_.inputs.size(); i++) sig += format("const void* __restrict__ in%d, ", (int)i);
+            for (size_t i = 0; i < g_.outputs.size(); i++) sig += format("void* __restrict__ out%d, ", (int)i);
+            k.vec = VEC_;
+            emit_finalize(s, sig + "void* __restrict__ scratch", offsets, column_outputs_, k);
+            k.scratch_bytes = scratch;
+        } else {
+            s << "}\n";
+            k.vec = VEC_;
+        }
         k.source = s.str();
         k.rows = R_;
         k.cols = C_;
         k.threads = T_ * RPB_;
         k.rows_per_block = RPB_;
-        k.vec = VEC_;
         k.n_inputs = (int)g_.inputs.size();
         k.n_outputs = (int)g_.outputs.size();
         for (int v : g_.inputs) k.types.push_back(g_.type(v));
@@ -1233,9 +1386,8 @@ class Generator {
         wide_index_ = R_ * C_ >= (1LL << 31) - 4096;
         pair_ = VEC_ >= 2 && computes_bf16();
         // both passes: 256 threads = 32 column lanes (VEC columns each) x 8 row lanes (pass 2: slice lanes)
-        const int threads = 256, col_lanes = 32, row_lanes = 8, fin_threads = 256;
+        const int threads = 256, col_lanes = 32, row_lanes = 8;
         int64_t col_blocks = std::max<int64_t>((C_ + (int64_t)col_lanes * VEC_ - 1) / ((int64_t)col_lanes * VEC_), 1);
-        int64_t fin_blocks = col_blocks;
         // enough slices to fill the GPU a few times over, each at least 64 rows long
         int64_t slices = std::min<int64_t>(std::max<int64_t>(1, (148 * 4 + col_blocks - 1) / col_blocks), std::max<int64_t>(R_ / 64, 1));
         int64_t rows_per_slice = (R_ + slices - 1) / std::max<int64_t>(slices, 1);
@@ -1279,36 +1431,6 @@ class Generator {
             scratch += (size_t)slices * C_ * width;
             scratch = (scratch + 255) & ~(size_t)255;
         }
-        // pass 2
-        Phase fin;
-        std::ostringstream totals;
-        for (size_t k = 0; k < col_reduces_.size(); k++) {
-            const Node& n = *g_.node_of(col_reduces_[k]);
-            const TensorType& t = g_.type(n.output);
-            CType ct = ctype(t.dtype);
-            std::string init, combine;
-            reduce_ops(n, t, &init, &combine);
-            // slice lane y adds slices y, y + 8, ... in order; the lanes are then combined in lane order
-            totals << ct.compute << " tot" << k << "[VEC];\n#pragma unroll\nfor (int e = 0; e < VEC; e++) tot" << k << "[e] = " << init << ";\n";
-            totals << "if (in_range) {\n#pragma unroll 4\n    for (int s = row_lane; s < SLICES; s += " << row_lanes << ") {\n#pragma unroll\n        for (int e = 0; e < VEC; e++) { "
-                   << ct.compute << " pv = ((const " << ct.compute << "*)((const char*)scratch + " << offsets[k] << "))[(idx_t)s * NCOLS + c0 + e]; tot" << k
-                   << "[e] = " << subst(combine, format("tot%d[e]", (int)k), "pv") << "; }\n    }\n}\n";
-            totals << "__shared__ " << ct.compute << " fred" << k << "[" << row_lanes << "][" << col_lanes << " * VEC];\n";
-            totals << "#pragma unroll\nfor (int e = 0; e < VEC; e++) fred" << k << "[row_lane][col_lane * VEC + e] = tot" << k << "[e];\n__syncthreads();\n";
-            totals << "if (row_lane == 0) {\n#pragma unroll\n    for (int e = 0; e < VEC; e++)\n        for (int y = 1; y < " << row_lanes << "; y++) tot" << k << "[e] = "
-                   << subst(combine, format("tot%d[e]", (int)k), format("fred%d[y][col_lane * VEC + e]", (int)k)) << ";\n}\n";
-        }
-        for (size_t k = 0; k < g_.outputs.size(); k++) {
-            const TensorType& t = g_.type(g_.outputs[k]);
-            if (t.numel() != C_) fail(LB_ERR_UNSUPPORTED, format("column-reduction fusion output %s does not have %lld elements", t.str().c_str(), (long long)C_));
-            Index idx = unravel(flat_c, t.shape);
-            std::string val = gen(g_.outputs[k], idx, fin);
-            CType ct = ctype(t.dtype);
-            fin.pre += format("__align__(16) %s ob%d[VEC];\n", ct.memory, (int)k);
-            fin.body += store_element(format("ob%d", (int)k), t.dtype, val);
-            fin.post += format("stv<%s, VEC>((%s*)out%d + c0, ob%d);\n", ct.memory, ct.memory, (int)k, (int)k);
-        }
-
         std::ostringstream s;
         s << "// generated by lumen_b200: column reduction over [" << R_ << " rows, " << C_ << " columns], " << slices << " row slices\n";
         s << kPreamble;
@@ -1329,17 +1451,11 @@ class Generator {
         s << "        #pragma unroll\n        for (int e = 0; e < VEC; e += " << (pair_ ? 2 : 1) << ") {\n" << indent(part.body, 12) << "        }\n    }\n";
         s << indent(store.str(), 4);
         s << "}\n";
-        s << "extern \"C\" __global__ void __launch_bounds__(" << fin_threads << ") fused_finalize(" << sig << ") {\n";
-        s << "    const int col_lane = threadIdx.x & " << col_lanes - 1 << ", row_lane = threadIdx.x >> 5;\n";
-        s << "    const idx_t c0 = ((idx_t)blockIdx.x * " << col_lanes << " + col_lane) * VEC;\n    const bool in_range = c0 < NCOLS;\n";
-        s << indent(totals.str(), 4);
-        s << "    if (row_lane != 0 || !in_range) return;\n";
-        s << indent(fin.pre, 4);
-        s << "    #pragma unroll\n    for (int e = 0; e < VEC; e += " << (pair_ ? 2 : 1) << ") {\n" << indent(fin.body, 8) << "    }\n";
-        s << indent(fin.post, 4);
-        s << "}\n";
-
         FusedKernel k;
+        std::vector<int> outputs(g_.outputs.size());
+        for (size_t i = 0; i < outputs.size(); i++) outputs[i] = (int)i;
+        k.slices = (int)slices;
+        emit_finalize(s, sig, offsets, outputs, k);
         k.source = s.str();
         k.rows = R_, k.cols = C_, k.threads = threads, k.rows_per_block = 1, k.vec = VEC_;
         k.n_inputs = (int)g_.inputs.size(), k.n_outputs = (int)g_.outputs.size();
@@ -1348,10 +1464,61 @@ class Generator {
         k.two_pass = true;
         k.slices = (int)slices;
         k.col_blocks = col_blocks;
-        k.fin_threads = fin_threads;
-        k.fin_blocks = fin_blocks;
         k.scratch_bytes = scratch;
         return k;
+    }
+
+    // The second kernel of a column reduction: adds the slices' partial sums and applies the epilogue. A block takes 32
+    // lanes of two columns and eight or 32 slice lanes: few columns and slices per thread, so that the chains of loads stay
+    // short (1184 slices of 1024 columns took 19 us with eight slice lanes).
+    void emit_finalize(std::ostringstream& s, const std::string& sig, const std::vector<size_t>& offsets, const std::vector<int>& outputs, FusedKernel& k) {
+        column_mode_ = true;
+        VEC_ = std::min(VEC_, 2);
+        pair_ = VEC_ >= 2 && computes_bf16();
+        const int col_lanes = 32, row_lanes = k.slices * k.col_blocks > 64 ? 32 : 8, threads = col_lanes * row_lanes;
+        Comp flat_c;
+        flat_c.base = "c0", flat_c.expr = "(c0 + e)";
+        flat_c.lane = flat_c.e_dep = flat_c.c_dep = true;
+        Phase fin;
+        std::ostringstream totals;
+        for (size_t k = 0; k < col_reduces_.size(); k++) {
+            const Node& n = *g_.node_of(col_reduces_[k]);
+            const TensorType& t = g_.type(n.output);
+            CType ct = ctype(t.dtype);
+            std::string init, combine;
+            reduce_ops(n, t, &init, &combine);
+            // slice lane y adds slices y, y + (lanes), ... in order; the lanes are then combined in lane order
+            totals << ct.compute << " tot" << k << "[VEC];\n#pragma unroll\nfor (int e = 0; e < VEC; e++) tot" << k << "[e] = " << init << ";\n";
+            totals << "if (in_range) {\n#pragma unroll 8\n    for (int s = row_lane; s < SLICES; s += " << row_lanes << ") {\n#pragma unroll\n        for (int e = 0; e < VEC; e++) { "
+                   << ct.compute << " pv = ((const " << ct.compute << "*)((const char*)scratch + " << offsets[k] << "))[(idx_t)s * NCOLS + c0 + e]; tot" << k
+                   << "[e] = " << subst(combine, format("tot%d[e]", (int)k), "pv") << "; }\n    }\n}\n";
+            totals << "__shared__ " << ct.compute << " fred" << k << "[" << row_lanes << "][" << col_lanes << " * VEC];\n";
+            totals << "#pragma unroll\nfor (int e = 0; e < VEC; e++) fred" << k << "[row_lane][col_lane * VEC + e] = tot" << k << "[e];\n__syncthreads();\n";
+            totals << "if (row_lane == 0) {\n#pragma unroll\n    for (int e = 0; e < VEC; e++) {\n#pragma unroll\n        for (int y = 1; y < " << row_lanes << "; y++) tot" << k << "[e] = "
+                   << subst(combine, format("tot%d[e]", (int)k), format("fred%d[y][col_lane * VEC + e]", (int)k)) << ";\n    }\n}\n";
+        }
+        for (int o : outputs) {
+            const TensorType& t = g_.type(g_.outputs[o]);
+            if (t.numel() != C_) fail(LB_ERR_UNSUPPORTED, format("column-reduction fusion output %s does not have %lld elements", t.str().c_str(), (long long)C_));
+            Index idx = unravel(flat_c, t.shape);
+            std::string val = gen(g_.outputs[o], idx, fin);
+            CType ct = ctype(t.dtype);
+            fin.pre += format("__align__(16) %s ob%d[VEC];\n", ct.memory, o);
+            fin.body += store_element(format("ob%d", o), t.dtype, val);
+            fin.post += format("stv<%s, VEC>((%s*)out%d + c0, ob%d);\n", ct.memory, ct.memory, o, o);
+        }
+        s << "#undef VEC\n#define VEC " << VEC_ << "\n";
+        s << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") fused_finalize(" << sig << ") {\n";
+        s << "    const int col_lane = threadIdx.x & " << col_lanes - 1 << ", row_lane = threadIdx.x >> 5;\n";
+        s << "    const idx_t c0 = ((idx_t)blockIdx.x * " << col_lanes << " + col_lane) * VEC;\n    const bool in_range = c0 < NCOLS;\n";
+        s << indent(totals.str(), 4);
+        s << "    if (row_lane != 0 || !in_range) return;\n";
+        s << indent(fin.pre, 4);
+        s << "    #pragma unroll\n    for (int e = 0; e < VEC; e += " << (pair_ ? 2 : 1) << ") {\n" << indent(fin.body, 8) << "    }\n";
+        s << indent(fin.post, 4);
+        s << "}\n";
+        k.fin_threads = threads;
+        k.fin_blocks = std::max<int64_t>((C_ + (int64_t)col_lanes * VEC_ - 1) / ((int64_t)col_lanes * VEC_), 1);
     }
 
     // identity and combine format of a reduction node with result type `t`
@@ -1382,8 +1549,27 @@ class Generator {
         }
         return any;
     }
+    static bool some_columns(const Graph& g) {
+        int lead;
+        for (const Node& n : g.nodes)
+            if ((n.op == "reduce_sum" || n.op == "reduce_max") && leading_axes(n, g.type(n.inputs[0]), &lead)) return true;
+        return false;
+    }
+    // whether an output is not computed from a column total
+    static bool leaves_rows(const Graph& g) {
+        std::set<int> behind;
+        for (const Node& n : g.nodes) {
+            bool in = n.op == "reduce_sum" || n.op == "reduce_max";
+            for (int v : n.inputs) in |= behind.count(v) != 0;
+            if (in) behind.insert(n.output);
+        }
+        for (int v : g.outputs)
+            if (!behind.count(v)) return true;
+        return false;
+    }
     void set_inplace(bool v) { inplace_ = v; }
     void set_multi(bool v) { multi_ = v; }
+    void set_mixed(bool v) { mixed_ = v; }
 
 };
 
@@ -1399,7 +1585,8 @@ FusedKernel generate_fused(const Module& module) {
     gen.set_multi(module.options.count("multi") != 0);
     if (module.options.count("multi") && (reduces || Generator::wants_columns(g)))
         fail(LB_ERR_UNSUPPORTED, "option multi: a horizontally fused kernel cannot hold a reduction");
-    if (Generator::wants_columns(g)) return gen.run_columns();
+    if (Generator::wants_columns(g) && !Generator::leaves_rows(g)) return gen.run_columns();
+    if (Generator::some_columns(g) && !module.options.count("inplace")) gen.set_mixed(true);
     // With a reduction followed by further use of the row, inputs are kept in registers across phases.
     gen.set_multi_phase(reduces >= 1);
     return gen.run();

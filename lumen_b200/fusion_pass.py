@@ -64,9 +64,13 @@ class FusionPass:
                 constant.add(i)
         for i in range(len(graph.nodes) - 1, -1, -1):
             n = graph.nodes[i]
-            if (n.op in INLINED or i in constant) and n.output not in self.outputs and self.uses.get(n.output) and all(
+            if (n.op in INLINED or i in constant or self.widens(n)) and n.output not in self.outputs and self.uses.get(n.output) and all(
                     graph.nodes[u].op in ELEMENTWISE | REDUCTIONS or u in self.transparent for u in self.uses[n.output]):
                 self.transparent.add(i)
+
+    def widens(self, n) -> bool:
+        """A cast of a 16-bit float to float32: every reader repeats it on the narrow value, which is half the bytes."""
+        return n.op == "cast" and self.g.types[n.inputs[0]].dtype in ("bfloat16", "float16") and self.g.types[n.output].dtype == "float32"
 
     def readers(self, v: int) -> list[int]:
         """The nodes that read `v`, looking through transparent nodes."""
@@ -120,17 +124,73 @@ class FusionPass:
         return v in self.outputs or any(u not in member_set for u in self.readers(v))
 
     # ---- growing groups --------------------------------------------------------------------------------------
-    def can_join(self, group: _Group, i: int) -> bool:
-        """Node `i` may join `group` when the group still runs before every reader of its values (no reader outside the
-        group sits before `i`) and the backend has one kernel for the larger body."""
-        member_set = set(group.members)
-        for m in group.members:
+    def one_kernel(self, members: list[int]) -> bool:
+        """Whether `members` (node indices in order) may be emitted as one group where the last of them stands - no reader
+        outside the group sits before that - and the backend has one kernel for them."""
+        member_set = set(members)
+        for m in members:
             for u in self.readers(self.g.nodes[m].output):
-                if u < i and u not in member_set:
+                if u < members[-1] and u not in member_set:
                     return False
-        members = group.members + [i]
+        if not self.shares_well(members):
+            return False
         body, _, leaving = self.body_of(members)
         return bool(leaving) and self.accepts(body)
+
+    # Rows and columns reduced in one kernel leave a slice of partial column sums per block: that pays where it saves a pass
+    # over an operand in HBM, not over one that stays in the L2 anyway (below 256 KB).
+    SMALLEST_MIXED = 1 << 16
+
+    def shares_well(self, members: list[int]) -> bool:
+        def kind(m):
+            n = self.g.nodes[m]
+            if n.op not in REDUCTIONS:
+                return None
+            x = self.g.types[n.inputs[0]]
+            return ("columns" if min(n.params["axes"]) == 0 and len(n.params["axes"]) < len(x.shape) else "rows"), x.numel
+
+        kinds = [k for k in map(kind, members) if k]
+        columns = [size for which, size in kinds if which == "columns"]
+        if not columns or min(columns) >= self.SMALLEST_MIXED:
+            return True
+        behind: set[int] = set()  # values computed from a reduction
+        for m in members:
+            n = self.g.nodes[m]
+            if n.op in REDUCTIONS or any(v in behind for v in n.inputs):
+                behind.add(n.output)
+        return len(columns) == len(kinds) and all(self.g.nodes[m].output in behind or not self.leaves(self.g.nodes[m].output, set(members)) for m in members)
+
+    def can_join(self, group: _Group, i: int) -> bool:
+        """Node `i` may join `group`: the group still runs before every reader of its values."""
+        return self.one_kernel(group.members + [i])
+
+    def absorb(self, group: _Group, others: list[_Group], members: list[int]) -> None:
+        group.members = members
+        for m in members:
+            self.group_of[m] = group
+        self.groups = [g for g in self.groups if g not in others]
+
+    def merge_siblings(self) -> None:
+        """Groups that read the same full-size operand, or one the other's values, become one group where the backend has one
+        kernel for both (a layer norm's backward rows and the column sums of its weight gradients): the operand is read once."""
+        def big_operands(grp):
+            _, operands, leaving = self.body_of(grp.members)
+            sizes = [self.g.types[v].numel for v in (*operands, *leaving)]
+            return {v for v in (*operands, *leaving) if self.g.types[v].numel == max(sizes, default=0)}
+
+        touched = {id(grp): big_operands(grp) for grp in self.groups}
+        again = True
+        while again:
+            again = False
+            for a in list(self.groups):
+                for b in list(self.groups):
+                    if a is b or a not in self.groups or b not in self.groups or a.members[0] > b.members[0] or not touched[id(a)] & touched[id(b)]:
+                        continue
+                    members = sorted(a.members + b.members)
+                    if self.one_kernel(members):
+                        self.absorb(a, [b], members)
+                        touched[id(a)] = big_operands(a)
+                        again = True
 
     def run(self) -> G.Graph:
         g = self.g
@@ -159,6 +219,11 @@ class FusionPass:
                     if grp not in candidates:
                         candidates.append(grp)
             candidates.sort(key=lambda grp: -grp.last)
+            if len(candidates) > 1:  # the node may close the gap between its operands' groups
+                members = sorted(m for grp in candidates for m in grp.members) + [i]
+                if self.one_kernel(members):
+                    self.absorb(candidates[0], candidates[1:], members)
+                    continue
             for grp in candidates:
                 if self.can_join(grp, i):
                     grp.members.append(i)
@@ -169,6 +234,7 @@ class FusionPass:
                 grp.members.append(i)
                 self.groups.append(grp)
                 self.group_of[i] = grp
+        self.merge_siblings()
         return self.emit()
 
     # ---- GEMM epilogues ----------------------------------------------------------------------------------------

@@ -263,3 +263,28 @@ def test_inplace_update(cuda):
 
 
 _ = BF16
+
+
+@pytest.mark.parametrize("shape", [(64, 64), (257, 40), (1000, 1000), (3, 4096), (5000, 33), (600, 8200), (2, 16384)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_row_and_column_reductions_in_one_kernel(cuda, shape, dtype):
+    """Rows centred, and the column sums of the rows and of the centred rows, from one kernel: narrow rows (several to a
+    block), rows of one and of several chunks per thread, fewer rows than blocks, widths without a vector's divisor.
+    Sums within 1e-5 of the sums of magnitudes (float32 accumulation of at most 5000 terms in any order: 5000 * 2^-24
+    = 3e-4 at the very worst, about its square root of terms in practice); a 16-bit result adds its own rounding."""
+    rows, cols = shape
+    x = np.random.default_rng(rows).standard_normal(shape).astype(np.float32)
+    x = bf16(x) if dtype == "bfloat16" else x
+
+    def program(a):
+        w = a.to("float32")
+        c = w - prims.reduce_sum(w, (1,), "float32").reshape(rows, 1) * (1.0 / cols)
+        return c.to(dtype), prims.reduce_sum(w, (0,), "float32"), prims.reduce_sum(c * c, (0,), "float32").to(dtype)
+
+    c, s, q = (to_numpy(t).astype(np.float64) for t in Fusion(tracer.trace(program, (dtype, shape)))(to_torch(x, cuda)))
+    x64 = x.astype(np.float64)
+    want = x64 - x64.mean(1, keepdims=True)
+    half = 2.0**-8 if dtype == "bfloat16" else 0.0
+    assert (np.abs(c - want) <= (half + 1e-6) * np.abs(want) + 1e-5).all()
+    assert (np.abs(s - x64.sum(0)) <= 1e-5 * np.abs(x64).sum(0)).all()
+    assert (np.abs(q - (want * want).sum(0)) <= (half + 2e-5) * (want * want).sum(0)).all()
