@@ -382,11 +382,14 @@ CUtensorMap make_bsnh_map(const lb_tensor& t, const char* what, int box_rows = 1
 
 CUtensorMap attention_map_rows(const lb_tensor& t, const char* what, int box_rows) { return make_bsnh_map(t, what, box_rows); }
 
+bool attention_decodes(const lb_tensor& q, const lb_tensor& k);
+void attention_decode(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o,
+                      const lb_tensor* lse, void* stream);
+
 void attention_fwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o,
                    const lb_tensor* lse, void* stream) {
     if (q.rank != 4 || k.rank != 4 || v.rank != 4) fail(LB_ERR_INVALID, "attention: operands must be [B, S, N, H] tensors");
     if (q.shape[0] == 0 || q.shape[1] == 0 || q.shape[2] == 0) return;  // nothing to compute: no launch (and no tensor map over nothing)
-    CUtensorMap mq = make_bsnh_map(q, "query"), mk = make_bsnh_map(k, "key"), mv = make_bsnh_map(v, "value");
     const long long B = q.shape[0], Sq = q.shape[1], N = q.shape[2], D = q.shape[3];
     const long long Sk = k.shape[1], Nkv = k.shape[2];
     if (k.shape[0] != B || v.shape[0] != B || k.shape[3] != D || v.shape[1] != Sk || v.shape[2] != Nkv || Nkv == 0 || N % Nkv)
@@ -398,6 +401,12 @@ void attention_fwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor
     if (lse) check_dense(*lse, LB_F32, {B, N, Sq}, "attention log-sum-exp");
     if (!(desc.scale > 0.0f)) fail(LB_ERR_UNSUPPORTED, "attention: the softmax scale must be positive");
     if (B == 0 || Sq == 0 || N == 0) return;
+    if (attention_decodes(q, k)) {
+        driver();
+        attention_decode(desc, q, k, v, o, lse, stream);
+        return;
+    }
+    CUtensorMap mq = make_bsnh_map(q, "query"), mk = make_bsnh_map(k, "key"), mv = make_bsnh_map(v, "value");
     FwdArgs p{};
     p.B = (int)B, p.N = (int)N, p.Nkv = (int)Nkv, p.Sq = (int)Sq, p.Sk = (int)Sk;
     p.causal = desc.causal;

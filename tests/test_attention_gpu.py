@@ -306,3 +306,24 @@ def test_cuda_core_attention_against_float64(cuda, case):
     for name, got, want in zip(("o", "lse", "dq", "dk", "dv"), (o, lse, *grads), (out, torch.logsumexp(s, -1), *(t.grad for t in x))):
         want = want.detach().numpy()
         assert np.abs(to_numpy(got) - want).max() <= 2e-5 * max(np.abs(want).max(), 1.0), name
+
+
+# (B, Sq, Sk, N, Nkv, H): few query rows per key head - one and two 16-row tiles, one key, ragged slices of 16 keys, fewer
+# slices than warps, one and many CTAs per key head, positions that see different numbers of keys
+DECODE_CASES = [((1, 1, 1, 1, 1, 64), False), ((2, 1, 17, 4, 4, 128), True), ((1, 1, 4097, 8, 1, 128), True), ((3, 4, 1000, 8, 2, 64), True),
+                ((1, 4, 333, 16, 4, 128), True), ((2, 2, 2050, 32, 2, 128), True), ((1, 16, 40, 2, 1, 64), False), ((1, 5, 3, 2, 2, 64), False),
+                ((40, 1, 129, 16, 16, 64), True), ((1, 1, 16384, 2, 2, 128), True), ((1, 32, 32, 1, 1, 64), True)]
+
+
+@pytest.mark.parametrize("case", DECODE_CASES)
+def test_few_query_rows_against_float64(cuda, case):
+    """The reference's 16-bit tolerance (2e-2), log-sum-exp to 1e-3, on strided views."""
+    (b, sq, sk, n, nkv, h), causal = case
+    q, k, v = qkv(b, sq, sk, n, nkv, h)
+    cache = torch.empty((b, sk, 2, nkv, h), dtype=torch.bfloat16, device=cuda)
+    cache[:, :, 0], cache[:, :, 1] = to_torch(k, cuda), to_torch(v, cuda)
+    o, lse = attention_forward(to_torch(q, cuda), cache[:, :, 0], cache[:, :, 1], causal=causal)
+    device_status()
+    want, want_lse = attention_f64(q, k, v, causal)
+    np.testing.assert_allclose(to_numpy(o).astype(np.float64), want, rtol=TOL, atol=TOL)
+    np.testing.assert_allclose(to_numpy(lse), want_lse, rtol=1e-3, atol=1e-3)
