@@ -8,10 +8,9 @@
 //   dS^T  = P^T * (dP^T - delta) * scale   (rounded to bf16),  P^T rounded to bf16
 //   dV   += P^T dO,  dK += dS^T Q,  dQ += dS K
 //
-// One kernel template runs in two modes. Both keep a 128-row pair of tiles resident in shared memory, stream
-// 64-row tile pairs through a 3-stage TMA ring, compute X = R1 T1^T and Y = R2 T2^T with tcgen05.mma into
-// double-buffered tensor memory, turn them into bf16 P and Z = dS (one row per thread, written back over X and Y
-// as TMEM operands) and accumulate in tensor memory:
+// One kernel template runs in two modes. Both keep a 128-row pair of tiles resident in shared memory, stream tile pairs
+// through a TMA ring, compute X = R1 T1^T and Y = R2 T2^T with tcgen05.mma into tensor memory, turn them into bf16 P and
+// Z = dS (one row per thread, written back to tensor memory as operands) and accumulate in tensor memory:
 //   dK/dV mode: CTA = (key tile, kv head, batch); R = (K, V), T = (Q, dO) over every query head of the group and
 //               every query tile that sees the keys; acc_a = dK += Z Q, acc_b = dV += P dO.
 //   dQ mode:    CTA = (query tile, head, batch); R = (Q, dO), T = (K, V) over the visible key tiles; acc_a = dQ += Z K.
@@ -42,24 +41,23 @@ __device__ __forceinline__ float fast_exp2(float x) {
 }
 
 constexpr int BR = 128;  // resident rows (thread = row)
-constexpr int BT = 64;   // streamed rows per step
-// warp 0: TMA, warp 1: MMA + TMEM owner, then WGS compute warpgroups of four warps, over BUFS X/Y buffers.
-//  BUFS = WGS = 2 (head dim 128): warpgroup w takes iterations w, w + WGS, ... on its own X/Y buffer;
-//  one CTA per SM. An iteration is a chain MMA -> commit -> wake -> tensor-memory load -> element-wise -> store ->
-//  arrive -> wake -> MMA of about 2000 cycles, most of it signalling and load latency (a commit-to-wake takes about
-//  350 cycles, an arrive-to-wake 280, a tensor-memory load 170), so throughput is set by how many chains are in
-//  flight.
-//  BUFS = 1 (head dim 64): single X/Y buffers, 256 tensor-memory columns and half the shared memory, so that TWO CTAs
-//  share an SM and one CTA's prologue, epilogue and element-wise latency are covered by the other's MMAs. With
-//  WGS = 2 both warpgroups work on EVERY iteration, each on 32 of the 64 streamed columns (the kernels are bound by
-//  latency, not by a pipe: 16 compute warps per SM hide twice as much of it as 8).
-//  In that mode P and Z are written over Y's columns only, so X is free as soon as every thread has loaded it: the
-//  next tile's X product is issued while this tile's element-wise phase runs, and the exponentials (which need X
-//  alone) start before the next Y - which has to wait for the accumulation products that read P and Z - has landed.
-//  The serial chain per tile shrinks from math + accumulate + X/Y + signalling to roughly accumulate + Y + the Z half
-//  of the math. The two-buffer configuration of head dim 128 already overlaps two chains, so it keeps one load round
-//  trip for X and Y together.
-constexpr int threads_of(int wgs) { return 64 + 128 * wgs; }
+// warp 0: TMA, warp 1: MMA + TMEM owner, then two compute warpgroups, each on half of the BT streamed columns of every
+// iteration. X is free as soon as every thread has loaded it: the next tile's X product is issued while this tile's
+// element-wise phase runs, and the exponentials (X alone) do not wait for Y.
+//  dK/dV mode: P and Z are written over Y's columns (each thread's over the columns it read), so the next Y follows the
+//  accumulation products that read them - the tensor pipe runs in order - and the serial chain per tile is accumulate,
+//  Y, signalling and the Z half of the element-wise work.
+//  dQ mode: the second accumulator's columns hold Z, Y is handed back like X, and both products of the next tile run
+//  under this tile's element-wise phase.
+//
+//  BT = 128 (head dim 128): one CTA per SM on all 512 columns (X 128, Y 128, accumulators 2 x 128). A product with both
+//  operands in shared memory reads its 128 x 16 A operand in about 68 cycles whatever N is, so 64 streamed columns - as
+//  the two-buffer form this replaces had, on alternating warpgroups - paid for 128: the tensor unit was busy for 67 %
+//  of the kernels' time at 41 % of its rate. Batch 8, 32 heads, sequence 4096, causal: backward 4.66 -> 3.48 ms
+//  (790 TFLOP/s), of which 0.26 came from issuing the products warp-wide.
+//  BT = 64 (head dim 64): 256 columns and half the shared memory, so that TWO CTAs share an SM and one CTA's prologue,
+//  epilogue and element-wise latency are covered by the other's products (128 and one CTA: 470 -> 548 us at batch 8,
+//  16 heads, sequence 2048).
 
 struct BwdArgs {
     int B, N, Nkv, Sq, Sk;
@@ -75,26 +73,30 @@ struct BwdArgs {
     int* status;
 };
 
-template <int D, int BUFS>
-struct BwdSmem {
-    static constexpr int kResident = BR * D * 2;
-    static constexpr int kStream = BT * D * 2;
-    // ring of streamed tile pairs: deep enough to hide a tile's TMA latency behind several iterations
-    static constexpr int STAGES = BUFS == 1 ? 4 : (D == 64 ? 8 : 4);
-    static constexpr int kBytes = 2 * kResident + STAGES * 2 * kStream + 1024 + 256 + 8192;  // tiles, alignment, barriers, column statistics
+template <int D, bool DKDV, int BT>
+struct BwdConfig {
+    static constexpr int kCtas = BT == 64 ? 2 : 1;       // per SM
+    static constexpr int kFirst = BT == 64 ? 2 : 4;      // first compute warp (register budgets are set per aligned group of four warps)
+    static constexpr int kThreads = 32 * kFirst + 256;
+    static constexpr int kTmemCols = 512 / kCtas;
+    static constexpr int kResident = BR * D * 2, kStream = BT * D * 2;
+    // rings of streamed tiles: T1 is read until the tile's accumulation has completed, T2 in dQ mode only by Y
+    static constexpr int S1 = BT == 64 ? 4 : (DKDV ? 2 : 3), S2 = BT == 64 ? 4 : 2;
+    static constexpr int kCols = BT / 2;                 // streamed columns of one thread
+    static constexpr int kStats = DKDV ? 8 * 2 * kCols * 4 : 0;
+    static constexpr int kBytes = 2 * kResident + (S1 + S2) * kStream + 1024 + 256 + kStats;  // tiles, alignment, barriers, column statistics
+    // BT = 128: what the compiler assigns under __launch_bounds__(384, 1) and the roles' budgets (setmaxnreg)
+    static constexpr int kLaunchRegs = 168, kRegsLight = 72, kRegsCompute = 216;
+    static_assert(BT == 64 || 128 * kRegsLight + 256 * kRegsCompute <= kLaunchRegs * kThreads, "register budgets exceed the launch allocation");
+    static_assert(2 * BT + 2 * D <= kTmemCols && (2 * (S1 + S2) + 9) * 8 + 8 <= 256, "tensor memory / barrier space");
 };
 
-template <int D, bool DKDV, int BUFS, int WGS>
-__global__ void __launch_bounds__(threads_of(WGS), BUFS == 1 ? 2 : 1)
+template <int D, bool DKDV, int BT>
+__global__ void __launch_bounds__(BwdConfig<D, DKDV, BT>::kThreads, BwdConfig<D, DKDV, BT>::kCtas)
 attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant__ CUtensorMap map_r2,
                      const __grid_constant__ CUtensorMap map_t1, const __grid_constant__ CUtensorMap map_t2, const BwdArgs p) {
-    constexpr int kResident = BwdSmem<D, BUFS>::kResident, kStream = BwdSmem<D, BUFS>::kStream, STAGES = BwdSmem<D, BUFS>::STAGES;
-    constexpr int kTmemCols = BUFS == 1 ? 256 : 512;
-    constexpr bool SPLIT = BUFS == 1 && WGS == 2;  // both warpgroups on every iteration, half of the streamed columns each
-    static_assert(BUFS == 1 || BUFS == 2, "one X/Y buffer (two CTAs per SM) or two");
-    static_assert(BUFS == 2 || D == 64, "single X/Y buffers with 256 columns only fit the accumulators of head dim 64");
-    static_assert(BUFS == 1 || WGS == BUFS, "several X/Y buffers are worked by one warpgroup each");
-    static_assert(2 * BUFS * 64 + 2 * D <= kTmemCols && (1 + 2 * STAGES + 4 * BUFS + 2) * 8 + 8 <= 256, "tensor memory / barrier space");
+    using C = BwdConfig<D, DKDV, BT>;
+    constexpr int kResident = C::kResident, kStream = C::kStream, S1 = C::S1, S2 = C::S2, kTmemCols = C::kTmemCols, COLS = C::kCols;
     constexpr int kRBlock = BR * 128, kTBlock = BT * 128;  // bytes of one 64-wide head-dim block of a tile
     constexpr int DB = D / 64;
     extern __shared__ uint8_t smem_raw[];
@@ -102,24 +104,27 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
     uint8_t* sr1 = smem;
     uint8_t* sr2 = smem + kResident;
     uint8_t* st1 = smem + 2 * kResident;
-    uint8_t* st2 = st1 + STAGES * kStream;
-    uint64_t* bars = (uint64_t*)(st2 + STAGES * kStream);
+    uint8_t* st2 = st1 + S1 * kStream;
+    uint64_t* bars = (uint64_t*)(st2 + S2 * kStream);
     uint64_t* r_full = bars;             // 1
-    uint64_t* t_full = bars + 1;             // STAGES
-    uint64_t* t_empty = t_full + STAGES;     // STAGES
-    uint64_t* xy_full = t_empty + STAGES;    // BUFS
-    uint64_t* pz_ready = xy_full + BUFS;     // BUFS (one arrival per compute thread)
-    uint64_t* acc_full = pz_ready + BUFS;    // 1
-    uint64_t* y_full = acc_full + 1;         // BUFS, split columns only: Y lands on its own (xy_full then means X)
-    uint64_t* x_empty = y_full + BUFS;       // BUFS, split columns only: every compute thread has loaded its X values
-    uint64_t* z_free = x_empty + BUFS;       // 1, split columns in dQ mode: the accumulation that read Z has completed
-    uint32_t* tmem_slot = (uint32_t*)(z_free + 1);
+    uint64_t* t1_full = bars + 1;        // S1
+    uint64_t* t1_empty = t1_full + S1;   // S1
+    uint64_t* t2_full = t1_empty + S1;   // S2
+    uint64_t* t2_empty = t2_full + S2;   // S2
+    uint64_t* x_full = t2_empty + S2;    // X is in tensor memory
+    uint64_t* y_full = x_full + 1;       // Y is
+    uint64_t* x_empty = y_full + 1;      // every compute thread has loaded its X values
+    uint64_t* y_empty = x_empty + 1;     // dQ mode: ... its Y values
+    uint64_t* pz_ready = y_empty + 1;    // every compute thread has written P and Z
+    uint64_t* z_free = pz_ready + 1;     // dQ mode: the accumulation that read Z has completed
+    uint64_t* acc_full = z_free + 1;     // everything has
+    uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
-    // dkdv mode: log-sum-exp (in log2 units) and delta of the streamed query tile, one private copy per compute warp
-    // ([warp][lse|delta][BT]) so that staging needs no barrier across warps
+    // dkdv mode: minus the log-sum-exp (in log2 units) and minus delta * scale of a compute warp's streamed columns, one
+    // private copy per warp ([warp][lse|delta][COLS]) so that staging needs no barrier across warps
     float* col_stats = (float*)((uint8_t*)bars + 256);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform for the compiler too
     const int tile = DKDV ? (int)blockIdx.x : (int)(gridDim.x - 1 - blockIdx.x);
     const int head = blockIdx.y, batch = blockIdx.z;  // kv head in dkdv mode, query head in dq mode
     const int group = p.N / p.Nkv;
@@ -146,18 +151,21 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
 
     if (threadIdx.x == 0) {
         mbar_init(r_full, 1);
-        for (int s = 0; s < STAGES; s++) {
-            mbar_init(&t_full[s], 1);
-            mbar_init(&t_empty[s], 1);
+        for (int s = 0; s < S1; s++) {
+            mbar_init(&t1_full[s], 1);
+            mbar_init(&t1_empty[s], 1);
         }
-        for (int s = 0; s < BUFS; s++) {
-            mbar_init(&xy_full[s], 1);
-            mbar_init(&pz_ready[s], SPLIT ? 256 : 128);
-            mbar_init(&y_full[s], 1);
-            mbar_init(&x_empty[s], 256);
+        for (int s = 0; s < S2; s++) {
+            mbar_init(&t2_full[s], 1);
+            mbar_init(&t2_empty[s], 1);
         }
-        mbar_init(acc_full, 1);
+        mbar_init(x_full, 1);
+        mbar_init(y_full, 1);
+        mbar_init(x_empty, 256);
+        mbar_init(y_empty, 256);
+        mbar_init(pz_ready, 256);
         mbar_init(z_free, 1);
+        mbar_init(acc_full, 1);
         *abort_flag = 0;
         fence_barrier_init();
     }
@@ -168,31 +176,21 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-    const uint32_t tmem_x = tmem_base;                    // BUFS X buffers of 64 columns (P written over their first 32)
-    const uint32_t tmem_y = tmem_base + BUFS * 64;        // BUFS Y buffers (Z over their first 32 columns)
-    const uint32_t tmem_a = tmem_base + 2 * BUFS * 64;    // acc_a: D columns
-    const uint32_t tmem_b = tmem_a + D;                   // acc_b: D columns
-    // iteration `it` uses X/Y buffer it % BUFS; its barriers complete once per BUFS iterations
-    // bf16 P / Z of 16 streamed rows take 8 columns. A thread writes them over the START of the columns it read, so
-    // with split columns the second warpgroup's halves sit at columns 32.. (never over columns the first still reads)
-    auto pz_col = [](int k) { return SPLIT ? (k >> 1) * 32 + (k & 1) * 8 : k * 8; };  // k-th group of 16 streamed rows
-    // dK/dV mode with split columns: P and Z share the X buffer (P in the first, Z in the second 16 of a thread's 32
-    // columns), written with ONE tensor-memory store per iteration - a store's issue cost is paid once
-    // With split columns P and Z live in the Y buffer (dK/dV mode: P in the first, Z in the second 16 of a thread's 32
-    // columns, written with ONE tensor-memory store; dQ mode: Z alone), so that X is free as soon as every thread has
-    // loaded it: the next tile's X product is issued during this tile's element-wise phase, and its exponentials start
-    // before the next Y - which has to wait for the accumulation products that read P and Z - has landed.
-    // In dQ mode with split columns the second accumulator's columns are unused: Z goes there, so Y is free once it is
-    // loaded as well, and BOTH products of the next tile run under this tile's element-wise phase.
-    constexpr bool PZ_TOGETHER = SPLIT && DKDV;
-    constexpr bool DQ_EARLY = SPLIT && !DKDV;
-    const uint32_t tmem_p = SPLIT ? tmem_y : tmem_x;
-    const uint32_t tmem_z = PZ_TOGETHER ? tmem_y + 16 : (DQ_EARLY ? tmem_b : tmem_y);
-    auto buf_of = [](int it) { return it % BUFS; };
-    auto par_of = [](int it) { return (uint32_t)(it / BUFS) & 1u; };
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    const uint32_t tmem_x = tmem_base;
+    const uint32_t tmem_y = tmem_base + BT;
+    const uint32_t tmem_a = tmem_base + 2 * BT;  // acc_a: D columns
+    const uint32_t tmem_b = tmem_a + D;          // acc_b: D columns (dkdv mode)
+    // bf16 values of 16 streamed rows take 8 columns; a warpgroup's lie within the COLS columns it read: in dkdv mode P in
+    // the first and Z in the second half of them
+    auto pz_col = [](int k) { return k / (COLS / 16) * COLS + k % (COLS / 16) * 8; };  // k-th group of 16 streamed rows
+    const uint32_t tmem_p = tmem_y;
+    const uint32_t tmem_z = DKDV ? tmem_y + COLS / 2 : tmem_b;
 
-    if (warp == 0) {
+    // each register budget is set inside the branch it governs: code after a join is compiled for the smallest one
+    if (warp < C::kFirst) {
+      if constexpr (BT == 128) regs_dec<C::kRegsLight>();
+      if (warp == 0) {
         if (lane == 0 && n_iter > 0) {
             tma_prefetch_desc(&map_r1);
             tma_prefetch_desc(&map_r2);
@@ -205,131 +203,139 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
             }
             bool ok = true;
             for (int it = 0; it < n_iter && ok; it++) {
-                const int stage = it % STAGES;
-                const uint32_t ph = (uint32_t)(it / STAGES) & 1;
+                const int a = it % S1, b = it % S2;
                 const int hh = it / per_head;
                 const int t = t_begin + it - hh * per_head;
                 const int t_head = DKDV ? head * group + hh : kv_head_of_q;
-                if (!(ok = mbar_wait(&t_empty[stage], ph ^ 1, abort_flag))) break;
-                mbar_expect_tx(&t_full[stage], 2 * kStream);
-                for (int d = 0; d < DB; d++) {
-                    tma_load_4d(st1 + stage * kStream + d * kTBlock, &map_t1, &t_full[stage], d * 64, t_head, t * BT, batch);
-                    tma_load_4d(st2 + stage * kStream + d * kTBlock, &map_t2, &t_full[stage], d * 64, t_head, t * BT, batch);
-                }
+                if (!(ok = mbar_wait(&t1_empty[a], ((uint32_t)(it / S1) & 1) ^ 1, abort_flag))) break;
+                mbar_expect_tx(&t1_full[a], kStream);
+                for (int d = 0; d < DB; d++) tma_load_4d(st1 + a * kStream + d * kTBlock, &map_t1, &t1_full[a], d * 64, t_head, t * BT, batch);
+                if (!(ok = mbar_wait(&t2_empty[b], ((uint32_t)(it / S2) & 1) ^ 1, abort_flag))) break;
+                mbar_expect_tx(&t2_full[b], kStream);
+                for (int d = 0; d < DB; d++) tma_load_4d(st2 + b * kStream + d * kTBlock, &map_t2, &t2_full[b], d * 64, t_head, t * BT, batch);
             }
         }
-    } else if (warp == 1) {
-        if (lane == 0 && n_iter > 0) {
+      } else if (warp == 1) {
+        if (n_iter > 0) {  // the whole warp: the operands stay in uniform registers
+            const bool leader = elect_one();
             const uint32_t idesc_xy = make_idesc(BR, BT, true, false, false);
             const uint32_t idesc_acc = make_idesc(BR, D, true, false, true);
-            bool ok = mbar_wait(r_full, 0, abort_flag);
-            // Descriptors are built once and advanced by adds: the one issuing thread is otherwise bound by its own
-            // integer instructions, not by the tensor pipe (47 cycles per N = 64 MMA against 94 with rebuilt descriptors).
+            bool ok = mbar_wait_warp(r_full, 0, abort_flag);
+            // descriptors are built once and advanced by adds
             const uint64_t dr1 = make_smem_desc(smem_u32(sr1), 16, 1024), dr2 = make_smem_desc(smem_u32(sr2), 16, 1024);
             const uint64_t dt1 = make_smem_desc(smem_u32(st1), 16, 1024), dt2 = make_smem_desc(smem_u32(st2), 16, 1024);
             const uint64_t dt1_mn = make_smem_desc(smem_u32(st1), kTBlock, 1024), dt2_mn = make_smem_desc(smem_u32(st2), kTBlock, 1024);
             auto issue_x = [&](int it) -> bool {
-                const int stage = it % STAGES;
-                if (!mbar_wait(&t_full[stage], (uint32_t)(it / STAGES) & 1, abort_flag)) return false;
+                const int stage = it % S1;
+                if (!mbar_wait_warp(&t1_full[stage], (uint32_t)(it / S1) & 1, abort_flag)) return false;
                 tc_fence_after();
-                const int buf = buf_of(it);
                 const uint64_t t1 = desc_advance(dt1, (uint32_t)(stage * kStream));
 #pragma unroll
                 for (int k = 0; k < D / 16; k++) {
                     const uint32_t roff = (uint32_t)((k / 4) * kRBlock + (k % 4) * 32), toff = (uint32_t)((k / 4) * kTBlock + (k % 4) * 32);
-                    mma_f16(tmem_x + buf * 64, desc_advance(dr1, roff), desc_advance(t1, toff), idesc_xy, k != 0);
+                    mma_f16(tmem_x, desc_advance(dr1, roff), desc_advance(t1, toff), idesc_xy, k != 0, leader);
                 }
-                if (SPLIT) mma_commit(&xy_full[buf]);
+                mma_commit(x_full, leader);
                 return true;
             };
-            auto issue_y = [&](int it) {  // after issue_x(it): the tile has landed
-                const int stage = it % STAGES, buf = buf_of(it);
+            auto issue_y = [&](int it) -> bool {
+                const int stage = it % S2;
+                if (!mbar_wait_warp(&t2_full[stage], (uint32_t)(it / S2) & 1, abort_flag)) return false;
+                tc_fence_after();
                 const uint64_t t2 = desc_advance(dt2, (uint32_t)(stage * kStream));
 #pragma unroll
                 for (int k = 0; k < D / 16; k++) {
                     const uint32_t roff = (uint32_t)((k / 4) * kRBlock + (k % 4) * 32), toff = (uint32_t)((k / 4) * kTBlock + (k % 4) * 32);
-                    mma_f16(tmem_y + buf * 64, desc_advance(dr2, roff), desc_advance(t2, toff), idesc_xy, k != 0);
+                    mma_f16(tmem_y, desc_advance(dr2, roff), desc_advance(t2, toff), idesc_xy, k != 0, leader);
                 }
-                mma_commit(SPLIT ? &y_full[buf] : &xy_full[buf]);
-            };
-            auto issue_xy = [&](int it) -> bool {
-                if (!issue_x(it)) return false;
-                issue_y(it);
+                mma_commit(y_full, leader);
+                if (!DKDV) mma_commit(&t2_empty[stage], leader);
                 return true;
             };
-            if (ok) ok = issue_xy(0);
-            for (int pre = 1; pre < BUFS && pre < n_iter && ok; pre++) ok = issue_xy(pre);
+            if (ok) ok = issue_x(0) && issue_y(0);
             for (int it = 0; it < n_iter && ok; it++) {
-                const int buf = buf_of(it), stage = it % STAGES;
-                if (SPLIT && it + 1 < n_iter) {  // X is free once it is loaded: the next one runs under this tile's element-wise phase
-                    if (!(ok = mbar_wait(&x_empty[buf], par_of(it), abort_flag))) break;
+                const uint32_t par = (uint32_t)it & 1;
+                if (it + 1 < n_iter) {
+                    if (!(ok = mbar_wait_warp(x_empty, par, abort_flag))) break;
                     tc_fence_after();
                     if (!(ok = issue_x(it + 1))) break;
-                    if (DQ_EARLY) issue_y(it + 1);  // x_empty then says that X and Y are both in registers
+                    if (!DKDV) {
+                        if (!(ok = mbar_wait_warp(y_empty, par, abort_flag))) break;
+                        tc_fence_after();
+                        if (!(ok = issue_y(it + 1))) break;
+                    }
                 }
-                if (!(ok = mbar_wait(&pz_ready[buf], par_of(it), abort_flag))) break;
+                if (!(ok = mbar_wait_warp(pz_ready, par, abort_flag))) break;
                 tc_fence_after();
-                const uint64_t t1 = desc_advance(dt1_mn, (uint32_t)(stage * kStream)), t2 = desc_advance(dt2_mn, (uint32_t)(stage * kStream));
+                const int a = it % S1, b = it % S2;
+                const uint64_t t1 = desc_advance(dt1_mn, (uint32_t)(a * kStream)), t2 = desc_advance(dt2_mn, (uint32_t)(b * kStream));
 #pragma unroll
                 for (int k = 0; k < BT / 16; k++)  // acc_a += Z . T1   (T1 as an MN-major operand: 16 rows = 2048 bytes per step)
-                    mma_f16_ts(tmem_a, tmem_z + buf * 64 + pz_col(k), desc_advance(t1, k * 2048), idesc_acc, (it | k) != 0);
+                    mma_f16_ts(tmem_a, tmem_z + pz_col(k), desc_advance(t1, k * 2048), idesc_acc, (it | k) != 0, leader);
+                mma_commit(&t1_empty[a], leader);
                 if (DKDV) {
 #pragma unroll
                     for (int k = 0; k < BT / 16; k++)  // acc_b += P . T2
-                        mma_f16_ts(tmem_b, tmem_p + buf * 64 + pz_col(k), desc_advance(t2, k * 2048), idesc_acc, (it | k) != 0);
-                }
-                mma_commit(&t_empty[stage]);
-                if (DQ_EARLY) {
-                    mma_commit(z_free);
-                } else if (SPLIT) {
-                    if (it + 1 < n_iter) issue_y(it + 1);  // behind the products that read P and Z in Y's columns: the tensor pipe runs in order
-                } else if (it + BUFS < n_iter) {
-                    ok = issue_xy(it + BUFS);  // behind the products that read P and Z
+                        mma_f16_ts(tmem_b, tmem_p + pz_col(k), desc_advance(t2, k * 2048), idesc_acc, (it | k) != 0, leader);
+                    mma_commit(&t2_empty[b], leader);
+                    if (it + 1 < n_iter) ok = issue_y(it + 1);  // behind the products that read P and Z in Y's columns: the tensor pipe runs in order
+                } else {
+                    mma_commit(z_free, leader);
                 }
             }
-            if (ok) mma_commit(acc_full);
+            if (ok) mma_commit(acc_full, leader);
         }
+      }
     } else {
-        // ---- compute warps: thread = resident row. Two warpgroups (warps 2..5 and 6..9) take alternate iterations, each
-        // owning one X/Y buffer, so that two rows of exponentials and conversions are in flight per scheduler. ----
-        const int wg = (warp - 2) >> 2;
+        if constexpr (BT == 128) regs_inc<C::kRegsCompute>();
+        // ---- compute warps: thread = resident row, warpgroup = half of the streamed columns ----
+        const int wg = (warp - C::kFirst) >> 2;
         const int quarter = warp & 3;
         const int row_in_tile = quarter * 32 + lane;
         const long long row = (long long)r0 + row_in_tile;  // key index (dkdv) or query index (dq)
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+        const uint32_t my_x = tmem_x + lane_addr + wg * COLS, my_y = tmem_y + lane_addr + wg * COLS;
         const float LOG2E = 1.4426950408889634f;
-        float row_lse = 0.0f, row_delta = 0.0f;
+        float row_lse = 0.0f, row_delta = 0.0f;  // negated, as the staged columns' are
         if (!DKDV && row < p.Sq) {
             const long long at = ((long long)batch * p.N + head) * p.Sq + row;
-            row_lse = p.lse[at] * LOG2E;
-            row_delta = p.delta[at] * p.scale;
+            row_lse = -(p.lse[at] * LOG2E);
+            row_delta = -(p.delta[at] * p.scale);
         }
+        // dkdv: the lane's share of the next tile's column statistics is fetched one iteration ahead
+        float next_lse[COLS / 32], next_delta[COLS / 32];
+        auto fetch_stats = [&](int it) {
+            const int hh = it / per_head;
+            const long long at = ((long long)batch * p.N + (head * group + hh)) * p.Sq;
+            const long long c = (long long)(t_begin + it - hh * per_head) * BT + wg * COLS + lane;
+#pragma unroll
+            for (int u = 0; u < COLS / 32; u++) {
+                const long long cc = min(c + 32 * u, (long long)p.Sq - 1);
+                next_lse[u] = __ldg(p.lse + at + cc);
+                next_delta[u] = __ldg(p.delta + at + cc);
+            }
+        };
+        if (DKDV && n_iter > 0) fetch_stats(0);
+        float* stat_lse = col_stats + (warp - C::kFirst) * 2 * COLS;
+        float* stat_delta = stat_lse + COLS;
         bool ok = true;
-        constexpr int NC = SPLIT ? 1 : BT / 32;  // 32-column chunks of the streamed tile this thread works on ...
-        const int c_first = SPLIT ? wg : 0;      // ... starting at this one
-        for (int it = SPLIT ? 0 : wg; it < n_iter && ok; it += SPLIT ? 1 : WGS) {
-            const int buf = buf_of(it);
+        for (int it = 0; it < n_iter && ok; it++) {
+            const uint32_t par = (uint32_t)it & 1;
             const int hh = it / per_head;
             const int t = t_begin + it - hh * per_head;
-            const long long c0 = (long long)t * BT;  // first streamed index: query (dkdv) or key (dq)
-            float* stat_lse = col_stats + (warp - 2) * 2 * BT;
-            float* stat_delta = stat_lse + BT;
+            const long long c0 = (long long)t * BT + wg * COLS;  // this thread's first streamed index: query (dkdv) or key (dq)
             if (DKDV) {
-                // each warp stages the tile's 64 log-sum-exps and 64 deltas once; its lanes then read them as shared-memory
+                // each warp stages its columns' log-sum-exps and deltas once; its lanes then read them as shared-memory
                 // broadcasts instead of two global loads per score
-                const long long at = ((long long)batch * p.N + (head * group + hh)) * p.Sq;
                 __syncwarp();  // every lane is done with the previous tile's values
 #pragma unroll
-                for (int u = 0; u < BT / 32; u++) {
-                    const long long cc = min(c0 + lane + 32 * u, (long long)p.Sq - 1);
-                    stat_lse[lane + 32 * u] = __ldg(p.lse + at + cc) * LOG2E;
-                    stat_delta[lane + 32 * u] = __ldg(p.delta + at + cc) * p.scale;
+                for (int u = 0; u < COLS / 32; u++) {
+                    stat_lse[lane + 32 * u] = -(next_lse[u] * LOG2E);
+                    stat_delta[lane + 32 * u] = -(next_delta[u] * p.scale);
                 }
                 __syncwarp();
+                if (it + 1 < n_iter) fetch_stats(it + 1);
             }
-            if (!(ok = mbar_wait(&xy_full[buf], par_of(it), abort_flag))) break;
-            __syncwarp();
-            tc_fence_after();
             // columns visible to this row: dkdv: query i sees key `row` iff row <= i + off  <=>  i >= row - off, and i < Sq
             //                              dq:   key j visible iff j <= row + off and j < Sk
             long long col_lo, col_hi;  // visible columns are [col_lo, col_hi)
@@ -340,155 +346,81 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
                 col_lo = 0;
                 col_hi = p.causal ? min((long long)p.Sk, row + p.causal_offset + 1) : (long long)p.Sk;
             }
-            // tile-relative visible range [lo, hi) in 32-bit; the unmasked version runs unless some row of the warp is cut
-            const int lo = (int)max(0LL, min(col_lo - c0, (long long)BT)), hi = (int)max(0LL, min(col_hi - c0, (long long)BT));
-            const bool masked_tile = __any_sync(0xffffffffu, lo > 0 || hi < BT);
-            // two-buffer form (head dim 128): X and Y in one load round trip, P over X and Z over Y
-            bool early_ok = true;
-            auto compute = [&](auto masked) {
-                // P and Z = dS of one 32-column chunk from its scores and dP values, written back as bf16 TMEM operands
-                auto chunk = [&](int c, const uint32_t* x, const uint32_t* y) {
-                    uint32_t pp[16], zz[16];
+            // visible range [lo, hi) relative to the thread's columns, in 32-bit; no mask is applied unless some row of the
+            // warp is cut
+            const int lo = (int)max(0LL, min(col_lo - c0, (long long)COLS)), hi = (int)max(0LL, min(col_hi - c0, (long long)COLS));
+            const bool masked_tile = __any_sync(0xffffffffu, lo > 0 || hi < COLS);
+            if (!(ok = mbar_wait(x_full, par, abort_flag))) break;
+            __syncwarp();
+            tc_fence_after();
+            float pr[COLS];
+            {
+                uint32_t x[COLS];
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4) {
-                        float lse4[4], dsc4[4];  // log-sum-exp (log2 units) and delta * scale of the four columns
-                        if (DKDV) {
-                            const float4 l4 = *(const float4*)(stat_lse + c * 32 + i), d4 = *(const float4*)(stat_delta + c * 32 + i);
-                            lse4[0] = l4.x, lse4[1] = l4.y, lse4[2] = l4.z, lse4[3] = l4.w;
-                            dsc4[0] = d4.x, dsc4[1] = d4.y, dsc4[2] = d4.z, dsc4[3] = d4.w;
-                        } else {
-#pragma unroll
-                            for (int u = 0; u < 4; u++) lse4[u] = row_lse, dsc4[u] = row_delta;
-                        }
-                        // two columns per instruction (packed float32 FMA / MUL of sm_100): the element-wise phase is bound by
-                        // instruction issue while it runs, and each lane's roundings are those of the scalar form
-                        float pv[4], zv[4];
-#pragma unroll
-                        for (int u = 0; u < 4; u += 2) {
-                            const int e = c * 32 + i + u;  // column within the streamed tile
-                            const float2 arg = __ffma2_rn(make_float2(__uint_as_float(x[i + u]), __uint_as_float(x[i + u + 1])),
-                                                          make_float2(p.scale_log2, p.scale_log2), make_float2(-lse4[u], -lse4[u + 1]));
-                            float2 pr = make_float2(fast_exp2(arg.x), fast_exp2(arg.y));
-                            if (decltype(masked)::value) {
-                                if (e < lo || e >= hi) pr.x = 0.0f;
-                                if (e + 1 < lo || e + 1 >= hi) pr.y = 0.0f;
-                            }
-                            const float2 t = __ffma2_rn(make_float2(__uint_as_float(y[i + u]), __uint_as_float(y[i + u + 1])),
-                                                        make_float2(p.scale, p.scale), make_float2(-dsc4[u], -dsc4[u + 1]));
-                            const float2 z = __fmul2_rn(pr, t);  // P * (dP - delta) * scale
-                            pv[u] = pr.x, pv[u + 1] = pr.y, zv[u] = z.x, zv[u + 1] = z.y;
-                        }
-#pragma unroll
-                        for (int u = 0; u < 4; u += 2) {
-                            __nv_bfloat162 ph2 = __floats2bfloat162_rn(pv[u], pv[u + 1]);
-                            __nv_bfloat162 zh2 = __floats2bfloat162_rn(zv[u], zv[u + 1]);
-                            pp[(i + u) / 2] = *(uint32_t*)&ph2;
-                            zz[(i + u) / 2] = *(uint32_t*)&zh2;
-                        }
-                    }
-                    if (DKDV) tmem_st_32x16(tmem_x + lane_addr + buf * 64 + pz_col(2 * c), pp);
-                    tmem_st_32x16(tmem_z + lane_addr + buf * 64 + pz_col(2 * c), zz);
-                };
-                // all of the thread's scores and dP values in one round trip to tensor memory
-                uint32_t x[NC * 32], y[NC * 32];
-#pragma unroll
-                for (int cc = 0; cc < NC; cc++) {
-                    tmem_ld_32x32(tmem_x + lane_addr + buf * 64 + (c_first + cc) * 32, x + cc * 32);
-                    tmem_ld_32x32(tmem_y + lane_addr + buf * 64 + (c_first + cc) * 32, y + cc * 32);
-                }
-                tmem_ld_wait();
-                if (DQ_EARLY) {
-                    // X and Y are in registers: both products of the next tile may run now. Z(it) goes where Z(it - 1) was:
-                    // the accumulation that read it has completed, unless this warp overtook the tensor pipe.
-                    tc_fence_before();
-                    mbar_arrive(&x_empty[buf]);
-                    if (it > 0) {
-                        early_ok = __all_sync(0xffffffffu, mbar_wait(z_free, (uint32_t)(it - 1) & 1, abort_flag));  // warp-uniform
-                        if (!early_ok) return;
-                        tc_fence_after();
-                    }
-                }
-#pragma unroll
-                for (int cc = 0; cc < NC; cc++) chunk(c_first + cc, x + cc * 32, y + cc * 32);
-            };
-            // Split columns: the exponentials run on X alone while the tensor pipe is still busy with the previous tile's
-            // accumulation and this tile's Y; X is handed back for the next tile's product as soon as it is in registers.
-            auto compute_split = [&](auto masked) -> bool {
-                const int c = c_first;  // this warpgroup's 32 of the 64 streamed columns
-                uint32_t x[32];
-                tmem_ld_32x32(tmem_x + lane_addr + buf * 64 + c * 32, x);
+                for (int c = 0; c < COLS; c += 32) tmem_ld_32x32(my_x + c, x + c);
                 tmem_ld_wait();
                 tc_fence_before();
-                mbar_arrive(&x_empty[buf]);
-                float pr[32];
+                mbar_arrive(x_empty);  // X is handed back for the next tile's product
+                // two columns per instruction (packed float32 FMA / MUL of sm_100); each lane's roundings are those of the scalar form
 #pragma unroll
-                for (int i = 0; i < 32; i += 4) {
-                    float lse4[4];
-                    if (DKDV) {
-                        const float4 l4 = *(const float4*)(stat_lse + c * 32 + i);
-                        lse4[0] = l4.x, lse4[1] = l4.y, lse4[2] = l4.z, lse4[3] = l4.w;
-                    } else {
-#pragma unroll
-                        for (int u = 0; u < 4; u++) lse4[u] = row_lse;
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; u += 2) {
-                        const int e = c * 32 + i + u;  // column within the streamed tile
-                        const float2 arg = __ffma2_rn(make_float2(__uint_as_float(x[i + u]), __uint_as_float(x[i + u + 1])),
-                                                      make_float2(p.scale_log2, p.scale_log2), make_float2(-lse4[u], -lse4[u + 1]));
-                        float2 q = make_float2(fast_exp2(arg.x), fast_exp2(arg.y));
-                        if (decltype(masked)::value) {
-                            if (e < lo || e >= hi) q.x = 0.0f;
-                            if (e + 1 < lo || e + 1 >= hi) q.y = 0.0f;
-                        }
-                        pr[i + u] = q.x, pr[i + u + 1] = q.y;
-                    }
+                for (int i = 0; i < COLS; i += 4) {
+                    float4 l4 = make_float4(row_lse, row_lse, row_lse, row_lse);
+                    if (DKDV) l4 = *(const float4*)(stat_lse + i);
+                    const float2 s2 = make_float2(p.scale_log2, p.scale_log2);
+                    const float2 u = __ffma2_rn(make_float2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])), s2, make_float2(l4.x, l4.y));
+                    const float2 v = __ffma2_rn(make_float2(__uint_as_float(x[i + 2]), __uint_as_float(x[i + 3])), s2, make_float2(l4.z, l4.w));
+                    pr[i] = fast_exp2(u.x), pr[i + 1] = fast_exp2(u.y), pr[i + 2] = fast_exp2(v.x), pr[i + 3] = fast_exp2(v.y);
                 }
-                if (!mbar_wait(&y_full[buf], par_of(it), abort_flag)) return false;
-                __syncwarp();
-                tc_fence_after();
-                uint32_t y[32], both[32];
-                tmem_ld_32x32(tmem_y + lane_addr + buf * 64 + c * 32, y);
-                tmem_ld_wait();
+                if (masked_tile) {
 #pragma unroll
-                for (int i = 0; i < 32; i += 4) {
-                    float dsc4[4];  // delta * scale of the four columns
-                    if (DKDV) {
-                        const float4 d4 = *(const float4*)(stat_delta + c * 32 + i);
-                        dsc4[0] = d4.x, dsc4[1] = d4.y, dsc4[2] = d4.z, dsc4[3] = d4.w;
-                    } else {
-#pragma unroll
-                        for (int u = 0; u < 4; u++) dsc4[u] = row_delta;
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; u += 2) {
-                        const float2 t = __ffma2_rn(make_float2(__uint_as_float(y[i + u]), __uint_as_float(y[i + u + 1])),
-                                                    make_float2(p.scale, p.scale), make_float2(-dsc4[u], -dsc4[u + 1]));
-                        const float2 z = __fmul2_rn(make_float2(pr[i + u], pr[i + u + 1]), t);  // P * (dP - delta) * scale
-                        __nv_bfloat162 ph2 = __floats2bfloat162_rn(pr[i + u], pr[i + u + 1]);
-                        __nv_bfloat162 zh2 = __floats2bfloat162_rn(z.x, z.y);
-                        both[(i + u) / 2] = *(uint32_t*)&ph2;
-                        both[16 + (i + u) / 2] = *(uint32_t*)&zh2;
-                    }
+                    for (int i = 0; i < COLS; i++)
+                        if (i < lo || i >= hi) pr[i] = 0.0f;
                 }
-                tmem_st_32x32(tmem_y + lane_addr + buf * 64 + c * 32, both);  // P in the first, Z in the second 16 columns
-                return true;
-            };
-            if (PZ_TOGETHER) {
-                if (!(ok = masked_tile ? compute_split(std::true_type{}) : compute_split(std::false_type{}))) break;
+            }
+            if (!(ok = mbar_wait(y_full, par, abort_flag))) break;
+            __syncwarp();
+            tc_fence_after();
+            uint32_t y[COLS];
+#pragma unroll
+            for (int c = 0; c < COLS; c += 32) tmem_ld_32x32(my_y + c, y + c);
+            tmem_ld_wait();
+            if (!DKDV) {
+                tc_fence_before();
+                mbar_arrive(y_empty);
+            }
+            uint32_t pz[DKDV ? COLS : COLS / 2];  // P (dkdv mode), then Z, as bf16 pairs
+            constexpr int kZ = DKDV ? COLS / 2 : 0;
+#pragma unroll
+            for (int i = 0; i < COLS; i += 4) {
+                float4 d4 = make_float4(row_delta, row_delta, row_delta, row_delta);
+                if (DKDV) d4 = *(const float4*)(stat_delta + i);
+                const float2 s2 = make_float2(p.scale, p.scale);
+                const float2 u = __ffma2_rn(make_float2(__uint_as_float(y[i]), __uint_as_float(y[i + 1])), s2, make_float2(d4.x, d4.y));
+                const float2 v = __ffma2_rn(make_float2(__uint_as_float(y[i + 2]), __uint_as_float(y[i + 3])), s2, make_float2(d4.z, d4.w));
+                const float2 zu = __fmul2_rn(make_float2(pr[i], pr[i + 1]), u), zv = __fmul2_rn(make_float2(pr[i + 2], pr[i + 3]), v);  // P * (dP - delta) * scale
+                const __nv_bfloat162 hu = __floats2bfloat162_rn(zu.x, zu.y), hv = __floats2bfloat162_rn(zv.x, zv.y);
+                pz[kZ + i / 2] = *(const uint32_t*)&hu, pz[kZ + i / 2 + 1] = *(const uint32_t*)&hv;
+                if (DKDV) {
+                    const __nv_bfloat162 pu = __floats2bfloat162_rn(pr[i], pr[i + 1]), pv = __floats2bfloat162_rn(pr[i + 2], pr[i + 3]);
+                    pz[i / 2] = *(const uint32_t*)&pu, pz[i / 2 + 1] = *(const uint32_t*)&pv;
+                }
+            }
+            if constexpr (DKDV) {
+#pragma unroll
+                for (int c = 0; c < COLS; c += 32) tmem_st_32x32(my_y + c, pz + c);
             } else {
-                if (DQ_EARLY) {  // Y was issued with X: it has landed or is about to
-                    if (!(ok = mbar_wait(&y_full[buf], par_of(it), abort_flag))) break;
+                // Z(it) goes where Z(it - 1) was: the accumulation that read it has completed, unless this warp overtook the tensor pipe
+                if (it > 0) {
+                    if (!(ok = mbar_wait(z_free, par ^ 1, abort_flag))) break;
                     __syncwarp();
                     tc_fence_after();
                 }
-                if (masked_tile) compute(std::true_type{});
-                else compute(std::false_type{});
-                if (!(ok = early_ok)) break;
+                if constexpr (COLS == 64) tmem_st_32x32(tmem_z + lane_addr + wg * COLS, pz);
+                else tmem_st_32x16(tmem_z + lane_addr + wg * COLS, pz);
             }
             tmem_st_wait();
             tc_fence_before();
-            mbar_arrive(&pz_ready[buf]);
+            mbar_arrive(pz_ready);
         }
         // ---- epilogue: accumulators -> bf16 rows ----
         if (n_iter > 0) ok = ok && mbar_wait(acc_full, 0, abort_flag);
@@ -496,15 +428,14 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
         if (ok) {
             tc_fence_after();
             const long long limit = DKDV ? p.Sk : p.Sq;
-#pragma unroll 1
-            // dkdv: with several warpgroups, 0 writes dK and 1 writes dV; a single warpgroup writes both
-            for (int which = (DKDV && WGS >= 2) ? wg : 0; which < (DKDV ? (WGS >= 2 ? min(wg + 1, 2) : 2) : 1); which++) {
+            {
+                const int which = DKDV ? wg : 0;  // dkdv: warpgroup 0 writes dK, warpgroup 1 dV
                 uint16_t* base = (uint16_t*)(which == 0 ? p.out_a : p.out_b);
                 const long long sb = which == 0 ? p.a_sb : p.b_sb, ss = which == 0 ? p.a_ss : p.b_ss, sn = which == 0 ? p.a_sn : p.b_sn;
                 uint16_t* out = base + (long long)batch * sb + row * ss + (long long)head * sn;
                 const bool vec = (sb % 8 == 0) && (ss % 8 == 0) && (sn % 8 == 0) && (((uintptr_t)base & 15) == 0);
 #pragma unroll 1
-                for (int c = (DKDV || WGS == 1) ? 0 : wg; c < D / 32; c += (DKDV || WGS == 1) ? 1 : WGS) {  // dq: the warpgroups take 32-column chunks in turn
+                for (int c = DKDV ? 0 : wg; c < D / 32; c += DKDV ? 1 : 2) {  // dq: the warpgroups take 32-column chunks in turn
                     uint32_t v[32];
                     if (n_iter > 0) {
                         tmem_ld_32x32((which == 0 ? tmem_a : tmem_b) + lane_addr + c * 32, v);
@@ -527,7 +458,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
                             }
                             packed[i / 8] = make_uint4(w[0], w[1], w[2], w[3]);
                         }
-                        store_rows_coalesced<4>((uint4*)(sr1 + (warp - 2) * 2048), packed, (uint8_t*)(out - (long long)lane * ss + c * 32), ss * 2,
+                        store_rows_coalesced<4>((uint4*)(sr1 + (warp - C::kFirst) * 2048), packed, (uint8_t*)(out - (long long)lane * ss + c * 32), ss * 2,
                                                 (int)max(0LL, min(32LL, limit - (row - lane))), lane);
                     } else if (row < limit) {
 #pragma unroll
@@ -616,20 +547,34 @@ void launch_delta(const lb_tensor& o, const lb_tensor& d_o, float* delta, cudaSt
     LB_CUDA(cudaGetLastError());
 }
 
-template <int D>
-void launch_bwd(const CUtensorMap& mq128, const CUtensorMap& mdo128, const CUtensorMap& mk128, const CUtensorMap& mv128,
-                const CUtensorMap& mq64, const CUtensorMap& mdo64, const CUtensorMap& mk64, const CUtensorMap& mv64, BwdArgs dkdv,
-                BwdArgs dq, cudaStream_t s) {
-    constexpr int BUFS = D == 64 ? 1 : 2, WGS = 2;  // head dim 64: two CTAs per SM, both warpgroups on every iteration
-    constexpr int kBytes = BwdSmem<D, BUFS>::kBytes, kThreads = threads_of(WGS);
-    if (first_use_on_device((const void*)attention_bwd_kernel<D, true, BUFS, WGS>)) {
-        LB_CUDA(cudaFuncSetAttribute(attention_bwd_kernel<D, true, BUFS, WGS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes));
-        LB_CUDA(cudaFuncSetAttribute(attention_bwd_kernel<D, false, BUFS, WGS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes));
+template <int D, bool DKDV, int BT>
+void launch_bwd_kernel(const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap& t1, const CUtensorMap& t2, dim3 grid, const BwdArgs& p,
+                       cudaStream_t s) {
+    using C = BwdConfig<D, DKDV, BT>;
+    static const int regs = launch_regs((const void*)attention_bwd_kernel<D, DKDV, BT>);
+    if (BT == 128 && regs != C::kLaunchRegs)
+        fail(LB_ERR_UNSUPPORTED, format("attention backward: the kernel was built with %d registers per thread, its register budgets assume %d",
+                                        regs, C::kLaunchRegs));
+    if (first_use_on_device((const void*)attention_bwd_kernel<D, DKDV, BT>))
+        LB_CUDA(cudaFuncSetAttribute(attention_bwd_kernel<D, DKDV, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kBytes));
+    attention_bwd_kernel<D, DKDV, BT><<<grid, C::kThreads, C::kBytes, s>>>(r1, r2, t1, t2, p);
+}
+
+// The two kernels; `rows` makes the map of an operand's tiles, 128 or 64 rows high.
+template <class Rows>
+void launch_bwd(long long D, const Rows& rows, const lb_tensor& q, const lb_tensor& d_o, const lb_tensor& k, const lb_tensor& v, const BwdArgs& dkdv,
+                const BwdArgs& dq, cudaStream_t s) {
+    const CUtensorMap mq128 = rows(q, "query", 128), mdo128 = rows(d_o, "dO", 128), mk128 = rows(k, "key", 128), mv128 = rows(v, "value", 128);
+    const dim3 grid_kv((unsigned)((dkdv.Sk + BR - 1) / BR), (unsigned)dkdv.Nkv, (unsigned)dkdv.B);
+    const dim3 grid_q((unsigned)((dq.Sq + BR - 1) / BR), (unsigned)dq.N, (unsigned)dq.B);
+    if (D == 128) {
+        launch_bwd_kernel<128, true, 128>(mk128, mv128, mq128, mdo128, grid_kv, dkdv, s);
+        launch_bwd_kernel<128, false, 128>(mq128, mdo128, mk128, mv128, grid_q, dq, s);
+    } else {
+        const CUtensorMap mq64 = rows(q, "query", 64), mdo64 = rows(d_o, "dO", 64), mk64 = rows(k, "key", 64), mv64 = rows(v, "value", 64);
+        launch_bwd_kernel<64, true, 64>(mk128, mv128, mq64, mdo64, grid_kv, dkdv, s);
+        launch_bwd_kernel<64, false, 64>(mq128, mdo128, mk64, mv64, grid_q, dq, s);
     }
-    dim3 grid_kv((unsigned)((dkdv.Sk + BR - 1) / BR), (unsigned)dkdv.Nkv, (unsigned)dkdv.B);
-    attention_bwd_kernel<D, true, BUFS, WGS><<<grid_kv, kThreads, kBytes, s>>>(mk128, mv128, mq64, mdo64, dkdv);
-    dim3 grid_q((unsigned)((dq.Sq + BR - 1) / BR), (unsigned)dq.N, (unsigned)dq.B);
-    attention_bwd_kernel<D, false, BUFS, WGS><<<grid_q, kThreads, kBytes, s>>>(mq128, mdo128, mk64, mv64, dq);
 }
 
 }  // namespace
@@ -676,17 +621,13 @@ void attention_bwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor
     kv.out_b = dv.ptr, kv.b_sb = dv.stride[0], kv.b_ss = dv.stride[1], kv.b_sn = dv.stride[2];
     qq.out_a = dq.ptr, qq.a_sb = dq.stride[0], qq.a_ss = dq.stride[1], qq.a_sn = dq.stride[2];
     if (Sk == 0 || Sq == 0) fail(LB_ERR_UNSUPPORTED, "attention backward: empty sequences");
-    CUtensorMap mq128 = attention_map_rows(q, "query", 128), mdo128 = attention_map_rows(d_o, "dO", 128);
-    CUtensorMap mk128 = attention_map_rows(k, "key", 128), mv128 = attention_map_rows(v, "value", 128);
     if (dq_acc && attention_bwd_atomic_supported(q, dq)) {
         check_dense(*dq_acc, LB_F32, {B, Sq, N, D}, "attention dQ accumulator");
-        attention_bwd_atomic_launch(desc, mk128, mv128, mq128, mdo128, q, k, a.lse, a.delta, (float*)dq_acc->ptr, dq, dk, dv, s);
+        attention_bwd_atomic_launch(desc, attention_map_rows(k, "key", 128), attention_map_rows(v, "value", 128),
+                                    attention_map_rows(q, "query", 128), attention_map_rows(d_o, "dO", 128), q, k, a.lse, a.delta, (float*)dq_acc->ptr, dq, dk, dv, s);
         return;
     }
-    CUtensorMap mq64 = attention_map_rows(q, "query", 64), mdo64 = attention_map_rows(d_o, "dO", 64);
-    CUtensorMap mk64 = attention_map_rows(k, "key", 64), mv64 = attention_map_rows(v, "value", 64);
-    if (D == 128) launch_bwd<128>(mq128, mdo128, mk128, mv128, mq64, mdo64, mk64, mv64, kv, qq, s);
-    else launch_bwd<64>(mq128, mdo128, mk128, mv128, mq64, mdo64, mk64, mv64, kv, qq, s);
+    launch_bwd(D, attention_map_rows, q, d_o, k, v, kv, qq, s);
     LB_CUDA(cudaGetLastError());
 }
 
@@ -829,12 +770,7 @@ void attention_bwd_static(const lb_attn_desc& desc, const lb_tensor& q, const lb
     kv.out_a = dk.ptr, kv.a_sb = dk.stride[0], kv.a_ss = dk.stride[1], kv.a_sn = dk.stride[2];
     kv.out_b = dv.ptr, kv.b_sb = dv.stride[0], kv.b_ss = dv.stride[1], kv.b_sn = dv.stride[2];
     qq.out_a = dq.ptr, qq.a_sb = dq.stride[0], qq.a_ss = dq.stride[1], qq.a_sn = dq.stride[2];
-    CUtensorMap mq128 = static_map(st, q, "query", 128), mdo128 = static_map(st, d_o, "dO", 128);
-    CUtensorMap mk128 = static_map(st, k, "key", 128), mv128 = static_map(st, v, "value", 128);
-    CUtensorMap mq64 = static_map(st, q, "query", 64), mdo64 = static_map(st, d_o, "dO", 64);
-    CUtensorMap mk64 = static_map(st, k, "key", 64), mv64 = static_map(st, v, "value", 64);
-    if (D == 128) launch_bwd<128>(mq128, mdo128, mk128, mv128, mq64, mdo64, mk64, mv64, kv, qq, s);
-    else launch_bwd<64>(mq128, mdo128, mk128, mv128, mq64, mdo64, mk64, mv64, kv, qq, s);
+    launch_bwd(D, [&](const lb_tensor& t, const char* what, int box_rows) { return static_map(st, t, what, box_rows); }, q, d_o, k, v, kv, qq, s);
     LB_CUDA(cudaGetLastError());
 }
 

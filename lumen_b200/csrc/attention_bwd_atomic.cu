@@ -80,11 +80,6 @@ __device__ __forceinline__ void tma_reduce_add_4d(const CUtensorMap* map, const 
                  "r"(smem_u32(src_smem)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                  : "memory");
 }
-// Register budget of the calling warpgroup (all four of its warps execute this): the kernel starts with 128 per thread.
-template <int N>
-__device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N>
-__device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 // Barrier `id` over `count` threads (a warpgroup): the CTA-wide barrier 0 stays free for the other roles.
 __device__ __forceinline__ void named_barrier(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
@@ -118,7 +113,7 @@ attention_bwd_atomic_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform for the compiler too
     const int tile = (int)blockIdx.x, head = (int)blockIdx.y, batch = (int)blockIdx.z;  // key tile, kv head
     const int group = p.N / p.Nkv;
     const int r0 = tile * BR;
@@ -151,7 +146,7 @@ attention_bwd_atomic_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const uint32_t tmem_x = tmem_base, tmem_y = tmem_base + 128, tmem_dk = tmem_base + 256, tmem_dv = tmem_base + 320;
     const uint32_t tmem_dq = tmem_base + 384, tmem_p = tmem_base + 448;
 
@@ -181,11 +176,12 @@ attention_bwd_atomic_kernel(const __grid_constant__ CUtensorMap map_k, const __g
             }
         }
       } else if (warp == 1) {
-        if (lane == 0 && n_iter > 0) {
+        if (n_iter > 0) {  // the whole warp: the operands stay in uniform registers
+            const bool leader = elect_one();
             const uint32_t idesc_xy = make_idesc(BR, BT, true, false, false);  // K-major A and B
             const uint32_t idesc_acc = make_idesc(BR, D, true, false, true);   // A from tensor memory or K-major, B MN-major
             const uint32_t idesc_dq = make_idesc(BT, D, true, true, true);     // A and B MN-major
-            bool ok = mbar_wait(r_full, 0, abort_flag);
+            bool ok = mbar_wait_warp(r_full, 0, abort_flag);
             const uint64_t dk_k = make_smem_desc(smem_u32(sk), 16, 1024), dv_k = make_smem_desc(smem_u32(sv), 16, 1024);
             const uint64_t dk_mn = make_smem_desc(smem_u32(sk), kTile, 1024);
             const uint64_t dq_k = make_smem_desc(smem_u32(sq), 16, 1024), ddo_k = make_smem_desc(smem_u32(sdo), 16, 1024);
@@ -193,14 +189,14 @@ attention_bwd_atomic_kernel(const __grid_constant__ CUtensorMap map_k, const __g
             const uint64_t dz_k = make_smem_desc(smem_u32(sz), 16, 1024), dz_mn = make_smem_desc(smem_u32(sz), kZBlock, 1024);
             auto issue_xy = [&](int it) -> bool {
                 const int st = it % STAGES;
-                if (!mbar_wait(&t_full[st], (uint32_t)(it / STAGES) & 1, abort_flag)) return false;
+                if (!mbar_wait_warp(&t_full[st], (uint32_t)(it / STAGES) & 1, abort_flag)) return false;
                 tc_fence_after();
                 const uint64_t tq = desc_advance(dq_k, (uint32_t)(st * kTile)), tdo = desc_advance(ddo_k, (uint32_t)(st * kTile));
 #pragma unroll
-                for (int k = 0; k < D / 16; k++) mma_f16(tmem_x, desc_advance(dk_k, k * 32), desc_advance(tq, k * 32), idesc_xy, k != 0);
+                for (int k = 0; k < D / 16; k++) mma_f16(tmem_x, desc_advance(dk_k, k * 32), desc_advance(tq, k * 32), idesc_xy, k != 0, leader);
 #pragma unroll
-                for (int k = 0; k < D / 16; k++) mma_f16(tmem_y, desc_advance(dv_k, k * 32), desc_advance(tdo, k * 32), idesc_xy, k != 0);
-                mma_commit(xy_full);
+                for (int k = 0; k < D / 16; k++) mma_f16(tmem_y, desc_advance(dv_k, k * 32), desc_advance(tdo, k * 32), idesc_xy, k != 0, leader);
+                mma_commit(xy_full, leader);
                 return true;
             };
             if (ok) ok = issue_xy(0);
@@ -208,31 +204,31 @@ attention_bwd_atomic_kernel(const __grid_constant__ CUtensorMap map_k, const __g
                 const int st = it % STAGES;
                 const uint32_t par = (uint32_t)it & 1;
                 if (it + 1 < n_iter) {  // X and Y are in registers: the next tile's products run under this tile's element-wise phase
-                    if (!(ok = mbar_wait(xy_empty, par, abort_flag))) break;
+                    if (!(ok = mbar_wait_warp(xy_empty, par, abort_flag))) break;
                     tc_fence_after();
                     if (!(ok = issue_xy(it + 1))) break;
                 }
-                if (!(ok = mbar_wait(pz_ready, par, abort_flag))) break;
+                if (!(ok = mbar_wait_warp(pz_ready, par, abort_flag))) break;
                 tc_fence_after();
                 const uint64_t tq = desc_advance(dq_mn, (uint32_t)(st * kTile)), tdo = desc_advance(ddo_mn, (uint32_t)(st * kTile));
 #pragma unroll
                 for (int k = 0; k < BT / 16; k++)  // dV += P dO: 16 queries = 8 packed columns of P, 16 rows (2048 bytes) of dO
-                    mma_f16_ts(tmem_dv, tmem_p + k * 8, desc_advance(tdo, k * 2048), idesc_acc, (it | k) != 0);
+                    mma_f16_ts(tmem_dv, tmem_p + k * 8, desc_advance(tdo, k * 2048), idesc_acc, (it | k) != 0, leader);
 #pragma unroll
                 for (int k = 0; k < BT / 16; k++)  // dK += Z Q: Z K-major, 16 queries = 32 bytes of a row, 64-query blocks kZBlock apart
-                    mma_f16(tmem_dk, desc_advance(dz_k, (uint32_t)((k / 4) * kZBlock + (k % 4) * 32)), desc_advance(tq, k * 2048), idesc_acc, (it | k) != 0);
+                    mma_f16(tmem_dk, desc_advance(dz_k, (uint32_t)((k / 4) * kZBlock + (k % 4) * 32)), desc_advance(tq, k * 2048), idesc_acc, (it | k) != 0, leader);
                 if (it > 0) {
-                    if (!(ok = mbar_wait(dq_empty, par ^ 1, abort_flag))) break;
+                    if (!(ok = mbar_wait_warp(dq_empty, par ^ 1, abort_flag))) break;
                     tc_fence_after();
                 }
 #pragma unroll
                 for (int k = 0; k < BR / 16; k++)  // dQ' = Z^T K: Z MN-major (16 key rows = 2048 bytes per step), K MN-major
-                    mma_f16(tmem_dq, desc_advance(dz_mn, k * 2048), desc_advance(dk_mn, k * 2048), idesc_dq, k != 0);
-                mma_commit(&t_empty[st]);
-                mma_commit(pz_free);
-                mma_commit(dq_full);
+                    mma_f16(tmem_dq, desc_advance(dz_mn, k * 2048), desc_advance(dk_mn, k * 2048), idesc_dq, k != 0, leader);
+                mma_commit(&t_empty[st], leader);
+                mma_commit(pz_free, leader);
+                mma_commit(dq_full, leader);
             }
-            if (ok) mma_commit(acc_full);
+            if (ok) mma_commit(acc_full, leader);
         }
       }
     } else if (warp < 8) {
@@ -306,11 +302,11 @@ attention_bwd_atomic_kernel(const __grid_constant__ CUtensorMap map_k, const __g
             const uint32_t par = (uint32_t)it & 1;
             const int hh = it / per_head;
             const long long c0 = (long long)(t_begin + it - hh * per_head) * BT + wg * 64;  // first query column of this warpgroup
-            // each warp stages its 64 columns' statistics once (log2 units, times the scale): its lanes then read them as
+            // each warp stages its 64 columns' statistics once (log2 units, times the scale, negated): its lanes then read them as
             // shared-memory broadcasts
             __syncwarp();
 #pragma unroll
-            for (int u = 0; u < 2; u++) stat_lse[lane + 32 * u] = nl[u] * LOG2E, stat_delta[lane + 32 * u] = nd[u] * p.scale;
+            for (int u = 0; u < 2; u++) stat_lse[lane + 32 * u] = -(nl[u] * LOG2E), stat_delta[lane + 32 * u] = -(nd[u] * p.scale);
             __syncwarp();
             if (it + 1 < n_iter) load_stats(it + 1);
             if (!(ok = __all_sync(0xffffffffu, mbar_wait(xy_full, par, abort_flag)))) break;
@@ -338,14 +334,14 @@ attention_bwd_atomic_kernel(const __grid_constant__ CUtensorMap map_k, const __g
                         for (int u = 0; u < 4; u += 2) {
                             const int e = c * 32 + i + u, f = i + u;
                             const float2 arg = __ffma2_rn(make_float2(__uint_as_float(x[f]), __uint_as_float(x[f + 1])),
-                                                          make_float2(p.scale_log2, p.scale_log2), make_float2(-lse4[u], -lse4[u + 1]));
+                                                          make_float2(p.scale_log2, p.scale_log2), make_float2(lse4[u], lse4[u + 1]));
                             float2 pr = make_float2(fast_exp2(arg.x), fast_exp2(arg.y));
                             if (decltype(masked)::value) {
                                 if (e < lo || e >= hi) pr.x = 0.0f;
                                 if (e + 1 < lo || e + 1 >= hi) pr.y = 0.0f;
                             }
                             const float2 t = __ffma2_rn(make_float2(__uint_as_float(y[f]), __uint_as_float(y[f + 1])),
-                                                        make_float2(p.scale, p.scale), make_float2(-dsc4[u], -dsc4[u + 1]));
+                                                        make_float2(p.scale, p.scale), make_float2(dsc4[u], dsc4[u + 1]));
                             const float2 z = __fmul2_rn(pr, t);  // P * (dP - delta) * scale
                             __nv_bfloat162 ph2 = __floats2bfloat162_rn(pr.x, pr.y);
                             __nv_bfloat162 zh2 = __floats2bfloat162_rn(z.x, z.y);
@@ -495,14 +491,12 @@ void attention_bwd_atomic_launch(const lb_attn_desc& desc, const CUtensorMap& mk
     a.dk = dk.ptr, a.k_sb = dk.stride[0], a.k_ss = dk.stride[1], a.k_sn = dk.stride[2];
     a.dv = dv.ptr, a.v_sb = dv.stride[0], a.v_ss = dv.stride[1], a.v_sn = dv.stride[2];
     a.status = status_word();
-    if (first_use_on_device((const void*)attention_bwd_atomic_kernel)) {
-        cudaFuncAttributes attr;
-        LB_CUDA(cudaFuncGetAttributes(&attr, attention_bwd_atomic_kernel));
-        if (attr.numRegs != kLaunchRegs)
-            fail(LB_ERR_UNSUPPORTED, format("attention backward: the single-kernel form was built with %d registers per thread, its register "
-                                            "budgets assume %d", attr.numRegs, kLaunchRegs));
+    static const int regs = launch_regs((const void*)attention_bwd_atomic_kernel);
+    if (regs != kLaunchRegs)
+        fail(LB_ERR_UNSUPPORTED, format("attention backward: the single-kernel form was built with %d registers per thread, its register "
+                                        "budgets assume %d", regs, kLaunchRegs));
+    if (first_use_on_device((const void*)attention_bwd_atomic_kernel))
         LB_CUDA(cudaFuncSetAttribute(attention_bwd_atomic_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    }
     LB_CUDA(cudaMemsetAsync(dq_acc, 0, (size_t)B * Sq * N * D * 4, s));
     dim3 grid((unsigned)((Sk + BR - 1) / BR), (unsigned)Nkv, (unsigned)B);
     if (((uintptr_t)dq_acc & 15) != 0) fail(LB_ERR_UNSUPPORTED, "attention backward: the dQ accumulator must be 16-byte aligned");

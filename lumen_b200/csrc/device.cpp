@@ -126,6 +126,12 @@ bool first_use_on_device(const void* key) {
     return seen.emplace(dev, key).second;
 }
 
+int launch_regs(const void* kernel) {
+    cudaFuncAttributes attr;
+    LB_CUDA(cudaFuncGetAttributes(&attr, kernel));
+    return attr.numRegs;
+}
+
 int sm_count_hint() {
     int count = 0;
     if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0) {

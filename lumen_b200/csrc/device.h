@@ -63,6 +63,7 @@ struct GemmTuning {
 
 // SM count of the current device, or a B200's 148 where no device is usable (plan lowering on a CPU-only machine).
 int sm_count_hint();
+int launch_regs(const void* kernel);  // registers per thread a kernel was built with
 
 // Compiles CUDA C++ `source` for sm_100a and returns the cubin. `name` labels diagnostics.
 std::string nvrtc_compile(const std::string& name, const std::string& source);

@@ -327,3 +327,25 @@ def test_few_query_rows_against_float64(cuda, case):
     want, want_lse = attention_f64(q, k, v, causal)
     np.testing.assert_allclose(to_numpy(o).astype(np.float64), want, rtol=TOL, atol=TOL)
     np.testing.assert_allclose(to_numpy(lse), want_lse, rtol=1e-3, atol=1e-3)
+
+
+# (B, Sq, Sk, N, Nkv, H): the backward's 128-row streamed tiles at head dim 128 - one row of a second tile on either side, rings
+# that wrap (more tiles than stages), a group of heads walked by one CTA, more keys than queries, keys no query sees
+TILE_EDGE_CASES = [((1, 129, 129, 1, 1, 128), True), ((1, 1, 129, 2, 1, 128), False), ((1, 128, 257, 2, 2, 128), True), ((1, 641, 640, 4, 1, 128), False),
+                   ((2, 900, 1030, 4, 2, 128), True), ((1, 40, 400, 1, 1, 128), True)]
+
+
+@pytest.mark.parametrize("case", TILE_EDGE_CASES)
+def test_backward_tile_edges_against_float64(cuda, case):
+    """The reference's 16-bit tolerance (2e-2 of the value and of the largest), bit-identical from run to run."""
+    (b, sq, sk, n, nkv, h), causal = case
+    q, k, v = qkv(b, sq, sk, n, nkv, h)
+    do = bf16(np.random.default_rng(4).standard_normal(q.shape))
+    tq, tk, tv, tdo = (to_torch(a, cuda) for a in (q, k, v, do))
+    o, lse = attention_forward(tq, tk, tv, causal=causal)
+    got = attention_backward(tq, tk, tv, o, tdo, lse, causal=causal)
+    again = attention_backward(tq, tk, tv, o, tdo, lse, causal=causal)
+    device_status()
+    for a, a2, w in zip(got, again, attention_f64(q, k, v, causal, do)[2]):
+        close(to_numpy(a).astype(np.float32), w)
+        assert torch.equal(a, a2)
