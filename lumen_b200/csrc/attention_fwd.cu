@@ -3,19 +3,21 @@
 // (lumen/codegen/attention/cuda/ampere/forward.py:810-1157, lumen/codegen/attention/cuda/mod.rs:261-294) and of the
 // traced program it replaces (lumen/functional/attention/flash.py:30-49).
 //
-// One CTA per (128-query tile, head, batch), two CTAs per SM. Q, K, V are read in place from their [B, S, N, H] views
-// by TMA (4-d tensor maps, 128-byte swizzle). Per 128-key tile:
+// Two kernels with the same softmax: one 128-query tile per CTA and two CTAs per SM (attention_fwd_kernel: few or short
+// queries), and two tiles per CTA (attention_fwd_pair_kernel: enough of them to fill the GPU). Q, K, V are read in place
+// from their [B, S, N, H] views by TMA (4-d tensor maps, 128-byte swizzle). Per 128-key tile and query tile:
 //   S = Q K^T            tcgen05.mma, both operands K-major in shared memory, fp32 scores in tensor memory
 //   P = exp2(S*c - m)    four softmax warps, one query row per thread holding the whole row of 128 scores in registers
 //                        (one tensor-memory round trip per tile); P is rounded to bf16 and written back over S
 //                        (head dim 128) or into 64 columns of its own (head dim 64: S 128 + O 64 + P 64 = 256)
 //   O += P V             tcgen05.mma with P as the TMEM operand and V as an MN-major shared-memory operand; O stays
-//                        in tensor memory for the whole CTA
-// m is a reference maximum that is raised lazily (softmax_rows). At head dim 128 the tensor core, the softmax warps
-// and the TMA producer of ONE CTA work in turn (S and O are single-buffered: 256 columns) and the other CTA on the
-// SM fills the gaps. At head dim 64 S is free as soon as the softmax threads hold it in registers, so S(j + 1) is
-// computed during softmax(j) and only P(j) V(j) sits between two softmax passes. Probabilities are rounded to bf16 before the PV product as the traced program does (flash.py:38-45); sums
-// and the output accumulate in fp32. Every barrier wait is bounded.
+//                        in tensor memory for the whole tile
+// m is a reference maximum that is raised lazily (softmax_rows). At head dim 128 the tensor core and the softmax warps
+// of ONE query tile work in turn (S and O are single-buffered: 256 columns) and the other tile on the SM fills the gaps.
+// At head dim 64 S is free as soon as the softmax threads hold it in registers, so S(j + 1) is computed during
+// softmax(j) and only P(j) V(j) sits between two softmax passes. Probabilities are rounded to bf16 before the PV product
+// as the traced program does (flash.py:38-45); sums and the output accumulate in fp32. Every barrier wait is bounded.
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -49,6 +51,7 @@ struct FwdArgs {
     long long o_sb, o_ss, o_sn;
     float* lse;               // [B, N, Sq] or null
     int* status;
+    int tiles, heads_at_once;  // two-tile kernel: CTAs per (batch, head), (batch, head)s walked together
 };
 
 template <int D, int NS>
@@ -57,16 +60,17 @@ struct FwdSmem {
     static constexpr int kBytes = (1 + 2 * NS) * kTile + 1024 + 256;  // Q, NS stages of K and of V, alignment, barriers
 };
 
-// The softmax warpgroup of the one-warpgroup kernel (thread = query row). The output accumulates in tensor memory
+// The softmax warpgroup of one query tile (thread = query row), over the key tiles of one (query tile, head, batch). The output accumulates in tensor memory
 // (O += P V by the tensor core), so the thread's registers hold a whole row of scores: ONE tensor-memory round trip
 // per key tile instead of one per 32 columns and pass. Probabilities are taken against a reference maximum that is
 // only raised when the row's maximum outgrows it by more than 2^8 (then O and the running sum are rescaled, after
 // the previous tile's product has landed); a stale reference changes no result beyond rounding, since it cancels
 // in O / l and in the log-sum-exp.
-template <int D>
-__device__ __forceinline__ void softmax_rows(const FwdArgs& p, int n_kv, long long q_row, uint32_t lane_addr, uint32_t tmem_s,
-                                               uint32_t tmem_o, uint64_t* s_full, uint64_t* p_ready, uint64_t* pv_full,
-                                               volatile int* abort_flag, int head, int batch, uint32_t tmem_p, uint64_t* s_empty) {
+template <int D, bool HALVES>
+__device__ __forceinline__ bool softmax_rows(const FwdArgs& p, int n_kv, long long q_row, uint32_t lane_addr, uint32_t tmem_s,
+                                               uint32_t tmem_o, uint64_t* s_full, uint64_t* p_half, uint64_t* p_ready, uint64_t* pv_full,
+                                               volatile int* abort_flag, int head, int batch, uint32_t tmem_p, uint64_t* s_empty,
+                                               uint32_t done) {  // `done`: key tiles these barriers have seen before
     constexpr float kRaise = 8.0f;  // log2 of the largest probability tolerated before the reference is raised
     const uint32_t s_addr = tmem_s + lane_addr, o_addr = tmem_o + lane_addr, p_addr = tmem_p + lane_addr;
     const bool separate_p = tmem_p != tmem_s;  // P has columns of its own (head dim 64)
@@ -74,7 +78,7 @@ __device__ __forceinline__ void softmax_rows(const FwdArgs& p, int n_kv, long lo
     float m_ref = -INFINITY, l = 0.0f;
     bool ok = true;
     for (int j = 0; j < n_kv && ok; j++) {
-        if (!(ok = mbar_wait(s_full, (uint32_t)j & 1, abort_flag))) break;
+        if (!(ok = mbar_wait(s_full, (done + j) & 1, abort_flag))) break;
         __syncwarp();
         tc_fence_after();
         uint32_t x[BKV];
@@ -92,8 +96,28 @@ __device__ __forceinline__ void softmax_rows(const FwdArgs& p, int n_kv, long lo
             for (int i = 0; i < BKV; i++)
                 if (i > limit) x[i] = 0xff800000u;  // -inf: drops out of the maximum, exp2 gives 0
         }
-        // eight independent chains: with one or two warps per scheduler a single chain of 128 dependent maxima (or sums,
-        // below) would run at the instruction latency, not the issue rate
+        // probabilities of PART keys, rounded to bf16 in `packed` and summed in float32: two keys per instruction (packed
+        // float32 FMA / ADD of sm_100), four independent pairs of partial sums
+        constexpr int PART = HALVES ? BKV / 2 : BKV / 4;
+        float2 sums[4] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
+        uint32_t packed[PART / 2];
+        auto exponentials = [&](int first) {
+            const float m_use = m_ref == -INFINITY ? 0.0f : m_ref;
+            const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), shift2 = make_float2(-m_use, -m_use);
+#pragma unroll
+            for (int i = 0; i < PART; i += 2) {
+                const float2 arg = __ffma2_rn(make_float2(__uint_as_float(x[first + i]), __uint_as_float(x[first + i + 1])), scale2, shift2);
+                const float2 pr = make_float2(fast_exp2(arg.x), fast_exp2(arg.y));
+                __nv_bfloat162 h = __floats2bfloat162_rn(pr.x, pr.y);  // low half = the even key
+                packed[i / 2] = *(uint32_t*)&h;
+                sums[(i / 2) & 3] = __fadd2_rn(sums[(i / 2) & 3], pr);  // the normaliser sums the float32 probabilities
+            }
+        };
+        // HALVES: the first 64 probabilities are taken against the reference as it stands, while the maximum that may raise it
+        // is found - the two streams of instructions fill each other's gaps - and once more after a raise, which is rare.
+        if constexpr (HALVES) exponentials(0);
+        // eight independent chains: with one or two warps per scheduler a single chain of 128 dependent maxima (or sums)
+        // would run at the instruction latency, not the issue rate
         float mx[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) mx[i] = __uint_as_float(x[i]);
@@ -107,7 +131,7 @@ __device__ __forceinline__ void softmax_rows(const FwdArgs& p, int n_kv, long lo
             if (raise) m_ref = m_new, l *= alpha;
             if (j > 0) {
                 // O *= alpha, once the previous tile's product has landed (tensor-memory accesses are warp-wide)
-                if (!(ok = mbar_wait(pv_full, (uint32_t)(j - 1) & 1, abort_flag))) break;
+                if (!(ok = mbar_wait(pv_full, (done + j - 1) & 1, abort_flag))) break;
                 __syncwarp();
                 tc_fence_after();
 #pragma unroll
@@ -124,30 +148,32 @@ __device__ __forceinline__ void softmax_rows(const FwdArgs& p, int n_kv, long lo
                     tmem_st_32x16(o_addr + c * 32 + 16, v + 16);
                 }
             }
+            if constexpr (HALVES) {
+                sums[0] = sums[1] = sums[2] = sums[3] = make_float2(0.0f, 0.0f);
+                exponentials(0);
+            }
         }
-        const float m_use = m_ref == -INFINITY ? 0.0f : m_ref;
-        // two keys per instruction (packed float32 FMA / ADD of sm_100), four independent pairs of partial sums
-        float2 sums[4] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
-        const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), shift2 = make_float2(-m_use, -m_use);
         if (separate_p && j > 0) {
             // P(j) goes where P(j - 1) was: the product that read it has to have completed (it has, unless this row's
             // softmax overtook the tensor pipe)
-            if (!(ok = mbar_wait(pv_full, (uint32_t)(j - 1) & 1, abort_flag))) break;
+            if (!(ok = mbar_wait(pv_full, (done + j - 1) & 1, abort_flag))) break;
             __syncwarp();
             tc_fence_after();
         }
+        if constexpr (HALVES) {
+            // the product starts on the first 64 keys while the exponentials of the others are taken
+            tmem_st_32x32(p_addr, packed);
+            tmem_st_wait();
+            tc_fence_before();
+            mbar_arrive(p_half);
+            exponentials(PART);
+            tmem_st_32x32(p_addr + PART / 2, packed);
+        } else {
 #pragma unroll
-        for (int c = 0; c < BKV / 32; c++) {
-            uint32_t packed[16];
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-                const float2 arg = __ffma2_rn(make_float2(__uint_as_float(x[c * 32 + i]), __uint_as_float(x[c * 32 + i + 1])), scale2, shift2);
-                const float2 pr = make_float2(fast_exp2(arg.x), fast_exp2(arg.y));
-                __nv_bfloat162 h = __floats2bfloat162_rn(pr.x, pr.y);  // low half = the even key
-                packed[i / 2] = *(uint32_t*)&h;
-                sums[(i / 2) & 3] = __fadd2_rn(sums[(i / 2) & 3], pr);  // the normaliser sums the float32 probabilities
+            for (int c = 0; c < BKV / PART; c++) {
+                exponentials(c * PART);
+                tmem_st_32x16(p_addr + c * (PART / 2), packed);
             }
-            tmem_st_32x16(p_addr + c * 16, packed);
         }
         tmem_st_wait();
         tc_fence_before();
@@ -155,9 +181,9 @@ __device__ __forceinline__ void softmax_rows(const FwdArgs& p, int n_kv, long lo
         const float2 s01 = __fadd2_rn(sums[0], sums[1]), s23 = __fadd2_rn(sums[2], sums[3]);
         l += (s01.x + s01.y) + (s23.x + s23.y);
     }
-    if (n_kv > 0) ok = ok && mbar_wait(pv_full, (uint32_t)(n_kv - 1) & 1, abort_flag);
+    if (n_kv > 0) ok = ok && mbar_wait(pv_full, (done + n_kv - 1) & 1, abort_flag);
     ok = __all_sync(0xffffffffu, ok);
-    if (!ok) return;
+    if (!ok) return false;
     tc_fence_after();
     const bool live = q_row < p.Sq;
     const float inv = 1.0f / l;  // a row that sees no key is 0 / 0 in the traced program: NaN
@@ -195,6 +221,7 @@ __device__ __forceinline__ void softmax_rows(const FwdArgs& p, int n_kv, long lo
         }
     }
     if (live && p.lse) p.lse[((long long)batch * p.N + head) * p.Sq + q_row] = (m_ref + log2f(l)) * 0.6931471805599453f;
+    return true;
 }
 
 template <int D, int NS>
@@ -227,7 +254,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     uint32_t* tmem_slot = (uint32_t*)(bars + 13);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform for the compiler too
     const int q_tile = gridDim.x - 1 - blockIdx.x;  // longest (most keys under a causal mask) first
     const int head = blockIdx.y, batch = blockIdx.z;
     const int kv_head = head / (p.N / p.Nkv);
@@ -258,7 +285,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     // At head dim 64 the CTA's 256 columns hold S (128), O (64) and P (64) side by side: S is free as soon as the
     // softmax threads have loaded it, so S(j + 1) is computed during softmax(j) instead of behind P(j) V(j).
     // At head dim 128 P overwrites the first 64 columns of S.
@@ -287,48 +314,49 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && n_kv > 0) {
+        if (n_kv > 0) {  // the whole warp: the operands stay in uniform registers
+            const bool leader = elect_one();
             const uint32_t idesc_s = make_idesc(BQ, BKV, true, false, false);
             const uint32_t idesc_pv = make_idesc(BQ, D, true, false, true);
-            bool ok = mbar_wait(q_full, 0, abort_flag);
+            bool ok = mbar_wait_warp(q_full, 0, abort_flag);
             // Descriptors are built once and advanced by adds: the one issuing thread is otherwise bound by its own
             // integer instructions, not by the tensor pipe.
             const uint64_t dq0 = make_smem_desc(smem_u32(sq), 16, 1024), dk0 = make_smem_desc(smem_u32(sk), 16, 1024);
             const uint64_t dv0 = make_smem_desc(smem_u32(sv), kHalf, 1024);
             auto issue_s = [&](int j) -> bool {
                 const int st = kst(j);
-                if (!mbar_wait(&k_full[st], kph(j), abort_flag)) return false;
+                if (!mbar_wait_warp(&k_full[st], kph(j), abort_flag)) return false;
                 tc_fence_after();
                 const uint64_t kd = desc_advance(dk0, (uint32_t)(st * kTile));
 #pragma unroll
                 for (int k = 0; k < D / 16; k++) {
                     const uint32_t off = (uint32_t)((k / 4) * kHalf + (k % 4) * 32);
-                    mma_f16(tmem_s, desc_advance(dq0, off), desc_advance(kd, off), idesc_s, k != 0);
+                    mma_f16(tmem_s, desc_advance(dq0, off), desc_advance(kd, off), idesc_s, k != 0, leader);
                 }
-                mma_commit(&k_empty[st]);
-                mma_commit(s_full);
+                mma_commit(&k_empty[st], leader);
+                mma_commit(s_full, leader);
                 return true;
             };
             if (ok) ok = issue_s(0);
             for (int j = 0; j < n_kv && ok; j++) {
                 const int vs = kst(j);
                 if (kSeparateP && j + 1 < n_kv) {
-                    if (!(ok = mbar_wait(s_empty, (uint32_t)j & 1, abort_flag))) break;
+                    if (!(ok = mbar_wait_warp(s_empty, (uint32_t)j & 1, abort_flag))) break;
                     tc_fence_after();
                     if (!(ok = issue_s(j + 1))) break;
                 }
-                if (!(ok = mbar_wait(p_ready, (uint32_t)j & 1, abort_flag))) break;
-                if (!(ok = mbar_wait(&v_full[vs], kph(j), abort_flag))) break;
+                if (!(ok = mbar_wait_warp(p_ready, (uint32_t)j & 1, abort_flag))) break;
+                if (!(ok = mbar_wait_warp(&v_full[vs], kph(j), abort_flag))) break;
                 tc_fence_after();
                 const uint64_t vd = desc_advance(dv0, (uint32_t)(vs * kTile));
 #pragma unroll
                 for (int k = 0; k < BKV / 16; k++) {
                     // O += P V. P: 16 keys = 8 packed columns per step. V (MN-major): 16 key rows of 128 bytes = 2048 bytes
                     // per step, 64-wide head-dimension blocks kHalf apart.
-                    mma_f16_ts(tmem_o, tmem_p + k * 8, desc_advance(vd, k * 2048), idesc_pv, (j | k) != 0);
+                    mma_f16_ts(tmem_o, tmem_p + k * 8, desc_advance(vd, k * 2048), idesc_pv, (j | k) != 0, leader);
                 }
-                mma_commit(&v_empty[vs]);
-                mma_commit(pv_full);
+                mma_commit(&v_empty[vs], leader);
+                mma_commit(pv_full, leader);
                 if (!kSeparateP && j + 1 < n_kv) ok = issue_s(j + 1);  // behind PV(j), which reads P from the S buffer: the tensor pipe runs in order
             }
         }
@@ -337,7 +365,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         const int quarter = warp & 3;
         const long long q_row = (long long)q0 + quarter * 32 + lane;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-        softmax_rows<D>(p, n_kv, q_row, lane_addr, tmem_s, tmem_o, s_full, p_ready, pv_full, abort_flag, head, batch, tmem_p, s_empty);
+        softmax_rows<D, false>(p, n_kv, q_row, lane_addr, tmem_s, tmem_o, s_full, nullptr, p_ready, pv_full, abort_flag, head, batch, tmem_p, s_empty, 0);
     }
 
     tc_fence_before();
@@ -354,6 +382,286 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         tc_fence_after();
         tmem_dealloc(tmem_base, kTmemCols);
     }
+}
+
+// ---- two query tiles per CTA ------------------------------------------------------------------------------------
+// What bounds it: the softmax chain of a tile (about 2000 cycles) against the tensor pipe's 1024 per tile. Two CTAs of the
+// one-tile kernel fall into step - both in their softmax, then both waiting for products that the tensor pipe interleaves;
+// here one warp issues the products of both tiles in turn, so that one tile's run under the other's softmax, K and V cross
+// shared memory once for both, and the CTA stays: it takes over the work of CTAs that have not been launched
+// (clusterlaunchcontrol), so that the next item's Q, K and first scores are under way while the softmax warps write out O.
+// Batch 8, 32 heads, sequence 4096, head dim 128, causal: 1340 -> 1040 us (1060 TFLOP/s), of which 160 us came from issuing
+// the products warp-wide.
+template <int D>
+struct FwdPairSmem {
+    static constexpr int kTile = BKV * D * 2;
+    static constexpr int NS = D == 128 ? 2 : 4;  // stages of K and of V
+    static constexpr int kBytes = (2 + 2 * NS) * kTile + 1024 + 512;
+};
+// warp 0: TMA and the next work item, warp 1: MMA (warps 2, 3 idle: register budgets are set per aligned group of four
+// warps), warps 4..7 / 8..11: softmax of query tile 0 / 1, whose threads hold a row of 128 scores each
+constexpr int kPairThreads = 128 + 256;
+constexpr int kPairLaunchRegs = 168;  // what the compiler assigns under __launch_bounds__(384, 1); checked before a launch
+constexpr int kPairRegsLight = 72, kPairRegsSoftmax = 216;
+static_assert(128 * kPairRegsLight + 256 * kPairRegsSoftmax <= kPairLaunchRegs * kPairThreads, "register budgets exceed the launch allocation");
+
+struct FwdWork {
+    int q0, head, batch, n[2], n_max;  // n[t]: key tiles that query tile t sees
+};
+// CTA `id` of the grid: (batch, head)s in groups whose keys and values fit the L2 together; within a group the longest
+// tiles (most keys under a causal mask) of all heads come first, so that the last CTAs to run are short ones.
+__device__ __forceinline__ FwdWork fwd_work(const FwdArgs& p, int id) {
+    FwdWork w;
+    const int per_group = p.tiles * p.heads_at_once, first_bn = id / per_group * p.heads_at_once;
+    const int rest = id % per_group, heads = min(p.heads_at_once, p.B * p.N - first_bn);
+    const int bn = first_bn + rest % heads;
+    w.q0 = (p.tiles - 1 - rest / heads) * 2 * BQ;
+    w.batch = bn / p.N, w.head = bn % p.N;
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+        const int first = w.q0 + t * BQ;
+        const long long last_key = p.causal ? min((long long)p.Sk - 1, (long long)first + BQ - 1 + p.causal_offset) : (long long)p.Sk - 1;
+        w.n[t] = first >= p.Sq || last_key < 0 ? 0 : (int)(last_key / BKV) + 1;
+    }
+    w.n_max = max(w.n[0], w.n[1]);
+    return w;
+}
+
+template <int D>
+__global__ void __launch_bounds__(kPairThreads, 1)
+attention_fwd_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                          const __grid_constant__ CUtensorMap map_v, const FwdArgs p) {
+    constexpr int kTile = FwdPairSmem<D>::kTile, NS = FwdPairSmem<D>::NS;
+    constexpr int kHalf = 128 * 128, DB = D / 64;
+    constexpr bool kSeparateP = D == 64;  // S 2 x 128, O 2 x 64, P 2 x 64; at head dim 128 P overwrites S
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* sq = smem;                     // two tiles
+    uint8_t* sk = smem + 2 * kTile;         // NS stages
+    uint8_t* sv = sk + NS * kTile;          // NS stages
+    uint64_t* bars = (uint64_t*)(sv + NS * kTile);
+    uint64_t* q_full = bars;                // 1
+    uint64_t* q_empty = bars + 1;           // 1: every score product of the item has completed
+    uint64_t* k_full = bars + 2;            // NS
+    uint64_t* k_empty = k_full + NS;        // NS
+    uint64_t* v_full = k_empty + NS;        // NS
+    uint64_t* v_empty = v_full + NS;        // NS
+    uint64_t* s_full = v_empty + NS;        // 2, one per query tile, as the next four
+    uint64_t* s_empty = s_full + 2;         // 2
+    uint64_t* p_half = s_empty + 2;         // 2: the first 64 keys of P are in tensor memory
+    uint64_t* p_ready = p_half + 2;         // 2: all of P is
+    uint64_t* pv_full = p_ready + 2;        // 2
+    uint64_t* next_full = pv_full + 2;      // 2
+    uint64_t* next_empty = next_full + 2;   // 2: one arrival of the MMA warp, one of each softmax warp
+    uint8_t* next_slot = (uint8_t*)(((uintptr_t)(next_empty + 2) + 15) & ~(uintptr_t)15);  // 2 x 16 bytes
+    uint32_t* tmem_slot = (uint32_t*)(next_slot + 32);
+    volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    static_assert((2 + 4 * NS + 14) * 8 + 16 + 32 + 8 <= 512, "barrier space");
+
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform for the compiler too
+    const int group = p.N / p.Nkv;
+    if (threadIdx.x == 0) {
+        mbar_init(q_full, 1);
+        mbar_init(q_empty, 1);
+        for (int s = 0; s < NS; s++) {
+            mbar_init(&k_full[s], 1);
+            mbar_init(&k_empty[s], 1);
+            mbar_init(&v_full[s], 1);
+            mbar_init(&v_empty[s], 1);
+        }
+        for (int t = 0; t < 2; t++) {
+            mbar_init(&s_full[t], 1);
+            mbar_init(&s_empty[t], 128);
+            mbar_init(&p_half[t], 128);
+            mbar_init(&p_ready[t], 128);
+            mbar_init(&pv_full[t], 1);
+            mbar_init(&next_full[t], 1);
+            mbar_init(&next_empty[t], 9);
+        }
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 256;  // S(t) at + 128 t, O(t) at + D t
+    const uint32_t tmem_p = kSeparateP ? tmem_base + 256 + 2 * D : tmem_s;
+    constexpr uint32_t kPStep = kSeparateP ? 64 : 128;
+
+    FwdWork w = fwd_work(p, blockIdx.x);
+    int next;
+    // each register budget is set inside the branch it governs: code after a join is compiled for the smallest one
+    if (warp < 4) {
+      regs_dec<kPairRegsLight>();
+      if (warp == 0) {
+        if (lane == 0) {
+            tma_prefetch_desc(&map_q);
+            tma_prefetch_desc(&map_k);
+            tma_prefetch_desc(&map_v);
+            bool ok = true;
+            uint32_t kv = 0, loads = 0;  // key tiles and query tile pairs fetched so far
+            for (uint32_t item = 0; ok; item++) {
+                const int slot = item & 1;
+                if (item >= 2 && !(ok = mbar_wait(&next_empty[slot], ((item >> 1) - 1) & 1, abort_flag))) break;
+                mbar_expect_tx(&next_full[slot], 16);
+                next_cta_request(next_slot + slot * 16, &next_full[slot]);
+                if (w.n_max > 0) {
+                    const int kv_head = w.head / group, live = w.q0 + BQ < p.Sq ? 2 : 1;
+                    if (loads > 0) ok = mbar_wait(q_empty, (loads - 1) & 1, abort_flag);
+                    if (ok) {
+                        loads++;
+                        mbar_expect_tx(q_full, live * kTile);
+                        for (int t = 0; t < live; t++)
+                            for (int d = 0; d < DB; d++) tma_load_4d(sq + t * kTile + d * kHalf, &map_q, q_full, d * 64, w.head, w.q0 + t * BQ, w.batch);
+                    }
+                    for (int j = 0; j < w.n_max && ok; j++, kv++) {
+                        const uint32_t st = kv % NS, ph = (kv / NS) & 1;
+                        if (!(ok = mbar_wait(&k_empty[st], ph ^ 1, abort_flag))) break;
+                        mbar_expect_tx(&k_full[st], kTile);
+                        for (int d = 0; d < DB; d++) tma_load_4d(sk + st * kTile + d * kHalf, &map_k, &k_full[st], d * 64, kv_head, j * BKV, w.batch);
+                        if (!(ok = mbar_wait(&v_empty[st], ph ^ 1, abort_flag))) break;
+                        mbar_expect_tx(&v_full[st], kTile);
+                        for (int d = 0; d < DB; d++) tma_load_4d(sv + st * kTile + d * kHalf, &map_v, &v_full[st], d * 64, kv_head, j * BKV, w.batch);
+                    }
+                }
+                if (!mbar_wait(&next_full[slot], (item >> 1) & 1, abort_flag) || !ok) break;  // the answer is never in flight at the exit
+                if (!next_cta_answer(next_slot + slot * 16, next)) break;
+                w = fwd_work(p, next);
+            }
+        }
+      } else if (warp == 1) {
+        {  // the whole warp: the operands stay in uniform registers
+            const bool leader = elect_one();
+            const uint32_t idesc_s = make_idesc(BQ, BKV, true, false, false);
+            const uint32_t idesc_pv = make_idesc(BQ, D, true, false, true);
+            const uint64_t dq0 = make_smem_desc(smem_u32(sq), 16, 1024), dk0 = make_smem_desc(smem_u32(sk), 16, 1024);
+            const uint64_t dv0 = make_smem_desc(smem_u32(sv), kHalf, 1024);
+            bool ok = true;
+            uint32_t kv = 0, loads = 0, done[2] = {0, 0};  // done[t]: key tiles of earlier items
+            // S(t) of key tile number `tile`, the `nth` of query tile buffer t
+            auto issue_s = [&](int t, uint32_t tile, uint32_t nth) -> bool {
+                const uint32_t st = tile % NS;
+                if (!mbar_wait_warp(&k_full[st], (tile / NS) & 1, abort_flag)) return false;
+                if (kSeparateP && nth > 0 && !mbar_wait_warp(&s_empty[t], (nth - 1) & 1, abort_flag)) return false;
+                tc_fence_after();
+                const uint64_t qd = desc_advance(dq0, (uint32_t)(t * kTile)), kd = desc_advance(dk0, st * kTile);
+#pragma unroll
+                for (int k = 0; k < D / 16; k++) {
+                    const uint32_t off = (uint32_t)((k / 4) * kHalf + (k % 4) * 32);
+                    mma_f16(tmem_s + t * 128, desc_advance(qd, off), desc_advance(kd, off), idesc_s, k != 0, leader);
+                }
+                mma_commit(&s_full[t], leader);
+                return true;
+            };
+            auto issue_pv = [&](int t, uint32_t tile, uint32_t nth, bool first) -> bool {
+                const uint32_t st = tile % NS;
+                if (!mbar_wait_warp(&v_full[st], (tile / NS) & 1, abort_flag)) return false;
+                const uint64_t vd = desc_advance(dv0, st * kTile);
+#pragma unroll
+                for (int k = 0; k < BKV / 16; k++) {
+                    if (k % (BKV / 32) == 0) {
+                        if (!mbar_wait_warp(k == 0 ? &p_half[t] : &p_ready[t], nth & 1, abort_flag)) return false;
+                        tc_fence_after();
+                    }
+                    mma_f16_ts(tmem_o + t * D, tmem_p + t * kPStep + k * 8, desc_advance(vd, k * 2048), idesc_pv, !first || k != 0, leader);
+                }
+                mma_commit(&pv_full[t], leader);
+                return true;
+            };
+            for (uint32_t item = 0; ok; item++) {
+                if (w.n_max > 0) {
+                    if (!(ok = mbar_wait_warp(q_full, loads & 1, abort_flag))) break;
+                    loads++;
+                    for (int j = -1; j < w.n_max && ok; j++) {
+                        if (!kSeparateP) {  // the next scores behind the product that reads P from their columns: the tensor pipe runs in order
+#pragma unroll
+                            for (int t = 0; t < 2; t++) {
+                                if (ok && j >= 0 && j < w.n[t]) ok = issue_pv(t, kv + j, done[t] + j, j == 0);
+                                if (ok && j + 1 < w.n[t]) ok = issue_s(t, kv + j + 1, done[t] + j + 1);
+                            }
+                        } else {
+#pragma unroll
+                            for (int t = 0; t < 2; t++)
+                                if (ok && j + 1 < w.n[t]) ok = issue_s(t, kv + j + 1, done[t] + j + 1);
+#pragma unroll
+                            for (int t = 0; t < 2; t++)
+                                if (ok && j >= 0 && j < w.n[t]) ok = issue_pv(t, kv + j, done[t] + j, j == 0);
+                        }
+                        if (!ok) break;
+                        if (j + 1 < w.n_max) mma_commit(&k_empty[(kv + j + 1) % NS], leader);
+                        if (j + 2 == w.n_max) mma_commit(q_empty, leader);
+                        if (j >= 0) mma_commit(&v_empty[(kv + j) % NS], leader);
+                    }
+                    kv += w.n_max, done[0] += w.n[0], done[1] += w.n[1];
+                }
+                const int slot = item & 1;
+                if (!ok || !(ok = mbar_wait_warp(&next_full[slot], (item >> 1) & 1, abort_flag))) break;
+                const bool more = next_cta_answer(next_slot + slot * 16, next);
+                fence_proxy_async();  // the slot is read before the next answer is written there
+                __syncwarp();
+                if (leader) mbar_arrive(&next_empty[slot]);
+                if (!__all_sync(0xffffffffu, more)) break;
+                w = fwd_work(p, __reduce_max_sync(0xffffffffu, next));  // uniform
+            }
+        }
+      }
+    } else {
+        regs_inc<kPairRegsSoftmax>();
+        const int t = (warp - 4) >> 2, quarter = warp & 3;
+        const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+        uint32_t done = 0;
+        for (uint32_t item = 0;; item++) {
+            const long long q_row = (long long)w.q0 + t * BQ + quarter * 32 + lane;
+            const int n = t ? w.n[1] : w.n[0];
+            if (!softmax_rows<D, true>(p, n, q_row, lane_addr, tmem_s + t * 128, tmem_o + t * D, &s_full[t], &p_half[t], &p_ready[t], &pv_full[t],
+                                       abort_flag, w.head, w.batch, tmem_p + t * kPStep, &s_empty[t], done))
+                break;
+            done += n;
+            const int slot = item & 1;
+            if (!mbar_wait_warp(&next_full[slot], (item >> 1) & 1, abort_flag)) break;
+            const bool more = next_cta_answer(next_slot + slot * 16, next);
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&next_empty[slot]);
+            if (!more) break;
+            w = fwd_work(p, next);
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (*abort_flag) {
+        if (threadIdx.x == 0) atomicExch(p.status, LB_ERR_TIMEOUT);
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000) {
+        }
+        __syncthreads();
+    }
+    if (warp == 1) {
+        __syncwarp();
+        tc_fence_after();
+        tmem_dealloc(tmem_base, 512);
+    }
+}
+
+template <int D>
+void launch_fwd_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, FwdArgs p, cudaStream_t s) {
+    constexpr int kBytes = FwdPairSmem<D>::kBytes;
+    static const int regs = launch_regs((const void*)attention_fwd_pair_kernel<D>);
+    if (regs != kPairLaunchRegs)
+        fail(LB_ERR_UNSUPPORTED, format("attention: the two-tile forward kernel was built with %d registers per thread, its register budgets "
+                                        "assume %d", regs, kPairLaunchRegs));
+    if (first_use_on_device((const void*)attention_fwd_pair_kernel<D>))
+        LB_CUDA(cudaFuncSetAttribute(attention_fwd_pair_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes));
+    p.tiles = (p.Sq + 2 * BQ - 1) / (2 * BQ);
+    const long long heads = (long long)p.B * p.N, bytes_per_head = std::max(1LL, (long long)p.Sk * D * 4 * p.Nkv / p.N);
+    p.heads_at_once = (int)std::min(heads, std::max(1LL, (48LL << 20) / bytes_per_head));
+    attention_fwd_pair_kernel<D><<<(unsigned)(heads * p.tiles), kPairThreads, kBytes, s>>>(mq, mk, mv, p);
 }
 
 // 4-d tensor map over a [B, S, N, H] view: dims innermost first {H, N, S, B}; box = 64 head-dim elements x `box_rows` rows.
@@ -417,6 +725,18 @@ void attention_fwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor
     p.status = status_word();
     dim3 grid((unsigned)((Sq + BQ - 1) / BQ), (unsigned)N, (unsigned)B);
     cudaStream_t s = (cudaStream_t)stream;
+    // Which kernel (measured, us, one tile per CTA -> two): the second has half the CTAs, so it needs enough of them to fill
+    // the GPU - 4 heads x 4096 at head dim 128: 62 -> 64, 2 x 8 x 1024: 21 -> 23, 32 heads x 4096: 180 -> 130 - and a query
+    // length that gives the second tile rows (8 x 32 x 100 against 4000: 93 -> 115). From two CTAs per SM of the first
+    // kernel on it is ahead at head dim 128 (4 x 16 x 1000: 47 -> 45); at head dim 64, where the one-tile kernel overlaps S
+    // with the softmax as well, from four (4 x 16 x 1000: 40 -> 41, 2 x 32 x 1531: 55 -> 49, 32 x 4096: 144 -> 118).
+    const long long tiles = (Sq + BQ - 1) / BQ * N * B;
+    if (Sq > BQ && tiles > (D == 128 ? 2LL : 4LL) * sm_count_hint()) {
+        if (D == 128) launch_fwd_pair<128>(mq, mk, mv, p, s);
+        else launch_fwd_pair<64>(mq, mk, mv, p, s);
+        LB_CUDA(cudaGetLastError());
+        return;
+    }
     // One warpgroup, O in tensor memory, two CTAs per SM: two K/V stages at head dim 64, one at head dim 128 (96 KB per CTA)
     if (D == 128) {
         if (first_use_on_device((const void*)attention_fwd_kernel<128, 1>))

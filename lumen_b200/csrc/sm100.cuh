@@ -86,6 +86,30 @@ __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
 
+// ---- dynamic work: a running CTA takes over the work of one that has not been launched ----------------------------
+// Asks for the next CTA of this grid; the 16-byte answer lands at `slot` and counts on `bar` (expect 16 bytes first).
+// Not to be asked again once an answer said that none was left.
+__device__ __forceinline__ void next_cta_request(void* slot, uint64_t* bar) {
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                 ::"r"(smem_u32(slot)), "r"(smem_u32(bar))
+                 : "memory");
+}
+// The answer: false when every CTA of the grid has been launched, else the (x) index of the one taken over.
+__device__ __forceinline__ bool next_cta_answer(const void* slot, int& x) {
+    uint32_t got, cx = 0, cy = 0, cz = 0;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
+        "ld.shared.b128 h, [%4];\n\t"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+        "selp.u32 %3, 1, 0, p;\n\t"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%0, %1, %2, _}, h;\n\t}"
+        : "+r"(cx), "+r"(cy), "+r"(cz), "=r"(got)
+        : "r"(smem_u32(slot))
+        : "memory");
+    x = (int)cx;
+    return got != 0;
+}
+
 // ---- registers ----
 // Register budget of the calling warpgroup (all four of its warps execute this). An increase draws on what the block was
 // launched with and waits until it is there: the warpgroups' budgets may not add up to more.

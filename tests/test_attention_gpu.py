@@ -349,3 +349,41 @@ def test_backward_tile_edges_against_float64(cuda, case):
     for a, a2, w in zip(got, again, attention_f64(q, k, v, causal, do)[2]):
         close(to_numpy(a).astype(np.float32), w)
         assert torch.equal(a, a2)
+
+
+# (B, Sq, Sk, N, Nkv, H): enough query tiles for the two-tile forward kernel (more than two per SM at head dim 128, four at
+# 64) - a second tile of one row, a last CTA with one tile, a key tail, more keys than queries, CTAs that go on to further
+# work with more and with fewer key tiles
+PAIR_CASES = [((20, 129, 129, 16, 4, 128), True), ((10, 257, 257, 16, 16, 128), False), ((2, 300, 777, 64, 8, 128), True), ((1, 1024, 1024, 40, 8, 128), True),
+              ((20, 129, 129, 32, 4, 64), True), ((10, 257, 257, 32, 16, 64), False), ((4, 300, 500, 64, 8, 64), True), ((2, 1100, 1100, 40, 8, 64), True)]
+
+
+@pytest.mark.parametrize("case", PAIR_CASES)
+def test_two_tile_forward_against_float64(cuda, case):
+    """The reference's 16-bit tolerance (2e-2), log-sum-exp to 1e-3. Later keys have larger scores, so that the reference
+    maximum is raised on the way (a factor of 2^8 between raises), and the result repeats bit for bit."""
+    (b, sq, sk, n, nkv, h), causal = case
+    q, k, v = qkv(b, sq, sk, n, nkv, h)
+    k = bf16(k.astype(np.float32) * np.linspace(0.1, 6.0, sk, dtype=np.float32)[None, :, None, None])
+    tq, tk, tv = (to_torch(a, cuda) for a in (q, k, v))
+    o, lse = attention_forward(tq, tk, tv, causal=causal)
+    again, _ = attention_forward(tq, tk, tv, causal=causal)
+    device_status()
+    want, want_lse = attention_f64(q, k, v, causal)
+    close(to_numpy(o).astype(np.float32), want)
+    np.testing.assert_allclose(to_numpy(lse), want_lse, rtol=1e-3, atol=1e-3)
+    assert torch.equal(o, again)
+
+
+@pytest.mark.parametrize("n", [2, 40])
+def test_forward_rows_that_see_no_key_and_rows_of_nan(cuda, n):
+    """One and two query tiles per CTA: a causal mask aligned to the last of fewer keys leaves the first rows none (0 / 0 in
+    the traced program); a NaN key makes the rows that see it NaN and no other."""
+    q, k, v = (to_torch(a, cuda) for a in qkv(4, 300, 200, n, n, 128))
+    o, lse = attention_forward(q, k, v, causal=True)
+    device_status()
+    assert torch.isnan(o[:, :100]).all() and not torch.isnan(o[:, 100:]).any() and not torch.isnan(lse[..., 100:]).any()
+    k[:, 150] = float("nan")
+    o, _ = attention_forward(q, k, v, causal=True)
+    device_status()
+    assert torch.isnan(o[:, 250:]).all() and not torch.isnan(o[:, 100:250]).any()
