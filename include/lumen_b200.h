@@ -127,6 +127,9 @@ typedef struct {
 } lb_gemm_cfg;
 /* Scratch bytes that let lb_gemm split K for this problem (0 when it would not split). */
 size_t lb_gemm_scratch_bytes(int64_t m, int64_t n, int64_t k, int64_t batch);
+/* The same for a product step of a plan, which runs on the kernel lb_gemm picks by itself: 0 also where that one cuts K inside
+ * a thread-block cluster. */
+size_t lb_gemm_step_scratch_bytes(int64_t m, int64_t n, int64_t k);
 int lb_gemm(const lb_tensor* a, const lb_tensor* b, const lb_gemm_out* out, const lb_gemm_cfg* cfg /* nullable */,
             void* stream);
 

@@ -100,6 +100,8 @@ def lib():
         ]  # fmt: skip
         _lib.lb_gemm_scratch_bytes.argtypes = [ctypes.c_int64] * 4
         _lib.lb_gemm_scratch_bytes.restype = ctypes.c_size_t
+        _lib.lb_gemm_step_scratch_bytes.argtypes = [ctypes.c_int64] * 3
+        _lib.lb_gemm_step_scratch_bytes.restype = ctypes.c_size_t
         T = ctypes.POINTER(LbTensor)
         _lib.lb_attention_fwd.argtypes = [ctypes.POINTER(LbAttnDesc), T, T, T, T, T, ctypes.c_void_p]
         _lib.lb_attention_bwd.argtypes = [ctypes.POINTER(LbAttnDesc)] + [T] * 10 + [ctypes.c_void_p]

@@ -852,10 +852,10 @@ def attention_params(body: G.Graph):
 
 
 def gemm_scratch_bytes(m: int, n: int, k: int) -> int:
-    """Split-K scratch the backend wants for an [m, k] x [k, n] product (0 when it does not split)."""
+    """Split-K scratch a plan's [m, k] x [k, n] product step takes (0 when it does not split, or splits inside a cluster)."""
     from lumen_b200 import _lib
 
-    return _lib.lib().lb_gemm_scratch_bytes(m, n, k, 1)
+    return _lib.lib().lb_gemm_step_scratch_bytes(m, n, k)
 
 
 _SCRATCH_CACHE: dict[str, int] = {}

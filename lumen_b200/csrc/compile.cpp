@@ -20,7 +20,7 @@
 #include "fused.h"
 #include "graph_text.h"
 
-extern "C" size_t lb_gemm_scratch_bytes(int64_t m, int64_t n, int64_t k, int64_t batch);
+extern "C" size_t lb_gemm_step_scratch_bytes(int64_t m, int64_t n, int64_t k);
 
 namespace lb {
 namespace {
@@ -657,7 +657,7 @@ struct Lowering {
         }
         View d = fresh(t.dtype, t.shape, result);
         views[result] = d;
-        const size_t sb = lb_gemm_scratch_bytes(a.shape[0], b.shape[1], a.shape[1], 1);
+        const size_t sb = lb_gemm_step_scratch_bytes(a.shape[0], b.shape[1], a.shape[1]);
         std::ostringstream s;
         s << "s gemm " << label << " " << tid(a) << " " << tid(b) << " " << tid(d) << " " << epilogue << " " << (sb ? tid(scratch(sb)) : -1) << " " << (aux ? tid(*aux) : -1);
         push_step(s.str() + "\n");

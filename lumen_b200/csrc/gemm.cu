@@ -688,6 +688,7 @@ CUtensorMap make_map(const View3& v, bool contiguous_is_cols, int box_inner, int
 // picks it: waves of (tile, range) units times the k-blocks of a range, at the measured 4 x 171 cycles per k-block of
 // a 128 x 256 tile, plus the float32 partial tiles written by the GEMM and re-read by the reduction kernel at HBM
 // speed and that kernel's launch. A split has to win by a tenth to be taken; each range keeps at least 16 k-blocks.
+size_t gemm_scratch_bytes(long long M, long long N, long long K, long long batch);
 int gemm_splits(long long M, long long N, long long K, long long batch, int sms) {
     const long long tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * batch, total_kb = (K + BK - 1) / BK;
     if (tiles >= 4LL * sms || total_kb < 32) return 1;
@@ -703,6 +704,26 @@ int gemm_splits(long long M, long long N, long long K, long long batch, int sms)
     for (int s = 2; s <= 32 && total_kb / s >= 16; s++)
         if (cost(s) < best_us) best = s, best_us = cost(s);
     return best;
+}
+
+// K ranges (CTAs of a cluster) with which a product runs on the 128 x 64 tiles of gemm_small.cu, 0 where 256 x 256 tiles are
+// better. The line is one CTA per SM: with no more tiles than SMs, ranges are doubled while they still have an SM each and
+// two 64-wide blocks of K, and once more, two CTAs to an SM, where a range would be longer than 64 blocks. Measured (us, large
+// tiles -> these), bfloat16: 64^3 8.2 -> 6.2, 512^3 13.5 -> 8.5, 200 x 4096 K 1024 16.4 -> 11.5, 200 x 1024 K 4096 24.6 -> 12.3
+// (4 ranges), 1000^3 18.5 -> 12.3, 128 x 8192 K 8192 49 -> 35, 1024 x 1024 K 8192 35 -> 28 (39 with one range); beyond the line
+// 4096 x 1024 K 200 12.3 -> 16.4, 700 x 4096 K 1024 16.4 -> 20.5, 2048^3 22.6 -> 32.7.
+int gemm_small_splits(long long M, long long N, long long K, long long batch, int sms) {
+    const long long tiles = (M + 127) / 128 * ((N + 63) / 64) * batch, total_kb = (K + BK - 1) / BK;
+    if (tiles > sms) return 0;
+    int s = 1;
+    while (s < 8 && tiles * 2 * s <= sms && total_kb >= 4 * s) s *= 2;
+    if (s < 8 && total_kb > 64 * s && tiles * s <= sms) s *= 2;
+    return total_kb <= 128 * s ? s : 0;  // longer ranges: not measured, left to the split-K kernels
+}
+
+// Scratch a plan's product step takes: none where the narrow tiles run.
+extern "C" size_t lb_gemm_step_scratch_bytes(int64_t m, int64_t n, int64_t k) {
+    return gemm_small_splits(m, n, k, 1, sm_count_hint()) ? 0 : gemm_scratch_bytes(m, n, k, 1);
 }
 
 // CTA pairs of gemm_tcgen05_pair that can be resident on `dev` at once (asked of the runtime once per device).
@@ -800,6 +821,16 @@ void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
         bt.rows = b.cols, bt.cols = b.rows, bt.sr = b.sc, bt.sc = b.sr;
         CUtensorMap map_b = p.b_mn_major ? make_map(bt, false, 64, BK) : make_map(bt, true, BK, pairs ? BN / 2 : BN);
         const DeviceInfo& dev = device_info();
+        // no kernel asked for and no split or raster tuned: narrow tiles where they fit (gemm_small_splits)
+        if (const int ranges = kernel_choice == 0 && !(tuning && (tuning->splits > 0 || tuning->group_m > 0)) ? gemm_small_splits(M, N, K, batch, dev.sms) : 0) {
+            SmallGemmArgs q{};
+            q.M = p.M, q.N = p.N, q.K = p.K, q.a_mn_major = p.a_mn_major, q.b_mn_major = p.b_mn_major, q.in_bf16 = p.in_bf16;
+            q.d = p.d, q.d_bf16 = p.d_bf16, q.d_f16 = p.d_f16, q.ldd = p.ldd, q.d_batch_stride = p.d_batch_stride;
+            q.epilogue = p.epilogue, q.aux = p.aux, q.ld_aux = p.ld_aux, q.aux_batch_stride = p.aux_batch_stride, q.status = p.status;
+            q.splits = ranges;
+            gemm_small(map_a, p.b_mn_major ? map_b : make_map(bt, true, BK, 64), q, (int)batch, dev.sms, s);
+            return;
+        }
         if (first_use_on_device((const void*)gemm_tcgen05_pair)) {
             LB_CUDA(cudaFuncSetAttribute(gemm_tcgen05, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
             LB_CUDA(cudaFuncSetAttribute(gemm_tcgen05_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes));

@@ -1,5 +1,7 @@
-// What the tensor-core and the CUDA-core GEMM share.
+// What the GEMM kernels' files share.
 #pragma once
+#include <cuda.h>
+
 #include "device.h"
 
 namespace lb {
@@ -21,5 +23,23 @@ struct SimtArgs {
 };
 
 void gemm_simt(const void* a, const void* b, int dtype, const SimtArgs& p, int sms, cudaStream_t s);
+
+// 128 x 64 tiles with the K range of a tile over a cluster (gemm_small.cu): 16-bit operands, maps with boxes of 64
+// elements along the contiguous axis by 128 rows of A, 64 of B (K-major) or 64 (M- / N-major).
+struct SmallGemmArgs {
+    int M, N, K;
+    int a_mn_major, b_mn_major, in_bf16;
+    void* d;
+    int d_bf16, d_f16;  // else float32
+    long long ldd, d_batch_stride;
+    int epilogue;
+    const void* aux;
+    long long ld_aux, aux_batch_stride;
+    int splits;  // CTAs of a cluster: 1, 2, 4 or 8, no more than the 64-wide blocks of K
+    int* status;
+    int tiles_m, tiles_n, vec;  // set by gemm_small
+};
+
+void gemm_small(const CUtensorMap& map_a, const CUtensorMap& map_b, SmallGemmArgs p, int batch, int sms, cudaStream_t s);
 
 }  // namespace lb

@@ -1,0 +1,224 @@
+// 16-bit matrix products too small for 256 x 256 tiles to fill the GPU: 128 x 64 tiles, the K range of a tile cut over a
+// thread-block cluster of up to eight CTAs.
+//
+// What bounds it: the latency of one pass - first TMA load, the ring, the accumulator's way out - and how many SMs pull
+// operands meanwhile. A product of 200 x 4096 with K = 1024 has 16 tiles of 256 x 256 (32 of 148 SMs), one of 200 x 1024
+// with K = 4096 four. Narrow tiles and split K ranges give every SM work; the partial sums of a tile meet in distributed
+// shared memory, added in rank order (no scratch memory, no second kernel, the same bits every run), each CTA of the
+// cluster writing its share of the rows in whole 128-byte lines.
+#include <cuda_fp16.h>
+
+#include "gemm.h"
+#include "sm100.cuh"
+
+namespace lb {
+namespace {
+
+using namespace sm100;
+
+constexpr int BM = 128, BN = 64, BK = 64;
+constexpr int kThreads = 192;  // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2..5: accumulator rows; all: sums and stores
+constexpr int kStageA = BM * BK * 2, kStageB = BN * BK * 2;
+// A load takes about a microsecond to arrive, a stage's products 0.15: eight stages where an SM has one CTA, four where two
+constexpr int smem_bytes(int stages) { return stages * (kStageA + kStageB) + 1024 /*alignment*/ + 256 /*barriers*/; }
+static_assert(BM * BN * 4 <= 4 * (kStageA + kStageB), "the partial tile takes the drained ring's place");
+
+__device__ __forceinline__ float4 load_cluster(uint32_t addr, uint32_t rank) {
+    float4 v;
+    asm volatile(
+        "{\n\t.reg .b32 ra;\n\t"
+        "mapa.shared::cluster.u32 ra, %4, %5;\n\t"
+        "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n\t}"
+        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+        : "r"(addr), "r"(rank)
+        : "memory");
+    return v;
+}
+// byte offset of 16-byte chunk `c` of row `r` of the partial tile: eight rows' equal chunks fall in different banks
+__device__ __forceinline__ uint32_t chunk_at(int r, int c) { return (uint32_t)(r * BN * 4 + ((c ^ (r & 7)) << 4)); }
+
+template <int STAGES>
+__global__ void __launch_bounds__(kThreads, 8 / STAGES)
+gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const SmallGemmArgs p) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t *sa = smem, *sb = smem + STAGES * kStageA;
+    uint64_t* full = (uint64_t*)(smem + STAGES * (kStageA + kStageB));
+    uint64_t* empty = full + STAGES;
+    uint64_t* acc_full = empty + STAGES;
+    uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
+    volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform for the compiler too
+    const int rank = p.splits > 1 ? (int)cluster_ctarank() : 0, unit = blockIdx.x / p.splits;
+    const int n_blk = unit % p.tiles_n, m_blk = unit / p.tiles_n % p.tiles_m, b = unit / (p.tiles_n * p.tiles_m);
+    const int total_kb = (p.K + BK - 1) / BK;
+    const int kb0 = total_kb * rank / p.splits, num_kb = total_kb * (rank + 1) / p.splits - kb0;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(acc_full, 1);
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, BN);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+
+    if (warp == 0) {
+        if (lane == 0) {
+            for (int i = 0; i < num_kb; i++) {
+                const int st = i % STAGES, k = (kb0 + i) * BK;
+                if (!mbar_wait(&empty[st], ((uint32_t)(i / STAGES) & 1) ^ 1, abort_flag)) break;
+                mbar_expect_tx(&full[st], kStageA + kStageB);
+                if (!p.a_mn_major) {
+                    tma_load_3d(sa + st * kStageA, &map_a, &full[st], k, m_blk * BM, b);  // box {64 k, 128 m}
+                } else {
+                    for (int j = 0; j < BM / 64; j++) tma_load_3d(sa + st * kStageA + j * (64 * BK * 2), &map_a, &full[st], m_blk * BM + j * 64, k, b);
+                }
+                if (!p.b_mn_major) tma_load_3d(sb + st * kStageB, &map_b, &full[st], k, n_blk * BN, b);  // box {64 k, 64 n}
+                else tma_load_3d(sb + st * kStageB, &map_b, &full[st], n_blk * BN, k, b);                 // box {64 n, 64 k}
+            }
+        }
+    } else if (warp == 1) {  // the whole warp: the operands stay in uniform registers
+        const bool leader = elect_one();
+        const uint32_t idesc = make_idesc(BM, BN, p.in_bf16 != 0, p.a_mn_major, p.b_mn_major);
+        const uint64_t da0 = make_smem_desc(smem_u32(sa), p.a_mn_major ? 64 * BK * 2 : 16, 1024);
+        const uint64_t db0 = make_smem_desc(smem_u32(sb), p.b_mn_major ? 64 * BK * 2 : 16, 1024);
+        const uint32_t a_step = p.a_mn_major ? 2048u : 32u, b_step = p.b_mn_major ? 2048u : 32u;
+        bool ok = true;
+        for (int i = 0; i < num_kb && ok; i++) {
+            const int st = i % STAGES;
+            if (!(ok = mbar_wait_warp(&full[st], (uint32_t)(i / STAGES) & 1, abort_flag))) break;
+            tc_fence_after();
+            const uint64_t da = desc_advance(da0, (uint32_t)(st * kStageA)), db = desc_advance(db0, (uint32_t)(st * kStageB));
+#pragma unroll
+            for (int k = 0; k < BK / 16; k++) mma_f16(tmem, desc_advance(da, k * a_step), desc_advance(db, k * b_step), idesc, (i | k) != 0, leader);
+            mma_commit(&empty[st], leader);
+        }
+        if (ok) mma_commit(acc_full, leader);
+    } else {
+        // every product has completed, so every load has landed: the ring is free for the partial tile
+        const int quarter = warp & 3, row = quarter * 32 + lane;
+        if (mbar_wait_warp(acc_full, 0, abort_flag)) {
+            tc_fence_after();
+            uint32_t v[BN];
+            tmem_ld_32x32(tmem + ((uint32_t)(quarter * 32) << 16), v);
+            tmem_ld_32x32(tmem + ((uint32_t)(quarter * 32) << 16) + 32, v + 32);
+            tmem_ld_wait();
+#pragma unroll
+            for (int c = 0; c < BN / 4; c++) *(uint4*)(smem + chunk_at(row, c)) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+            tc_fence_before();
+        }
+    }
+    __syncwarp();
+    if (p.splits > 1) cluster_sync();
+    else __syncthreads();
+
+    // this CTA's share of the rows: eight columns per thread
+    if (!*abort_flag) {
+        const int rows = BM / p.splits;
+        for (int i = threadIdx.x; i < rows * (BN / 8); i += kThreads) {
+            const int r = rank * rows + i / (BN / 8), q = i % (BN / 8);
+            const long long row = (long long)m_blk * BM + r;
+            const int col = n_blk * BN + q * 8;
+            if (row >= p.M || col >= p.N) continue;
+            float x[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+            if (p.splits > 1) {
+                const uint32_t at0 = smem_u32(smem) + chunk_at(r, 2 * q), at1 = smem_u32(smem) + chunk_at(r, 2 * q + 1);
+                for (int s = 0; s < p.splits; s++) {
+                    const float4 u = load_cluster(at0, s), w = load_cluster(at1, s);
+                    x[0] += u.x, x[1] += u.y, x[2] += u.z, x[3] += u.w, x[4] += w.x, x[5] += w.y, x[6] += w.z, x[7] += w.w;
+                }
+            } else {
+                const float4 u = *(const float4*)(smem + chunk_at(r, 2 * q)), w = *(const float4*)(smem + chunk_at(r, 2 * q + 1));
+                x[0] = u.x, x[1] = u.y, x[2] = u.z, x[3] = u.w, x[4] = w.x, x[5] = w.y, x[6] = w.z, x[7] = w.w;
+            }
+            const int live = min(8, p.N - col);
+            const uint16_t* aux = (const uint16_t*)p.aux + (long long)b * p.aux_batch_stride + row * p.ld_aux + col;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                if (p.epilogue == EPI_RELU) x[j] = fmaxf(x[j], 0.0f);
+                if (p.epilogue >= EPI_ADD && j < live) {  // 16-bit outputs only; the product is rounded first, as its own primitive
+                    const uint16_t a16 = aux[j];
+                    float prod, other;
+                    if (p.d_bf16) prod = __bfloat162float(__float2bfloat16_rn(x[j])), other = __uint_as_float((uint32_t)a16 << 16);
+                    else prod = __half2float(__float2half_rn(x[j])), other = __half2float(__ushort_as_half(a16));
+                    x[j] = p.epilogue == EPI_ADD ? __fadd_rn(other, prod) : (other > 0.0f ? prod : 0.0f);
+                }
+            }
+            const long long at = (long long)b * p.d_batch_stride + row * p.ldd + col;
+            if (p.d_bf16 || p.d_f16) {
+                uint16_t h[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) h[j] = p.d_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(x[j])) : __half_as_ushort(__float2half_rn(x[j]));
+                uint16_t* out = (uint16_t*)p.d + at;
+                if (p.vec && live == 8) {
+                    *(uint4*)out = make_uint4(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16, h[4] | (uint32_t)h[5] << 16, h[6] | (uint32_t)h[7] << 16);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        if (j < live) out[j] = h[j];
+                }
+            } else {
+                float* out = (float*)p.d + at;
+                if (p.vec && live == 8) {
+                    *(float4*)out = make_float4(x[0], x[1], x[2], x[3]);
+                    *(float4*)(out + 4) = make_float4(x[4], x[5], x[6], x[7]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        if (j < live) out[j] = x[j];
+                }
+            }
+        }
+    }
+    __syncthreads();
+    if (*abort_flag) {
+        if (threadIdx.x == 0) atomicExch(p.status, LB_ERR_TIMEOUT);
+        // give copies and products still in flight a bounded time to land before shared and tensor memory are released
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000) {
+        }
+    }
+    __syncwarp();
+    if (p.splits > 1) cluster_sync();  // no CTA leaves while another reads its partial tile
+    else __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, BN);
+    }
+}
+
+}  // namespace
+
+template <int STAGES>
+static void launch_small(const CUtensorMap& map_a, const CUtensorMap& map_b, const SmallGemmArgs& p, int batch, cudaStream_t s) {
+    if (first_use_on_device((const void*)gemm_small_kernel<STAGES>))
+        LB_CUDA(cudaFuncSetAttribute(gemm_small_kernel<STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(STAGES)));
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = p.splits, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)((long long)p.tiles_m * p.tiles_n * batch * p.splits)), cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem_bytes(STAGES), cfg.stream = s, cfg.attrs = attr, cfg.numAttrs = 1;
+    LB_CUDA(cudaLaunchKernelEx(&cfg, gemm_small_kernel<STAGES>, map_a, map_b, p));
+}
+
+void gemm_small(const CUtensorMap& map_a, const CUtensorMap& map_b, SmallGemmArgs p, int batch, int sms, cudaStream_t s) {
+    p.tiles_m = (p.M + BM - 1) / BM, p.tiles_n = (p.N + BN - 1) / BN;
+    const int per_line = p.d_bf16 || p.d_f16 ? 8 : 4;
+    p.vec = (uintptr_t)p.d % 16 == 0 && p.ldd % per_line == 0 && p.d_batch_stride % per_line == 0;
+    if ((long long)p.tiles_m * p.tiles_n * batch * p.splits <= sms) launch_small<8>(map_a, map_b, p, batch, s);
+    else launch_small<4>(map_a, map_b, p, batch, s);
+}
+
+}  // namespace lb

@@ -234,3 +234,46 @@ def test_tcgen05_gemm_takes_float16_operands(cuda, kernel):
     device_status()
     want16 = np.maximum(want, 0).astype(np.float16).astype(np.float32)
     np.testing.assert_allclose(to_numpy(narrow).astype(np.float32), want16, rtol=2**-9, atol=2**-9 * np.abs(want16).max())
+
+
+# (batch, M, N, K): the narrow tiles' edges - one element, one row past a tile, N that is no multiple of 8, a K tail, 1 to 8 K
+# ranges in a cluster, two CTAs per SM, batches
+NARROW_CASES = [(1, 1, 8, 8), (1, 129, 72, 200), (1, 128, 64, 64), (1, 200, 136, 1096), (1, 300, 1000, 512), (1, 64, 64, 2056), (1, 1100, 1024, 4608),
+                (3, 130, 200, 264)]
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
+@pytest.mark.parametrize("majors", ["kn", "kk", "mn", "mk"])
+@pytest.mark.parametrize("case", NARROW_CASES)
+def test_narrow_tiles_against_float64(cuda, case, majors, dtype):
+    """Products of the automatically chosen kernel in every operand order, float32 and rounded outputs and epilogues: a
+    float32 sum of K terms of size 1/sqrt(K) is off by less than sqrt(K) * 2^-24 * 4 of the largest result, a rounded one by a
+    unit in the last place more; bit-identical from run to run."""
+    b, m, n, k = case
+    if (majors[0] == "m" and m % 8) or (majors[1] == "n" and n % 8):
+        m, n = (m + 7) // 8 * 8, (n + 7) // 8 * 8  # a contiguous axis has to be a multiple of 16 bytes
+    if majors in ("kk", "kn", "mk") and k % 8:
+        k = (k + 7) // 8 * 8
+    gen = torch.Generator(device=cuda).manual_seed(7)
+    t = getattr(torch, dtype)
+    a = (torch.randn((b, m, k) if majors[0] == "k" else (b, k, m), generator=gen, device=cuda) / k**0.5).to(t)
+    w = torch.randn((b, k, n) if majors[1] == "n" else (b, n, k), generator=gen, device=cuda).to(t)
+    a, w = a if majors[0] == "k" else a.transpose(1, 2), w if majors[1] == "n" else w.transpose(1, 2)
+    aux = torch.randn((b, m, n), generator=gen, device=cuda).to(t)
+    if b == 1:
+        a, w, aux = a[0], w[0], aux[0]
+    want = a.double() @ w.double()
+    top = want.abs().max()
+    out32 = torch.full(want.shape, float("nan"), device=cuda)
+    gemm(a, w, out32)
+    assert (out32.double() - want).abs().max() <= 4 * k**0.5 * 2.0**-24 * top
+    ulp = 2.0**-8 if dtype == "bfloat16" else 2.0**-11
+    for epilogue in (None, "relu", "add", "mask_positive"):
+        out, again = (torch.full(want.shape, float("nan"), dtype=t, device=cuda) for _ in range(2))
+        for o in (out, again):
+            gemm(a, w, o, epilogue=epilogue, aux=aux if epilogue in ("add", "mask_positive") else None)
+        ref = {None: want, "relu": want.clamp(min=0), "add": want + aux.double(), "mask_positive": torch.where(aux > 0, want, torch.zeros_like(want))}[epilogue]
+        # one rounding of the product and, for "add", one of the sum
+        assert ((out.double() - ref).abs() <= 2 * ulp * torch.maximum(ref.abs(), want.abs()) + 4 * k**0.5 * 2.0**-24 * top).all(), epilogue
+        assert torch.equal(out, again)
+    device_status()
