@@ -466,7 +466,13 @@ class Generator {
         VEC_ = std::min(8, 16 / min_size);
         while (VEC_ > 1 && C_ % VEC_ != 0) VEC_ /= 2;
         int64_t nvec = std::max<int64_t>((C_ + VEC_ - 1) / VEC_, 1);
-        int64_t want = (nvec + 3) / 4;
+        // Vectors of a row per thread: four of 16 bytes, more of the narrow ones that a width without a power of two allows - a
+        // row over 1024 threads of three 2-byte loads each is bound by its barriers and by loads in flight. The
+        // multiply-add-relu-square-sum chain, us, 4 -> 16 vectors of one element: 5000 x 3001 bfloat16 24.7 -> 20.0, 20000 x 513
+        // 22.7 -> 14.6, 60000 x 257 float32 27.8 -> 23.0 (100000 x 101 18.5 either way); 4 -> 8 of two: 5000 x 3002 float32
+        // 26.7 -> 21.1 (16: 24.9), bfloat16 12.6 either way.
+        const int64_t per = std::max(4, 16 / VEC_);
+        int64_t want = (nvec + per - 1) / per;
         T_ = 1;
         while (T_ < want && T_ < 1024) T_ *= 2;
         RPB_ = T_ >= 32 ? 1 : 256 / T_;

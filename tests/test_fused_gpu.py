@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 import torch
 
+import lumen_b200
 from lumen_b200 import functional as F
 from lumen_b200 import prims, tracer
 from lumen_b200.runtime import Fusion
@@ -288,3 +289,24 @@ def test_row_and_column_reductions_in_one_kernel(cuda, shape, dtype):
     assert (np.abs(c - want) <= (half + 1e-6) * np.abs(want) + 1e-5).all()
     assert (np.abs(s - x64.sum(0)) <= 1e-5 * np.abs(x64).sum(0)).all()
     assert (np.abs(q - (want * want).sum(0)) <= (half + 2e-5) * (want * want).sum(0)).all()
+
+
+# widths whose vectors are one or two elements: one thread per row up to a whole block, remainders of a thread's share
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("rows,cols", [(3, 1), (70, 15), (9, 17), (33, 257), (5, 511), (5, 514), (7, 3001), (4, 4097), (3, 8190), (2, 16383)])
+def test_rows_of_odd_widths(cuda, rows, cols, dtype):
+    """y is exact; a float32 sum of `cols` non-negative terms in any order is within cols * 2^-24 of the float64 one."""
+    gen = torch.Generator(device=cuda).manual_seed(cols)
+    t = getattr(torch, dtype)
+    x, g, b = (torch.randn(s, generator=gen, device=cuda).to(t) for s in ((rows, cols), (cols,), (cols,)))
+
+    def chain(x_, g_, b_):
+        y_ = F.relu(x_ * g_ + b_)
+        return y_, prims.reduce_sum(y_ * y_, (1,), "float32")
+
+    y, s = lumen_b200.compile(chain)(x, g, b)
+    y, s = torch.as_tensor(y, device=cuda), torch.as_tensor(s, device=cuda)
+    want = torch.relu(x * g + b)
+    assert torch.equal(y.view(t) if y.dtype != t else y, want)
+    total = (want * want).double().sum(1)
+    assert ((s.double() - total).abs() <= cols * 2.0**-24 * total + 1e-30).all()
