@@ -1309,6 +1309,7 @@ class Generator {
             k.slices = 1;
             std::vector<size_t> offsets;
             size_t scratch = 0;
+            if (RPB_ > 1) s << "    __shared__ __align__(16) char shared[NCOLS * 8];\n";
             for (size_t i = 0; i < col_reduces_.size(); i++) {
                 const Node& n = *g_.node_of(col_reduces_[i]);
                 const TensorType& t = g_.type(n.output);
@@ -1318,11 +1319,11 @@ class Generator {
                 reduce_ops(n, t, &init, &combine);
                 s << "    {\n        " << type << "* part = (" << type << "*)((char*)scratch + " << scratch << ") + (idx_t)blockIdx.x * NCOLS;\n";
                 if (RPB_ > 1) {  // the block's rows in order, through shared memory
-                    s << "        __shared__ " << type << " csum" << i << "[NCOLS];\n";
+                    s << "        " << type << "* csum" << i << " = (" << type << "*)shared;\n";
                     s << "        for (int y = 0; y < RPB; y++) {\n            if (row_in_block == y) { CHUNK_LOOP_BEGIN _Pragma(\"unroll\") for (int e = 0; e < VEC; e++) csum"
                       << i << "[c0 + e] = y ? " << subst(combine, format("csum%d[c0 + e]", (int)i), format("cacc%d[ch][e]", (int)i)) << " : cacc" << i
                       << "[ch][e]; CHUNK_LOOP_END }\n            __syncthreads();\n        }\n";
-                    s << "        for (int c = threadIdx.x; c < NCOLS; c += TPR * RPB) part[c] = csum" << i << "[c];\n    }\n";
+                    s << "        for (int c = threadIdx.x; c < NCOLS; c += TPR * RPB) part[c] = csum" << i << "[c];\n        __syncthreads();\n    }\n";
                 } else {
                     s << "        CHUNK_LOOP_BEGIN _Pragma(\"unroll\") for (int e = 0; e < VEC; e++) part[c0 + e] = cacc" << i << "[ch][e]; CHUNK_LOOP_END\n    }\n";
                 }
@@ -1409,6 +1410,7 @@ class Generator {
         Phase part;
         std::ostringstream decl, store;
         size_t scratch = 0;
+        int widest = 1;  // all reductions use one area of shared memory in turn: any number of them fits
         std::vector<size_t> offsets;
         for (size_t k = 0; k < col_reduces_.size(); k++) {
             const Node& n = *g_.node_of(col_reduces_[k]);
@@ -1429,7 +1431,9 @@ class Generator {
                         : (std::string(ct.compute) == "float" || std::string(ct.compute) == "i32" || std::string(ct.compute) == "u32") ? 4
                         : dtype_size(t.dtype);
             // the 8 row lanes of a column are combined in lane order through shared memory, then lane 0 stores the slice's partial
-            store << "__shared__ " << ct.compute << " red" << k << "[" << row_lanes << "][" << col_lanes << " * VEC];\n";
+            widest = std::max(widest, width);
+            if (k) store << "__syncthreads();\n";
+            store << "auto red" << k << " = (" << ct.compute << "(*)[" << col_lanes << " * VEC])shared;\n";
             store << "#pragma unroll\nfor (int e = 0; e < VEC; e++) red" << k << "[row_lane][col_lane * VEC + e] = acc" << k << "[e];\n__syncthreads();\n";
             store << "if (row_lane == 0 && in_range) {\n#pragma unroll\n    for (int e = 0; e < VEC; e++) {\n        " << ct.compute << " t = acc" << k
                   << "[e];\n        for (int y = 1; y < " << row_lanes << "; y++) t = " << subst(combine, "t", format("red%d[y][col_lane * VEC + e]", (int)k))
@@ -1450,6 +1454,7 @@ class Generator {
         s << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") fused_kernel(" << sig << ") {\n";
         s << "    const int col_lane = threadIdx.x & " << col_lanes - 1 << ", row_lane = threadIdx.x >> 5;\n";
         s << "    const idx_t c0 = ((idx_t)blockIdx.x * " << col_lanes << " + col_lane) * VEC;\n    const bool in_range = c0 < NCOLS;\n";
+        s << "    __shared__ __align__(16) char shared[" << row_lanes * col_lanes << " * VEC * " << widest << "];\n";
         s << indent(decl.str(), 4);
         s << "    const idx_t r_end = in_range ? (idx_t)(((idx_t)blockIdx.y + 1) * ROWS_PER_SLICE < NROWS ? ((idx_t)blockIdx.y + 1) * ROWS_PER_SLICE : NROWS) : 0;\n";
         s << "    for (idx_t r = (idx_t)blockIdx.y * ROWS_PER_SLICE + row_lane; r < r_end; r += " << row_lanes << ") {\n";
@@ -1487,6 +1492,7 @@ class Generator {
         flat_c.lane = flat_c.e_dep = flat_c.c_dep = true;
         Phase fin;
         std::ostringstream totals;
+        int widest = 1;  // of the compute types; one area of shared memory serves the reductions in turn
         for (size_t k = 0; k < col_reduces_.size(); k++) {
             const Node& n = *g_.node_of(col_reduces_[k]);
             const TensorType& t = g_.type(n.output);
@@ -1498,7 +1504,9 @@ class Generator {
             totals << "if (in_range) {\n#pragma unroll 8\n    for (int s = row_lane; s < SLICES; s += " << row_lanes << ") {\n#pragma unroll\n        for (int e = 0; e < VEC; e++) { "
                    << ct.compute << " pv = ((const " << ct.compute << "*)((const char*)scratch + " << offsets[k] << "))[(idx_t)s * NCOLS + c0 + e]; tot" << k
                    << "[e] = " << subst(combine, format("tot%d[e]", (int)k), "pv") << "; }\n    }\n}\n";
-            totals << "__shared__ " << ct.compute << " fred" << k << "[" << row_lanes << "][" << col_lanes << " * VEC];\n";
+            widest = std::max(widest, t.dtype == LB_BF16 || t.dtype == LB_F16 ? 4 : dtype_size(t.dtype));
+            if (k) totals << "__syncthreads();\n";
+            totals << "auto fred" << k << " = (" << ct.compute << "(*)[" << col_lanes << " * VEC])shared;\n";
             totals << "#pragma unroll\nfor (int e = 0; e < VEC; e++) fred" << k << "[row_lane][col_lane * VEC + e] = tot" << k << "[e];\n__syncthreads();\n";
             totals << "if (row_lane == 0) {\n#pragma unroll\n    for (int e = 0; e < VEC; e++) {\n#pragma unroll\n        for (int y = 1; y < " << row_lanes << "; y++) tot" << k << "[e] = "
                    << subst(combine, format("tot%d[e]", (int)k), format("fred%d[y][col_lane * VEC + e]", (int)k)) << ";\n    }\n}\n";
@@ -1517,6 +1525,7 @@ class Generator {
         s << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") fused_finalize(" << sig << ") {\n";
         s << "    const int col_lane = threadIdx.x & " << col_lanes - 1 << ", row_lane = threadIdx.x >> 5;\n";
         s << "    const idx_t c0 = ((idx_t)blockIdx.x * " << col_lanes << " + col_lane) * VEC;\n    const bool in_range = c0 < NCOLS;\n";
+        s << "    __shared__ __align__(16) char shared[" << threads << " * VEC * " << widest << "];\n";
         s << indent(totals.str(), 4);
         s << "    if (row_lane != 0 || !in_range) return;\n";
         s << indent(fin.pre, 4);

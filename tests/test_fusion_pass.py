@@ -120,3 +120,28 @@ def test_long_reductions_are_split_without_changing_their_values(shape):
     assert after[0].shape == before[0].shape and after[1].shape == before[1].shape
     assert (np.abs(after[0] - exact) <= 1e-6 * magnitude).all()
     np.testing.assert_array_equal(after[1], before[1])
+
+
+@pytest.mark.parametrize("count,dtype,beside", [(6, "float32", False), (7, "float32", False), (16, "float32", False), (4, "float64", False), (7, "bfloat16", False),
+                                                (8, "float32", True), (5, "float64", True)])
+def test_any_number_of_column_reductions_of_one_operand_compiles(count, dtype, beside):
+    """Statistics per feature (column sums of `count` functions of one operand), alone and beside a row-wise output: the
+    groups that read the operand are merged, and every kernel of the result is built (generation alone does not see limits
+    of the hardware such as 48 KB of static shared memory)."""
+    from lumen_b200.runtime import Fusion
+
+    accum = "float64" if dtype == "float64" else "float32"
+
+    def program(x):
+        powers = [x]
+        for _ in range(count - 1):
+            powers.append(powers[-1] * x)
+        sums = tuple(prims.reduce_sum(p, (0,), accum) for p in powers)
+        return (F.relu(x), *sums) if beside else sums
+
+    rows = 8192 if not beside else 70000  # narrow rows beside: several to a block, whose sums meet in shared memory
+    g = tracer.trace(program, (dtype, (rows, 1024 if not beside else 64)))
+    fused = fuse(g)
+    assert not bare(fused)
+    for f in fusions(fused):
+        Fusion(f.params["body"])
