@@ -155,14 +155,15 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attention_decode_kernel(const 
             for (int h = 0; h < 2; h++) {  // rows lane / 4 and lane / 4 + 8
                 float x[4] = {s[t][0][2 * h], s[t][0][2 * h + 1], s[t][1][2 * h], s[t][1][2 * h + 1]};
 #pragma unroll
-                for (int i = 0; i < 4; i++) x[i] = key0 + (i & 1) + (i >> 1) * 8 <= limit[t][h] ? x[i] * p.scale_log2 : -INFINITY;
+                for (int i = 0; i < 4; i++)
+                    if (key0 + (i & 1) + (i >> 1) * 8 > limit[t][h]) x[i] = -INFINITY;
                 float top = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
                 top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
                 top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
-                const float m_new = fmaxf(m[t][h], top), shift = m_new == -INFINITY ? 0.0f : m_new;
+                const float m_new = fmaxf(m[t][h], top * p.scale_log2), shift = m_new == -INFINITY ? 0.0f : m_new;
                 const float alpha = exp2_fast(m[t][h] - shift);
 #pragma unroll
-                for (int i = 0; i < 4; i++) x[i] = exp2_fast(x[i] - shift);
+                for (int i = 0; i < 4; i++) x[i] = exp2_fast(fmaf(x[i], p.scale_log2, -shift));  // rounded once, as in the tile kernel
                 l[t][h] = l[t][h] * alpha + ((x[0] + x[1]) + (x[2] + x[3]));  // this thread's keys; the quad is added up at the end
                 pf[t][h] = pack(x[0], x[1]), pf[t][2 + h] = pack(x[2], x[3]);
                 m[t][h] = m_new;
@@ -236,7 +237,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attention_decode_kernel(const 
         __nv_bfloat16* o = p.o + b * p.o_sb + (long long)position * p.o_ss + (long long)head * p.o_sn + d;
         if (p.pair_stores) *(__nv_bfloat162*)o = __floats2bfloat162_rn(x * inv, y * inv);
         else o[0] = __float2bfloat16_rn(x * inv), o[1] = __float2bfloat16_rn(y * inv);
-        if (d == 0 && p.lse) p.lse[((long long)b * p.N + head) * p.Sq + position] = (whole + log2f(sum)) * 0.6931471805599453f;
+        // one rounding at the size of the result: (whole + log2f(sum)) * ln 2 has two, one of them at 1.44 times the size
+        if (d == 0 && p.lse) p.lse[((long long)b * p.N + head) * p.Sq + position] = fmaf(whole, 0.6931471805599453f, logf(sum));
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // nobody leaves while it is read
 }
