@@ -214,9 +214,25 @@ __device__ __forceinline__ float dot_row(const float* own, const float* tile, in
     }
     return total;
 }
-// acc[u] += sum over the chunk of weight[row] * tile[row][lane + 32 u], in row order
+// acc[u] += sum over the chunk's rows [lo, hi) of weight[row] * tile[row][lane + 32 u], in row order. The other rows are not
+// read: their weights are 0, but a value behind the mask may be infinite or NaN, and 0 times that is NaN.
 template <int DU>
-__device__ __forceinline__ void add_weighted(float* acc, const float* weight, const float* tile, int lane) {
+__device__ __forceinline__ void add_weighted(float* acc, const float* weight, const float* tile, int lane, int lo, int hi) {
+    if (lo > 0 || hi < kChunk) {  // warp-uniform
+#pragma unroll 1
+        for (int j = lo & ~3; j < hi; j += 4) {
+            const float4 w = *(const float4*)(weight + j);
+            const float* t = tile + j * AttnSmem<DU>::kPitch + lane;
+#pragma unroll
+            for (int u = 0; u < DU; u++, t += 32) {
+                acc[u] = fmaf(w.x, j >= lo ? t[0] : 0.0f, acc[u]);
+                acc[u] = fmaf(w.y, j + 1 >= lo && j + 1 < hi ? t[AttnSmem<DU>::kPitch] : 0.0f, acc[u]);
+                acc[u] = fmaf(w.z, j + 2 >= lo && j + 2 < hi ? t[2 * AttnSmem<DU>::kPitch] : 0.0f, acc[u]);
+                acc[u] = fmaf(w.w, j + 3 >= lo && j + 3 < hi ? t[3 * AttnSmem<DU>::kPitch] : 0.0f, acc[u]);
+            }
+        }
+        return;
+    }
 #pragma unroll (DU > 2 ? 2 : 8)
     for (int j = 0; j < kChunk; j += 4) {
         const float4 w = *(const float4*)(weight + j);
@@ -273,7 +289,7 @@ attention_simt_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, cons
         for (int u = 0; u < DU; u++) acc[u] *= alpha;
         __syncwarp();
         // the normaliser is applied at the end
-        add_weighted<DU>(acc, sm.weight[0][warp], sm.tile[1], lane);
+        add_weighted<DU>(acc, sm.weight[0][warp], sm.tile[1], lane, 0, (int)min((long long)kChunk, last + 1 - j0));
         __syncwarp();
         m = m_new;
     }
@@ -318,7 +334,7 @@ attention_simt_dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const
         }
         sm.weight[0][warp][lane] = ds;
         __syncwarp();
-        add_weighted<DU>(acc, sm.weight[0][warp], sm.tile[0], lane);
+        add_weighted<DU>(acc, sm.weight[0][warp], sm.tile[0], lane, 0, (int)min((long long)kChunk, last + 1 - j0));
         __syncwarp();
     }
     if (!live) return;
@@ -364,8 +380,9 @@ attention_simt_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, con
             }
             sm.weight[0][warp][lane] = ds, sm.weight[1][warp][lane] = pr;
             __syncwarp();
-            add_weighted<DU>(ak, sm.weight[0][warp], sm.tile[0], lane);
-            add_weighted<DU>(av, sm.weight[1][warp], sm.tile[1], lane);
+            const int lo = (int)max(0LL, first - i0), hi = (int)min((long long)kChunk, s.Sq - i0);
+            add_weighted<DU>(ak, sm.weight[0][warp], sm.tile[0], lane, lo, hi);
+            add_weighted<DU>(av, sm.weight[1][warp], sm.tile[1], lane, lo, hi);
             __syncwarp();
         }
     }

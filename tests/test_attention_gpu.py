@@ -433,3 +433,32 @@ def test_cuda_core_scores_are_as_exact_as_a_warp_wide_sum(cuda, h):
         return float(np.sqrt(np.mean((to_numpy(x).astype(np.float64) - want) ** 2)))
 
     assert rms(lse) <= 1.1 * rms(torch.logsumexp(scores, -1).float())
+
+
+@pytest.mark.parametrize("h,dtype", [(32, "float32"), (128, "float32"), (200, "float32"), (80, "bfloat16")])
+def test_cuda_core_attention_keeps_masked_rows_of_nan_out(cuda, h, dtype):
+    """A causal mask: a NaN in a value, key, query or gradient row reaches the rows that see it (or that it sees) and no other,
+    wherever the rows lie in their blocks of eight and chunks of 32."""
+    s = 70
+    rng = np.random.default_rng(h)
+    q, k, v, do = (to_torch(rng.standard_normal((1, s, 2, h)).astype(np.float32), cuda).to(getattr(torch, dtype)) for _ in range(4))
+    o, lse = attention_forward(q, k, v, causal=True)
+    nan = float("nan")
+
+    def with_nan(x, row):
+        x = x.clone()
+        x[:, row] = nan
+        return x
+
+    def rows_of_nan(x):
+        return torch.isnan(x).flatten(2).any(2)[0].nonzero().flatten().tolist()
+
+    for at in (0, 5, 31, 37, 64):
+        assert rows_of_nan(attention_forward(q, k, with_nan(v, at), causal=True)[0]) == list(range(at, s))
+        dq, _, _ = attention_backward(q, with_nan(k, at), v, o, do, lse, causal=True)
+        assert rows_of_nan(dq) == list(range(at, s))
+        _, dk, dv = attention_backward(with_nan(q, at), k, v, o, do, lse, causal=True)
+        assert rows_of_nan(dk) == list(range(at + 1)) and rows_of_nan(dv) == list(range(at + 1))
+        _, dk, dv = attention_backward(q, k, v, o, with_nan(do, at), lse, causal=True)
+        assert rows_of_nan(dk) == list(range(at + 1)) and rows_of_nan(dv) == list(range(at + 1))
+    device_status()
