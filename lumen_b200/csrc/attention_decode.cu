@@ -305,7 +305,7 @@ void launch(const DecodeArgs& p, int batch, long long keys, cudaStream_t s) {
 // Whether attention_decode takes the problem: all rows of a key head's group in two 16-row tiles. (Operands as the
 // tensor-core kernels need them: bfloat16, head dim 64 or 128, unit head-dim stride, 16-byte aligned rows.)
 bool attention_decodes(const lb_tensor& q, const lb_tensor& k) {
-    return q.shape[0] > 0 && k.shape[2] > 0 && q.shape[2] % k.shape[2] == 0 && q.shape[0] <= 65535 && k.shape[2] <= 65535 &&
+    return q.shape[0] > 0 && k.shape[1] > 0 && k.shape[2] > 0 && q.shape[2] % k.shape[2] == 0 && q.shape[0] <= 65535 && k.shape[2] <= 65535 &&
            q.shape[1] > 0 && q.shape[2] / k.shape[2] * q.shape[1] <= kMaxRows;
 }
 

@@ -7,6 +7,7 @@ import torch
 
 from lumen_b200 import functional as F
 from lumen_b200 import tracer
+from lumen_b200._lib import LumenError
 from lumen_b200.runtime import attention_backward, attention_forward, device_status
 from tests.helpers import attention_f64, bf16, run_oracle, to_numpy, to_torch
 
@@ -462,3 +463,10 @@ def test_cuda_core_attention_keeps_masked_rows_of_nan_out(cuda, h, dtype):
         _, dk, dv = attention_backward(q, k, v, o, with_nan(do, at), lse, causal=True)
         assert rows_of_nan(dk) == list(range(at + 1)) and rows_of_nan(dv) == list(range(at + 1))
     device_status()
+
+
+@pytest.mark.parametrize("sq", [1, 32, 64])
+def test_attention_without_keys_is_refused(cuda, sq):
+    q, k = (torch.zeros((1, s, 2, 64), dtype=torch.bfloat16, device=cuda) for s in (sq, 0))
+    with pytest.raises(LumenError):
+        attention_forward(q, k, k)
