@@ -149,6 +149,11 @@ typedef struct {
 } lb_attn_desc;
 int lb_attention_fwd(const lb_attn_desc* desc, const lb_tensor* q, const lb_tensor* k, const lb_tensor* v,
                      const lb_tensor* o, const lb_tensor* lse /* nullable */, void* stream);
+/* Which kernel lb_attention_fwd runs on these operands (pointers matter by their alignment only; without a device, as on
+ * a B200): 0 the CUDA-core kernel, 1 one 128-query tile per CTA, 2 two of them, 3 the kernel for few query rows per key
+ * head. Results of different kernels agree to the rounding of the operands' dtype, not bit for bit; which one runs, and
+ * into how many key ranges kernel 3 cuts its work, depends on every dimension, the batch included. */
+int lb_attention_fwd_kernel(const lb_attn_desc* desc, const lb_tensor* q, const lb_tensor* k, const lb_tensor* v, int32_t* kernel);
 /* Backward of lb_attention_fwd, FlashAttention-2's as the reference traces it
  * (lumen/functional/attention/flash.py:51-85): probabilities recomputed from `lse`; `delta` [B, N, Sq] float32 is
  * caller-provided scratch that receives rowsum(dO * O); dq, dk, dv are bfloat16 views shaped like q, k, v. The

@@ -17,7 +17,7 @@
 #include <map>
 #include <mutex>
 
-#include "device.h"
+#include "attention.h"
 
 namespace lb {
 namespace {
@@ -243,43 +243,54 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attention_decode_kernel(const 
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // nobody leaves while it is read
 }
 
+// How the kernel does on a problem, in microseconds of a B200: a CTA costs `base + per_row * rows` (prologue, merge, the way out)
+// and `per_slice` per slice that a warp walks, and the keys and values cross HBM at most at `gb` GB/s. Fitted to 1373 timings of
+// 1 to 32 rows, 4 to 4096 (batch, key head)s and 32 to 8192 keys (root mean square of the error 15 to 20 %).
+struct DecodeCost {
+    int resident;  // CTAs per SM: shared memory at head dim 128, registers at 64
+    double base, per_row, per_slice, gb;
+};
+constexpr DecodeCost decode_cost(int D, int MT) {
+    return D == 64 ? (MT == 1 ? DecodeCost{4, 3.4, 0.14, 1.37, 6100} : DecodeCost{2, 4.9, 0.11, 1.01, 4400})
+                   : (MT == 1 ? DecodeCost{2, 3.8, 0.26, 1.31, 6600} : DecodeCost{1, 5.5, 0.245, 1.2, 3500});
+}
 // CTAs that share one key head's keys: the number that spreads the slices most evenly over the CTAs that fit the SMs, in
-// units of slices per warp; a CTA costs about six slices besides (prologue, merge). More than eight (a cluster size not every
-// part has) only where the runtime says that such clusters can be resident.
-template <int D, int MT>
-int pick_splits(long long pairs, long long keys, int sms) {
-    auto kernel = attention_decode_kernel<D, MT>;
-    constexpr int resident = D == 64 ? (MT == 1 ? 4 : 2) : (MT == 1 ? 2 : 1);  // CTAs per SM: shared memory at 128, registers at 64
-    const long long slices = (keys + kSlice - 1) / kSlice, slots = (long long)resident * sms;
+// units of slices per warp; a CTA counts as six slices besides (the costs above: 3 to 6 with one tile of rows, 7 to 11 with two).
+int pick_splits(const DecodeCost& cost, long long pairs, long long keys, int sms) {
+    const long long slices = (keys + kSlice - 1) / kSlice, slots = (long long)cost.resident * sms;
     int best = 1;
     double best_cost = 1e30;
     for (int s = 1; s <= kMaxSplits; s++) {
         if (s > 1 && (long long)s * kWarps > slices) break;
         const double waves = (double)((pairs * s + slots - 1) / slots);
-        const double cost = waves * ((double)((slices + s * kWarps - 1) / (s * kWarps)) + 6.0);
-        if (cost < best_cost * 0.98) best = s, best_cost = cost;
-    }
-    if (best > 8) {
-        static std::map<int, bool> fits;  // by device
-        static std::mutex mutex;
-        int dev = 0;
-        LB_CUDA(cudaGetDevice(&dev));
-        std::lock_guard<std::mutex> lock(mutex);
-        auto it = fits.find(dev);
-        if (it == fits.end()) {
-            int clusters = 0;
-            cudaLaunchConfig_t cfg = {};
-            cudaLaunchAttribute attr;
-            attr.id = cudaLaunchAttributeClusterDimension;
-            attr.val.clusterDim.x = kMaxSplits, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-            cfg.gridDim = dim3(kMaxSplits), cfg.blockDim = dim3(kWarps * 32), cfg.dynamicSmemBytes = DecodeSmem<D, MT>::kBytes;
-            cfg.attrs = &attr, cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) cudaGetLastError(), clusters = 0;
-            it = fits.emplace(dev, clusters > 0).first;
-        }
-        if (!it->second) best = 8;
+        const double units = waves * ((double)((slices + s * kWarps - 1) / (s * kWarps)) + 6.0);
+        if (units < best_cost * 0.98) best = s, best_cost = units;
     }
     return best;
+}
+// Clusters of more than eight CTAs (a size not every part has) only where the runtime says that they can be resident.
+template <int D, int MT>
+int resident_splits(int splits) {
+    if (splits <= 8) return splits;
+    auto kernel = attention_decode_kernel<D, MT>;
+    static std::map<int, bool> fits;  // by device
+    static std::mutex mutex;
+    int dev = 0;
+    LB_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mutex);
+    auto it = fits.find(dev);
+    if (it == fits.end()) {
+        int clusters = 0;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = kMaxSplits, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(kMaxSplits), cfg.blockDim = dim3(kWarps * 32), cfg.dynamicSmemBytes = DecodeSmem<D, MT>::kBytes;
+        cfg.attrs = &attr, cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) cudaGetLastError(), clusters = 0;
+        it = fits.emplace(dev, clusters > 0).first;
+    }
+    return it->second ? splits : 8;
 }
 
 template <int D, int MT>
@@ -290,7 +301,7 @@ void launch(const DecodeArgs& p, int batch, long long keys, cudaStream_t s) {
         LB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
         LB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     }
-    const int splits = pick_splits<D, MT>((long long)batch * p.Nkv, keys, device_info().sms);
+    const int splits = resident_splits<D, MT>(pick_splits(decode_cost(D, MT), (long long)batch * p.Nkv, keys, device_info().sms));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
@@ -307,6 +318,15 @@ void launch(const DecodeArgs& p, int batch, long long keys, cudaStream_t s) {
 bool attention_decodes(const lb_tensor& q, const lb_tensor& k) {
     return q.shape[0] > 0 && k.shape[1] > 0 && k.shape[2] > 0 && q.shape[2] % k.shape[2] == 0 && q.shape[0] <= 65535 && k.shape[2] <= 65535 &&
            q.shape[1] > 0 && q.shape[2] / k.shape[2] * q.shape[1] <= kMaxRows;
+}
+
+double attention_decode_us(const lb_tensor& q, const lb_tensor& k, int sms) {
+    const long long pairs = q.shape[0] * k.shape[2], rows = q.shape[2] / k.shape[2] * q.shape[1], keys = k.shape[1], D = q.shape[3];
+    const DecodeCost cost = decode_cost((int)D, rows <= 16 ? 1 : 2);
+    const long long splits = pick_splits(cost, pairs, keys, sms), slots = (long long)cost.resident * sms;
+    const long long waves = (pairs * splits + slots - 1) / slots, slices = ((keys + kSlice - 1) / kSlice + splits * kWarps - 1) / (splits * kWarps);
+    const double bytes = (double)pairs * keys * D * 4;
+    return std::max(waves * (cost.base + cost.per_row * rows + cost.per_slice * slices), bytes / (cost.gb * 1e3));
 }
 
 void attention_decode(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o,

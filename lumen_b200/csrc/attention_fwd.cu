@@ -21,7 +21,7 @@
 #include <mutex>
 #include <type_traits>
 
-#include "device.h"
+#include "attention.h"
 #include "sm100.cuh"
 
 namespace lb {
@@ -690,9 +690,30 @@ CUtensorMap make_bsnh_map(const lb_tensor& t, const char* what, int box_rows = 1
 
 CUtensorMap attention_map_rows(const lb_tensor& t, const char* what, int box_rows) { return make_bsnh_map(t, what, box_rows); }
 
-bool attention_decodes(const lb_tensor& q, const lb_tensor& k);
-void attention_decode(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o,
-                      const lb_tensor* lse, void* stream);
+namespace {
+// Microseconds of the one-tile kernel when its queries are at most 32 rows of one tile (two CTAs per SM, each walking all keys)
+double one_tile_few_us(const lb_tensor& q, const lb_tensor& k, int sms) {
+    const long long ctas = q.shape[0] * q.shape[2], waves = (ctas + 2 * sms - 1) / (2 * sms), tiles = (k.shape[1] + BKV - 1) / BKV;
+    const double bytes = (double)k.shape[0] * k.shape[1] * k.shape[2] * k.shape[3] * 4;
+    return std::max(1.0 + waves * (k.shape[3] == 64 ? 3.5 + 1.4 * tiles : 4.0 + 1.8 * tiles), bytes / 5.4e6);
+}
+
+// The kernel for operands that the tensor-core kernels take, by the modelled times of the two that come into question.
+//  * Few rows per key head: the tile kernel has a CTA per query head however many rows of its 128 are live, the other shares
+//    the keys among a group's heads and cuts them into ranges, at a cost per row. Of 1373 timed problems the choice is 0.3 % off
+//    the better kernel on average; always taking the second, as before, was up to 5.6 times slower (4096 heads of 32 queries
+//    and 128 keys at head dim 128: 84 -> 439 us), never taking it 10 times (8 heads of 4 queries and 13568 keys).
+AttentionKernel choose_kernel(const lb_tensor& q, const lb_tensor& k, int sms) {
+    if (attention_decodes(q, k) && attention_decode_us(q, k, sms) < one_tile_few_us(q, k, sms)) return ATTN_FEW_ROWS;
+    // Which kernel (measured, us, one tile per CTA -> two): the second has half the CTAs, so it needs enough of them to fill
+    // the GPU - 4 heads x 4096 at head dim 128: 62 -> 64, 2 x 8 x 1024: 21 -> 23, 32 heads x 4096: 180 -> 130 - and a query
+    // length that gives the second tile rows (8 x 32 x 100 against 4000: 93 -> 115). From two CTAs per SM of the first
+    // kernel on it is ahead at head dim 128 (4 x 16 x 1000: 47 -> 45); at head dim 64, where the one-tile kernel overlaps S
+    // with the softmax as well, from four (4 x 16 x 1000: 40 -> 41, 2 x 32 x 1531: 55 -> 49, 32 x 4096: 144 -> 118).
+    const long long tiles = (q.shape[1] + BQ - 1) / BQ * q.shape[2] * q.shape[0];
+    return q.shape[1] > BQ && tiles > (q.shape[3] == 128 ? 2LL : 4LL) * sms ? ATTN_TWO_TILES : ATTN_ONE_TILE;
+}
+}  // namespace
 
 void attention_fwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o,
                    const lb_tensor* lse, void* stream) {
@@ -709,8 +730,9 @@ void attention_fwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor
     if (lse) check_dense(*lse, LB_F32, {B, N, Sq}, "attention log-sum-exp");
     if (!(desc.scale > 0.0f)) fail(LB_ERR_UNSUPPORTED, "attention: the softmax scale must be positive");
     if (B == 0 || Sq == 0 || N == 0) return;
-    if (attention_decodes(q, k)) {
-        driver();
+    driver();
+    const AttentionKernel kernel = choose_kernel(q, k, device_info().sms);
+    if (kernel == ATTN_FEW_ROWS) {
         attention_decode(desc, q, k, v, o, lse, stream);
         return;
     }
@@ -725,13 +747,7 @@ void attention_fwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor
     p.status = status_word();
     dim3 grid((unsigned)((Sq + BQ - 1) / BQ), (unsigned)N, (unsigned)B);
     cudaStream_t s = (cudaStream_t)stream;
-    // Which kernel (measured, us, one tile per CTA -> two): the second has half the CTAs, so it needs enough of them to fill
-    // the GPU - 4 heads x 4096 at head dim 128: 62 -> 64, 2 x 8 x 1024: 21 -> 23, 32 heads x 4096: 180 -> 130 - and a query
-    // length that gives the second tile rows (8 x 32 x 100 against 4000: 93 -> 115). From two CTAs per SM of the first
-    // kernel on it is ahead at head dim 128 (4 x 16 x 1000: 47 -> 45); at head dim 64, where the one-tile kernel overlaps S
-    // with the softmax as well, from four (4 x 16 x 1000: 40 -> 41, 2 x 32 x 1531: 55 -> 49, 32 x 4096: 144 -> 118).
-    const long long tiles = (Sq + BQ - 1) / BQ * N * B;
-    if (Sq > BQ && tiles > (D == 128 ? 2LL : 4LL) * sm_count_hint()) {
+    if (kernel == ATTN_TWO_TILES) {
         if (D == 128) launch_fwd_pair<128>(mq, mk, mv, p, s);
         else launch_fwd_pair<64>(mq, mk, mv, p, s);
         LB_CUDA(cudaGetLastError());
@@ -765,6 +781,11 @@ bool attention_on_tensor_cores(const lb_tensor& q, const lb_tensor& k, const lb_
     return ok(q) && ok(k) && ok(v) && (q.shape[3] == 64 || q.shape[3] == 128) && v.shape[3] == q.shape[3];
 }
 
+AttentionKernel attention_forward_kernel(const lb_tensor& q, const lb_tensor& k, const lb_tensor& v) {
+    if (q.rank != 4 || k.rank != 4 || v.rank != 4) fail(LB_ERR_INVALID, "attention: operands must be [B, S, N, H] tensors");
+    return attention_on_tensor_cores(q, k, v) ? choose_kernel(q, k, sm_count_hint()) : ATTN_CUDA_CORES;
+}
+
 void attention_forward(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o,
                        const lb_tensor* lse, void* stream) {
     if (attention_on_tensor_cores(q, k, v)) attention_fwd(desc, q, k, v, o, lse, stream);
@@ -777,5 +798,12 @@ extern "C" int lb_attention_fwd(const lb_attn_desc* desc, const lb_tensor* q, co
     return lb::guarded([&] {
         if (!desc || !q || !k || !v || !o) lb::fail(LB_ERR_INVALID, "lb_attention_fwd: null argument");
         lb::attention_forward(*desc, *q, *k, *v, *o, lse, stream);
+    });
+}
+
+extern "C" int lb_attention_fwd_kernel(const lb_attn_desc* desc, const lb_tensor* q, const lb_tensor* k, const lb_tensor* v, int32_t* kernel) {
+    return lb::guarded([&] {
+        if (!desc || !q || !k || !v || !kernel) lb::fail(LB_ERR_INVALID, "lb_attention_fwd_kernel: null argument");
+        *kernel = lb::attention_forward_kernel(*q, *k, *v);
     });
 }

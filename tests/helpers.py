@@ -72,3 +72,16 @@ def attention_f64(q, k, v, causal, d_o=None):
                 grads[1][bi, :, kv] += ds.T @ qh
                 grads[2][bi, :, kv] += p.T @ g
     return (o, lse) if d_o is None else (o, lse, grads)
+
+
+def attention_kernel(b, sq, sk, n, nkv, h, causal=True, dtype="bfloat16"):
+    """Which kernel lb_attention_fwd runs on dense operands of these sizes: "cuda cores", "one tile", "two tiles" or "few rows"."""
+    import ctypes
+
+    from lumen_b200 import _lib
+
+    desc = _lib.LbAttnDesc(h**-0.5, int(causal), sk - sq)
+    q, k, v = (_lib.dense(1 << 20, dtype, s) for s in ((b, sq, n, h), (b, sk, nkv, h), (b, sk, nkv, h)))
+    kernel = ctypes.c_int32()
+    _lib.check(_lib.lib().lb_attention_fwd_kernel(ctypes.byref(desc), ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(kernel)))
+    return ("cuda cores", "one tile", "two tiles", "few rows")[kernel.value]

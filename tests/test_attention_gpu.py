@@ -9,7 +9,7 @@ from lumen_b200 import functional as F
 from lumen_b200 import tracer
 from lumen_b200._lib import LumenError
 from lumen_b200.runtime import attention_backward, attention_forward, device_status
-from tests.helpers import attention_f64, bf16, run_oracle, to_numpy, to_torch
+from tests.helpers import attention_kernel, attention_f64, bf16, run_oracle, to_numpy, to_torch
 
 pytestmark = pytest.mark.gpu
 
@@ -316,10 +316,17 @@ DECODE_CASES = [((1, 1, 1, 1, 1, 64), False), ((2, 1, 17, 4, 4, 128), True), ((1
                 ((40, 1, 129, 16, 16, 64), True), ((1, 1, 16384, 2, 2, 128), True), ((1, 32, 32, 1, 1, 64), True)]
 
 
-@pytest.mark.parametrize("case", DECODE_CASES)
+# ... that the choice of kernel sends to the one for few rows, with two 16-row tiles (17 to 32 rows per key head)
+TWO_ROW_TILES = [((1, 17, 4000, 2, 2, 64), True), ((1, 32, 16384, 4, 4, 128), True), ((2, 3, 2070, 32, 4, 64), True), ((1, 5, 3001, 5, 1, 128), False),
+                 ((1, 1, 3000, 32, 1, 128), True)]
+
+
+@pytest.mark.parametrize("case", DECODE_CASES + TWO_ROW_TILES)
 def test_few_query_rows_against_float64(cuda, case):
     """The reference's 16-bit tolerance (2e-2), log-sum-exp to 1e-3, on strided views."""
     (b, sq, sk, n, nkv, h), causal = case
+    if case in TWO_ROW_TILES:
+        assert attention_kernel(*case[0], causal) == "few rows"
     q, k, v = qkv(b, sq, sk, n, nkv, h)
     cache = torch.empty((b, sk, 2, nkv, h), dtype=torch.bfloat16, device=cuda)
     cache[:, :, 0], cache[:, :, 1] = to_torch(k, cuda), to_torch(v, cuda)

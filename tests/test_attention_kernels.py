@@ -1,0 +1,31 @@
+"""Which forward kernel a problem takes (no GPU: the choice is arithmetic on sizes)."""
+
+import pytest
+
+from tests.helpers import attention_kernel
+
+# (B, Sq, Sk, N, Nkv, H) and the faster kernel, with the times (us on a B200) of the tile kernel and of the one for few rows
+FEW_ROWS_OR_A_TILE = [
+    ((16, 1, 4097, 32, 8, 128), "few rows"),   # 156 / 43: decoding
+    ((1, 32, 16384, 4, 4, 128), "few rows"),   # 242 / 29: few heads, keys cut into ranges
+    ((32, 4, 4096, 32, 4, 128), "few rows"),   # 296 / 86: a tile per query head reads the keys eight times
+    ((512, 4, 64, 16, 16, 64), "few rows"),    # 143 / 80
+    ((16, 16, 4096, 32, 32, 64), "few rows"),  # 118 / 88
+    ((64, 32, 32, 16, 16, 64), "one tile"),    # 20 / 38: short sequences
+    ((64, 32, 32, 16, 16, 128), "one tile"),   # 23 / 98
+    ((32, 16, 512, 32, 32, 128), "one tile"),  # 55 / 77
+    ((32, 32, 128, 32, 32, 128), "one tile"),  # 23 / 110
+    ((16, 32, 4096, 32, 32, 128), "one tile"),  # 169 / 347
+    ((8, 17, 512, 32, 32, 128), "one tile"),   # 15 / 36
+    ((1, 33, 4096, 1, 1, 64), "one tile"),     # more rows than the kernel has
+]
+
+
+@pytest.mark.parametrize("case,kernel", FEW_ROWS_OR_A_TILE)
+def test_few_rows_take_the_faster_kernel(case, kernel):
+    assert attention_kernel(*case) == kernel
+
+
+def test_what_the_tensor_core_kernels_do_not_take():
+    assert attention_kernel(16, 1, 100, 8, 8, 64, dtype="float32") == "cuda cores"
+    assert attention_kernel(16, 1, 100, 8, 8, 96) == "cuda cores"
