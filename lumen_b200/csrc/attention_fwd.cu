@@ -18,8 +18,10 @@
 // softmax(j) and only P(j) V(j) sits between two softmax passes. Probabilities are rounded to bf16 before the PV product
 // as the traced program does (flash.py:38-45); sums and the output accumulate in fp32. Every barrier wait is bounded.
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 #include <type_traits>
+#include <vector>
 
 #include "attention.h"
 #include "sm100.cuh"
@@ -698,20 +700,59 @@ double one_tile_few_us(const lb_tensor& q, const lb_tensor& k, int sms) {
     return std::max(1.0 + waves * (k.shape[3] == 64 ? 3.5 + 1.4 * tiles : 4.0 + 1.8 * tiles), bytes / 5.4e6);
 }
 
+// Microseconds of a run of CTAs, `slots` of them at a time, (batch, head)s one after the other and the costs of a head's CTAs
+// given: whole waves where all cost the same, else (longest first) the work spread evenly and half a CTA at the end.
+double makespan(double heads, const std::vector<double>& costs, double slots, bool even) {
+    double total = 0.0, longest = 0.0;
+    for (double c : costs) total += c, longest = std::max(longest, c);
+    const double ctas = heads * costs.size();
+    if (even) return std::ceil(ctas / slots) * longest;
+    return std::max(longest, heads * total / slots + (ctas > slots ? 0.5 * total / costs.size() : 0.0));
+}
+// Key tiles that query tile `t` sees.
+long long visible_tiles(const lb_attn_desc& desc, long long Sq, long long Sk, long long t) {
+    const long long last = desc.causal ? std::min(Sk - 1, std::min((t + 1) * BQ, Sq) - 1 + desc.causal_offset) : Sk - 1;
+    return last < 0 ? 0 : last / BKV + 1;
+}
+// Microseconds of the kernels with one and with two query tiles per CTA, for more than one query tile. A CTA costs a constant
+// and so much per key tile (for two tiles: those of the longer and of the shorter range). Fitted to 360 problems of 129 to
+// 4096 queries, 4 to 512 (batch, head)s, with and without a causal mask (root mean square of the error 3 to 7 %).
+double one_tile_us(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, int sms) {
+    const bool wide = q.shape[3] == 128;
+    const double start = wide ? (desc.causal ? 0.90 : 2.11) : 3.05, base = wide ? 5.9 : 3.24, per_tile = wide ? (desc.causal ? 2.34 : 1.98) : 1.89;
+    std::vector<double> costs;
+    for (long long t = 0; t < (q.shape[1] + BQ - 1) / BQ; t++) costs.push_back(base + per_tile * visible_tiles(desc, q.shape[1], k.shape[1], t));
+    return start + makespan((double)q.shape[0] * q.shape[2], costs, 2.0 * sms, !desc.causal);
+}
+double two_tiles_us(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, int sms) {
+    const bool wide = q.shape[3] == 128;
+    const double start = wide ? (desc.causal ? 4.33 : 4.77) : 5.06, base = wide ? (desc.causal ? 5.13 : 4.57) : 2.36;
+    const double longer = wide ? (desc.causal ? 1.16 : 0.916) : 1.22, shorter = wide ? (desc.causal ? 0.76 : 0.916) : 0.525;
+    const long long tiles = (q.shape[1] + BQ - 1) / BQ;
+    std::vector<double> costs;
+    for (long long t = 0; t < tiles; t += 2) {
+        const long long a = visible_tiles(desc, q.shape[1], k.shape[1], t), b = t + 1 < tiles ? visible_tiles(desc, q.shape[1], k.shape[1], t + 1) : 0;
+        costs.push_back(base + longer * std::max(a, b) + shorter * std::min(a, b));
+    }
+    return start + makespan((double)q.shape[0] * q.shape[2], costs, sms, !desc.causal);
+}
+
 // The kernel for operands that the tensor-core kernels take, by the modelled times of the two that come into question.
 //  * Few rows per key head: the tile kernel has a CTA per query head however many rows of its 128 are live, the other shares
 //    the keys among a group's heads and cuts them into ranges, at a cost per row. Of 1373 timed problems the choice is 0.3 % off
 //    the better kernel on average; always taking the second, as before, was up to 5.6 times slower (4096 heads of 32 queries
 //    and 128 keys at head dim 128: 84 -> 439 us), never taking it 10 times (8 heads of 4 queries and 13568 keys).
-AttentionKernel choose_kernel(const lb_tensor& q, const lb_tensor& k, int sms) {
+//  * One query tile per CTA and two CTAs per SM, or two tiles per CTA: the second needs more tiles than the first takes at once, both
+//    tiles of a CTA to have rows, and at head dim 64, where the first overlaps S with the softmax as well, a causal mask: without one
+//    it was 10 % slower on average, at best 6 % faster. Of the 360 problems the choice is 0.6 % off the better kernel on average, by
+//    the number of tiles alone 3 % (16 x 16 heads at head dim 128, causal: 257 queries 30 us with one tile, 41 with two, 4096 queries
+//    1438 and 1050). Beyond 32 query tiles the ends of a run no longer matter.
+AttentionKernel choose_kernel(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, int sms) {
     if (attention_decodes(q, k) && attention_decode_us(q, k, sms) < one_tile_few_us(q, k, sms)) return ATTN_FEW_ROWS;
-    // Which kernel (measured, us, one tile per CTA -> two): the second has half the CTAs, so it needs enough of them to fill
-    // the GPU - 4 heads x 4096 at head dim 128: 62 -> 64, 2 x 8 x 1024: 21 -> 23, 32 heads x 4096: 180 -> 130 - and a query
-    // length that gives the second tile rows (8 x 32 x 100 against 4000: 93 -> 115). From two CTAs per SM of the first
-    // kernel on it is ahead at head dim 128 (4 x 16 x 1000: 47 -> 45); at head dim 64, where the one-tile kernel overlaps S
-    // with the softmax as well, from four (4 x 16 x 1000: 40 -> 41, 2 x 32 x 1531: 55 -> 49, 32 x 4096: 144 -> 118).
-    const long long tiles = (q.shape[1] + BQ - 1) / BQ * q.shape[2] * q.shape[0];
-    return q.shape[1] > BQ && tiles > (q.shape[3] == 128 ? 2LL : 4LL) * sms ? ATTN_TWO_TILES : ATTN_ONE_TILE;
+    const long long tiles = q.shape[0] * q.shape[2] * ((q.shape[1] + BQ - 1) / BQ);
+    if (q.shape[1] <= BQ || tiles <= 2LL * sms || (q.shape[3] == 64 && !desc.causal)) return ATTN_ONE_TILE;
+    if (q.shape[1] > 32 * BQ) return ATTN_TWO_TILES;
+    return two_tiles_us(desc, q, k, sms) < one_tile_us(desc, q, k, sms) ? ATTN_TWO_TILES : ATTN_ONE_TILE;
 }
 }  // namespace
 
@@ -731,7 +772,7 @@ void attention_fwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor
     if (!(desc.scale > 0.0f)) fail(LB_ERR_UNSUPPORTED, "attention: the softmax scale must be positive");
     if (B == 0 || Sq == 0 || N == 0) return;
     driver();
-    const AttentionKernel kernel = choose_kernel(q, k, device_info().sms);
+    const AttentionKernel kernel = choose_kernel(desc, q, k, device_info().sms);
     if (kernel == ATTN_FEW_ROWS) {
         attention_decode(desc, q, k, v, o, lse, stream);
         return;
@@ -781,9 +822,9 @@ bool attention_on_tensor_cores(const lb_tensor& q, const lb_tensor& k, const lb_
     return ok(q) && ok(k) && ok(v) && (q.shape[3] == 64 || q.shape[3] == 128) && v.shape[3] == q.shape[3];
 }
 
-AttentionKernel attention_forward_kernel(const lb_tensor& q, const lb_tensor& k, const lb_tensor& v) {
+AttentionKernel attention_forward_kernel(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v) {
     if (q.rank != 4 || k.rank != 4 || v.rank != 4) fail(LB_ERR_INVALID, "attention: operands must be [B, S, N, H] tensors");
-    return attention_on_tensor_cores(q, k, v) ? choose_kernel(q, k, sm_count_hint()) : ATTN_CUDA_CORES;
+    return attention_on_tensor_cores(q, k, v) ? choose_kernel(desc, q, k, sm_count_hint()) : ATTN_CUDA_CORES;
 }
 
 void attention_forward(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o,
@@ -804,6 +845,6 @@ extern "C" int lb_attention_fwd(const lb_attn_desc* desc, const lb_tensor* q, co
 extern "C" int lb_attention_fwd_kernel(const lb_attn_desc* desc, const lb_tensor* q, const lb_tensor* k, const lb_tensor* v, int32_t* kernel) {
     return lb::guarded([&] {
         if (!desc || !q || !k || !v || !kernel) lb::fail(LB_ERR_INVALID, "lb_attention_fwd_kernel: null argument");
-        *kernel = lb::attention_forward_kernel(*q, *k, *v);
+        *kernel = lb::attention_forward_kernel(*desc, *q, *k, *v);
     });
 }

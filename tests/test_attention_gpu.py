@@ -366,11 +366,18 @@ PAIR_CASES = [((20, 129, 129, 16, 4, 128), True), ((10, 257, 257, 16, 16, 128), 
               ((20, 129, 129, 32, 4, 64), True), ((10, 257, 257, 32, 16, 64), False), ((4, 300, 500, 64, 8, 64), True), ((2, 1100, 1100, 40, 8, 64), True)]
 
 
-@pytest.mark.parametrize("case", PAIR_CASES)
+# ... that the choice of kernel sends to the two-tile kernel
+TWO_TILE_CASES = [((20, 129, 129, 32, 4, 64), True), ((4, 385, 500, 40, 8, 64), True), ((1, 1200, 1337, 40, 8, 64), True), ((20, 255, 255, 16, 4, 128), False),
+                  ((2, 639, 777, 64, 8, 128), False), ((1, 1024, 1024, 40, 8, 128), True), ((40, 129, 513, 16, 4, 128), True)]
+
+
+@pytest.mark.parametrize("case", PAIR_CASES + TWO_TILE_CASES)
 def test_two_tile_forward_against_float64(cuda, case):
     """The reference's 16-bit tolerance (2e-2), log-sum-exp to 1e-3. Later keys have larger scores, so that the reference
     maximum is raised on the way (a factor of 2^8 between raises), and the result repeats bit for bit."""
     (b, sq, sk, n, nkv, h), causal = case
+    if case in TWO_TILE_CASES:
+        assert attention_kernel(*case[0], causal) == "two tiles"
     q, k, v = qkv(b, sq, sk, n, nkv, h)
     k = bf16(k.astype(np.float32) * np.linspace(0.1, 6.0, sk, dtype=np.float32)[None, :, None, None])
     tq, tk, tv = (to_torch(a, cuda) for a in (q, k, v))
@@ -477,3 +484,16 @@ def test_attention_without_keys_is_refused(cuda, sq):
     q, k = (torch.zeros((1, s, 2, 64), dtype=torch.bfloat16, device=cuda) for s in (sq, 0))
     with pytest.raises(LumenError):
         attention_forward(q, k, k)
+
+
+def test_two_tiles_rows_that_see_no_key_and_rows_of_nan(cuda):
+    """As the test above, on a problem that the two-tile kernel takes."""
+    assert attention_kernel(12, 400, 300, 32, 32, 128) == "two tiles"
+    q, k, v = (to_torch(a, cuda) for a in qkv(12, 400, 300, 32, 32, 128))
+    o, lse = attention_forward(q, k, v, causal=True)
+    device_status()
+    assert torch.isnan(o[:, :100]).all() and not torch.isnan(o[:, 100:]).any() and not torch.isnan(lse[..., 100:]).any()
+    k[:, 150] = float("nan")
+    o, _ = attention_forward(q, k, v, causal=True)
+    device_status()
+    assert torch.isnan(o[:, 250:]).all() and not torch.isnan(o[:, 100:250]).any()

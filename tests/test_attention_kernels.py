@@ -26,6 +26,26 @@ def test_few_rows_take_the_faster_kernel(case, kernel):
     assert attention_kernel(*case) == kernel
 
 
+# (B, Sq, Sk, N, Nkv, H), causal, the faster kernel, and the times with one and with two tiles per CTA
+ONE_OR_TWO_TILES = [
+    ((16, 4096, 4096, 16, 16, 128), True, "two tiles"),   # 1438 / 1050
+    ((8, 4096, 4096, 16, 16, 64), True, "two tiles"),     # 469 / 423
+    ((2, 1531, 1531, 32, 8, 128), True, "two tiles"),     # 77 / 59
+    ((4, 2048, 2048, 16, 16, 128), False, "two tiles"),
+    ((16, 257, 257, 16, 16, 128), True, "one tile"),      # 30 / 41: the second tile of every other CTA has one row
+    ((16, 300, 500, 16, 16, 64), False, "one tile"),      # 34 / 43
+    ((2, 4096, 4096, 16, 16, 64), False, "one tile"),     # 206 / 224
+    ((2, 1100, 1100, 16, 16, 128), True, "one tile"),     # 25 / 31: fewer tiles than the first kernel takes at once
+    ((64, 128, 4096, 32, 32, 128), False, "one tile"),    # no second tile
+    ((1, 1 << 20, 1 << 20, 1, 1, 128), True, "two tiles"),
+]
+
+
+@pytest.mark.parametrize("case,causal,kernel", ONE_OR_TWO_TILES)
+def test_one_or_two_tiles_by_the_faster(case, causal, kernel):
+    assert attention_kernel(*case, causal) == kernel
+
+
 def test_what_the_tensor_core_kernels_do_not_take():
     assert attention_kernel(16, 1, 100, 8, 8, 64, dtype="float32") == "cuda cores"
     assert attention_kernel(16, 1, 100, 8, 8, 96) == "cuda cores"
