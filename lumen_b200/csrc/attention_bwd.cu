@@ -130,21 +130,23 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
     const int group = p.N / p.Nkv;
     const int r0 = tile * BR;
 
-    // streamed range: [t_begin, t_end) in units of BT rows, per head; heads_here heads are walked in dkdv mode
-    int t_begin, t_end, heads_here;
+    // streamed rows, per head: tiles of BT from stream0 on; heads_here heads are walked in dkdv mode. Whole blocks of 64 rows that
+    // no resident row sees (or that see none) are left out at either tile height: their weights would be 0, but 0 times a NaN is not.
+    int stream0, per_head, heads_here;
     if (DKDV) {
         // queries that see at least the first key of this tile: i >= r0 - offset
-        long long first_q = p.causal ? max(0LL, (long long)r0 - p.causal_offset) : 0LL;
-        t_begin = (int)(first_q / BT);
-        t_end = (p.Sq + BT - 1) / BT;
+        const long long first_q = p.causal ? min((long long)p.Sq, max(0LL, (long long)r0 - p.causal_offset)) : 0LL;
+        stream0 = (int)(first_q / 64) * 64;
+        per_head = (p.Sq - stream0 + BT - 1) / BT;
+        if (first_q >= p.Sq) per_head = 0;
         heads_here = group;
     } else {
-        long long last_key = p.causal ? min((long long)p.Sk - 1, (long long)r0 + BR - 1 + p.causal_offset) : (long long)p.Sk - 1;
-        t_begin = 0;
-        t_end = last_key < 0 ? 0 : (int)(last_key / BT) + 1;
+        const long long last_key = p.causal ? min((long long)p.Sk - 1, (long long)r0 + BR - 1 + p.causal_offset) : (long long)p.Sk - 1;
+        const int blocks = last_key < 0 ? 0 : (int)(last_key / 64) + 1;
+        stream0 = BT == 128 && blocks % 2 ? -64 : 0;  // an odd block: the first tile starts before the keys (TMA reads zeros there)
+        per_head = (blocks * 64 - stream0) / BT;
         heads_here = 1;
     }
-    const int per_head = max(t_end - t_begin, 0);
     const int n_iter = per_head * heads_here;
     const int r_head = head;                          // resident tiles: kv head (dkdv) / query head (dq)
     const int kv_head_of_q = DKDV ? head : head / group;
@@ -205,14 +207,14 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
             for (int it = 0; it < n_iter && ok; it++) {
                 const int a = it % S1, b = it % S2;
                 const int hh = it / per_head;
-                const int t = t_begin + it - hh * per_head;
+                const int row0 = stream0 + (it - hh * per_head) * BT;
                 const int t_head = DKDV ? head * group + hh : kv_head_of_q;
                 if (!(ok = mbar_wait(&t1_empty[a], ((uint32_t)(it / S1) & 1) ^ 1, abort_flag))) break;
                 mbar_expect_tx(&t1_full[a], kStream);
-                for (int d = 0; d < DB; d++) tma_load_4d(st1 + a * kStream + d * kTBlock, &map_t1, &t1_full[a], d * 64, t_head, t * BT, batch);
+                for (int d = 0; d < DB; d++) tma_load_4d(st1 + a * kStream + d * kTBlock, &map_t1, &t1_full[a], d * 64, t_head, row0, batch);
                 if (!(ok = mbar_wait(&t2_empty[b], ((uint32_t)(it / S2) & 1) ^ 1, abort_flag))) break;
                 mbar_expect_tx(&t2_full[b], kStream);
-                for (int d = 0; d < DB; d++) tma_load_4d(st2 + b * kStream + d * kTBlock, &map_t2, &t2_full[b], d * 64, t_head, t * BT, batch);
+                for (int d = 0; d < DB; d++) tma_load_4d(st2 + b * kStream + d * kTBlock, &map_t2, &t2_full[b], d * 64, t_head, row0, batch);
             }
         }
       } else if (warp == 1) {
@@ -307,7 +309,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
         auto fetch_stats = [&](int it) {
             const int hh = it / per_head;
             const long long at = ((long long)batch * p.N + (head * group + hh)) * p.Sq;
-            const long long c = (long long)(t_begin + it - hh * per_head) * BT + wg * COLS + lane;
+            const long long c = stream0 + (long long)(it - hh * per_head) * BT + wg * COLS + lane;
 #pragma unroll
             for (int u = 0; u < COLS / 32; u++) {
                 const long long cc = min(c + 32 * u, (long long)p.Sq - 1);
@@ -322,8 +324,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
         for (int it = 0; it < n_iter && ok; it++) {
             const uint32_t par = (uint32_t)it & 1;
             const int hh = it / per_head;
-            const int t = t_begin + it - hh * per_head;
-            const long long c0 = (long long)t * BT + wg * COLS;  // this thread's first streamed index: query (dkdv) or key (dq)
+            const long long c0 = stream0 + (long long)(it - hh * per_head) * BT + wg * COLS;  // this thread's first streamed index: query (dkdv) or key (dq)
             if (DKDV) {
                 // each warp stages its columns' log-sum-exps and deltas once; its lanes then read them as shared-memory
                 // broadcasts instead of two global loads per score

@@ -497,3 +497,22 @@ def test_two_tiles_rows_that_see_no_key_and_rows_of_nan(cuda):
     o, _ = attention_forward(q, k, v, causal=True)
     device_status()
     assert torch.isnan(o[:, 250:]).all() and not torch.isnan(o[:, 100:250]).any()
+
+
+@pytest.mark.parametrize("h", [64, 128])
+def test_backward_leaves_blocks_behind_the_mask_out(cuda, h):
+    """Blocks of 64 rows that a tile of 128 does not see at all (more keys than queries, so that the mask's edge lies 64 off the
+    tiles) do not enter it: a NaN there changes no bit of its gradients."""
+    q, k, v, do = (to_torch(bf16(np.random.default_rng(i).standard_normal((1, s, 2, h))), cuda) for i, s in enumerate((200, 264, 264, 200)))
+    o, lse = attention_forward(q, k, v, causal=True)
+    dq, dk, dv = attention_backward(q, k, v, o, do, lse, causal=True)
+    for name in ("q", "do"):
+        t = {"q": q.clone(), "do": do.clone()}
+        t[name][:, 10] = float("nan")  # sees keys up to 74: the second tile of keys starts at 128
+        _, dk2, dv2 = attention_backward(t["q"], k, v, o, t["do"], lse, causal=True)
+        assert torch.equal(dk2[:, 128:], dk[:, 128:]) and torch.equal(dv2[:, 128:], dv[:, 128:])
+    k2 = k.clone()
+    k2[:, 200] = float("nan")  # seen from query 136 on: the first tile of queries ends at 127
+    dq2, _, _ = attention_backward(q, k2, v, o, do, lse, causal=True)
+    device_status()
+    assert torch.equal(dq2[:, :128], dq[:, :128]) and torch.isnan(dq2[:, 136:]).all()
