@@ -55,6 +55,8 @@ constexpr int BR = 128;  // resident rows (thread = row)
 //  the two-buffer form this replaces had, on alternating warpgroups - paid for 128: the tensor unit was busy for 67 %
 //  of the kernels' time at 41 % of its rate. Batch 8, 32 heads, sequence 4096, causal: backward 4.66 -> 3.48 ms
 //  (790 TFLOP/s), of which 0.26 came from issuing the products warp-wide.
+//  BT = 64 at head dim 128: one, three or five blocks of 64 streamed rows, which 128-row tiles would fill to a half at the end
+//  (launch_bwd).
 //  BT = 64 (head dim 64): 256 columns and half the shared memory, so that TWO CTAs share an SM and one CTA's prologue,
 //  epilogue and element-wise latency are covered by the other's products (128 and one CTA: 470 -> 548 us at batch 8,
 //  16 heads, sequence 2048).
@@ -75,7 +77,7 @@ struct BwdArgs {
 
 template <int D, bool DKDV, int BT>
 struct BwdConfig {
-    static constexpr int kCtas = BT == 64 ? 2 : 1;       // per SM
+    static constexpr int kCtas = D == 64 ? 2 : 1;        // per SM
     static constexpr int kFirst = BT == 64 ? 2 : 4;      // first compute warp (register budgets are set per aligned group of four warps)
     static constexpr int kThreads = 32 * kFirst + 256;
     static constexpr int kTmemCols = 512 / kCtas;
@@ -552,30 +554,41 @@ template <int D, bool DKDV, int BT>
 void launch_bwd_kernel(const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap& t1, const CUtensorMap& t2, dim3 grid, const BwdArgs& p,
                        cudaStream_t s) {
     using C = BwdConfig<D, DKDV, BT>;
-    static const int regs = launch_regs((const void*)attention_bwd_kernel<D, DKDV, BT>);
-    if (BT == 128 && regs != C::kLaunchRegs)
-        fail(LB_ERR_UNSUPPORTED, format("attention backward: the kernel was built with %d registers per thread, its register budgets assume %d",
-                                        regs, C::kLaunchRegs));
     if (first_use_on_device((const void*)attention_bwd_kernel<D, DKDV, BT>))
         LB_CUDA(cudaFuncSetAttribute(attention_bwd_kernel<D, DKDV, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kBytes));
     attention_bwd_kernel<D, DKDV, BT><<<grid, C::kThreads, C::kBytes, s>>>(r1, r2, t1, t2, p);
 }
 
-// The two kernels; `rows` makes the map of an operand's tiles, 128 or 64 rows high.
+// The two kernels; `rows` makes the map of an operand's tiles, 128 or 64 rows high. Head dim 64 streams 64 rows a tile. Head dim 128
+// streams 128, but 64 where the streamed rows are one, three or five blocks of 64: the last 128-row tile would be half empty, which
+// shows while tiles are few. Measured (us, 128 rows a tile -> 64 for dK/dV and dQ together), 64 x 4 heads: 16 rows 23.4 -> 17.4 and,
+// one head to a key head, 16.9 -> 13.7; 160 rows 32.8 -> 28.9, 21.3 -> 19.0; 320 rows 49.0 -> 45.6; two and four blocks are as fast or
+// faster with 128 (128 rows 21.6 -> 22.0, 256 30.7 -> 33.5). The 64-row form also stands in where the compiler did not assign the
+// registers that the budgets of the 128-row form (setmaxnreg) are drawn from.
+template <int D, class Rows>
+void launch_bwd_pair(const Rows& rows, const lb_tensor& q, const lb_tensor& d_o, const lb_tensor& k, const lb_tensor& v, const BwdArgs& dkdv,
+                     const BwdArgs& dq, cudaStream_t s) {
+    const CUtensorMap mq = rows(q, "query", 128), mdo = rows(d_o, "dO", 128), mk = rows(k, "key", 128), mv = rows(v, "value", 128);
+    const dim3 grid_kv((unsigned)((dkdv.Sk + BR - 1) / BR), (unsigned)dkdv.Nkv, (unsigned)dkdv.B);
+    const dim3 grid_q((unsigned)((dq.Sq + BR - 1) / BR), (unsigned)dq.N, (unsigned)dq.B);
+    bool tall_kv = false, tall_q = false;  // 128 streamed rows a tile
+    if constexpr (D == 128) {
+        static const bool budgets = launch_regs((const void*)attention_bwd_kernel<128, true, 128>) >= BwdConfig<128, true, 128>::kLaunchRegs &&
+                                    launch_regs((const void*)attention_bwd_kernel<128, false, 128>) >= BwdConfig<128, false, 128>::kLaunchRegs;
+        auto tall = [&](int streamed) { return budgets && ((streamed + 63) / 64 % 2 == 0 || streamed > 5 * 64); };
+        tall_kv = tall(dkdv.Sq), tall_q = tall(dq.Sk);
+        if (tall_kv) launch_bwd_kernel<128, true, 128>(mk, mv, mq, mdo, grid_kv, dkdv, s);
+    }
+    if (!tall_kv) launch_bwd_kernel<D, true, 64>(mk, mv, rows(q, "query", 64), rows(d_o, "dO", 64), grid_kv, dkdv, s);
+    if constexpr (D == 128)
+        if (tall_q) launch_bwd_kernel<128, false, 128>(mq, mdo, mk, mv, grid_q, dq, s);
+    if (!tall_q) launch_bwd_kernel<D, false, 64>(mq, mdo, rows(k, "key", 64), rows(v, "value", 64), grid_q, dq, s);
+}
 template <class Rows>
 void launch_bwd(long long D, const Rows& rows, const lb_tensor& q, const lb_tensor& d_o, const lb_tensor& k, const lb_tensor& v, const BwdArgs& dkdv,
                 const BwdArgs& dq, cudaStream_t s) {
-    const CUtensorMap mq128 = rows(q, "query", 128), mdo128 = rows(d_o, "dO", 128), mk128 = rows(k, "key", 128), mv128 = rows(v, "value", 128);
-    const dim3 grid_kv((unsigned)((dkdv.Sk + BR - 1) / BR), (unsigned)dkdv.Nkv, (unsigned)dkdv.B);
-    const dim3 grid_q((unsigned)((dq.Sq + BR - 1) / BR), (unsigned)dq.N, (unsigned)dq.B);
-    if (D == 128) {
-        launch_bwd_kernel<128, true, 128>(mk128, mv128, mq128, mdo128, grid_kv, dkdv, s);
-        launch_bwd_kernel<128, false, 128>(mq128, mdo128, mk128, mv128, grid_q, dq, s);
-    } else {
-        const CUtensorMap mq64 = rows(q, "query", 64), mdo64 = rows(d_o, "dO", 64), mk64 = rows(k, "key", 64), mv64 = rows(v, "value", 64);
-        launch_bwd_kernel<64, true, 64>(mk128, mv128, mq64, mdo64, grid_kv, dkdv, s);
-        launch_bwd_kernel<64, false, 64>(mq128, mdo128, mk64, mv64, grid_q, dq, s);
-    }
+    if (D == 128) launch_bwd_pair<128>(rows, q, d_o, k, v, dkdv, dq, s);
+    else launch_bwd_pair<64>(rows, q, d_o, k, v, dkdv, dq, s);
 }
 
 }  // namespace

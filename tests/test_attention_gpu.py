@@ -343,7 +343,12 @@ TILE_EDGE_CASES = [((1, 129, 129, 1, 1, 128), True), ((1, 1, 129, 2, 1, 128), Fa
                    ((2, 900, 1030, 4, 2, 128), True), ((1, 40, 400, 1, 1, 128), True)]
 
 
-@pytest.mark.parametrize("case", TILE_EDGE_CASES)
+# ... and those of its 64-row tiles, which one, three and five blocks of 64 streamed rows take on either side
+SHORT_CASES = [((1, 1, 1, 1, 1, 128), False), ((2, 64, 64, 4, 1, 128), True), ((1, 65, 64, 2, 2, 128), False), ((2, 129, 130, 4, 2, 128), True), ((1, 192, 320, 2, 1, 128), True),
+               ((1, 320, 300, 4, 4, 128), False), ((1, 321, 384, 1, 1, 128), True), ((3, 20, 500, 8, 2, 128), True)]
+
+
+@pytest.mark.parametrize("case", TILE_EDGE_CASES + SHORT_CASES)
 def test_backward_tile_edges_against_float64(cuda, case):
     """The reference's 16-bit tolerance (2e-2 of the value and of the largest), bit-identical from run to run."""
     (b, sq, sk, n, nkv, h), causal = case
