@@ -651,13 +651,15 @@ attention_fwd_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     }
 }
 
+// Whether the register budgets of the two-tile kernel (setmaxnreg) can be drawn from what the compiler assigned to it.
+template <int D>
+bool pair_has_registers() {
+    static const bool enough = launch_regs((const void*)attention_fwd_pair_kernel<D>) >= kPairLaunchRegs;
+    return enough;
+}
 template <int D>
 void launch_fwd_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, FwdArgs p, cudaStream_t s) {
     constexpr int kBytes = FwdPairSmem<D>::kBytes;
-    static const int regs = launch_regs((const void*)attention_fwd_pair_kernel<D>);
-    if (regs != kPairLaunchRegs)
-        fail(LB_ERR_UNSUPPORTED, format("attention: the two-tile forward kernel was built with %d registers per thread, its register budgets "
-                                        "assume %d", regs, kPairLaunchRegs));
     if (first_use_on_device((const void*)attention_fwd_pair_kernel<D>))
         LB_CUDA(cudaFuncSetAttribute(attention_fwd_pair_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes));
     p.tiles = (p.Sq + 2 * BQ - 1) / (2 * BQ);
@@ -788,7 +790,7 @@ void attention_fwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor
     p.status = status_word();
     dim3 grid((unsigned)((Sq + BQ - 1) / BQ), (unsigned)N, (unsigned)B);
     cudaStream_t s = (cudaStream_t)stream;
-    if (kernel == ATTN_TWO_TILES) {
+    if (kernel == ATTN_TWO_TILES && (D == 128 ? pair_has_registers<128>() : pair_has_registers<64>())) {  // else the one-tile kernel does as well
         if (D == 128) launch_fwd_pair<128>(mq, mk, mv, p, s);
         else launch_fwd_pair<64>(mq, mk, mv, p, s);
         LB_CUDA(cudaGetLastError());

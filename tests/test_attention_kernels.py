@@ -49,3 +49,19 @@ def test_one_or_two_tiles_by_the_faster(case, causal, kernel):
 def test_what_the_tensor_core_kernels_do_not_take():
     assert attention_kernel(16, 1, 100, 8, 8, 64, dtype="float32") == "cuda cores"
     assert attention_kernel(16, 1, 100, 8, 8, 96) == "cuda cores"
+
+
+@pytest.mark.parametrize("source,kernel,registers,count", [("attention_fwd", "attention_fwd_pair_kernel", 168, 2), ("attention_bwd", "attention_bwd_kernelILi128ELb[01]ELi128E", 168, 2),
+                                                           ("attention_bwd_atomic", "attention_bwd_atomic_kernel", 128, 1)])
+def test_kernels_with_register_budgets_have_the_registers_they_divide(source, kernel, registers, count):
+    """Budgets (setmaxnreg) add up to what a block is launched with. Another compiler may assign another number: the library then
+    takes its other kernels (or refuses, for the single-kernel backward), which is slower; this is where that shows."""
+    import os
+    import re
+
+    log = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "lumen_b200", "csrc", "build", source + ".ptxas.log")
+    if not os.path.exists(log):
+        pytest.skip("the library was not built here")
+    entries = re.findall(r"Compiling entry function '(\S+)'.*?Used (\d+) registers", open(log).read(), flags=re.S)
+    used = [int(n) for name, n in entries if re.search(kernel, name)]
+    assert used == [registers] * count
