@@ -10,7 +10,7 @@ Every rewrite here leaves each remaining value bit-identical when the graph is e
   pass re-traces broadcasts, iotas and constants the forward already has);
 * `simplify`: `reshape` to the operand's own shape, `transpose` by the identity, `cast` to the operand's own dtype and
   `broadcast_in_dim` to the same shape are removed; a transpose of a transpose becomes one; a reshape of a reshape
-  becomes one; the transpose of a product used nowhere else becomes the product of the swapped operands;
+  becomes one; the transpose of a 16-bit product of two matrices used nowhere else becomes the product of the swapped operands;
   `cast(dot_general(..), t)` with the product used nowhere else becomes the product's `output_dtype`
   (the accumulator is rounded once either way).
 """
@@ -117,8 +117,9 @@ def simplify(graph: G.Graph) -> G.Graph:
             second = tuple(n.params["permutation"])
             n = G.Node("transpose", (src(inner.inputs[0]),), n.output, {"permutation": tuple(first[p] for p in second)})
         elif (n.op == "transpose" and tuple(n.params["permutation"]) == (1, 0) and inner is not None and inner.op == "dot_general"
-              and uses.get(inner.output, 0) == 1 and types[inner.inputs[0]].dtype in ("bfloat16", "float16") and inner in nodes):
-            # a transposed product (a weight gradient) is the product of the swapped operands: the same sums of the same
+              and uses.get(inner.output, 0) == 1 and types[inner.inputs[0]].dtype in ("bfloat16", "float16") and inner in nodes
+              and all(len(types[v].shape) == 2 for v in inner.inputs) and not inner.params["lhs_batch"]):
+            # a transposed product of two matrices (a weight gradient) is the product of the swapped operands: the same sums of the same
             # products in the same order, without a pass over the result. 16-bit operands only: at 1024 x 4096 the pass
             # took as long as half the tensor-core product; beside a CUDA-core product of float32 it does not show.
             at = nodes.index(inner)
