@@ -132,8 +132,8 @@ class Compiled:
         else:
             bound = sig.plan.bind(inputs, sig.results)
             sig.plan.run_bound(bound)
-            if self.use_graphs and sig.bound_to == pointers:
-                sig.recorded = sig.plan.record(bound)  # second call with these pointers: record for the next ones
+            # second call with these pointers: record for the next ones (a recording of other memory is dropped)
+            sig.recorded = sig.plan.record(bound) if self.use_graphs and sig.bound_to == pointers else None
             sig.bound_to, sig.keep = pointers, (inputs, bound)
         return sig.returned
 

@@ -155,3 +155,11 @@ def test_compile_takes_dlpack_arrays_in_place(cuda):
     got = f(Foreign(x), Foreign(y))
     torch.testing.assert_close(got, torch.relu(x - y), rtol=0, atol=0)
     assert f.latest.keep[0][0].data_ptr() == x.data_ptr()
+
+
+def test_a_recorded_call_is_not_replayed_for_other_memory(cuda):
+    """With `use_graphs` a call that returns to other argument memory runs on that memory, from its first call there on."""
+    f = lumen_b200.compile(lambda x: x + x, use_graphs=True)
+    a, b = (torch.full((64, 64), v, device=cuda) for v in (1.0, 10.0))
+    for x in (a, a, a, b, b, b, b, a, b, a, a, a, a):
+        assert torch.equal(f(x), x + x)
