@@ -131,4 +131,4 @@ def dense(ptr: int, dtype: str, shape) -> LbTensor:
 
 
 def strided(ptr: int, dtype: str, shape, strides) -> LbTensor:
-    return LbTensor(ptr, DTYPE_CODES[dtype], len(shape), shape, strides)  # array fields take tuples of up to MAX_RANK numbers
+    return LbTensor(ptr, DTYPE_CODES[dtype], len(shape), tuple(shape), tuple(strides))  # array fields take tuples of up to MAX_RANK numbers

@@ -53,16 +53,18 @@ bool read_pointer(PyObject* t, void** out) {
     return !PyErr_Occurred();
 }
 
-// A tuple of at most LB_MAX_RANK integers.
+// A sequence of at most LB_MAX_RANK integers (a tuple, as torch and this package give it, or what another framework does).
+// Steals the reference.
 bool read_longs(PyObject* tuple, int64_t* out, int32_t* count, const char* what) {
     bool ok = false;
-    if (tuple && PyTuple_Check(tuple) && PyTuple_GET_SIZE(tuple) <= LB_MAX_RANK) {
+    if (tuple && !PyTuple_Check(tuple)) Py_SETREF(tuple, PySequence_Tuple(tuple));
+    if (tuple && PyTuple_GET_SIZE(tuple) <= LB_MAX_RANK) {
         *count = (int32_t)PyTuple_GET_SIZE(tuple);
         ok = true;
         for (int32_t k = 0; k < *count; k++) out[k] = PyLong_AsLongLong(PyTuple_GET_ITEM(tuple, k));
         if (PyErr_Occurred()) ok = false;
     } else if (tuple) {
-        PyErr_Format(PyExc_TypeError, "a tensor's %s must be a tuple of at most %d integers", what, LB_MAX_RANK);
+        PyErr_Format(PyExc_TypeError, "a tensor's %s must be at most %d integers", what, LB_MAX_RANK);
     }
     Py_XDECREF(tuple);
     return ok;
