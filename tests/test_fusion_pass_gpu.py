@@ -159,6 +159,8 @@ def test_compile_takes_dlpack_arrays_in_place(cuda):
 
 def test_a_recorded_call_is_not_replayed_for_other_memory(cuda):
     """With `use_graphs` a call that returns to other argument memory runs on that memory, from its first call there on."""
+    import lumen_b200
+
     f = lumen_b200.compile(lambda x: x + x, use_graphs=True)
     a, b = (torch.full((64, 64), v, device=cuda) for v in (1.0, 10.0))
     for x in (a, a, a, b, b, b, b, a, b, a, a, a, a):
