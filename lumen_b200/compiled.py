@@ -76,6 +76,7 @@ class _Signature:
         self.results = [_empty_like_input(like, self.graph.types[v].shape, self.graph.types[v].dtype) for v in self.graph.outputs]
         self.recorded = None
         self.bound_to = None
+        self.native = set()  # the argument types with which calls run natively
         self.returned = self.results[0] if len(self.results) == 1 else tuple(self.results)
 
 
@@ -120,8 +121,9 @@ class Compiled:
         sig = self.signatures.get(key)
         if sig is None:
             sig = self.signatures[key] = _Signature(self.fn, args, self.device, self.lowering)
-            if not self.use_graphs and len(inputs) == len(args):
-                self._add(sig, inputs)
+        kinds = tuple(type(a) for a in inputs)
+        if kinds not in sig.native and not self.use_graphs and len(inputs) == len(args):
+            self._add(sig, kinds, inputs)
         self.calls.latest = sig
         for k, a in enumerate(inputs):
             if _tensor_types[type(a)] and not (_on_current_gpu(a, self.device) and a.is_contiguous()):
@@ -137,8 +139,9 @@ class Compiled:
             sig.bound_to, sig.keep = pointers, (inputs, bound)
         return sig.returned
 
-    def _add(self, sig, inputs):
+    def _add(self, sig, kinds, inputs):
         """Calls with arguments like these from now on run natively."""
+        sig.native.add(kinds)
         torches = tuple(_tensor_types[type(a)] for a in inputs)
         if any(torches):
             torch = sys.modules["torch"]

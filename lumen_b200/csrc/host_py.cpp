@@ -8,7 +8,10 @@
 #include <Python.h>
 #include <structmember.h>
 
+#include <algorithm>
 #include <deque>
+#include <new>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/lumen_b200.h"
@@ -185,17 +188,19 @@ PyObject* gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // ---- the calls of one compiled function -----------------------------------------------------------------------------
-// The signatures a `lumen_b200.compile`d function has met whose arguments are all tensors. `call(args, stream)` finds
-// the one that `args` match, runs its plan and returns its results; it returns None when the call needs the general
-// path (an unknown signature, host or strided or foreign arguments).
+// The signatures a `lumen_b200.compile`d function has met whose arguments are all tensors, by a hash of the arguments' types,
+// dtypes and shapes: a call costs the same with one signature as with thousands (a cache that grows by a token a
+// call). `call(args, stream, device)` finds the one that `args` match, runs its plan and returns its results; it returns None
+// when the call needs the general path (an unknown signature, host or strided or foreign arguments).
 struct Arg {
-    PyObject* type;   // exact type met
-    PyObject* dtype;  // the dtype attribute met
-    bool torch;       // a torch tensor: has to be on the GPU and contiguous
-    std::vector<int64_t> shape;
+    PyObject* type;   // exact type
+    PyObject* dtype;  // the dtype attribute
+    int32_t rank;
+    int64_t shape[LB_MAX_RANK];
 };
 struct Entry {
-    std::vector<Arg> args;
+    std::vector<Arg> args;  // owns its references
+    std::vector<char> torch;  // by argument: a torch tensor, which has to be on the GPU and contiguous
     const lb_plan* plan;
     void* workspace;
     std::vector<void*> outputs;
@@ -204,6 +209,8 @@ struct Entry {
 struct CallTable {
     PyObject_HEAD
     std::deque<Entry>* entries;  // references stay valid while other threads add signatures
+    std::unordered_multimap<uint64_t, Entry*>* index;
+    std::vector<PyObject*>* types;  // the argument types of the entries (held by them): anything else is not looked up
     PyObject* latest;  // the signature object of the latest call
 };
 
@@ -214,22 +221,31 @@ void drop(Entry& e) {
 PyObject* table_new(PyTypeObject* type, PyObject*, PyObject*) {
     CallTable* t = (CallTable*)type->tp_alloc(type, 0);
     if (!t) return nullptr;
-    t->entries = new std::deque<Entry>();
+    t->entries = new (std::nothrow) std::deque<Entry>();
+    t->index = new (std::nothrow) std::unordered_multimap<uint64_t, Entry*>();
+    t->types = new (std::nothrow) std::vector<PyObject*>();
     t->latest = Py_NewRef(Py_None);
+    if (!t->entries || !t->index || !t->types) {
+        Py_DECREF(t);
+        return PyErr_NoMemory();
+    }
     return (PyObject*)t;
 }
 int table_traverse(CallTable* t, visitproc visit, void* arg) {
-    for (Entry& e : *t->entries) {
-        Py_VISIT(e.signature);
-        Py_VISIT(e.returned);
-        Py_VISIT(e.keep);
-    }
+    if (t->entries)
+        for (Entry& e : *t->entries) {
+            Py_VISIT(e.signature);
+            Py_VISIT(e.returned);
+            Py_VISIT(e.keep);
+        }
     Py_VISIT(t->latest);
     return 0;
 }
 int table_clear(CallTable* t) {
     std::deque<Entry> gone;
-    gone.swap(*t->entries);
+    if (t->index) t->index->clear();
+    if (t->types) t->types->clear();
+    if (t->entries) gone.swap(*t->entries);
     for (Entry& e : gone) drop(e);
     Py_CLEAR(t->latest);
     return 0;
@@ -238,7 +254,28 @@ void table_dealloc(CallTable* t) {
     PyObject_GC_UnTrack(t);
     table_clear(t);
     delete t->entries;
+    delete t->index;
+    delete t->types;
     Py_TYPE(t)->tp_free((PyObject*)t);
+}
+
+// What a call's argument is looked up by; the references are the caller's (`dtype` is new, `type` borrowed).
+bool read_arg(PyObject* x, Arg* out) {
+    out->type = (PyObject*)Py_TYPE(x);
+    out->dtype = PyObject_GetAttr(x, names.dtype);
+    return out->dtype && read_longs(PyObject_GetAttr(x, names.shape), out->shape, &out->rank, "shape");
+}
+bool hash_args(const Arg* args, size_t count, uint64_t* out) {
+    uint64_t h = 0x9e3779b97f4a7c15ull;
+    auto mix = [&](uint64_t v) { h = (h ^ v) * 0xff51afd7ed558ccdull, h ^= h >> 32; };
+    for (size_t k = 0; k < count; k++) {
+        const Py_hash_t d = PyObject_Hash(args[k].dtype);
+        if (d == -1 && PyErr_Occurred()) return false;
+        mix((uint64_t)(uintptr_t)args[k].type), mix((uint64_t)d), mix((uint64_t)args[k].rank);
+        for (int32_t r = 0; r < args[k].rank; r++) mix((uint64_t)args[k].shape[r]);
+    }
+    *out = h;
+    return true;
 }
 
 // add(args, torch_flags, plan handle, workspace pointer, output pointers, signature, returned)
@@ -249,62 +286,87 @@ PyObject* table_add(CallTable* t, PyObject* const* a, Py_ssize_t n) {
         return nullptr;
     }
     Entry e = {};
-    e.plan = (const lb_plan*)PyLong_AsVoidPtr(a[2]);
-    e.workspace = PyLong_AsVoidPtr(a[3]);
-    for (Py_ssize_t k = 0; k < PyTuple_GET_SIZE(a[4]); k++) e.outputs.push_back(PyLong_AsVoidPtr(PyTuple_GET_ITEM(a[4], k)));
-    bool ok = !PyErr_Occurred();
-    for (Py_ssize_t k = 0; ok && k < PyTuple_GET_SIZE(a[0]); k++) {
-        PyObject* x = PyTuple_GET_ITEM(a[0], k);
-        Arg arg;
-        int64_t shape[LB_MAX_RANK];
-        int32_t rank = 0;
-        arg.torch = PyTuple_GET_ITEM(a[1], k) == Py_True;
-        ok = read_longs(PyObject_GetAttr(x, names.shape), shape, &rank, "shape");
-        arg.shape.assign(shape, shape + rank);
-        arg.dtype = ok ? PyObject_GetAttr(x, names.dtype) : nullptr;
-        arg.type = Py_NewRef((PyObject*)Py_TYPE(x));
-        ok = ok && arg.dtype;
-        e.args.push_back(std::move(arg));
-    }
-    e.signature = Py_NewRef(a[5]), e.returned = Py_NewRef(a[6]);
-    if (!ok) {
+    try {
+        e.plan = (const lb_plan*)PyLong_AsVoidPtr(a[2]);
+        e.workspace = PyLong_AsVoidPtr(a[3]);
+        for (Py_ssize_t k = 0; k < PyTuple_GET_SIZE(a[4]); k++) e.outputs.push_back(PyLong_AsVoidPtr(PyTuple_GET_ITEM(a[4], k)));
+        bool ok = !PyErr_Occurred();
+        for (Py_ssize_t k = 0; ok && k < PyTuple_GET_SIZE(a[0]); k++) {
+            e.args.push_back(Arg{});
+            ok = read_arg(PyTuple_GET_ITEM(a[0], k), &e.args.back());
+            Py_XINCREF(e.args.back().type);
+            e.torch.push_back(PyTuple_GET_ITEM(a[1], k) == Py_True);
+        }
+        uint64_t h = 0;
+        if (!ok || !hash_args(e.args.data(), e.args.size(), &h)) {
+            drop(e);
+            return nullptr;
+        }
+        for (const Arg& arg : e.args)
+            if (std::find(t->types->begin(), t->types->end(), arg.type) == t->types->end()) t->types->push_back(arg.type);
+        t->entries->push_back(e);
+        e = {};  // the table's now
+        Entry& kept = t->entries->back();
+        kept.signature = Py_NewRef(a[5]), kept.returned = Py_NewRef(a[6]);
+        t->index->emplace(h, &kept);
+    } catch (const std::bad_alloc&) {
         drop(e);
-        return nullptr;
+        return PyErr_NoMemory();
     }
-    t->entries->push_back(std::move(e));
     Py_RETURN_NONE;
 }
 
-// 1: `x` is what `want` describes and its pointer is in *ptr; 0: it is not; -1: a Python error
-int matches(PyObject* x, const Arg& want, long device, void** ptr) {
-    if ((PyObject*)Py_TYPE(x) != want.type) return 0;
-    PyObject* d = PyObject_GetAttr(x, names.dtype);
-    if (!d) return -1;
-    int same = d == want.dtype ? 1 : PyObject_RichCompareBool(d, want.dtype, Py_EQ);
-    Py_DECREF(d);
-    if (same <= 0) return same;
-    PyObject* shape = PyObject_GetAttr(x, names.shape);
-    if (!shape) return -1;
-    same = PyTuple_Check(shape) && PyTuple_GET_SIZE(shape) == (Py_ssize_t)want.shape.size();
-    for (size_t k = 0; same && k < want.shape.size(); k++) same = PyLong_AsLongLong(PyTuple_GET_ITEM(shape, k)) == want.shape[k];
-    Py_DECREF(shape);
-    if (PyErr_Occurred()) return -1;
-    if (!same) return 0;
-    if (want.torch) {
-        bool yes = false;
-        if (!truth(PyObject_GetAttr(x, names.is_cuda), &yes)) return -1;
-        if (!yes) return 0;
-        if (!truth(PyObject_CallMethodNoArgs(x, names.is_contiguous), &yes)) return -1;
-        if (!yes) return 0;
-        if (device >= 0) {
-            PyObject* g = PyObject_CallMethodNoArgs(x, names.get_device);
-            if (!g) return -1;
-            long at = PyLong_AsLong(g);
-            Py_DECREF(g);
-            if (at != device) return PyErr_Occurred() ? -1 : 0;
+bool same_args(const Arg* got, const Entry& e) {
+    for (size_t k = 0; k < e.args.size(); k++) {
+        const Arg& want = e.args[k];
+        if (got[k].type != want.type || got[k].rank != want.rank) return false;
+        for (int32_t r = 0; r < want.rank; r++)
+            if (got[k].shape[r] != want.shape[r]) return false;
+        if (got[k].dtype != want.dtype) {
+            const int same = PyObject_RichCompareBool(got[k].dtype, want.dtype, Py_EQ);
+            if (same < 0) PyErr_Clear();
+            if (same <= 0) return false;
         }
     }
-    return read_pointer(x, ptr) ? 1 : -1;
+    return true;
+}
+// 1: the torch tensor can be read where it is; 0: it cannot (on the host, strided, on another GPU); -1: a Python error
+int in_place(PyObject* x, long device) {
+    bool yes = false;
+    if (!truth(PyObject_GetAttr(x, names.is_cuda), &yes)) return -1;
+    if (!yes) return 0;
+    if (!truth(PyObject_CallMethodNoArgs(x, names.is_contiguous), &yes)) return -1;
+    if (!yes) return 0;
+    if (device >= 0) {
+        PyObject* g = PyObject_CallMethodNoArgs(x, names.get_device);
+        if (!g) return -1;
+        const long at = PyLong_AsLong(g);
+        Py_DECREF(g);
+        if (at != device) return PyErr_Occurred() ? -1 : 0;
+    }
+    return 1;
+}
+
+// The entry that the arguments match, or null (with a Python error set where reading one failed).
+Entry* find(CallTable* t, PyObject* args) {
+    constexpr Py_ssize_t kMost = 64;
+    const Py_ssize_t count = PyTuple_GET_SIZE(args);
+    if (count > kMost) return nullptr;
+    for (Py_ssize_t k = 0; k < count; k++)
+        if (std::find(t->types->begin(), t->types->end(), (PyObject*)Py_TYPE(PyTuple_GET_ITEM(args, k))) == t->types->end()) return nullptr;
+    Arg got[kMost];
+    Py_ssize_t read = 0;
+    bool ok = true;
+    for (; ok && read < count; read++) ok = read_arg(PyTuple_GET_ITEM(args, read), &got[read]);
+    Entry* found = nullptr;
+    uint64_t h = 0;
+    if (ok && hash_args(got, (size_t)count, &h)) {
+        auto range = t->index->equal_range(h);
+        for (auto it = range.first; it != range.second && !found; ++it)
+            if ((Py_ssize_t)it->second->args.size() == count && same_args(got, *it->second)) found = it->second;
+    }
+    for (Py_ssize_t k = 0; k < read; k++) Py_XDECREF(got[k].dtype);
+    return found;
 }
 
 // call(args, stream, device): stream 0 means the caller's current stream; `device`: the current device's index, which the
@@ -312,47 +374,57 @@ int matches(PyObject* x, const Arg& want, long device, void** ptr) {
 PyObject* table_call(CallTable* t, PyObject* const* a, Py_ssize_t n) {
     if (!wants(n, 3)) return nullptr;
     PyObject* args = a[0];
+    if (!PyTuple_Check(args)) {
+        PyErr_SetString(PyExc_TypeError, "call: a tuple of arguments");
+        return nullptr;
+    }
     void* stream = PyLong_AsVoidPtr(a[1]);
     const long device = PyLong_AsLong(a[2]);
     if (PyErr_Occurred()) return nullptr;
+    Entry* entry = find(t, args);
+    if (!entry) {
+        if (PyErr_Occurred()) return nullptr;
+        Py_RETURN_NONE;
+    }
+    Entry& e = *entry;
+    PyObject *returned = Py_NewRef(e.returned), *signature = Py_NewRef(e.signature);  // hold the plan and its memory
     const Py_ssize_t count = PyTuple_GET_SIZE(args);
     void* pointers[64];
-    if (count > 64) Py_RETURN_NONE;
-    for (size_t k = 0; k < t->entries->size(); k++) {
-        Entry& e = (*t->entries)[k];
-        if ((Py_ssize_t)e.args.size() != count) continue;
-        int same = 1;
-        bool torch = false;
-        for (Py_ssize_t i = 0; same == 1 && i < count; i++) {
-            same = matches(PyTuple_GET_ITEM(args, i), e.args[i], device, &pointers[i]);
-            torch |= e.args[i].torch;
-        }
-        if (same < 0) return nullptr;
-        if (!same) continue;
-        if (!stream) {
-            PyObject* s = torch && raw_stream != Py_None ? PyObject_CallFunction(raw_stream, "l", device < 0 ? 0L : device)
-                                                         : PyObject_CallNoArgs(current_stream);
-            if (!s) return nullptr;
-            stream = PyLong_AsVoidPtr(s);
-            Py_DECREF(s);
-            if (PyErr_Occurred()) return nullptr;
-        }
-        PyObject *returned = Py_NewRef(e.returned), *signature = Py_NewRef(e.signature);  // hold the plan and its memory
-        PyObject* before = e.keep;
-        e.keep = Py_NewRef(args);
-        int rc;
-        Py_BEGIN_ALLOW_THREADS
-        rc = lb_plan_run(e.plan, e.workspace, pointers, (int)count, e.outputs.data(), (int)e.outputs.size(), 0, -1, stream);
-        Py_END_ALLOW_THREADS
-        Py_XDECREF(before);
-        Py_XSETREF(t->latest, signature);
-        if (rc != LB_OK) {
-            Py_DECREF(returned);
-            return finish(rc);
-        }
-        return returned;
+    int usable = 1;
+    bool torch = false;
+    for (Py_ssize_t k = 0; usable == 1 && k < count; k++) {
+        PyObject* x = PyTuple_GET_ITEM(args, k);
+        if (e.torch[k]) torch = true, usable = in_place(x, device);
+        if (usable == 1 && !read_pointer(x, &pointers[k])) usable = -1;
     }
-    Py_RETURN_NONE;
+    if (usable == 1 && !stream) {
+        PyObject* s = torch && raw_stream != Py_None ? PyObject_CallFunction(raw_stream, "l", device < 0 ? 0L : device)
+                                                     : PyObject_CallNoArgs(current_stream);
+        if (s) stream = PyLong_AsVoidPtr(s);
+        Py_XDECREF(s);
+        if (PyErr_Occurred()) usable = -1;
+    }
+    if (usable != 1) {
+        Py_DECREF(returned);
+        Py_DECREF(signature);
+        if (usable < 0) return nullptr;
+        Py_RETURN_NONE;
+    }
+    PyObject* before = e.keep;
+    e.keep = Py_NewRef(args);
+    const lb_plan* plan = e.plan;
+    void* workspace = e.workspace;
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = lb_plan_run(plan, workspace, pointers, (int)count, e.outputs.data(), (int)e.outputs.size(), 0, -1, stream);
+    Py_END_ALLOW_THREADS
+    Py_XDECREF(before);
+    Py_XSETREF(t->latest, signature);
+    if (rc != LB_OK) {
+        Py_DECREF(returned);
+        return finish(rc);
+    }
+    return returned;
 }
 
 PyMethodDef table_methods[] = {
