@@ -287,6 +287,7 @@ void lb_graph_destroy(lb_graph* graph);
  * hold: blocks freed meanwhile return only at release (cuda.rs:123-170). */
 typedef struct lb_region lb_region;
 int lb_set_device(int device);     /* makes `device` current; fails unless it is an sm_100 part */
+int lb_get_device(int* device);    /* the device that is current for the calling thread */
 int lb_device_count(void);
 int lb_device_synchronize(void);
 int lb_device_memory(size_t* free_bytes, size_t* total_bytes);

@@ -16,6 +16,7 @@ import sys
 from lumen_b200 import _lib, runtime, tracer
 from lumen_b200.compiler import compile_graph
 from lumen_b200.device import Tensor as DeviceTensor
+from lumen_b200.device import current_device
 from lumen_b200.plan import Plan
 from lumen_b200.runtime import _empty_like_input, dtype_name, require_cuda
 
@@ -39,10 +40,18 @@ def _on_current_gpu(a, device) -> bool:
 _tensor_types: dict = {}  # argument types met that are tensors -> whether they are torch's
 
 
+_gpus = 0  # GPUs of the process, once asked
+
+
 def _device_index() -> int:
-    """What `CallTable.call` checks torch arguments against: the current device, or -1 in a process with one GPU."""
+    """The current device, on which a signature's memory and the arguments have to be; -1 in a process with one GPU."""
+    global _gpus
+    if _gpus == 0:
+        _gpus = _lib.lib().lb_device_count()
+    if _gpus <= 1:
+        return -1
     torch = sys.modules.get("torch")
-    return -1 if torch is None or torch.cuda.device_count() <= 1 else torch.cuda.current_device()
+    return torch.cuda.current_device() if torch is not None else current_device()
 
 
 class _Signature:
@@ -96,14 +105,15 @@ class Compiled:
         return self.calls.latest
 
     def __call__(self, *args):
-        out = self.calls.call(args, runtime._current[0], _device_index())
-        return out if out is not None else self._general_call(args)
+        device = _device_index()
+        out = self.calls.call(args, runtime._current[0], device)
+        return out if out is not None else self._general_call(args, device)
 
-    def _general_call(self, args):
+    def _general_call(self, args, device):
         require_cuda()
         # any array that speaks DLPack (the reference's tensors import and export it, lumen/tensor/dlpack.rs) is taken
         # in place, without a copy when it already lives on this device
-        key, inputs = [], []
+        key, inputs = [device], []  # a signature's workspace and results live on one GPU
         for a in args:
             kind = type(a)
             if kind not in _tensor_types:
@@ -111,7 +121,7 @@ class Compiled:
                     if hasattr(a, "__dlpack__"):
                         import torch  # the DLPack importer of a harness that passes foreign arrays
 
-                        return self._general_call([torch.from_dlpack(x) if not _is_tensor(x) and hasattr(x, "__dlpack__") else x for x in args])
+                        return self._general_call([torch.from_dlpack(x) if not _is_tensor(x) and hasattr(x, "__dlpack__") else x for x in args], device)
                     key.append(("static", a))
                     continue
                 _tensor_types[kind] = not isinstance(a, DeviceTensor)
@@ -123,7 +133,7 @@ class Compiled:
             sig = self.signatures[key] = _Signature(self.fn, args, self.device, self.lowering)
         kinds = tuple(type(a) for a in inputs)
         if kinds not in sig.native and not self.use_graphs and len(inputs) == len(args):
-            self._add(sig, kinds, inputs)
+            self._add(sig, kinds, inputs, device)
         self.calls.latest = sig
         for k, a in enumerate(inputs):
             if _tensor_types[type(a)] and not (_on_current_gpu(a, self.device) and a.is_contiguous()):
@@ -139,16 +149,16 @@ class Compiled:
             sig.bound_to, sig.keep = pointers, (inputs, bound)
         return sig.returned
 
-    def _add(self, sig, kinds, inputs):
+    def _add(self, sig, kinds, inputs, device):
         """Calls with arguments like these from now on run natively."""
         sig.native.add(kinds)
         torches = tuple(_tensor_types[type(a)] for a in inputs)
         if any(torches):
             torch = sys.modules["torch"]
-            if self.device != "cuda" or (torch.cuda.device_count() > 1 and not all(torches)):
+            if self.device != "cuda" or (device >= 0 and not all(torches)):
                 return
             _lib.host().for_torch(getattr(torch._C, "_cuda_getCurrentRawStream", None))
-        self.calls.add(tuple(inputs), torches, sig.plan.handle.value, sig.plan.workspace_ptr, tuple(t.data_ptr() for t in sig.results),
+        self.calls.add(tuple(inputs), torches, device, sig.plan.handle.value, sig.plan.workspace_ptr, tuple(t.data_ptr() for t in sig.results),
                        sig, sig.returned)
 
     def __str__(self) -> str:

@@ -189,7 +189,7 @@ PyObject* gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 // ---- the calls of one compiled function -----------------------------------------------------------------------------
 // The signatures a `lumen_b200.compile`d function has met whose arguments are all tensors, by a hash of the arguments' types,
-// dtypes and shapes: a call costs the same with one signature as with thousands (a cache that grows by a token a
+// dtypes and shapes and of the device: a call costs the same with one signature as with thousands (a cache that grows by a token a
 // call). `call(args, stream, device)` finds the one that `args` match, runs its plan and returns its results; it returns None
 // when the call needs the general path (an unknown signature, host or strided or foreign arguments).
 struct Arg {
@@ -201,6 +201,7 @@ struct Arg {
 struct Entry {
     std::vector<Arg> args;  // owns its references
     std::vector<char> torch;  // by argument: a torch tensor, which has to be on the GPU and contiguous
+    long device;            // the GPU that the plan's workspace and results live on (-1: the process has one)
     const lb_plan* plan;
     void* workspace;
     std::vector<void*> outputs;
@@ -265,8 +266,8 @@ bool read_arg(PyObject* x, Arg* out) {
     out->dtype = PyObject_GetAttr(x, names.dtype);
     return out->dtype && read_longs(PyObject_GetAttr(x, names.shape), out->shape, &out->rank, "shape");
 }
-bool hash_args(const Arg* args, size_t count, uint64_t* out) {
-    uint64_t h = 0x9e3779b97f4a7c15ull;
+bool hash_args(const Arg* args, size_t count, long device, uint64_t* out) {
+    uint64_t h = (uint64_t)device + 0x9e3779b97f4a7c15ull;
     auto mix = [&](uint64_t v) { h = (h ^ v) * 0xff51afd7ed558ccdull, h ^= h >> 32; };
     for (size_t k = 0; k < count; k++) {
         const Py_hash_t d = PyObject_Hash(args[k].dtype);
@@ -278,18 +279,19 @@ bool hash_args(const Arg* args, size_t count, uint64_t* out) {
     return true;
 }
 
-// add(args, torch_flags, plan handle, workspace pointer, output pointers, signature, returned)
+// add(args, torch_flags, device, plan handle, workspace pointer, output pointers, signature, returned)
 PyObject* table_add(CallTable* t, PyObject* const* a, Py_ssize_t n) {
-    if (!wants(n, 7)) return nullptr;
-    if (!PyTuple_Check(a[0]) || !PyTuple_Check(a[1]) || !PyTuple_Check(a[4]) || PyTuple_GET_SIZE(a[0]) != PyTuple_GET_SIZE(a[1])) {
+    if (!wants(n, 8)) return nullptr;
+    if (!PyTuple_Check(a[0]) || !PyTuple_Check(a[1]) || !PyTuple_Check(a[5]) || PyTuple_GET_SIZE(a[0]) != PyTuple_GET_SIZE(a[1])) {
         PyErr_SetString(PyExc_TypeError, "add: tuples of arguments, flags and output pointers");
         return nullptr;
     }
     Entry e = {};
     try {
-        e.plan = (const lb_plan*)PyLong_AsVoidPtr(a[2]);
-        e.workspace = PyLong_AsVoidPtr(a[3]);
-        for (Py_ssize_t k = 0; k < PyTuple_GET_SIZE(a[4]); k++) e.outputs.push_back(PyLong_AsVoidPtr(PyTuple_GET_ITEM(a[4], k)));
+        e.device = PyLong_AsLong(a[2]);
+        e.plan = (const lb_plan*)PyLong_AsVoidPtr(a[3]);
+        e.workspace = PyLong_AsVoidPtr(a[4]);
+        for (Py_ssize_t k = 0; k < PyTuple_GET_SIZE(a[5]); k++) e.outputs.push_back(PyLong_AsVoidPtr(PyTuple_GET_ITEM(a[5], k)));
         bool ok = !PyErr_Occurred();
         for (Py_ssize_t k = 0; ok && k < PyTuple_GET_SIZE(a[0]); k++) {
             e.args.push_back(Arg{});
@@ -298,7 +300,7 @@ PyObject* table_add(CallTable* t, PyObject* const* a, Py_ssize_t n) {
             e.torch.push_back(PyTuple_GET_ITEM(a[1], k) == Py_True);
         }
         uint64_t h = 0;
-        if (!ok || !hash_args(e.args.data(), e.args.size(), &h)) {
+        if (!ok || !hash_args(e.args.data(), e.args.size(), e.device, &h)) {
             drop(e);
             return nullptr;
         }
@@ -307,7 +309,7 @@ PyObject* table_add(CallTable* t, PyObject* const* a, Py_ssize_t n) {
         t->entries->push_back(e);
         e = {};  // the table's now
         Entry& kept = t->entries->back();
-        kept.signature = Py_NewRef(a[5]), kept.returned = Py_NewRef(a[6]);
+        kept.signature = Py_NewRef(a[6]), kept.returned = Py_NewRef(a[7]);
         t->index->emplace(h, &kept);
     } catch (const std::bad_alloc&) {
         drop(e);
@@ -348,7 +350,7 @@ int in_place(PyObject* x, long device) {
 }
 
 // The entry that the arguments match, or null (with a Python error set where reading one failed).
-Entry* find(CallTable* t, PyObject* args) {
+Entry* find(CallTable* t, PyObject* args, long device) {
     constexpr Py_ssize_t kMost = 64;
     const Py_ssize_t count = PyTuple_GET_SIZE(args);
     if (count > kMost) return nullptr;
@@ -360,17 +362,17 @@ Entry* find(CallTable* t, PyObject* args) {
     for (; ok && read < count; read++) ok = read_arg(PyTuple_GET_ITEM(args, read), &got[read]);
     Entry* found = nullptr;
     uint64_t h = 0;
-    if (ok && hash_args(got, (size_t)count, &h)) {
+    if (ok && hash_args(got, (size_t)count, device, &h)) {
         auto range = t->index->equal_range(h);
         for (auto it = range.first; it != range.second && !found; ++it)
-            if ((Py_ssize_t)it->second->args.size() == count && same_args(got, *it->second)) found = it->second;
+            if ((Py_ssize_t)it->second->args.size() == count && it->second->device == device && same_args(got, *it->second)) found = it->second;
     }
     for (Py_ssize_t k = 0; k < read; k++) Py_XDECREF(got[k].dtype);
     return found;
 }
 
-// call(args, stream, device): stream 0 means the caller's current stream; `device`: the current device's index, which the
-// arguments have to be on (< 0: the process sees one GPU only)
+// call(args, stream, device): stream 0 means the caller's current stream; `device`: the current device's index, on which the
+// signature's memory and the arguments have to be (< 0: the process sees one GPU only)
 PyObject* table_call(CallTable* t, PyObject* const* a, Py_ssize_t n) {
     if (!wants(n, 3)) return nullptr;
     PyObject* args = a[0];
@@ -381,7 +383,7 @@ PyObject* table_call(CallTable* t, PyObject* const* a, Py_ssize_t n) {
     void* stream = PyLong_AsVoidPtr(a[1]);
     const long device = PyLong_AsLong(a[2]);
     if (PyErr_Occurred()) return nullptr;
-    Entry* entry = find(t, args);
+    Entry* entry = find(t, args, device);
     if (!entry) {
         if (PyErr_Occurred()) return nullptr;
         Py_RETURN_NONE;

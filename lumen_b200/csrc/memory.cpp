@@ -63,6 +63,14 @@ int lb_set_device(int device) {
     });
 }
 
+int lb_get_device(int* device) {
+    return lb::guarded([&] {
+        if (!device) lb::fail(LB_ERR_INVALID, "lb_get_device: null argument");
+        lb::driver();
+        LB_CUDA(cudaGetDevice(device));
+    });
+}
+
 int lb_device_count(void) {
     int n = 0;
     if (cudaGetDeviceCount(&n) != cudaSuccess) {

@@ -28,6 +28,7 @@ def _bound():
     vp, sz = ctypes.c_void_p, ctypes.c_size_t
     P = ctypes.POINTER
     lib.lb_set_device.argtypes = [ctypes.c_int]
+    lib.lb_get_device.argtypes = [P(ctypes.c_int)]
     lib.lb_device_memory.argtypes = [P(sz), P(sz)]
     lib.lb_region_create.argtypes = [sz, P(vp)]
     lib.lb_region_destroy.argtypes = [vp]
@@ -55,6 +56,13 @@ def _bound():
 def set_device(index: int) -> None:
     """Makes GPU `index` current for this thread (fails unless it is an sm_100 part)."""
     _lib.check(_bound().lb_set_device(int(index)))
+
+
+def current_device() -> int:
+    """The GPU that is current for this thread."""
+    index = ctypes.c_int()
+    _lib.check(_bound().lb_get_device(ctypes.byref(index)))
+    return index.value
 
 
 def device_count() -> int:

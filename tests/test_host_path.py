@@ -77,10 +77,10 @@ def ran():
     return pytest.raises(_lib.LumenError, match="null plan")
 
 
-def table(*signatures):
+def table(*signatures, device=-1):
     t = _lib.host().CallTable()
     for args in signatures:
-        t.add(args, tuple(isinstance(a, Torch) for a in args), 0, 0, (0,), "signature", "returned")
+        t.add(args, tuple(isinstance(a, Torch) for a in args), device, 0, 0, (0,), "signature", "returned")
     return t
 
 
@@ -116,10 +116,24 @@ def test_torch_tensors_have_to_be_readable_in_place():
     assert t.call((Torch((4, 8), cuda=False),), 1, -1) is None
     assert t.call((Torch((4, 8), contiguous=False),), 1, -1) is None
     assert t.call((Parameter((4, 8)),), 1, -1) is None
-    t.add((Parameter((4, 8)),), (True,), 0, 0, (0,), "signature", "returned")
+    t.add((Parameter((4, 8)),), (True,), -1, 0, 0, (0,), "signature", "returned")
     for x in (Torch((4, 8)), Parameter((4, 8))):
         with ran():
             t.call((x,), 1, -1)
+
+
+def test_a_signature_belongs_to_the_device_of_its_memory():
+    """After a first call on GPU 0, tensors of the same shape on GPU 1, with that one current, are another signature."""
+    t = table((Torch((4, 8), device=0),), device=0)
+    assert t.call((Torch((4, 8), device=1),), 1, 1) is None
+    assert t.call((Torch((4, 8), device=1),), 1, 0) is None
+    assert t.call((Torch((4, 8), device=0),), 1, 1) is None
+    with ran():
+        t.call((Torch((4, 8), device=0),), 1, 0)
+    t.add((Torch((4, 8)),), (True,), 1, 0, 0, (0,), "signature of GPU 1", "returned")
+    with ran():
+        t.call((Torch((4, 8), device=1),), 1, 1)
+    assert t.latest == "signature of GPU 1"
 
 
 def test_a_call_costs_the_same_among_many_signatures():
@@ -154,9 +168,9 @@ def test_errors_of_an_argument_are_raised():
 
     t = _lib.host().CallTable()
     with pytest.raises(RuntimeError, match="no shape"):
-        t.add((Broken((4,)),), (False,), 0, 0, (0,), "signature", "returned")
+        t.add((Broken((4,)),), (False,), -1, 0, 0, (0,), "signature", "returned")
     with pytest.raises(TypeError):
-        t.add([Array((4,))], (False,), 0, 0, (0,), "signature", "returned")
+        t.add([Array((4,))], (False,), -1, 0, 0, (0,), "signature", "returned")
     with pytest.raises(TypeError):
         t.call([Array((4,))], 1, -1)
 
@@ -171,7 +185,7 @@ def test_threads_add_and_call_at_once():
         try:
             for n in range(200):
                 x = Array((k + 2, n + 1))
-                t.add((x,), (False,), 0, 0, (0,), "signature", "returned")
+                t.add((x,), (False,), -1, 0, 0, (0,), "signature", "returned")
                 with ran():
                     t.call((Array((k + 2, n + 1)),), 1, -1)
                 with ran():
