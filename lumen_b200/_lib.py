@@ -5,6 +5,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "liblumen_b200.so")
@@ -52,14 +53,15 @@ _host = None
 
 
 def host():
-    """The native call path (`_host.so` beside the library), set up on first use."""
+    """The native call path (`_host` beside the library, an extension module of this interpreter), set up on first use."""
     global _host
     if _host is None:
         lib()
         try:
             from lumen_b200 import _host as module
         except ImportError as e:
-            raise ImportError("lumen_b200/_host.so is missing or does not load: build it with `make -C lumen_b200/csrc`") from e
+            raise ImportError(f"lumen_b200/_host is missing for {sys.executable} or does not load: build it with "
+                              f"`make -C lumen_b200/csrc PYTHON={sys.executable}` (needs that interpreter's headers)") from e
         from lumen_b200.runtime import current_stream, dtype_name
 
         codes = dict(DTYPE_CODES)

@@ -83,3 +83,19 @@ def test_launch_without_a_gpu_fails_loudly():
     descs = (_lib.LbTensor * 2)(_lib.dense(ctypes.addressof(buf), "float32", (8,)), _lib.dense(ctypes.addressof(buf), "float32", (8,)))
     rc = _lib.lib().lb_fusion_launch(handle, descs, 2, None, None)
     assert rc == 3 and b"no CPU fallback" in _lib.lib().lb_last_error()
+
+
+def test_the_library_builds_without_python_headers():
+    """The default target is the library and, for the interpreter it is built with, the call path under that one's tag; without an
+    interpreter (or its headers) the library alone."""
+    import subprocess
+    import sys
+    import sysconfig
+
+    def commands(python):
+        make = ["make", "-n", "-B", "-C", os.path.join(ROOT, "lumen_b200", "csrc"), f"PYTHON={python}"]
+        return subprocess.run(make, check=True, capture_output=True, text=True).stdout
+
+    assert "liblumen_b200.so.tmp" in commands("false") and "host_py.cpp" not in commands("false")
+    assert f"_host{sysconfig.get_config_var('EXT_SUFFIX')}" in commands(sys.executable)
+    assert _lib.host().__file__.endswith(f"_host{sysconfig.get_config_var('EXT_SUFFIX')}")
