@@ -1318,11 +1318,13 @@ class Generator {
                 std::string init, combine;
                 reduce_ops(n, t, &init, &combine);
                 s << "    {\n        " << type << "* part = (" << type << "*)((char*)scratch + " << scratch << ") + (idx_t)blockIdx.x * NCOLS;\n";
-                if (RPB_ > 1) {  // the block's rows in order, through shared memory
+                if (RPB_ > 1) {  // the rows of a warp as a tree, then the warps in order, through shared memory
+                    const std::string acc = format("cacc%d[ch][e]", (int)i), sum = format("csum%d[c0 + e]", (int)i);
                     s << "        " << type << "* csum" << i << " = (" << type << "*)shared;\n";
-                    s << "        for (int y = 0; y < RPB; y++) {\n            if (row_in_block == y) { CHUNK_LOOP_BEGIN _Pragma(\"unroll\") for (int e = 0; e < VEC; e++) csum"
-                      << i << "[c0 + e] = y ? " << subst(combine, format("csum%d[c0 + e]", (int)i), format("cacc%d[ch][e]", (int)i)) << " : cacc" << i
-                      << "[ch][e]; CHUNK_LOOP_END }\n            __syncthreads();\n        }\n";
+                    s << "        _Pragma(\"unroll\") for (int ch = 0; ch < NCH; ch++) { _Pragma(\"unroll\") for (int e = 0; e < VEC; e++) { _Pragma(\"unroll\") for (int m = TPR; m < 32; m *= 2) "
+                      << acc << " = " << subst(combine, acc, format("shfl_xor_any<%s>(%s, m)", type.c_str(), acc.c_str())) << "; } }\n";
+                    s << "        for (int y = 0; y < TPR * RPB / 32; y++) {\n            if (threadIdx.x / 32 == y && threadIdx.x % 32 < TPR) { CHUNK_LOOP_BEGIN _Pragma(\"unroll\") for (int e = 0; e < VEC; e++) "
+                      << sum << " = y ? " << subst(combine, sum, acc) << " : " << acc << "; CHUNK_LOOP_END }\n            __syncthreads();\n        }\n";
                     s << "        for (int c = threadIdx.x; c < NCOLS; c += TPR * RPB) part[c] = csum" << i << "[c];\n        __syncthreads();\n    }\n";
                 } else {
                     s << "        CHUNK_LOOP_BEGIN _Pragma(\"unroll\") for (int e = 0; e < VEC; e++) part[c0 + e] = cacc" << i << "[ch][e]; CHUNK_LOOP_END\n    }\n";
@@ -1480,37 +1482,59 @@ class Generator {
     }
 
     // The second kernel of a column reduction: adds the slices' partial sums and applies the epilogue. A block takes 32
-    // lanes of two columns and eight or 32 slice lanes: few columns and slices per thread, so that the chains of loads stay
+    // lanes of two columns and one (up to eight slices), eight or 32 slice lanes: few columns and slices per thread, so that the chains of loads stay
     // short (1184 slices of 1024 columns took 19 us with eight slice lanes).
     void emit_finalize(std::ostringstream& s, const std::string& sig, const std::vector<size_t>& offsets, const std::vector<int>& outputs, FusedKernel& k) {
         column_mode_ = true;
         VEC_ = std::min(VEC_, 2);
         pair_ = VEC_ >= 2 && computes_bf16();
-        const int col_lanes = 32, row_lanes = k.slices * k.col_blocks > 64 ? 32 : 8, threads = col_lanes * row_lanes;
+        const int col_lanes = 32, row_lanes = k.slices * k.col_blocks > 64 ? 32 : k.slices * k.col_blocks > 8 ? 8 : 1, threads = col_lanes * row_lanes;
         Comp flat_c;
         flat_c.base = "c0", flat_c.expr = "(c0 + e)";
         flat_c.lane = flat_c.e_dep = flat_c.c_dep = true;
         Phase fin;
         std::ostringstream totals;
         int widest = 1;  // of the compute types; one area of shared memory serves the reductions in turn
-        for (size_t k = 0; k < col_reduces_.size(); k++) {
-            const Node& n = *g_.node_of(col_reduces_[k]);
-            const TensorType& t = g_.type(n.output);
-            CType ct = ctype(t.dtype);
-            std::string init, combine;
-            reduce_ops(n, t, &init, &combine);
-            // slice lane y adds slices y, y + (lanes), ... in order; the lanes are then combined in lane order
-            totals << ct.compute << " tot" << k << "[VEC];\n#pragma unroll\nfor (int e = 0; e < VEC; e++) tot" << k << "[e] = " << init << ";\n";
-            totals << "if (in_range) {\n#pragma unroll 8\n    for (int s = row_lane; s < SLICES; s += " << row_lanes << ") {\n#pragma unroll\n        for (int e = 0; e < VEC; e++) { "
-                   << ct.compute << " pv = ((const " << ct.compute << "*)((const char*)scratch + " << offsets[k] << "))[(idx_t)s * NCOLS + c0 + e]; tot" << k
-                   << "[e] = " << subst(combine, format("tot%d[e]", (int)k), "pv") << "; }\n    }\n}\n";
-            widest = std::max(widest, t.dtype == LB_BF16 || t.dtype == LB_F16 ? 4 : dtype_size(t.dtype));
-            if (k) totals << "__syncthreads();\n";
-            totals << "auto fred" << k << " = (" << ct.compute << "(*)[" << col_lanes << " * VEC])shared;\n";
-            totals << "#pragma unroll\nfor (int e = 0; e < VEC; e++) fred" << k << "[row_lane][col_lane * VEC + e] = tot" << k << "[e];\n__syncthreads();\n";
-            totals << "if (row_lane == 0) {\n#pragma unroll\n    for (int e = 0; e < VEC; e++) {\n#pragma unroll\n        for (int y = 1; y < " << row_lanes << "; y++) tot" << k << "[e] = "
-                   << subst(combine, format("tot%d[e]", (int)k), format("fred%d[y][col_lane * VEC + e]", (int)k)) << ";\n    }\n}\n";
+        // Slice lane y adds slices y, y + (lanes), ... in four sums in turn, whose loads are in flight together; the sums and then the
+        // lanes are combined as trees (one chain a lane and the lanes in order had up to 1.6 times the error of a float32 sum over
+        // 1184 slices). For the second tree a column's lanes lie side by side in a warp (rows padded by one against bank
+        // conflicts), for as many reductions at once as 40 KB of shared memory hold.
+        for (int v : col_reduces_) {
+            const int dtype = g_.type(v).dtype;
+            widest = std::max(widest, dtype == LB_BF16 || dtype == LB_F16 ? 4 : dtype_size(dtype));
         }
+        const int lane_bytes = row_lanes * (col_lanes * VEC_ + 1) * widest, sum_bytes = col_lanes * VEC_ * widest;
+        const size_t batch = std::min<size_t>(col_reduces_.size(), std::max(1, 40 * 1024 / (lane_bytes + sum_bytes)));
+        for (size_t k0 = 0; k0 < col_reduces_.size(); k0 += batch) {
+            std::ostringstream trees, reads;
+            for (size_t k = k0; k < std::min(k0 + batch, col_reduces_.size()); k++) {
+                const Node& n = *g_.node_of(col_reduces_[k]);
+                const TensorType& t = g_.type(n.output);
+                const std::string type = ctype(t.dtype).compute, run = format("run%d", (int)k), tot = format("tot%d", (int)k);
+                std::string init, combine;
+                reduce_ops(n, t, &init, &combine);
+                auto each = [&](const std::string& body) { return "_Pragma(\"unroll\") for (int e = 0; e < VEC; e++) { " + body + " }"; };
+                auto add = [&](const std::string& to, const std::string& x) { return to + " = " + subst(combine, to, x) + ";"; };
+                const std::string from = format("((const %s*)((const char*)scratch + %zu))[(idx_t)(s + u * %d) * NCOLS + c0 + e]", type.c_str(), offsets[k], row_lanes);
+                totals << type << " " << tot << "[VEC];\n{\n    " << type << " " << run << "[4][VEC];\n    _Pragma(\"unroll\") for (int u = 0; u < 4; u++) " << each(run + "[u][e] = " + init + ";") << "\n"
+                       << "    if (in_range) {\n        int s = row_lane;\n        #pragma unroll 2\n        for (; s + " << 3 * row_lanes << " < SLICES; s += " << 4 * row_lanes << ") {\n            " << type
+                       << " pv[4][VEC];\n            _Pragma(\"unroll\") for (int u = 0; u < 4; u++) " << each("pv[u][e] = " + from + ";") << "\n            _Pragma(\"unroll\") for (int u = 0; u < 4; u++) "
+                       << each(add(run + "[u][e]", "pv[u][e]")) << "\n        }\n        _Pragma(\"unroll\") for (int u = 0; u < 3; u++) if (s + u * " << row_lanes << " < SLICES) "
+                       << each("const " + type + " pv = " + from + "; " + add(run + "[u][e]", "pv")) << "\n    }\n    "
+                       << each(add(run + "[0][e]", run + "[1][e]") + " " + add(run + "[2][e]", run + "[3][e]") + " " + tot + "[e] = " + subst(combine, run + "[0][e]", run + "[2][e]") + ";") << "\n    "
+                       << (row_lanes == 1 ? "" : format("auto lanes = (%s(*)[%d * VEC + 1])(shared + %zu);\n    ", type.c_str(), col_lanes, (k - k0) * lane_bytes) + each("lanes[row_lane][col_lane * VEC + e] = " + tot + "[e];") + "\n")
+                       << "}\n";
+                trees << "{\n    auto lanes = (" << type << "(*)[" << col_lanes << " * VEC + 1])(shared + " << (k - k0) * lane_bytes << ");\n    " << type << "* sums = (" << type << "*)(shared + " << batch * lane_bytes + (k - k0) * sum_bytes
+                      << ");\n    const int lane = threadIdx.x % " << row_lanes << ", col = threadIdx.x / " << row_lanes << ";\n    "
+                      << each(type + " v = lanes[lane][col * VEC + e]; _Pragma(\"unroll\") for (int m = " + std::to_string(row_lanes / 2) + "; m >= 1; m /= 2) " + add("v", "shfl_xor_any<" + type + ">(v, m)") +
+                              " if (lane == 0) sums[col * VEC + e] = v;")
+                      << "\n}\n";
+                reads << each(tot + "[e] = ((const " + type + "*)(shared + " + std::to_string(batch * lane_bytes + (k - k0) * sum_bytes) + "))[col_lane * VEC + e];") << "\n";
+            }
+            if (row_lanes > 1) totals << "__syncthreads();\n" << trees.str() << "__syncthreads();\n" << reads.str();
+            // (the next batch writes `lanes`, which were read before the last barrier; its trees write `sums` after another one)
+        }
+        const size_t shared_bytes = row_lanes == 1 ? 16 : batch * (lane_bytes + sum_bytes);
         for (int o : outputs) {
             const TensorType& t = g_.type(g_.outputs[o]);
             if (t.numel() != C_) fail(LB_ERR_UNSUPPORTED, format("column-reduction fusion output %s does not have %lld elements", t.str().c_str(), (long long)C_));
@@ -1525,7 +1549,7 @@ class Generator {
         s << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") fused_finalize(" << sig << ") {\n";
         s << "    const int col_lane = threadIdx.x & " << col_lanes - 1 << ", row_lane = threadIdx.x >> 5;\n";
         s << "    const idx_t c0 = ((idx_t)blockIdx.x * " << col_lanes << " + col_lane) * VEC;\n    const bool in_range = c0 < NCOLS;\n";
-        s << "    __shared__ __align__(16) char shared[" << threads << " * VEC * " << widest << "];\n";
+        s << "    __shared__ __align__(16) char shared[" << shared_bytes << "];\n";
         s << indent(totals.str(), 4);
         s << "    if (row_lane != 0 || !in_range) return;\n";
         s << indent(fin.pre, 4);

@@ -310,3 +310,47 @@ def test_rows_of_odd_widths(cuda, rows, cols, dtype):
     assert torch.equal(y.view(t) if y.dtype != t else y, want)
     total = (want * want).double().sum(1)
     assert ((s.double() - total).abs() <= cols * 2.0**-24 * total + 1e-30).all()
+
+
+def column_sums_in_slices(x):
+    """float32 column sums in the order of the two-pass column reduction: slices of at least 64 rows, eight row lanes each that add every
+    eighth row, eight slice lanes that add every eighth slice, lanes in order."""
+    rows, cols = x.shape
+    col_blocks = -(-cols // 128)
+    slices = min(max(1, -(-592 // col_blocks)), max(rows // 64, 1))
+    per = -(-rows // slices)
+
+    def lanes(rows_, n=8):  # [.., k, cols] -> [.., cols]
+        pad = -rows_.shape[-2] % n
+        rows_ = torch.cat([rows_, rows_.new_zeros(*rows_.shape[:-2], pad, cols)], -2).unflatten(-2, (-1, n))
+        total = rows_[..., 0, :, :]
+        for k in range(1, rows_.shape[-3]):
+            total = total + rows_[..., k, :, :]
+        out = total[..., 0, :]
+        for y in range(1, n):
+            out = out + total[..., y, :]
+        return out
+
+    whole = torch.cat([x, x.new_zeros(-(-rows // per) * per - rows, cols)]).unflatten(0, (-1, per))
+    return lanes(lanes(whole))
+
+
+@pytest.mark.parametrize("rows,cols", [(4096, 64), (1020, 260), (512, 512), (8192, 1024), (20000, 1000), (2048, 4096)])
+@pytest.mark.parametrize("beside", [False, True])
+def test_column_sums_are_as_exact_as_in_slices(cuda, rows, cols, beside):
+    """Alone and beside row outputs (one kernel for both), the root mean square of a column sum's error is no larger than in the
+    order above, whose chains of adds are about as long; over the columns it varies by 1 / sqrt(2 * cols), of which three are allowed."""
+    x = torch.randn((rows, cols), generator=torch.Generator(device=cuda).manual_seed(rows), device=cuda)
+
+    def program(a):
+        s = prims.reduce_sum(a, (0,), "float32")
+        return (a - prims.reduce_sum(a, (1,), "float32").reshape(rows, 1), s) if beside else s
+
+    s = lumen_b200.compile(program)(x)
+    s = torch.as_tensor(s[1] if beside else s, device=cuda)
+    want = x.double().sum(0)
+
+    def rms(t):
+        return float(((t.double() - want) ** 2).mean() ** 0.5)
+
+    assert rms(s) <= (1 + 3 / (2 * cols) ** 0.5) * rms(column_sums_in_slices(x))
