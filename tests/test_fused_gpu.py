@@ -354,3 +354,23 @@ def test_column_sums_are_as_exact_as_in_slices(cuda, rows, cols, beside):
         return float(((t.double() - want) ** 2).mean() ** 0.5)
 
     assert rms(s) <= (1 + 3 / (2 * cols) ** 0.5) * rms(column_sums_in_slices(x))
+
+
+# rows that one block of 288 to 384 threads would take with eight elements a thread, and the widths beside them
+@pytest.mark.parametrize("rows,cols", [(50, 2048), (50, 2052), (301, 2304), (40, 3001), (60, 3072), (33, 3076), (7, 2311)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_rows_between_one_and_two_blocks_an_sm(cuda, rows, cols, dtype):
+    """As test_row_and_column_reductions_in_one_kernel, the column sums no worse than twice the error of a tree over the rows."""
+    x = torch.randn((rows, cols), generator=torch.Generator(device=cuda).manual_seed(cols), device=cuda).to(getattr(torch, dtype))
+
+    def program(a):
+        w = a.to("float32")
+        c = w - prims.reduce_sum(w, (1,), "float32").reshape(rows, 1) * (1.0 / cols)
+        return c, prims.reduce_sum(w, (0,), "float32"), prims.reduce_sum(c * c, (0,), "float32")
+
+    c, s, q = Fusion(tracer.trace(program, (dtype, (rows, cols))))(x)
+    w = x.double()
+    want = w - w.mean(1, keepdim=True)
+    assert ((c.double() - want).abs() <= 1e-6 * want.abs() + 1e-5).all()
+    assert ((s.double() - w.sum(0)).abs() <= rows * 2.0**-24 * w.abs().sum(0)).all()
+    assert ((q.double() - (want * want).sum(0)).abs() <= (rows * 2.0**-24 + 1e-5) * (want * want).sum(0)).all()
