@@ -15,6 +15,8 @@ from __future__ import annotations
 
 from lumen_b200 import graph as G
 
+NARROW = frozenset(("bool", "int8", "uint8", "int16", "uint16", "float16", "bfloat16"))  # at most 16 bits an element
+
 # `gather` (rows of a table picked by an index tensor) is generated inside elementwise kernels like any other load
 ELEMENTWISE = set(G.ELEMENTWISE_BINARY) | set(G.FLOAT_UNARY) | set(G.ANY_UNARY) | {"cast", "select", "is_finite", "gather"}
 REDUCTIONS = {"reduce_sum", "reduce_max"}
@@ -137,9 +139,26 @@ class FusionPass:
         body, _, leaving = self.body_of(members)
         return bool(leaving) and self.accepts(body)
 
-    # Rows and columns reduced in one kernel leave a slice of partial column sums per block: that pays where it saves a pass
-    # over an operand in HBM, not over one that stays in the L2 anyway (below 256 KB).
+    # Rows and columns reduced in one kernel leave a slice of partial column sums per block and hold them in registers beside the
+    # row. Smaller operands than this are left apart (a line that was not drawn by time: one kernel is 0.5 to 0.9 of two there).
     SMALLEST_MIXED = 1 << 16
+
+    @staticmethod
+    def one_pass_pays(rows: int, cols: int, narrow: bool, row_sums: int) -> bool:
+        """Whether one kernel for row and column reductions of [rows, cols] is faster than separate ones, measured on 540 problems
+        (one kernel's time over the separate kernels'). `narrow`: 16-bit operands; `row_sums`: reductions over rows in it.
+
+        With several sums per row (a layer norm and its gradients) the separate kernels are many: 0.3 to 0.8 up to 8192
+        columns. Wider rows take blocks of 1024 threads whose 64 registers do not hold a row and its sums: float32 1.0 at
+        16384 columns, 1.2 at 32768; 16-bit 1.1 to 1.4 from 12288 columns on, 0.7 to 0.9 up to 24576 with a thousand rows and more.
+        One sum per row or none is two kernels, the second of which finds its operand in the L2: float32 0.6 to 1.1 up to 6144 columns, and
+        up to 16384 with a thousand rows and more (fewer: 1.1 to 1.6); 16-bit 0.6 to 1.0 up to 2^18 elements of narrow rows, 1.0 to
+        1.4 beyond (5.6 at 65536 columns), 0.7 to 0.9 again where the operand is larger than the L2 and rows are wide."""
+        if row_sums >= 2:
+            return cols <= (8192 if narrow else 16384) or (narrow and cols <= 24576 and rows >= 1024)
+        if narrow and cols % 4 == 0:
+            return (rows * cols <= 1 << 18 and cols <= 3072) or (rows * cols >= 1 << 26 and 8192 <= cols <= 16384)
+        return cols <= 6144 or (cols <= 16384 and rows >= 1024)
 
     def shares_well(self, members: list[int]) -> bool:
         def kind(m):
@@ -147,18 +166,26 @@ class FusionPass:
             if n.op not in REDUCTIONS:
                 return None
             x = self.g.types[n.inputs[0]]
-            return ("columns" if min(n.params["axes"]) == 0 and len(n.params["axes"]) < len(x.shape) else "rows"), x.numel
+            return ("columns" if min(n.params["axes"]) == 0 and len(n.params["axes"]) < len(x.shape) else "rows"), n
 
         kinds = [k for k in map(kind, members) if k]
-        columns = [size for which, size in kinds if which == "columns"]
-        if not columns or min(columns) >= self.SMALLEST_MIXED:
+        columns = [n for which, n in kinds if which == "columns"]
+        if not columns:
             return True
         behind: set[int] = set()  # values computed from a reduction
         for m in members:
             n = self.g.nodes[m]
             if n.op in REDUCTIONS or any(v in behind for v in n.inputs):
                 behind.add(n.output)
-        return len(columns) == len(kinds) and all(self.g.nodes[m].output in behind or not self.leaves(self.g.nodes[m].output, set(members)) for m in members)
+        if len(columns) == len(kinds) and all(self.g.nodes[m].output in behind or not self.leaves(self.g.nodes[m].output, set(members)) for m in members):
+            return True
+        sizes = [self.g.types[n.inputs[0]].numel for n in columns]
+        if min(sizes) < self.SMALLEST_MIXED:
+            return False
+        size, cols = sizes[0], self.g.types[columns[0].output].numel
+        _, operands, leaving = self.body_of(members)
+        narrow = any(self.g.types[v].numel == size and self.g.types[v].dtype in NARROW for v in (*operands, *leaving))
+        return self.one_pass_pays(size // max(cols, 1), cols, narrow, len(kinds) - len(columns))
 
     def can_join(self, group: _Group, i: int) -> bool:
         """Node `i` may join `group`: the group still runs before every reader of its values."""

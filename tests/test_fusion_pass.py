@@ -57,7 +57,7 @@ def test_softmax_row_is_one_fusion_and_a_reduction_keeps_its_epilogue():
     same_values(g, fused, [rng.standard_normal((32, 128), dtype=np.float32), rng.standard_normal((32, 128), dtype=np.float32)])
 
 
-def test_column_and_row_reductions_do_not_share_a_kernel():
+def test_small_column_and_row_reductions_do_not_share_a_kernel():
     def program(x):
         return F.sum(x, 0), F.sum(x, 1)
 
@@ -145,3 +145,55 @@ def test_any_number_of_column_reductions_of_one_operand_compiles(count, dtype, b
     assert not bare(fused)
     for f in fusions(fused):
         Fusion(f.params["body"])
+
+
+def row_and_column_sums(x):
+    return F.sum(x, 0), F.sum(x, 1)
+
+
+def relu_and_column_sums(x):
+    return F.relu(x), prims.reduce_sum(x, (0,), "float32")
+
+
+def norm_gradients(x, dy):
+    w, g = x.to("float32"), dy.to("float32")
+    m = F.sum(w, 1, keepdim=True) * (1.0 / x.shape[1])
+    r = F.rsqrt(F.sum((w - m) * (w - m), 1, keepdim=True) * (1.0 / x.shape[1]))
+    h = (w - m) * r
+    dx = r * (g - F.sum(g, 1, keepdim=True) * (1.0 / x.shape[1]) - h * (F.sum(g * h, 1, keepdim=True) * (1.0 / x.shape[1])))
+    return dx.to(x.dtype), F.sum(g * h, 0).to(x.dtype), F.sum(g, 0).to(x.dtype)
+
+
+@pytest.mark.parametrize("program,dtype,shape,together", [
+    (relu_and_column_sums, "float32", (4096, 4096), True),
+    (relu_and_column_sums, "float32", (256, 16384), False),   # 9 us apart, 13 together
+    (relu_and_column_sums, "float32", (2048, 16384), True),   # 68 and 52
+    (relu_and_column_sums, "float32", (256, 40000), False),   # 15 and 31
+    (relu_and_column_sums, "bfloat16", (256, 1024), True),
+    (relu_and_column_sums, "bfloat16", (1024, 1024), False),  # 5.6 and 7.9
+    (relu_and_column_sums, "bfloat16", (256, 40000), False),  # 11 and 39
+    (relu_and_column_sums, "bfloat16", (8192, 8192), True),   # 70 and 56: larger than the L2
+    (relu_and_column_sums, "bfloat16", (4096, 3001), True),   # 18 and 14
+    (norm_gradients, "float32", (8192, 1024), True),
+    (norm_gradients, "float32", (256, 32768), False),         # 167 and 187 (with its forward)
+    (norm_gradients, "bfloat16", (8192, 1024), True),
+    (norm_gradients, "bfloat16", (256, 16384), False),        # 49 and 61
+    (norm_gradients, "bfloat16", (1024, 16384), True),        # 166 and 124
+])
+def test_rows_and_columns_share_a_kernel_where_that_is_faster(program, dtype, shape, together):
+    from lumen_b200.runtime import Fusion
+
+    g = tracer.trace(program, *[(dtype, shape)] * program.__code__.co_argcount)
+    fused = fuse(g)
+    assert (len(fusions(fused)) == 1) == together and not bare(fused)
+    for f in fusions(fused):
+        Fusion(f.params["body"])
+
+
+@pytest.mark.parametrize("program", [row_and_column_sums, relu_and_column_sums, norm_gradients])
+def test_groups_joined_by_an_operand_give_the_same_values(program):
+    g = tracer.trace(program, *[("float32", (300, 260))] * program.__code__.co_argcount)
+    fused = fuse(g)
+    assert len(fusions(fused)) == 1
+    rng = np.random.default_rng(7)
+    same_values(g, fused, [rng.standard_normal((300, 260), dtype=np.float32) for _ in range(program.__code__.co_argcount)])
