@@ -1203,8 +1203,11 @@ class Generator {
             // this one's reads and one barrier is enough
             s << "    A* sm = (A*)smem; const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;\n";
             s << "    if (lane == 0) sm[warp] = v;\n    __syncthreads();\n";
-            if (T_ <= 256) {
-                s << "    v = sm[0];\n    #pragma unroll\n    for (int w = 1; w < " << T_ / 32 << "; w++) v = f(v, sm[w]);\n";
+            if (T_ <= 256) {  // every thread adds the warps' sums as the tree that the shuffles below are
+                int warps = T_ / 32, p = 1;
+                while (p < warps) p *= 2;
+                s << "    A w[" << p << "];\n    #pragma unroll\n    for (int k = 0; k < " << p << "; k++) w[k] = k < " << warps << " ? sm[k] : identity;\n";
+                s << "    #pragma unroll\n    for (int h = " << p / 2 << "; h >= 1; h /= 2) {\n        #pragma unroll\n        for (int k = 0; k < h; k++) w[k] = f(w[k], w[k + h]);\n    }\n    v = w[0];\n";
             } else {
                 s << "    v = lane < " << T_ / 32 << " ? sm[lane] : identity;\n";
                 s << "    #pragma unroll\n    for (int m = 16; m >= 1; m >>= 1) v = f(v, shfl_xor_any<A>(v, m));\n";

@@ -374,3 +374,24 @@ def test_rows_between_one_and_two_blocks_an_sm(cuda, rows, cols, dtype):
     assert ((c.double() - want).abs() <= 1e-6 * want.abs() + 1e-5).all()
     assert ((s.double() - w.sum(0)).abs() <= rows * 2.0**-24 * w.abs().sum(0)).all()
     assert ((q.double() - (want * want).sum(0)).abs() <= (rows * 2.0**-24 + 1e-5) * (want * want).sum(0)).all()
+
+
+@pytest.mark.parametrize("cols", [1024, 2048, 4096, 8192])
+def test_a_rows_warps_are_added_as_a_tree(cuda, cols):
+    """Row sums whose rows are taken by two to eight warps with four vectors of four a thread, bit for bit: a thread's elements in order,
+    lanes by xor 16, 8, 4, 2, 1 (pairs differ in the lane's highest bit first), warps likewise."""
+    x = torch.randn((70, cols), generator=torch.Generator(device=cuda).manual_seed(cols), device=cuda)
+    threads = cols // 16
+    v = x.reshape(70, 4, threads, 4)  # chunk, thread, element
+    total = torch.zeros((70, threads), device=cuda)
+    for chunk in range(4):
+        for e in range(4):
+            total = total + v[:, chunk, :, e]
+    total = total.reshape(70, -1, 32)
+    for half in (16, 8, 4, 2, 1):
+        total = total[..., :half] + total[..., half:]
+    total = total[..., 0]
+    while total.shape[1] > 1:
+        total = total[:, : total.shape[1] // 2] + total[:, total.shape[1] // 2 :]
+    s = Fusion(tracer.trace(lambda a: prims.reduce_sum(a, (1,), "float32"), ("float32", (70, cols))))(x)[0]
+    assert torch.equal(s, total[:, 0])
