@@ -466,12 +466,7 @@ class Generator {
         VEC_ = std::min(8, 16 / min_size);
         while (VEC_ > 1 && C_ % VEC_ != 0) VEC_ /= 2;
         int64_t nvec = std::max<int64_t>((C_ + VEC_ - 1) / VEC_, 1);
-        // Vectors of a row per thread: four of 16 bytes, more of the narrow ones that a width without a power of two allows - a
-        // row over 1024 threads of three 2-byte loads each is bound by its barriers and by loads in flight. The
-        // multiply-add-relu-square-sum chain, us, 4 -> 16 vectors of one element: 5000 x 3001 bfloat16 24.7 -> 20.0, 20000 x 513
-        // 22.7 -> 14.6, 60000 x 257 float32 27.8 -> 23.0 (100000 x 101 18.5 either way); 4 -> 8 of two: 5000 x 3002 float32
-        // 26.7 -> 21.1 (16: 24.9), bfloat16 12.6 either way.
-        const int64_t per = std::max(4, 16 / VEC_);
+        const int64_t per = vectors_per_thread(nvec);
         int64_t want = (nvec + per - 1) / per;
         T_ = 1;
         while (T_ < want && T_ < 1024) T_ *= 2;
@@ -509,6 +504,30 @@ class Generator {
             if (g_.type(v).numel() >= (1LL << 31) - 4096) wide_index_ = true;
         if (multi_) wide_index_ = true;  // a group's row count is a run-time value
         pair_ = VEC_ >= 2 && computes_bf16();
+    }
+
+    // Vectors of a row per thread: four of 16 bytes. Of the narrow ones that a width without a power of two allows, 16 (eight of
+    // two elements) where rows are long and many: a row over 1024 threads of three 2-byte loads each is bound by its barriers and by
+    // loads in flight, and a power of two of threads may leave a quarter to a half of them idle. The multiply-add-relu-square-sum
+    // chain, us, 4 -> 16 vectors of one element: 5000 x 3001 bfloat16 21.0 -> 16.6, 20000 x 513 18.5 -> 12.0, 5000 x 1025 10.7 -> 6.7,
+    // 100000 x 257 float32 42 -> 36; but 64 x 513 1.8 -> 1.9, 20000 x 511 12.1 -> 14.9, 20000 x 127 4.4 -> 7.0, 100000 x 31 5.4 -> 13.3 and 3 x 255 1.6 -> 3.2.
+    // Eight instead of 16 where those are slower: 5000 x 129 4.0 -> 2.8, 100000 x 65 12.7 -> 9.7. Each further reduction of a row (softmax,
+    // norms) adds barriers: 5000 x 3001 bfloat16 28.4 -> 14.8, 20000 x 511 12.8 -> 8.5. Rows without a reduction: 20000 x 1025 18.7 -> 16.2,
+    // 64 x 2047 1.4 -> 1.7.
+    int64_t vectors_per_thread(int64_t nvec) const {
+        if (VEC_ > 2) return 4;
+        if (!has_reduce_) return R_ * nvec >= 1 << 19 ? 16 / VEC_ : 4;
+        int row_sums = 0;
+        for (const Node& n : g_.nodes) row_sums += n.op == "reduce_sum" || n.op == "reduce_max";
+        const bool several = row_sums > 1;
+        if (R_ < (nvec > 1024 ? 256 : 512)) return 4;
+        if (VEC_ == 2) return nvec > (several ? 256 : 512) ? 8 : 4;
+        int64_t threads = 1;
+        while (threads < (nvec + 3) / 4) threads *= 2;
+        const bool idle = nvec * 4 < 3 * threads * ((nvec + threads - 1) / threads);  // over a quarter, with four vectors a thread
+        if (nvec > 1024 || (nvec > 256 && (idle || (several && R_ >= 4096))) || (nvec > 768 && (several || R_ >= 4096)) || (nvec > 96 && idle && several && R_ >= 4096)) return 16;
+        if ((nvec > 128 && nvec <= 256) || (nvec > 64 && idle && R_ >= (several ? 4096 : 16384))) return 8;
+        return 4;
     }
 
     // pair mode pays where packed bfloat16 instructions replace scalar ones
