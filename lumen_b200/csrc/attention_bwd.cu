@@ -34,12 +34,6 @@ namespace {
 
 using namespace sm100;
 
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 constexpr int BR = 128;  // resident rows (thread = row)
 // warp 0: TMA, warp 1: MMA + TMEM owner, then two compute warpgroups, each on half of the BT streamed columns of every
 // iteration. X is free as soon as every thread has loaded it: the next tile's X product is issued while this tile's

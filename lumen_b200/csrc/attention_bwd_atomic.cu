@@ -31,12 +31,6 @@ namespace {
 
 using namespace sm100;
 
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 constexpr int D = 64;        // head dim
 constexpr int BR = 128;      // resident key rows (thread = key row)
 constexpr int BT = 128;      // streamed query rows per iteration

@@ -18,9 +18,12 @@
 #include <mutex>
 
 #include "attention.h"
+#include "sm100.cuh"
 
 namespace lb {
 namespace {
+
+using namespace sm100;
 
 constexpr int kWarps = 4, kSlice = 16, kStages = 3, kMaxRows = 32, kMaxSplits = 16;
 
@@ -35,7 +38,6 @@ struct DecodeArgs {
     int pair_stores;  // the output's rows are 4-byte aligned
 };
 
-__device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void copy_16(uint32_t dst, const void* src, bool live) {  // zeros where there is no row
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
 }
@@ -51,11 +53,6 @@ __device__ __forceinline__ void mma_16816(float* c, const uint32_t* a, uint32_t 
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ float exp2_fast(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
 }
 __device__ __forceinline__ uint32_t pack(float lo, float hi) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
@@ -103,7 +100,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attention_decode_kernel(const 
     uint8_t* mine = ring + warp * (kStages * 2 * L::kTile);
     auto fetch = [&](int slice) {
         if (slice < last) {
-            const uint32_t at = smem_at(mine + (slice - first) % kStages * (2 * L::kTile));
+            const uint32_t at = smem_u32(mine + (slice - first) % kStages * (2 * L::kTile));
 #pragma unroll
             for (int i = 0; i < kSlice * (D / 8) / 32; i++) {
                 const int r = (i * 32 + lane) / (D / 8), c = (i * 32 + lane) % (D / 8);
@@ -123,7 +120,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attention_decode_kernel(const 
 #pragma unroll
     for (int t = 0; t < MT; t++)
 #pragma unroll
-        for (int k = 0; k < D / 16; k++) ldmatrix_x4(qf[t][k], smem_at(sq) + chunk_at<D>(t * 16 + (lane & 15), k * 2 + (lane >> 4)));
+        for (int k = 0; k < D / 16; k++) ldmatrix_x4(qf[t][k], smem_u32(sq) + chunk_at<D>(t * 16 + (lane & 15), k * 2 + (lane >> 4)));
     float acc[MT][D / 8][4] = {}, m[MT][2], l[MT][2];
     long long limit[MT][2];  // last visible key of this thread's two rows per tile
 #pragma unroll
@@ -138,7 +135,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attention_decode_kernel(const 
         copies_wait<kStages - 2>();
         __syncwarp();
         fetch(slice + kStages - 1);  // into the stage read in the last round
-        const uint32_t at = smem_at(mine + (slice - first) % kStages * (2 * L::kTile));
+        const uint32_t at = smem_u32(mine + (slice - first) % kStages * (2 * L::kTile));
         float s[MT][2][4] = {};
 #pragma unroll
         for (int k = 0; k < D / 16; k++) {
@@ -161,9 +158,9 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attention_decode_kernel(const 
                 top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
                 top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
                 const float m_new = fmaxf(m[t][h], top * p.scale_log2), shift = m_new == -INFINITY ? 0.0f : m_new;
-                const float alpha = exp2_fast(m[t][h] - shift);
+                const float alpha = fast_exp2(m[t][h] - shift);
 #pragma unroll
-                for (int i = 0; i < 4; i++) x[i] = exp2_fast(fmaf(x[i], p.scale_log2, -shift));  // rounded once, as in the tile kernel
+                for (int i = 0; i < 4; i++) x[i] = fast_exp2(fmaf(x[i], p.scale_log2, -shift));  // rounded once, as in the tile kernel
                 l[t][h] = l[t][h] * alpha + ((x[0] + x[1]) + (x[2] + x[3]));  // this thread's keys; the quad is added up at the end
                 pf[t][h] = pack(x[0], x[1]), pf[t][2 + h] = pack(x[2], x[3]);
                 m[t][h] = m_new;
@@ -200,7 +197,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attention_decode_kernel(const 
                 *(float2*)(merge + (warp * L::kRows + r) * D + d * 8 + (lane & 3) * 2) = make_float2(acc[t][d][2 * h], acc[t][d][2 * h + 1]);
         }
     __syncthreads();
-    auto weight = [](float part, float whole) { return part == -INFINITY ? 0.0f : exp2_fast(part - whole); };
+    auto weight = [](float part, float whole) { return part == -INFINITY ? 0.0f : fast_exp2(part - whole); };
     for (int i = threadIdx.x; i < rows * D; i += kWarps * 32) {
         const int r = i / D, d = i % D;
         float whole = -INFINITY, sum = 0.0f, o = 0.0f;
@@ -215,11 +212,11 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attention_decode_kernel(const 
         if (d == 0) max_w[kWarps * L::kRows + r] = whole, sum_w[kWarps * L::kRows + r] = sum;
     }
     // ---- the cluster's CTAs into one: each writes its share of the outputs ----
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_sync();
     auto remote = [](const float* at, int rank) {
         uint32_t there;
         float x;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(smem_at(at)), "r"(rank));
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(smem_u32(at)), "r"(rank));
         asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(there) : "memory");
         return x;
     };
@@ -240,7 +237,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attention_decode_kernel(const 
         // one rounding at the size of the result: (whole + log2f(sum)) * ln 2 has two, one of them at 1.44 times the size
         if (d == 0 && p.lse) p.lse[((long long)b * p.N + head) * p.Sq + position] = fmaf(whole, 0.6931471805599453f, logf(sum));
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // nobody leaves while it is read
+    cluster_sync();  // nobody leaves while it is read
 }
 
 // How the kernel does on a problem, in microseconds of a B200: a CTA costs `base + per_row * rows` (prologue, merge, the way out)

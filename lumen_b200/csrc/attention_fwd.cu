@@ -31,12 +31,6 @@ namespace {
 
 using namespace sm100;
 
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 constexpr int BQ = 128, BKV = 128;
 // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2..5: softmax (thread = query row). 256 tensor-memory columns (S 128,
 // O up to 128) and at most 96 KB of shared memory per CTA, so that TWO CTAs share an SM: one CTA's prologue, epilogue

@@ -110,6 +110,13 @@ __device__ __forceinline__ bool next_cta_answer(const void* slot, int& x) {
     return got != 0;
 }
 
+// ---- arithmetic ----
+__device__ __forceinline__ float fast_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // ---- registers ----
 // Register budget of the calling warpgroup (all four of its warps execute this). An increase draws on what the block was
 // launched with and waits until it is there: the warpgroups' budgets may not add up to more.
@@ -153,6 +160,7 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t desc_a, uint64
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader)
         : "memory");
 }
+// D[tmem] (+)= A[tmem] * B[smem]: the A operand (128 x 16 of 16-bit values per instruction) is read from tensor memory.
 __device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, bool leader) {
     asm volatile(
         "{\n\t.reg .pred p, e;\n\t"
@@ -173,15 +181,6 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar, bool leader) {
 // mbar_wait of a convergent warp with a warp-uniform answer.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
-}
-// D[tmem] (+)= A[tmem] * B[smem]: the A operand (128 x 16 of 16-bit values per instruction) is read from tensor memory.
-__device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
 }
 // Arrives on `bar` once every tcgen05.mma issued so far by this thread has completed (implies fence::before_thread_sync).
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
