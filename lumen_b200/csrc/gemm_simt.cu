@@ -84,7 +84,8 @@ template <> struct SimtVec<4> { typedef float4 type; };
 
 // A TM x TN output tile per CTA, RM x RN outputs per thread. Slices of SK contracting indices are double-buffered in shared
 // memory and the next one is in flight to registers meanwhile. Products and sums are rounded one by one in contracting
-// order. Indices past K are zeros on both sides, which leaves a sum as it is (a sum that starts from +0 is never -0).
+// order. A last slice that K does not fill is summed index by index: with a whole slice of zeros instead, 4096 x 4096 with K = 1
+// took 49 us against 20, 1024 x 1024 with K = 15 9.9 against 5.9.
 template <class T, int TM, int TN, int RM, int RN, int SK>
 __global__ void __launch_bounds__(TM / RM * (TN / RN)) gemm_simt_kernel(const T* __restrict__ a, const T* __restrict__ b, const SimtArgs p) {
     constexpr int THREADS = TM / RM * (TN / RN);
@@ -112,6 +113,18 @@ __global__ void __launch_bounds__(TM / RM * (TN / RN)) gemm_simt_kernel(const T*
         if (k0 + SK < p.K) {
             fa.fetch(ab, m0, p.M, k0 + SK, p.K, p.a_sm, p.a_sk, a_k, a_whole && k0 + 2 * SK <= p.K);
             fb.fetch(bb, n0, p.N, k0 + SK, p.K, p.b_sn, p.b_sk, b_k, b_whole && k0 + 2 * SK <= p.K);
+        }
+        if (p.K - k0 < SK) {  // the last slice of a K that is no multiple: only its indices
+#pragma unroll 4
+            for (int k = 0; k < p.K - k0; k++) {
+                const VecA a1 = *(const VecA*)(sa[buf] + SliceA::slot(k, ty * RM));
+                const VecB b1 = *(const VecB*)(sb[buf] + SliceB::slot(k, tx * RN));
+#pragma unroll
+                for (int i = 0; i < RM; i++)
+#pragma unroll
+                    for (int j = 0; j < RN; j++) acc[i][j] = __fadd_rn(acc[i][j], __fmul_rn(((const float*)&a1)[i], ((const float*)&b1)[j]));
+            }
+            break;
         }
         // 32 indices unrolled: the row permutation has that period, so its XORs become eight precomputed addresses per
         // operand. Values are read from shared memory a group of four indices ahead of their use.

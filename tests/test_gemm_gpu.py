@@ -36,7 +36,7 @@ def test_float32_gemm_is_bit_exact(cuda, shape):
     np.testing.assert_array_equal(to_numpy(out), oracle_matmul(a, b, "float32", "float32"))
 
 
-@pytest.mark.parametrize("shape", [(16, 32, 64), (17, 33, 65), (400, 410, 70), (416, 384, 128), (1100, 1121, 33), (1152, 1152, 64)])
+@pytest.mark.parametrize("shape", [(300, 320, 1), (1100, 1121, 3), (400, 410, 15), (40, 70, 63), (16, 32, 64), (17, 33, 65), (400, 410, 70), (416, 384, 128), (1100, 1121, 33), (1152, 1152, 64)])
 @pytest.mark.parametrize("majors", ["nn", "nt", "tn", "tt"])
 def test_float32_gemm_tiles_and_majors_are_bit_exact(cuda, shape, majors):
     """Each tile size the CUDA-core kernel picks (few, some, many output tiles), whole and ragged, with either operand
