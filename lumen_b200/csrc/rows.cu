@@ -154,6 +154,7 @@ struct AttnShape {
     int causal;
     long long offset;
     float scale;
+    int tile_rows;  // CUDA-core attention: rows of the streamed tiles in shared memory (launch_attn)
 };
 
 // CUDA-core attention: one warp per row (a query of the forward and dQ kernels, a key of the dK/dV kernel), eight
@@ -165,22 +166,39 @@ struct AttnShape {
 constexpr int kAttnRows = 8, kChunk = 32;
 
 // DU: head-dim elements per lane. Row pitch: a multiple of four floats whose 16-byte groups fall in different banks for
-// eight neighbouring rows.
+// eight neighbouring rows. The streamed tiles have as many rows as there are to stream, at most a chunk: with full tiles of
+// zeros, which left room for two blocks an SM, 1024 heads of one query and one key of 256 elements took 34 us (now 12; one row at a time,
+// without shared memory, 3.6: seven of a block's eight warps idle there), of eight 43 us (now 26), of 16 89 us (now 62).
 template <int DU>
 struct AttnSmem {
     static constexpr int kD = DU * 32, kPitch = kD + 4;
-    float tile[2][kChunk * kPitch];   // streamed rows
-    float own[2][kAttnRows * kD];     // the warps' rows
-    float weight[2][kAttnRows][kChunk];
+    float (*weight)[kAttnRows][kChunk];  // [2]
+    float* own[2];                       // the warps' rows, kD apart
+    float* tile[2];                      // streamed rows, kPitch apart
+    __device__ __forceinline__ AttnSmem(uint8_t* raw, int tile_rows) {
+        weight = (float(*)[kAttnRows][kChunk])raw;
+        own[0] = (float*)raw + 2 * kAttnRows * kChunk, own[1] = own[0] + kAttnRows * kD;
+        tile[0] = own[1] + kAttnRows * kD, tile[1] = tile[0] + tile_rows * kPitch;
+    }
+    static int bytes(int tile_rows) { return (2 * kAttnRows * (kChunk + kD) + 2 * tile_rows * kPitch) * (int)sizeof(float); }
 };
 
+// Rows [row0, row0 + kChunk) of those before `end`; nothing is stored for the others, which no lane may then read. Unrolled to eight
+// elements at most: a whole chunk of 256-wide rows held 32, and with 170 to 210 registers a thread one block an SM (head dim 256, 8 heads x
+// 1024: 900 -> 669 us forward, 2238 -> 1824 backward).
 template <class T, int DU>
 __device__ __forceinline__ void load_chunk(float* dst, const T* base, long long stride, long long row0, long long end, int D) {
     constexpr int kD = AttnSmem<DU>::kD;
-#pragma unroll
-    for (int i = threadIdx.x; i < kChunk * kD; i += kAttnRows * 32) {
+    auto element = [&](int i) {
         const int r = i / kD, d = i % kD;
-        dst[r * AttnSmem<DU>::kPitch + d] = row0 + r < end && d < D ? to_f(base[(row0 + r) * stride + d]) : 0.0f;
+        dst[r * AttnSmem<DU>::kPitch + d] = d < D ? to_f(base[(row0 + r) * stride + d]) : 0.0f;
+    };
+    if (end - row0 >= kChunk) {
+#pragma unroll (DU > 2 ? 8 : 4 * DU)
+        for (int i = threadIdx.x; i < kChunk * kD; i += kAttnRows * 32) element(i);
+    } else {
+#pragma unroll 2
+        for (int i = threadIdx.x; i < (int)(end - row0) * kD; i += kAttnRows * 32) element(i);
     }
 }
 template <class T, int DU>
@@ -257,7 +275,7 @@ __global__ void __launch_bounds__(kAttnRows * 32)
 attention_simt_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ o,
                           float* __restrict__ lse, AttnShape s) {
     extern __shared__ __align__(16) uint8_t raw[];
-    AttnSmem<DU>& sm = *(AttnSmem<DU>*)raw;
+    AttnSmem<DU> sm(raw, s.tile_rows);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int i0, n, b;
     block_rows(s.Sq, s.N, i0, n, b);
@@ -307,7 +325,7 @@ __global__ void __launch_bounds__(kAttnRows * 32)
 attention_simt_dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ g,
                          const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dq, AttnShape s) {
     extern __shared__ __align__(16) uint8_t raw[];
-    AttnSmem<DU>& sm = *(AttnSmem<DU>*)raw;
+    AttnSmem<DU> sm(raw, s.tile_rows);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int i0, n, b;
     block_rows(s.Sq, s.N, i0, n, b);
@@ -350,7 +368,7 @@ __global__ void __launch_bounds__(kAttnRows * 32)
 attention_simt_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ g,
                            const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dk, T* __restrict__ dv, AttnShape s) {
     extern __shared__ __align__(16) uint8_t raw[];
-    AttnSmem<DU>& sm = *(AttnSmem<DU>*)raw;
+    AttnSmem<DU> sm(raw, s.tile_rows);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int k0, nk, b;
     block_rows(s.Sk, s.Nkv, k0, nk, b);
@@ -658,12 +676,13 @@ unsigned attn_blocks(long long batch, long long heads, long long rows) {
     if (blocks > INT32_MAX) fail(LB_ERR_UNSUPPORTED, "attention: too many rows for the CUDA-core kernels' grid");
     return (unsigned)blocks;
 }
+// `streamed`: the rows that the kernel walks per head
 template <int DU, class Kernel, class... Args>
-void launch_attn(Kernel kernel, unsigned blocks, cudaStream_t st, Args... args) {
-    constexpr int bytes = (int)sizeof(AttnSmem<DU>);
-    if (bytes > 48 * 1024 && first_use_on_device((const void*)kernel))
-        LB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    kernel<<<blocks, kAttnRows * 32, bytes, st>>>(args...);
+void launch_attn(Kernel kernel, unsigned blocks, int streamed, cudaStream_t st, AttnShape s, Args... args) {
+    if (AttnSmem<DU>::bytes(kChunk) > 48 * 1024 && first_use_on_device((const void*)kernel))
+        LB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnSmem<DU>::bytes(kChunk)));
+    s.tile_rows = std::min(kChunk, (std::max(streamed, 1) + 3) / 4 * 4);
+    kernel<<<blocks, kAttnRows * 32, AttnSmem<DU>::bytes(s.tile_rows), st>>>(args..., s);
 }
 // calls `f` with the head-dim elements per lane as a compile-time number: 1, 2, 4 or 8
 template <class F>
@@ -676,7 +695,7 @@ void with_dims_per_lane(int D, F&& f) {
 template <class T>
 void simt_fwd(const AttnShape& s, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o, float* lse, cudaStream_t st) {
     with_dims_per_lane(s.D, [&](auto du) {
-        launch_attn<du>(attention_simt_fwd_kernel<T, du>, attn_blocks(s.B, s.N, s.Sq), st, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr, (T*)o.ptr, lse, s);
+        launch_attn<du>(attention_simt_fwd_kernel<T, du>, attn_blocks(s.B, s.N, s.Sq), s.Sk, st, s, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr, (T*)o.ptr, lse);
     });
 }
 template <class T>
@@ -685,10 +704,10 @@ void simt_bwd(const AttnShape& s, const lb_tensor& q, const lb_tensor& k, const 
     const long long warps = (long long)s.B * s.N * s.Sq;
     attention_delta_simt<T><<<(unsigned)((warps * 32 + 255) / 256), 256, 0, st>>>((const T*)o.ptr, (const T*)g.ptr, delta, s);
     with_dims_per_lane(s.D, [&](auto du) {
-        launch_attn<du>(attention_simt_dq_kernel<T, du>, attn_blocks(s.B, s.N, s.Sq), st, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr,
-                        (const T*)g.ptr, lse, (const float*)delta, (T*)dq.ptr, s);
-        launch_attn<du>(attention_simt_dkdv_kernel<T, du>, attn_blocks(s.B, s.Nkv, s.Sk), st, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr,
-                        (const T*)g.ptr, lse, (const float*)delta, (T*)dk.ptr, (T*)dv.ptr, s);
+        launch_attn<du>(attention_simt_dq_kernel<T, du>, attn_blocks(s.B, s.N, s.Sq), s.Sk, st, s, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr,
+                        (const T*)g.ptr, lse, (const float*)delta, (T*)dq.ptr);
+        launch_attn<du>(attention_simt_dkdv_kernel<T, du>, attn_blocks(s.B, s.Nkv, s.Sk), s.Sq, st, s, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr,
+                        (const T*)g.ptr, lse, (const float*)delta, (T*)dk.ptr, (T*)dv.ptr);
     });
 }
 }  // namespace

@@ -285,7 +285,12 @@ SIMT_CASES = [((1, 8, 32, 1, 1, 32), True), ((2, 9, 33, 2, 1, 33), True), ((1, 7
               ((1, 40, 40, 4, 2, 129), True), ((1, 33, 70, 1, 1, 256), True)]
 
 
-@pytest.mark.parametrize("case", SIMT_CASES)
+# ... and of few rows with few to stream: tiles of as many rows as are streamed
+SIMT_SHORT_CASES = [((40, 1, 1, 8, 8, 256), True), ((3, 2, 5, 4, 2, 128), False), ((2, 3, 16, 2, 1, 64), True), ((2, 5, 17, 2, 1, 64), True),
+                    ((2, 16, 3, 2, 2, 200), False), ((1, 31, 31, 2, 1, 256), True)]
+
+
+@pytest.mark.parametrize("case", SIMT_CASES + SIMT_SHORT_CASES)
 def test_cuda_core_attention_against_float64(cuda, case):
     """float32 operands: every result within 2e-5 of its largest value. A score is a float32 sum of H <= 256 products of
     size about 1 / sqrt(H) each (error under 256 * 2^-24 = 1.5e-5 of a score, typically its square root), and __expf is
