@@ -379,10 +379,6 @@ class Generator {
     // outputs among them by position.
     std::set<int> behind_columns_;
     std::vector<int> column_outputs_;
-    // Values of a phase that a later phase of the same row reads again and that cost more to compute than to keep: by
-    // key, the row-scope array they are kept in.
-    std::map<std::string, std::string> kept_;
-    int kept_regs_ = 0;
     int resident_ = 1;  // CTAs per SM a kernel with column sums is built for and launched with
 
     std::string fresh(const char* prefix) { return format("%s%d", prefix, counter_++); }
@@ -474,7 +470,7 @@ class Generator {
         if (T_ > 32) RPB_ = 1;
         else RPB_ = std::max(1, 256 / T_);
         if (mixed_) {
-            // Column sums and kept values live in registers beside the row: eight elements of a row per thread where a
+            // Column sums live in registers beside the row: eight elements of a row per thread where a
             // block can be that wide. Residual + layer norm forward and backward of 8192 x 1024 bfloat16 in one such kernel:
             // 31 us + 6 us for its totals, against 125 us for the nine kernels of one kind of reduction each; bound by
             // instructions in flight (63 per element, issued 43 % of the time; with 16 elements it spills: 59 us; with four,
@@ -856,34 +852,9 @@ class Generator {
         std::string key = key_of(v, idx);
         auto it = ph.memo.find(key);
         if (it != ph.memo.end()) return it->second;
-        std::string name = kept(v, key, idx, ph);
-        if (name.empty()) name = gen_uncached(v, idx, ph);
+        std::string name = gen_uncached(v, idx, ph);
         ph.memo[key] = name;
         return name;
-    }
-
-    // The value from an earlier phase's registers, or "" where it is computed (again): divisions and functions of float32
-    // elements, while they fit 64 registers per thread.
-    std::string kept(int v, const std::string& key, const Index& idx, Phase& ph) {
-        static const std::set<std::string> costly = {"div", "exp", "log", "sqrt", "rsqrt", "tanh", "logistic", "exp2", "log2", "sin", "cos", "pow"};
-        const Node* n = g_.node_of(v);
-        if (!n || column_mode_ || !ph.chunked || !e_dep(idx) || g_.type(v).dtype != LB_F32 || !costly.count(n->op)) return "";
-        if (n->op == "exp" && normaliser_term(*n)) return "";
-        for (Phase& before : phases_) {
-            if (!before.chunked || !before.memo.count(key)) continue;
-            auto it = kept_.find(key);
-            if (it == kept_.end()) {
-                if (kept_regs_ + NCH_ * VEC_ > 64) return "";
-                kept_regs_ += NCH_ * VEC_;
-                it = kept_.emplace(key, fresh("kept")).first;
-                row_decls_ += format("float %s[NCH][VEC];\n", it->second.c_str());
-                const std::string& name = before.memo[key];
-                before.body += pair_ ? both_lanes(format("%s[ch][e] = LX(%s);\n", it->second.c_str(), name.c_str()))
-                                     : format("%s[ch][e] = %s;\n", it->second.c_str(), name.c_str());
-            }
-            return define(ph, "float", it->second + "[ch][e]", true, nullptr, LB_F32);
-        }
-        return "";
     }
 
     // the index of a column reduction's operand at row r, column c0 + e
