@@ -96,7 +96,9 @@ int lb_launch_fused(const char* body_text, const lb_tensor* tensors, int n_input
  * transposed views the same way (lumen/codegen/dot_general/cuda/mod.rs:722-732). Accumulation is float32; the
  * product is written row-major as float32 or rounded once to the operands' dtype. bfloat16 and float16 operands run on
  * the tcgen05/TMEM/TMA kernels; float32 operands (and layouts TMA cannot address) run on a CUDA-core kernel that
- * accumulates in contracting order exactly like the reference interpreter (no hidden TF32 narrowing). */
+ * accumulates in contracting order exactly like the reference interpreter (no hidden TF32 narrowing). The tensor-core
+ * kernels repeat bit for bit on the same problem; how many K ranges they add up depends on M, N, K, the batch and the GPU's
+ * number of SMs, so the rows of a product may differ in the last bit from those of the same rows in a larger one. */
 /* Epilogues applied after the float32 accumulation, spelled as the primitives they stand for so that results equal
  * the unfused program's: RELU = max(acc, 0) before the output rounding; ADD = round(round(acc) + aux); MASK_POSITIVE
  * = aux > 0 ? round(acc) : 0 (the backward of a relu whose output is `aux`). ADD and MASK_POSITIVE take `aux`, a

@@ -159,7 +159,9 @@ def gemm(a, b, out, epilogue=None, kernel="auto", stream=None, scratch=None, aux
     """`out[.., M, N] = a[.., M, K] @ b[.., K, N]` with float32 accumulation through `lb_gemm`. `a` and `b` may be
     transposed views (any unit-stride major); `out` is float32 or the operands' dtype, row-major. `scratch` (a
     uint8 tensor of `gemm_scratch_bytes` bytes) lets few-tile, long-K problems split K. Epilogues: "relu";
-    "add" (`round(product) + aux`) and "mask_positive" (`aux > 0 ? round(product) : 0`) with `aux` shaped like `out`."""
+    "add" (`round(product) + aux`) and "mask_positive" (`aux > 0 ? round(product) : 0`) with `aux` shaped like `out`.
+    Bit-identical from call to call; the same rows in a larger product may differ in the last bit (another number of K
+    ranges, which depends on every dimension)."""
     require_cuda()
     scratch_ptr, scratch_bytes = (scratch.data_ptr(), scratch.numel() * scratch.element_size()) if scratch is not None else (0, 0)
     _lib.host().gemm(a, b, out, aux, EPILOGUES[epilogue], GEMM_KERNELS[kernel], scratch_ptr, scratch_bytes, _stream(stream))
@@ -173,7 +175,9 @@ def device_status() -> None:
 
 def attention_forward(q, k, v, scale=None, causal=False, out=None, lse=None, stream=None):
     """Flash attention forward through `lb_attention_fwd`: `q` [B, Sq, N, H], `k`/`v` [B, Sk, Nkv, H] bfloat16 views;
-    returns `(o, lse)` with `o` [B, Sq, N, H] bfloat16 and `lse` [B, N, Sq] float32."""
+    returns `(o, lse)` with `o` [B, Sq, N, H] bfloat16 and `lse` [B, N, Sq] float32. Bit-identical from call to call; the
+    same sequence in another batch may differ by a rounding of the probabilities to bfloat16 (another kernel, or another
+    number of key ranges when few queries meet many keys)."""
     require_cuda()
     b, sq, n, h = q.shape
     sk = k.shape[1]
