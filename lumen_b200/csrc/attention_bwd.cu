@@ -20,6 +20,7 @@
 #include <type_traits>
 
 #include "device.h"
+#include "launch.cuh"
 #include "sm100.cuh"
 
 namespace lb {
@@ -175,6 +176,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    grid_wait();
     const uint32_t tmem_x = tmem_base;
     const uint32_t tmem_y = tmem_base + BT;
     const uint32_t tmem_a = tmem_base + 2 * BT;  // acc_a: D columns
@@ -505,6 +507,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
 __global__ void __launch_bounds__(256) attention_delta(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                                                         float* __restrict__ delta, int S, int N, int D, int n_shift, long long o_sb,
                                                         long long o_ss, long long o_sn, long long g_sb, long long g_ss, long long g_sn) {
+    grid_wait();
     const int lanes = D >> 3;  // 8 (D = 64) or 16 (D = 128)
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned row = t / (unsigned)lanes;  // (s, n) of this batch entry; lanes is a power of two
@@ -538,10 +541,8 @@ void launch_delta(const lb_tensor& o, const lb_tensor& d_o, float* delta, cudaSt
     for (int k = 0; k < 31; k++)
         if ((1LL << k) == N) n_shift = k;
     const unsigned blocks = (unsigned)((S * N * (D / 8) + 255) / 256);
-    attention_delta<<<dim3(blocks, (unsigned)B), 256, 0, s>>>((const __nv_bfloat16*)o.ptr, (const __nv_bfloat16*)d_o.ptr, delta, (int)S, (int)N,
-                                                              (int)D, n_shift, o.stride[0], o.stride[1], o.stride[2], d_o.stride[0],
-                                                              d_o.stride[1], d_o.stride[2]);
-    LB_CUDA(cudaGetLastError());
+    launch_overlapped(attention_delta, dim3(blocks, (unsigned)B), dim3(256), 0, s, 0, (const __nv_bfloat16*)o.ptr, (const __nv_bfloat16*)d_o.ptr, delta,
+                      (int)S, (int)N, (int)D, n_shift, o.stride[0], o.stride[1], o.stride[2], d_o.stride[0], d_o.stride[1], d_o.stride[2]);
 }
 
 template <int D, bool DKDV, int BT>
@@ -550,7 +551,7 @@ void launch_bwd_kernel(const CUtensorMap& r1, const CUtensorMap& r2, const CUten
     using C = BwdConfig<D, DKDV, BT>;
     if (first_use_on_device((const void*)attention_bwd_kernel<D, DKDV, BT>))
         LB_CUDA(cudaFuncSetAttribute(attention_bwd_kernel<D, DKDV, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kBytes));
-    attention_bwd_kernel<D, DKDV, BT><<<grid, C::kThreads, C::kBytes, s>>>(r1, r2, t1, t2, p);
+    launch_overlapped(attention_bwd_kernel<D, DKDV, BT>, grid, dim3(C::kThreads), C::kBytes, s, 0, r1, r2, t1, t2, p);
 }
 
 // The two kernels; `rows` makes the map of an operand's tiles, 128 or 64 rows high. Head dim 64 streams 64 rows a tile. Head dim 128
@@ -636,7 +637,6 @@ void attention_bwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor
         return;
     }
     launch_bwd(D, attention_map_rows, q, d_o, k, v, kv, qq, s);
-    LB_CUDA(cudaGetLastError());
 }
 
 }  // namespace lb
@@ -779,7 +779,6 @@ void attention_bwd_static(const lb_attn_desc& desc, const lb_tensor& q, const lb
     kv.out_b = dv.ptr, kv.b_sb = dv.stride[0], kv.b_ss = dv.stride[1], kv.b_sn = dv.stride[2];
     qq.out_a = dq.ptr, qq.a_sb = dq.stride[0], qq.a_ss = dq.stride[1], qq.a_sn = dq.stride[2];
     launch_bwd(D, [&](const lb_tensor& t, const char* what, int box_rows) { return static_map(st, t, what, box_rows); }, q, d_o, k, v, kv, qq, s);
-    LB_CUDA(cudaGetLastError());
 }
 
 }  // namespace

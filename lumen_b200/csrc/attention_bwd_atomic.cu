@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "device.h"
+#include "launch.cuh"
 #include "sm100.cuh"
 
 namespace lb {
@@ -141,6 +142,7 @@ attention_bwd_atomic_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    grid_wait();
     const uint32_t tmem_x = tmem_base, tmem_y = tmem_base + 128, tmem_dk = tmem_base + 256, tmem_dv = tmem_base + 320;
     const uint32_t tmem_dq = tmem_base + 384, tmem_p = tmem_base + 448;
 
@@ -435,6 +437,7 @@ attention_bwd_atomic_kernel(const __grid_constant__ CUtensorMap map_k, const __g
 // dq[b, s, n, :] = bf16(acc[b, s, n, :]): 8 values (32 bytes in, 16 out) per thread; the accumulator is dense, dq a view.
 __global__ void __launch_bounds__(256) attention_dq_round(const float* __restrict__ acc, uint16_t* __restrict__ dq, long long rows, int N,
                                                            long long sb_rows, long long q_sb, long long q_ss, long long q_sn) {
+    grid_wait();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long r = t >> 3;  // (b, s, n) row of 64 values
     const int part = (int)(t & 7);
@@ -494,12 +497,10 @@ void attention_bwd_atomic_launch(const lb_attn_desc& desc, const CUtensorMap& mk
     LB_CUDA(cudaMemsetAsync(dq_acc, 0, (size_t)B * Sq * N * D * 4, s));
     dim3 grid((unsigned)((Sk + BR - 1) / BR), (unsigned)Nkv, (unsigned)B);
     if (((uintptr_t)dq_acc & 15) != 0) fail(LB_ERR_UNSUPPORTED, "attention backward: the dQ accumulator must be 16-byte aligned");
-    attention_bwd_atomic_kernel<<<grid, kThreads, kSmemBytes, s>>>(mk, mv, mq, mdo, make_acc_map(dq_acc, B, Sq, N), a);
-    LB_CUDA(cudaGetLastError());
+    launch_overlapped(attention_bwd_atomic_kernel, grid, dim3(kThreads), kSmemBytes, s, 0, mk, mv, mq, mdo, make_acc_map(dq_acc, B, Sq, N), a);
     const long long rows = B * Sq * N;
-    attention_dq_round<<<(unsigned)((rows * 8 + 255) / 256), 256, 0, s>>>(dq_acc, (uint16_t*)dq.ptr, rows, (int)N, Sq, dq.stride[0], dq.stride[1],
-                                                                           dq.stride[2]);
-    LB_CUDA(cudaGetLastError());
+    launch_overlapped(attention_dq_round, dim3((unsigned)((rows * 8 + 255) / 256)), dim3(256), 0, s, 0, dq_acc, (uint16_t*)dq.ptr, rows, (int)N, Sq, dq.stride[0],
+                      dq.stride[1], dq.stride[2]);
 }
 
 }  // namespace lb

@@ -18,6 +18,7 @@
 #include <mutex>
 
 #include "attention.h"
+#include "launch.cuh"
 #include "sm100.cuh"
 
 namespace lb {
@@ -84,6 +85,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) attention_decode_kernel(const 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int split = blockIdx.x, splits = gridDim.x, kv = blockIdx.y, b = blockIdx.z;
     const int group = p.N / p.Nkv, rows = group * p.Sq;  // row r: query head kv * group + r % group, position r / group
+    grid_wait();
 
     for (int i = threadIdx.x; i < L::kRows * (D / 8); i += kWarps * 32) {
         const int r = i / (D / 8), c = i % (D / 8);
@@ -299,13 +301,7 @@ void launch(const DecodeArgs& p, int batch, long long keys, cudaStream_t s) {
         LB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     }
     const int splits = resident_splits<D, MT>(pick_splits(decode_cost(D, MT), (long long)batch * p.Nkv, keys, device_info().sms));
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = (unsigned)splits, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)splits, (unsigned)p.Nkv, (unsigned)batch), cfg.blockDim = dim3(kWarps * 32), cfg.dynamicSmemBytes = bytes, cfg.stream = s;
-    cfg.attrs = &attr, cfg.numAttrs = 1;
-    LB_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
+    launch_overlapped(kernel, dim3((unsigned)splits, (unsigned)p.Nkv, (unsigned)batch), dim3(kWarps * 32), bytes, s, (unsigned)splits, p);
 }
 
 }  // namespace

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "attention.h"
+#include "launch.cuh"
 #include "sm100.cuh"
 
 namespace lb {
@@ -282,6 +283,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    grid_wait();
     // At head dim 64 the CTA's 256 columns hold S (128), O (64) and P (64) side by side: S is free as soon as the
     // softmax threads have loaded it, so S(j + 1) is computed during softmax(j) instead of behind P(j) V(j).
     // At head dim 128 P overwrites the first 64 columns of S.
@@ -485,6 +487,7 @@ attention_fwd_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    grid_wait();
     const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 256;  // S(t) at + 128 t, O(t) at + D t
     const uint32_t tmem_p = kSeparateP ? tmem_base + 256 + 2 * D : tmem_s;
     constexpr uint32_t kPStep = kSeparateP ? 64 : 128;
@@ -659,7 +662,7 @@ void launch_fwd_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
     p.tiles = (p.Sq + 2 * BQ - 1) / (2 * BQ);
     const long long heads = (long long)p.B * p.N, bytes_per_head = std::max(1LL, (long long)p.Sk * D * 4 * p.Nkv / p.N);
     p.heads_at_once = (int)std::min(heads, std::max(1LL, (48LL << 20) / bytes_per_head));
-    attention_fwd_pair_kernel<D><<<(unsigned)(heads * p.tiles), kPairThreads, kBytes, s>>>(mq, mk, mv, p);
+    launch_overlapped(attention_fwd_pair_kernel<D>, dim3((unsigned)(heads * p.tiles)), dim3(kPairThreads), kBytes, s, 0, mq, mk, mv, p);
 }
 
 // 4-d tensor map over a [B, S, N, H] view: dims innermost first {H, N, S, B}; box = 64 head-dim elements x `box_rows` rows.
@@ -787,20 +790,18 @@ void attention_fwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor
     if (kernel == ATTN_TWO_TILES && (D == 128 ? pair_has_registers<128>() : pair_has_registers<64>())) {  // else the one-tile kernel does as well
         if (D == 128) launch_fwd_pair<128>(mq, mk, mv, p, s);
         else launch_fwd_pair<64>(mq, mk, mv, p, s);
-        LB_CUDA(cudaGetLastError());
         return;
     }
     // One warpgroup, O in tensor memory, two CTAs per SM: two K/V stages at head dim 64, one at head dim 128 (96 KB per CTA)
     if (D == 128) {
         if (first_use_on_device((const void*)attention_fwd_kernel<128, 1>))
             LB_CUDA(cudaFuncSetAttribute(attention_fwd_kernel<128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem<128, 1>::kBytes));
-        attention_fwd_kernel<128, 1><<<grid, kThreads, FwdSmem<128, 1>::kBytes, s>>>(mq, mk, mv, p);
+        launch_overlapped(attention_fwd_kernel<128, 1>, grid, dim3(kThreads), FwdSmem<128, 1>::kBytes, s, 0, mq, mk, mv, p);
     } else {
         if (first_use_on_device((const void*)attention_fwd_kernel<64, 2>))
             LB_CUDA(cudaFuncSetAttribute(attention_fwd_kernel<64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem<64, 2>::kBytes));
-        attention_fwd_kernel<64, 2><<<grid, kThreads, FwdSmem<64, 2>::kBytes, s>>>(mq, mk, mv, p);
+        launch_overlapped(attention_fwd_kernel<64, 2>, grid, dim3(kThreads), FwdSmem<64, 2>::kBytes, s, 0, mq, mk, mv, p);
     }
-    LB_CUDA(cudaGetLastError());
 }
 
 }  // namespace lb

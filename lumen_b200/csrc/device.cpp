@@ -31,7 +31,7 @@ const Driver& driver() {
     };
     get("cuModuleLoadData", (void**)&d.cuModuleLoadData);
     get("cuModuleGetFunction", (void**)&d.cuModuleGetFunction);
-    get("cuLaunchKernel", (void**)&d.cuLaunchKernel);
+    get("cuLaunchKernelEx", (void**)&d.cuLaunchKernelEx);
     get("cuFuncSetAttribute", (void**)&d.cuFuncSetAttribute);
     get("cuGetErrorString", (void**)&d.cuGetErrorString);
     get("cuTensorMapEncodeTiled", (void**)&d.cuTensorMapEncodeTiled);

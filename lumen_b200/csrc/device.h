@@ -22,8 +22,7 @@ namespace lb {
 struct Driver {
     CUresult (*cuModuleLoadData)(CUmodule*, const void*);
     CUresult (*cuModuleGetFunction)(CUfunction*, CUmodule, const char*);
-    CUresult (*cuLaunchKernel)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned,
-                               CUstream, void**, void**);
+    CUresult (*cuLaunchKernelEx)(const CUlaunchConfig*, CUfunction, void**, void**);
     CUresult (*cuFuncSetAttribute)(CUfunction, CUfunction_attribute, int);
     CUresult (*cuGetErrorString)(CUresult, const char**);
     CUresult (*cuTensorMapEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

@@ -34,6 +34,19 @@ static lb_fusion* compile(const std::string& text) {
     return raw;
 }
 
+// Launches a generated kernel so that it may become resident while the kernel before it in the stream still runs: its first
+// instruction waits for that one (the generated grid_wait; launch.cuh says what the two rely on).
+static void launch_kernel(CUfunction fn, int64_t grid_x, int64_t grid_y, int threads, void* stream, void** params, const char* what) {
+    CUlaunchAttribute attr = {};
+    attr.id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+    attr.value.programmaticStreamSerializationAllowed = 1;
+    CUlaunchConfig cfg = {};
+    cfg.gridDimX = (unsigned)grid_x, cfg.gridDimY = (unsigned)grid_y, cfg.gridDimZ = 1;
+    cfg.blockDimX = (unsigned)threads, cfg.blockDimY = cfg.blockDimZ = 1;
+    cfg.hStream = (CUstream)stream, cfg.attrs = &attr, cfg.numAttrs = 1;
+    check_cu(driver().cuLaunchKernelEx(&cfg, fn, params, nullptr), what);
+}
+
 static void launch(lb_fusion* f, const lb_tensor* tensors, int n, void* scratch, void* stream) {
     const FusedKernel& k = f->kernel;
     if (k.multi) fail(LB_ERR_INVALID, "this kernel was generated in horizontal form (option multi): launch it with a table of groups");
@@ -66,20 +79,14 @@ static void launch(lb_fusion* f, const lb_tensor* tensors, int n, void* scratch,
         if (k.cols == 0) return;
         if (((uintptr_t)scratch & 15) != 0) fail(LB_ERR_INVALID, "fusion scratch must be 16-byte aligned");
         params.push_back(&scratch);
-        check_cu(driver().cuLaunchKernel(fn.function, (unsigned)k.col_blocks, (unsigned)k.slices, 1, (unsigned)k.threads, 1, 1, 0,
-                                         (CUstream)stream, params.data(), nullptr),
-                 "cuLaunchKernel(fused_kernel)");
-        check_cu(driver().cuLaunchKernel(fn.finalize, (unsigned)k.fin_blocks, 1, 1, (unsigned)k.fin_threads, 1, 1, 0, (CUstream)stream,
-                                         params.data(), nullptr),
-                 "cuLaunchKernel(fused_finalize)");
+        launch_kernel(fn.function, k.col_blocks, k.slices, k.threads, stream, params.data(), "cuLaunchKernelEx(fused_kernel)");
+        launch_kernel(fn.finalize, k.fin_blocks, 1, k.fin_threads, stream, params.data(), "cuLaunchKernelEx(fused_finalize)");
         return;
     }
     int64_t row_blocks = (k.rows + k.rows_per_block - 1) / k.rows_per_block;
     int per_sm = std::max(1, 2048 / k.threads);
     int64_t grid = std::min<int64_t>(row_blocks, (int64_t)dev.sms * per_sm);
-    check_cu(driver().cuLaunchKernel(fn.function, (unsigned)grid, 1, 1, (unsigned)k.threads, 1, 1, 0, (CUstream)stream,
-                                     params.data(), nullptr),
-             "cuLaunchKernel(fused_kernel)");
+    launch_kernel(fn.function, grid, 1, k.threads, stream, params.data(), "cuLaunchKernelEx(fused_kernel)");
 }
 
 void launch_fusion(lb_fusion* f, const lb_tensor* tensors, int n, void* scratch, void* stream) { launch(f, tensors, n, scratch, stream); }
@@ -136,8 +143,7 @@ void launch_fusion_multi(lb_fusion* f, const lb_tensor* tensors, int n_groups, v
         const int per_sm = std::max(1, 2048 / k.threads);
         const long long grid = std::min<long long>(most_blocks, (long long)dev.sms * per_sm);
         void* params[1] = {table.data()};
-        check_cu(driver().cuLaunchKernel(fn.function, (unsigned)grid, 1, 1, (unsigned)k.threads, 1, 1, 0, (CUstream)stream, params, nullptr),
-                 "cuLaunchKernel(fused_kernel, horizontal)");
+        launch_kernel(fn.function, grid, 1, k.threads, stream, params, "cuLaunchKernelEx(fused_kernel, horizontal)");
     }
 }
 lb_fusion* compile_fusion(const std::string& text) { return compile(text); }

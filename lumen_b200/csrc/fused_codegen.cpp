@@ -51,6 +51,13 @@ __device__ __forceinline__ double fmin_nan(double a, double b) { return (a != a 
 // are literal negations 0 - x comes out as the extremum over x and -x together (a stand-alone kernel shows it with
 // `neg.s32` in inline assembly as well, so it happens after PTX); a subtraction from a register does not.
 #define RT_ZERO blockIdx.z
+// The thread's index, once the kernels before this one in the stream have completed: this kernel may have been made resident
+// before that. Every address is computed from it, so no load can be moved in front of the wait.
+__device__ __forceinline__ u32 grid_wait() {
+    u32 tid = threadIdx.x;
+    asm volatile("griddepcontrol.wait;" : "+r"(tid) : : "memory");
+    return tid;
+}
 template <class T> __device__ __forceinline__ T imax(T a, T b) { return a > b ? a : b; }
 template <class T> __device__ __forceinline__ T imin(T a, T b) { return a < b ? a : b; }
 // division by zero gives all ones and leaves the remainder a; a signed -1 divisor negates (wrapping at the lowest
@@ -1175,6 +1182,10 @@ class Generator {
         return out;
     }
 
+    static std::string wait_for_grid(int threads) {
+        return format("    const u32 tid = grid_wait();\n    __builtin_assume(tid < %du);\n", threads);
+    }
+
     FusedKernel emit() {
         FusedKernel k;
         std::ostringstream s;
@@ -1223,6 +1234,7 @@ class Generator {
             s << "struct MultiTable { int n; int pad; long long rows[" << k.multi_max_groups << "]; void* ptr[" << k.multi_max_groups << "]["
               << n_ptrs << "]; };\n";
             s << "extern \"C\" __global__ void __launch_bounds__(" << T_ * RPB_ << ") fused_kernel(const MultiTable table) {\n";
+            s << wait_for_grid(T_ * RPB_);
             // The groups' row blocks form ONE sequence dealt to the CTAs in turn: a group smaller than the grid does not
             // always land on the first CTAs (most parameters of a model have fewer row blocks than the grid has CTAs).
             s << "  long long blocks_before = 0;\n";
@@ -1242,7 +1254,8 @@ class Generator {
             s << ") {\n";
         }
         s << "    __shared__ unsigned long long red_smem[2][32];\n    int red_turn = 0;\n";
-        s << "    const int lane_in_row = threadIdx.x % TPR, row_in_block = threadIdx.x / TPR;\n";
+        if (!multi_) s << wait_for_grid(T_ * RPB_);
+        s << "    const int lane_in_row = tid % TPR, row_in_block = tid / TPR;\n";
         s << "    const idx_t row_blocks = (idx_t)((NROWS + RPB - 1) / RPB);\n";
         s << indent(kernel_cache_, 4);
         for (size_t i = 0; i < col_reduces_.size(); i++) {
@@ -1467,7 +1480,8 @@ class Generator {
         for (size_t i = 0; i < g_.outputs.size(); i++) sig += format("void* __restrict__ out%d, ", (int)i);
         sig += "void* __restrict__ scratch";
         s << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") fused_kernel(" << sig << ") {\n";
-        s << "    const int col_lane = threadIdx.x & " << col_lanes - 1 << ", row_lane = threadIdx.x >> 5;\n";
+        s << wait_for_grid(threads);
+        s << "    const int col_lane = tid & " << col_lanes - 1 << ", row_lane = tid >> 5;\n";
         s << "    const idx_t c0 = ((idx_t)blockIdx.x * " << col_lanes << " + col_lane) * VEC;\n    const bool in_range = c0 < NCOLS;\n";
         s << "    __shared__ __align__(16) char shared[" << row_lanes * col_lanes << " * VEC * " << widest << "];\n";
         s << indent(decl.str(), 4);
@@ -1560,7 +1574,8 @@ class Generator {
         }
         s << "#undef VEC\n#define VEC " << VEC_ << "\n";
         s << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") fused_finalize(" << sig << ") {\n";
-        s << "    const int col_lane = threadIdx.x & " << col_lanes - 1 << ", row_lane = threadIdx.x >> 5;\n";
+        s << wait_for_grid(threads);
+        s << "    const int col_lane = tid & " << col_lanes - 1 << ", row_lane = tid >> 5;\n";
         s << "    const idx_t c0 = ((idx_t)blockIdx.x * " << col_lanes << " + col_lane) * VEC;\n    const bool in_range = c0 < NCOLS;\n";
         s << "    __shared__ __align__(16) char shared[" << shared_bytes << "];\n";
         s << indent(totals.str(), 4);

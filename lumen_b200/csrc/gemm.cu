@@ -18,6 +18,7 @@
 #include <mutex>
 
 #include "gemm.h"
+#include "launch.cuh"
 #include "sm100.cuh"
 
 namespace lb {
@@ -294,6 +295,7 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
+    grid_wait();
 
     if (warp == 0) {
         // ---- TMA producer ----
@@ -476,6 +478,7 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     cluster_sync();  // barriers of both CTAs are initialised and both allocations are done before anyone signals across
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
+    grid_wait();
 
     if (warp == 0) {
         // ---- TMA producer (both CTAs) ----
@@ -611,6 +614,7 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
 // Adds the split-K partial tiles in split order (fixed, so results are reproducible), applies the epilogue and rounds once.
 __global__ void splitk_reduce(const float* __restrict__ partial, GemmArgs p) {
+    grid_wait();
     const long long per = (long long)p.batch * p.M * p.N;
     for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < per; i += (long long)gridDim.x * blockDim.x * 4) {
         float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -851,16 +855,14 @@ void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
         if (pairs) {
             const int resident = max_pairs > 0 ? max_pairs : sms / 2;
             int grid = 2 * (int)std::min<long long>(tiles * p.splits, resident);
-            gemm_tcgen05_pair<<<grid, kThreads, kPairSmemBytes, s>>>(map_a, map_b, p);
+            launch_overlapped(gemm_tcgen05_pair, dim3((unsigned)grid), dim3(kThreads), kPairSmemBytes, s, 0, map_a, map_b, p);
         } else {
             int grid = (int)std::min<long long>(tiles * p.splits, sms);
-            gemm_tcgen05<<<grid, kThreads, kSmemBytes, s>>>(map_a, map_b, p);
+            launch_overlapped(gemm_tcgen05, dim3((unsigned)grid), dim3(kThreads), kSmemBytes, s, 0, map_a, map_b, p);
         }
-        LB_CUDA(cudaGetLastError());
         if (p.splits > 1) {
             long long groups = ((long long)batch * M * N + 3) / 4;
-            splitk_reduce<<<(unsigned)std::min<long long>((groups + 255) / 256, sms * 8), 256, 0, s>>>(p.partial, p);
-            LB_CUDA(cudaGetLastError());
+            launch_overlapped(splitk_reduce, dim3((unsigned)std::min<long long>((groups + 255) / 256, sms * 8)), dim3(256), 0, s, 0, p.partial, p);
         }
         return;
     }

@@ -4,6 +4,7 @@
 #include <cuda_fp16.h>
 
 #include "gemm.h"
+#include "launch.cuh"
 
 namespace lb {
 namespace {
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(TM / RM * (TN / RN)) gemm_simt_kernel(const T*
     const T* bb = b + (long long)bz * p.b_sb;
     const bool a_k = p.a_sk == 1, b_k = p.b_sn != 1;  // fetch along whichever axis is contiguous
     const bool a_whole = p.a_vec && m0 + TM <= p.M, b_whole = p.b_vec && n0 + TN <= p.N;
+    grid_wait();
     float acc[RM][RN] = {};
     SliceA fa;
     SliceB fb;
@@ -188,9 +190,9 @@ template <class T>
 void launch_simt(const T* a, const T* b, const SimtArgs& p, int sms, cudaStream_t s) {
     auto grid = [&](int tm, int tn) { return dim3((unsigned)((p.N + tn - 1) / tn), (unsigned)((p.M + tm - 1) / tm), (unsigned)p.batch); };
     auto tiles = [](dim3 g) { return (long long)g.x * g.y * g.z; };
-    if (tiles(grid(64, 64)) >= 2LL * sms) gemm_simt_kernel<T, 64, 64, 4, 4, 32><<<grid(64, 64), 256, 0, s>>>(a, b, p);
-    else if (tiles(grid(32, 32)) >= sms) gemm_simt_kernel<T, 32, 32, 2, 4, 64><<<grid(32, 32), 128, 0, s>>>(a, b, p);
-    else gemm_simt_kernel<T, 16, 32, 2, 2, 64><<<grid(16, 32), 128, 0, s>>>(a, b, p);
+    if (tiles(grid(64, 64)) >= 2LL * sms) launch_overlapped(gemm_simt_kernel<T, 64, 64, 4, 4, 32>, grid(64, 64), dim3(256), 0, s, 0, a, b, p);
+    else if (tiles(grid(32, 32)) >= sms) launch_overlapped(gemm_simt_kernel<T, 32, 32, 2, 4, 64>, grid(32, 32), dim3(128), 0, s, 0, a, b, p);
+    else launch_overlapped(gemm_simt_kernel<T, 16, 32, 2, 2, 64>, grid(16, 32), dim3(128), 0, s, 0, a, b, p);
 }
 
 }  // namespace
@@ -199,7 +201,6 @@ void gemm_simt(const void* a, const void* b, int dtype, const SimtArgs& p, int s
     if (dtype == LB_F32) launch_simt<float>((const float*)a, (const float*)b, p, sms, s);
     else if (dtype == LB_BF16) launch_simt<__nv_bfloat16>((const __nv_bfloat16*)a, (const __nv_bfloat16*)b, p, sms, s);
     else launch_simt<__half>((const __half*)a, (const __half*)b, p, sms, s);
-    LB_CUDA(cudaGetLastError());
 }
 
 }  // namespace lb

@@ -9,6 +9,7 @@
 #include <cuda_fp16.h>
 
 #include "gemm.h"
+#include "launch.cuh"
 #include "sm100.cuh"
 
 namespace lb {
@@ -72,6 +73,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    grid_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -204,13 +206,8 @@ template <int STAGES>
 static void launch_small(const CUtensorMap& map_a, const CUtensorMap& map_b, const SmallGemmArgs& p, int batch, cudaStream_t s) {
     if (first_use_on_device((const void*)gemm_small_kernel<STAGES>))
         LB_CUDA(cudaFuncSetAttribute(gemm_small_kernel<STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(STAGES)));
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = p.splits, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)((long long)p.tiles_m * p.tiles_n * batch * p.splits)), cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem_bytes(STAGES), cfg.stream = s, cfg.attrs = attr, cfg.numAttrs = 1;
-    LB_CUDA(cudaLaunchKernelEx(&cfg, gemm_small_kernel<STAGES>, map_a, map_b, p));
+    launch_overlapped(gemm_small_kernel<STAGES>, dim3((unsigned)((long long)p.tiles_m * p.tiles_n * batch * p.splits)), dim3(kThreads), smem_bytes(STAGES), s,
+                      (unsigned)p.splits, map_a, map_b, p);
 }
 
 void gemm_small(const CUtensorMap& map_a, const CUtensorMap& map_b, SmallGemmArgs p, int batch, int sms, cudaStream_t s) {

@@ -8,7 +8,7 @@
 //  * attention_simt_fwd / attention_simt_bwd: float32 or bfloat16, any head dim up to 256, one warp per query row,
 //    scores and sums in float32. Used for float32 graphs (no hidden narrowing to bf16 tensor cores)
 //    and head dims other than 64/128.
-#include "device.h"
+#include "launch.cuh"
 
 #include <cuda_bf16.h>
 
@@ -28,6 +28,7 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float
 template <class T, class I>
 __global__ void scatter_add_rows_kernel(float* __restrict__ acc, const I* __restrict__ ids, const T* __restrict__ updates,
                                         long long tokens, long long rows, int width) {
+    grid_wait();
     const long long t = blockIdx.x;
     if (t >= tokens) return;
     long long r = (long long)ids[t];
@@ -37,6 +38,7 @@ __global__ void scatter_add_rows_kernel(float* __restrict__ acc, const I* __rest
 
 template <class T>
 __global__ void add_convert_kernel(T* __restrict__ out, const T* __restrict__ x, const float* __restrict__ acc, long long n, int has_x) {
+    grid_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     // out = x + sum(updates): one rounding of the float32 sum into the operand dtype
@@ -52,12 +54,14 @@ __device__ __forceinline__ int clamped_row(const I* ids, long long t, long long 
 
 template <class I>
 __global__ void scatter_count_kernel(int* __restrict__ counts, const I* __restrict__ ids, long long tokens, long long rows) {
+    grid_wait();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < tokens) atomicAdd(counts + clamped_row(ids, t, rows), 1);  // integer atomics: the counts do not depend on order
 }
 
 // starts[r] = sum of counts[0 .. r), starts[rows] = tokens; one block walks the rows in chunks of its size.
 __global__ void scatter_starts_kernel(int* __restrict__ starts, const int* __restrict__ counts, long long rows) {
+    grid_wait();
     __shared__ int warp_sums[32];
     __shared__ int carry;
     if (threadIdx.x == 0) carry = 0;
@@ -96,6 +100,7 @@ __global__ void scatter_starts_kernel(int* __restrict__ starts, const int* __res
 template <class I>
 __global__ void scatter_place_kernel(int* __restrict__ order, int* __restrict__ cursor, const int* __restrict__ starts,
                                      const I* __restrict__ ids, long long tokens, long long rows) {
+    grid_wait();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= tokens) return;
     const int r = clamped_row(ids, t, rows);
@@ -111,6 +116,7 @@ template <class T>
 __global__ void scatter_rows_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __restrict__ updates, const int* __restrict__ starts,
                                     const int* __restrict__ order, int* __restrict__ sorted, int width, int has_x) {
     __shared__ int picks[kSortSmem];
+    grid_wait();
     const long long r = blockIdx.x;
     const int begin = starts[r], n = starts[r + 1] - begin;
     const int* list = picks;
@@ -276,6 +282,7 @@ attention_simt_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, cons
                           float* __restrict__ lse, AttnShape s) {
     extern __shared__ __align__(16) uint8_t raw[];
     AttnSmem<DU> sm(raw, s.tile_rows);
+    grid_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int i0, n, b;
     block_rows(s.Sq, s.N, i0, n, b);
@@ -326,6 +333,7 @@ attention_simt_dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const
                          const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dq, AttnShape s) {
     extern __shared__ __align__(16) uint8_t raw[];
     AttnSmem<DU> sm(raw, s.tile_rows);
+    grid_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int i0, n, b;
     block_rows(s.Sq, s.N, i0, n, b);
@@ -369,6 +377,7 @@ attention_simt_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, con
                            const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dk, T* __restrict__ dv, AttnShape s) {
     extern __shared__ __align__(16) uint8_t raw[];
     AttnSmem<DU> sm(raw, s.tile_rows);
+    grid_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int k0, nk, b;
     block_rows(s.Sk, s.Nkv, k0, nk, b);
@@ -414,6 +423,7 @@ attention_simt_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, con
 
 template <class T>
 __global__ void attention_delta_simt(const T* __restrict__ o, const T* __restrict__ g, float* __restrict__ delta, AttnShape s) {
+    grid_wait();
     const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= (long long)s.B * s.N * s.Sq) return;
@@ -432,6 +442,7 @@ __global__ void attention_delta_simt(const T* __restrict__ o, const T* __restric
 template <class T>
 __global__ void __launch_bounds__(256) transpose_kernel(const T* __restrict__ in, T* __restrict__ out, int rows, int cols) {
     __shared__ T tile[32][33];
+    grid_wait();
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
 #pragma unroll
@@ -457,6 +468,7 @@ void fill_strides(long long* dst, const lb_tensor& t) {
 // bfloat16 noise in [-1, 1) from a linear congruential generator, over a whole buffer: what an autotuner times its
 // candidates on (a GPU's clocks under all-zero operands differ from those under real data).
 __global__ void fill_noise_kernel(uint16_t* __restrict__ out, size_t n) {
+    grid_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         uint32_t x = (uint32_t)i * 1664525u + 1013904223u;
         x = x * 1664525u + 1013904223u;
@@ -469,7 +481,7 @@ void fill_noise(void* ptr, size_t bytes, void* stream) {
     const size_t n = bytes / 2;
     if (n == 0) return;
     driver();
-    fill_noise_kernel<<<(unsigned)std::min<size_t>((n + 255) / 256, 148 * 16), 256, 0, (cudaStream_t)stream>>>((uint16_t*)ptr, n);
+    launch_overlapped(fill_noise_kernel, dim3((unsigned)std::min<size_t>((n + 255) / 256, 148 * 16)), dim3(256), 0, (cudaStream_t)stream, 0, (uint16_t*)ptr, n);
     LB_CUDA(cudaGetLastError());
 }
 
@@ -503,20 +515,20 @@ void scatter_add_rows(const lb_tensor& x, const lb_tensor& ids, const lb_tensor&
         LB_CUDA(cudaMemsetAsync(counts, 0, (size_t)rows * 2 * 4, s));  // counts and cursor start at zero
         if (tokens > 0) {
             const unsigned blocks = (unsigned)((tokens + 255) / 256);
-            if (ids.dtype == LB_I64) scatter_count_kernel<long long><<<blocks, 256, 0, s>>>(counts, (const long long*)ids.ptr, tokens, rows);
-            else scatter_count_kernel<int><<<blocks, 256, 0, s>>>(counts, (const int*)ids.ptr, tokens, rows);
+            if (ids.dtype == LB_I64) launch_overlapped(scatter_count_kernel<long long>, dim3(blocks), dim3(256), 0, s, 0, counts, (const long long*)ids.ptr, tokens, rows);
+            else launch_overlapped(scatter_count_kernel<int>, dim3(blocks), dim3(256), 0, s, 0, counts, (const int*)ids.ptr, tokens, rows);
         }
-        scatter_starts_kernel<<<1, 1024, 0, s>>>(starts, counts, rows);
+        launch_overlapped(scatter_starts_kernel, dim3(1), dim3(1024), 0, s, 0, starts, counts, rows);
         if (tokens > 0) {
             const unsigned blocks = (unsigned)((tokens + 255) / 256);
-            if (ids.dtype == LB_I64) scatter_place_kernel<long long><<<blocks, 256, 0, s>>>(order, cursor, starts, (const long long*)ids.ptr, tokens, rows);
-            else scatter_place_kernel<int><<<blocks, 256, 0, s>>>(order, cursor, starts, (const int*)ids.ptr, tokens, rows);
+            if (ids.dtype == LB_I64) launch_overlapped(scatter_place_kernel<long long>, dim3(blocks), dim3(256), 0, s, 0, order, cursor, starts, (const long long*)ids.ptr, tokens, rows);
+            else launch_overlapped(scatter_place_kernel<int>, dim3(blocks), dim3(256), 0, s, 0, order, cursor, starts, (const int*)ids.ptr, tokens, rows);
         }
         const int threads = (int)std::min<long long>(256, ((width + 31) / 32) * 32);
         if (x.dtype == LB_F32)
-            scatter_rows_kernel<float><<<(unsigned)rows, threads, 0, s>>>((float*)out.ptr, (const float*)x.ptr, (const float*)updates.ptr, starts, order, sorted, (int)width, !x_is_zero);
+            launch_overlapped(scatter_rows_kernel<float>, dim3((unsigned)rows), dim3(threads), 0, s, 0, (float*)out.ptr, (const float*)x.ptr, (const float*)updates.ptr, starts, order, sorted, (int)width, !x_is_zero);
         else
-            scatter_rows_kernel<__nv_bfloat16><<<(unsigned)rows, threads, 0, s>>>((__nv_bfloat16*)out.ptr, (const __nv_bfloat16*)x.ptr, (const __nv_bfloat16*)updates.ptr, starts, order, sorted, (int)width, !x_is_zero);
+            launch_overlapped(scatter_rows_kernel<__nv_bfloat16>, dim3((unsigned)rows), dim3(threads), 0, s, 0, (__nv_bfloat16*)out.ptr, (const __nv_bfloat16*)x.ptr, (const __nv_bfloat16*)updates.ptr, starts, order, sorted, (int)width, !x_is_zero);
         LB_CUDA(cudaGetLastError());
         return;
     }
@@ -525,17 +537,17 @@ void scatter_add_rows(const lb_tensor& x, const lb_tensor& ids, const lb_tensor&
     if (tokens > 0 && width > 0) {
         int threads = (int)std::min<long long>(256, ((width + 31) / 32) * 32);
         if (x.dtype == LB_F32) {
-            if (ids.dtype == LB_I64) scatter_add_rows_kernel<float, long long><<<(unsigned)tokens, threads, 0, s>>>(acc, (const long long*)ids.ptr, (const float*)updates.ptr, tokens, rows, (int)width);
-            else scatter_add_rows_kernel<float, int><<<(unsigned)tokens, threads, 0, s>>>(acc, (const int*)ids.ptr, (const float*)updates.ptr, tokens, rows, (int)width);
+            if (ids.dtype == LB_I64) launch_overlapped(scatter_add_rows_kernel<float, long long>, dim3((unsigned)tokens), dim3(threads), 0, s, 0, acc, (const long long*)ids.ptr, (const float*)updates.ptr, tokens, rows, (int)width);
+            else launch_overlapped(scatter_add_rows_kernel<float, int>, dim3((unsigned)tokens), dim3(threads), 0, s, 0, acc, (const int*)ids.ptr, (const float*)updates.ptr, tokens, rows, (int)width);
         } else {
-            if (ids.dtype == LB_I64) scatter_add_rows_kernel<__nv_bfloat16, long long><<<(unsigned)tokens, threads, 0, s>>>(acc, (const long long*)ids.ptr, (const __nv_bfloat16*)updates.ptr, tokens, rows, (int)width);
-            else scatter_add_rows_kernel<__nv_bfloat16, int><<<(unsigned)tokens, threads, 0, s>>>(acc, (const int*)ids.ptr, (const __nv_bfloat16*)updates.ptr, tokens, rows, (int)width);
+            if (ids.dtype == LB_I64) launch_overlapped(scatter_add_rows_kernel<__nv_bfloat16, long long>, dim3((unsigned)tokens), dim3(threads), 0, s, 0, acc, (const long long*)ids.ptr, (const __nv_bfloat16*)updates.ptr, tokens, rows, (int)width);
+            else launch_overlapped(scatter_add_rows_kernel<__nv_bfloat16, int>, dim3((unsigned)tokens), dim3(threads), 0, s, 0, acc, (const int*)ids.ptr, (const __nv_bfloat16*)updates.ptr, tokens, rows, (int)width);
         }
     }
     const long long n = rows * width;
     if (n > 0) {
-        if (x.dtype == LB_F32) add_convert_kernel<float><<<(unsigned)((n + 255) / 256), 256, 0, s>>>((float*)out.ptr, (const float*)x.ptr, acc, n, !x_is_zero);
-        else add_convert_kernel<__nv_bfloat16><<<(unsigned)((n + 255) / 256), 256, 0, s>>>((__nv_bfloat16*)out.ptr, (const __nv_bfloat16*)x.ptr, acc, n, !x_is_zero);
+        if (x.dtype == LB_F32) launch_overlapped(add_convert_kernel<float>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, 0, (float*)out.ptr, (const float*)x.ptr, acc, n, !x_is_zero);
+        else launch_overlapped(add_convert_kernel<__nv_bfloat16>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, 0, (__nv_bfloat16*)out.ptr, (const __nv_bfloat16*)x.ptr, acc, n, !x_is_zero);
     }
     LB_CUDA(cudaGetLastError());
 }
@@ -561,8 +573,8 @@ void transpose_2d(const lb_tensor& in, const lb_tensor& out, void* stream) {
         fail(LB_ERR_UNSUPPORTED, "transpose: matrix too large for the kernel's grid");
     dim3 grid((unsigned)((cols + 31) / 32), (unsigned)((rows + 31) / 32));
     const int size = dtype_size(in.dtype);
-    if (size == 2) transpose_kernel<uint16_t><<<grid, 256, 0, (cudaStream_t)stream>>>((const uint16_t*)in.ptr, (uint16_t*)out.ptr, (int)rows, (int)cols);
-    else if (size == 4) transpose_kernel<uint32_t><<<grid, 256, 0, (cudaStream_t)stream>>>((const uint32_t*)in.ptr, (uint32_t*)out.ptr, (int)rows, (int)cols);
+    if (size == 2) launch_overlapped(transpose_kernel<uint16_t>, dim3(grid), dim3(256), 0, (cudaStream_t)stream, 0, (const uint16_t*)in.ptr, (uint16_t*)out.ptr, (int)rows, (int)cols);
+    else if (size == 4) launch_overlapped(transpose_kernel<uint32_t>, dim3(grid), dim3(256), 0, (cudaStream_t)stream, 0, (const uint32_t*)in.ptr, (uint32_t*)out.ptr, (int)rows, (int)cols);
     else fail(LB_ERR_UNSUPPORTED, "transpose: 2-byte and 4-byte elements");
     LB_CUDA(cudaGetLastError());
 }
@@ -578,6 +590,7 @@ struct CopyDims {
 
 template <class T>
 __global__ void strided_copy_kernel(const T* __restrict__ src, T* __restrict__ dst, CopyDims d, long long total) {
+    grid_wait();
     const long long step = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += step) {
         long long rest = i, from = 0, to = 0;
@@ -597,6 +610,7 @@ template <class T>
 __global__ void __launch_bounds__(256) tiled_copy_kernel(const T* __restrict__ src, T* __restrict__ dst, CopyDims d, int a, int b, long long tiles_a,
                                                          long long tiles_b) {
     __shared__ T tile[32][33];
+    grid_wait();
     long long block = blockIdx.x;
     const long long ta = block % tiles_a;
     block /= tiles_a;
@@ -650,10 +664,10 @@ void strided_copy(const lb_tensor& in, const lb_tensor& out, void* stream) {
         const long long blocks = total / (d.shape[a] * d.shape[b]) * tiles_a * tiles_b;
         if (blocks <= 0x7fffffffLL) {
             switch (dtype_size(in.dtype)) {
-                case 1: tiled_copy_kernel<uint8_t><<<(unsigned)blocks, 256, 0, st>>>((const uint8_t*)in.ptr, (uint8_t*)out.ptr, d, a, b, tiles_a, tiles_b); break;
-                case 2: tiled_copy_kernel<uint16_t><<<(unsigned)blocks, 256, 0, st>>>((const uint16_t*)in.ptr, (uint16_t*)out.ptr, d, a, b, tiles_a, tiles_b); break;
-                case 4: tiled_copy_kernel<uint32_t><<<(unsigned)blocks, 256, 0, st>>>((const uint32_t*)in.ptr, (uint32_t*)out.ptr, d, a, b, tiles_a, tiles_b); break;
-                default: tiled_copy_kernel<uint64_t><<<(unsigned)blocks, 256, 0, st>>>((const uint64_t*)in.ptr, (uint64_t*)out.ptr, d, a, b, tiles_a, tiles_b); break;
+                case 1: launch_overlapped(tiled_copy_kernel<uint8_t>, dim3((unsigned)blocks), dim3(256), 0, st, 0, (const uint8_t*)in.ptr, (uint8_t*)out.ptr, d, a, b, tiles_a, tiles_b); break;
+                case 2: launch_overlapped(tiled_copy_kernel<uint16_t>, dim3((unsigned)blocks), dim3(256), 0, st, 0, (const uint16_t*)in.ptr, (uint16_t*)out.ptr, d, a, b, tiles_a, tiles_b); break;
+                case 4: launch_overlapped(tiled_copy_kernel<uint32_t>, dim3((unsigned)blocks), dim3(256), 0, st, 0, (const uint32_t*)in.ptr, (uint32_t*)out.ptr, d, a, b, tiles_a, tiles_b); break;
+                default: launch_overlapped(tiled_copy_kernel<uint64_t>, dim3((unsigned)blocks), dim3(256), 0, st, 0, (const uint64_t*)in.ptr, (uint64_t*)out.ptr, d, a, b, tiles_a, tiles_b); break;
             }
             LB_CUDA(cudaGetLastError());
             return;
@@ -661,10 +675,10 @@ void strided_copy(const lb_tensor& in, const lb_tensor& out, void* stream) {
     }
     const unsigned blocks = (unsigned)std::min<long long>((total + 255) / 256, 148LL * 16);
     switch (dtype_size(in.dtype)) {
-        case 1: strided_copy_kernel<uint8_t><<<blocks, 256, 0, st>>>((const uint8_t*)in.ptr, (uint8_t*)out.ptr, d, total); break;
-        case 2: strided_copy_kernel<uint16_t><<<blocks, 256, 0, st>>>((const uint16_t*)in.ptr, (uint16_t*)out.ptr, d, total); break;
-        case 4: strided_copy_kernel<uint32_t><<<blocks, 256, 0, st>>>((const uint32_t*)in.ptr, (uint32_t*)out.ptr, d, total); break;
-        default: strided_copy_kernel<uint64_t><<<blocks, 256, 0, st>>>((const uint64_t*)in.ptr, (uint64_t*)out.ptr, d, total); break;
+        case 1: launch_overlapped(strided_copy_kernel<uint8_t>, dim3(blocks), dim3(256), 0, st, 0, (const uint8_t*)in.ptr, (uint8_t*)out.ptr, d, total); break;
+        case 2: launch_overlapped(strided_copy_kernel<uint16_t>, dim3(blocks), dim3(256), 0, st, 0, (const uint16_t*)in.ptr, (uint16_t*)out.ptr, d, total); break;
+        case 4: launch_overlapped(strided_copy_kernel<uint32_t>, dim3(blocks), dim3(256), 0, st, 0, (const uint32_t*)in.ptr, (uint32_t*)out.ptr, d, total); break;
+        default: launch_overlapped(strided_copy_kernel<uint64_t>, dim3(blocks), dim3(256), 0, st, 0, (const uint64_t*)in.ptr, (uint64_t*)out.ptr, d, total); break;
     }
     LB_CUDA(cudaGetLastError());
 }
@@ -682,7 +696,7 @@ void launch_attn(Kernel kernel, unsigned blocks, int streamed, cudaStream_t st, 
     if (AttnSmem<DU>::bytes(kChunk) > 48 * 1024 && first_use_on_device((const void*)kernel))
         LB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnSmem<DU>::bytes(kChunk)));
     s.tile_rows = std::min(kChunk, (std::max(streamed, 1) + 3) / 4 * 4);
-    kernel<<<blocks, kAttnRows * 32, AttnSmem<DU>::bytes(s.tile_rows), st>>>(args..., s);
+    launch_overlapped(kernel, dim3(blocks), dim3(kAttnRows * 32), AttnSmem<DU>::bytes(s.tile_rows), st, 0, args..., s);
 }
 // calls `f` with the head-dim elements per lane as a compile-time number: 1, 2, 4 or 8
 template <class F>
@@ -702,7 +716,7 @@ template <class T>
 void simt_bwd(const AttnShape& s, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o, const lb_tensor& g,
               const float* lse, float* delta, const lb_tensor& dq, const lb_tensor& dk, const lb_tensor& dv, cudaStream_t st) {
     const long long warps = (long long)s.B * s.N * s.Sq;
-    attention_delta_simt<T><<<(unsigned)((warps * 32 + 255) / 256), 256, 0, st>>>((const T*)o.ptr, (const T*)g.ptr, delta, s);
+    launch_overlapped(attention_delta_simt<T>, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256), 0, st, 0, (const T*)o.ptr, (const T*)g.ptr, delta, s);
     with_dims_per_lane(s.D, [&](auto du) {
         launch_attn<du>(attention_simt_dq_kernel<T, du>, attn_blocks(s.B, s.N, s.Sq), s.Sk, st, s, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr,
                         (const T*)g.ptr, lse, (const float*)delta, (T*)dq.ptr);
