@@ -103,16 +103,17 @@ void launch_fusion_multi(lb_fusion* f, const lb_tensor* tensors, int n_groups, v
         if (!slot.function) slot.function = load_kernel(f->cubin, "fused_kernel");
         fn = slot;
     }
-    // the table as the generated source lays it out: { int n; int pad; long long rows[MAX]; void* ptr[MAX][per]; }
+    // the table as the generated source lays it out: { int n; u32 blocks; long long rows[MAX]; void* ptr[MAX][per]; u32 first[MAX]; }
     const int max_groups = k.multi_max_groups;
-    std::vector<char> table(8 + (size_t)max_groups * 8 + (size_t)max_groups * per * 8);
+    std::vector<char> table((8 + (size_t)max_groups * 8 + (size_t)max_groups * per * 8 + (size_t)max_groups * 4 + 7) / 8 * 8);
     for (int first = 0; first < n_groups; first += max_groups) {
         const int count = std::min(max_groups, n_groups - first);
         std::fill(table.begin(), table.end(), 0);
         *(int*)table.data() = count;
         long long* rows = (long long*)(table.data() + 8);
         void** ptrs = (void**)(table.data() + 8 + (size_t)max_groups * 8);
-        long long most_blocks = 1;
+        unsigned* firsts = (unsigned*)(table.data() + 8 + (size_t)max_groups * 8 + (size_t)max_groups * per * 8);
+        long long blocks = 0;
         for (int g = 0; g < count; g++) {
             const lb_tensor* t = tensors + (size_t)(first + g) * per;
             int64_t n = -1;
@@ -137,11 +138,15 @@ void launch_fusion_multi(lb_fusion* f, const lb_tensor* tensors, int n_groups, v
                 if (k.vec > 1 && ((uintptr_t)t[i].ptr & 15) != 0) fail(LB_ERR_INVALID, "horizontal launch: tensors must be 16-byte aligned");
                 ptrs[(size_t)g * per + i] = t[i].ptr;
             }
-            rows[g] = n / k.cols;
-            most_blocks = std::max<long long>(most_blocks, (rows[g] + k.rows_per_block - 1) / k.rows_per_block);
+            rows[g] = k.cols ? n / k.cols : 0;
+            firsts[g] = (unsigned)blocks;
+            blocks += (rows[g] + k.rows_per_block - 1) / k.rows_per_block;
         }
+        if (blocks == 0) continue;
+        if (blocks > INT32_MAX) fail(LB_ERR_UNSUPPORTED, "horizontal launch: too many row blocks for one launch");
+        *(unsigned*)(table.data() + 4) = (unsigned)blocks;
         const int per_sm = std::max(1, 2048 / k.threads);
-        const long long grid = std::min<long long>(most_blocks, (long long)dev.sms * per_sm);
+        const long long grid = std::min<long long>(blocks, (long long)dev.sms * per_sm);
         void* params[1] = {table.data()};
         launch_kernel(fn.function, grid, 1, k.threads, stream, params, "cuLaunchKernelEx(fused_kernel, horizontal)");
     }

@@ -1230,15 +1230,19 @@ class Generator {
             if (!kernel_cache_.empty() || !row_caches_.empty() || !row_decls_.empty())
                 fail(LB_ERR_UNSUPPORTED, "a horizontally fused kernel takes full-shape operands and constants only");
             k.multi = true;
-            k.multi_max_groups = std::max(1, (4000 - 16) / (8 * (n_ptrs + 1)));  // the table fits the 4 KB parameter space
-            s << "struct MultiTable { int n; int pad; long long rows[" << k.multi_max_groups << "]; void* ptr[" << k.multi_max_groups << "]["
-              << n_ptrs << "]; };\n";
+            k.multi_max_groups = std::max(1, (4000 - 24) / (8 * (n_ptrs + 1) + 4));  // the table fits the 4 KB parameter space
+            s << "struct MultiTable { int n; u32 blocks; long long rows[" << k.multi_max_groups << "]; void* ptr[" << k.multi_max_groups << "]["
+              << n_ptrs << "]; u32 first[" << k.multi_max_groups << "]; };\n";
             s << "extern \"C\" __global__ void __launch_bounds__(" << T_ * RPB_ << ") fused_kernel(const MultiTable table) {\n";
             s << wait_for_grid(T_ * RPB_);
-            // The groups' row blocks form ONE sequence dealt to the CTAs in turn: a group smaller than the grid does not
-            // always land on the first CTAs (most parameters of a model have fewer row blocks than the grid has CTAs).
-            s << "  long long blocks_before = 0;\n";
-            s << "  for (int group = 0; group < table.n; group++) {\n";
+            // The groups' row blocks form ONE sequence (`first`: each group's first place in it) dealt to the CTAs, of which there
+            // are as many as blocks while they fit the GPU: a CTA looks its group up once and walks on. What bounds a small model's
+            // update is latency: with every CTA visiting every group, as many CTAs as the largest group has blocks and a 64-bit
+            // remainder per group, SGD over the 21 parameters of a 2-layer model took 16.7 us, now 4 (the whole step 310 -> 297).
+            s << "  u32 group = 0;\n"
+              << "  for (u32 below = table.n; below - group > 1;) { const u32 mid = (group + below) / 2; if (table.first[mid] <= blockIdx.x) group = mid; else below = mid; }\n";
+            s << "  for (u32 block = blockIdx.x; block < table.blocks; block += gridDim.x) {\n";
+            s << "    while (group + 1 < table.n && table.first[group + 1] <= block) group++;\n";
             s << "    const long long group_rows = table.rows[group];\n";
             for (size_t i = 0; i < g_.inputs.size(); i++) s << "    const void*" << restrict_kw << " in" << i << " = table.ptr[group][" << i << "];\n";
             for (size_t i = 0; i < g_.outputs.size(); i++)
@@ -1256,7 +1260,7 @@ class Generator {
         s << "    __shared__ unsigned long long red_smem[2][32];\n    int red_turn = 0;\n";
         if (!multi_) s << wait_for_grid(T_ * RPB_);
         s << "    const int lane_in_row = tid % TPR, row_in_block = tid / TPR;\n";
-        s << "    const idx_t row_blocks = (idx_t)((NROWS + RPB - 1) / RPB);\n";
+        if (!multi_) s << "    const idx_t row_blocks = (idx_t)((NROWS + RPB - 1) / RPB);\n";
         s << indent(kernel_cache_, 4);
         for (size_t i = 0; i < col_reduces_.size(); i++) {
             const Node& n = *g_.node_of(col_reduces_[i]);
@@ -1279,10 +1283,8 @@ class Generator {
             s << "    if ((idx_t)blockIdx.x < row_blocks) {\n        idx_t r = (idx_t)blockIdx.x * RPB + row_in_block;\n"
               << "        if (r >= NROWS) r = (idx_t)(NROWS - 1);\n" << indent(next_loads, 8) << "    }\n";
         }
-        if (multi_)
-            s << "    const idx_t first_rb = (idx_t)(((long long)blockIdx.x + gridDim.x - blocks_before % gridDim.x) % gridDim.x);\n"
-              << "    blocks_before += row_blocks;\n";
-        s << "    for (idx_t rb = " << (multi_ ? "first_rb" : "blockIdx.x") << "; rb < row_blocks; rb += gridDim.x) {\n";
+        if (multi_) s << "    {\n        const idx_t rb = block - table.first[group];\n";
+        else s << "    for (idx_t rb = blockIdx.x; rb < row_blocks; rb += gridDim.x) {\n";
         s << "        idx_t r = rb * RPB + row_in_block;\n";
         s << "        const bool active = r < NROWS;\n";
         s << "        if (!active) r = (idx_t)(NROWS - 1);\n";

@@ -139,3 +139,29 @@ def test_autotuned_plan_gives_the_same_results(cuda):
     want = a.float() @ b.float()
     for out in outs:
         torch.testing.assert_close(out, want, rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("cols, rows", [
+    (64, [1]),                                   # one block in all
+    (64, [7, 1, 300, 2, 2, 64]),                 # fewer blocks than CTAs fit the GPU
+    (4096, [1, 3000, 5, 1999]),                  # more: a CTA walks from group to group
+    (96, [1 + k % 5 for k in range(260)]),       # more groups than one launch's table holds
+])
+def test_horizontal_launch_reaches_every_block_of_every_group(cuda, cols, rows):
+    import ctypes
+
+    import torch
+
+    from lumen_b200 import _lib, tracer
+    from lumen_b200.runtime import Fusion, current_stream, desc
+
+    body = tracer.trace(lambda p, g: p - g * 0.5, ("float32", (2, cols)), ("float32", (2, cols)))
+    fusion = Fusion("option multi\n" + body.to_text())
+    groups = [[torch.randn(r, cols, device=cuda), torch.randn(r, cols, device=cuda), torch.full((r, cols), float("nan"), device=cuda)] for r in rows]
+    tensors = [desc(t) for g in groups for t in g]
+    lib = _lib.lib()
+    lib.lb_fusion_launch_groups.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
+    table = (_lib.LbTensor * len(tensors))(*tensors)
+    _lib.check(lib.lb_fusion_launch_groups(fusion.handle, table, len(groups), current_stream()))
+    for p, g, out in groups:
+        assert torch.equal(out, p - g * 0.5)
