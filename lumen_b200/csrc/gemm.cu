@@ -3,7 +3,7 @@
 // lumen/codegen/dot_general/cuda/mod.rs:658-757) rebuilt for Blackwell:
 //
 //  * gemm_tcgen05: 16-bit operands, explicit fp32 accumulation in tensor memory. Persistent, warp-specialised:
-//    warp 0 issues TMA tile loads into a 4-stage ring of 128-byte-swizzled shared-memory tiles, one thread of warp 1
+//    warp 0 issues TMA tile loads into a 4-stage ring of 128-byte-swizzled shared-memory tiles, warp 1 (its elected lane)
 //    issues tcgen05.mma (128x256x16 per instruction) and commits stage/accumulator barriers, warps 2-9 drain the
 //    previous tile's accumulator (tcgen05.ld) through the epilogue while the next tile's MMAs run into the other
 //    half of the 512 TMEM columns. All four operand majors (row- or column-major A and B) are handled by the tensor
@@ -33,6 +33,17 @@ constexpr int kStageBytesA = BM * BK * 2, kStageBytesB = BN * BK * 2;
 constexpr int kEpilogueStageBytes = 8 * 4096;  // one 4 KB staging area per epilogue warp (store_rows_coalesced)
 constexpr int kSmemBytes = STAGES * (kStageBytesA + kStageBytesB) + 1024 /*alignment slack*/ + 256 /*barriers*/ + kEpilogueStageBytes;
 
+// n / d for 0 <= n < 2^31 as a multiply and a shift (Granlund and Montgomery's round-up method): where a tile lies is worked out by
+// every warp between two tiles, and six integer divisions took 1200 cycles there.
+struct Divisor {
+    uint32_t d = 1, mul = 1, shift = 0;
+    void set(uint32_t by) {
+        d = by, shift = 0;
+        while ((1ull << shift) < d) shift++;
+        mul = (uint32_t)(((1ull << 32) * ((1ull << shift) - d)) / d + 1);
+    }
+    __device__ __forceinline__ uint32_t div(uint32_t n) const { return (__umulhi(n, mul) + n) >> shift; }
+};
 struct GemmArgs {
     int M, N, K, batch;
     int a_mn_major, b_mn_major;
@@ -46,30 +57,33 @@ struct GemmArgs {
     long long ld_aux, aux_batch_stride;
     int* status;          // device word: set to LB_ERR_TIMEOUT when a bounded wait gave up
     int tiles_m, tiles_n, group_m;
+    Divisor by_tiles, by_batch, by_group, by_rows, by_last_rows;  // all tiles; tiles of a batch entry; of a group; a group's rows, the last one's
     // split-K: the K loop of every tile is cut into `splits` ranges of `kb_per_split` 64-wide blocks; each (tile, range)
     // unit writes a float32 partial tile to `partial` [splits][batch][M][N] and splitk_reduce adds them in order
     int splits, kb_per_split;
     float* partial;
 };
 
-__device__ __forceinline__ void tile_coords(const GemmArgs& p, int tile, int& b, int& m_blk, int& n_blk) {
-    int per_batch = p.tiles_m * p.tiles_n;
-    b = tile / per_batch;
-    int t = tile - b * per_batch;
+// Unit `unit` of the grid: split * tiles + tile, neighbours share a K range.
+__device__ __forceinline__ int tile_coords(const GemmArgs& p, int unit, int& b, int& m_blk, int& n_blk) {
+    const int split = p.by_tiles.div(unit), tile = unit - split * (int)p.by_tiles.d;
+    b = p.by_batch.div(tile);
+    const int t = tile - b * (int)p.by_batch.d;
     // grouped raster: GROUP_M row-blocks share each column-block while they are resident together in L2
-    int group_size = p.group_m * p.tiles_n;
-    int g = t / group_size;
-    int first_m = g * p.group_m;
-    int rows = min(p.tiles_m - first_m, p.group_m);
-    int in_group = t - g * group_size;
-    m_blk = first_m + in_group % rows;
-    n_blk = in_group / rows;
+    const int g = p.by_group.div(t), first_m = g * p.group_m, in_group = t - g * (int)p.by_group.d;
+    const bool last = p.tiles_m - first_m < p.group_m;
+    const int rows = last ? p.tiles_m - first_m : p.group_m;
+    n_blk = last ? p.by_last_rows.div(in_group) : p.by_rows.div(in_group);
+    m_blk = first_m + in_group - n_blk * rows;
+    return split;
 }
 
 // Drains 128 accumulator columns (this warp's half of a 256-wide tile) of the thread's row from tensor memory and
-// stores them: float32 partial sums when K is split, otherwise the epilogue and one rounding to the output dtype.
+// stores them: float32 partial sums when K is split, otherwise the epilogue and one rounding to the output dtype. `release` hands
+// the accumulator back to the MMA warp, once its last columns are in registers.
+template <class Release>
 __device__ __forceinline__ void drain_tile(const GemmArgs& p, uint32_t tbase, int row, long long row_off, int col_base, int b, int split,
-                                           bool vec_ok, uint4* stage, int lane) {
+                                           bool vec_ok, uint4* stage, int lane, Release release) {
 #pragma unroll 1
     for (int c2 = 0; c2 < BN / 2 / 64; c2++) {
         // warp-uniform: 16-bit rows of 64 whole columns leave through the staging area, 128 contiguous bytes per row
@@ -79,6 +93,7 @@ __device__ __forceinline__ void drain_tile(const GemmArgs& p, uint32_t tbase, in
         tmem_ld_32x32(tbase + c2 * 64, vv);  // two loads in flight, one wait
         tmem_ld_32x32(tbase + c2 * 64 + 32, vv + 32);
         tmem_ld_wait();
+        if (c2 == BN / 2 / 64 - 1) release();
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             uint32_t* v = vv + h * 32;
@@ -201,21 +216,23 @@ __device__ __forceinline__ void aux_load(const uint16_t* ax_warp, long long ld_a
 }
 // Turns what aux_load fetched into each lane's own row (16 packed pairs) through 2 KB of the warp's staging area.
 __device__ __forceinline__ void aux_to_rows(uint4* stage_aux, const uint4* raw, uint32_t* aw, int lane) {
+    const uint32_t area = smem_u32(stage_aux);
     __syncwarp();
 #pragma unroll
     for (int t = 0; t < 4; t++) {
         const int r = t * 8 + (lane >> 2), q = lane & 3;
-        stage_aux[r * 4 + (q ^ ((r >> 1) & 3))] = raw[t];
+        st_shared(area + (r * 4 + (q ^ ((r >> 1) & 3))) * 16, raw[t]);
     }
     __syncwarp();
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-        const uint4 x = stage_aux[lane * 4 + (q ^ ((lane >> 1) & 3))];
+        const uint4 x = ld_shared(area + (lane * 4 + (q ^ ((lane >> 1) & 3))) * 16);
         aw[4 * q] = x.x, aw[4 * q + 1] = x.y, aw[4 * q + 2] = x.z, aw[4 * q + 3] = x.w;
     }
 }
+template <class Release>
 __device__ __forceinline__ void drain_tile_aux(const GemmArgs& p, uint32_t tbase, long long row_off, const uint16_t* ax_warp, uint4* raw,
-                                               uint4* stage, int lane) {
+                                               uint4* stage, int lane, Release release) {
     uint8_t* out0 = (uint8_t*)((uint16_t*)p.d + (row_off - (long long)lane * p.ldd));  // the warp's first row (all 32 are inside M)
 #pragma unroll 1
     for (int c = 0; c < BN / 2 / 32; c++) {
@@ -224,6 +241,7 @@ __device__ __forceinline__ void drain_tile_aux(const GemmArgs& p, uint32_t tbase
         aux_to_rows(stage + 128, raw, aw, lane);
         if (c + 1 < BN / 2 / 32) aux_load(ax_warp + (c + 1) * 32, p.ld_aux, lane, raw);
         tmem_ld_wait();
+        if (c == BN / 2 / 32 - 1) release();
         uint4 packed[4];
 #pragma unroll
         for (int j = 0; j < 32; j += 8) {
@@ -268,7 +286,7 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
     uint32_t* tmem_base_slot = (uint32_t*)(tmem_empty + 2);
     volatile int* abort_flag = (volatile int*)(tmem_base_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform for the compiler too
     const int num_tiles = p.tiles_m * p.tiles_n * p.batch;
     const int total_kb = (p.K + BK - 1) / BK;
     const int num_units = num_tiles * p.splits;  // unit = split * num_tiles + tile: neighbours share a K range
@@ -294,7 +312,7 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_base_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_base_slot, 0);
     grid_wait();
 
     if (warp == 0) {
@@ -305,8 +323,7 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             bool ok = true;
             for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x) {
                 int b, m_blk, n_blk;
-                tile_coords(p, unit % num_tiles, b, m_blk, n_blk);
-                const int kb0 = (unit / num_tiles) * p.kb_per_split, kb1 = min(total_kb, kb0 + p.kb_per_split);
+                const int kb0 = tile_coords(p, unit, b, m_blk, n_blk) * p.kb_per_split, kb1 = min(total_kb, kb0 + p.kb_per_split);
                 for (int kb = kb0; kb < kb1; kb++) {
                     if (!(ok = mbar_wait(&empty[stage], phase ^ 1, abort_flag))) break;
                     mbar_expect_tx(&full[stage], kStageBytesA + kStageBytesB);
@@ -332,8 +349,9 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             }
         }
     } else if (warp == 1) {
-        // ---- MMA issuer ----
-        if (lane == 0) {
+        // ---- MMA issuer: the whole warp, so that the operands stay in uniform registers ----
+        {
+            const bool leader = elect_one();
             const uint32_t idesc = make_idesc(BM, BN, p.in_bf16 != 0, p.a_mn_major, p.b_mn_major);
             // descriptors of stage 0; a stage and a 16-wide k step only move the address field.
             // K-major: 16 k-elements = 32 bytes further inside the swizzled 128-byte row.
@@ -348,27 +366,27 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x, local++) {
                 const int buf = local & 1;
                 const uint32_t use = (uint32_t)(local >> 1);
-                if (!(ok = mbar_wait(&tmem_empty[buf], (use & 1) ^ 1, abort_flag))) break;
+                if (!(ok = mbar_wait_warp(&tmem_empty[buf], (use & 1) ^ 1, abort_flag))) break;
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + (uint32_t)(buf * BN);
-                const int kb0 = (unit / num_tiles) * p.kb_per_split;
+                const int kb0 = (int)p.by_tiles.div(unit) * p.kb_per_split;
                 const int num_kb = min(total_kb, kb0 + p.kb_per_split) - kb0;
                 for (int kb = 0; kb < num_kb; kb++) {
-                    if (!(ok = mbar_wait(&full[stage], phase, abort_flag))) break;
+                    if (!(ok = mbar_wait_warp(&full[stage], phase, abort_flag))) break;
                     tc_fence_after();
                     uint64_t da = desc_advance(da0, (uint32_t)(stage * kStageBytesA)), db = desc_advance(db0, (uint32_t)(stage * kStageBytesB));
 #pragma unroll
                     for (int k = 0; k < BK / 16; k++) {
-                        mma_f16(tmem_d, da, db, idesc, (kb | k) != 0);
+                        mma_f16(tmem_d, da, db, idesc, (kb | k) != 0, leader);
                         da = desc_advance(da, a_step), db = desc_advance(db, b_step);
                     }
-                    mma_commit(&empty[stage]);  // frees the stage once these MMAs have read it
+                    mma_commit(&empty[stage], leader);  // frees the stage once these MMAs have read it
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
                     }
                 }
-                if (ok) mma_commit(&tmem_full[buf]);
+                if (ok) mma_commit(&tmem_full[buf], leader);
             }
         }
     } else {
@@ -385,8 +403,7 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             const int buf = local & 1;
             const uint32_t use = (uint32_t)(local >> 1);
             int b, m_blk, n_blk;
-            tile_coords(p, unit % num_tiles, b, m_blk, n_blk);
-            const int split = unit / num_tiles;
+            const int split = tile_coords(p, unit, b, m_blk, n_blk);
             const int row = m_blk * BM + quarter * 32 + lane;
             const int col_base = n_blk * BN + col_half * (BN / 2);
             const long long row_off = (long long)b * p.d_batch_stride + (long long)row * p.ldd;
@@ -398,11 +415,13 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             __syncwarp();
             tc_fence_after();
             const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + col_half * (BN / 2));
-            if (fast) drain_tile_aux(p, tbase, row_off + col_base, ax_warp, raw, stage, lane);
-            else drain_tile(p, tbase, row, row_off, col_base, b, split, vec_ok, stage, lane);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+            auto release = [&] {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+            };
+            if (fast) drain_tile_aux(p, tbase, row_off + col_base, ax_warp, raw, stage, lane, release);
+            else drain_tile(p, tbase, row, row_off, col_base, b, split, vec_ok, stage, lane, release);
         }
     }
 
@@ -431,6 +450,13 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
 // operand-fetch ceiling. The leader (rank 0) issues all MMAs; its commits arrive on the barriers of both CTAs. Both
 // CTAs load their own tiles with TMA, counting bytes on the leader's `full` barrier. Each CTA drains its own 128
 // accumulator rows; "accumulator drained" arrivals from both CTAs go to the leader's `tmem_empty` barrier.
+//
+// What bounds it: with K of 2048 and more the products (16384 x 4096 x 4096: 91 % of the tensor pipe's rate between two tiles, then
+// the power cap); with shorter K the time a tile needs for its way out, so that the hand-over is kept short: the accumulator goes back
+// once its last columns are in registers, by an arrival that waits for no global store; where a tile lies is found without
+// divisions; the staging area is addressed as shared memory; and products are issued warp-wide. Together, us a product, bfloat16:
+// 16384 x 4096 with K = 64 92 -> 45, K = 512 108 -> 74, K = 1024 142 -> 119; 16384 x 32768 x 1024 1100 -> 920; 6442 x 1120 x 280
+// 17.8 -> 12.9; 3000 x 3000 x 600 23.8 -> 18.8; 16384 x 1024 x 4096 121 -> 117; 8192^3 885 -> 858.
 constexpr int PSTAGES = 6;
 constexpr int kPairStageBytesA = BM * BK * 2, kPairStageBytesB = (BN / 2) * BK * 2;
 constexpr int kPairSmemBytes = PSTAGES * (kPairStageBytesA + kPairStageBytesB) + 1024 + 256 + kEpilogueStageBytes;
@@ -448,7 +474,7 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     uint32_t* tmem_base_slot = (uint32_t*)(tmem_empty + 2);
     volatile int* abort_flag = (volatile int*)(tmem_base_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform for the compiler too
     const uint32_t rank = cluster_ctarank();
     const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
     const int num_tiles = p.tiles_m * p.tiles_n * p.batch;  // tiles_m counts 256-row pair tiles here
@@ -477,7 +503,7 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     __syncthreads();
     cluster_sync();  // barriers of both CTAs are initialised and both allocations are done before anyone signals across
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_base_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_base_slot, 0);
     grid_wait();
 
     if (warp == 0) {
@@ -488,9 +514,9 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             bool ok = true;
             for (int unit = pair; unit < num_units && ok; unit += num_pairs) {
                 int b, m_blk, n_blk;
-                tile_coords(p, unit % num_tiles, b, m_blk, n_blk);
+                const int kb0 = tile_coords(p, unit, b, m_blk, n_blk) * p.kb_per_split;
                 const int row0 = m_blk * 2 * BM + (int)rank * BM, col0 = n_blk * BN + (int)rank * (BN / 2);
-                const int kb0 = (unit / num_tiles) * p.kb_per_split, kb1 = min(total_kb, kb0 + p.kb_per_split);
+                const int kb1 = min(total_kb, kb0 + p.kb_per_split);
                 for (int kb = kb0; kb < kb1; kb++) {
                     if (!(ok = mbar_wait(&empty[stage], phase ^ 1, abort_flag))) break;
                     if (rank == 0) mbar_expect_tx(&full[stage], 2 * (kPairStageBytesA + kPairStageBytesB));
@@ -524,8 +550,9 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
         }
     } else if (warp == 1) {
-        // ---- MMA issuer (leader only) ----
-        if (lane == 0 && rank == 0) {
+        // ---- MMA issuer (leader CTA only): the whole warp, so that the operands stay in uniform registers ----
+        if (rank == 0) {
+            const bool leader = elect_one();
             const uint32_t idesc = make_idesc(2 * BM, BN, p.in_bf16 != 0, p.a_mn_major, p.b_mn_major);
             const uint64_t da0 = p.a_mn_major ? make_smem_desc(smem_u32(smem_a), 64 * BK * 2, 1024) : make_smem_desc(smem_u32(smem_a), 16, 1024);
             const uint64_t db0 = p.b_mn_major ? make_smem_desc(smem_u32(smem_b), 64 * BK * 2, 1024) : make_smem_desc(smem_u32(smem_b), 16, 1024);
@@ -537,27 +564,27 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             for (int unit = pair; unit < num_units && ok; unit += num_pairs, local++) {
                 const int buf = local & 1;
                 const uint32_t use = (uint32_t)(local >> 1);
-                if (!(ok = mbar_wait_cluster(&tmem_empty[buf], (use & 1) ^ 1, abort_flag))) break;
+                if (!(ok = mbar_wait_cluster_warp(&tmem_empty[buf], (use & 1) ^ 1, abort_flag))) break;
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + (uint32_t)(buf * BN);
-                const int kb0 = (unit / num_tiles) * p.kb_per_split;
+                const int kb0 = (int)p.by_tiles.div(unit) * p.kb_per_split;
                 const int num_kb = min(total_kb, kb0 + p.kb_per_split) - kb0;
                 for (int kb = 0; kb < num_kb; kb++) {
-                    if (!(ok = mbar_wait(&full[stage], phase, abort_flag))) break;
+                    if (!(ok = mbar_wait_warp(&full[stage], phase, abort_flag))) break;
                     tc_fence_after();
                     uint64_t da = desc_advance(da0, (uint32_t)(stage * kPairStageBytesA)), db = desc_advance(db0, (uint32_t)(stage * kPairStageBytesB));
 #pragma unroll
                     for (int k = 0; k < BK / 16; k++) {
-                        mma_f16_pair(tmem_d, da, db, idesc, (kb | k) != 0);
+                        mma_f16_pair(tmem_d, da, db, idesc, (kb | k) != 0, leader);
                         da = desc_advance(da, a_step), db = desc_advance(db, b_step);
                     }
-                    mma_commit_pair(&empty[stage], 3);  // frees the stage in both CTAs
+                    mma_commit_pair(&empty[stage], 3, leader);  // frees the stage in both CTAs
                     if (++stage == PSTAGES) {
                         stage = 0;
                         phase ^= 1;
                     }
                 }
-                if (ok) mma_commit_pair(&tmem_full[buf], 3);
+                if (ok) mma_commit_pair(&tmem_full[buf], 3, leader);
             }
         }
     } else {
@@ -573,8 +600,7 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             const int buf = local & 1;
             const uint32_t use = (uint32_t)(local >> 1);
             int b, m_blk, n_blk;
-            tile_coords(p, unit % num_tiles, b, m_blk, n_blk);
-            const int split = unit / num_tiles;
+            const int split = tile_coords(p, unit, b, m_blk, n_blk);
             const int row = m_blk * 2 * BM + (int)rank * BM + quarter * 32 + lane;
             const int col_base = n_blk * BN + col_half * (BN / 2);
             const long long row_off = (long long)b * p.d_batch_stride + (long long)row * p.ldd;
@@ -586,11 +612,13 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             __syncwarp();
             tc_fence_after();
             const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + col_half * (BN / 2));
-            if (fast) drain_tile_aux(p, tbase, row_off + col_base, ax_warp, raw, stage, lane);
-            else drain_tile(p, tbase, row, row_off, col_base, b, split, vec_ok, stage, lane);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(&tmem_empty[buf], 0);
+            auto release = [&] {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(&tmem_empty[buf], 0);
+            };
+            if (fast) drain_tile_aux(p, tbase, row_off + col_base, ax_warp, raw, stage, lane, release);
+            else drain_tile(p, tbase, row, row_off, col_base, b, split, vec_ok, stage, lane, release);
         }
     }
 
@@ -852,6 +880,11 @@ void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
             p.kb_per_split = (total_kb + want - 1) / want;
             p.splits = (total_kb + p.kb_per_split - 1) / p.kb_per_split;
         }
+        if (tiles * p.splits > INT32_MAX) fail(LB_ERR_UNSUPPORTED, "gemm: too many output tiles for one launch");
+        p.by_tiles.set((uint32_t)tiles), p.by_batch.set((uint32_t)(p.tiles_m * p.tiles_n));
+        p.group_m = std::min(p.group_m, p.tiles_m);
+        p.by_group.set((uint32_t)(p.group_m * p.tiles_n)), p.by_rows.set((uint32_t)p.group_m);
+        p.by_last_rows.set((uint32_t)(p.tiles_m % p.group_m ? p.tiles_m % p.group_m : p.group_m));
         if (pairs) {
             const int resident = max_pairs > 0 ? max_pairs : sms / 2;
             int grid = 2 * (int)std::min<long long>(tiles * p.splits, resident);

@@ -139,18 +139,9 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem] * B[smem], one CTA, 16-bit inputs, issued by one thread.
-__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// The same executed by a whole convergent warp, of which the lane with `leader` set (elect_one) issues it. The operands
-// then stay in the warp's uniform registers, where the instruction wants them; in a branch of one lane every operand of
-// every product is moved there first (head dim 128, forward: 114 cycles per 128 x 128 x 16 product in the issuing thread).
+// D[tmem] (+)= A[smem] * B[smem], one CTA, 16-bit inputs: executed by a whole convergent warp, of which the lane with `leader`
+// set (elect_one) issues it. The operands then stay in the warp's uniform registers, where the instruction wants them; in a
+// branch of one lane every operand of every product is moved there first (head dim 128, forward: 114 cycles per 128 x 128 x 16 product in the issuing thread).
 __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, bool leader) {
     asm volatile(
         "{\n\t.reg .pred p, e;\n\t"
@@ -170,6 +161,7 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uin
         ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader)
         : "memory");
 }
+// Arrives on `bar` once every tcgen05.mma issued so far by the leader lane has completed (implies fence::before_thread_sync).
 __device__ __forceinline__ void mma_commit(uint64_t* bar, bool leader) {
     asm volatile(
         "{\n\t.reg .pred e;\n\t"
@@ -182,11 +174,6 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar, bool leader) {
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
-// Arrives on `bar` once every tcgen05.mma issued so far by this thread has completed (implies fence::before_thread_sync).
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 // 32 consecutive fp32 columns of this thread's TMEM lane (the warp's 32-lane quarter) into registers.
 __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t* v) {
     asm volatile(
@@ -262,12 +249,13 @@ __device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorM
         ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar) & kLeaderMask), "r"(c0), "r"(c1), "r"(c2)
         : "memory");
 }
-// Arrives on the barrier at `bar`'s offset in CTA `rank` of the cluster.
+// Arrives on the barrier at `bar`'s offset in CTA `rank` of the cluster. Orders tensor-memory accesses only (with the tcgen05
+// fences on both sides): a release at cluster scope would first wait, about a microsecond, for the thread's global stores.
 __device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, uint32_t rank) {
     asm volatile(
         "{\n\t.reg .b32 ra;\n\t"
         "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
-        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}"
+        "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [ra];\n\t}"
         ::"r"(smem_u32(bar)), "r"(rank)
         : "memory");
 }
@@ -304,20 +292,28 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t addr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
 }
-// D[tmem of both CTAs] (+)= A * B over the pair (M = 256: 128 rows per CTA), issued by one thread of the leader.
-__device__ __forceinline__ void mma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ bool mbar_wait_cluster_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag));
+}
+// D[tmem of both CTAs] (+)= A * B over the pair (M = 256: 128 rows per CTA), executed by a whole convergent warp of the leader
+// CTA and issued by its lane with `leader` set, as mma_f16.
+__device__ __forceinline__ void mma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, bool leader) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, e;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        "setp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader)
         : "memory");
 }
 // Arrives on the barrier at `bar`'s offset in every CTA of `cta_mask` once the pair's MMAs issued so far have completed.
-__device__ __forceinline__ void mma_commit_pair(uint64_t* bar, uint16_t cta_mask) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(smem_u32(bar)), "h"(cta_mask)
-                 : "memory");
+__device__ __forceinline__ void mma_commit_pair(uint64_t* bar, uint16_t cta_mask, bool leader) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\t"
+        "setp.ne.b32 e, %2, 0;\n\t"
+        "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+        ::"r"(smem_u32(bar)), "h"(cta_mask), "r"((uint32_t)leader)
+        : "memory");
 }
 
 // ---- descriptors --------------------------------------------------------------------------------------------
@@ -353,22 +349,34 @@ __host__ __device__ constexpr uint32_t make_idesc(int m, int n, bool bf16, bool 
 // shared memory, so that one store instruction covers whole rows of SEGS * 16 contiguous bytes (four 128-byte lines
 // for SEGS = 8) instead of one 16-byte piece of 32 different lines. Segments are XOR-swizzled within a row: both the
 // row-per-lane writes and the segment-per-lane reads are free of bank conflicts. Called by all lanes of the warp.
+// The area is addressed in the shared window: through generic pointers each read waited for the global store before it, which might
+// have gone to the same place (64 columns of a 256 x 256 product tile took 3000 cycles, most of them such waits).
 constexpr int kStageBytesPerWarp = 4096;
+__device__ __forceinline__ void st_shared(uint32_t addr, uint4 x) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(x.x), "r"(x.y), "r"(x.z), "r"(x.w) : "memory");
+}
+__device__ __forceinline__ uint4 ld_shared(uint32_t addr) {
+    uint4 x;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "r"(addr) : "memory");
+    return x;
+}
 template <int SEGS>
 __device__ __forceinline__ void store_rows_coalesced(uint4* stage, const uint4* w, uint8_t* out0, long long ld_bytes, int rows_valid, int lane) {
     constexpr int RP = 32 / SEGS;  // rows per store instruction
     auto swz = [](int row) { return SEGS == 8 ? (row & 7) : ((row >> 1) & 3); };
+    const uint32_t area = smem_u32(stage);
     __syncwarp();  // the previous pass has been read out
 #pragma unroll
-    for (int q = 0; q < SEGS; q++) stage[lane * SEGS + (q ^ swz(lane))] = w[q];
+    for (int q = 0; q < SEGS; q++) st_shared(area + (lane * SEGS + (q ^ swz(lane))) * 16, w[q]);
     __syncwarp();
     const int q = lane % SEGS, sub = lane / SEGS;
+    uint4 x[SEGS];
 #pragma unroll
-    for (int t = 0; t < SEGS; t++) {
-        const int r = t * RP + sub;
-        const uint4 x = stage[r * SEGS + (q ^ swz(r))];
-        if (r < rows_valid) *(uint4*)(out0 + (long long)r * ld_bytes + q * 16) = x;
-    }
+    for (int t = 0; t < SEGS; t++) x[t] = ld_shared(area + ((t * RP + sub) * SEGS + (q ^ swz(t * RP + sub))) * 16);
+    uint8_t* out = out0 + (long long)sub * ld_bytes + q * 16;
+#pragma unroll
+    for (int t = 0; t < SEGS; t++, out += RP * ld_bytes)
+        if (t * RP + sub < rows_valid) *(uint4*)out = x[t];
 }
 
 }  // namespace sm100
