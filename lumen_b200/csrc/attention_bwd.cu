@@ -97,7 +97,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
     constexpr int kRBlock = BR * 128, kTBlock = BT * 128;  // bytes of one 64-wide head-dim block of a tile
     constexpr int DB = D / 64;
     extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* smem = align_1024(smem_raw);
     uint8_t* sr1 = smem;
     uint8_t* sr2 = smem + kResident;
     uint8_t* st1 = smem + 2 * kResident;

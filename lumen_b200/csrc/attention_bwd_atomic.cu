@@ -86,7 +86,7 @@ attention_bwd_atomic_kernel(const __grid_constant__ CUtensorMap map_k, const __g
                             const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
                             const __grid_constant__ CUtensorMap map_acc, const AtomicArgs p) {
     extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* smem = align_1024(smem_raw);
     uint8_t* sk = smem;
     uint8_t* sv = smem + kTile;
     uint8_t* sq = smem + 2 * kTile;             // STAGES tiles

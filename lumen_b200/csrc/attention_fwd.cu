@@ -234,7 +234,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     auto kst = [](int j) { return j % NS; };
     auto kph = [](int j) { return (uint32_t)(j / NS) & 1u; };
     extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* smem = align_1024(smem_raw);
     uint8_t* sq = smem;
     uint8_t* sk = smem + kTile;             // NS stages
     uint8_t* sv = smem + (1 + NS) * kTile;  // NS stages
@@ -433,7 +433,7 @@ attention_fwd_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     constexpr int kHalf = 128 * 128, DB = D / 64;
     constexpr bool kSeparateP = D == 64;  // S 2 x 128, O 2 x 64, P 2 x 64; at head dim 128 P overwrites S
     extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* smem = align_1024(smem_raw);
     uint8_t* sq = smem;                     // two tiles
     uint8_t* sk = smem + 2 * kTile;         // NS stages
     uint8_t* sv = sk + NS * kTile;          // NS stages
@@ -451,10 +451,10 @@ attention_fwd_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     uint64_t* pv_full = p_ready + 2;        // 2
     uint64_t* next_full = pv_full + 2;      // 2
     uint64_t* next_empty = next_full + 2;   // 2: one arrival of the MMA warp, one of each softmax warp
-    uint8_t* next_slot = (uint8_t*)(((uintptr_t)(next_empty + 2) + 15) & ~(uintptr_t)15);  // 2 x 16 bytes
+    uint8_t* next_slot = (uint8_t*)(next_empty + 2);  // 2 x 16 bytes, 16-byte aligned: an even number of barriers before them
     uint32_t* tmem_slot = (uint32_t*)(next_slot + 32);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
-    static_assert((2 + 4 * NS + 14) * 8 + 16 + 32 + 8 <= 512, "barrier space");
+    static_assert((2 + 4 * NS + 14) % 2 == 0 && (2 + 4 * NS + 14) * 8 + 32 + 8 <= 512, "barrier space");
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform for the compiler too
     const int group = p.N / p.Nkv;

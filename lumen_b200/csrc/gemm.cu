@@ -276,7 +276,7 @@ __device__ __forceinline__ void drain_tile_aux(const GemmArgs& p, uint32_t tbase
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmArgs p) {
     extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* smem = align_1024(smem_raw);
     uint8_t* smem_a = smem;
     uint8_t* smem_b = smem + STAGES * kStageBytesA;
     uint64_t* full = (uint64_t*)(smem + STAGES * (kStageBytesA + kStageBytesB));
@@ -464,7 +464,7 @@ constexpr int kPairSmemBytes = PSTAGES * (kPairStageBytesA + kPairStageBytesB) +
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmArgs p) {
     extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* smem = align_1024(smem_raw);
     uint8_t* smem_a = smem;
     uint8_t* smem_b = smem + PSTAGES * kPairStageBytesA;
     uint64_t* full = (uint64_t*)(smem + PSTAGES * (kPairStageBytesA + kPairStageBytesB));

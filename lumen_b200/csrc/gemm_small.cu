@@ -42,7 +42,7 @@ template <int STAGES>
 __global__ void __launch_bounds__(kThreads, 8 / STAGES)
 gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const SmallGemmArgs p) {
     extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* smem = align_1024(smem_raw);
     uint8_t *sa = smem, *sb = smem + STAGES * kStageA;
     uint64_t* full = (uint64_t*)(smem + STAGES * (kStageA + kStageB));
     uint64_t* empty = full + STAGES;

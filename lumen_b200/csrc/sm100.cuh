@@ -13,6 +13,12 @@ namespace sm100 {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// The next 1024-byte boundary at or after `p`, which points into shared memory. An offset is added instead of rounding the
+// address, so that the compiler still sees where the pointer leads and loads and stores through it are those of shared memory.
+// (Through generic pointers every read waits behind stores it might alias. Attention forward and backward, us: 8 x 16 heads x 2048 x
+// 64 causal 488 -> 449, 8 x 32 x 4096 x 128 5156 -> 4765; prefill of 2 x 32 heads x 1531 x 128 57.0 -> 54.2.)
+__device__ __forceinline__ uint8_t* align_1024(uint8_t* p) { return p + ((0u - smem_u32(p)) & 1023u); }
+
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred;
     asm volatile(
