@@ -42,6 +42,7 @@ void attention_backward(const lb_attn_desc& desc, const lb_tensor& q, const lb_t
 void scatter_add_rows(const lb_tensor& x, const lb_tensor& ids, const lb_tensor& updates, const lb_tensor& out, void* scratch,
                       bool x_is_zero, bool deterministic, void* stream);
 size_t scatter_add_scratch_bytes(long long rows, long long width, long long tokens, bool deterministic);
+int scatter_add_launches(long long rows, long long tokens, bool deterministic);
 void comm_all_reduce(lb_comm* c, const void* send, void* recv, size_t count, int dtype, int op, void* stream);
 int comm_world(const lb_comm* c);
 
@@ -551,7 +552,13 @@ int lb_plan_kernel_launches(const lb_plan* plan) {
             case lb::GEMM: n += s.scratch >= 0 ? 2 : 1; break;  // split-K partial tiles + reduction
             case lb::ATTN_FWD: n += 1; break;
             case lb::ATTN_BWD: n += 3; break;  // delta, then dK/dV and dQ - or the single kernel and the rounding of dQ
-            case lb::SCATTER_ADD: n += s.epilogue ? 4 : 2; break;
+            case lb::SCATTER_ADD: {
+                const lb_tensor &ids = plan->views.at((size_t)s.args.at(1)).t, &out = plan->views.at((size_t)s.args.at(3)).t;
+                long long tokens = 1;
+                for (int d = 0; d < ids.rank; d++) tokens *= ids.shape[d];
+                n += lb::scatter_add_launches(out.shape[0], tokens, s.epilogue != 0);
+                break;
+            }
             case lb::TRANSPOSE: n += 1; break;
             case lb::COPY: n += lb::copy_form(plan->views.at((size_t)s.args.at(0)).t, plan->views.at((size_t)s.args.at(1)).t) == 2 ? 1 : 0; break;
             default: break;  // block and 2-d copies, fills, collectives and waits launch no kernel of this library

@@ -154,6 +154,53 @@ __global__ void scatter_rows_kernel(T* __restrict__ out, const T* __restrict__ x
     }
 }
 
+// The same in one kernel for few updates: every block looks through all destinations and keeps the updates of its row, in update
+// order: each of its eight warps those of a stretch, found by ballots. What bounds it is latency, one pass over the destinations
+// and one over the row's updates, where the counting sort is a memset and four kernels in a chain; the destinations are read by every
+// row, so the rule keeps rows, updates and their product small. us: 512 updates of 128 float32 into 256 rows 10.5 -> 2.9, 1024 into
+// 512 rows 10.5 -> 4.2, 336 of 256 bfloat16 into 1280 rows 8.4 -> 7.1, 4096 of 512 into 1024 rows 11.9 -> 9.7; beyond it 512 of 1024
+// into 8192 rows 26 -> 40.
+constexpr int kFewUpdates = 4096, kFewRows = 2048;
+constexpr long long kFewReads = 1LL << 22;
+template <class T, class I>
+__global__ void __launch_bounds__(256) scatter_rows_few_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __restrict__ updates, const I* __restrict__ ids,
+                                                               int tokens, long long rows, int width, int has_x) {
+    constexpr int kWarps = 8, kBallots = kFewUpdates / (32 * kWarps);
+    __shared__ int picks[kFewUpdates], counts[kWarps];
+    grid_wait();
+    const int r = (int)blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int stretch = (tokens + 32 * kWarps - 1) / (32 * kWarps) * 32, first = warp * stretch;
+    unsigned hits[kBallots];
+    int mine = 0;
+#pragma unroll
+    for (int i = 0; i < kBallots; i++) {
+        const int t = first + i * 32 + lane;
+        const bool hit = i * 32 < stretch && t < tokens && clamped_row(ids, t, rows) == r;
+        hits[i] = __ballot_sync(0xffffffffu, hit);
+        mine += __popc(hits[i]);
+    }
+    if (lane == 0) counts[warp] = mine;
+    __syncthreads();
+    int at = 0, n = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) {
+        if (w == warp) at = n;
+        n += counts[w];
+    }
+#pragma unroll
+    for (int i = 0; i < kBallots; i++) {
+        if (hits[i] >> lane & 1) picks[at + __popc(hits[i] & ((1u << lane) - 1))] = first + i * 32 + lane;
+        at += __popc(hits[i]);
+    }
+    __syncthreads();
+    for (int d = threadIdx.x; d < width; d += blockDim.x) {
+        float acc = has_x ? to_f(x[(long long)r * width + d]) : 0.0f;
+#pragma unroll 4
+        for (int i = 0; i < n; i++) acc = to_f(from_f<T>(__fadd_rn(acc, to_f(updates[(long long)picks[i] * width + d]))));
+        out[(long long)r * width + d] = from_f<T>(acc);
+    }
+}
+
 struct AttnShape {
     int B, Sq, Sk, N, Nkv, D;
     long long q_s[3], k_s[3], v_s[3], o_s[3], g_s[3], dq_s[3], dk_s[3], dv_s[3];  // strides of dims B, S, N (head dim is dense)
@@ -490,6 +537,11 @@ size_t scatter_add_scratch_bytes(long long rows, long long width, long long toke
     return deterministic ? (size_t)(3 * rows + 1 + 2 * tokens) * 4 : (size_t)rows * width * 4;
 }
 
+// Kernels that scatter_add_rows launches.
+int scatter_add_launches(long long rows, long long tokens, bool deterministic) {
+    return !deterministic ? 2 : tokens <= kFewUpdates && rows <= kFewRows && rows * tokens <= kFewReads ? 1 : 4;
+}
+
 void scatter_add_rows(const lb_tensor& x, const lb_tensor& ids, const lb_tensor& updates, const lb_tensor& out, void* scratch,
                       bool x_is_zero, bool deterministic, void* stream) {
     if (x.rank != 2) fail(LB_ERR_UNSUPPORTED, "scatter_add: a [rows, width] operand scattered along axis 0");
@@ -506,6 +558,20 @@ void scatter_add_rows(const lb_tensor& x, const lb_tensor& ids, const lb_tensor&
     driver();
     cudaStream_t s = (cudaStream_t)stream;
     if (rows == 0 || width == 0) return;
+    if (scatter_add_launches(rows, tokens, deterministic) == 1) {
+        auto launch = [&](auto* o, auto* i) {
+            using T = std::remove_pointer_t<decltype(o)>;
+            using I = std::remove_const_t<std::remove_pointer_t<decltype(i)>>;
+            launch_overlapped(scatter_rows_few_kernel<T, I>, dim3((unsigned)rows), dim3(256), 0, s, 0, o, (const T*)x.ptr, (const T*)updates.ptr, i, (int)tokens, rows, (int)width, !x_is_zero);
+        };
+        auto by_ids = [&](auto* o) {
+            if (ids.dtype == LB_I64) launch(o, (const long long*)ids.ptr);
+            else launch(o, (const int*)ids.ptr);
+        };
+        if (x.dtype == LB_F32) by_ids((float*)out.ptr);
+        else by_ids((__nv_bfloat16*)out.ptr);
+        return;
+    }
     if (deterministic) {
         int* counts = (int*)scratch;
         int* cursor = counts + rows;

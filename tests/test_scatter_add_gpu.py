@@ -27,6 +27,9 @@ CASES = [
     (16, 40, 5000, np.int64, "bfloat16", 2),      # two rows take 2500 picks each: the rank-sorted long-segment path
     (33, 8, 1, np.int64, "float32", 33),
     (128, 1024, 4096, np.int64, "bfloat16", 128),
+    # one kernel for few updates: its largest numbers of updates and rows, one past each; all on one row; stretches of a warp
+    (2048, 4, 2048, np.int64, "float32", 2048), (2049, 4, 100, np.int32, "float32", 2049), (1024, 8, 4096, np.int64, "float32", 1024), (1025, 8, 4096, np.int32, "float32", 1025), (128, 24, 4097, np.int64, "bfloat16", 128),
+    (5, 300, 4096, np.int32, "bfloat16", 1), (300, 33, 257, np.int64, "float32", 300), (300, 33, 255, np.int64, "bfloat16", 300),
 ]
 
 
