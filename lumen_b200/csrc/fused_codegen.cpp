@@ -1512,12 +1512,15 @@ class Generator {
 
     // The second kernel of a column reduction: adds the slices' partial sums and applies the epilogue. A block takes 32
     // lanes of two columns and one (up to eight slices), eight or 32 slice lanes: few columns and slices per thread, so that the chains of loads stay
-    // short (1184 slices of 1024 columns took 19 us with eight slice lanes).
+    // short (1184 slices of 1024 columns took 19 us with eight slice lanes). Many slices of few columns take 128 slice lanes, on eight
+    // column lanes: four times the blocks, and a thread's chain of loads a quarter (a residual layer norm of 8192 x 1024 with its backward, whose totals are 592 slices of 1024 columns, 36.1 -> 33.5 us).
     void emit_finalize(std::ostringstream& s, const std::string& sig, const std::vector<size_t>& offsets, const std::vector<int>& outputs, FusedKernel& k) {
         column_mode_ = true;
         VEC_ = std::min(VEC_, 2);
         pair_ = VEC_ >= 2 && computes_bf16();
-        const int col_lanes = 32, row_lanes = k.slices * k.col_blocks > 64 ? 32 : k.slices * k.col_blocks > 8 ? 8 : 1, threads = col_lanes * row_lanes;
+        const int64_t slices = k.slices * k.col_blocks;
+        const bool many = slices > 256 && C_ <= 64LL * VEC_ * 32;
+        const int col_lanes = many ? 8 : 32, row_lanes = many ? 128 : slices > 64 ? 32 : slices > 8 ? 8 : 1, threads = col_lanes * row_lanes;
         Comp flat_c;
         flat_c.base = "c0", flat_c.expr = "(c0 + e)";
         flat_c.lane = flat_c.e_dep = flat_c.c_dep = true;
@@ -1554,8 +1557,9 @@ class Generator {
                        << (row_lanes == 1 ? "" : format("auto lanes = (%s(*)[%d * VEC + 1])(shared + %zu);\n    ", type.c_str(), col_lanes, (k - k0) * lane_bytes) + each("lanes[row_lane][col_lane * VEC + e] = " + tot + "[e];") + "\n")
                        << "}\n";
                 trees << "{\n    auto lanes = (" << type << "(*)[" << col_lanes << " * VEC + 1])(shared + " << (k - k0) * lane_bytes << ");\n    " << type << "* sums = (" << type << "*)(shared + " << batch * lane_bytes + (k - k0) * sum_bytes
-                      << ");\n    const int lane = threadIdx.x % " << row_lanes << ", col = threadIdx.x / " << row_lanes << ";\n    "
-                      << each(type + " v = lanes[lane][col * VEC + e]; _Pragma(\"unroll\") for (int m = " + std::to_string(row_lanes / 2) + "; m >= 1; m /= 2) " + add("v", "shfl_xor_any<" + type + ">(v, m)") +
+                      << ");\n    const int lane = threadIdx.x % " << std::min(row_lanes, 32) << ", col = threadIdx.x / " << std::min(row_lanes, 32) << ";\n    "
+                      << (many ? format("if (col < %d) ", col_lanes) : "") << each(type + " v = lanes[lane][col * VEC + e]; " + (many ? type + " v1 = lanes[lane + 32][col * VEC + e], v2 = lanes[lane + 64][col * VEC + e]; " +
+                              add("v", "v1") + " v1 = lanes[lane + 96][col * VEC + e]; " + add("v2", "v1") + " " + add("v", "v2") + " " : "") + "_Pragma(\"unroll\") for (int m = " + std::to_string(std::min(row_lanes, 32) / 2) + "; m >= 1; m /= 2) " + add("v", "shfl_xor_any<" + type + ">(v, m)") +
                               " if (lane == 0) sums[col * VEC + e] = v;")
                       << "\n}\n";
                 reads << each(tot + "[e] = ((const " + type + "*)(shared + " + std::to_string(batch * lane_bytes + (k - k0) * sum_bytes) + "))[col_lane * VEC + e];") << "\n";
@@ -1577,7 +1581,7 @@ class Generator {
         s << "#undef VEC\n#define VEC " << VEC_ << "\n";
         s << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") fused_finalize(" << sig << ") {\n";
         s << wait_for_grid(threads);
-        s << "    const int col_lane = tid & " << col_lanes - 1 << ", row_lane = tid >> 5;\n";
+        s << "    const int col_lane = tid & " << col_lanes - 1 << ", row_lane = tid / " << col_lanes << ";\n";
         s << "    const idx_t c0 = ((idx_t)blockIdx.x * " << col_lanes << " + col_lane) * VEC;\n    const bool in_range = c0 < NCOLS;\n";
         s << "    __shared__ __align__(16) char shared[" << shared_bytes << "];\n";
         s << indent(totals.str(), 4);

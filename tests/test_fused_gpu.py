@@ -422,3 +422,21 @@ def test_row_sums_of_odd_widths_are_as_exact_as_of_1024_threads(cuda, cols):
         return float(((t.double() - want) ** 2).mean() ** 0.5)
 
     assert rms(s) <= (1 + 3 / 8000**0.5) * rms(total[:, 0])
+
+
+# totals of 257 slices and more over few columns take 128 slice lanes: columns that are no multiple of a block's, one column, the
+# widest of them and one past, more sums than shared memory holds at once; 256 slices and fewer do not
+@pytest.mark.parametrize("rows,cols", [(300, 1), (257, 15), (256, 15), (600, 17), (5000, 1023), (700, 2047), (700, 2049), (900, 4096), (900, 4098)])
+@pytest.mark.parametrize("sums", [1, 6])
+def test_totals_of_many_slices(cuda, rows, cols, sums):
+    """Small integers: every order of the additions gives the same sum."""
+    x = torch.randint(-8, 9, (rows, cols), generator=torch.Generator(device=cuda).manual_seed(cols), device=cuda).float()
+
+    def program(a):
+        beside = prims.reduce_sum(a, (1,), "float32").reshape(rows, 1)
+        return (a + beside, *[prims.reduce_sum(a * float(k + 1), (0,), "float32") for k in range(sums)])
+
+    out = Fusion(tracer.trace(program, ("float32", (rows, cols))))(x)
+    assert torch.equal(out[0], x + x.sum(1, keepdim=True))
+    for k in range(sums):
+        assert torch.equal(out[1 + k], x.sum(0) * (k + 1))
