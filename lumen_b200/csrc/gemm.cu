@@ -79,15 +79,15 @@ __device__ __forceinline__ int tile_coords(const GemmArgs& p, int unit, int& b, 
 }
 
 // Drains 128 accumulator columns (this warp's half of a 256-wide tile) of the thread's row from tensor memory and
-// stores them: float32 partial sums when K is split, otherwise the epilogue and one rounding to the output dtype. `release` hands
-// the accumulator back to the MMA warp, once its last columns are in registers.
+// stores them with the epilogue and one rounding to the output dtype. `release` hands the accumulator back to the MMA warp, once its
+// last columns are in registers.
 template <class Release>
-__device__ __forceinline__ void drain_tile(const GemmArgs& p, uint32_t tbase, int row, long long row_off, int col_base, int b, int split,
+__device__ __forceinline__ void drain_tile(const GemmArgs& p, uint32_t tbase, int row, long long row_off, int col_base, int b,
                                            bool vec_ok, uint4* stage, int lane, Release release) {
 #pragma unroll 1
     for (int c2 = 0; c2 < BN / 2 / 64; c2++) {
         // warp-uniform: 16-bit rows of 64 whole columns leave through the staging area, 128 contiguous bytes per row
-        const bool coalesced = vec_ok && p.splits == 1 && (p.d_bf16 || p.d_f16) && col_base + c2 * 64 + 64 <= p.N;
+        const bool coalesced = vec_ok && (p.d_bf16 || p.d_f16) && col_base + c2 * 64 + 64 <= p.N;
         uint4 packed[8];
         uint32_t vv[64];
         tmem_ld_32x32(tbase + c2 * 64, vv);  // two loads in flight, one wait
@@ -99,21 +99,8 @@ __device__ __forceinline__ void drain_tile(const GemmArgs& p, uint32_t tbase, in
             uint32_t* v = vv + h * 32;
             const int col0 = col_base + c2 * 64 + h * 32;
             // warp-uniform: a float32 row piece of 32 whole columns is one 128-byte line and leaves through the staging area too
-            const bool staged32 = vec_ok && p.splits == 1 && !(p.d_bf16 || p.d_f16) && col0 + 32 <= p.N;
-            if (p.splits > 1) {
-                // a partial sum: float32, dense [split][batch][M][N]; the epilogue and rounding happen in splitk_reduce
-                if (row < p.M && col0 < p.N) {
-                    float* out = p.partial + ((long long)(split * p.batch + b) * p.M + row) * p.N + col0;
-                    if (col0 + 32 <= p.N && p.N % 4 == 0) {
-#pragma unroll
-                        for (int j = 0; j < 32; j += 4) *(uint4*)(out + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; j++)
-                            if (col0 + j < p.N) out[j] = __uint_as_float(v[j]);
-                    }
-                }
-            } else if (row < p.M && col0 < p.N) {
+            const bool staged32 = vec_ok && !(p.d_bf16 || p.d_f16) && col0 + 32 <= p.N;
+            if (row < p.M && col0 < p.N) {
                 if (p.epilogue == EPI_RELU) {
 #pragma unroll
                     for (int j = 0; j < 32; j++) v[j] = __float_as_uint(fmaxf(__uint_as_float(v[j]), 0.0f));
@@ -196,6 +183,33 @@ __device__ __forceinline__ void drain_tile(const GemmArgs& p, uint32_t tbase, in
         if (coalesced)  // rows past M hold nothing and are not written
             store_rows_coalesced<8>(stage, packed, (uint8_t*)((uint16_t*)p.d + (row_off - (long long)lane * p.ldd) + col_base + c2 * 64),
                                     p.ldd * 2, p.M - (row - lane), lane);
+    }
+}
+
+// The same where K is split: float32 partial sums, dense [split][batch][M][N]; the epilogue and the rounding happen in splitk_reduce.
+// Whole pieces of 32 columns leave as 128-byte lines through the staging area.
+template <class Release>
+__device__ __forceinline__ void drain_partial(const GemmArgs& p, uint32_t tbase, int row, int col_base, int b, int split, uint4* stage, int lane,
+                                              Release release) {
+    float* row0 = p.partial + ((long long)(split * p.batch + b) * p.M + (row - lane)) * p.N;  // the warp's first row
+#pragma unroll 1
+    for (int c = 0; c < BN / 2 / 32; c++) {
+        const int col0 = col_base + c * 32;
+        uint32_t v[32];
+        tmem_ld_32x32(tbase + c * 32, v);
+        tmem_ld_wait();
+        if (c == BN / 2 / 32 - 1) release();
+        if (p.N % 4 == 0 && col0 + 32 <= p.N) {
+            uint4 packed[8];
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) packed[j / 4] = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            store_rows_coalesced<8>(stage, packed, (uint8_t*)(row0 + col0), (long long)p.N * 4, p.M - (row - lane), lane);
+        } else if (row < p.M) {
+            float* out = row0 + (long long)lane * p.N + col0;
+#pragma unroll
+            for (int j = 0; j < 32; j++)
+                if (col0 + j < p.N) out[j] = __uint_as_float(v[j]);
+        }
     }
 }
 
@@ -421,7 +435,8 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                 if (lane == 0) mbar_arrive(&tmem_empty[buf]);
             };
             if (fast) drain_tile_aux(p, tbase, row_off + col_base, ax_warp, raw, stage, lane, release);
-            else drain_tile(p, tbase, row, row_off, col_base, b, split, vec_ok, stage, lane, release);
+            else if (p.splits > 1) drain_partial(p, tbase, row, col_base, b, split, stage, lane, release);
+            else drain_tile(p, tbase, row, row_off, col_base, b, vec_ok, stage, lane, release);
         }
     }
 
@@ -618,7 +633,8 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 if (lane == 0) mbar_arrive_cluster(&tmem_empty[buf], 0);
             };
             if (fast) drain_tile_aux(p, tbase, row_off + col_base, ax_warp, raw, stage, lane, release);
-            else drain_tile(p, tbase, row, row_off, col_base, b, split, vec_ok, stage, lane, release);
+            else if (p.splits > 1) drain_partial(p, tbase, row, col_base, b, split, stage, lane, release);
+            else drain_tile(p, tbase, row, row_off, col_base, b, vec_ok, stage, lane, release);
         }
     }
 
@@ -640,37 +656,53 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
 }
 
-// Adds the split-K partial tiles in split order (fixed, so results are reproducible), applies the epilogue and rounds once.
-__global__ void splitk_reduce(const float* __restrict__ partial, GemmArgs p) {
+// Adds the split-K partial tiles in split order (fixed, so results are reproducible), applies the epilogue and rounds once. Bound by
+// memory: four elements of a row a thread (VEC: N is a multiple of four, rows of the result and of the epilogue's operand are aligned),
+// found by one division where twelve 64-bit ones took most of the time. With the partial tiles stored in whole lines, us a product:
+// 1192 x 1736 x 6944 46.9 -> 40.4, 704 x 1504 x 8000 32.7 -> 23.0, 1024 x 1024 x 8192 30.5 -> 24.0.
+template <bool VEC>
+__global__ void __launch_bounds__(256) splitk_reduce(const float* __restrict__ partial, GemmArgs p) {
     grid_wait();
+    constexpr int W = VEC ? 4 : 1;
     const long long per = (long long)p.batch * p.M * p.N;
-    for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < per; i += (long long)gridDim.x * blockDim.x * 4) {
-        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        const bool vec = p.N % 4 == 0;  // then a group of 4 never crosses a row
+    for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * W; i < per; i += (long long)gridDim.x * blockDim.x * W) {
+        float acc[W] = {};
+#pragma unroll 4
         for (int s = 0; s < p.splits; s++) {
-            if (vec) {
+            if constexpr (VEC) {
                 const float4 v = *(const float4*)(partial + s * per + i);
                 acc[0] += v.x, acc[1] += v.y, acc[2] += v.z, acc[3] += v.w;
             } else {
-                for (int j = 0; j < 4 && i + j < per; j++) acc[j] += partial[s * per + i + j];
+                acc[0] += partial[s * per + i];
             }
         }
-        for (int j = 0; j < 4 && i + j < per; j++) {
-            const long long e = i + j;
-            const long long b = e / ((long long)p.M * p.N), r = (e / p.N) % p.M, c = e % p.N;
+        const long long row = i / p.N, b = p.batch > 1 ? row / p.M : 0, r = row - b * p.M, c = i - row * p.N;
+        const uint16_t* aux = (const uint16_t*)p.aux + b * p.aux_batch_stride + r * p.ld_aux + c;
+        __align__(8) uint16_t a16[W], out16[W];
+        if (p.epilogue >= EPI_ADD) {
+            if constexpr (VEC) *(uint2*)a16 = *(const uint2*)aux;
+            else a16[0] = *aux;
+        }
+#pragma unroll
+        for (int j = 0; j < W; j++) {
             float x = acc[j];
             if (p.epilogue == EPI_RELU) x = fmaxf(x, 0.0f);
             if (p.epilogue >= EPI_ADD) {
-                const uint16_t a16 = ((const uint16_t*)p.aux)[b * p.aux_batch_stride + r * p.ld_aux + c];
                 float prod, other;
-                if (p.d_bf16) prod = __bfloat162float(__float2bfloat16_rn(x)), other = __uint_as_float((uint32_t)a16 << 16);
-                else prod = __half2float(__float2half_rn(x)), other = __half2float(__ushort_as_half(a16));
+                if (p.d_bf16) prod = __bfloat162float(__float2bfloat16_rn(x)), other = __uint_as_float((uint32_t)a16[j] << 16);
+                else prod = __half2float(__float2half_rn(x)), other = __half2float(__ushort_as_half(a16[j]));
                 x = p.epilogue == EPI_ADD ? __fadd_rn(other, prod) : (other > 0.0f ? prod : 0.0f);
             }
-            const long long at = b * p.d_batch_stride + r * p.ldd + c;
-            if (p.d_bf16) ((__nv_bfloat16*)p.d)[at] = __float2bfloat16_rn(x);
-            else if (p.d_f16) ((__half*)p.d)[at] = __float2half_rn(x);
-            else ((float*)p.d)[at] = x;
+            acc[j] = x;
+            out16[j] = p.d_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(x)) : __half_as_ushort(__float2half_rn(x));
+        }
+        const long long at = b * p.d_batch_stride + r * p.ldd + c;
+        if (p.d_bf16 || p.d_f16) {
+            if constexpr (VEC) *(uint2*)((uint16_t*)p.d + at) = make_uint2(out16[0] | (uint32_t)out16[1] << 16, out16[2] | (uint32_t)out16[3] << 16);
+            else ((uint16_t*)p.d)[at] = out16[0];
+        } else {
+            if constexpr (VEC) *(float4*)((float*)p.d + at) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+            else ((float*)p.d)[at] = acc[0];
         }
     }
 }
@@ -744,18 +776,23 @@ int gemm_splits(long long M, long long N, long long K, long long batch, int sms)
 // tiles -> these), bfloat16: 64^3 8.2 -> 6.2, 512^3 13.5 -> 8.5, 200 x 4096 K 1024 16.4 -> 11.5, 200 x 1024 K 4096 24.6 -> 12.3
 // (4 ranges), 1000^3 18.5 -> 12.3, 128 x 8192 K 8192 49 -> 35, 1024 x 1024 K 8192 35 -> 28 (39 with one range); beyond the line
 // 4096 x 1024 K 200 12.3 -> 16.4, 700 x 4096 K 1024 16.4 -> 20.5, 2048^3 22.6 -> 32.7.
-int gemm_small_splits(long long M, long long N, long long K, long long batch, int sms) {
+// Where scratch lets large tiles cut K (`large_split`), ranges that would be 64 blocks and longer with one CTA to an SM go there, since a
+// narrow tile fetches twice the bytes per product: 1024 x 1024 (us, these -> large) K 16384 43.7 -> 32.7, 8192 29.0 -> 23.5, 4096 22.1 -> 17.9,
+// 768 x 768 x 8192 20.8 -> 16.8, 768 x 1024 x 16384 41.6 -> 26.7; but 32 blocks: 512 x 512 x 8192 14.6 -> 15.7, 1024 x 1024 x 2048 13.0 -> 17.1.
+int gemm_small_splits(long long M, long long N, long long K, long long batch, int sms, bool large_split) {
     const long long tiles = (M + 127) / 128 * ((N + 63) / 64) * batch, total_kb = (K + BK - 1) / BK;
     if (tiles > sms) return 0;
     int s = 1;
     while (s < 8 && tiles * 2 * s <= sms && total_kb >= 4 * s) s *= 2;
+    if (large_split && total_kb >= 64 * s) return 0;
     if (s < 8 && total_kb > 64 * s && tiles * s <= sms) s *= 2;
     return total_kb <= 128 * s ? s : 0;  // longer ranges: not measured, left to the split-K kernels
 }
 
 // Scratch a plan's product step takes: none where the narrow tiles run.
 extern "C" size_t lb_gemm_step_scratch_bytes(int64_t m, int64_t n, int64_t k) {
-    return gemm_small_splits(m, n, k, 1, sm_count_hint()) ? 0 : gemm_scratch_bytes(m, n, k, 1);
+    const size_t bytes = gemm_scratch_bytes(m, n, k, 1);
+    return gemm_small_splits(m, n, k, 1, sm_count_hint(), bytes > 0) ? 0 : bytes;
 }
 
 // CTA pairs of gemm_tcgen05_pair that can be resident on `dev` at once (asked of the runtime once per device).
@@ -854,7 +891,9 @@ void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
         CUtensorMap map_b = p.b_mn_major ? make_map(bt, false, 64, BK) : make_map(bt, true, BK, pairs ? BN / 2 : BN);
         const DeviceInfo& dev = device_info();
         // no kernel asked for and no split or raster tuned: narrow tiles where they fit (gemm_small_splits)
-        if (const int ranges = kernel_choice == 0 && !(tuning && (tuning->splits > 0 || tuning->group_m > 0)) ? gemm_small_splits(M, N, K, batch, dev.sms) : 0) {
+        const int split = scratch ? gemm_splits(M, N, K, batch, dev.sms) : 1;
+        const bool large_split = split > 1 && scratch_bytes >= (size_t)split * batch * M * N * 4 && ((uintptr_t)scratch & 15) == 0;
+        if (const int ranges = kernel_choice == 0 && !(tuning && (tuning->splits > 0 || tuning->group_m > 0)) ? gemm_small_splits(M, N, K, batch, dev.sms, large_split) : 0) {
             SmallGemmArgs q{};
             q.M = p.M, q.N = p.N, q.K = p.K, q.a_mn_major = p.a_mn_major, q.b_mn_major = p.b_mn_major, q.in_bf16 = p.in_bf16;
             q.d = p.d, q.d_bf16 = p.d_bf16, q.d_f16 = p.d_f16, q.ldd = p.ldd, q.d_batch_stride = p.d_batch_stride;
@@ -873,7 +912,7 @@ void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
         p.splits = 1;
         p.kb_per_split = (int)((K + BK - 1) / BK);
         p.partial = (float*)scratch;
-        int want = scratch ? gemm_splits(M, N, K, batch, sms) : 1;
+        int want = split;
         if (tuning && tuning->splits > 0) want = scratch ? tuning->splits : 1;  // a tuned split count, if the scratch holds it
         if (want > 1 && scratch_bytes >= (size_t)want * batch * M * N * 4 && ((uintptr_t)scratch & 15) == 0) {
             const int total_kb = p.kb_per_split;
@@ -894,8 +933,13 @@ void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
             launch_overlapped(gemm_tcgen05, dim3((unsigned)grid), dim3(kThreads), kSmemBytes, s, 0, map_a, map_b, p);
         }
         if (p.splits > 1) {
-            long long groups = ((long long)batch * M * N + 3) / 4;
-            launch_overlapped(splitk_reduce, dim3((unsigned)std::min<long long>((groups + 255) / 256, sms * 8)), dim3(256), 0, s, 0, p.partial, p);
+            const size_t quad = d.dtype == LB_F32 ? 16 : 8;  // bytes of four elements
+            const bool vec = N % 4 == 0 && p.ldd % 4 == 0 && p.d_batch_stride % 4 == 0 && (uintptr_t)p.d % quad == 0 &&
+                             (epilogue < EPI_ADD || (p.ld_aux % 4 == 0 && p.aux_batch_stride % 4 == 0 && (uintptr_t)p.aux % 8 == 0));
+            const long long items = (long long)batch * M * N / (vec ? 4 : 1);
+            const dim3 blocks((unsigned)std::min<long long>((items + 255) / 256, sms * 8));
+            if (vec) launch_overlapped(splitk_reduce<true>, blocks, dim3(256), 0, s, 0, (const float*)p.partial, p);
+            else launch_overlapped(splitk_reduce<false>, blocks, dim3(256), 0, s, 0, (const float*)p.partial, p);
         }
         return;
     }

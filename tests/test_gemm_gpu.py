@@ -277,3 +277,34 @@ def test_narrow_tiles_against_float64(cuda, case, majors, dtype):
         assert ((out.double() - ref).abs() <= 2 * ulp * torch.maximum(ref.abs(), want.abs()) + 4 * k**0.5 * 2.0**-24 * top).all(), epilogue
         assert torch.equal(out, again)
     device_status()
+
+
+# (M, N, K) whose K is cut: whole and ragged columns of a partial tile's 32, N that no group of four divides, rows past a tile; `ld`: rows
+# of the result further apart than N, where its groups of four are not aligned
+@pytest.mark.parametrize("shape", [(300, 520, 8192), (257, 40, 16384), (130, 33, 8192), (300, 264, 8200)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("epilogue", [None, "add"])
+@pytest.mark.parametrize("pad", [0, 2])
+def test_split_products_at_edges(cuda, shape, dtype, epilogue, pad):
+    """Against float64: 16-bit products are exact in float32, so only the order of K additions differs (K * 2^-24 of the sum of magnitudes
+    at the very worst, its root in practice: 64 * 2^-24 allowed), and the result's own rounding, twice with an epilogue."""
+    m, n, k = shape
+    if epilogue and dtype == "float32":
+        return  # built for 16-bit results
+    gen = torch.Generator(device=cuda).manual_seed(n)
+    td = getattr(torch, dtype)
+    a = torch.randn(m, k, generator=gen, device=cuda).bfloat16()
+    b = torch.randn(n, k, generator=gen, device=cuda).bfloat16().t()
+    aux = torch.randn(m, n + pad, generator=gen, device=cuda).to(td)[:, :n] if epilogue else None
+    out = torch.full((m, n + pad), 7.0, dtype=td, device=cuda)
+    scratch = torch.empty(max(gemm_scratch_bytes(m, n, k), 1 << 20), dtype=torch.uint8, device=cuda)
+    gemm(a, b, out[:, :n], epilogue=epilogue, aux=aux, scratch=scratch, kernel="tcgen05")
+    want, size = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+    tol = 64 * 2.0**-24 * size
+    if dtype == "bfloat16":
+        tol = tol + 2.0**-8 * want.abs()
+        if epilogue:
+            want = want + aux.double()
+            tol = tol + 2.0**-8 * want.abs() + 2.0**-16 * size
+    assert ((out[:, :n].double() - want).abs() <= tol).all()
+    assert (out[:, n:] == 7.0).all()
