@@ -311,8 +311,8 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
 #pragma unroll
             for (int u = 0; u < COLS / 32; u++) {
                 const long long cc = min(c + 32 * u, (long long)p.Sq - 1);
-                next_lse[u] = __ldg(p.lse + at + cc);
-                next_delta[u] = __ldg(p.delta + at + cc);
+                next_lse[u] = p.lse[at + cc];
+                next_delta[u] = p.delta[at + cc];
             }
         };
         if (DKDV && n_iter > 0) fetch_stats(0);
@@ -507,7 +507,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
 __global__ void __launch_bounds__(256) attention_delta(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                                                         float* __restrict__ delta, int S, int N, int D, int n_shift, long long o_sb,
                                                         long long o_ss, long long o_sn, long long g_sb, long long g_ss, long long g_sn) {
-    grid_wait();
+    grid_wait(o, d_o);
     const int lanes = D >> 3;  // 8 (D = 64) or 16 (D = 128)
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned row = t / (unsigned)lanes;  // (s, n) of this batch entry; lanes is a power of two

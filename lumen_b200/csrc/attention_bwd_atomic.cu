@@ -289,8 +289,8 @@ attention_bwd_atomic_kernel(const __grid_constant__ CUtensorMap map_k, const __g
 #pragma unroll
             for (int u = 0; u < 2; u++) {
                 const long long cc = min(cj + lane + 32 * u, (long long)p.Sq - 1);
-                nl[u] = __ldg(p.lse + at + cc);  // scaled when they are staged: a use here would wait for the load
-                nd[u] = __ldg(p.delta + at + cc);
+                nl[u] = p.lse[at + cc];  // scaled when they are staged: a use here would wait for the load
+                nd[u] = p.delta[at + cc];
             }
         };
         if (n_iter > 0) load_stats(0);
@@ -437,7 +437,7 @@ attention_bwd_atomic_kernel(const __grid_constant__ CUtensorMap map_k, const __g
 // dq[b, s, n, :] = bf16(acc[b, s, n, :]): 8 values (32 bytes in, 16 out) per thread; the accumulator is dense, dq a view.
 __global__ void __launch_bounds__(256) attention_dq_round(const float* __restrict__ acc, uint16_t* __restrict__ dq, long long rows, int N,
                                                            long long sb_rows, long long q_sb, long long q_ss, long long q_sn) {
-    grid_wait();
+    grid_wait(acc);
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long r = t >> 3;  // (b, s, n) row of 64 values
     const int part = (int)(t & 7);

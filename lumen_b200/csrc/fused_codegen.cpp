@@ -51,12 +51,19 @@ __device__ __forceinline__ double fmin_nan(double a, double b) { return (a != a 
 // are literal negations 0 - x comes out as the extremum over x and -x together (a stand-alone kernel shows it with
 // `neg.s32` in inline assembly as well, so it happens after PTX); a subtraction from a register does not.
 #define RT_ZERO blockIdx.z
-// The thread's index, once the kernels before this one in the stream have completed: this kernel may have been made resident
-// before that. Every address is computed from it, so no load can be moved in front of the wait.
+// Waits for the kernels before this one in the stream, which this one may have become resident before: the thread's index, and then
+// the pointers through which the kernel reads, as values that come out of the wait. Every load's address is computed from one of
+// those pointers, so none can be moved in front of the wait - also not the loads of read-only memory (__ldg), which a compiler may
+// move across a memory clobber, where neither the thread nor the block is part of the address (a scalar, a row's own operand).
 __device__ __forceinline__ u32 grid_wait() {
     u32 tid = threadIdx.x;
     asm volatile("griddepcontrol.wait;" : "+r"(tid) : : "memory");
     return tid;
+}
+template <class T> __device__ __forceinline__ T* behind_wait(T* p, u32 tid) {
+    size_t at = __cvta_generic_to_global(p);
+    asm volatile("" : "+l"(at) : "r"(tid));
+    return (T*)__cvta_global_to_generic(at);  // known to lead to global memory
 }
 template <class T> __device__ __forceinline__ T imax(T a, T b) { return a > b ? a : b; }
 template <class T> __device__ __forceinline__ T imin(T a, T b) { return a < b ? a : b; }
@@ -1182,8 +1189,16 @@ class Generator {
         return out;
     }
 
-    static std::string wait_for_grid(int threads) {
-        return format("    const u32 tid = grid_wait();\n    __builtin_assume(tid < %du);\n", threads);
+    // `reads`: the kernel's parameters that it reads through
+    static std::string wait_for_grid(int threads, const std::vector<std::string>& reads) {
+        std::string s = "    const u32 tid = grid_wait();\n";
+        for (const std::string& p : reads) s += "    " + p + " = behind_wait(" + p + ", tid);\n";
+        return s + format("    __builtin_assume(tid < %du);\n", threads);
+    }
+    std::vector<std::string> input_names() const {
+        std::vector<std::string> names;
+        for (size_t i = 0; i < g_.inputs.size(); i++) names.push_back(format("in%d", (int)i));
+        return names;
     }
 
     FusedKernel emit() {
@@ -1234,7 +1249,7 @@ class Generator {
             s << "struct MultiTable { int n; u32 blocks; long long rows[" << k.multi_max_groups << "]; void* ptr[" << k.multi_max_groups << "]["
               << n_ptrs << "]; u32 first[" << k.multi_max_groups << "]; };\n";
             s << "extern \"C\" __global__ void __launch_bounds__(" << T_ * RPB_ << ") fused_kernel(const MultiTable table) {\n";
-            s << wait_for_grid(T_ * RPB_);
+            s << wait_for_grid(T_ * RPB_, {});
             // The groups' row blocks form ONE sequence (`first`: each group's first place in it) dealt to the CTAs, of which there
             // are as many as blocks while they fit the GPU: a CTA looks its group up once and walks on. What bounds a small model's
             // update is latency: with every CTA visiting every group, as many CTAs as the largest group has blocks and a 64-bit
@@ -1244,7 +1259,7 @@ class Generator {
             s << "  for (u32 block = blockIdx.x; block < table.blocks; block += gridDim.x) {\n";
             s << "    while (group + 1 < table.n && table.first[group + 1] <= block) group++;\n";
             s << "    const long long group_rows = table.rows[group];\n";
-            for (size_t i = 0; i < g_.inputs.size(); i++) s << "    const void*" << restrict_kw << " in" << i << " = table.ptr[group][" << i << "];\n";
+            for (size_t i = 0; i < g_.inputs.size(); i++) s << "    const void*" << restrict_kw << " in" << i << " = behind_wait(table.ptr[group][" << i << "], tid);\n";
             for (size_t i = 0; i < g_.outputs.size(); i++)
                 s << "    void*" << restrict_kw << " out" << i << " = table.ptr[group][" << g_.inputs.size() + i << "];\n";
         } else {
@@ -1258,7 +1273,7 @@ class Generator {
             s << ") {\n";
         }
         s << "    __shared__ unsigned long long red_smem[2][32];\n    int red_turn = 0;\n";
-        if (!multi_) s << wait_for_grid(T_ * RPB_);
+        if (!multi_) s << wait_for_grid(T_ * RPB_, input_names());
         s << "    const int lane_in_row = tid % TPR, row_in_block = tid / TPR;\n";
         if (!multi_) s << "    const idx_t row_blocks = (idx_t)((NROWS + RPB - 1) / RPB);\n";
         s << indent(kernel_cache_, 4);
@@ -1482,7 +1497,7 @@ class Generator {
         for (size_t i = 0; i < g_.outputs.size(); i++) sig += format("void* __restrict__ out%d, ", (int)i);
         sig += "void* __restrict__ scratch";
         s << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") fused_kernel(" << sig << ") {\n";
-        s << wait_for_grid(threads);
+        s << wait_for_grid(threads, input_names());
         s << "    const int col_lane = tid & " << col_lanes - 1 << ", row_lane = tid >> 5;\n";
         s << "    const idx_t c0 = ((idx_t)blockIdx.x * " << col_lanes << " + col_lane) * VEC;\n    const bool in_range = c0 < NCOLS;\n";
         s << "    __shared__ __align__(16) char shared[" << row_lanes * col_lanes << " * VEC * " << widest << "];\n";
@@ -1580,7 +1595,9 @@ class Generator {
         }
         s << "#undef VEC\n#define VEC " << VEC_ << "\n";
         s << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") fused_finalize(" << sig << ") {\n";
-        s << wait_for_grid(threads);
+        std::vector<std::string> reads = input_names();
+        reads.push_back("scratch");
+        s << wait_for_grid(threads, reads);
         s << "    const int col_lane = tid & " << col_lanes - 1 << ", row_lane = tid / " << col_lanes << ";\n";
         s << "    const idx_t c0 = ((idx_t)blockIdx.x * " << col_lanes << " + col_lane) * VEC;\n    const bool in_range = c0 < NCOLS;\n";
         s << "    __shared__ __align__(16) char shared[" << shared_bytes << "];\n";

@@ -662,7 +662,7 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 // 1192 x 1736 x 6944 46.9 -> 40.4, 704 x 1504 x 8000 32.7 -> 23.0, 1024 x 1024 x 8192 30.5 -> 24.0.
 template <bool VEC>
 __global__ void __launch_bounds__(256) splitk_reduce(const float* __restrict__ partial, GemmArgs p) {
-    grid_wait();
+    grid_wait(partial);
     constexpr int W = VEC ? 4 : 1;
     const long long per = (long long)p.batch * p.M * p.N;
     for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * W; i < per; i += (long long)gridDim.x * blockDim.x * W) {

@@ -7,6 +7,11 @@
 // once the kernels before it have completed and their writes are visible. As each of them did the same, that holds for the
 // whole stream before it, and what is launched in the ordinary way afterwards is ordered as ever.
 //
+// The wait is a barrier to ordinary loads and stores, but a compiler takes what is read through `const __restrict__` parameters
+// (and __ldg) for constant while the kernel runs and may move such a load across it. `grid_wait` is therefore given those
+// parameters and makes them values that come out of the wait, so that the addresses computed from them do too. Pointers in a
+// struct of arguments are read by ordinary loads.
+//
 // No kernel lets the next one come earlier (griddepcontrol.launch_dependents): its blocks would be dealt to the SMs that this
 // one leaves idle, several to one SM, and stay there. Measured (us a pass, ordinary launches -> these -> these with the next
 // kernel let in from the start): MLP forward and backward of 200 tokens x 1024 x 4096, bfloat16, eight kernels 81.6 -> 64.5 ->
@@ -16,7 +21,17 @@
 
 namespace lb {
 
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class P>
+__device__ __forceinline__ void behind_wait(P& pointer) {
+    size_t at = __cvta_generic_to_global(pointer);
+    asm volatile("" : "+l"(at)::"memory");
+    pointer = (P)__cvta_global_to_generic(at);  // known to lead to global memory
+}
+template <class... P>
+__device__ __forceinline__ void grid_wait(P&... read) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    (behind_wait(read), ...);
+}
 
 // kernel<<<grid, block, smem, stream>>>(args...), overlapping the kernel before it; `cluster`: CTAs per cluster along x where
 // the kernel does not fix them itself.

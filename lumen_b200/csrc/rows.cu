@@ -43,7 +43,7 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
 template <class T, class I, bool VEC>
 __global__ void scatter_add_rows_kernel(float* __restrict__ acc, const I* __restrict__ ids, const T* __restrict__ updates,
                                         long long tokens, long long rows, int width) {
-    grid_wait();
+    grid_wait(ids, updates);
     const long long t = blockIdx.x;
     if (t >= tokens) return;
     long long r = (long long)ids[t];
@@ -62,7 +62,7 @@ __global__ void scatter_add_rows_kernel(float* __restrict__ acc, const I* __rest
 // out = x + sum(updates): one rounding of the float32 sum into the operand dtype
 template <class T, bool VEC>
 __global__ void add_convert_kernel(T* __restrict__ out, const T* __restrict__ x, const float* __restrict__ acc, long long n, int has_x) {
-    grid_wait();
+    grid_wait(x, acc);
     const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * (VEC ? 4 : 1);
     if (i >= n) return;
     if constexpr (VEC) {
@@ -86,14 +86,14 @@ __device__ __forceinline__ int clamped_row(const I* ids, long long t, long long 
 
 template <class I>
 __global__ void scatter_count_kernel(int* __restrict__ counts, const I* __restrict__ ids, long long tokens, long long rows) {
-    grid_wait();
+    grid_wait(ids);
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < tokens) atomicAdd(counts + clamped_row(ids, t, rows), 1);  // integer atomics: the counts do not depend on order
 }
 
 // starts[r] = sum of counts[0 .. r), starts[rows] = tokens; one block walks the rows in chunks of its size.
 __global__ void scatter_starts_kernel(int* __restrict__ starts, const int* __restrict__ counts, long long rows) {
-    grid_wait();
+    grid_wait(counts);
     __shared__ int warp_sums[32];
     __shared__ int carry;
     if (threadIdx.x == 0) carry = 0;
@@ -132,7 +132,7 @@ __global__ void scatter_starts_kernel(int* __restrict__ starts, const int* __res
 template <class I>
 __global__ void scatter_place_kernel(int* __restrict__ order, int* __restrict__ cursor, const int* __restrict__ starts,
                                      const I* __restrict__ ids, long long tokens, long long rows) {
-    grid_wait();
+    grid_wait(starts, ids);
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= tokens) return;
     const int r = clamped_row(ids, t, rows);
@@ -148,7 +148,7 @@ template <class T>
 __global__ void scatter_rows_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __restrict__ updates, const int* __restrict__ starts,
                                     const int* __restrict__ order, int* __restrict__ sorted, int width, int has_x) {
     __shared__ int picks[kSortSmem];
-    grid_wait();
+    grid_wait(x, updates, starts, order);
     const long long r = blockIdx.x;
     const int begin = starts[r], n = starts[r + 1] - begin;
     const int* list = picks;
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(256) scatter_rows_few_kernel(T* __restrict__ o
                                                                int tokens, long long rows, int width, int has_x) {
     constexpr int kWarps = 8, kBallots = kFewUpdates / (32 * kWarps);
     __shared__ int picks[kFewUpdates], counts[kWarps];
-    grid_wait();
+    grid_wait(x, updates, ids);
     const int r = (int)blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int stretch = (tokens + 32 * kWarps - 1) / (32 * kWarps) * 32, first = warp * stretch;
     unsigned hits[kBallots];
@@ -361,7 +361,7 @@ attention_simt_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, cons
                           float* __restrict__ lse, AttnShape s) {
     extern __shared__ __align__(16) uint8_t raw[];
     AttnSmem<DU> sm(raw, s.tile_rows);
-    grid_wait();
+    grid_wait(q, k, v);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int i0, n, b;
     block_rows(s.Sq, s.N, i0, n, b);
@@ -412,7 +412,7 @@ attention_simt_dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const
                          const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dq, AttnShape s) {
     extern __shared__ __align__(16) uint8_t raw[];
     AttnSmem<DU> sm(raw, s.tile_rows);
-    grid_wait();
+    grid_wait(q, k, v, g, lse, delta);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int i0, n, b;
     block_rows(s.Sq, s.N, i0, n, b);
@@ -456,7 +456,7 @@ attention_simt_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, con
                            const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dk, T* __restrict__ dv, AttnShape s) {
     extern __shared__ __align__(16) uint8_t raw[];
     AttnSmem<DU> sm(raw, s.tile_rows);
-    grid_wait();
+    grid_wait(q, k, v, g, lse, delta);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int k0, nk, b;
     block_rows(s.Sk, s.Nkv, k0, nk, b);
@@ -502,7 +502,7 @@ attention_simt_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, con
 
 template <class T>
 __global__ void attention_delta_simt(const T* __restrict__ o, const T* __restrict__ g, float* __restrict__ delta, AttnShape s) {
-    grid_wait();
+    grid_wait(o, g);
     const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= (long long)s.B * s.N * s.Sq) return;
@@ -521,7 +521,7 @@ __global__ void attention_delta_simt(const T* __restrict__ o, const T* __restric
 template <class T>
 __global__ void __launch_bounds__(256) transpose_kernel(const T* __restrict__ in, T* __restrict__ out, int rows, int cols) {
     __shared__ T tile[32][33];
-    grid_wait();
+    grid_wait(in);
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
 #pragma unroll
@@ -697,7 +697,7 @@ struct CopyDims {
 
 template <class T>
 __global__ void strided_copy_kernel(const T* __restrict__ src, T* __restrict__ dst, CopyDims d, long long total) {
-    grid_wait();
+    grid_wait(src);
     const long long step = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += step) {
         long long rest = i, from = 0, to = 0;
@@ -717,7 +717,7 @@ template <class T>
 __global__ void __launch_bounds__(256) tiled_copy_kernel(const T* __restrict__ src, T* __restrict__ dst, CopyDims d, int a, int b, long long tiles_a,
                                                          long long tiles_b) {
     __shared__ T tile[32][33];
-    grid_wait();
+    grid_wait(src);
     long long block = blockIdx.x;
     const long long ta = block % tiles_a;
     block /= tiles_a;

@@ -1,13 +1,15 @@
 """Kernels that become resident before the one before them has completed read nothing early: dependent kernels of every family, queued
 without a wait between them, on inputs that change from pass to pass, give the bits that they give one at a time."""
 
+import ctypes
+
 import pytest
 import torch
 
 import lumen_b200
+from lumen_b200 import _lib, prims, tracer
 from lumen_b200 import functional as F
-from lumen_b200 import prims
-from lumen_b200.runtime import attention_backward, attention_forward, gemm, scatter_add_rows
+from lumen_b200.runtime import Fusion, attention_backward, attention_forward, current_stream, desc, gemm, scatter_add_rows
 
 pytestmark = pytest.mark.gpu
 
@@ -71,6 +73,88 @@ def test_queued_passes_equal_passes_one_at_a_time(cuda, rows, width):
         return got
 
     want = run(torch.cuda.synchronize)
+    for _ in range(5):
+        for g, w in zip(run(lambda: None), want):
+            assert all(torch.equal(a, b) for a, b in zip(g, w))
+
+
+@pytest.fixture(scope="module")
+def fusions():
+    """Kernels of a block a row whose operands are a scalar and a value of each row (their addresses depend on the block at most),
+    row and column totals in one, and the horizontal form."""
+    rows, cols = 600, 4096
+    shape = ("float32", (rows, cols))
+    body = tracer.trace(lambda p, g: p - g * 0.5, ("float32", (2, 64)), ("float32", (2, 64)))
+    return {
+        "totals": Fusion(tracer.trace(lambda x: (prims.reduce_sum(x, (1,), "float32").reshape(rows, 1), prims.reduce_sum(x, (0,), "float32")), shape)),
+        "one": Fusion(tracer.trace(lambda c: prims.reduce_sum(c, (0,), "float32").reshape(1, 1), ("float32", (cols,)))),
+        "scale": Fusion(tracer.trace(lambda x, r, o: x * r + o, shape, ("float32", (rows, 1)), ("float32", (1, 1)))),
+        "multi": Fusion("option multi\n" + body.to_text()),
+        # through transpose_kernel, tiled_copy_kernel and strided_copy_kernel
+        "turned": lumen_b200.compile(lambda x: prims.transpose(x, (1, 0))),
+        "swapped": lumen_b200.compile(lambda x: prims.transpose(x, (2, 1, 0))),
+        "cut": lumen_b200.compile(lambda x: prims.slice(x, (1, 1, 1), x.shape)),
+    }
+
+
+def horizontal(fusion, groups):
+    lib = _lib.lib()
+    lib.lb_fusion_launch_groups.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
+    tensors = [desc(t) for g in groups for t in g]
+    _lib.check(lib.lb_fusion_launch_groups(fusion.handle, (_lib.LbTensor * len(tensors))(*tensors), len(groups), current_stream()))
+    return [g[-1] for g in groups]
+
+
+def others(s, f, after):
+    """One pass over the families that `chain` leaves out; every call reads what the one before it wrote."""
+    out = []
+
+    def step(t):
+        after()
+        out.append(t)
+        return t
+
+    x = s["x"]
+    r, c = f["totals"](x)
+    after()
+    y = step(f["scale"](x, r, f["one"](c)[0])[0])
+    t = step(f["turned"](y).clone())
+    u = step(f["swapped"](t.view(64, 64, 600)).clone())
+    w = step(f["cut"](u).clone())  # [599, 63, 63]
+    q = (w.reshape(-1)[: 8 * 128 * 2 * 64].view(8, 128, 2, 64) * 1e-3).contiguous()
+    o, lse = attention_forward(q, q, q, causal=True)  # CUDA cores
+    step(o), step(lse)
+    for g in attention_backward(q, q, q, o, o, lse, causal=True):
+        step(g)
+    kv = o.to(torch.bfloat16)
+    d, lse = attention_forward(kv[:, :1].repeat(1, 1, 4, 1), kv, kv)  # decode
+    step(d), step(lse)
+    table = o.reshape(-1, 64)  # 2048 rows
+    for g in horizontal(f["multi"], [[table[:n], table[n : 2 * n], torch.empty(n, 64, device=x.device)] for n in (1, 7, 300, 1024)]):
+        step(g)
+    step(scatter_add_rows(table, s["ids"], table.flip(0).contiguous(), deterministic=False))  # every row once: one order of additions
+    step(scatter_add_rows(table, s["many"], table.repeat(3, 1)))  # more updates than one kernel takes
+    return out
+
+
+def test_queued_passes_of_the_other_families(cuda, fusions):
+    gen = torch.Generator(device=cuda).manual_seed(3)
+    s = {"x": torch.empty(600, 4096, device=cuda), "ids": torch.randperm(2048, generator=gen, device=cuda),
+         "many": torch.randint(0, 2048, (3 * 2048,), generator=gen, device=cuda)}
+    inputs = [torch.randn(600, 4096, generator=gen, device=cuda) for _ in range(6)]
+
+    def run(after):
+        got = []
+        for x in inputs:
+            s["x"].copy_(x)
+            after()
+            got.append(others(s, fusions, after))
+        torch.cuda.synchronize()
+        return got
+
+    want = run(torch.cuda.synchronize)
+    x, y = inputs[0], want[0][0]
+    assert torch.allclose(y.double(), x.double() * x.double().sum(1, keepdim=True) + x.double().sum(), rtol=1e-4, atol=1e-1)
     for _ in range(5):
         for g, w in zip(run(lambda: None), want):
             assert all(torch.equal(a, b) for a, b in zip(g, w))
