@@ -7,7 +7,10 @@ liblumen_b200's."""
 from __future__ import annotations
 
 import ctypes
+import math
 import sys
+import threading
+from collections import OrderedDict
 
 from lumen_b200 import _lib
 from lumen_b200.graph import Graph
@@ -99,7 +102,6 @@ class Fusion:
         self.n_outputs = _lib.lib().lb_fusion_num_outputs(handle)
         self.scratch_bytes = _lib.lib().lb_fusion_scratch_bytes(handle)
         self.body = body if isinstance(body, Graph) else None
-        self._scratch = None
 
     @property
     def source(self) -> str:
@@ -120,12 +122,9 @@ class Fusion:
             raise RuntimeError("calling a Fusion built from text needs explicit outputs: use launch_raw")
         if out is None:
             out = [_empty_like_input(inputs[0], self.body.types[v].shape, self.body.types[v].dtype) for v in self.body.outputs]
-        scratch = None
-        if self.scratch_bytes:
-            if self._scratch is None or self._scratch.numel() < self.scratch_bytes:
-                self._scratch = _empty_like_input(inputs[0], (self.scratch_bytes,), "uint8")
-            scratch = self._scratch.data_ptr()
-        self.launch_raw([desc(t) for t in (*inputs, *out)], scratch, stream)
+        # partial sums between the call's two kernels: another call must not meet them, on whatever stream, thread or device
+        scratch = _workspace(inputs[0], (self.scratch_bytes,), "uint8", stream) if self.scratch_bytes else None
+        self.launch_raw([desc(t) for t in (*inputs, *out)], scratch.data_ptr() if scratch is not None else None, stream)
         return out
 
 
@@ -139,8 +138,6 @@ def _empty_like_input(like, shape, dtype: str):
         return sys.modules["torch"].empty(shape, dtype=TORCH_DTYPES[dtype], device=like.device)
     from lumen_b200.device import ITEMSIZE, Region
 
-    import math
-
     nbytes = max(math.prod(shape) * ITEMSIZE[dtype], 1)
     for region in _scratch_region:
         try:
@@ -149,6 +146,38 @@ def _empty_like_input(like, shape, dtype: str):
             continue
     _scratch_region.append(Region(max(nbytes + 4096, 256 << 20)))
     return _scratch_region[-1].empty(shape, dtype)
+
+
+_workspaces: OrderedDict = OrderedDict()  # (device, stream) -> region, the latest used last
+_workspaces_lock = threading.Lock()
+_WORKSPACE_STREAMS = 8
+
+
+def _workspace(like, shape, dtype: str, stream):
+    """Memory of one call on `stream`, which may be dropped as soon as the call's kernels are queued: what the memory is given to next
+    is queued on the same stream. From torch's allocator with `stream` current for a torch tensor, else from a region that serves
+    this stream of the current device alone; the regions of the eight latest streams are kept (freeing one waits for its work)."""
+    handle = _stream(stream)
+    if type(like).__module__.startswith("torch"):
+        torch = sys.modules["torch"]
+        if not like.is_cuda or handle == torch.cuda.current_stream(like.device).cuda_stream:
+            return _empty_like_input(like, shape, dtype)
+        with torch.cuda.stream(torch.cuda.ExternalStream(handle, like.device) if handle else torch.cuda.default_stream(like.device)):
+            return _empty_like_input(like, shape, dtype)
+    from lumen_b200.device import ITEMSIZE, Region, current_device
+
+    key = (current_device(), handle)
+    with _workspaces_lock:
+        if key in _workspaces:
+            _workspaces.move_to_end(key)
+            try:
+                return _workspaces[key].empty(shape, dtype)
+            except _lib.LumenError:  # too small, or in use by other threads' calls: a region of its own takes its place
+                del _workspaces[key]
+        region = _workspaces[key] = Region(max(math.prod(shape) * ITEMSIZE[dtype] + 4096, 32 << 20))
+        while len(_workspaces) > _WORKSPACE_STREAMS:
+            _workspaces.popitem(last=False)
+        return region.empty(shape, dtype)
 
 
 GEMM_KERNELS = {"auto": 0, "tcgen05": 1, "simt": 2, "tcgen05_1cta": 3}

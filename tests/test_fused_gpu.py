@@ -440,3 +440,47 @@ def test_totals_of_many_slices(cuda, rows, cols, sums):
     assert torch.equal(out[0], x + x.sum(1, keepdim=True))
     for k in range(sums):
         assert torch.equal(out[1 + k], x.sum(0) * (k + 1))
+
+
+@pytest.mark.parametrize("own", [False, True])  # torch's memory, the backend's own
+def test_one_fusion_on_several_streams_and_threads(cuda, own):
+    """Column totals of different inputs at once: small integers, so every order of the additions gives the same sum."""
+    import threading
+
+    from lumen_b200 import device as D
+
+    rows, cols = 20000, 512
+    fusion = Fusion(tracer.trace(lambda a: prims.reduce_sum(a, (0,), "float32"), ("float32", (rows, cols))))
+    gen = torch.Generator(device=cuda).manual_seed(5)
+    xs = [torch.randint(-8, 9, (rows, cols), generator=gen, device=cuda).float() for _ in range(4)]
+    wants = [x.sum(0) for x in xs]
+    streams = [D.Stream() for _ in range(2)]
+    region = D.Region(256 << 20)
+    outs = [[region.empty((cols,), "float32") if own else torch.empty(cols, device=cuda) for _ in range(20)] for _ in xs]
+    if own:
+        inputs = [region.empty((rows, cols), "float32") for _ in xs]
+        for a, x in zip(inputs, xs):
+            a.copy_from_host(x.cpu().numpy())
+    else:
+        inputs = xs
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(i):  # two threads to a stream
+        try:
+            torch.cuda.set_device(cuda)
+            for out in outs[i]:
+                fusion(inputs[i], out=[out], stream=streams[i % 2].handle)
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(xs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors
+    for got, want in zip(outs, wants):
+        for out in got:
+            assert torch.equal(torch.as_tensor(out, device=cuda), want)

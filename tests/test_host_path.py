@@ -199,3 +199,23 @@ def test_threads_add_and_call_at_once():
     for th in threads:
         th.join()
     assert not failures
+
+
+def test_calls_of_a_fusion_share_no_partial_sums(monkeypatch):
+    """A call that another thread or stream makes before the first one's second kernel is queued gets memory of its own."""
+    from lumen_b200 import prims, runtime, tracer
+
+    f = runtime.Fusion(tracer.trace(lambda x: prims.reduce_sum(x, (0,), "float32"), ("float32", (512, 100))))
+    assert f.scratch_bytes > 0
+    x, seen = torch.zeros(512, 100), []
+
+    def launch(self, descs, scratch=None, stream=None):
+        seen.append(scratch)
+        if len(seen) == 1:
+            f(x)
+
+    monkeypatch.setattr(runtime, "require_cuda", lambda: None)
+    monkeypatch.setattr(runtime, "desc", lambda t: t)
+    monkeypatch.setattr(runtime.Fusion, "launch_raw", launch)
+    f(x)
+    assert len(seen) == 2 and seen[0] != seen[1]
