@@ -157,16 +157,15 @@ def _workspace(like, shape, dtype: str, stream):
     """Memory of one call on `stream`, which may be dropped as soon as the call's kernels are queued: what the memory is given to next
     is queued on the same stream. From torch's allocator with `stream` current for a torch tensor, else from a region that serves
     this stream of the current device alone; the regions of the eight latest streams are kept (freeing one waits for its work)."""
-    handle = _stream(stream)
     if type(like).__module__.startswith("torch"):
-        torch = sys.modules["torch"]
-        if not like.is_cuda or handle == torch.cuda.current_stream(like.device).cuda_stream:
+        if stream is None and _current[0] == 0:  # torch's current stream
             return _empty_like_input(like, shape, dtype)
+        torch, handle = sys.modules["torch"], _stream(stream)
         with torch.cuda.stream(torch.cuda.ExternalStream(handle, like.device) if handle else torch.cuda.default_stream(like.device)):
             return _empty_like_input(like, shape, dtype)
     from lumen_b200.device import ITEMSIZE, Region, current_device
 
-    key = (current_device(), handle)
+    key = (current_device(), _stream(stream))
     with _workspaces_lock:
         if key in _workspaces:
             _workspaces.move_to_end(key)
@@ -228,8 +227,8 @@ def attention_backward(q, k, v, o, d_o, lse, scale=None, causal=False, delta=Non
     sk = k.shape[1]
     dq, dk, dv = (_empty_like_input(t, tuple(t.shape), dtype_name(t.dtype)) for t in (q, k, v))
     if delta is None:
-        delta = _empty_like_input(q, (b, n, sq), "float32")
-    dq_accum = None if deterministic else _empty_like_input(q, (b, sq, n, h), "float32")
+        delta = _workspace(q, (b, n, sq), "float32", stream)
+    dq_accum = None if deterministic else _workspace(q, (b, sq, n, h), "float32", stream)
     _lib.host().attention_bwd(float(scale if scale is not None else h**-0.5), bool(causal), sk - sq, q, k, v, o, d_o, lse, delta,
                               dq_accum, dq, dk, dv, _stream(stream))
     return dq, dk, dv
@@ -252,9 +251,10 @@ def scatter_add_rows(x, ids, updates, deterministic=True, stream=None):
     lib.lb_scatter_add_rows.argtypes = [T, T, T, T, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int, ctypes.c_void_p]
     rows, width = x.shape
     nbytes = lib.lb_scatter_add_scratch_bytes(rows, width, ids.numel(), int(deterministic))
-    scratch = _empty_like_input(x, (max(nbytes, 4),), "uint8")
+    scratch = _workspace(x, (max(nbytes, 4),), "uint8", stream)
     out = _empty_like_input(x, tuple(x.shape), dtype_name(x.dtype))
-    dx, di, du, do = desc(x), desc(ids), desc(updates.reshape(-1, width)), desc(out)
+    updates = updates.reshape(-1, width)  # held until the kernels are queued: a view, or a copy of one with other strides
+    dx, di, du, do = desc(x), desc(ids), desc(updates), desc(out)
     _lib.check(lib.lb_scatter_add_rows(ctypes.byref(dx), ctypes.byref(di), ctypes.byref(du), ctypes.byref(do), scratch.data_ptr(),
                                        nbytes, int(deterministic), current_stream() if stream is None else stream))
     return out

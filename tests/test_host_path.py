@@ -219,3 +219,44 @@ def test_calls_of_a_fusion_share_no_partial_sums(monkeypatch):
     monkeypatch.setattr(runtime.Fusion, "launch_raw", launch)
     f(x)
     assert len(seen) == 2 and seen[0] != seen[1]
+
+
+def test_temporaries_of_a_call_come_from_its_stream(monkeypatch):
+    """The backward's delta and dQ sums and the scatter-add's sums are dropped when the call returns, with its kernels in flight: they
+    are memory of the stream that the call names."""
+    from lumen_b200 import runtime
+
+    asked = []
+
+    class Nothing:
+        def __getattr__(self, name):
+            return lambda *a: 0
+
+    def workspace(like, shape, dtype, stream):
+        asked.append((tuple(shape), dtype, stream))
+        return torch.empty(shape, dtype=runtime.TORCH_DTYPES[dtype])
+
+    monkeypatch.setattr(runtime, "require_cuda", lambda: None)
+    monkeypatch.setattr(runtime, "_workspace", workspace)
+    monkeypatch.setattr(runtime._lib, "host", Nothing)
+    q = torch.zeros(2, 8, 4, 64, dtype=torch.bfloat16)
+    lse = torch.zeros(2, 4, 8)
+    runtime.attention_backward(q, q, q, q, q, lse, stream=7)
+    assert asked == [((2, 4, 8), "float32", 7)]
+    runtime.attention_backward(q, q, q, q, q, lse, stream=7, deterministic=False)
+    assert asked[1:] == [((2, 4, 8), "float32", 7), ((2, 8, 4, 64), "float32", 7)]
+    monkeypatch.setattr(runtime, "desc", lambda t: runtime._lib.strided(0, "float32", t.shape, t.stride()))
+
+    class Answer:
+        def __init__(self, value):
+            self.value = value
+
+        def __call__(self, *a):
+            return self.value
+
+    class Library:
+        lb_scatter_add_scratch_bytes, lb_scatter_add_rows = Answer(640), Answer(0)
+
+    monkeypatch.setattr(runtime._lib, "lib", Library)
+    runtime.scatter_add_rows(torch.zeros(4, 40), torch.zeros(3, dtype=torch.int64), torch.zeros(3, 40), stream=9)
+    assert asked[3:] == [((640,), "uint8", 9)]
