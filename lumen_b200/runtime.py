@@ -128,24 +128,26 @@ class Fusion:
         return out
 
 
-_scratch_region = []
+_regions: dict = {}  # device -> its regions, as they were reserved
 
 
 def _empty_like_input(like, shape, dtype: str):
     """A new dense device tensor of `shape`/`dtype` in the framework `like` comes from: torch for a torch tensor (the
-    harness's convenience), else the backend's own region (grown in 256 MiB reservations)."""
+    harness's convenience), else the backend's own regions of the current device (grown in 256 MiB reservations)."""
     if type(like).__module__.startswith("torch"):
         return sys.modules["torch"].empty(shape, dtype=TORCH_DTYPES[dtype], device=like.device)
-    from lumen_b200.device import ITEMSIZE, Region
+    from lumen_b200.device import ITEMSIZE, Region, current_device
 
     nbytes = max(math.prod(shape) * ITEMSIZE[dtype], 1)
-    for region in _scratch_region:
+    regions = _regions.setdefault(current_device(), [])
+    for region in regions:
         try:
             return region.empty(shape, dtype)
         except _lib.LumenError:
             continue
-    _scratch_region.append(Region(max(nbytes + 4096, 256 << 20)))
-    return _scratch_region[-1].empty(shape, dtype)
+    region = Region(max(nbytes + 4096, 256 << 20))
+    regions.append(region)
+    return region.empty(shape, dtype)
 
 
 _workspaces: OrderedDict = OrderedDict()  # (device, stream) -> region, the latest used last

@@ -260,3 +260,24 @@ def test_temporaries_of_a_call_come_from_its_stream(monkeypatch):
     monkeypatch.setattr(runtime._lib, "lib", Library)
     runtime.scatter_add_rows(torch.zeros(4, 40), torch.zeros(3, dtype=torch.int64), torch.zeros(3, 40), stream=9)
     assert asked[3:] == [((640,), "uint8", 9)]
+
+
+def test_results_come_from_a_region_of_the_current_device(monkeypatch):
+    from lumen_b200 import device, runtime
+
+    on = [0]
+
+    class Region:
+        def __init__(self, nbytes):
+            self.device = on[0]
+
+        def empty(self, shape, dtype):
+            return self
+
+    monkeypatch.setattr(device, "Region", Region)
+    monkeypatch.setattr(device, "current_device", lambda: on[0])
+    for name in ("_regions", "_workspaces"):
+        monkeypatch.setattr(runtime, name, type(getattr(runtime, name, {}))(), raising=False)
+    for on[0] in (0, 1, 0):
+        assert runtime._empty_like_input(Array((4,)), (4,), "float32").device == on[0]
+        assert runtime._workspace(Array((4,)), (4,), "float32", 5).device == on[0]
