@@ -545,26 +545,28 @@ int lb_plan_num_collectives(const lb_plan* plan) { return plan ? plan->n_collect
 int lb_plan_kernel_launches(const lb_plan* plan) {
     if (!plan) return -1;
     int n = 0;
-    for (const lb::Step& s : plan->steps) {
-        switch (s.kind) {
-            case lb::FUSION: n += s.fusion && s.fusion->kernel.empty ? 0 : (s.scratch >= 0 ? 2 : 1); break;  // partial sums + finalize
-            case lb::MULTI: n += s.fusion && s.fusion->kernel.multi_max_groups > 0 ? (s.aux + s.fusion->kernel.multi_max_groups - 1) / s.fusion->kernel.multi_max_groups : 1; break;
-            case lb::GEMM: n += s.scratch >= 0 ? 2 : 1; break;  // split-K partial tiles + reduction
-            case lb::ATTN_FWD: n += 1; break;
-            case lb::ATTN_BWD: n += 3; break;  // delta, then dK/dV and dQ - or the single kernel and the rounding of dQ
-            case lb::SCATTER_ADD: {
-                const lb_tensor &ids = plan->views.at((size_t)s.args.at(1)).t, &out = plan->views.at((size_t)s.args.at(3)).t;
-                long long tokens = 1;
-                for (int d = 0; d < ids.rank; d++) tokens *= ids.shape[d];
-                n += lb::scatter_add_launches(out.shape[0], tokens, s.epilogue != 0);
-                break;
+    const int rc = lb::guarded([&] {  // a step may name a tensor that the plan does not define
+        for (const lb::Step& s : plan->steps) {
+            switch (s.kind) {
+                case lb::FUSION: n += s.fusion && s.fusion->kernel.empty ? 0 : (s.scratch >= 0 ? 2 : 1); break;  // partial sums + finalize
+                case lb::MULTI: n += s.fusion && s.fusion->kernel.multi_max_groups > 0 ? (s.aux + s.fusion->kernel.multi_max_groups - 1) / s.fusion->kernel.multi_max_groups : 1; break;
+                case lb::GEMM: n += s.scratch >= 0 ? 2 : 1; break;  // split-K partial tiles + reduction
+                case lb::ATTN_FWD: n += 1; break;
+                case lb::ATTN_BWD: n += 3; break;  // delta, then dK/dV and dQ - or the single kernel and the rounding of dQ
+                case lb::SCATTER_ADD: {
+                    const lb_tensor &ids = plan->views.at((size_t)s.args.at(1)).t, &out = plan->views.at((size_t)s.args.at(3)).t;
+                    long long tokens = 1;
+                    for (int d = 0; d < ids.rank; d++) tokens *= ids.shape[d];
+                    n += lb::scatter_add_launches(out.shape[0], tokens, s.epilogue != 0);
+                    break;
+                }
+                case lb::TRANSPOSE: n += 1; break;
+                case lb::COPY: n += lb::copy_form(plan->views.at((size_t)s.args.at(0)).t, plan->views.at((size_t)s.args.at(1)).t) == 2 ? 1 : 0; break;
+                default: break;  // block and 2-d copies, fills, collectives and waits launch no kernel of this library
             }
-            case lb::TRANSPOSE: n += 1; break;
-            case lb::COPY: n += lb::copy_form(plan->views.at((size_t)s.args.at(0)).t, plan->views.at((size_t)s.args.at(1)).t) == 2 ? 1 : 0; break;
-            default: break;  // block and 2-d copies, fills, collectives and waits launch no kernel of this library
         }
-    }
-    return n;
+    });
+    return rc == LB_OK ? n : -1;
 }
 
 size_t lb_scatter_add_scratch_bytes(int64_t rows, int64_t width, int64_t updates, int deterministic) {

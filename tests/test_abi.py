@@ -99,3 +99,14 @@ def test_the_library_builds_without_python_headers():
     assert "liblumen_b200.so.tmp" in commands("false") and "host_py.cpp" not in commands("false")
     assert f"_host{sysconfig.get_config_var('EXT_SUFFIX')}" in commands(sys.executable)
     assert _lib.host().__file__.endswith(f"_host{sysconfig.get_config_var('EXT_SUFFIX')}")
+
+
+@pytest.mark.parametrize("step", ["s scatter_add x 0 7 1 2 3 1", "s copy x 0 9"])
+def test_counting_the_launches_of_a_plan_with_undefined_tensors_is_an_error(step):
+    lib = _lib.lib()
+    lib.lb_plan_create.argtypes = [ctypes.c_char_p, ctypes.POINTER(ctypes.c_void_p)]
+    lib.lb_plan_kernel_launches.argtypes = lib.lb_plan_destroy.argtypes = [ctypes.c_void_p]
+    handle = ctypes.c_void_p()
+    _lib.check(lib.lb_plan_create(f"plan 1 1 256\nt 0 float32 i0 0 2 4 8 8 1\n{step}\nend\n".encode(), ctypes.byref(handle)))
+    assert lib.lb_plan_kernel_launches(handle) == -1
+    lib.lb_plan_destroy(handle)
