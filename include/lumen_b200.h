@@ -132,6 +132,9 @@ size_t lb_gemm_scratch_bytes(int64_t m, int64_t n, int64_t k, int64_t batch);
 /* The same for a product step of a plan, which runs on the kernel lb_gemm picks by itself: 0 also where that one cuts K inside
  * a thread-block cluster. */
 size_t lb_gemm_step_scratch_bytes(int64_t m, int64_t n, int64_t k);
+/* The same for these operands, of whose `ptr` only the alignment counts: 0 also where the product runs on the CUDA cores
+ * (float32 operands; 16-bit ones whose rows are not 16-byte aligned), which never cut K. */
+size_t lb_gemm_operands_scratch_bytes(const lb_tensor* a, const lb_tensor* b);
 int lb_gemm(const lb_tensor* a, const lb_tensor* b, const lb_gemm_out* out, const lb_gemm_cfg* cfg /* nullable */,
             void* stream);
 

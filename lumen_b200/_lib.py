@@ -105,6 +105,8 @@ def lib():
         _lib.lb_gemm_step_scratch_bytes.argtypes = [ctypes.c_int64] * 3
         _lib.lb_gemm_step_scratch_bytes.restype = ctypes.c_size_t
         T = ctypes.POINTER(LbTensor)
+        _lib.lb_gemm_operands_scratch_bytes.argtypes = [T, T]
+        _lib.lb_gemm_operands_scratch_bytes.restype = ctypes.c_size_t
         _lib.lb_attention_fwd.argtypes = [ctypes.POINTER(LbAttnDesc), T, T, T, T, T, ctypes.c_void_p]
         _lib.lb_attention_fwd_kernel.argtypes = [ctypes.POINTER(LbAttnDesc), T, T, T, ctypes.POINTER(ctypes.c_int32)]
         _lib.lb_attention_bwd.argtypes = [ctypes.POINTER(LbAttnDesc)] + [T] * 10 + [ctypes.c_void_p]

@@ -411,7 +411,7 @@ class Lowering:
         b = rhs if rc == 0 else View(rhs.buffer, rhs.offset, rhs.dtype, rhs.shape[::-1], rhs.strides[::-1])
         b = self.k_major_copy(b, a.shape[0])
         out = self.fresh(out_value)
-        nbytes = gemm_scratch_bytes(a.shape[0], b.shape[1], a.shape[1])
+        nbytes = gemm_scratch_bytes(a, b)
         scratch = View(self.new_buffer(nbytes), 0, "uint8", (nbytes,), (1,)) if nbytes else None
         code = int(relu)
         aux = self.views[aux_value] if aux_value is not None else None
@@ -851,11 +851,14 @@ def attention_params(body: G.Graph):
     return scale, causal, offset
 
 
-def gemm_scratch_bytes(m: int, n: int, k: int) -> int:
-    """Split-K scratch a plan's [m, k] x [k, n] product step takes (0 when it does not split, or splits inside a cluster)."""
+def gemm_scratch_bytes(a: View, b: View) -> int:
+    """Split-K scratch a plan's product step of these operands takes (0 when it does not split, or splits inside a cluster)."""
+    import ctypes
+
     from lumen_b200 import _lib
 
-    return _lib.lib().lb_gemm_step_scratch_bytes(m, n, k)
+    operands = [_lib.strided(v.offset, v.dtype, v.shape, v.strides) for v in (a, b)]
+    return _lib.lib().lb_gemm_operands_scratch_bytes(*map(ctypes.byref, operands))
 
 
 _SCRATCH_CACHE: dict[str, int] = {}

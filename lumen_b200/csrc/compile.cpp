@@ -20,8 +20,6 @@
 #include "fused.h"
 #include "graph_text.h"
 
-extern "C" size_t lb_gemm_step_scratch_bytes(int64_t m, int64_t n, int64_t k);
-
 namespace lb {
 namespace {
 
@@ -42,6 +40,15 @@ struct View {
         return true;
     }
 };
+
+// The view as operands are described to the library, with its offset for an address (buffers and arguments start aligned).
+lb_tensor descriptor(const View& v) {
+    lb_tensor t{};
+    t.ptr = (void*)v.offset, t.dtype = v.dtype, t.rank = (int)v.shape.size();
+    std::copy(v.shape.begin(), v.shape.end(), t.shape);
+    std::copy(v.strides.begin(), v.strides.end(), t.stride);
+    return t;
+}
 
 std::vector<int64_t> dense_strides(const std::vector<int64_t>& shape) {
     std::vector<int64_t> s(shape.size(), 1);
@@ -657,7 +664,8 @@ struct Lowering {
         }
         View d = fresh(t.dtype, t.shape, result);
         views[result] = d;
-        const size_t sb = lb_gemm_step_scratch_bytes(a.shape[0], b.shape[1], a.shape[1]);
+        const lb_tensor operands[2] = {descriptor(a), descriptor(b)};
+        const size_t sb = lb_gemm_operands_scratch_bytes(&operands[0], &operands[1]);
         std::ostringstream s;
         s << "s gemm " << label << " " << tid(a) << " " << tid(b) << " " << tid(d) << " " << epilogue << " " << (sb ? tid(scratch(sb)) : -1) << " " << (aux ? tid(*aux) : -1);
         push_step(s.str() + "\n");

@@ -789,12 +789,6 @@ int gemm_small_splits(long long M, long long N, long long K, long long batch, in
     return total_kb <= 128 * s ? s : 0;  // longer ranges: not measured, left to the split-K kernels
 }
 
-// Scratch a plan's product step takes: none where the narrow tiles run.
-extern "C" size_t lb_gemm_step_scratch_bytes(int64_t m, int64_t n, int64_t k) {
-    const size_t bytes = gemm_scratch_bytes(m, n, k, 1);
-    return gemm_small_splits(m, n, k, 1, sm_count_hint(), bytes > 0) ? 0 : bytes;
-}
-
 // CTA pairs of gemm_tcgen05_pair that can be resident on `dev` at once (asked of the runtime once per device).
 static int resident_pairs(const DeviceInfo& dev) {
     static std::mutex mutex;
@@ -817,6 +811,54 @@ int gemm_model_splits(long long M, long long N, long long K, long long batch) { 
 size_t gemm_scratch_bytes(long long M, long long N, long long K, long long batch) {
     const int s = gemm_splits(M, N, K, batch, sm_count_hint());
     return s > 1 ? (size_t)s * batch * M * N * 4 : 0;
+}
+
+// Scratch a plan's product step takes: none where the narrow tiles run.
+static size_t gemm_step_scratch_bytes(long long M, long long N, long long K, long long batch) {
+    const size_t bytes = gemm_scratch_bytes(M, N, K, batch);
+    return gemm_small_splits(M, N, K, batch, sm_count_hint(), bytes > 0) ? 0 : bytes;
+}
+
+// Where a product of 16-bit operands runs: on narrow tiles with `ranges` CTAs a cluster, or (ranges 0) on large tiles with K cut into
+// `splits` ranges of `kb_per_split` 64-wide blocks.
+struct GemmRoute {
+    int ranges, splits, kb_per_split;
+};
+static GemmRoute gemm_route(long long M, long long N, long long K, long long batch, int sms, int kernel_choice, size_t scratch_bytes, const GemmTuning* tuning) {
+    const int split = scratch_bytes ? gemm_splits(M, N, K, batch, sms) : 1;
+    auto holds = [&](int s) { return s > 1 && scratch_bytes >= (size_t)s * batch * M * N * 4; };
+    // no kernel asked for and no split or raster tuned: narrow tiles where they fit
+    if (kernel_choice == 0 && !(tuning && (tuning->splits > 0 || tuning->group_m > 0)))
+        if (const int ranges = gemm_small_splits(M, N, K, batch, sms, holds(split))) return {ranges, 1, 0};
+    const int want = tuning && tuning->splits > 0 ? tuning->splits : split;  // a tuned split count, if the scratch holds it
+    const int total_kb = (int)((K + BK - 1) / BK), kb = holds(want) ? (total_kb + want - 1) / want : total_kb;
+    return {0, (total_kb + kb - 1) / kb, kb};
+}
+
+// Whether two operands can be read by the tensor-core kernels, and which of their axes is contiguous.
+static bool tensor_core_operands(const View3& a, const View3& b, bool& a_cols, bool& b_cols) {
+    auto major = [](const View3& v, bool& cols_contig) {
+        if (v.sc == 1 || v.cols == 1) { cols_contig = true; return true; }
+        if (v.sr == 1 || v.rows == 1) { cols_contig = false; return true; }
+        return false;
+    };
+    // TMA: 16-byte aligned base, strides multiples of 16 bytes
+    auto aligned = [](const View3& v, bool cols_contig) {
+        long long inner = cols_contig ? v.cols : v.rows, outer = cols_contig ? v.rows : v.cols;
+        long long ld = outer == 1 ? inner : (cols_contig ? v.sr : v.sc);
+        return ((uintptr_t)v.ptr & 15) == 0 && ld % 8 == 0 && ld >= inner && (v.batch == 1 || v.sb % 8 == 0);
+    };
+    return (a.dtype == LB_BF16 || a.dtype == LB_F16) && a.cols > 0 && major(a, a_cols) && major(b, b_cols) && aligned(a, a_cols) && aligned(b, b_cols) &&
+           a.rows <= INT32_MAX && b.cols <= INT32_MAX && a.cols <= INT32_MAX;
+}
+
+// Kernels that gemm launches.
+int gemm_launches(const lb_tensor& a_t, const lb_tensor& b_t, size_t scratch_bytes, int kernel_choice, const GemmTuning* tuning) {
+    const View3 a = view3(a_t, "a"), b = view3(b_t, "b");
+    if (a.rows == 0 || b.cols == 0 || a.batch == 0) return 0;
+    bool a_cols, b_cols;
+    if (kernel_choice == 2 || !tensor_core_operands(a, b, a_cols, b_cols)) return 1;
+    return gemm_route(a.rows, b.cols, a.cols, a.batch, sm_count_hint(), kernel_choice, scratch_bytes, tuning).splits > 1 ? 2 : 1;
 }
 
 void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int epilogue, int kernel_choice, void* stream,
@@ -844,22 +886,8 @@ void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
     driver();
     cudaStream_t s = (cudaStream_t)stream;
 
-    auto major = [](const View3& v, bool& cols_contig) {
-        if (v.sc == 1 || v.cols == 1) { cols_contig = true; return true; }
-        if (v.sr == 1 || v.rows == 1) { cols_contig = false; return true; }
-        return false;
-    };
     bool a_cols, b_cols;
-    bool tc_ok = (a.dtype == LB_BF16 || a.dtype == LB_F16) && K > 0 && major(a, a_cols) && major(b, b_cols) && kernel_choice != 2;
-    if (tc_ok) {
-        // TMA: 16-byte aligned base, strides multiples of 16 bytes
-        auto aligned = [](const View3& v, bool cols_contig) {
-            long long inner = cols_contig ? v.cols : v.rows, outer = cols_contig ? v.rows : v.cols;
-            long long ld = outer == 1 ? inner : (cols_contig ? v.sr : v.sc);
-            return ((uintptr_t)v.ptr & 15) == 0 && ld % 8 == 0 && ld >= inner && (v.batch == 1 || v.sb % 8 == 0);
-        };
-        tc_ok = aligned(a, a_cols) && aligned(b, b_cols) && M <= INT32_MAX && N <= INT32_MAX && K <= INT32_MAX;
-    }
+    const bool tc_ok = kernel_choice != 2 && tensor_core_operands(a, b, a_cols, b_cols);
     if (kernel_choice == 1 && !tc_ok) fail(LB_ERR_UNSUPPORTED, "gemm: the tcgen05 kernels need bfloat16 or float16 operands with a unit stride and 16-byte aligned rows");
 
     if (tc_ok) {
@@ -890,15 +918,13 @@ void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
         bt.rows = b.cols, bt.cols = b.rows, bt.sr = b.sc, bt.sc = b.sr;
         CUtensorMap map_b = p.b_mn_major ? make_map(bt, false, 64, BK) : make_map(bt, true, BK, pairs ? BN / 2 : BN);
         const DeviceInfo& dev = device_info();
-        // no kernel asked for and no split or raster tuned: narrow tiles where they fit (gemm_small_splits)
-        const int split = scratch ? gemm_splits(M, N, K, batch, dev.sms) : 1;
-        const bool large_split = split > 1 && scratch_bytes >= (size_t)split * batch * M * N * 4 && ((uintptr_t)scratch & 15) == 0;
-        if (const int ranges = kernel_choice == 0 && !(tuning && (tuning->splits > 0 || tuning->group_m > 0)) ? gemm_small_splits(M, N, K, batch, dev.sms, large_split) : 0) {
+        const GemmRoute route = gemm_route(M, N, K, batch, dev.sms, kernel_choice, ((uintptr_t)scratch & 15) == 0 && scratch ? scratch_bytes : 0, tuning);
+        if (route.ranges) {
             SmallGemmArgs q{};
             q.M = p.M, q.N = p.N, q.K = p.K, q.a_mn_major = p.a_mn_major, q.b_mn_major = p.b_mn_major, q.in_bf16 = p.in_bf16;
             q.d = p.d, q.d_bf16 = p.d_bf16, q.d_f16 = p.d_f16, q.ldd = p.ldd, q.d_batch_stride = p.d_batch_stride;
             q.epilogue = p.epilogue, q.aux = p.aux, q.ld_aux = p.ld_aux, q.aux_batch_stride = p.aux_batch_stride, q.status = p.status;
-            q.splits = ranges;
+            q.splits = route.ranges;
             gemm_small(map_a, p.b_mn_major ? map_b : make_map(bt, true, BK, 64), q, (int)batch, dev.sms, s);
             return;
         }
@@ -909,16 +935,8 @@ void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
         const int max_pairs = resident_pairs(dev);
         long long tiles = (long long)p.tiles_m * p.tiles_n * batch;
         const int sms = dev.sms;
-        p.splits = 1;
-        p.kb_per_split = (int)((K + BK - 1) / BK);
+        p.splits = route.splits, p.kb_per_split = route.kb_per_split;
         p.partial = (float*)scratch;
-        int want = split;
-        if (tuning && tuning->splits > 0) want = scratch ? tuning->splits : 1;  // a tuned split count, if the scratch holds it
-        if (want > 1 && scratch_bytes >= (size_t)want * batch * M * N * 4 && ((uintptr_t)scratch & 15) == 0) {
-            const int total_kb = p.kb_per_split;
-            p.kb_per_split = (total_kb + want - 1) / want;
-            p.splits = (total_kb + p.kb_per_split - 1) / p.kb_per_split;
-        }
         if (tiles * p.splits > INT32_MAX) fail(LB_ERR_UNSUPPORTED, "gemm: too many output tiles for one launch");
         p.by_tiles.set((uint32_t)tiles), p.by_batch.set((uint32_t)(p.tiles_m * p.tiles_n));
         p.group_m = std::min(p.group_m, p.tiles_m);
@@ -974,6 +992,19 @@ int lb_gemm(const lb_tensor* a, const lb_tensor* b, const lb_gemm_out* out, cons
 }
 
 size_t lb_gemm_scratch_bytes(int64_t m, int64_t n, int64_t k, int64_t batch) { return lb::gemm_scratch_bytes(m, n, k, batch); }
+
+size_t lb_gemm_step_scratch_bytes(int64_t m, int64_t n, int64_t k) { return lb::gemm_step_scratch_bytes(m, n, k, 1); }
+
+size_t lb_gemm_operands_scratch_bytes(const lb_tensor* a, const lb_tensor* b) {
+    size_t bytes = 0;
+    lb::guarded([&] {
+        if (!a || !b) lb::fail(LB_ERR_INVALID, "lb_gemm_operands_scratch_bytes: null argument");
+        const lb::View3 x = lb::view3(*a, "a"), y = lb::view3(*b, "b");
+        bool a_cols, b_cols;
+        if (lb::tensor_core_operands(x, y, a_cols, b_cols)) bytes = lb::gemm_step_scratch_bytes(x.rows, y.cols, x.cols, x.batch);
+    });
+    return bytes;
+}
 
 int lb_device_status(void) {
     int status = 0;

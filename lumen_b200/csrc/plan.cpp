@@ -30,6 +30,7 @@ struct lb_comm;
 namespace lb {
 void gemm(const lb_tensor& a, const lb_tensor& b, const lb_tensor& d, int epilogue, int kernel_choice, void* stream,
           void* scratch, size_t scratch_bytes, const lb_tensor* aux, const GemmTuning* tuning);
+int gemm_launches(const lb_tensor& a, const lb_tensor& b, size_t scratch_bytes, int kernel_choice, const GemmTuning* tuning);
 int gemm_model_splits(long long M, long long N, long long K, long long batch);
 void fill_noise(void* ptr, size_t bytes, void* stream);
 void transpose_2d(const lb_tensor& in, const lb_tensor& out, void* stream);
@@ -550,7 +551,17 @@ int lb_plan_kernel_launches(const lb_plan* plan) {
             switch (s.kind) {
                 case lb::FUSION: n += s.fusion && s.fusion->kernel.empty ? 0 : (s.scratch >= 0 ? 2 : 1); break;  // partial sums + finalize
                 case lb::MULTI: n += s.fusion && s.fusion->kernel.multi_max_groups > 0 ? (s.aux + s.fusion->kernel.multi_max_groups - 1) / s.fusion->kernel.multi_max_groups : 1; break;
-                case lb::GEMM: n += s.scratch >= 0 ? 2 : 1; break;  // split-K partial tiles + reduction
+                case lb::GEMM: {  // split-K partial tiles + reduction, or one kernel
+                    auto operand = [&](int i) {
+                        const lb::View& v = plan->views.at((size_t)s.args.at(i));
+                        lb_tensor t = v.t;
+                        t.ptr = (void*)v.offset;
+                        return t;
+                    };
+                    const size_t bytes = s.scratch >= 0 ? lb::view_bytes(plan->views.at((size_t)s.scratch).t) : 0;
+                    n += lb::gemm_launches(operand(0), operand(1), bytes, s.tuned_kernel, &s.tuning);
+                    break;
+                }
                 case lb::ATTN_FWD: n += 1; break;
                 case lb::ATTN_BWD: n += 3; break;  // delta, then dK/dV and dQ - or the single kernel and the rounding of dQ
                 case lb::SCATTER_ADD: {

@@ -3,6 +3,7 @@
 compiles every fused kernel and builds the plan - steps, places, workspace size - or rejects the module with a message
 naming the primitive it has no kernel for (lumen/codegen/devices/cuda/mod.rs:140-189 does the same)."""
 
+import ctypes
 import json
 
 import pytest
@@ -215,4 +216,20 @@ def test_both_lowerings_place_the_same_collectives_in_random_data_parallel_steps
         assert places([s["kind"] for s in steps]) == places(python_kinds), what
         assert [s["label"] for s in steps] == python.labels, what
         assert lib.lb_plan_workspace_bytes(handle) == python.workspace_bytes, what
+        lib.lb_plan_destroy(handle)
+
+
+@pytest.mark.parametrize("dtype, k, split", [("float32", 8192, False), ("bfloat16", 8192, True), ("bfloat16", 8191, False)])
+def test_products_on_cuda_cores_take_no_split_scratch(dtype, k, split):
+    """K is cut by the tensor-core kernels alone: float32 products and rows of 16 bits that are not 16-byte aligned take no memory for
+    partial tiles and count as one launch, in both lowerings."""
+    from lumen_b200.compiler import compile_graph
+
+    g = tracer.trace(lambda x, w: F.matmul(x, w, "float32", dtype), (dtype, (1024, k)), (dtype, (k, 1024)))
+    lib, native, python = _bind(), lower_native(fuse(clean(g))), ctypes.c_void_p()
+    compiled = compile_graph(g)
+    _lib.check(lib.lb_plan_create(compiled.text.encode(), ctypes.byref(python)))
+    assert lib.lb_plan_workspace_bytes(native) == compiled.workspace_bytes and (compiled.workspace_bytes > 0) == split
+    for handle in (native, python):
+        assert lib.lb_plan_kernel_launches(handle) == 1 + split
         lib.lb_plan_destroy(handle)
