@@ -308,3 +308,30 @@ def test_split_products_at_edges(cuda, shape, dtype, epilogue, pad):
             tol = tol + 2.0**-8 * want.abs() + 2.0**-16 * size
     assert ((out[:, :n].double() - want).abs() <= tol).all()
     assert (out[:, n:] == 7.0).all()
+
+
+@pytest.mark.parametrize("shape, large", [((768, 768, 8192), True), ((300, 1000, 8200), True), ((768, 768, 8128), False), ((384, 1536, 8192), False),
+                                          ((128, 8192, 4096), False)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_scratch_decides_between_narrow_and_cut_large_tiles(cuda, shape, large, dtype):
+    """Both sides of the line, by the bits of the kernel that is named: with enough scratch large tiles where the rule says so, with
+    too little or none (or where it does not) the narrow ones. All within the K-order bound of float64."""
+    m, n, k = shape
+    gen = torch.Generator(device=cuda).manual_seed(k)
+    a = torch.randn(m, k, generator=gen, device=cuda).bfloat16()
+    b = torch.randn(n, k, generator=gen, device=cuda).bfloat16().t()
+    nbytes = gemm_scratch_bytes(m, n, k)
+    assert nbytes > 0
+
+    def product(kernel, scratch_bytes):
+        out = torch.empty(m, n, dtype=getattr(torch, dtype), device=cuda)
+        return gemm(a, b, out, kernel=kernel, scratch=torch.empty(scratch_bytes, dtype=torch.uint8, device=cuda) if scratch_bytes else None)
+
+    narrow, cut = product("auto", 0), product("tcgen05", nbytes)
+    assert not torch.equal(narrow, cut)  # else the test could not tell them apart
+    assert torch.equal(product("auto", nbytes), cut if large else narrow)
+    assert torch.equal(product("auto", nbytes - 16), narrow)
+    want, size = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+    for out in (narrow, cut):  # 64 * 2^-24 of the sum of magnitudes for the order of K additions, the result's rounding
+        assert ((out.double() - want).abs() <= 64 * 2.0**-24 * size + (2.0**-8 * want.abs() if dtype == "bfloat16" else 0)).all()
+    device_status()

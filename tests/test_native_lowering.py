@@ -233,3 +233,17 @@ def test_products_on_cuda_cores_take_no_split_scratch(dtype, k, split):
     for handle in (native, python):
         assert lib.lb_plan_kernel_launches(handle) == 1 + split
         lib.lb_plan_destroy(handle)
+
+
+@pytest.mark.parametrize("m, n, k, split", [
+    (1024, 1024, 8192, True), (768, 768, 8192, True),  # 128 blocks of K for two ranges of narrow tiles: the line
+    (768, 768, 8128, False), (512, 512, 4096, False),  # shorter ranges
+    (384, 3072, 6144, False), (384, 1536, 8192, False),  # more units than pairs of SMs: 384 rows are two row tiles
+    (128, 9216, 4096, False), (16, 8192, 4096, False), (128, 4096, 12288, False),  # the one-CTA kernel
+    (128, 8192, 17000, True),  # longer ranges than the narrow tiles take
+])
+def test_long_products_that_narrow_tiles_fit_are_cut_on_large_tiles_only_where_that_is_faster(m, n, k, split):
+    lib = _bind()
+    assert (lib.lb_gemm_step_scratch_bytes(m, n, k) > 0) == split
+    if split:
+        assert lib.lb_gemm_step_scratch_bytes(m, n, k) == lib.lb_gemm_scratch_bytes(m, n, k, 1)
