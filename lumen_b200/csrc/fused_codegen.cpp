@@ -1528,7 +1528,11 @@ class Generator {
     // The second kernel of a column reduction: adds the slices' partial sums and applies the epilogue. A block takes 32
     // lanes of two columns and one (up to eight slices), eight or 32 slice lanes: few columns and slices per thread, so that the chains of loads stay
     // short (1184 slices of 1024 columns took 19 us with eight slice lanes). Many slices of few columns take 128 slice lanes, on eight
-    // column lanes: four times the blocks, and a thread's chain of loads a quarter (a residual layer norm of 8192 x 1024 with its backward, whose totals are 592 slices of 1024 columns, 36.1 -> 33.5 us).
+    // column lanes: four times the blocks, and a thread's chain of loads a quarter (a residual layer norm of 8192 x 1024 with its
+    // backward, whose totals are 592 slices of 1024 columns, 36.1 -> 33.5 us). Where the line lies, by the time of a whole kernel pair with
+    // 128 lanes over that with 32: 1184 slices of 512 columns 0.60 - 0.73, 592 of 1024 0.71 - 0.88, 296 of 2048 0.90 - 0.98, 260 of 500
+    // to 2048 0.85 - 0.94, 296 of 3072 1.00; 296 of 2049, one column a thread, 1.00 - 1.01; 148 of 6144 1.02 - 1.21. Fewer slices were
+    // measured faster too (200 of 500 to 2048 0.89 - 0.95, 128 of up to 256 0.93) down to 64 (1.01), but are left as they are.
     void emit_finalize(std::ostringstream& s, const std::string& sig, const std::vector<size_t>& offsets, const std::vector<int>& outputs, FusedKernel& k) {
         column_mode_ = true;
         VEC_ = std::min(VEC_, 2);

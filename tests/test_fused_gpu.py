@@ -424,22 +424,34 @@ def test_row_sums_of_odd_widths_are_as_exact_as_of_1024_threads(cuda, cols):
     assert rms(s) <= (1 + 3 / 8000**0.5) * rms(total[:, 0])
 
 
-# totals of 257 slices and more over few columns take 128 slice lanes: columns that are no multiple of a block's, one column, the
-# widest of them and one past, more sums than shared memory holds at once; 256 slices and fewer do not
-@pytest.mark.parametrize("rows,cols", [(300, 1), (257, 15), (256, 15), (600, 17), (5000, 1023), (700, 2047), (700, 2049), (900, 4096), (900, 4098)])
-@pytest.mark.parametrize("sums", [1, 6])
-def test_totals_of_many_slices(cuda, rows, cols, sums):
+# totals of 257 slices and more over few columns take 128 slice lanes (on eight column lanes): beside a row sum and alone, two columns a
+# thread and one, columns that are no multiple of a block's, one column, the widest of them and one past; 256 slices do not
+@pytest.mark.parametrize("rows,cols,beside,many", [
+    (5000, 1024, True, True), (5000, 64, True, True), (5000, 1022, True, True), (600, 3072, True, True), (257, 500, True, True),
+    (5000, 1023, True, True), (20000, 17, True, True), (700, 2047, True, True),
+    (256, 500, True, False), (700, 2049, True, False), (300, 4096, True, False),
+    (20000, 64, False, True), (40000, 20, False, True), (65536, 256, False, True), (65536, 1, False, True), (16448, 64, False, True),
+    (16384, 64, False, False), (40000, 300, False, False),
+])  # fmt: skip
+@pytest.mark.parametrize("sums", [1, 6])  # six: more than shared memory holds at once
+def test_totals_of_many_slices(cuda, rows, cols, beside, many, sums):
     """Small integers: every order of the additions gives the same sum."""
     x = torch.randint(-8, 9, (rows, cols), generator=torch.Generator(device=cuda).manual_seed(cols), device=cuda).float()
 
     def program(a):
-        beside = prims.reduce_sum(a, (1,), "float32").reshape(rows, 1)
-        return (a + beside, *[prims.reduce_sum(a * float(k + 1), (0,), "float32") for k in range(sums)])
+        totals = [prims.reduce_sum(a * float(k + 1), (0,), "float32") for k in range(sums - 1)] + [prims.reduce_max(a, (0,)) if sums > 1 else
+                                                                                                   prims.reduce_sum(a, (0,), "float32")]
+        return tuple(totals + ([a + prims.reduce_sum(a, (1,), "float32").reshape(rows, 1)] if beside else []))
 
-    out = Fusion(tracer.trace(program, ("float32", (rows, cols))))(x)
-    assert torch.equal(out[0], x + x.sum(1, keepdim=True))
-    for k in range(sums):
-        assert torch.equal(out[1 + k], x.sum(0) * (k + 1))
+    fusion = Fusion(tracer.trace(program, ("float32", (rows, cols))))
+    assert ("row_lane = tid / 8;" in fusion.source) == many
+    out = fusion(x)
+    for k in range(max(sums - 1, 1)):
+        assert torch.equal(out[k], x.sum(0) * (k + 1))
+    if sums > 1:
+        assert torch.equal(out[sums - 1], x.amax(0))
+    if beside:
+        assert torch.equal(out[sums], x + x.sum(1, keepdim=True))
 
 
 @pytest.mark.parametrize("own", [False, True])  # torch's memory, the backend's own
