@@ -279,35 +279,56 @@ def test_narrow_tiles_against_float64(cuda, case, majors, dtype):
     device_status()
 
 
-# (M, N, K) whose K is cut: whole and ragged columns of a partial tile's 32, N that no group of four divides, rows past a tile; `ld`: rows
-# of the result further apart than N, where its groups of four are not aligned
-@pytest.mark.parametrize("shape", [(300, 520, 8192), (257, 40, 16384), (130, 33, 8192), (300, 264, 8200)])
-@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-@pytest.mark.parametrize("epilogue", [None, "add"])
-@pytest.mark.parametrize("pad", [0, 2])
-def test_split_products_at_edges(cuda, shape, dtype, epilogue, pad):
+# (batch, M, N, K) whose K is cut: whole and ragged columns of a partial tile's 32, N that no group of four divides, rows past a tile, one
+# row tile of the one-CTA kernel, several problems; `pad`: rows of the result further apart than N, where its groups of four are not
+# aligned; `gap`: elements between the results of a batch, which no group of four divides
+@pytest.mark.parametrize("shape, kernel", [
+    ((1, 300, 520, 8192), "tcgen05"), ((1, 257, 40, 16384), "tcgen05"), ((1, 130, 33, 8192), "tcgen05"), ((1, 300, 264, 8200), "tcgen05"),
+    ((2, 300, 264, 8192), "tcgen05"), ((3, 130, 33, 8192), "tcgen05"),
+    ((1, 100, 520, 8192), "tcgen05"), ((1, 128, 33, 16384), "tcgen05"), ((2, 70, 296, 8192), "tcgen05"), ((1, 300, 520, 8192), "tcgen05_1cta"), ((2, 257, 33, 8192), "tcgen05_1cta"),
+])  # fmt: skip
+@pytest.mark.parametrize("operands, dtype, epilogue", [
+    ("bfloat16", "float32", None), ("bfloat16", "bfloat16", None), ("bfloat16", "bfloat16", "add"), ("bfloat16", "bfloat16", "mask_positive"),
+    ("float16", "float32", "relu"), ("float16", "float16", None), ("float16", "float16", "add"),
+])  # fmt: skip
+@pytest.mark.parametrize("pad, gap", [(0, 0), (2, 0), (0, 6)])
+def test_split_products_at_edges(cuda, shape, kernel, operands, dtype, epilogue, pad, gap):
     """Against float64: 16-bit products are exact in float32, so only the order of K additions differs (K * 2^-24 of the sum of magnitudes
     at the very worst, its root in practice: 64 * 2^-24 allowed), and the result's own rounding, twice with an epilogue."""
-    m, n, k = shape
-    if epilogue and dtype == "float32":
-        return  # built for 16-bit results
+    batch, m, n, k = shape
     gen = torch.Generator(device=cuda).manual_seed(n)
-    td = getattr(torch, dtype)
-    a = torch.randn(m, k, generator=gen, device=cuda).bfloat16()
-    b = torch.randn(n, k, generator=gen, device=cuda).bfloat16().t()
-    aux = torch.randn(m, n + pad, generator=gen, device=cuda).to(td)[:, :n] if epilogue else None
-    out = torch.full((m, n + pad), 7.0, dtype=td, device=cuda)
-    scratch = torch.empty(max(gemm_scratch_bytes(m, n, k), 1 << 20), dtype=torch.uint8, device=cuda)
-    gemm(a, b, out[:, :n], epilogue=epilogue, aux=aux, scratch=scratch, kernel="tcgen05")
+    od, td = getattr(torch, operands), getattr(torch, dtype)
+
+    def rows_apart(fill):  # [batch, m, n] in rows of n + pad, problems m * (n + pad) + gap apart
+        memory = torch.full((batch, m * (n + pad) + gap), 7.0, dtype=td, device=cuda)
+        view = memory[:, : m * (n + pad)].view(batch, m, n + pad)[:, :, :n]
+        if fill is not None:
+            view.copy_(fill)
+        return memory, view
+
+    a = torch.randn(batch, m, k, generator=gen, device=cuda).to(od)
+    b = torch.randn(batch, n, k, generator=gen, device=cuda).to(od).transpose(1, 2)
+    aux = rows_apart(torch.randn(batch, m, n, generator=gen, device=cuda))[1] if epilogue in ("add", "mask_positive") else None
+    memory, out = rows_apart(None)
+    nbytes = gemm_scratch_bytes(m, n, k, batch)
+    assert nbytes > 0
+    scratch = torch.full((nbytes,), 255, dtype=torch.uint8, device=cuda)  # NaN: every partial sum that is read has been written
+    one = (lambda t: t) if batch > 1 else (lambda t: None if t is None else t[0])
+    gemm(one(a), one(b), one(out), epilogue=epilogue, aux=one(aux), scratch=scratch, kernel=kernel)
     want, size = a.double() @ b.double(), a.double().abs() @ b.double().abs()
-    tol = 64 * 2.0**-24 * size
-    if dtype == "bfloat16":
-        tol = tol + 2.0**-8 * want.abs()
-        if epilogue:
-            want = want + aux.double()
-            tol = tol + 2.0**-8 * want.abs() + 2.0**-16 * size
-    assert ((out[:, :n].double() - want).abs() <= tol).all()
-    assert (out[:, n:] == 7.0).all()
+    tol, half = 64 * 2.0**-24 * size, {"float32": 0.0, "bfloat16": 2.0**-8, "float16": 2.0**-11}[dtype]
+    tol = tol + half * want.abs()
+    if epilogue == "relu":
+        want = want.clamp(min=0)
+    elif epilogue == "add":
+        want = want + aux.double()
+        tol = tol + half * want.abs() + half * half * size
+    elif epilogue == "mask_positive":
+        want = torch.where(aux > 0, want, 0.0)
+    assert ((out.double() - want).abs() <= tol).all()
+    out.fill_(7.0)
+    assert (memory == 7.0).all()  # nothing was written beside the result
+    device_status()
 
 
 @pytest.mark.parametrize("shape, large", [((768, 768, 8192), True), ((300, 1000, 8200), True), ((768, 768, 8128), False), ((384, 1536, 8192), False),
