@@ -97,11 +97,11 @@ __global__ void __launch_bounds__(TM / RM * (TN / RN)) gemm_simt_kernel(const T*
     typedef typename SimtVec<RN>::type VecB;
     const int bz = blockIdx.z, m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
     const int tx = threadIdx.x % (TN / RN), ty = threadIdx.x / (TN / RN);
-    grid_wait(a, b);
     const T* ab = a + (long long)bz * p.a_sb;
     const T* bb = b + (long long)bz * p.b_sb;
     const bool a_k = p.a_sk == 1, b_k = p.b_sn != 1;  // fetch along whichever axis is contiguous
     const bool a_whole = p.a_vec && m0 + TM <= p.M, b_whole = p.b_vec && n0 + TN <= p.N;
+    grid_wait(ab, bb);
     float acc[RM][RN] = {};
     SliceA fa;
     SliceB fb;

@@ -9,8 +9,8 @@
 //
 // The wait is a barrier to ordinary loads and stores, but a compiler takes what is read through `const __restrict__` parameters
 // (and __ldg) for constant while the kernel runs and may move such a load across it. `grid_wait` is therefore given those
-// parameters and makes them values that come out of the wait, so that the addresses computed from them do too. Pointers in a
-// struct of arguments are read by ordinary loads.
+// parameters (or what was computed from them) and makes them values that come out of the wait, so that the addresses computed from
+// them do too. Pointers in a struct of arguments are read by ordinary loads.
 //
 // No kernel lets the next one come earlier (griddepcontrol.launch_dependents): its blocks would be dealt to the SMs that this
 // one leaves idle, several to one SM, and stay there. Measured (us a pass, ordinary launches -> these -> these with the next

@@ -33,12 +33,16 @@ def faults(name, params, body):
     before, found = re.sub(r"\[[^\]]*\]\s*\([^()]*\)\s*\{[^{}]*\}", "", body[: wait.start()]), []  # without one-line lambdas
     if before.count("{") != before.count("}") or re.search(r"\breturn\b", before) or re.search(r"\b(if|for|while)\b[^;{}]*$", before):
         found.append(f"{name}: the wait is not reached by every thread")
+    given = [x.strip() for x in wait.group(1).split(",")]
+    for stands_for, pointer in re.findall(r"const \w+\* (\w+) = (\w+) \+ [^;]*;", before):  # an address, and not a load through it
+        if stands_for in given and not re.search(rf"\b{pointer}\b", body[wait.end() :]):
+            before = re.sub(rf"const \w+\* {stands_for} = [^;]*;", "", before)
+            given.append(pointer)
     pointers = re.findall(r"\*\s*(?:__restrict__\s*)?(\w+)\s*(?:,|$)", params)
     found += [f"{name}: {p} is used in front of the wait" for p in pointers if re.search(rf"\b{p}\b", before)]
     if re.search(r"\b__ldg\(|\bp\.\w+\[|ld\.global", before):
         found.append(f"{name}: a load in front of the wait")
     constant = re.findall(r"const \w+\s*\* __restrict__ (\w+)", params)
-    given = [x.strip() for x in wait.group(1).split(",")]
     found += [f"{name}: {p} does not come out of the wait" for p in constant if p not in given]
     found += [f"{name}: __ldg of {p}" for p in re.findall(r"__ldg\((?:\([^()]*\)\(?)?(\w+)", body) if p not in given]
     return found
