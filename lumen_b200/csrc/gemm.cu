@@ -776,27 +776,32 @@ int gemm_splits(long long M, long long N, long long K, long long batch, int sms)
 // tiles -> these), bfloat16: 64^3 8.2 -> 6.2, 512^3 13.5 -> 8.5, 200 x 4096 K 1024 16.4 -> 11.5, 200 x 1024 K 4096 24.6 -> 12.3
 // (4 ranges), 1000^3 18.5 -> 12.3, 128 x 8192 K 8192 49 -> 35, 1024 x 1024 K 8192 35 -> 28 (39 with one range); beyond the line
 // 4096 x 1024 K 200 12.3 -> 16.4, 700 x 4096 K 1024 16.4 -> 20.5, 2048^3 22.6 -> 32.7.
-// Where large tiles cut K (`large_split`, large_split_pays), ranges that would be 64 blocks and longer with one CTA to an SM go there,
-// since a narrow tile fetches twice the bytes per product: 1024 x 1024 (us, these -> large) K 16384 43.7 -> 32.7, 8192 29.0 -> 23.5, 4096
-// 22.1 -> 17.9, 768 x 768 x 8192 20.8 -> 16.8, 768 x 1024 x 16384 41.6 -> 26.7; but 32 blocks: 512 x 512 x 8192 14.6 -> 15.7,
-// 1024 x 1024 x 2048 13.0 -> 17.1.
-int gemm_small_splits(long long M, long long N, long long K, long long batch, int sms, bool large_split) {
+// Where scratch lets large tiles cut K into `large_split` ranges, ranges that would be 64 blocks and longer with one CTA to an SM may go
+// there, since a narrow tile fetches twice the bytes per product: 1024 x 1024 (us, these -> large) K 16384 43.7 -> 32.7, 8192 29.0 -> 23.5,
+// 4096 22.1 -> 17.9, 768 x 768 x 8192 20.8 -> 16.8, 768 x 1024 x 16384 41.6 -> 26.7; but 32 blocks: 512 x 512 x 8192 14.6 -> 15.7,
+// 1024 x 1024 x 2048 13.0 -> 17.1. They do where the large tiles are CTA pairs' and on the GPU all at once (170 shapes of 136 to 2100
+// rows, 300 to 4400 columns and K of 4096 to 17000, operands in the L2 or not: 0.41 - 0.87 of the time), and else where an SM would walk
+// 130 blocks of narrow tiles and two and a quarter times those of large ones (47 shapes: 0.53 - 1.01; 90 shapes drawn after both lines were set: 0.4 - 0.93). What is left to narrow tiles by
+// this line (142 shapes) takes 0.62 to 1.22 times as long on large ones, a quarter of it longer: 384 x 3072 x 6144 (two row tiles, two
+// waves) 22.2 -> 26.3, 384 x 1536 x 8192 18.4 -> 21.6, on the one-CTA kernel 128 x 9216 x 4096 23.2 -> 27.9, 16 x 9216 x 4096 16.4 -> 19.3.
+int gemm_small_splits(long long M, long long N, long long K, long long batch, int sms, int large_split) {
     const long long tiles = (M + 127) / 128 * ((N + 63) / 64) * batch, total_kb = (K + BK - 1) / BK;
     if (tiles > sms) return 0;
     int s = 1;
     while (s < 8 && tiles * 2 * s <= sms && total_kb >= 4 * s) s *= 2;
-    if (large_split && total_kb >= 64 * s) return 0;
+    const bool long_ranges = total_kb >= 64 * s;
     if (s < 8 && total_kb > 64 * s && tiles * s <= sms) s *= 2;
-    return total_kb <= 128 * s ? s : 0;  // longer ranges: not measured, left to the split-K kernels
-}
-
-// Whether a product that narrow tiles fit may go to large ones with K cut into `split` ranges instead: where these are CTA pairs' tiles
-// (more than 128 rows) and all of them are on the GPU at once. Over 100 such shapes of 192 to 2048 rows, 512 to 4096 columns and K of
-// 4096 to 16384, operands in the L2 or not, the times of narrow tiles fall to 0.49 - 0.87, over 70 drawn ragged ones to 0.41 - 0.82. With more units than pairs of SMs (384 rows
-// are two row tiles: 384 x 3072 x 6144 22.2 -> 26.3, 384 x 1536 x 8192 18.4 -> 21.6) or on the one-CTA kernel (128 x 9216 x 4096 23.2 ->
-// 27.9, 16 x 9216 x 4096 16.4 -> 19.3, 128 x 4096 x 12288 27.2 -> 29.3) they rise for a quarter of the shapes, by up to 1.22.
-static bool large_split_pays(long long M, long long N, long long batch, int split, int sms) {
-    return split > 1 && M > BM && (M + 2 * BM - 1) / (2 * BM) * ((N + BN - 1) / BN) * batch * split <= sms / 2;
+    if (total_kb > 128 * s) return 0;  // longer ranges: not measured, left to the split-K kernels
+    if (large_split > 1 && long_ranges) {
+        const bool pairs = M > BM;
+        const int at_once = pairs ? sms / 2 : sms;
+        const long long units = (M + (pairs ? 2 * BM : BM) - 1) / (pairs ? 2 * BM : BM) * ((N + BN - 1) / BN) * batch * large_split;
+        if (pairs && units <= at_once) return 0;
+        const long long narrow_kb = (tiles * s + sms - 1) / sms * ((total_kb + s - 1) / s);
+        const long long large_kb = (units + at_once - 1) / at_once * ((total_kb + large_split - 1) / large_split);
+        if (narrow_kb >= 130 && 4 * narrow_kb >= 9 * large_kb) return 0;
+    }
+    return s;
 }
 
 // CTA pairs of gemm_tcgen05_pair that can be resident on `dev` at once (asked of the runtime once per device).
@@ -826,7 +831,7 @@ size_t gemm_scratch_bytes(long long M, long long N, long long K, long long batch
 // Scratch a plan's product step takes: none where the narrow tiles run.
 static size_t gemm_step_scratch_bytes(long long M, long long N, long long K, long long batch) {
     const int sms = sm_count_hint(), split = gemm_splits(M, N, K, batch, sms);
-    return gemm_small_splits(M, N, K, batch, sms, large_split_pays(M, N, batch, split, sms)) ? 0 : gemm_scratch_bytes(M, N, K, batch);
+    return gemm_small_splits(M, N, K, batch, sms, split) ? 0 : gemm_scratch_bytes(M, N, K, batch);
 }
 
 // Where a product of 16-bit operands runs: on narrow tiles with `ranges` CTAs a cluster, or (ranges 0) on large tiles with K cut into
@@ -839,7 +844,7 @@ static GemmRoute gemm_route(long long M, long long N, long long K, long long bat
     auto holds = [&](int s) { return s > 1 && scratch_bytes >= (size_t)s * batch * M * N * 4; };
     // no kernel asked for and no split or raster tuned: narrow tiles where they fit
     if (kernel_choice == 0 && !(tuning && (tuning->splits > 0 || tuning->group_m > 0)))
-        if (const int ranges = gemm_small_splits(M, N, K, batch, sms, holds(split) && large_split_pays(M, N, batch, split, sms))) return {ranges, 1, 0};
+        if (const int ranges = gemm_small_splits(M, N, K, batch, sms, holds(split) ? split : 1)) return {ranges, 1, 0};
     const int want = tuning && tuning->splits > 0 ? tuning->splits : split;  // a tuned split count, if the scratch holds it
     const int total_kb = (int)((K + BK - 1) / BK), kb = holds(want) ? (total_kb + want - 1) / want : total_kb;
     return {0, (total_kb + kb - 1) / kb, kb};

@@ -331,8 +331,8 @@ def test_split_products_at_edges(cuda, shape, kernel, operands, dtype, epilogue,
     device_status()
 
 
-@pytest.mark.parametrize("shape, large", [((768, 768, 8192), True), ((300, 1000, 8200), True), ((768, 768, 8128), False), ((384, 1536, 8192), False),
-                                          ((128, 8192, 4096), False)])
+@pytest.mark.parametrize("shape, large", [((768, 768, 8192), True), ((300, 1000, 8200), True), ((816, 512, 17376), True), ((70, 9216, 12288), True),
+                                          ((768, 768, 8128), False), ((384, 1536, 8192), False), ((128, 8192, 4096), False)])
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_scratch_decides_between_narrow_and_cut_large_tiles(cuda, shape, large, dtype):
     """Both sides of the line, by the bits of the kernel that is named: with enough scratch large tiles where the rule says so, with
