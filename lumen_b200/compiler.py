@@ -68,7 +68,7 @@ class CompiledPlan:
     comms: list = field(default_factory=list)  # Comm, in program order
     arena_bytes: int = 0
     labels: list = field(default_factory=list)
-    kernel_launches: int = 0  # kernels one run launches (a column reduction is 2, split-K 2, attention backward 3, scatter-add 2)
+    kernel_launches: int = 0  # kernels one run launches (a column reduction is 2, split-K 2, attention backward 3, scatter-add 1 to 4)
     buckets: list = field(default_factory=list)  # {"start", "end", "ready", "dtype", "op"} per all_reduce step, in queue order
 
 

@@ -781,9 +781,10 @@ int gemm_splits(long long M, long long N, long long K, long long batch, int sms)
 // 4096 22.1 -> 17.9, 768 x 768 x 8192 20.8 -> 16.8, 768 x 1024 x 16384 41.6 -> 26.7; but 32 blocks: 512 x 512 x 8192 14.6 -> 15.7,
 // 1024 x 1024 x 2048 13.0 -> 17.1. They do where the large tiles are CTA pairs' and on the GPU all at once (170 shapes of 136 to 2100
 // rows, 300 to 4400 columns and K of 4096 to 17000, operands in the L2 or not: 0.41 - 0.87 of the time), and else where an SM would walk
-// 130 blocks of narrow tiles and two and a quarter times those of large ones (47 shapes: 0.53 - 1.01; 90 shapes drawn after both lines were set: 0.4 - 0.93). What is left to narrow tiles by
-// this line (142 shapes) takes 0.62 to 1.22 times as long on large ones, a quarter of it longer: 384 x 3072 x 6144 (two row tiles, two
-// waves) 22.2 -> 26.3, 384 x 1536 x 8192 18.4 -> 21.6, on the one-CTA kernel 128 x 9216 x 4096 23.2 -> 27.9, 16 x 9216 x 4096 16.4 -> 19.3.
+// 130 blocks of narrow tiles and two and a quarter times those of large ones (47 shapes: 0.53 - 1.01). 90 shapes drawn after both lines
+// were set took 0.40 - 0.93. What is left to narrow tiles by them (142 shapes) takes 0.62 to 1.22 times as long on large ones, a quarter
+// of it longer: 384 x 3072 x 6144 (two row tiles, two waves) 22.2 -> 26.3, 384 x 1536 x 8192 18.4 -> 21.6, on the one-CTA kernel
+// 128 x 9216 x 4096 23.2 -> 27.9, 16 x 9216 x 4096 16.4 -> 19.3.
 int gemm_small_splits(long long M, long long N, long long K, long long batch, int sms, int large_split) {
     const long long tiles = (M + 127) / 128 * ((N + 63) / 64) * batch, total_kb = (K + BK - 1) / BK;
     if (tiles > sms) return 0;
