@@ -1540,6 +1540,7 @@ class Generator {
         const int64_t slices = k.slices * k.col_blocks;
         const bool many = slices > 256 && C_ <= 64LL * VEC_ * 32;
         const int col_lanes = many ? 8 : 32, row_lanes = many ? 128 : slices > 64 ? 32 : slices > 8 ? 8 : 1, threads = col_lanes * row_lanes;
+        const int warp_lanes = std::min(row_lanes, 32);  // lanes of a column that are added by shuffles
         Comp flat_c;
         flat_c.base = "c0", flat_c.expr = "(c0 + e)";
         flat_c.lane = flat_c.e_dep = flat_c.c_dep = true;
@@ -1567,21 +1568,37 @@ class Generator {
                 auto each = [&](const std::string& body) { return "_Pragma(\"unroll\") for (int e = 0; e < VEC; e++) { " + body + " }"; };
                 auto add = [&](const std::string& to, const std::string& x) { return to + " = " + subst(combine, to, x) + ";"; };
                 const std::string from = format("((const %s*)((const char*)scratch + %zu))[(idx_t)(s + u * %d) * NCOLS + c0 + e]", type.c_str(), offsets[k], row_lanes);
-                totals << type << " " << tot << "[VEC];\n{\n    " << type << " " << run << "[4][VEC];\n    _Pragma(\"unroll\") for (int u = 0; u < 4; u++) " << each(run + "[u][e] = " + init + ";") << "\n"
-                       << "    if (in_range) {\n        int s = row_lane;\n        #pragma unroll 2\n        for (; s + " << 3 * row_lanes << " < SLICES; s += " << 4 * row_lanes << ") {\n            " << type
-                       << " pv[4][VEC];\n            _Pragma(\"unroll\") for (int u = 0; u < 4; u++) " << each("pv[u][e] = " + from + ";") << "\n            _Pragma(\"unroll\") for (int u = 0; u < 4; u++) "
-                       << each(add(run + "[u][e]", "pv[u][e]")) << "\n        }\n        _Pragma(\"unroll\") for (int u = 0; u < 3; u++) if (s + u * " << row_lanes << " < SLICES) "
-                       << each("const " + type + " pv = " + from + "; " + add(run + "[u][e]", "pv")) << "\n    }\n    "
-                       << each(add(run + "[0][e]", run + "[1][e]") + " " + add(run + "[2][e]", run + "[3][e]") + " " + tot + "[e] = " + subst(combine, run + "[0][e]", run + "[2][e]") + ";") << "\n    "
-                       << (row_lanes == 1 ? "" : format("auto lanes = (%s(*)[%d * VEC + 1])(shared + %zu);\n    ", type.c_str(), col_lanes, (k - k0) * lane_bytes) + each("lanes[row_lane][col_lane * VEC + e] = " + tot + "[e];") + "\n")
-                       << "}\n";
-                trees << "{\n    auto lanes = (" << type << "(*)[" << col_lanes << " * VEC + 1])(shared + " << (k - k0) * lane_bytes << ");\n    " << type << "* sums = (" << type << "*)(shared + " << batch * lane_bytes + (k - k0) * sum_bytes
-                      << ");\n    const int lane = threadIdx.x % " << std::min(row_lanes, 32) << ", col = threadIdx.x / " << std::min(row_lanes, 32) << ";\n    "
-                      << (many ? format("if (col < %d) ", col_lanes) : "") << each(type + " v = lanes[lane][col * VEC + e]; " + (many ? type + " v1 = lanes[lane + 32][col * VEC + e], v2 = lanes[lane + 64][col * VEC + e]; " +
-                              add("v", "v1") + " v1 = lanes[lane + 96][col * VEC + e]; " + add("v2", "v1") + " " + add("v", "v2") + " " : "") + "_Pragma(\"unroll\") for (int m = " + std::to_string(std::min(row_lanes, 32) / 2) + "; m >= 1; m /= 2) " + add("v", "shfl_xor_any<" + type + ">(v, m)") +
-                              " if (lane == 0) sums[col * VEC + e] = v;")
-                      << "\n}\n";
-                reads << each(tot + "[e] = ((const " + type + "*)(shared + " + std::to_string(batch * lane_bytes + (k - k0) * sum_bytes) + "))[col_lane * VEC + e];") << "\n";
+                const std::string unrolled = "_Pragma(\"unroll\") for (int u = 0; u < %d; u++) ", four = format(unrolled.c_str(), 4), three = format(unrolled.c_str(), 3);
+                const std::string lanes = format("auto lanes = (%s(*)[%d * VEC + 1])(shared + %zu);\n    ", type.c_str(), col_lanes, (k - k0) * lane_bytes);
+                const size_t sums_at = batch * lane_bytes + (k - k0) * sum_bytes;
+                // a lane's slices: four at once, then the up to three that are left, then the four sums
+                totals << type << " " << tot << "[VEC];\n{\n"
+                       << "    " << type << " " << run << "[4][VEC];\n"
+                       << "    " << four << each(run + "[u][e] = " + init + ";") << "\n"
+                       << "    if (in_range) {\n"
+                       << "        int s = row_lane;\n"
+                       << "        #pragma unroll 2\n"
+                       << "        for (; s + " << 3 * row_lanes << " < SLICES; s += " << 4 * row_lanes << ") {\n"
+                       << "            " << type << " pv[4][VEC];\n"
+                       << "            " << four << each("pv[u][e] = " + from + ";") << "\n"
+                       << "            " << four << each(add(run + "[u][e]", "pv[u][e]")) << "\n"
+                       << "        }\n"
+                       << "        " << three << "if (s + u * " << row_lanes << " < SLICES) " << each("const " + type + " pv = " + from + "; " + add(run + "[u][e]", "pv")) << "\n"
+                       << "    }\n"
+                       << "    " << each(add(run + "[0][e]", run + "[1][e]") + " " + add(run + "[2][e]", run + "[3][e]") + " " + tot + "[e] = " + subst(combine, run + "[0][e]", run + "[2][e]") + ";") << "\n    ";
+                if (row_lanes > 1) totals << lanes << each("lanes[row_lane][col_lane * VEC + e] = " + tot + "[e];") << "\n";
+                totals << "}\n";
+                // the lanes of a column, which a warp takes side by side: 128 are four to a thread of the first `col_lanes` warps
+                std::string tree = type + " v = lanes[lane][col * VEC + e]; ";
+                if (many)
+                    tree += type + " v1 = lanes[lane + 32][col * VEC + e], v2 = lanes[lane + 64][col * VEC + e]; " + add("v", "v1") +
+                            " v1 = lanes[lane + 96][col * VEC + e]; " + add("v2", "v1") + " " + add("v", "v2") + " ";
+                tree += format("_Pragma(\"unroll\") for (int m = %d; m >= 1; m /= 2) ", warp_lanes / 2) + add("v", "shfl_xor_any<" + type + ">(v, m)") +
+                        " if (lane == 0) sums[col * VEC + e] = v;";
+                trees << "{\n    " << lanes << type << "* sums = (" << type << "*)(shared + " << sums_at << ");\n"
+                      << "    const int lane = threadIdx.x % " << warp_lanes << ", col = threadIdx.x / " << warp_lanes << ";\n"
+                      << "    " << (many ? format("if (col < %d) ", col_lanes) : "") << each(tree) << "\n}\n";
+                reads << each(tot + "[e] = ((const " + type + "*)(shared + " + std::to_string(sums_at) + "))[col_lane * VEC + e];") << "\n";
             }
             if (row_lanes > 1) totals << "__syncthreads();\n" << trees.str() << "__syncthreads();\n" << reads.str();
             // (the next batch writes `lanes`, which were read before the last barrier; its trees write `sums` after another one)
