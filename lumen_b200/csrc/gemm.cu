@@ -779,12 +779,12 @@ int gemm_splits(long long M, long long N, long long K, long long batch, int sms)
 // Where scratch lets large tiles cut K into `large_split` ranges, ranges that would be 64 blocks and longer with one CTA to an SM may go
 // there, since a narrow tile fetches twice the bytes per product: 1024 x 1024 (us, these -> large) K 16384 43.7 -> 32.7, 8192 29.0 -> 23.5,
 // 4096 22.1 -> 17.9, 768 x 768 x 8192 20.8 -> 16.8, 768 x 1024 x 16384 41.6 -> 26.7; but 32 blocks: 512 x 512 x 8192 14.6 -> 15.7,
-// 1024 x 1024 x 2048 13.0 -> 17.1. They do where the large tiles are CTA pairs' and on the GPU all at once (170 shapes of 136 to 2100
-// rows, 300 to 4400 columns and K of 4096 to 17000, operands in the L2 or not: 0.41 - 0.87 of the time), and else where an SM would walk
-// 130 blocks of narrow tiles and two and a quarter times those of large ones (47 shapes: 0.53 - 1.01). 90 shapes drawn after both lines
-// were set took 0.40 - 0.93. What is left to narrow tiles by them (142 shapes) takes 0.62 to 1.22 times as long on large ones, a quarter
-// of it longer: 384 x 3072 x 6144 (two row tiles, two waves) 22.2 -> 26.3, 384 x 1536 x 8192 18.4 -> 21.6, on the one-CTA kernel
-// 128 x 9216 x 4096 23.2 -> 27.9, 16 x 9216 x 4096 16.4 -> 19.3.
+// 1024 x 1024 x 2048 13.0 -> 17.1. They do where the large tiles are CTA pairs' and on the GPU all at once (235 shapes of 136 to 2900
+// rows, 128 to 4400 columns and K of 4096 to 30000, every operand major, operands in the L2 or not: 0.40 - 0.87 of the time), and else
+// where an SM would walk 130 blocks of narrow tiles, 105 where pairs' tiles cover hardly more than the result, and two and a quarter times
+// those of large ones (143 shapes of 16 rows and more: 0.53 - 1.03; 1664 x 256 x 14296 41.5 -> 27.8). What is left to narrow tiles (213
+// shapes) takes 0.56 to 1.35 times as long on large ones, a fifth of it longer: 384 x 3072 x 6144 (two row tiles, two waves) 22.2 ->
+// 26.3, 384 x 1536 x 8192 18.4 -> 21.6, on the one-CTA kernel 128 x 9216 x 4096 23.2 -> 27.9, 16 x 9216 x 4096 16.4 -> 19.3.
 int gemm_small_splits(long long M, long long N, long long K, long long batch, int sms, int large_split) {
     const long long tiles = (M + 127) / 128 * ((N + 63) / 64) * batch, total_kb = (K + BK - 1) / BK;
     if (tiles > sms) return 0;
@@ -795,12 +795,13 @@ int gemm_small_splits(long long M, long long N, long long K, long long batch, in
     if (total_kb > 128 * s) return 0;  // longer ranges: not measured, left to the split-K kernels
     if (large_split > 1 && long_ranges) {
         const bool pairs = M > BM;
-        const int at_once = pairs ? sms / 2 : sms;
-        const long long units = (M + (pairs ? 2 * BM : BM) - 1) / (pairs ? 2 * BM : BM) * ((N + BN - 1) / BN) * batch * large_split;
+        const int at_once = pairs ? sms / 2 : sms, rows = pairs ? 2 * BM : BM;
+        const long long large_tiles = (M + rows - 1) / rows * ((N + BN - 1) / BN) * batch, units = large_tiles * large_split;
         if (pairs && units <= at_once) return 0;
         const long long narrow_kb = (tiles * s + sms - 1) / sms * ((total_kb + s - 1) / s);
         const long long large_kb = (units + at_once - 1) / at_once * ((total_kb + large_split - 1) / large_split);
-        if (narrow_kb >= 130 && 4 * narrow_kb >= 9 * large_kb) return 0;
+        const bool well_filled = pairs && 20 * (large_tiles * rows * BN) <= 23 * (tiles * 128 * 64);  // at most 1.15 times the narrow tiles' area
+        if (narrow_kb >= (well_filled ? 105 : 130) && 4 * narrow_kb >= 9 * large_kb) return 0;
     }
     return s;
 }

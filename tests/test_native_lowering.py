@@ -241,6 +241,7 @@ def test_products_on_cuda_cores_take_no_split_scratch(dtype, k, split):
     (384, 3072, 6144, False), (384, 1536, 8192, False),  # more units than pairs of SMs: 384 rows are two row tiles
     (128, 9216, 4096, False), (16, 8192, 4096, False), (128, 4096, 12288, False),  # the one-CTA kernel
     (816, 512, 17376, True), (128, 9216, 12288, True), (16, 4864, 16384, True),  # 130 blocks an SM and 2.25 times the large tiles'
+    (1664, 256, 14296, True), (896, 496, 11008, False),  # 112 and 86 blocks, the result covered by whole tiles
     (384, 1536, 16384, False), (384, 3072, 16384, False),  # 128 blocks; 256, twice the large tiles'
     (128, 8192, 17000, True),  # longer ranges than the narrow tiles take
 ])
