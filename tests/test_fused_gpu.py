@@ -312,6 +312,41 @@ def test_rows_of_odd_widths(cuda, rows, cols, dtype):
     assert ((s.double() - total).abs() <= cols * 2.0**-24 * total + 1e-30).all()
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("cols", [8, 96, 1024, 4100])
+def test_rows_divided_by_one_value_each(cuda, cols, dtype):
+    """Quotients by a row's own divisor - inside and outside the range in which they are taken by its reciprocal, at the ends of that
+    range, with zeros, subnormals, infinities and NaN among the elements - are the correctly rounded ones, also where a later phase
+    of the row divides the same again, and where few elements a thread keep them for it."""
+    rng = np.random.default_rng(cols)
+    edges = [1.0, 3.0, -3.0, 0.0, -0.0, np.inf, np.nan, 2.0**-40, 2.0**-41, 2.0**40, 2.0**41, 1e-45, 3e38, np.nextafter(np.float32(2), np.float32(1))]
+    d = np.concatenate([np.array(edges, np.float32), np.exp2(rng.uniform(-39, 39, 50)).astype(np.float32)])
+    rows = len(d)
+    x = (rng.standard_normal((rows, cols)) * np.exp2(rng.uniform(-30, 30, (rows, cols)))).astype(np.float32)
+    special = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 1e-45, -1e-40, 3e38, 2.0**-61, 2.0**61, 2.0**-60, 2.0**60], np.float32)
+    x[::3, : min(cols, 12)] = special[: min(cols, 12)]
+    x[1] = 0.0
+    if dtype == "bfloat16":
+        x = bf16(x)
+
+    def program(a, b):
+        w = a.to("float32")
+        q = w / b
+        big = prims.reduce_max(q, (1,)).reshape(rows, 1)
+        return q, w / b - big, prims.reduce_sum(q / b, (1,), "float32")
+
+    g = tracer.trace(program, (dtype, (rows, cols)), ("float32", (rows, 1)))
+    kernel = Fusion(g)
+    assert "divide_chunk<" in kernel.source
+    q, r, _ = (to_numpy(t) for t in kernel(to_torch(x, cuda), to_torch(d.reshape(rows, 1), cuda)))
+    with np.errstate(all="ignore"):
+        want = x.astype(np.float32) / d.reshape(rows, 1)
+        big = np.maximum.reduce(want, axis=1, keepdims=True)  # (propagates NaN, as the kernel's maximum does)
+        np.testing.assert_array_equal(q, want)
+        np.testing.assert_array_equal(np.signbit(q[want == 0]), np.signbit(want[want == 0]))
+        np.testing.assert_array_equal(r, want - big)
+
+
 def column_sums_in_slices(x):
     """float32 column sums in the order of the two-pass column reduction: slices of at least 64 rows, eight row lanes each that add every
     eighth row, eight slice lanes that add every eighth slice, lanes in order."""
