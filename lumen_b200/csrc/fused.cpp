@@ -55,13 +55,31 @@ static void launch(lb_fusion* f, const lb_tensor* tensors, int n, void* scratch,
                                     k.n_outputs, n));
     std::vector<void*> ptrs(n);
     std::vector<void*> params(n);
+    bool aligned = true;
     for (int i = 0; i < n; i++) {
         check_dense(tensors[i], k.types[i].dtype, k.types[i].shape, i < k.n_inputs ? "fusion input" : "fusion output");
         // vector accesses assume 16-byte aligned tensors (the plan aligns every buffer to 256 bytes)
-        if (k.vec > 1 && ((uintptr_t)tensors[i].ptr & 15) != 0)
-            fail(LB_ERR_INVALID, format("fusion tensor %d is not 16-byte aligned", i));
+        if (k.vec > 1 && ((uintptr_t)tensors[i].ptr & 15) != 0) {
+            if (!k.unaligned) fail(LB_ERR_INVALID, format("fusion tensor %d is not 16-byte aligned", i));
+            aligned = false;
+        }
         ptrs[i] = tensors[i].ptr;
         params[i] = &ptrs[i];
+    }
+    if (!aligned) {
+        lb_fusion* other;
+        {
+            std::lock_guard<std::mutex> lock(g_cache_mutex);
+            if (!f->unaligned) {
+                auto built = std::make_unique<lb_fusion>();
+                built->kernel = *k.unaligned;
+                built->cubin = nvrtc_compile("fused_kernel", built->kernel.source);
+                f->unaligned = std::move(built);
+            }
+            other = f->unaligned.get();
+        }
+        launch(other, tensors, n, scratch, stream);
+        return;
     }
     if (k.empty || (k.rows == 0 && !k.two_pass)) return;  // empty grid: nothing to launch (lumen/runtime/kernel/cuda/mod.rs:131-133)
     const DeviceInfo& dev = device_info();
@@ -83,9 +101,10 @@ static void launch(lb_fusion* f, const lb_tensor* tensors, int n, void* scratch,
         launch_kernel(fn.finalize, k.fin_blocks, 1, k.fin_threads, stream, params.data(), "cuLaunchKernelEx(fused_finalize)");
         return;
     }
-    int64_t row_blocks = (k.rows + k.rows_per_block - 1) / k.rows_per_block;
-    int per_sm = std::max(1, 2048 / k.threads);
-    int64_t grid = std::min<int64_t>(row_blocks, (int64_t)dev.sms * per_sm);
+    const int64_t together = (int64_t)k.rows_per_block * k.row_period;
+    int64_t row_blocks = (k.rows + together - 1) / together * k.row_period;
+    int per_sm = k.per_sm ? k.per_sm : std::max(1, 2048 / k.threads);
+    int64_t grid = std::min<int64_t>(row_blocks, (int64_t)dev.sms * per_sm / k.row_period * k.row_period);
     launch_kernel(fn.function, grid, 1, k.threads, stream, params.data(), "cuLaunchKernelEx(fused_kernel)");
 }
 

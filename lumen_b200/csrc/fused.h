@@ -1,6 +1,7 @@
 // Fused elementwise / reduction / row kernels: generation (fused_codegen.cpp), compilation cache and launch.
 #pragma once
 #include <map>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -27,6 +28,12 @@ struct FusedKernel {
     // shape [rows, cols] only fixes `cols`, every group brings its row count
     bool multi = false;
     int multi_max_groups = 0;
+    // Rows of a width that is no multiple of a vector, read from the aligned address before them: blocks walk rows `row_period` apart, so
+    // the grid is a multiple of it (or a block has one row block), and the tensors are 16-byte aligned. `unaligned` is for those that are not.
+    bool shifted = false;
+    int row_period = 1;
+    int per_sm = 0;  // blocks that an SM holds (0: as many as its threads)
+    std::shared_ptr<const FusedKernel> unaligned;
     bool empty = false;  // every output has zero elements: no kernel was generated, a launch does nothing
 };
 
@@ -54,4 +61,5 @@ struct lb_fusion {
     std::map<int, Loaded> loaded;  // by device ordinal: the cubin is loaded into a device's context on its first launch there
     std::string cubin;
     size_t scratch_bytes = 0;
+    std::unique_ptr<lb_fusion> unaligned;  // of kernel.unaligned, built when it is first launched
 };

@@ -108,6 +108,52 @@ template <class T, int V> __device__ __forceinline__ void stv(T* p, const T* src
     #pragma unroll
     for (int k = 0; k < B / P; k++) ((W*)p)[k] = ((const W*)src)[k];
 }
+// The same at element `at` (a multiple of V) of an array of `total`, of which the last V may lie partly behind its end (where the last
+// element stands in: a value as good as its neighbours, so that what is computed from it takes no path of its own)
+template <class T, int V, class I> __device__ __forceinline__ void ldv_within(const T* __restrict__ p, I at, I total, T* dst) {
+    if (at + V <= total) { ldv<T, V>(p + at, dst); return; }
+    #pragma unroll
+    for (int k = 0; k < V; k++) dst[k] = __ldg(p + (at + k < total ? at + k : total - 1));
+}
+template <class T, int V, class I> __device__ __forceinline__ void ldv_within_plain(const T* p, I at, I total, T* dst) {
+    if (at + V <= total) { ldv_plain<T, V>(p + at, dst); return; }
+    #pragma unroll
+    for (int k = 0; k < V; k++) dst[k] = p[at + k < total ? at + k : total - 1];
+}
+// Elements [at - shift, at - shift + V) of an array of `total`, 0 <= shift < V, at a multiple of V: two aligned pieces, whose bytes are
+// moved by the shift (the same for every thread). Others of the array's elements stand in before the first and behind the last.
+template <class T, int V, class I> __device__ __forceinline__ void ldv_shifted(const T* __restrict__ p, I at, int shift, I total, T* dst) {
+    constexpr int B = sizeof(T) * V;
+    if constexpr (B != 16 || sizeof(T) > 4 || sizeof(T) < 2) {
+        #pragma unroll
+        for (int k = 0; k < V; k++) { const I i = at - shift + k; dst[k] = __ldg(p + (i < 0 ? 0 : i < total ? i : total - 1)); }
+    } else {
+        u32 w[8];
+        ldv_within<T, V, I>(p, at >= V ? at - V : at, total, (T*)w);
+        ldv_within<T, V, I>(p, at, total, (T*)(w + 4));
+        const int from = B - shift * (int)sizeof(T);  // first byte, in (0, 16]
+        #pragma unroll
+        for (int k = 0; k < 8; k++) w[k] = from & 16 ? w[k < 4 ? k + 4 : k] : w[k];
+        #pragma unroll
+        for (int k = 0; k < 6; k++) w[k] = from & 8 ? w[k + 2] : w[k];
+        #pragma unroll
+        for (int k = 0; k < 5; k++) w[k] = from & 4 ? w[k + 1] : w[k];
+        if (sizeof(T) == 2) {
+            #pragma unroll
+            for (int k = 0; k < 4; k++) w[k] = from & 2 ? __funnelshift_r(w[k], w[k + 1], 16) : w[k];
+        }
+        #pragma unroll
+        for (int k = 0; k < 4; k++) ((u32*)dst)[k] = w[k];
+    }
+}
+// Stores those of V consecutive elements that lie in [0, cols), the first of them at column c of the row at p
+template <class T, int V, class I> __device__ __forceinline__ void stv_within(T* p, I c, I cols, const T* src) {
+    if (c >= 0 && c + V <= cols) { stv<T, V>(p + c, src); return; }
+    if constexpr (V > 1) {
+        stv_within<T, V / 2, I>(p, c, cols, src);
+        stv_within<T, V / 2, I>(p, c + V / 2, cols, src + V / 2);
+    }
+}
 template <class T> __device__ __forceinline__ T shfl_xor_any(T v, int m) {
     if (sizeof(T) == 8) { u64 b; memcpy(&b, &v, 8); b = __shfl_xor_sync(0xffffffffu, b, m); memcpy(&v, &b, 8); return v; }
     u32 b = 0; memcpy(&b, &v, sizeof(T)); b = __shfl_xor_sync(0xffffffffu, b, m); memcpy(&v, &b, sizeof(T)); return v;
@@ -406,8 +452,11 @@ class Generator {
             std::string buf = format("ob%d", k);
             home->pre += format("__align__(16) %s %s[VEC];\n", ct.memory, buf.c_str());
             home->body += store_element(buf, t.dtype, val);
-            home->post += format("if (active) stv<%s, VEC>((%s*)out%d + (r * (idx_t)NCOLS + c0), %s);\n", ct.memory,
-                                 ct.memory, k, buf.c_str());
+            if (shifted_)
+                home->post += format("if (active) stv_within<%s, VEC, idx_t>((%s*)out%d + r * (idx_t)NCOLS, c0, (idx_t)NCOLS, %s);\n", ct.memory, ct.memory, k, buf.c_str());
+            else
+                home->post += format("if (active) stv<%s, VEC>((%s*)out%d + (r * (idx_t)NCOLS + c0), %s);\n", ct.memory,
+                                     ct.memory, k, buf.c_str());
         }
         // Column sums: a thread keeps its columns for all the rows its CTA walks, so the partial sums stay in registers.
         for (size_t k = 0; k < col_reduces_.size(); k++) {
@@ -452,6 +501,8 @@ class Generator {
     std::set<int> behind_columns_;
     std::vector<int> column_outputs_;
     int resident_ = 1;  // CTAs per SM a kernel with column sums is built for and launched with
+    bool shifts_ = true, shifted_ = false;  // may start, starts a row's chunks at aligned addresses before its first element
+    int period_ = 1;                        // ... rows that far apart at the same distance
 
     std::string fresh(const char* prefix) { return format("%s%d", prefix, counter_++); }
 
@@ -531,13 +582,18 @@ class Generator {
         };
         for (int v : g_.inputs) consider(g_.type(v));
         for (int v : g_.outputs) consider(g_.type(v));
-        VEC_ = std::min(8, 16 / min_size);
+        const int widest = std::min(8, 16 / min_size);
+        VEC_ = widest;
         while (VEC_ > 1 && C_ % VEC_ != 0) VEC_ /= 2;
-        int64_t nvec = std::max<int64_t>((C_ + VEC_ - 1) / VEC_, 1);
+        shifted_ = VEC_ == 1 && widest == 8 && shifts_ && !mixed_ && shiftable(*space, widest);
+        if (shifted_) VEC_ = widest;
+        auto vectors = [&] { return std::max<int64_t>((C_ + VEC_ - 1 + (shifted_ ? VEC_ - 1 : 0)) / VEC_, 1); };
+        int64_t nvec = vectors();
         const int64_t per = vectors_per_thread(nvec);
         int64_t want = (nvec + per - 1) / per;
         T_ = 1;
         while (T_ < want && T_ < 1024) T_ *= 2;
+        if (shifted_ && T_ > 32) T_ = (int)std::min<int64_t>((want + 31) / 32 * 32, 1024);
         RPB_ = T_ >= 32 ? 1 : 256 / T_;
         if (T_ > 32) RPB_ = 1;
         else RPB_ = std::max(1, 256 / T_);
@@ -559,13 +615,19 @@ class Generator {
             // 192 to 256. Layer norm forward and backward of 14563 rows: 2304 wide float32 339 -> 205 us, bfloat16 196 -> 175; 2600 wide 366 -> 229,
             // 283 -> 185; 3001 wide 387 -> 244, 257 -> 214.
             if (T_ > 256 && T_ <= 384) {
-                if (VEC_ == 8) VEC_ = 4, nvec *= 2, chunks = 2;
+                if (VEC_ == 8) VEC_ = 4, nvec = vectors(), chunks = 2;
                 T_ = (int)threads_for(chunks * 3 / 2);
             }
             RPB_ = T_ > 32 ? 1 : 128 / T_;
             resident_ = std::max(1, 512 / (T_ * RPB_));  // 12 to 16 warps an SM, 128 registers a thread or more, down to 64 at 1024 threads
         }
         NCH_ = (int)((nvec + T_ - 1) / T_);
+        if (shifted_) {
+            period_ = VEC_;  // (the width is odd)
+            // As many blocks as are resident at once, so that each moves the columns' operands into place once for all its rows: 24 warps an
+            // SM where rows are summed, else 32. (5590 x 3001, us: 12.0; with as many blocks as an SM has threads for, 2048, 16.4.)
+            resident_ = (int)std::max<int64_t>(1, (has_reduce_ ? 768 : 1024) / (T_ * RPB_));
+        }
         if (NCH_ > 64) fail(LB_ERR_UNSUPPORTED, format("rows of %lld elements are too long for the fused row kernel", (long long)C_));
         wide_index_ = R_ * C_ >= (1LL << 31) - 4096;
         for (int v : g_.inputs)
@@ -573,6 +635,41 @@ class Generator {
         if (multi_) wide_index_ = true;  // a group's row count is a run-time value
         pair_ = VEC_ >= 2 && computes_bf16();
     }
+
+    // Whether rows of an odd width are read in whole vectors all the same. Their elements start at any address, but all tensors over
+    // the space start alike: a row's chunks begin at the aligned address at or before its first element, and its neighbours' elements
+    // in the first and the last chunk count for nothing and are not written. A block walks rows that start at the same distance from an
+    // aligned address (every eighth one does), so that a thread keeps its columns. The tensors are read as the space is laid out, by
+    // column, by row or as one value; the columns' operands are moved into place once a block.
+    // For bfloat16 pairs, one row sum at most and six million elements and more. What bounded such rows was one load and one store an
+    // element. Multiply-add-relu with and without a row sum of squares, and a row sum alone, us, 55 shapes of 6.3 to 34 million
+    // elements and 129 to 16383 columns, element by element -> so: 0.45 - 1.03 of the time (5590 x 3001 19.2 -> 12.0, 22.0 -> 13.4, 9.2 ->
+    // 6.5; 32704 x 513 19.7 -> 18.0; floor at the copy's bandwidth 10.3, 10.3, 5.1). Left as they were: 4 million elements (0.8 - 1.12),
+    // several row sums (softmax 1.1 - 1.5: three phases with their masks), float32 (0.8 - 1.3: four bytes a thread are half a line's
+    // worth already), float16 (0.9 - 1.6: no pairs), even widths (0.9 - 1.8), column sums in the same kernel (1.0 - 2.0).
+    bool shiftable(const TensorType& space, int widest) const {
+        if (multi_ || R_ < widest || C_ < kShiftedColumns || R_ * C_ < kShiftedElements) return false;
+        int row_sums = 0;
+        for (const Node& n : g_.nodes) {
+            if (n.op == "gather" || n.op == "iota" || n.op == "slice" || n.op == "transpose") return false;
+            row_sums += n.op == "reduce_sum" || n.op == "reduce_max";
+        }
+        if (row_sums > 1 || !computes_bf16()) return false;
+        for (int v : g_.inputs) {
+            const TensorType& t = g_.type(v);
+            const int64_t n = t.numel();
+            const bool spans = n == R_ * C_ && t.shape.back() == space.shape.back(), columns = n == C_ && t.shape.back() == C_;
+            if (!spans && !columns && n != R_ && n != 1) return false;
+            if (spans && space.shape.back() != C_ && t.shape != space.shape) return false;
+        }
+        for (int v : g_.outputs) {
+            const TensorType& t = g_.type(v);
+            if (t.numel() == R_ * C_ && t.shape.back() != space.shape.back()) return false;
+        }
+        return true;
+    }
+    static constexpr int64_t kShiftedColumns = 128, kShiftedElements = 6 << 20;
+    std::string column() const { return shifted_ ? "column(c0 + e)" : "(c0 + e)"; }
 
     // Vectors of a row per thread: four of 16 bytes. Of the narrow ones that a width without a power of two allows, 16 (eight of
     // two elements) where rows are long and many: a row over 1024 threads of three 2-byte loads each is bound by its barriers and by
@@ -615,9 +712,10 @@ class Generator {
     }
     Comp col_comp() {
         Comp c;
-        c.expr = "(c0 + e)";
+        c.expr = column();
         c.base = "c0";
-        c.lane = c.e_dep = c.c_dep = true;
+        c.lane = !shifted_;
+        c.e_dep = c.c_dep = true;
         return c;
     }
 
@@ -725,8 +823,9 @@ class Generator {
         }
         Comp flat;
         flat.base = format("(r * (idx_t)%lld + c0)", (long long)C_);
-        flat.expr = format("(r * (idx_t)%lld + c0 + e)", (long long)C_);
-        flat.lane = flat.e_dep = flat.c_dep = flat.row_dep = true;
+        flat.expr = shifted_ ? format("(r * (idx_t)%lld + %s)", (long long)C_, column().c_str()) : format("(r * (idx_t)%lld + c0 + e)", (long long)C_);
+        flat.lane = !shifted_;
+        flat.e_dep = flat.c_dep = flat.row_dep = true;
         return unravel(flat, t.shape);
     }
 
@@ -925,8 +1024,9 @@ class Generator {
     }
     // the statement(s) folding element e (and e + 1) of `val` into `acc`
     std::string accumulate(const std::string& acc, const std::string& combine, const std::string& val) {
-        if (!pair_) return format("%s = %s;\n", acc.c_str(), subst(combine, acc, val).c_str());
-        return both_lanes(format("%s = %s;\n", acc.c_str(), subst(combine, acc, "LX(" + val + ")").c_str()));
+        const char* counts = shifted_ ? "if (whole || in_row(c0 + e)) " : "";  // (a row's neighbours do not)
+        if (!pair_) return format("%s%s = %s;\n", counts, acc.c_str(), subst(combine, acc, val).c_str());
+        return both_lanes(format("%s%s = %s;\n", counts, acc.c_str(), subst(combine, acc, "LX(" + val + ")").c_str()));
     }
 
     // ---- loads ------------------------------------------------------------------------------------------
@@ -937,6 +1037,19 @@ class Generator {
         CType ct = ctype(t.dtype);
         Comp flat = ravel(idx, t.shape);
         std::string ptr = format("((const %s*)in%d)", ct.memory, position);
+        const char* plain = inplace_ ? "_plain" : "";
+        auto vector_load = [&](const std::string& dst) {
+            if (!shifted_) return format("ldv%s<%s, VEC>(%s + %s, %s);", plain, ct.memory, ptr.c_str(), flat.base.c_str(), dst.c_str());
+            if (flat.row_dep) return format("ldv_within%s<%s, VEC, idx_t>(%s, %s, (idx_t)%lldLL, %s);", plain, ct.memory, ptr.c_str(), flat.base.c_str(), (long long)(R_ * C_), dst.c_str());
+            return format("ldv_shifted<%s, VEC, idx_t>(%s, c0 + shift, shift, (idx_t)NCOLS, %s);", ct.memory, ptr.c_str(), dst.c_str());
+        };
+        if (shifted_ && ph.chunked && e_dep(idx)) {
+            if (t.numel() == R_ * C_ && key_of(0, idx) == key_of(0, output_index(t, true))) {
+                flat.lane = true, flat.base = format("(r * (idx_t)%lldLL + c0)", (long long)C_);
+            } else if (t.numel() == C_ && flat.expr == "(" + column() + ")" && !inplace_) {
+                flat.lane = true, flat.base = "c0";
+            }
+        }
         if (flat.lane && ph.chunked) {
             // contiguous along the vector lane: one vector load per chunk
             bool column_only = !flat.row_dep && !flat.dyn && !column_mode_;  // same for every row: cache once per CTA
@@ -947,8 +1060,7 @@ class Generator {
                 if (it == cached_loads_.end()) {
                     std::string buf = fresh("col");
                     kernel_cache_ += format("__align__(16) %s %s[NCH][VEC];\n", ct.memory, buf.c_str());
-                    kernel_cache_ += format("CHUNK_LOOP_BEGIN %s<%s, VEC>(%s + %s, %s[ch]); CHUNK_LOOP_END\n", inplace_ ? "ldv_plain" : "ldv", ct.memory,
-                                            ptr.c_str(), flat.base.c_str(), buf.c_str());
+                    kernel_cache_ += "CHUNK_LOOP_BEGIN " + vector_load(buf + "[ch]") + " CHUNK_LOOP_END\n";
                     cached_regs_ += NCH_ * VEC_ * std::max(1, dtype_size(t.dtype) / 4);
                     it = cached_loads_.emplace(key, buf).first;
                 }
@@ -960,12 +1072,8 @@ class Generator {
                 if (it == cached_loads_.end()) {
                     std::string buf = fresh("row");
                     row_cache_ += format("__align__(16) %s %s[NCH][VEC];\n", ct.memory, buf.c_str());
-                    row_cache_ += format("CHUNK_LOOP_BEGIN %s<%s, VEC>(%s + %s, %s[ch]); CHUNK_LOOP_END\n", inplace_ ? "ldv_plain" : "ldv", ct.memory,
-                                         ptr.c_str(), flat.base.c_str(), buf.c_str());
-                    row_caches_.push_back({ct.memory, buf,
-                                           format("CHUNK_LOOP_BEGIN %s<%s, VEC>(%s + %s, %s_nx[ch]); CHUNK_LOOP_END\n", inplace_ ? "ldv_plain" : "ldv",
-                                                  ct.memory, ptr.c_str(), flat.base.c_str(), buf.c_str()),
-                                           NCH_ * VEC_ * dtype_size(t.dtype)});
+                    row_cache_ += "CHUNK_LOOP_BEGIN " + vector_load(buf + "[ch]") + " CHUNK_LOOP_END\n";
+                    row_caches_.push_back({ct.memory, buf, "CHUNK_LOOP_BEGIN " + vector_load(buf + "_nx[ch]") + " CHUNK_LOOP_END\n", NCH_ * VEC_ * dtype_size(t.dtype)});
                     cached_regs_ += NCH_ * VEC_ * std::max(1, dtype_size(t.dtype) / 4);
                     it = cached_loads_.emplace(key, buf).first;
                 }
@@ -976,8 +1084,7 @@ class Generator {
             auto it = ph.memo.find(pkey);
             if (it == ph.memo.end()) {
                 std::string buf = fresh("ld");
-                ph.pre += format("__align__(16) %s %s[VEC]; %s<%s, VEC>(%s + %s, %s);\n", ct.memory, buf.c_str(),
-                                 inplace_ ? "ldv_plain" : "ldv", ct.memory, ptr.c_str(), flat.base.c_str(), buf.c_str());
+                ph.pre += format("__align__(16) %s %s[VEC]; %s\n", ct.memory, buf.c_str(), vector_load(buf).c_str());
                 it = ph.memo.emplace(pkey, buf).first;
             }
             vector_element_ = format("%s[e]", it->second.c_str());
@@ -1277,8 +1384,9 @@ class Generator {
             std::vector<int64_t> tail(x.shape.end() - axes.size(), x.shape.end());
             Comp flat;
             flat.base = "c0";
-            flat.expr = "(c0 + e)";
-            flat.lane = flat.e_dep = flat.c_dep = true;
+            flat.expr = column();
+            flat.lane = !shifted_;
+            flat.e_dep = flat.c_dep = true;
             Index tail_idx = unravel(flat, tail);
             src.insert(src.end(), tail_idx.begin(), tail_idx.end());
         }
@@ -1305,7 +1413,7 @@ class Generator {
             }
         }
         std::string val = gen(n.inputs[0], src, ph);
-        ph.body += accumulate(ph.acc + (four_sums() ? "[ch & 3]" : ""), ph.combine_a_b, val);
+        ph.body += accumulate(ph.acc + (sums() == 1 ? "" : shifted_ ? "[e]" : "[ch & 3]"), ph.combine_a_b, val);
         row_decls_ += format("%s %s;\n", ct.compute, ph.result.c_str());
         phases_.push_back(ph);
         reduce_memo_[key] = ph.result;
@@ -1313,8 +1421,8 @@ class Generator {
     }
 
     // A thread with many narrow vectors of a row keeps four sums: one chain over 16 elements, where wider vectors or more threads make it
-    // four, had 1.35 times the error of a float32 sum over 3001.
-    bool four_sums() const { return VEC_ <= 2 && NCH_ > 4; }
+    // four, had 1.35 times the error of a float32 sum over 3001. Shifted chunks, whose threads have as many elements, keep one a lane.
+    int sums() const { return shifted_ ? VEC_ : VEC_ <= 2 && NCH_ > 4 ? 4 : 1; }
 
     // ---- emission ---------------------------------------------------------------------------------------
     std::string indent(const std::string& code, int n) {
@@ -1348,8 +1456,14 @@ class Generator {
         s << "typedef " << (wide_index_ ? "long long" : "int") << " idx_t;\n";
         s << "#define VEC " << VEC_ << "\n#define NCH " << NCH_ << "\n#define TPR " << T_ << "\n#define RPB " << RPB_ << "\n";
         s << "#define NCOLS " << C_ << "LL\n#define NROWS " << (multi_ ? std::string("group_rows") : std::to_string(R_) + "LL") << "\n";
-        s << "#define CHUNK_LOOP_BEGIN _Pragma(\"unroll\") for (int ch = 0; ch < NCH; ch++) { const idx_t c0 = (idx_t)(ch * TPR + lane_in_row) * VEC; "
-          << (guard ? "if (c0 < NCOLS) {" : "{") << "\n";
+        if (shifted_) {
+            guard = true;
+            s << "#define PERIOD " << period_ << "\n";
+            s << "__device__ __forceinline__ idx_t column(idx_t c) { return c < 0 ? 0 : c < (idx_t)NCOLS ? c : (idx_t)(NCOLS - 1); }\n";
+            s << "__device__ __forceinline__ bool in_row(idx_t c) { return c >= 0 && c < (idx_t)NCOLS; }\n";
+        }
+        s << "#define CHUNK_LOOP_BEGIN _Pragma(\"unroll\") for (int ch = 0; ch < NCH; ch++) { const idx_t c0 = (idx_t)(ch * TPR + lane_in_row) * VEC"
+          << (shifted_ ? " - shift; const bool whole = c0 >= 0 && c0 + VEC <= (idx_t)NCOLS; " : "; ") << (guard ? "if (c0 < NCOLS) {" : "{") << "\n";
         s << "#define CHUNK_LOOP_END }}\n";
         // row reductions
         int width = std::min(T_, 32);
@@ -1401,7 +1515,7 @@ class Generator {
                 s << "    void*" << restrict_kw << " out" << i << " = table.ptr[group][" << g_.inputs.size() + i << "];\n";
         } else {
             s << "extern \"C\" __global__ void __launch_bounds__(" << T_ * RPB_;
-            if (mixed_) s << ", " << resident_;
+            if (mixed_ || shifted_) s << ", " << resident_;
             s << ") fused_kernel(";
             for (size_t i = 0; i < g_.inputs.size(); i++) s << (i ? ", " : "") << "const void*" << restrict_kw << " in" << i;
             for (size_t i = 0; i < g_.outputs.size(); i++)
@@ -1412,7 +1526,16 @@ class Generator {
         s << "    __shared__ unsigned long long red_smem[2][32];\n    int red_turn = 0;\n";
         if (!multi_) s << wait_for_grid(T_ * RPB_, input_names());
         s << "    const int lane_in_row = tid % TPR, row_in_block = tid / TPR;\n";
-        if (!multi_) s << "    const idx_t row_blocks = (idx_t)((NROWS + RPB - 1) / RPB);\n";
+        // the row of a thread in row block %s
+        auto row_of = [&](const std::string& rb) {
+            return shifted_ ? "(" + rb + ") / PERIOD * (PERIOD * RPB) + row_in_block * PERIOD + (" + rb + ") % PERIOD" : "(" + rb + ") * RPB + row_in_block";
+        };
+        // (a row that stands in for one behind the last: loads go there and nothing else)
+        auto stand_in = [&](const std::string& rb) { return shifted_ ? "(" + rb + ") % PERIOD" : std::string("(idx_t)(NROWS - 1)"); };
+        if (shifted_)
+            s << "    const idx_t row_blocks = (idx_t)((NROWS + PERIOD * RPB - 1) / (PERIOD * RPB)) * PERIOD;\n"
+              << "    const int shift = (int)((blockIdx.x % PERIOD) * (u32)(NCOLS % VEC) % VEC);  // the grid is a multiple of PERIOD, or a block has one row block\n";
+        else if (!multi_) s << "    const idx_t row_blocks = (idx_t)((NROWS + RPB - 1) / RPB);\n";
         s << indent(kernel_cache_, 4);
         for (size_t i = 0; i < col_reduces_.size(); i++) {
             const Node& n = *g_.node_of(col_reduces_[i]);
@@ -1432,14 +1555,14 @@ class Generator {
                 s << "    __align__(16) " << c.type << " " << c.buf << "_nx[NCH][VEC];\n";
                 next_loads += c.load;
             }
-            s << "    if ((idx_t)blockIdx.x < row_blocks) {\n        idx_t r = (idx_t)blockIdx.x * RPB + row_in_block;\n"
-              << "        if (r >= NROWS) r = (idx_t)(NROWS - 1);\n" << indent(next_loads, 8) << "    }\n";
+            s << "    if ((idx_t)blockIdx.x < row_blocks) {\n        idx_t r = " << row_of("(idx_t)blockIdx.x") << ";\n"
+              << "        if (r >= NROWS) r = " << stand_in("(idx_t)blockIdx.x") << ";\n" << indent(next_loads, 8) << "    }\n";
         }
         if (multi_) s << "    {\n        const idx_t rb = block - table.first[group];\n";
         else s << "    for (idx_t rb = blockIdx.x; rb < row_blocks; rb += gridDim.x) {\n";
-        s << "        idx_t r = rb * RPB + row_in_block;\n";
+        s << "        idx_t r = " << row_of("rb") << ";\n";
         s << "        const bool active = r < NROWS;\n";
-        s << "        if (!active) r = (idx_t)(NROWS - 1);\n";
+        s << "        if (!active) r = " << stand_in("rb") << ";\n";
         s << indent(row_decls_, 8);
         if (prefetch) {
             for (const RowCache& c : row_caches_) {
@@ -1447,17 +1570,19 @@ class Generator {
                 s << "        _Pragma(\"unroll\") for (int ch = 0; ch < NCH; ch++) { _Pragma(\"unroll\") for (int e = 0; e < VEC; e++) " << c.buf
                   << "[ch][e] = " << c.buf << "_nx[ch][e]; }\n";
             }
-            s << "        if (rb + (idx_t)gridDim.x < row_blocks) {\n            idx_t r = (rb + (idx_t)gridDim.x) * RPB + row_in_block;\n"
-              << "            if (r >= NROWS) r = (idx_t)(NROWS - 1);\n" << indent(next_loads, 12) << "        }\n";
+            s << "        if (rb + (idx_t)gridDim.x < row_blocks) {\n            idx_t r = " << row_of("rb + (idx_t)gridDim.x") << ";\n"
+              << "            if (r >= NROWS) r = " << stand_in("rb + (idx_t)gridDim.x") << ";\n" << indent(next_loads, 12) << "        }\n";
         } else {
             s << indent(row_cache_, 8);
         }
         for (size_t at = 0; at < phases_.size(); at++) {
             const Phase& ph = phases_[at];
             s << "        {\n";
-            if (ph.reduces && four_sums())
-                s << "            " << ph.acc_type << " " << ph.acc << "[4] = {" << ph.init << ", " << ph.init << ", " << ph.init << ", " << ph.init << "};\n";
-            else if (ph.reduces) s << "            " << ph.acc_type << " " << ph.acc << " = " << ph.init << ";\n";
+            if (ph.reduces && sums() > 1) {
+                s << "            " << ph.acc_type << " " << ph.acc << "[" << sums() << "] = {" << ph.init;
+                for (int n = 1; n < sums(); n++) s << ", " << ph.init;
+                s << "};\n";
+            } else if (ph.reduces) s << "            " << ph.acc_type << " " << ph.acc << " = " << ph.init << ";\n";
             if (ph.chunked) {
                 s << "            CHUNK_LOOP_BEGIN\n";
                 s << indent(ph.pre, 16);
@@ -1469,8 +1594,11 @@ class Generator {
             }
             if (ph.reduces) {
                 std::string sum = ph.acc;
-                if (four_sums())
-                    sum = subst(ph.combine_a_b, subst(ph.combine_a_b, ph.acc + "[0]", ph.acc + "[1]"), subst(ph.combine_a_b, ph.acc + "[2]", ph.acc + "[3]"));
+                std::vector<std::string> tree;
+                for (int n = 0; sums() > 1 && n < sums(); n++) tree.push_back(format("%s[%d]", ph.acc.c_str(), n));
+                for (; tree.size() > 1; tree.resize(tree.size() / 2))
+                    for (size_t n = 0; n < tree.size() / 2; n++) tree[n] = subst(ph.combine_a_b, tree[2 * n], tree[2 * n + 1]);
+                if (!tree.empty()) sum = tree[0];
                 s << "            " << ph.result << " = row_reduce<" << ph.acc_type << ">(" << sum << ", [](" << ph.acc_type
                   << " a, " << ph.acc_type << " b) { return " << subst(ph.combine_a_b, "a", "b") << "; }, (" << ph.acc_type
                   << ")" << ph.init << ", red_smem[red_turn ^= 1]);\n";
@@ -1518,13 +1646,15 @@ class Generator {
             k.scratch_bytes = scratch;
         } else {
             s << "}\n";
-            k.vec = VEC_;
+            k.vec = VEC_, k.shifted = shifted_;
         }
         k.source = s.str();
         k.rows = R_;
         k.cols = C_;
         k.threads = T_ * RPB_;
         k.rows_per_block = RPB_;
+        k.row_period = period_;
+        if (shifted_) k.per_sm = resident_;
         k.n_inputs = (int)g_.inputs.size();
         k.n_outputs = (int)g_.outputs.size();
         for (int v : g_.inputs) k.types.push_back(g_.type(v));
@@ -1815,12 +1945,13 @@ class Generator {
     void set_inplace(bool v) { inplace_ = v; }
     void set_multi(bool v) { multi_ = v; }
     void set_mixed(bool v) { mixed_ = v; }
+    void set_shifts(bool v) { shifts_ = v; }
 
 };
 
 }  // namespace
 
-FusedKernel generate_fused(const Module& module) {
+static FusedKernel generate(const Module& module, bool shifts) {
     const Graph& g = module.main();
     int reduces = 0;
     for (const Node& n : g.nodes)
@@ -1834,7 +1965,16 @@ FusedKernel generate_fused(const Module& module) {
     if (Generator::some_columns(g) && !module.options.count("inplace")) gen.set_mixed(true);
     // With a reduction followed by further use of the row, inputs are kept in registers across phases.
     gen.set_multi_phase(reduces >= 1);
+    gen.set_shifts(shifts);
     return gen.run();
+}
+
+FusedKernel generate_fused(const Module& module) {
+    FusedKernel k = generate(module, true);
+    if (!k.shifted) return k;
+    k.unaligned = std::make_shared<FusedKernel>(generate(module, false));
+    k.scratch_bytes = std::max(k.scratch_bytes, k.unaligned->scratch_bytes);
+    return k;
 }
 
 }  // namespace lb

@@ -347,6 +347,50 @@ def test_rows_divided_by_one_value_each(cuda, cols, dtype):
         np.testing.assert_array_equal(r, want - big)
 
 
+# odd rows of bfloat16 that start at every distance from an aligned address: several a block and one, one chunk a thread and four, fewer
+# rows than eight a block's share, a last row whose last chunk ends with the tensor
+@pytest.mark.parametrize("rows,cols", [(50001, 129), (25000, 257), (6300, 1001), (3100, 2047), (2500, 3001), (1601, 4095), (385, 16383), (97, 65533)])
+def test_rows_at_any_address(cuda, rows, cols):
+    """y is exact whether the tensors are aligned or not (then another kernel runs); float32 sums of `cols` non-negative terms are
+    within cols * 2^-24 of the float64 ones; nothing beside the results is written."""
+    gen = torch.Generator(device=cuda).manual_seed(cols)
+    x, g, b = (torch.randn(s, generator=gen, device=cuda).bfloat16() for s in ((rows, cols), (cols,), (cols,)))
+    r = torch.randn((rows, 1), generator=gen, device=cuda).bfloat16()
+
+    def program(x_, g_, b_):
+        y_ = F.relu(x_ * g_ + b_)
+        return y_, prims.reduce_sum(y_ * y_, (1,), "float32")
+
+    def largest(x_, r_):
+        return prims.reduce_max(x_ * r_, (1,)), (x_ * r_).to("float32")
+
+    def bare(x_, g_, b_):
+        return x_ * g_ + b_, (x_ - b_).to("float32")
+
+    def run(fn, *args):
+        kernel = Fusion(tracer.trace(fn, *[("bfloat16", tuple(a.shape)) for a in args]))
+        assert "PERIOD" in kernel.source or (fn is bare and cols < 1024)  # (shorter rows without a sum are put together)
+        types = [kernel.body.types[v] for v in kernel.body.outputs]
+        out = [torch.full((t.numel + 16,), 7.0, device=cuda, dtype=getattr(torch, t.dtype)) for t in types]
+        views = [o[8 : 8 + t.numel].reshape(t.shape) for o, t in zip(out, types)]
+        kernel(*args, out=views)
+        for o, t in zip(out, types):
+            assert (o[:8] == 7).all() and (o[8 + t.numel :] == 7).all()
+        return views
+
+    want = torch.relu(x * g + b)
+    total = (want * want).double().sum(1)
+    for shift in (0, 1):  # elements that the arguments start behind an aligned address
+        xs, gs, bs = (torch.cat([a.new_zeros(shift), a.flatten()])[shift:].reshape(a.shape) for a in (x, g, b))
+        y, s = run(program, xs, gs, bs)
+        assert torch.equal(y, want)
+        assert ((s.double() - total).abs() <= cols * 2.0**-24 * total + 1e-30).all()
+    m, w = run(largest, x, r)
+    assert torch.equal(m, (x * r).amax(1)) and torch.equal(w, (x * r).float())
+    u, v = run(bare, x, g, b)
+    assert torch.equal(u, x * g + b) and torch.equal(v, (x - b).float())
+
+
 def column_sums_in_slices(x):
     """float32 column sums in the order of the two-pass column reduction: slices of at least 64 rows, eight row lanes each that add every
     eighth row, eight slice lanes that add every eighth slice, lanes in order."""
