@@ -502,6 +502,7 @@ class Generator {
     std::vector<int> column_outputs_;
     int resident_ = 1;  // CTAs per SM a kernel with column sums is built for and launched with
     bool shifts_ = true, shifted_ = false;  // may start, starts a row's chunks at aligned addresses before its first element
+    bool narrow_ = false;                   // 16-bit tensors
     int period_ = 1;                        // ... rows that far apart at the same distance
 
     std::string fresh(const char* prefix) { return format("%s%d", prefix, counter_++); }
@@ -583,6 +584,7 @@ class Generator {
         for (int v : g_.inputs) consider(g_.type(v));
         for (int v : g_.outputs) consider(g_.type(v));
         const int widest = std::min(8, 16 / min_size);
+        narrow_ = min_size <= 2;
         VEC_ = widest;
         while (VEC_ > 1 && C_ % VEC_ != 0) VEC_ /= 2;
         shifted_ = VEC_ == 1 && widest == 8 && shifts_ && !mixed_ && shiftable(*space, widest);
@@ -598,11 +600,9 @@ class Generator {
         if (T_ > 32) RPB_ = 1;
         else RPB_ = std::max(1, 256 / T_);
         if (mixed_) {
-            // Column sums live in registers beside the row: eight elements of a row per thread where a
-            // block can be that wide. Residual + layer norm forward and backward of 8192 x 1024 bfloat16 in one such kernel:
-            // 31 us + 6 us for its totals, against 125 us for the nine kernels of one kind of reduction each; bound by
-            // instructions in flight (63 per element, issued 43 % of the time; with 16 elements it spills: 59 us; with four,
-            // or five blocks an SM, 30 - 32 us).
+            // Column sums live in registers beside the row: eight elements of a row per thread where a block can be that wide. Residual +
+            // layer norm forward and backward of 8192 x 1024 bfloat16 in one such kernel: 24 us + 4 us for its totals, against 125 us for
+            // the nine kernels of one kind of reduction each; bound by instructions in flight and the barriers of four row sums.
             int64_t chunks = std::max<int64_t>(1, 16 / VEC_ / 2);
             auto threads_for = [&](int64_t per_thread) {
                 const int64_t t = std::min<int64_t>((nvec + per_thread - 1) / per_thread, 1024);
@@ -610,16 +610,32 @@ class Generator {
                 while (p < t && p < 32) p *= 2;
                 return t > 32 ? (t + 31) / 32 * 32 : p;
             };
+            int64_t warps = 0;  // an SM, at least; otherwise up to 16, 128 registers a thread or more, down to 64 at 1024 threads
             T_ = (int)threads_for(chunks);
-            // A block of 288 to 384 threads would be alone on its SM with 9 to 12 warps: twelve elements a thread instead make two of
-            // 192 to 256. Layer norm forward and backward of 14563 rows: 2304 wide float32 339 -> 205 us, bfloat16 196 -> 175; 2600 wide 366 -> 229,
-            // 283 -> 185; 3001 wide 387 -> 244, 257 -> 214.
-            if (T_ > 256 && T_ <= 384) {
+            if (min_size == 2 && VEC_ >= 4 && C_ >= 1024 && (C_ <= 2048 || C_ > 3072 || R_ * C_ >= 1 << 21)) {
+                // Rows of 16 bits from 1024 columns on: two vectors of eight bytes a thread and as many blocks as 16 warps and more need, so
+                // that a block of 13 to 15 warps is not alone on its SM. (455 x 2304 9.9 -> 10.5: small ones of nine to twelve warps are left.) us, the sums above, one vector of 16 bytes a thread -> so: 2048 x 1024 12.9 ->
+                // 11.0, 4096 x 2048 32.6 -> 31.8, 3640 x 2304 42 -> 35, 2532 x 3312 52 -> 45, 1677 x 5000 48 -> 41, 1024 x 8192 58 -> 45.
+                VEC_ = 4, nvec = vectors(), chunks = 2;
+                T_ = (int)threads_for(chunks);
+                if (T_ > 288 && T_ <= 384 && C_ % (T_ * 8) != 0) T_ = (int)threads_for(3);  // (the last chunk a part: 2600 wide as fast, few rows faster)
+                else warps = 16;
+            } else if (min_size == 4 && VEC_ == 4 && nvec <= 1024 && R_ * C_ >= 1 << 21) {
+                // float32 rows: one vector a thread where that makes a warp or four and more, 32 warps an SM; two where more threads fit so,
+                // or as many but not all 1024. us, two vectors and 16 warps -> so: 16384 x 512 44 -> 33, 8192 x 1024 46 -> 35, 5461 x 1536 58 -> 40,
+                // 4096 x 2048 50 -> 40, 2532 x 3312 73 -> 55, 2048 x 4096 61 -> 44; fewer than two million elements are up to 1.16 slower.
+                const int64_t one = threads_for(1), in_ones = 1024 / one * one, in_twos = 1024 / T_ * T_;
+                if (one == 32 || (one >= 128 && (in_ones > in_twos || in_ones == 1024))) T_ = (int)one;
+                if (T_ >= 128 || one == 32) warps = 32;
+            } else if (T_ > 256 && T_ <= 384) {
+                // A block of 288 to 384 threads would be alone on its SM with 9 to 12 warps: twelve elements a thread instead make two of
+                // 192 to 256. The same sums of 14563 rows: 3001 wide float32 387 -> 244 us, bfloat16 257 -> 214.
                 if (VEC_ == 8) VEC_ = 4, nvec = vectors(), chunks = 2;
                 T_ = (int)threads_for(chunks * 3 / 2);
             }
             RPB_ = T_ > 32 ? 1 : 128 / T_;
-            resident_ = std::max(1, 512 / (T_ * RPB_));  // 12 to 16 warps an SM, 128 registers a thread or more, down to 64 at 1024 threads
+            const int64_t threads = T_ * RPB_;
+            resident_ = (int)std::max<int64_t>(1, warps ? std::min((warps * 32 + threads - 1) / threads, 1024 / threads) : 512 / threads);
         }
         NCH_ = (int)((nvec + T_ - 1) / T_);
         if (shifted_) {
@@ -943,9 +959,10 @@ class Generator {
         return name;
     }
 
-    // Whether a division of float32 elements by `divisor` is one by the same value for the whole chunk.
+    // Whether a division of float32 elements by `divisor` is one by the same value for the whole chunk. (Blocks of 800 threads and more
+    // with float32 rows and their column sums have no registers left for it: 7360 wide 1.05 to 1.1 of the time.)
     bool divides_chunk(const Phase& ph, const std::string& dividend, const std::string& divisor, bool pairs) const {
-        if (column_mode_ || multi_ || VEC_ < 4 || !ph.chunked || mentions_e(divisor) || divisor.find("LX(") != std::string::npos) return false;
+        if (column_mode_ || multi_ || VEC_ < 4 || (mixed_ && T_ > 768 && NCH_ > 1 && !narrow_) || !ph.chunked || mentions_e(divisor) || divisor.find("LX(") != std::string::npos) return false;
         if (!pairs) return body_names_.count(dividend) && !body_names_.count(divisor);
         auto it = pair_vars_.find(dividend);
         return it != pair_vars_.end() && it->second == LB_F32 && !pair_vars_.count(divisor);
