@@ -878,8 +878,16 @@ int gemm_launches(const lb_tensor& a_t, const lb_tensor& b_t, size_t scratch_byt
     return gemm_route(a.rows, b.cols, a.cols, a.batch, sm_count_hint(), kernel_choice, scratch_bytes, tuning).splits > 1 ? 2 : 1;
 }
 
-void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int epilogue, int kernel_choice, void* stream,
-          void* scratch, size_t scratch_bytes, const lb_tensor* aux_t, const GemmTuning* tuning) {
+// The sizes of a product of float32 operands, which decide its tiles; false if there is nothing to do.
+bool gemm_held(const lb_tensor& a_t, const lb_tensor& b_t, SimtProblem& q) {
+    const View3 a = view3(a_t, "a"), b = view3(b_t, "b");
+    q.p.M = (int)a.rows, q.p.N = (int)b.cols, q.p.K = (int)a.cols, q.p.batch = (int)a.batch;
+    return a.rows && b.cols && a.batch;
+}
+
+// With `held`, a product of the CUDA cores is written there instead of launched, and the answer is true.
+bool gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int epilogue, int kernel_choice, void* stream,
+          void* scratch, size_t scratch_bytes, const lb_tensor* aux_t, const GemmTuning* tuning, SimtProblem* held) {
     View3 a = view3(a_t, "a"), b = view3(b_t, "b"), d = view3(d_t, "output");
     if (epilogue < EPI_NONE || epilogue > EPI_MASK) fail(LB_ERR_INVALID, "gemm: unknown epilogue");
     View3 aux{};
@@ -899,7 +907,7 @@ void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
     if (a.dtype != LB_F32 && a.dtype != LB_BF16 && a.dtype != LB_F16) fail(LB_ERR_UNSUPPORTED, "gemm: float16, bfloat16 or float32 operands");
     if (d.dtype != LB_F32 && d.dtype != a.dtype) fail(LB_ERR_INVALID, "gemm: the output is float32 (the accumulator) or the operands' dtype");
     const long long M = a.rows, N = b.cols, K = a.cols, batch = a.batch;
-    if (M == 0 || N == 0 || batch == 0) return;
+    if (M == 0 || N == 0 || batch == 0) return false;
     driver();
     cudaStream_t s = (cudaStream_t)stream;
 
@@ -943,7 +951,7 @@ void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
             q.epilogue = p.epilogue, q.aux = p.aux, q.ld_aux = p.ld_aux, q.aux_batch_stride = p.aux_batch_stride, q.status = p.status;
             q.splits = route.ranges;
             gemm_small(map_a, p.b_mn_major ? map_b : make_map(bt, true, BK, 64), q, (int)batch, dev.sms, s);
-            return;
+            return false;
         }
         if (first_use_on_device((const void*)gemm_tcgen05_pair)) {
             LB_CUDA(cudaFuncSetAttribute(gemm_tcgen05, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
@@ -976,7 +984,7 @@ void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
             if (vec) launch_overlapped(splitk_reduce<true>, blocks, dim3(256), 0, s, 0, (const float*)p.partial, p);
             else launch_overlapped(splitk_reduce<false>, blocks, dim3(256), 0, s, 0, (const float*)p.partial, p);
         }
-        return;
+        return false;
     }
 
     SimtArgs p{};
@@ -992,7 +1000,12 @@ void gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
     };
     p.a_vec = p.a_sk == 1 ? vec(a, p.a_sk, p.a_sm) : vec(a, p.a_sm, p.a_sk);
     p.b_vec = p.b_sn == 1 ? vec(b, p.b_sn, p.b_sk) : vec(b, p.b_sk, p.b_sn);
+    if (held) {
+        *held = SimtProblem{a.ptr, b.ptr, p};
+        return true;
+    }
     gemm_simt(a.ptr, b.ptr, a.dtype, p, device_info().sms, s);
+    return false;
 }
 
 }  // namespace lb
@@ -1004,7 +1017,7 @@ int lb_gemm(const lb_tensor* a, const lb_tensor* b, const lb_gemm_out* out, cons
         if (!a || !b || !out) lb::fail(LB_ERR_INVALID, "lb_gemm: null argument");
         lb::GemmTuning tuning{cfg ? cfg->splits : 0, cfg ? cfg->group_m : 0};
         lb::gemm(*a, *b, out->product, out->epilogue, cfg ? cfg->kernel : 0, stream, cfg ? cfg->scratch : nullptr,
-                 cfg ? cfg->scratch_bytes : 0, out->epilogue >= 2 ? &out->aux : nullptr, &tuning);
+                 cfg ? cfg->scratch_bytes : 0, out->epilogue >= 2 ? &out->aux : nullptr, &tuning, nullptr);
     });
 }
 

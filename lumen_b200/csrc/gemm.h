@@ -24,6 +24,14 @@ struct SimtArgs {
 
 void gemm_simt(const void* a, const void* b, int dtype, const SimtArgs& p, int sms, cudaStream_t s);
 
+struct SimtProblem {
+    const void* a;
+    const void* b;
+    SimtArgs p;
+};
+constexpr int kSimtGroup = 4;
+int gemm_simt_many(const SimtProblem* problems, int n, int sms, bool launch, cudaStream_t s);
+
 // 128 x 64 tiles with the K range of a tile over a cluster (gemm_small.cu): 16-bit operands, maps with boxes of 64
 // elements along the contiguous axis by 128 rows of A, 64 of B (K-major) or 64 (M- / N-major).
 struct SmallGemmArgs {

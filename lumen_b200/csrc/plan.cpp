@@ -24,12 +24,14 @@
 #include <sstream>
 
 #include "fused.h"
+#include "gemm.h"
 
 struct lb_comm;
 
 namespace lb {
-void gemm(const lb_tensor& a, const lb_tensor& b, const lb_tensor& d, int epilogue, int kernel_choice, void* stream,
-          void* scratch, size_t scratch_bytes, const lb_tensor* aux, const GemmTuning* tuning);
+bool gemm(const lb_tensor& a, const lb_tensor& b, const lb_tensor& d, int epilogue, int kernel_choice, void* stream,
+          void* scratch, size_t scratch_bytes, const lb_tensor* aux, const GemmTuning* tuning, SimtProblem* held = nullptr);
+bool gemm_held(const lb_tensor& a, const lb_tensor& b, SimtProblem& q);
 int gemm_launches(const lb_tensor& a, const lb_tensor& b, size_t scratch_bytes, int kernel_choice, const GemmTuning* tuning);
 int gemm_model_splits(long long M, long long N, long long K, long long batch);
 void fill_noise(void* ptr, size_t bytes, void* stream);
@@ -270,12 +272,58 @@ void prepare_collectives(lb_plan& p) {
     }
 }
 
+// Products of float32 operands (always the CUDA cores') that follow one another and of which none reads or writes what another writes:
+// the two gradients of a linear layer, and the like. They are queued together (gemm_simt_many), at the latest before the
+// next step of another kind.
+struct Bytes {
+    uintptr_t begin, end;
+    explicit Bytes(const lb_tensor& t) {
+        long long low = 0, high = 1;
+        for (int d = 0; d < t.rank; d++) (t.stride[d] < 0 ? low : high) += (t.shape[d] - 1) * t.stride[d];
+        begin = (uintptr_t)t.ptr + low * (long long)dtype_size(t.dtype), end = (uintptr_t)t.ptr + high * (long long)dtype_size(t.dtype);
+    }
+    bool meets(const Bytes& o) const { return begin < o.end && o.begin < end; }
+};
+struct Products {
+    std::vector<SimtProblem> held;
+    std::vector<Bytes> read, written;
+    static bool takes(const Step& s, const lb_tensor& a) { return s.kind == GEMM && a.dtype == LB_F32; }
+    bool independent(const lb_tensor& a, const lb_tensor& b, const lb_tensor& d) const {
+        const Bytes x(a), y(b), z(d);
+        for (const Bytes& w : written)
+            if (w.meets(x) || w.meets(y) || w.meets(z)) return false;
+        for (const Bytes& r : read)
+            if (r.meets(z)) return false;
+        return true;
+    }
+    void add(const lb_tensor& a, const lb_tensor& b, const lb_tensor& d, const SimtProblem& q) {
+        held.push_back(q);
+        read.emplace_back(a), read.emplace_back(b), written.emplace_back(d);
+    }
+    int queue(int sms, bool launch, cudaStream_t s) {
+        if (held.empty()) return 0;
+        const int n = gemm_simt_many(held.data(), (int)held.size(), sms, launch, s);
+        held.clear(), read.clear(), written.clear();
+        return n;
+    }
+};
+
 void run(const lb_plan& p, void* ws, void* const* in, void* const* out, int first, int last, void* stream) {
     if (first < 0 || last > (int)p.steps.size() || first > last) fail(LB_ERR_INVALID, "plan: step range out of bounds");
     std::vector<lb_tensor> tensors;
+    Products products;
+    auto queue = [&] { products.queue(device_info().sms, true, (cudaStream_t)stream); };
     for (int k = first; k < last; k++) {
         const Step& s = p.steps[k];
         auto T = [&](int i) { return bind(p, s.args.at(i), ws, in, out); };
+        if (s.kind == GEMM && Products::takes(s, T(0))) {
+            const lb_tensor a = T(0), b = T(1), d = T(2);
+            if (!products.independent(a, b, d)) queue();
+            SimtProblem q{};
+            if (gemm(a, b, d, s.epilogue, s.tuned_kernel, stream, nullptr, 0, nullptr, &s.tuning, &q)) products.add(a, b, d, q);
+            continue;
+        }
+        queue();
         switch (s.kind) {
             case FUSION: {
                 tensors.clear();
@@ -363,6 +411,7 @@ void run(const lb_plan& p, void* ws, void* const* in, void* const* out, int firs
             }
         }
     }
+    queue();
 }
 
 }  // namespace
@@ -547,7 +596,24 @@ int lb_plan_kernel_launches(const lb_plan* plan) {
     if (!plan) return -1;
     int n = 0;
     const int rc = lb::guarded([&] {  // a step may name a tensor that the plan does not define
+        lb::Products products;  // told apart by where they lie in the workspace, which input and which output they are
+        const int sms = lb::sm_count_hint();
         for (const lb::Step& s : plan->steps) {
+            auto place = [&](int i) {
+                const lb::View& v = plan->views.at((size_t)s.args.at(i));
+                lb_tensor t = v.t;
+                const uintptr_t base = v.base_kind == 'w' ? 1 : 2 + 2 * (uintptr_t)v.base_index + (v.base_kind == 'o');
+                t.ptr = (void*)((base << 44) + v.offset);
+                return t;
+            };
+            if (s.kind == lb::GEMM && lb::Products::takes(s, place(0))) {
+                const lb_tensor a = place(0), b = place(1), d = place(2);
+                if (!products.independent(a, b, d)) n += products.queue(sms, false, nullptr);
+                lb::SimtProblem q{};
+                if (lb::gemm_held(a, b, q)) products.add(a, b, d, q);
+                continue;
+            }
+            n += products.queue(sms, false, nullptr);
             switch (s.kind) {
                 case lb::FUSION: n += s.fusion && s.fusion->kernel.empty ? 0 : (s.scratch >= 0 ? 2 : 1); break;  // partial sums + finalize
                 case lb::MULTI: n += s.fusion && s.fusion->kernel.multi_max_groups > 0 ? (s.aux + s.fusion->kernel.multi_max_groups - 1) / s.fusion->kernel.multi_max_groups : 1; break;
@@ -576,6 +642,7 @@ int lb_plan_kernel_launches(const lb_plan* plan) {
                 default: break;  // block and 2-d copies, fills, collectives and waits launch no kernel of this library
             }
         }
+        n += products.queue(sms, false, nullptr);
     });
     return rc == LB_OK ? n : -1;
 }

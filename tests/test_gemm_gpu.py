@@ -356,3 +356,40 @@ def test_scratch_decides_between_narrow_and_cut_large_tiles(cuda, shape, large, 
     for out in (narrow, cut):  # 64 * 2^-24 of the sum of magnitudes for the order of K additions, the result's rounding
         assert ((out.double() - want).abs() <= 64 * 2.0**-24 * size + (2.0**-8 * want.abs() if dtype == "bfloat16" else 0)).all()
     device_status()
+
+
+def products_plan(shapes):
+    from lumen_b200.compiler import compile_graph
+    from lumen_b200.plan import Plan
+
+    def program(*x):
+        return tuple(F.matmul(x[2 * i], x[2 * i + 1], "float32", "float32") for i in range(len(shapes)))
+
+    specs = [("float32", s) for m, n, k in shapes for s in ((m, k), (k, n))]
+    return Plan(compile_graph(tracer.trace(program, *specs)))
+
+
+@pytest.mark.parametrize("shapes", [
+    [(64, 48, 40), (33, 65, 70)], [(16, 32, 0), (1, 5, 7), (16, 33, 64)],  # tiles of 16 rows, one product without a sum
+    [(400, 410, 15), (17, 33, 65), (416, 384, 128), (40, 70, 63), (130, 70, 33), (64, 64, 64)],  # two sizes of tile, more than a launch takes
+    [(1100, 1121, 33), (256, 128, 512), (128, 512, 64)]])  # one that fills the GPU beside two that do not
+def test_float32_products_of_one_launch_are_those_of_several(cuda, shapes):
+    """Products of a plan that do not depend on one another share launches; every sum keeps its order."""
+    x = [to_torch(t, cuda) for i, (m, n, k) in enumerate(shapes) for t in (operands(m, n, k, i) if k else (np.zeros((m, 0), "f"), np.zeros((0, n), "f")))]
+    outs = [torch.full((m, n), float("nan"), device=cuda) for m, n, k in shapes]
+    products_plan(shapes).run(x, outs)
+    for i, out in enumerate(outs):
+        assert torch.equal(out, gemm(x[2 * i], x[2 * i + 1], torch.empty_like(out)))
+
+
+def test_a_float32_product_that_reads_anothers_result_comes_after_it(cuda):
+    """The memory given to a run decides: here the first result lies where the second product's operand does, the third's result where
+    the second reads."""
+    x = [to_torch(t, cuda) for i in range(3) for t in operands(64, 64, 64, i)]
+    first, second = torch.empty(64, 64, device=cuda), torch.empty(64, 64, device=cuda)
+    gemm(x[0], x[1], first)
+    gemm(first, x[3], second)
+    third = gemm(x[4], x[5], torch.empty_like(first))
+    got = torch.empty_like(second)
+    products_plan([(64, 64, 64)] * 3).run(x, [x[2], got, x[3]])
+    assert torch.equal(x[2], first) and torch.equal(got, second) and torch.equal(x[3], third)

@@ -235,6 +235,23 @@ def test_products_on_cuda_cores_take_no_split_scratch(dtype, k, split):
         lib.lb_plan_destroy(handle)
 
 
+@pytest.mark.parametrize("shapes, chained, launches", [
+    ([(64, 64, 64), (128, 32, 512)], False, 1), ([(64, 64, 64)] * 2, True, 2), ([(64, 64, 64)] * 5, False, 2), ([(64, 0, 64), (64, 64, 0)], False, 1),
+    ([(1088, 1152, 64), (64, 64, 64), (64, 64, 64)], False, 2)])  # 17 x 18 tiles of 64 x 64: two for each of 148 SMs, a launch of their own
+def test_float32_products_beside_one_another_share_a_launch(shapes, chained, launches):
+    """Those of which none reads another's result, four to a launch."""
+    def program(*x):
+        y = []
+        for i in range(len(shapes)):
+            y.append(F.matmul(y[-1] if chained and y else x[2 * i], x[2 * i + 1], "float32", "float32"))
+        return tuple(y)
+
+    g = tracer.trace(program, *[("float32", s) for m, n, k in shapes for s in ((m, k), (k, n))])
+    lib, native = _bind(), lower_native(fuse(clean(g)))
+    assert lib.lb_plan_kernel_launches(native) == launches
+    lib.lb_plan_destroy(native)
+
+
 @pytest.mark.parametrize("m, n, k, split", [
     (1024, 1024, 8192, True), (768, 768, 8192, True),  # 128 blocks of K for two ranges of narrow tiles: the line
     (768, 768, 8128, False), (512, 512, 4096, False),  # shorter ranges
