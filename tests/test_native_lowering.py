@@ -235,6 +235,16 @@ def test_products_on_cuda_cores_take_no_split_scratch(dtype, k, split):
         lib.lb_plan_destroy(handle)
 
 
+@pytest.mark.parametrize("m, n, k, copied", [(2048, 4096, 64, True), (2040, 4096, 64, False), (2048, 4096, 60, False), (2048, 4088, 64, False), (1024, 4096, 32, False), (4096, 4096, 32, True)])
+def test_weights_of_much_larger_products_are_transposed(m, n, k, copied):
+    """A K-major copy of a weight with long rows: in both lowerings, and never one that the tensor cores do not read."""
+    from lumen_b200.compiler import compile_graph
+
+    g = tracer.trace(lambda x, w: F.matmul(x, w, "float32", "bfloat16"), ("bfloat16", (m, k)), ("bfloat16", (k, n)))
+    steps, _ = plan_of(fuse(clean(g)))
+    assert [label for _, label in steps] == compile_graph(g).labels == ["weight_transpose"] * copied + ["dot_general"]
+
+
 @pytest.mark.parametrize("shapes, chained, launches", [
     ([(64, 64, 64), (128, 32, 512)], False, 1), ([(64, 64, 64)] * 2, True, 2), ([(64, 64, 64)] * 5, False, 2), ([(64, 0, 64), (64, 64, 0)], False, 1),
     ([(1088, 1152, 64), (64, 64, 64), (64, 64, 64)], False, 2)])  # 17 x 18 tiles of 64 x 64: two for each of 148 SMs, a launch of their own
