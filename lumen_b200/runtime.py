@@ -135,7 +135,12 @@ def _empty_like_input(like, shape, dtype: str):
     """A new dense device tensor of `shape`/`dtype` in the framework `like` comes from: torch for a torch tensor (the
     harness's convenience), else the backend's own regions of the current device (grown in 256 MiB reservations)."""
     if type(like).__module__.startswith("torch"):
-        return sys.modules["torch"].empty(shape, dtype=TORCH_DTYPES[dtype], device=like.device)
+        torch = sys.modules["torch"]
+        if type(like) is torch.Tensor:  # 1.5 and 2.0 us a tensor, where `empty` takes 2.4 to read its arguments
+            if like.shape == shape:
+                return torch.empty_like(like, dtype=TORCH_DTYPES[dtype], memory_format=torch.contiguous_format)
+            return like.new_empty(shape, dtype=TORCH_DTYPES[dtype])
+        return torch.empty(shape, dtype=TORCH_DTYPES[dtype], device=like.device)
     from lumen_b200.device import ITEMSIZE, Region, current_device
 
     nbytes = max(math.prod(shape) * ITEMSIZE[dtype], 1)
