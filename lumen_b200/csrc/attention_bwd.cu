@@ -503,9 +503,11 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
 // delta[b, n, s] = sum_d dO[b, s, n, d] * O[b, s, n, d] in fp32. D / 8 lanes per (s, n) row, 16 bytes per lane and
 // tensor, several rows per warp; heads of one token are adjacent so a warp reads contiguous memory. One grid row
 // (blockIdx.y) per batch entry and 32-bit index arithmetic: the kernel is a pure stream of 2 x 16 bytes per thread,
-// and 64-bit divisions per thread used to cost more than the loads.
+// and 64-bit divisions per thread used to cost more than the loads. `zeros` (optional): the dense float32 accumulator of dQ,
+// cleared on the way by the threads of the same rows: a separate clearing stood between this kernel and the next one's early launch.
+// us a backward: 8 x 2048 tokens, 16 heads 312.8 -> 305.4; 4 x 512, 16 heads 33.5 -> 30.3; 300 tokens, 8 heads 30.3 -> 27.7.
 __global__ void __launch_bounds__(256) attention_delta(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                                        float* __restrict__ delta, int S, int N, int D, int n_shift, long long o_sb,
+                                                        float* __restrict__ delta, float* zeros, int S, int N, int D, int n_shift, long long o_sb,
                                                         long long o_ss, long long o_sn, long long g_sb, long long g_ss, long long g_sn) {
     grid_wait(o, d_o);
     const int lanes = D >> 3;  // 8 (D = 64) or 16 (D = 128)
@@ -521,6 +523,10 @@ __global__ void __launch_bounds__(256) attention_delta(const __nv_bfloat16* __re
         else sq = row / (unsigned)N, n = row - sq * (unsigned)N;
         const uint4 x = __ldg((const uint4*)(o + b * o_sb + (long long)sq * o_ss + (long long)n * o_sn + part * 8));
         const uint4 y = __ldg((const uint4*)(d_o + b * g_sb + (long long)sq * g_ss + (long long)n * g_sn + part * 8));
+        if (zeros) {
+            float4* z = (float4*)(zeros + ((long long)b * S * N + row) * D + part * 8);
+            z[0] = z[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
         const __nv_bfloat162* xp = (const __nv_bfloat162*)&x;
         const __nv_bfloat162* yp = (const __nv_bfloat162*)&y;
 #pragma unroll
@@ -534,14 +540,14 @@ __global__ void __launch_bounds__(256) attention_delta(const __nv_bfloat16* __re
 }
 
 // Launches attention_delta over [B, S, N, D] views of o and dO.
-void launch_delta(const lb_tensor& o, const lb_tensor& d_o, float* delta, cudaStream_t s) {
+void launch_delta(const lb_tensor& o, const lb_tensor& d_o, float* delta, float* zeros, cudaStream_t s) {
     const long long B = o.shape[0], S = o.shape[1], N = o.shape[2], D = o.shape[3];
     if (S * N * (D / 8) >= (1LL << 31) || B > 65535) fail(LB_ERR_UNSUPPORTED, "attention backward: sequence x heads or batch too large for the delta kernel's grid");
     int n_shift = -1;
     for (int k = 0; k < 31; k++)
         if ((1LL << k) == N) n_shift = k;
     const unsigned blocks = (unsigned)((S * N * (D / 8) + 255) / 256);
-    launch_overlapped(attention_delta, dim3(blocks, (unsigned)B), dim3(256), 0, s, 0, (const __nv_bfloat16*)o.ptr, (const __nv_bfloat16*)d_o.ptr, delta,
+    launch_overlapped(attention_delta, dim3(blocks, (unsigned)B), dim3(256), 0, s, 0, (const __nv_bfloat16*)o.ptr, (const __nv_bfloat16*)d_o.ptr, delta, zeros,
                       (int)S, (int)N, (int)D, n_shift, o.stride[0], o.stride[1], o.stride[2], d_o.stride[0], d_o.stride[1], d_o.stride[2]);
 }
 
@@ -613,11 +619,16 @@ void attention_bwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor
     check_dense(delta, LB_F32, {B, N, Sq}, "attention delta");
     driver();
     cudaStream_t s = (cudaStream_t)stream;
+    const bool atomic = dq_acc && attention_bwd_atomic_supported(q, dq);
+    if (atomic) {
+        check_dense(*dq_acc, LB_F32, {B, Sq, N, D}, "attention dQ accumulator");
+        if (((uintptr_t)dq_acc->ptr & 15) != 0) fail(LB_ERR_UNSUPPORTED, "attention backward: the dQ accumulator must be 16-byte aligned");
+    }
     if (Sq > 0) {
         if (o.stride[0] % 8 || o.stride[1] % 8 || o.stride[2] % 8 || d_o.stride[0] % 8 || d_o.stride[1] % 8 || d_o.stride[2] % 8 ||
             ((uintptr_t)o.ptr & 15) || ((uintptr_t)d_o.ptr & 15))
             fail(LB_ERR_UNSUPPORTED, "attention backward: o and dO rows must be 16-byte aligned");
-        launch_delta(o, d_o, (float*)delta.ptr, s);
+        launch_delta(o, d_o, (float*)delta.ptr, atomic ? (float*)dq_acc->ptr : nullptr, s);
     }
     BwdArgs a{};
     a.B = (int)B, a.N = (int)N, a.Nkv = (int)Nkv, a.Sq = (int)Sq, a.Sk = (int)Sk;
@@ -630,8 +641,7 @@ void attention_bwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor
     kv.out_b = dv.ptr, kv.b_sb = dv.stride[0], kv.b_ss = dv.stride[1], kv.b_sn = dv.stride[2];
     qq.out_a = dq.ptr, qq.a_sb = dq.stride[0], qq.a_ss = dq.stride[1], qq.a_sn = dq.stride[2];
     if (Sk == 0 || Sq == 0) fail(LB_ERR_UNSUPPORTED, "attention backward: empty sequences");
-    if (dq_acc && attention_bwd_atomic_supported(q, dq)) {
-        check_dense(*dq_acc, LB_F32, {B, Sq, N, D}, "attention dQ accumulator");
+    if (atomic) {
         attention_bwd_atomic_launch(desc, attention_map_rows(k, "key", 128), attention_map_rows(v, "value", 128),
                                     attention_map_rows(q, "query", 128), attention_map_rows(d_o, "dO", 128), q, k, a.lse, a.delta, (float*)dq_acc->ptr, dq, dk, dv, s);
         return;
@@ -768,7 +778,7 @@ void attention_bwd_static(const lb_attn_desc& desc, const lb_tensor& q, const lb
         fail(LB_ERR_UNSUPPORTED, "lb_attention_bwd_static: o and dO rows must be 16-byte aligned");
     const StaticSetup& st = static_setup();
     cudaStream_t s = (cudaStream_t)stream;
-    launch_delta(o, d_o, st.delta, s);
+    launch_delta(o, d_o, st.delta, nullptr, s);
     BwdArgs a{};
     a.B = (int)B, a.N = (int)N, a.Nkv = (int)Nkv, a.Sq = (int)Sq, a.Sk = (int)Sk;
     a.causal = desc.causal, a.causal_offset = desc.causal_offset;

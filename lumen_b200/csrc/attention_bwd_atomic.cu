@@ -434,21 +434,21 @@ attention_bwd_atomic_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     }
 }
 
-// dq[b, s, n, :] = bf16(acc[b, s, n, :]): 8 values (32 bytes in, 16 out) per thread; the accumulator is dense, dq a view.
-__global__ void __launch_bounds__(256) attention_dq_round(const float* __restrict__ acc, uint16_t* __restrict__ dq, long long rows, int N,
-                                                           long long sb_rows, long long q_sb, long long q_ss, long long q_sn) {
+// dq[b, s, n, :] = bf16(acc[b, s, n, :]): 8 values (32 bytes in, 16 out) per thread; the accumulator is dense, dq a view. One grid row per
+// batch entry and 32-bit indices, as attention_delta has them.
+__global__ void __launch_bounds__(256) attention_dq_round(const float* __restrict__ acc, uint16_t* __restrict__ dq, unsigned rows, unsigned N, int n_shift,
+                                                           long long q_sb, long long q_ss, long long q_sn) {
     grid_wait(acc);
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long r = t >> 3;  // (b, s, n) row of 64 values
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned r = t >> 3;  // (s, n) row of 64 values of this batch entry
     const int part = (int)(t & 7);
     if (r >= rows) return;
-    const float4 a = __ldg((const float4*)(acc + r * D + part * 8)), b = __ldg((const float4*)(acc + r * D + part * 8 + 4));
-    const long long bs = r / N;
-    const int n = (int)(r - bs * N);
-    const long long bi = bs / sb_rows, s = bs - bi * sb_rows;
+    const long long at = ((long long)blockIdx.y * rows + r) * D + part * 8;
+    const float4 a = __ldg((const float4*)(acc + at)), b = __ldg((const float4*)(acc + at + 4));
+    const unsigned s = n_shift >= 0 ? r >> n_shift : r / N, n = r - s * N;
     __nv_bfloat162 h0 = __floats2bfloat162_rn(a.x, a.y), h1 = __floats2bfloat162_rn(a.z, a.w);
     __nv_bfloat162 h2 = __floats2bfloat162_rn(b.x, b.y), h3 = __floats2bfloat162_rn(b.z, b.w);
-    uint16_t* out = dq + bi * q_sb + s * q_ss + (long long)n * q_sn + part * 8;
+    uint16_t* out = dq + blockIdx.y * q_sb + s * q_ss + n * q_sn + part * 8;
     *(uint4*)out = make_uint4(*(uint32_t*)&h0, *(uint32_t*)&h1, *(uint32_t*)&h2, *(uint32_t*)&h3);
 }
 
@@ -460,7 +460,7 @@ bool attention_bwd_atomic_supported(const lb_tensor& q, const lb_tensor& dq) {
 
 size_t attention_bwd_atomic_scratch_bytes(const lb_tensor& q) { return (size_t)q.shape[0] * q.shape[1] * q.shape[2] * q.shape[3] * 4; }
 
-// The single-kernel backward over operands already validated by attention_bwd's caller; `delta` has been computed.
+// The single-kernel backward over operands already validated by attention_bwd; `delta` has been computed and `dq_acc` cleared.
 namespace {
 // 4-d map over the dense float32 accumulator [B, Sq, N, 64]: boxes of 32 columns x 128 query rows, 128-byte swizzle
 CUtensorMap make_acc_map(float* acc, long long B, long long Sq, long long N) {
@@ -494,13 +494,14 @@ void attention_bwd_atomic_launch(const lb_attn_desc& desc, const CUtensorMap& mk
                                         "budgets assume %d", regs, kLaunchRegs));
     if (first_use_on_device((const void*)attention_bwd_atomic_kernel))
         LB_CUDA(cudaFuncSetAttribute(attention_bwd_atomic_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    LB_CUDA(cudaMemsetAsync(dq_acc, 0, (size_t)B * Sq * N * D * 4, s));
     dim3 grid((unsigned)((Sk + BR - 1) / BR), (unsigned)Nkv, (unsigned)B);
-    if (((uintptr_t)dq_acc & 15) != 0) fail(LB_ERR_UNSUPPORTED, "attention backward: the dQ accumulator must be 16-byte aligned");
     launch_overlapped(attention_bwd_atomic_kernel, grid, dim3(kThreads), kSmemBytes, s, 0, mk, mv, mq, mdo, make_acc_map(dq_acc, B, Sq, N), a);
-    const long long rows = B * Sq * N;
-    launch_overlapped(attention_dq_round, dim3((unsigned)((rows * 8 + 255) / 256)), dim3(256), 0, s, 0, dq_acc, (uint16_t*)dq.ptr, rows, (int)N, Sq, dq.stride[0],
-                      dq.stride[1], dq.stride[2]);
+    const long long rows = Sq * N;  // rows * 8 < 2^31 and B <= 65535: checked for attention_delta
+    int n_shift = -1;
+    for (int i = 0; i < 31; i++)
+        if ((1LL << i) == N) n_shift = i;
+    launch_overlapped(attention_dq_round, dim3((unsigned)((rows * 8 + 255) / 256), (unsigned)B), dim3(256), 0, s, 0, dq_acc, (uint16_t*)dq.ptr, (unsigned)rows,
+                      (unsigned)N, n_shift, dq.stride[0], dq.stride[1], dq.stride[2]);
 }
 
 }  // namespace lb
