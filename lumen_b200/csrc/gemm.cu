@@ -800,10 +800,8 @@ int gemm_splits(long long M, long long N, long long K, long long batch, int sms)
 // better. The line is one CTA per SM: with no more tiles than SMs, ranges are doubled while they still have an SM each and
 // two 64-wide blocks of K, and once more, two CTAs to an SM, where a range would be longer than 64 blocks. Measured (us, large
 // tiles -> these), bfloat16: 64^3 8.2 -> 6.2, 512^3 13.5 -> 8.5, 200 x 4096 K 1024 16.4 -> 11.5, 200 x 1024 K 4096 24.6 -> 12.3
-// (4 ranges), 1000^3 18.5 -> 12.3, 128 x 8192 K 8192 49 -> 35, 1024 x 1024 K 8192 35 -> 28 (39 with one range). Beyond the line, two CTAs to an SM,
-// narrow tiles are still the better ones for up to two an SM and 32 blocks of K where the large ones are CTA pairs' (46 shapes: 0.62 - 1.01 of
-// the time; 384 x 4096 K 1024 9.8 -> 8.2, 176 x 7040 K 512 7.5 -> 6.0, 200 x 4896 K 2048 14.5 -> 12.8), but not for K of 3072 and more (up to
-// 1.03), not against the one-CTA kernel (up to 1.66: 20 x 13752 K 1024 10.1 -> 16.7) and not in greater number (up to 1.7).
+// (4 ranges), 1000^3 18.5 -> 12.3, 128 x 8192 K 8192 49 -> 35, 1024 x 1024 K 8192 35 -> 28 (39 with one range); beyond the line
+// 4096 x 1024 K 200 12.3 -> 16.4, 700 x 4096 K 1024 16.4 -> 20.5, 2048^3 22.6 -> 32.7.
 // Where scratch lets large tiles cut K into `large_split` ranges, ranges that would be 64 blocks and longer with one CTA to an SM may go
 // there, since a narrow tile fetches twice the bytes per product: 1024 x 1024 (us, these -> large) K 16384 43.7 -> 32.7, 8192 29.0 -> 23.5,
 // 4096 22.1 -> 17.9, 768 x 768 x 8192 20.8 -> 16.8, 768 x 1024 x 16384 41.6 -> 26.7; but 32 blocks: 512 x 512 x 8192 14.6 -> 15.7,
@@ -815,7 +813,7 @@ int gemm_splits(long long M, long long N, long long K, long long batch, int sms)
 // 26.3, 384 x 1536 x 8192 18.4 -> 21.6, on the one-CTA kernel 128 x 9216 x 4096 23.2 -> 27.9, 16 x 9216 x 4096 16.4 -> 19.3.
 int gemm_small_splits(long long M, long long N, long long K, long long batch, int sms, int large_split) {
     const long long tiles = (M + 127) / 128 * ((N + 63) / 64) * batch, total_kb = (K + BK - 1) / BK;
-    if (tiles > sms) return M > 128 && tiles <= 2LL * sms && total_kb <= 32 ? 1 : 0;
+    if (tiles > sms) return 0;
     int s = 1;
     while (s < 8 && tiles * 2 * s <= sms && total_kb >= 4 * s) s *= 2;
     const bool long_ranges = total_kb >= 64 * s;

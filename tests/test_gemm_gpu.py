@@ -412,18 +412,3 @@ def test_clusters_beyond_what_is_resident_at_once(cuda, fits, tiles, dtype):
     for t in tiles:
         assert torch.equal(product(t)[:, : 64 * fits], few)
     device_status()
-
-
-@pytest.mark.parametrize("m, n", [(129, 64 * 148), (129, 64 * 74 + 8), (300, 64 * 98 + 56), (136, 64 * 148 + 64), (128, 64 * 149)])  # two an SM: 296 tiles
-@pytest.mark.parametrize("k", [64, 200, 2048, 2056])  # 32 blocks of K and one more
-@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-def test_more_narrow_tiles_than_sms(cuda, m, n, k, dtype):
-    """Both sides of the line up to which narrow tiles run two to an SM, within the K-order bound of float64."""
-    gen = torch.Generator(device=cuda).manual_seed(n + k)
-    a = torch.randn(m, k, generator=gen, device=cuda).bfloat16()
-    b = torch.randn(n, k, generator=gen, device=cuda).bfloat16().t()
-    out = gemm(a, b, torch.full((m, n), float("nan"), dtype=getattr(torch, dtype), device=cuda))
-    want, size = a.double() @ b.double(), a.double().abs() @ b.double().abs()
-    # 64 * 2^-24 of the sum of magnitudes for the order of K additions, the result's rounding
-    assert ((out.double() - want).abs() <= 64 * 2.0**-24 * size + (2.0**-8 * want.abs() if dtype == "bfloat16" else 0)).all()
-    device_status()
