@@ -8,10 +8,6 @@
 // cluster writing its share of the rows in whole 128-byte lines.
 #include <cuda_fp16.h>
 
-#include <map>
-#include <mutex>
-#include <utility>
-
 #include "gemm.h"
 #include "launch.cuh"
 #include "sm100.cuh"
@@ -247,41 +243,12 @@ static void launch_small(const CUtensorMap& map_a, const CUtensorMap& map_b, con
     launch_overlapped(gemm_small_kernel<STAGES, EPI, DT>, dim3((unsigned)((long long)p.tiles_m * p.tiles_n * batch * p.splits)), dim3(kThreads), smem_bytes(STAGES), s,
                       (unsigned)p.splits, map_a, map_b, p);
 }
-// Clusters of `splits` CTAs with eight stages that can be resident on the current device at once (asked of the runtime once per device):
-// a cluster stays inside a group of SMs, so fewer than SMs / splits.
-static int resident_clusters(int splits) {
-    static std::mutex mutex;
-    static std::map<std::pair<int, int>, int> cache;
-    const int device = device_info().device;
-    std::lock_guard<std::mutex> lock(mutex);
-    auto it = cache.find({device, splits});
-    if (it != cache.end()) return it->second;
-    const auto kernel = gemm_small_kernel<8, EPI_NONE, LB_BF16>;  // all take the same threads, registers and shared memory
-    LB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(8)));
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)splits, attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)splits), cfg.blockDim = dim3(kThreads), cfg.dynamicSmemBytes = smem_bytes(8), cfg.attrs = attr, cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        n = 0;
-    }
-    return cache[{device, splits}] = n;
-}
-
 void gemm_small(const CUtensorMap& map_a, const CUtensorMap& map_b, SmallGemmArgs p, int batch, int sms, cudaStream_t s) {
     p.tiles_m = (p.M + BM - 1) / BM, p.tiles_n = (p.N + BN - 1) / BN;
     const int per_line = p.d_bf16 || p.d_f16 ? 8 : 4;
     p.whole = (uintptr_t)p.d % 16 == 0 && p.ldd % per_line == 0 && p.d_batch_stride % per_line == 0 &&
               (p.epilogue < EPI_ADD || ((uintptr_t)p.aux % 16 == 0 && p.ld_aux % 8 == 0 && p.aux_batch_stride % 8 == 0));
-    // Eight stages where every cluster finds room at once: fifteen of eight CTAs and 33 of four do, not the 18 and 37 that 148 SMs would
-    // hold. One that waits for another's end doubles the time; with four stages two CTAs share an SM. us, before -> after:
-    // 36 x 1152 x 4608 (18 clusters of eight) 12.5 -> 8.5, 64 x 1024 x 4096 (16) 12.8 -> 8.8, 200 x 1088 x 4096 (34 of four) 15.4 -> 10.5,
-    // 36 x 2304 x 2048 (36) 11.7 -> 7.8.
-    const long long clusters = (long long)p.tiles_m * p.tiles_n * batch;
-    const bool one_wave = clusters * p.splits <= sms && (p.splits < 4 || clusters <= resident_clusters(p.splits));
+    const bool one_wave = (long long)p.tiles_m * p.tiles_n * batch * p.splits <= sms;
     with_epilogue(p.epilogue, p.d_bf16 ? LB_BF16 : p.d_f16 ? LB_F16 : LB_F32, [&](auto epi, auto dt) {
         if (one_wave) launch_small<8, decltype(epi)::value, decltype(dt)::value>(map_a, map_b, p, batch, s);
         else launch_small<4, decltype(epi)::value, decltype(dt)::value>(map_a, map_b, p, batch, s);

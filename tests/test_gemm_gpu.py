@@ -393,22 +393,3 @@ def test_a_float32_product_that_reads_anothers_result_comes_after_it(cuda):
     got = torch.empty_like(second)
     products_plan([(64, 64, 64)] * 3).run(x, [x[2], got, x[3]])
     assert torch.equal(x[2], first) and torch.equal(got, second) and torch.equal(x[3], third)
-
-
-@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-@pytest.mark.parametrize("fits, tiles", [(15, [16, 17, 18]), (33, [34, 36, 37])])  # eight and four CTAs a cluster
-def test_clusters_beyond_what_is_resident_at_once(cuda, fits, tiles, dtype):
-    """Narrow tiles with K cut over a cluster, as many as find room at once with eight stages and more, which take four: a tile's bits
-    do not depend on how many others there are."""
-    m, k = 100, 4096
-    gen = torch.Generator(device=cuda).manual_seed(fits)
-    a = torch.randn(m, k, generator=gen, device=cuda).bfloat16()
-    b = torch.randn(64 * max(tiles), k, generator=gen, device=cuda).bfloat16().t()
-    product = lambda t: gemm(a, b[:, : 64 * t], torch.empty(m, 64 * t, dtype=getattr(torch, dtype), device=cuda))
-    few = product(fits)
-    want, size = a.double() @ b[:, : 64 * fits].double(), a.double().abs() @ b[:, : 64 * fits].double().abs()
-    # 64 * 2^-24 of the sum of magnitudes for the order of K additions, the result's rounding
-    assert ((few.double() - want).abs() <= 64 * 2.0**-24 * size + (2.0**-8 * want.abs() if dtype == "bfloat16" else 0)).all()
-    for t in tiles:
-        assert torch.equal(product(t)[:, : 64 * fits], few)
-    device_status()
