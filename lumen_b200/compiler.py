@@ -362,34 +362,24 @@ class Lowering:
     def dot_fusion_epilogue(body: G.Graph):
         """The tail of a `dot_general` fusion body as a GEMM epilogue: `(code, body input of the epilogue operand or
         None)`. 1: `max(product, 0)`; 2: `other + product`; 3: `select(0 < other, product, 0)` (a relu's backward
-        with `other` the relu's output); 4: `product * select(0 < other, 1, select(other == 0, 0.5, 0))` (the backward of
-        `max(other, 0)`); 5: two outputs, the product and `max(product, 0)`. Anything else has no kernel."""
+        with `other` the relu's output). Anything else has no kernel."""
         dots = [b for b in body.nodes if b.op == "dot_general"]
-        beside = len(dots) == 1 and len(body.outputs) == 2 and body.outputs[0] == dots[0].output
-        if len(dots) != 1 or (len(body.outputs) != 1 and not beside):
-            raise NotImplementedError("dot_general fusions are lowered for one product and one output, or its relu as a second one")
+        if len(dots) != 1 or len(body.outputs) != 1:
+            raise NotImplementedError("dot_general fusions are lowered for one product and one output")
         product = dots[0].output
         by_output = {b.output: b for b in body.nodes}
-        def number(value):  # a number in a traced body, "i:.." / "f:.." text in a parsed one
+        def is_zero(value):  # a number in a traced body, "i:.." / "f:.." text in a parsed one
             if isinstance(value, str):
                 kind, _, text = value.partition(":")
-                return float.fromhex(text) if kind == "f" else int(text)
-            return value
+                return (float.fromhex(text) if kind == "f" else int(text)) == 0
+            return value == 0
 
-        fills = {b.output: number(b.params.get("fill_value")) for b in body.nodes if b.op == "full"}
-        constants = {b.output: fills[b.inputs[0]] for b in body.nodes if b.op == "broadcast_in_dim" and b.inputs[0] in fills}
-        zeros = {v for v, c in constants.items() if c == 0}
-        tail = by_output.get(body.outputs[-1])
+        fills = {b.output for b in body.nodes if b.op == "full" and is_zero(b.params.get("fill_value"))}
+        zeros = {b.output for b in body.nodes if b.op == "broadcast_in_dim" and b.inputs[0] in fills}
+        tail = by_output.get(body.outputs[0])
         used = {dots[0].output: dots[0]}
-
-        def node(value, op):
-            found = by_output.get(value)
-            return found if found is not None and found.op == op else None
-
         if tail is not None and tail.op == "max" and product in tail.inputs and any(i in zeros for i in tail.inputs):
-            code, other = 5 if beside else 1, None
-        elif beside:
-            raise NotImplementedError("dot_general fusions are lowered for one product and one output, or its relu as a second one")
+            code, other = 1, None
         elif tail is not None and tail.op == "add" and product in tail.inputs:
             (other,) = [i for i in tail.inputs if i != product] or [None]
             code = 2
@@ -399,18 +389,8 @@ class Lowering:
                 raise NotImplementedError("dot_general fusion: the select's condition is not `0 < operand`")
             code, other = 3, cond.inputs[1]
             used[cond.output] = cond
-        elif tail is not None and tail.op == "mul" and product in tail.inputs:
-            outer = next((s for i in tail.inputs if (s := node(i, "select")) is not None), None)
-            inner = node(outer.inputs[2], "select") if outer is not None else None
-            above = node(outer.inputs[0], "lt") if outer is not None else None
-            equal = node(inner.inputs[0], "eq") if inner is not None else None
-            if (above is None or equal is None or above.inputs[0] not in zeros or constants.get(outer.inputs[1]) != 1 or constants.get(inner.inputs[1]) != 0.5
-                    or inner.inputs[2] not in zeros or not any(i in zeros for i in equal.inputs) or above.inputs[1] not in equal.inputs):
-                raise NotImplementedError("dot_general fusion: the factor is not what a maximum with zero passes back")
-            code, other = 4, above.inputs[1]
-            used.update((x.output, x) for x in (outer, inner, above, equal))
         else:
-            raise NotImplementedError("dot_general fusions are lowered for a relu, an add, a relu-backward select or a maximum's backward after the product")
+            raise NotImplementedError("dot_general fusions are lowered for a relu, an add or a relu-backward select after the product")
         used[tail.output] = tail
         for b in body.nodes:
             if b.output not in used and b.op not in ("full", "broadcast_in_dim"):
@@ -439,8 +419,7 @@ class Lowering:
             raise NotImplementedError("dot_general fusion: the epilogue operand must be row-major and shaped like the product")
         for x in (a, b, out, *([scratch] if scratch else []), *([aux] if aux else [])):
             self.touch(x)
-        label = {0: "dot_general", 1: "dot_general_relu", 2: "dot_general_add", 3: "dot_general_relu_backward",
-                 4: "dot_general_max_backward", 5: "dot_general_relu_beside"}[code]
+        label = {0: "dot_general", 1: "dot_general_relu", 2: "dot_general_add", 3: "dot_general_relu_backward"}[code]
         self.steps.append(("gemm", label, (a, b, out, code, scratch, aux)))
         self.views[out_value] = out
 
@@ -499,11 +478,6 @@ class Lowering:
             dot, code, other = self.dot_fusion_epilogue(body)
             operands = [n.inputs[body.inputs.index(i)] for i in dot.inputs]
             aux_value = n.inputs[body.inputs.index(other)] if other is not None else None
-            if code == 5:  # the product's relu, written beside it
-                aux_value = outs[1]
-                if aux_value is None:
-                    raise NotImplementedError("dot_general fusion: the relu beside the product is not read")
-                self.views[aux_value] = self.fresh(aux_value)
             self.lower_dot(dot, n, n.output, code, operands=operands, aux_value=aux_value)
             return
         found = n.params.get("attention")  # set by the attention pass: roles of every operand's dimensions, scale, mask

@@ -591,51 +591,34 @@ struct Lowering {
         }
         if (!dot) fail(LB_ERR_INVALID, "lb_compile: a dot_general fusion without a dot_general");
         // tails (the GEMM's epilogues): none; 1 max(product, 0); 2 other + product; 3 select(0 < other, product, 0), a relu's
-        // backward with `other` the relu's output; 4 product * select(0 < other, 1, select(other == 0, 0.5, 0)), the backward of
-        // max(other, 0); 5 the product and max(product, 0) beside it. Constants are broadcast to the product's shape.
-        std::map<int, double> fills, constants;
+        // backward with `other` the relu's output. Constants are zeros broadcast to the product's shape.
+        std::set<int> zero_fills, zeros;
         std::map<int, const Node*> by_output;
         for (const Node& bn : body.nodes) {
             by_output[bn.output] = &bn;
             if (bn.op == "full") {
                 const std::string& c = bn.attr("fill_value");
-                fills[bn.output] = std::strtod(c.c_str() + 2, nullptr);
+                if (c == "i:0" || std::strtod(c.c_str() + 2, nullptr) == 0.0) zero_fills.insert(bn.output);
             }
         }
         for (const Node& bn : body.nodes)
-            if (bn.op == "broadcast_in_dim" && fills.count(bn.inputs.at(0))) constants[bn.output] = fills[bn.inputs[0]];
-        auto is = [&](int value, double c) { return constants.count(value) && constants[value] == c; };
-        auto node = [&](int value, const char* op) -> const Node* { return by_output.count(value) && by_output[value]->op == op ? by_output[value] : nullptr; };
+            if (bn.op == "broadcast_in_dim" && zero_fills.count(bn.inputs.at(0))) zeros.insert(bn.output);
         int other = -1;
         std::set<const Node*> used = {dot};
-        const Node* tail = by_output.count(body.outputs.back()) ? by_output[body.outputs.back()] : nullptr;
-        const bool beside = body.outputs.size() == 2 && body.outputs[0] == dot->output;
-        if (body.outputs.size() != 1 && !beside) fail(LB_ERR_UNSUPPORTED, "lb_compile: a dot_general fusion with outputs other than one, or the product and its relu");
+        const Node* tail = by_output.count(body.outputs.at(0)) ? by_output[body.outputs.at(0)] : nullptr;
         auto has = [](const std::vector<int>& v, int x) { return std::find(v.begin(), v.end(), x) != v.end(); };
         if (tail == dot) {
             epilogue = 0;
-        } else if (tail && tail->op == "max" && has(tail->inputs, dot->output) && (is(tail->inputs[0], 0) || is(tail->inputs[1], 0))) {
-            epilogue = beside ? 5 : 1;
-        } else if (beside) {
-            fail(LB_ERR_UNSUPPORTED, "lb_compile: a dot_general fusion with outputs other than one, or the product and its relu");
+        } else if (tail && tail->op == "max" && has(tail->inputs, dot->output) && (zeros.count(tail->inputs[0]) || zeros.count(tail->inputs[1]))) {
+            epilogue = 1;
         } else if (tail && tail->op == "add" && has(tail->inputs, dot->output)) {
             epilogue = 2, other = tail->inputs[0] == dot->output ? tail->inputs[1] : tail->inputs[0];
-        } else if (tail && tail->op == "select" && tail->inputs.at(1) == dot->output && is(tail->inputs.at(2), 0)) {
-            const Node* cond = node(tail->inputs[0], "lt");
-            if (!cond || !is(cond->inputs.at(0), 0))
+        } else if (tail && tail->op == "select" && tail->inputs.at(1) == dot->output && zeros.count(tail->inputs.at(2))) {
+            const Node* cond = by_output.count(tail->inputs[0]) ? by_output[tail->inputs[0]] : nullptr;
+            if (!cond || cond->op != "lt" || !zeros.count(cond->inputs.at(0)))
                 fail(LB_ERR_UNSUPPORTED, "lb_compile: dot_general fusion: the select's condition is not `0 < operand`");
             epilogue = 3, other = cond->inputs.at(1);
             used.insert(cond);
-        } else if (tail && tail->op == "mul" && has(tail->inputs, dot->output)) {
-            const Node* outer = node(tail->inputs[0] == dot->output ? tail->inputs[1] : tail->inputs[0], "select");
-            const Node* inner = outer ? node(outer->inputs.at(2), "select") : nullptr;
-            const Node* above = outer ? node(outer->inputs[0], "lt") : nullptr;
-            const Node* equal = inner ? node(inner->inputs.at(0), "eq") : nullptr;
-            if (!above || !equal || !is(above->inputs.at(0), 0) || !is(outer->inputs.at(1), 1) || !is(inner->inputs.at(1), 0.5) || !is(inner->inputs.at(2), 0) ||
-                !(is(equal->inputs.at(0), 0) || is(equal->inputs.at(1), 0)) || !has(equal->inputs, above->inputs.at(1)))
-                fail(LB_ERR_UNSUPPORTED, "lb_compile: dot_general fusion: the factor is not what a maximum with zero passes back");
-            epilogue = 4, other = above->inputs[1];
-            used.insert({outer, inner, above, equal});
         } else {
             fail(LB_ERR_UNSUPPORTED, format("lb_compile: primitive `%s` after the product of a dot_general fusion has no epilogue", tail ? tail->op.c_str() : "?"));
         }
@@ -651,15 +634,13 @@ struct Lowering {
         };
         View aux;
         if (other >= 0) aux = operand(other);  // fails when the epilogue operand is computed inside the fusion
-        static const char* const kNames[] = {"dot_general", "dot_general_relu", "dot_general_add", "dot_general_relu_backward", "dot_general_max_backward", "dot_general_relu_beside"};
-        const TensorType& t = body.type(body.outputs.at(0));
-        const int second = beside ? fusion_outputs(n, body).at(1) : -1;
-        emit_gemm(*dot, n.output, t, epilogue, kNames[epilogue], operand, other >= 0 ? &aux : nullptr, beside, second);
+        static const char* const kNames[] = {"dot_general", "dot_general_relu", "dot_general_add", "dot_general_relu_backward"};
+        emit_gemm(*dot, n.output, body.type(body.outputs.at(0)), epilogue, kNames[epilogue], operand, other >= 0 ? &aux : nullptr);
     }
 
     template <class Operand>
     void emit_gemm(const Node& dot_node, int result, const TensorType& t, int epilogue, const std::string& label, Operand operand,
-                   const View* aux = nullptr, bool beside = false, int second = -1) {
+                   const View* aux = nullptr) {
         const Node* dot = &dot_node;
         if (!dot->ints("lhs_batch").empty() || dot->ints("lhs_contracting").size() != 1 || dot->ints("rhs_contracting").size() != 1)
             fail(LB_ERR_UNSUPPORTED, "lb_compile: dot_general with batch dimensions or several contracting dimensions");
@@ -685,12 +666,6 @@ struct Lowering {
         }
         View d = fresh(t.dtype, t.shape, result);
         views[result] = d;
-        View relu;
-        if (beside) {
-            relu = fresh(t.dtype, t.shape, second);
-            if (second >= 0) views[second] = relu;
-            aux = &relu;
-        }
         const lb_tensor operands[2] = {descriptor(a), descriptor(b)};
         const size_t sb = lb_gemm_operands_scratch_bytes(&operands[0], &operands[1]);
         std::ostringstream s;

@@ -53,7 +53,7 @@ struct GemmArgs {
     int in_bf16;          // operands bfloat16 (else float16): the MMA's operand format
     long long ldd, d_batch_stride;
     int epilogue;
-    void* aux;            // operand (EPI_RELU_BESIDE: second result) of an epilogue: same dtype as the output, row-major [batch, M, N] view
+    const void* aux;      // EPI_ADD / EPI_MASK operand: same dtype as the output, row-major [batch, M, N] view
     long long ld_aux, aux_batch_stride;
     int* status;          // device word: set to LB_ERR_TIMEOUT when a bounded wait gave up
     int tiles_m, tiles_n, group_m;
@@ -78,12 +78,11 @@ __device__ __forceinline__ int tile_coords(const GemmArgs& p, int unit, int& b, 
     return split;
 }
 
-// Whether the rows of the result, and of the one beside it, start and go on in whole 16-byte pieces.
-template <int EPI, int DT>
+// Whether the rows of the result start and go on in whole 16-byte pieces.
+template <int DT>
 __device__ __forceinline__ bool whole_lines(const GemmArgs& p) {
     constexpr int per = DT == LB_F32 ? 4 : 8;
-    return p.ldd % per == 0 && p.d_batch_stride % per == 0 && ((uintptr_t)p.d & 15) == 0 &&
-           (EPI != EPI_RELU_BESIDE || (p.ld_aux % 8 == 0 && p.aux_batch_stride % 8 == 0 && ((uintptr_t)p.aux & 15) == 0));
+    return p.ldd % per == 0 && p.d_batch_stride % per == 0 && ((uintptr_t)p.d & 15) == 0;
 }
 
 // Drains 128 accumulator columns (this warp's half of a 256-wide tile) of the thread's row from tensor memory and
@@ -141,7 +140,6 @@ __device__ __forceinline__ void drain_tile(const GemmArgs& p, uint32_t tbase, in
                 }
                 if constexpr (DT != LB_F32) {
                     uint16_t* out = (uint16_t*)p.d + row_off + col0;
-                    uint16_t* beside = (uint16_t*)p.aux + aux_off + col0;
                     if (full_chunk && vec_ok) {
 #pragma unroll
                         for (int j = 0; j < 32; j += 8) {
@@ -150,20 +148,12 @@ __device__ __forceinline__ void drain_tile(const GemmArgs& p, uint32_t tbase, in
                             for (int q = 0; q < 4; q++) w[q] = pair16<DT>(__uint_as_float(v[j + 2 * q]), __uint_as_float(v[j + 2 * q + 1]));
                             if (coalesced) packed[h * 4 + j / 8] = make_uint4(w[0], w[1], w[2], w[3]);
                             else *(uint4*)(out + j) = make_uint4(w[0], w[1], w[2], w[3]);
-                            if (EPI == EPI_RELU_BESIDE && !coalesced) {
-#pragma unroll
-                                for (int q = 0; q < 4; q++) w[q] = relu_pair(w[q], DT == LB_BF16);
-                                *(uint4*)(beside + j) = make_uint4(w[0], w[1], w[2], w[3]);
-                            }
                         }
                     } else {
 #pragma unroll
                         for (int j = 0; j < 32; j++) {  // unrolled with a predicate: keeps the fragment in registers
                             const uint16_t x16 = to16<DT>(__uint_as_float(v[j]));
-                            if (col0 + j < p.N) {
-                                out[j] = x16;
-                                if (EPI == EPI_RELU_BESIDE) beside[j] = relu_one(x16, DT == LB_BF16);
-                            }
+                            if (col0 + j < p.N) out[j] = x16;
                         }
                     }
                 } else {
@@ -185,17 +175,9 @@ __device__ __forceinline__ void drain_tile(const GemmArgs& p, uint32_t tbase, in
                 store_rows_coalesced<8>(stage, packed, (uint8_t*)((float*)p.d + (row_off - (long long)lane * p.ldd) + col0), p.ldd * 4,
                                         p.M - (row - lane), lane);
         }
-        if (coalesced) {  // rows past M hold nothing and are not written
+        if (coalesced)  // rows past M hold nothing and are not written
             store_rows_coalesced<8>(stage, packed, (uint8_t*)((uint16_t*)p.d + (row_off - (long long)lane * p.ldd) + col_base + c2 * 64),
                                     p.ldd * 2, p.M - (row - lane), lane);
-            if constexpr (EPI == EPI_RELU_BESIDE) {
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                    packed[j] = relu_16_bytes(packed[j], DT == LB_BF16);
-                store_rows_coalesced<8>(stage, packed, (uint8_t*)((uint16_t*)p.aux + (aux_off - (long long)lane * p.ld_aux) + col_base + c2 * 64),
-                                        p.ld_aux * 2, p.M - (row - lane), lane);
-            }
-        }
     }
 }
 
@@ -420,7 +402,7 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
         uint4* stage = (uint4*)(smem + STAGES * (kStageBytesA + kStageBytesB) + 256) + (warp - 2) * (kStageBytesPerWarp / 16);
         int local = 0;
         bool ok = true;
-        const bool vec_ok = EPI != EPI_PARTIAL && whole_lines<EPI, DT>(p);
+        const bool vec_ok = EPI != EPI_PARTIAL && whole_lines<DT>(p);
         for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x, local++) {
             const int buf = local & 1;
             const uint32_t use = (uint32_t)(local >> 1);
@@ -625,7 +607,7 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         uint4* stage = (uint4*)(smem + PSTAGES * (kPairStageBytesA + kPairStageBytesB) + 256) + (warp - 2) * (kStageBytesPerWarp / 16);
         int local = 0;
         bool ok = true;
-        const bool vec_ok = EPI != EPI_PARTIAL && whole_lines<EPI, DT>(p);
+        const bool vec_ok = EPI != EPI_PARTIAL && whole_lines<DT>(p);
         for (int unit = pair; unit < num_units && ok; unit += num_pairs, local++) {
             const int buf = local & 1;
             const uint32_t use = (uint32_t)(local >> 1);
@@ -699,7 +681,7 @@ __global__ void __launch_bounds__(256) splitk_reduce(const float* __restrict__ p
             }
         }
         const long long row = i / p.N, b = p.batch > 1 ? row / p.M : 0, r = row - b * p.M, c = i - row * p.N;
-        uint16_t* aux = (uint16_t*)p.aux + b * p.aux_batch_stride + r * p.ld_aux + c;
+        const uint16_t* aux = (const uint16_t*)p.aux + b * p.aux_batch_stride + r * p.ld_aux + c;
         __align__(8) uint16_t a16[W], out16[W];
         if (reads_aux(p.epilogue)) {
             if constexpr (VEC) *(uint2*)a16 = *(const uint2*)aux;
@@ -718,14 +700,8 @@ __global__ void __launch_bounds__(256) splitk_reduce(const float* __restrict__ p
         }
         const long long at = b * p.d_batch_stride + r * p.ldd + c;
         if (p.d_bf16 || p.d_f16) {
-            if constexpr (VEC) {
-                const uint2 w = make_uint2(out16[0] | (uint32_t)out16[1] << 16, out16[2] | (uint32_t)out16[3] << 16);
-                *(uint2*)((uint16_t*)p.d + at) = w;
-                if (p.epilogue == EPI_RELU_BESIDE) *(uint2*)aux = make_uint2(relu_pair(w.x, p.d_bf16), relu_pair(w.y, p.d_bf16));
-            } else {
-                ((uint16_t*)p.d)[at] = out16[0];
-                if (p.epilogue == EPI_RELU_BESIDE) *aux = relu_one(out16[0], p.d_bf16);
-            }
+            if constexpr (VEC) *(uint2*)((uint16_t*)p.d + at) = make_uint2(out16[0] | (uint32_t)out16[1] << 16, out16[2] | (uint32_t)out16[3] << 16);
+            else ((uint16_t*)p.d)[at] = out16[0];
         } else {
             if constexpr (VEC) *(float4*)((float*)p.d + at) = make_float4(acc[0], acc[1], acc[2], acc[3]);
             else ((float*)p.d)[at] = acc[0];
@@ -934,7 +910,7 @@ bool gemm_held(const lb_tensor& a_t, const lb_tensor& b_t, SimtProblem& q) {
 bool gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int epilogue, int kernel_choice, void* stream,
           void* scratch, size_t scratch_bytes, const lb_tensor* aux_t, const GemmTuning* tuning, SimtProblem* held) {
     View3 a = view3(a_t, "a"), b = view3(b_t, "b"), d = view3(d_t, "output");
-    if (epilogue < EPI_NONE || epilogue > EPI_RELU_BESIDE) fail(LB_ERR_INVALID, "gemm: unknown epilogue");
+    if (epilogue < EPI_NONE || epilogue > EPI_MASK) fail(LB_ERR_INVALID, "gemm: unknown epilogue");
     View3 aux{};
     if (epilogue >= EPI_ADD) {
         if (!aux_t || !aux_t->ptr) fail(LB_ERR_INVALID, "gemm: the add / mask epilogue needs its operand tensor");
@@ -1056,7 +1032,6 @@ extern "C" {
 int lb_gemm(const lb_tensor* a, const lb_tensor* b, const lb_gemm_out* out, const lb_gemm_cfg* cfg, void* stream) {
     return lb::guarded([&] {
         if (!a || !b || !out) lb::fail(LB_ERR_INVALID, "lb_gemm: null argument");
-        if (out->epilogue > LB_EPILOGUE_MASK_POSITIVE) lb::fail(LB_ERR_INVALID, "gemm: unknown epilogue");
         lb::GemmTuning tuning{cfg ? cfg->splits : 0, cfg ? cfg->group_m : 0};
         lb::gemm(*a, *b, out->product, out->epilogue, cfg ? cfg->kernel : 0, stream, cfg ? cfg->scratch : nullptr,
                  cfg ? cfg->scratch_bytes : 0, out->epilogue >= 2 ? &out->aux : nullptr, &tuning, nullptr);

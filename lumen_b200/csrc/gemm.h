@@ -10,33 +10,14 @@
 
 namespace lb {
 
-// EPI_ADD: out = round(round(acc) + aux); EPI_MASK: out = aux > 0 ? round(acc) : 0; EPI_GATE: out = round(round(acc) * (aux > 0 ? 1 :
-// aux == 0 ? 0.5 : 0)), what max(aux, 0) passes back - each exactly the primitives of the traced program (a rounded product followed by an
-// add / a select / a product), with `aux` a tensor shaped like the output. EPI_RELU_BESIDE: out = round(acc), and `aux` is written too:
-// max(out, 0), a NaN staying one. The last two are of plans alone (lb_gemm takes the others).
-// A relu that its own backward follows took two kernels of their own, bound by memory: one that read the product back and one that read the
-// second product and wrote it again. x + relu(x w1) w2 with its gradients, width 1024, bfloat16, us: 200 tokens 49.4 -> 47.5,
-// 2048 124.7 -> 120.4, 8192 397 -> 376; width 2048, 8192 tokens 1394 -> 1341.
-enum Epilogue : int { EPI_PARTIAL = -1 /* of a kernel: sums of a range of K */, EPI_NONE = 0, EPI_RELU = 1, EPI_ADD = 2, EPI_MASK = 3, EPI_GATE = 4, EPI_RELU_BESIDE = 5 };
+// EPI_ADD: out = round(round(acc) + aux); EPI_MASK: out = aux > 0 ? round(acc) : 0 - each exactly the two primitives
+// of the traced program (a rounded product followed by an add / a select), with `aux` a tensor shaped like the output
+enum Epilogue : int { EPI_PARTIAL = -1 /* of a kernel: sums of a range of K */, EPI_NONE = 0, EPI_RELU = 1, EPI_ADD = 2, EPI_MASK = 3 };
 #ifdef __CUDACC__
-__host__ __device__ constexpr bool reads_aux(int epilogue) { return epilogue >= EPI_ADD && epilogue <= EPI_GATE; }
+__host__ __device__ constexpr bool reads_aux(int epilogue) { return epilogue >= EPI_ADD; }
 // The second primitive on the rounded product.
 __device__ __forceinline__ float second_primitive(int epilogue, float product, float other) {
-    if (epilogue == EPI_ADD) return __fadd_rn(other, product);
-    if (epilogue == EPI_MASK) return other > 0.0f ? product : 0.0f;
-    return __fmul_rn(product, other > 0.0f ? 1.0f : other == 0.0f ? 0.5f : 0.0f);
-}
-// max(x, 0) of 16-bit elements by their bits (of two at a time), a NaN staying one.
-__device__ __forceinline__ uint32_t relu_pair(uint32_t w, bool bf16) {
-    if (bf16) {
-        const __nv_bfloat162 r = __hmax2_nan(*(const __nv_bfloat162*)&w, __floats2bfloat162_rn(0.0f, 0.0f));
-        return *(const uint32_t*)&r;
-    }
-    const __half2 r = __hmax2_nan(*(const __half2*)&w, __floats2half2_rn(0.0f, 0.0f));
-    return *(const uint32_t*)&r;
-}
-__device__ __forceinline__ uint4 relu_16_bytes(uint4 w, bool bf16) {
-    return make_uint4(relu_pair(w.x, bf16), relu_pair(w.y, bf16), relu_pair(w.z, bf16), relu_pair(w.w, bf16));
+    return epilogue == EPI_ADD ? __fadd_rn(other, product) : (other > 0.0f ? product : 0.0f);
 }
 // A 16-bit element's bits from and to float32.
 template <int DT>
@@ -57,7 +38,6 @@ __device__ __forceinline__ uint32_t pair16(float lo, float hi) {
         return *(const uint32_t*)&h;
     }
 }
-__device__ __forceinline__ uint16_t relu_one(uint16_t w, bool bf16) { return (uint16_t)relu_pair(w, bf16); }
 
 // Calls `launch` with the kernel's epilogue and type of the result as constants.
 template <class Launch>
@@ -71,8 +51,6 @@ void with_epilogue(int epilogue, int dtype, Launch launch) {
             switch (epilogue) {
                 case EPI_ADD: return launch(std::integral_constant<int, EPI_ADD>{}, dt);
                 case EPI_MASK: return launch(std::integral_constant<int, EPI_MASK>{}, dt);
-                case EPI_GATE: return launch(std::integral_constant<int, EPI_GATE>{}, dt);
-                case EPI_RELU_BESIDE: return launch(std::integral_constant<int, EPI_RELU_BESIDE>{}, dt);
             }
         }
         fail(LB_ERR_INVALID, "gemm: unknown epilogue");
@@ -90,7 +68,7 @@ struct SimtArgs {
     void* d;
     int d_dtype;
     int epilogue;
-    void* aux;  // operand (EPI_RELU_BESIDE: second result) of an epilogue: 16-bit, the output's dtype, rows ld_aux apart, batches aux_sb apart
+    const void* aux;  // EPI_ADD / EPI_MASK operand (16-bit, the output's dtype), rows ld_aux apart, batches aux_sb apart
     long long ld_aux, aux_sb;
     int a_vec, b_vec;  // groups of four elements along the operand's contiguous axis are aligned
 };
@@ -114,7 +92,7 @@ struct SmallGemmArgs {
     int d_bf16, d_f16;  // else float32
     long long ldd, d_batch_stride;
     int epilogue;
-    void* aux;
+    const void* aux;
     long long ld_aux, aux_batch_stride;
     int splits;  // CTAs of a cluster: 1, 2, 4 or 8, no more than the 64-wide blocks of K
     int* status;

@@ -164,20 +164,17 @@ __device__ __forceinline__ void simt_tile(const T* ab, const T* bb, const SimtAr
             if (gm >= p.M || gn >= p.N) continue;
             float x = acc[i][j];
             if (p.epilogue == EPI_RELU) x = fmaxf(x, 0.0f);
-            const long long at_aux = (long long)bz * p.aux_sb + (long long)gm * p.ld_aux + gn;
-            if (reads_aux(p.epilogue)) {  // the rounded product, then the second primitive on it (as the tensor-core kernels do)
-                const uint16_t a16 = ((const uint16_t*)p.aux)[at_aux];
+            if (p.epilogue >= EPI_ADD) {  // the rounded product, then the second primitive on it (as the tensor-core kernels do)
+                const uint16_t a16 = ((const uint16_t*)p.aux)[(long long)bz * p.aux_sb + (long long)gm * p.ld_aux + gn];
                 float prod, other;
                 if (p.d_dtype == LB_BF16) prod = __bfloat162float(__float2bfloat16_rn(x)), other = __uint_as_float((uint32_t)a16 << 16);
                 else prod = __half2float(__float2half_rn(x)), other = __half2float(__ushort_as_half(a16));
-                x = second_primitive(p.epilogue, prod, other);
+                x = p.epilogue == EPI_ADD ? __fadd_rn(other, prod) : (other > 0.0f ? prod : 0.0f);
             }
             long long at = (long long)bz * p.d_sb + (long long)gm * p.ldd + gn;
             if (p.d_dtype == LB_F32) ((float*)p.d)[at] = x;
             else if (p.d_dtype == LB_BF16) ((__nv_bfloat16*)p.d)[at] = __float2bfloat16_rn(x);
             else ((__half*)p.d)[at] = __float2half_rn(x);
-            if (p.epilogue == EPI_RELU_BESIDE)
-                ((uint16_t*)p.aux)[at_aux] = p.d_dtype == LB_BF16 ? relu_one(__bfloat16_as_ushort(__float2bfloat16_rn(x)), true) : relu_one(__half_as_ushort(__float2half_rn(x)), false);
         }
 }
 

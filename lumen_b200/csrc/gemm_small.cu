@@ -159,7 +159,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             const int col = n_blk * BN + q * 8;
             if (row >= p.M || col >= p.N) continue;
             const long long at = (long long)b * p.d_batch_stride + row * p.ldd + col;
-            uint16_t* aux = (uint16_t*)p.aux + (long long)b * p.aux_batch_stride + row * p.ld_aux + col;
+            const uint16_t* aux = (const uint16_t*)p.aux + (long long)b * p.aux_batch_stride + row * p.ld_aux + col;
             if (p.whole && col + 8 <= p.N) {
                 uint4 a16 = make_uint4(0, 0, 0, 0);
                 if constexpr (reads_aux(EPI)) a16 = *(const uint4*)aux;
@@ -190,7 +190,6 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 #pragma unroll
                     for (int j = 0; j < 4; j++) w[j] = pair16<DT>(x[2 * j], x[2 * j + 1]);
                     *(uint4*)((uint16_t*)p.d + at) = make_uint4(w[0], w[1], w[2], w[3]);
-                    if constexpr (EPI == EPI_RELU_BESIDE) *(uint4*)aux = relu_16_bytes(make_uint4(w[0], w[1], w[2], w[3]), DT == LB_BF16);
                 }
             } else {
 #pragma unroll 1
@@ -209,9 +208,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     if constexpr (DT == LB_F32) {
                         ((float*)p.d)[at + j] = x;
                     } else {
-                        const uint16_t h = to16<DT>(x);
-                        ((uint16_t*)p.d)[at + j] = h;
-                        if constexpr (EPI == EPI_RELU_BESIDE) aux[j] = relu_one(h, DT == LB_BF16);
+                        ((uint16_t*)p.d)[at + j] = to16<DT>(x);
                     }
                 }
             }

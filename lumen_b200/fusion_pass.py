@@ -267,9 +267,7 @@ class FusionPass:
     # ---- GEMM epilogues ----------------------------------------------------------------------------------------
     def find_dot_tails(self):
         """For each 16-bit `dot_general` read by one node only: the elementwise tail (with its zeros) the GEMM's epilogue
-        runs, when the compiler's matcher knows it (relu, `other + product`, `select(0 < other, product, 0)`, the factor a
-        maximum with zero passes back). For one that others read too, its relu if a product reads that: it has to be in memory
-        in any case, and the epilogue writes it without reading the first product back."""
+        runs, when the compiler's matcher knows it (relu, `other + product`, `select(0 < other, product, 0)`)."""
         from lumen_b200.compiler import Lowering
 
         g = self.g
@@ -277,16 +275,11 @@ class FusionPass:
             if n.op != "dot_general" or g.types[n.output].dtype == "float32" or n.output in self.outputs:
                 continue
             readers = self.uses.get(n.output, [])
-            if not readers:
+            if len(readers) != 1:
                 continue
             tail = readers[0]
-            if len(readers) > 1:
-                maxima = [u for u in readers if g.nodes[u].op == "max"]
-                if len(maxima) != 1 or min(readers) != maxima[0] or not any(g.nodes[u].op == "dot_general" for u in self.uses.get(g.nodes[maxima[0]].output, [])):
-                    continue
-                tail = maxima[0]
             t = g.nodes[tail]
-            if t.op not in ("max", "add", "select", "mul") or g.types[t.output].shape != g.types[n.output].shape:
+            if t.op not in ("max", "add", "select") or g.types[t.output].shape != g.types[n.output].shape:
                 continue
             members = [i, tail]
             if t.op == "select":  # the condition `0 < other` joins too when only the select reads it
@@ -294,24 +287,12 @@ class FusionPass:
                 if c is None or g.nodes[c].op != "lt" or self.uses.get(g.nodes[c].output, []) != [tail]:
                     continue
                 members = sorted([i, c, tail])
-            if t.op == "mul":  # the factor `select(0 < x, 1, select(x == 0, 0.5, 0))`, where nothing else reads its parts
-                def part(value, op, reader):
-                    p = self.producer.get(value)
-                    return p if p is not None and g.nodes[p].op == op and self.uses.get(value, []) == [reader] and value not in self.outputs else None
-
-                outer = next((p for v in t.inputs if (p := part(v, "select", tail)) is not None), None)
-                inner = part(g.nodes[outer].inputs[2], "select", outer) if outer is not None else None
-                above = part(g.nodes[outer].inputs[0], "lt", outer) if outer is not None else None
-                equal = part(g.nodes[inner].inputs[0], "eq", inner) if inner is not None else None
-                if above is None or equal is None:
-                    continue
-                members = sorted([i, above, equal, inner, outer, tail])
             # every operand of the tail other than the product has to exist before the dot runs
             outside = [v for m in members for v in g.nodes[m].inputs if self.producer.get(v) not in members]
             if any(self.producer.get(v, -1) > i and g.nodes[self.producer[v]].op not in INLINED for v in outside):
                 continue
             body, _, leaving = self.body_of(members)
-            if len(leaving) != (1 if len(readers) == 1 else 2):
+            if len(leaving) != 1:
                 continue
             try:
                 Lowering.dot_fusion_epilogue(body)

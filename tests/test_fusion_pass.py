@@ -4,8 +4,8 @@ fusion bodies primitive by primitive, so the fused graph must give bit-identical
 import numpy as np
 import pytest
 
-from lumen_b200 import autograd, prims, tracer
 from lumen_b200 import functional as F
+from lumen_b200 import prims, tracer
 from lumen_b200.compiler import compile_graph
 from lumen_b200.fusion_pass import fuse
 from tests.helpers import bf16, run_oracle
@@ -85,47 +85,6 @@ def test_gemm_takes_its_elementwise_tail_as_an_epilogue():
     assert labels == ["dot_general_add", "dot_general_relu", "dot_general_relu_backward"]
     rng = np.random.default_rng(3)
     same_values(g, fused, [bf16(rng.standard_normal((128, 128)) / 12) for _ in range(4)])
-
-
-def test_relu_beside_its_product_and_what_a_maximum_passes_back_are_epilogues():
-    """A relu of a product that others read too is written beside it, if a product reads the relu; the factor of its
-    backward is applied to the product it multiplies. Both lowerings make the same steps; what only resembles them stays apart."""
-    import json
-
-    from lumen_b200 import _lib
-    from lumen_b200.plan import _bind, lower_native
-    from lumen_b200.simplify import clean
-
-    def mlp(x, u, v, dy, early=False, half=0.5):
-        h = F.matmul(x, u, "float32", "bfloat16")
-        first = h + 1 if early else x  # a reader of the product that stands before its relu
-        a = F.relu(h)
-        y, back = F.matmul(a, v, "float32", "bfloat16"), prims.dot_general(dy, v, (((1,), (1,)), ((), ())), "float32", "bfloat16")
-        c = lambda value: prims.broadcast_in_dim(prims.full((), value, "bfloat16"), h.shape, ())
-        factor = prims.select(F.lt(0.0, h), c(1.0), prims.select(F.eq(h, 0.0), c(half), c(0.0)))
-        return (y, back * factor) + ((first,) if early else ())
-
-    def differentiated(x, u, v, dy):
-        f = lambda *p: F.matmul(F.relu(F.matmul(p[0], p[1], "float32", "bfloat16")), p[2], "float32", "bfloat16")
-        y, pull = autograd.vjp(f, x, u, v)
-        return (y, *pull(dy))
-
-    types = [("bfloat16", s) for s in ((24, 16), (16, 40), (40, 16), (24, 16))]
-    rng = np.random.default_rng(11)
-    inputs = [bf16(rng.standard_normal(s)) for _, s in types]
-    inputs[0][::5] = 0  # rows of zeros: where the maximum's operands are equal
-
-    beside, gated = "dot_general_relu_beside", "dot_general_max_backward"
-    for program, found in ((differentiated, [beside, gated]), (mlp, [beside, gated]), (lambda *x: mlp(*x, half=0.25), [beside]), (lambda *x: mlp(*x, early=True), [gated])):
-        g = tracer.trace(program, *types)
-        fused = fuse(clean(g))
-        labels = compile_graph(g).labels
-        assert [x for x in labels if x in (beside, gated)] == found
-        lib, native = _bind(), lower_native(fused)
-        assert [s["label"] for s in json.loads(lib.lb_plan_steps_json(native).decode())] == labels
-        assert lib.lb_plan_workspace_bytes(native) == compile_graph(g).workspace_bytes
-        lib.lb_plan_destroy(native)
-        same_values(g, fused, inputs)
 
 
 def test_traced_fusions_pass_through_and_constants_of_unfusible_readers_stay_plain():

@@ -55,51 +55,6 @@ def test_mlp_block_from_bare_prims_uses_gemm_epilogues(cuda):
     np.testing.assert_allclose(got[0].astype(np.float32), want, rtol=2**-6, atol=2**-6 * np.abs(want).max())
 
 
-@pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
-@pytest.mark.parametrize("m, n, k", [
-    (1, 8, 8), (200, 520, 64), (200, 4096, 1024),  # narrow tiles: one, ragged ones, K cut over a cluster
-    (2100, 2056, 40), (2304, 2048, 64),  # pairs of large tiles, with and without ragged ones
-    (128, 40008, 64), (70, 50002, 40), (2100, 2047, 40), (300, 513, 24),  # one row block; rows of the result that are not 16-byte aligned
-    (1024, 1024, 8192), (1024, 1021, 8192),  # K cut into ranges whose sums another kernel adds
-    (30, 33, 17), (300, 513, 25)])  # rows that the tensor cores' copies do not take
-def test_relu_beside_its_product_and_what_a_maximum_passes_back_on_the_gpu(cuda, m, n, k, dtype):
-    """Each kernel's epilogue bit for bit against the product of the same sizes by itself and the two primitives after it: where the
-    operand is zero (rows of zeros), infinite or not a number too."""
-    from lumen_b200 import autograd
-    from lumen_b200.runtime import gemm, gemm_scratch_bytes
-
-    torch_dtype, dims = TORCH_DTYPES[dtype], (((1,), (1,)), ((), ()))
-
-    def program(x, w, v, dy):
-        h = prims.dot_general(x, w, dims, "float32", dtype)
-        a, pull = autograd.vjp(F.relu, h)
-        y = F.matmul(a, v, "float32", dtype)
-        back = prims.dot_general(dy, w, dims, "float32", dtype)
-        return y, a, pull(back)[0], h * 1.0
-
-    g = tracer.trace(program, (dtype, (m, k)), (dtype, (n, k)), (dtype, (n, 8)), (dtype, (m, k)))
-    compiled = compile_graph(g)
-    assert "dot_general_relu_beside" in compiled.labels and "dot_general_max_backward" in compiled.labels
-    gen = torch.Generator(device=cuda).manual_seed(n)
-    x, w, v, dy = (torch.randn(s, generator=gen, device=cuda).to(torch_dtype) for s in ((m, k), (n, k), (n, 8), (m, k)))
-    x[::5] = 0
-    if m > 7:
-        x[3, 0], x[6, 1], dy[10 % m, 0] = float("inf"), float("nan"), -float("inf")
-    outs = [torch.empty(s, dtype=torch_dtype, device=cuda) for s in ((m, 8), (m, n), (m, n), (m, n))]
-    Plan(compiled).run([x, w, v, dy], outs)
-
-    def product(a):
-        scratch = torch.empty(gemm_scratch_bytes(m, n, k), dtype=torch.uint8, device=cuda)
-        return gemm(a, w.t(), torch.empty(m, n, dtype=torch_dtype, device=cuda), scratch=scratch if scratch.numel() else None)
-
-    h, back = product(x), product(dy)
-    factor = torch.where(h > 0, 1.0, torch.where(h == 0, 0.5, 0.0)).to(torch_dtype)
-    for got, want in ((outs[3], h), (outs[1], torch.clamp(h, min=0)), (outs[2], back * factor)):  # clamp keeps a NaN
-        assert torch.equal(torch.isnan(got), torch.isnan(want))
-        assert torch.equal(got.nan_to_num(0.0, None, None), want.nan_to_num(0.0, None, None))
-    device_status()
-
-
 def test_compile_surface_runs_a_traced_function(cuda, tmp_path):
     """`lumen_b200.compile(fn, device="cuda")`: traced on the first call per signature, results owned by the compiled
     function and overwritten by the next call, a second signature compiles its own plan."""
