@@ -78,24 +78,16 @@ __device__ __forceinline__ int tile_coords(const GemmArgs& p, int unit, int& b, 
     return split;
 }
 
-// Whether the rows of the result start and go on in whole 16-byte pieces.
-template <int DT>
-__device__ __forceinline__ bool whole_lines(const GemmArgs& p) {
-    constexpr int per = DT == LB_F32 ? 4 : 8;
-    return p.ldd % per == 0 && p.d_batch_stride % per == 0 && ((uintptr_t)p.d & 15) == 0;
-}
-
 // Drains 128 accumulator columns (this warp's half of a 256-wide tile) of the thread's row from tensor memory and
 // stores them with the epilogue and one rounding to the output dtype. `release` hands the accumulator back to the MMA warp, once its
 // last columns are in registers.
-template <int EPI, int DT, class Release>
+template <class Release>
 __device__ __forceinline__ void drain_tile(const GemmArgs& p, uint32_t tbase, int row, long long row_off, int col_base, int b,
                                            bool vec_ok, uint4* stage, int lane, Release release) {
-    const long long aux_off = (long long)b * p.aux_batch_stride + (long long)row * p.ld_aux;
 #pragma unroll 1
     for (int c2 = 0; c2 < BN / 2 / 64; c2++) {
         // warp-uniform: 16-bit rows of 64 whole columns leave through the staging area, 128 contiguous bytes per row
-        const bool coalesced = vec_ok && DT != LB_F32 && col_base + c2 * 64 + 64 <= p.N;
+        const bool coalesced = vec_ok && (p.d_bf16 || p.d_f16) && col_base + c2 * 64 + 64 <= p.N;
         uint4 packed[8];
         uint32_t vv[64];
         tmem_ld_32x32(tbase + c2 * 64, vv);  // two loads in flight, one wait
@@ -107,16 +99,16 @@ __device__ __forceinline__ void drain_tile(const GemmArgs& p, uint32_t tbase, in
             uint32_t* v = vv + h * 32;
             const int col0 = col_base + c2 * 64 + h * 32;
             // warp-uniform: a float32 row piece of 32 whole columns is one 128-byte line and leaves through the staging area too
-            const bool staged32 = vec_ok && DT == LB_F32 && col0 + 32 <= p.N;
+            const bool staged32 = vec_ok && !(p.d_bf16 || p.d_f16) && col0 + 32 <= p.N;
             if (row < p.M && col0 < p.N) {
-                if constexpr (EPI == EPI_RELU) {
+                if (p.epilogue == EPI_RELU) {
 #pragma unroll
                     for (int j = 0; j < 32; j++) v[j] = __float_as_uint(fmaxf(__uint_as_float(v[j]), 0.0f));
                 }
                 const bool full_chunk = col0 + 32 <= p.N;
-                if constexpr (reads_aux(EPI)) {
+                if (p.epilogue >= EPI_ADD) {
                     // 16-bit outputs only (checked by the host). The product is rounded first, as its own primitive.
-                    const uint16_t* ax = (const uint16_t*)p.aux + aux_off + col0;
+                    const uint16_t* ax = (const uint16_t*)p.aux + (long long)b * p.aux_batch_stride + (long long)row * p.ld_aux + col0;
                     uint32_t aw[16];
                     if (full_chunk && p.ld_aux % 8 == 0 && p.aux_batch_stride % 8 == 0 && ((uintptr_t)p.aux & 15) == 0) {
 #pragma unroll
@@ -135,25 +127,38 @@ __device__ __forceinline__ void drain_tile(const GemmArgs& p, uint32_t tbase, in
                     for (int j = 0; j < 32; j++) {
                         const uint16_t a16 = (uint16_t)(j & 1 ? aw[j / 2] >> 16 : aw[j / 2] & 0xffffu);
                         const float acc = __uint_as_float(v[j]);
-                        v[j] = __float_as_uint(second_primitive(EPI, from16<DT>(to16<DT>(acc)), from16<DT>(a16)));
+                        float prod, other;
+                        if (p.d_bf16) prod = __bfloat162float(__float2bfloat16_rn(acc)), other = __uint_as_float((uint32_t)a16 << 16);
+                        else prod = __half2float(__float2half_rn(acc)), other = __half2float(__ushort_as_half(a16));
+                        v[j] = __float_as_uint(p.epilogue == EPI_ADD ? __fadd_rn(other, prod) : (other > 0.0f ? prod : 0.0f));
                     }
                 }
-                if constexpr (DT != LB_F32) {
+                if (p.d_bf16 || p.d_f16) {
                     uint16_t* out = (uint16_t*)p.d + row_off + col0;
                     if (full_chunk && vec_ok) {
 #pragma unroll
                         for (int j = 0; j < 32; j += 8) {
                             uint32_t w[4];
 #pragma unroll
-                            for (int q = 0; q < 4; q++) w[q] = pair16<DT>(__uint_as_float(v[j + 2 * q]), __uint_as_float(v[j + 2 * q + 1]));
+                            for (int q = 0; q < 4; q++) {
+                                float lo = __uint_as_float(v[j + 2 * q]), hi = __uint_as_float(v[j + 2 * q + 1]);
+                                if (p.d_bf16) {
+                                    __nv_bfloat162 hh = __floats2bfloat162_rn(lo, hi);
+                                    w[q] = *(uint32_t*)&hh;
+                                } else {
+                                    __half2 hh = __floats2half2_rn(lo, hi);
+                                    w[q] = *(uint32_t*)&hh;
+                                }
+                            }
                             if (coalesced) packed[h * 4 + j / 8] = make_uint4(w[0], w[1], w[2], w[3]);
                             else *(uint4*)(out + j) = make_uint4(w[0], w[1], w[2], w[3]);
                         }
                     } else {
 #pragma unroll
                         for (int j = 0; j < 32; j++) {  // unrolled with a predicate: keeps the fragment in registers
-                            const uint16_t x16 = to16<DT>(__uint_as_float(v[j]));
-                            if (col0 + j < p.N) out[j] = x16;
+                            float x = __uint_as_float(v[j]);
+                            if (col0 + j < p.N)
+                                out[j] = p.d_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(x)) : __half_as_ushort(__float2half_rn(x));
                         }
                     }
                 } else {
@@ -212,9 +217,8 @@ __device__ __forceinline__ void drain_partial(const GemmArgs& p, uint32_t tbase,
 // operand and the output): the operand's 32-column chunks are loaded one chunk ahead - the first one before the
 // warp waits for the tile's MMAs - so that their global-memory latency never sits between the accumulator load
 // and the store.
-template <int EPI>
 __device__ __forceinline__ bool aux_fast_path(const GemmArgs& p, int row, int col_base, bool vec_ok) {
-    return reads_aux(EPI) && vec_ok && row < p.M && col_base + BN / 2 <= p.N && p.ld_aux % 8 == 0 &&
+    return p.epilogue >= EPI_ADD && p.splits == 1 && vec_ok && row < p.M && col_base + BN / 2 <= p.N && p.ld_aux % 8 == 0 &&
            p.aux_batch_stride % 8 == 0 && ((uintptr_t)p.aux & 15) == 0;
 }
 // Loads a 32-row x 32-column chunk of the operand with whole 64-byte row pieces per four lanes (eight rows per load
@@ -240,7 +244,7 @@ __device__ __forceinline__ void aux_to_rows(uint4* stage_aux, const uint4* raw, 
         aw[4 * q] = x.x, aw[4 * q + 1] = x.y, aw[4 * q + 2] = x.z, aw[4 * q + 3] = x.w;
     }
 }
-template <int EPI, int DT, class Release>
+template <class Release>
 __device__ __forceinline__ void drain_tile_aux(const GemmArgs& p, uint32_t tbase, long long row_off, const uint16_t* ax_warp, uint4* raw,
                                                uint4* stage, int lane, Release release) {
     uint8_t* out0 = (uint8_t*)((uint16_t*)p.d + (row_off - (long long)lane * p.ldd));  // the warp's first row (all 32 are inside M)
@@ -263,9 +267,19 @@ __device__ __forceinline__ void drain_tile_aux(const GemmArgs& p, uint32_t tbase
                 for (int u = 0; u < 2; u++) {
                     const uint32_t pair = aw[(j + 2 * q) / 2];
                     const uint16_t a16 = (uint16_t)(u ? pair >> 16 : pair & 0xffffu);
-                    r[u] = second_primitive(EPI, from16<DT>(to16<DT>(__uint_as_float(v[j + 2 * q + u]))), from16<DT>(a16));
+                    const float acc = __uint_as_float(v[j + 2 * q + u]);
+                    float prod, other;
+                    if (p.d_bf16) prod = __bfloat162float(__float2bfloat16_rn(acc)), other = __uint_as_float((uint32_t)a16 << 16);
+                    else prod = __half2float(__float2half_rn(acc)), other = __half2float(__ushort_as_half(a16));
+                    r[u] = p.epilogue == EPI_ADD ? __fadd_rn(other, prod) : (other > 0.0f ? prod : 0.0f);
                 }
-                w[q] = pair16<DT>(r[0], r[1]);
+                if (p.d_bf16) {
+                    __nv_bfloat162 hh = __floats2bfloat162_rn(r[0], r[1]);
+                    w[q] = *(uint32_t*)&hh;
+                } else {
+                    __half2 hh = __floats2half2_rn(r[0], r[1]);
+                    w[q] = *(uint32_t*)&hh;
+                }
             }
             packed[j / 8] = make_uint4(w[0], w[1], w[2], w[3]);
         }
@@ -273,11 +287,6 @@ __device__ __forceinline__ void drain_tile_aux(const GemmArgs& p, uint32_t tbase
     }
 }
 
-// One kernel for each epilogue EPI (EPI_PARTIAL: float32 sums of a range of K) and type DT of the result. A product of few tiles runs its
-// epilogue once, as fast as its instructions arrive: with the choices of all epilogues and types in one kernel they lay far apart, and were
-// fetched one after another at each launch. us a product, back to back, before -> after, plain and with an added operand:
-// 4122 x 832 x 208 8.4 -> 6.4, 10.2 -> 8.2; 1241 x 1632 x 408 9.3 -> 7.4, 11.6 -> 9.1; 8192 x 4096 x 1024 50.3 -> 48.5, 63.4 -> 62.9.
-template <int EPI, int DT>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmArgs p) {
     extern __shared__ uint8_t smem_raw[];
@@ -402,7 +411,8 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
         uint4* stage = (uint4*)(smem + STAGES * (kStageBytesA + kStageBytesB) + 256) + (warp - 2) * (kStageBytesPerWarp / 16);
         int local = 0;
         bool ok = true;
-        const bool vec_ok = EPI != EPI_PARTIAL && whole_lines<DT>(p);
+        const bool vec_ok = p.d_bf16 || p.d_f16 ? (p.ldd % 8 == 0 && p.d_batch_stride % 8 == 0 && ((uintptr_t)p.d & 15) == 0)
+                                                : (p.ldd % 4 == 0 && p.d_batch_stride % 4 == 0 && ((uintptr_t)p.d & 15) == 0);
         for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x, local++) {
             const int buf = local & 1;
             const uint32_t use = (uint32_t)(local >> 1);
@@ -411,12 +421,10 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             const int row = m_blk * BM + quarter * 32 + lane;
             const int col_base = n_blk * BN + col_half * (BN / 2);
             const long long row_off = (long long)b * p.d_batch_stride + (long long)row * p.ldd;
-            // warp-uniform: both drains load tensor memory warp-wide
-            const bool fast = reads_aux(EPI) && __all_sync(0xffffffffu, aux_fast_path<EPI>(p, row, col_base, vec_ok));
+            const bool fast = __all_sync(0xffffffffu, aux_fast_path(p, row, col_base, vec_ok));  // warp-uniform: both drains load tensor memory warp-wide
             const uint16_t* ax_warp = (const uint16_t*)p.aux + (long long)b * p.aux_batch_stride + (long long)(row - lane) * p.ld_aux + col_base;
             uint4 raw[4];
-            if constexpr (reads_aux(EPI))
-                if (fast) aux_load(ax_warp, p.ld_aux, lane, raw);
+            if (fast) aux_load(ax_warp, p.ld_aux, lane, raw);
             if (!(ok = mbar_wait(&tmem_full[buf], use & 1, abort_flag))) break;
             __syncwarp();
             tc_fence_after();
@@ -426,14 +434,9 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&tmem_empty[buf]);
             };
-            if constexpr (EPI == EPI_PARTIAL) {
-                drain_partial(p, tbase, row, col_base, b, split, stage, lane, release);
-            } else if constexpr (reads_aux(EPI)) {
-                if (fast) drain_tile_aux<EPI, DT>(p, tbase, row_off + col_base, ax_warp, raw, stage, lane, release);
-                else drain_tile<EPI, DT>(p, tbase, row, row_off, col_base, b, vec_ok, stage, lane, release);
-            } else {
-                drain_tile<EPI, DT>(p, tbase, row, row_off, col_base, b, vec_ok, stage, lane, release);
-            }
+            if (fast) drain_tile_aux(p, tbase, row_off + col_base, ax_warp, raw, stage, lane, release);
+            else if (p.splits > 1) drain_partial(p, tbase, row, col_base, b, split, stage, lane, release);
+            else drain_tile(p, tbase, row, row_off, col_base, b, vec_ok, stage, lane, release);
         }
     }
 
@@ -473,7 +476,6 @@ constexpr int PSTAGES = 6;
 constexpr int kPairStageBytesA = BM * BK * 2, kPairStageBytesB = (BN / 2) * BK * 2;
 constexpr int kPairSmemBytes = PSTAGES * (kPairStageBytesA + kPairStageBytesB) + 1024 + 256 + kEpilogueStageBytes;
 
-template <int EPI, int DT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmArgs p) {
     extern __shared__ uint8_t smem_raw[];
@@ -607,7 +609,8 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         uint4* stage = (uint4*)(smem + PSTAGES * (kPairStageBytesA + kPairStageBytesB) + 256) + (warp - 2) * (kStageBytesPerWarp / 16);
         int local = 0;
         bool ok = true;
-        const bool vec_ok = EPI != EPI_PARTIAL && whole_lines<DT>(p);
+        const bool vec_ok = p.d_bf16 || p.d_f16 ? (p.ldd % 8 == 0 && p.d_batch_stride % 8 == 0 && ((uintptr_t)p.d & 15) == 0)
+                                                : (p.ldd % 4 == 0 && p.d_batch_stride % 4 == 0 && ((uintptr_t)p.d & 15) == 0);
         for (int unit = pair; unit < num_units && ok; unit += num_pairs, local++) {
             const int buf = local & 1;
             const uint32_t use = (uint32_t)(local >> 1);
@@ -616,12 +619,10 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             const int row = m_blk * 2 * BM + (int)rank * BM + quarter * 32 + lane;
             const int col_base = n_blk * BN + col_half * (BN / 2);
             const long long row_off = (long long)b * p.d_batch_stride + (long long)row * p.ldd;
-            // warp-uniform: both drains load tensor memory warp-wide
-            const bool fast = reads_aux(EPI) && __all_sync(0xffffffffu, aux_fast_path<EPI>(p, row, col_base, vec_ok));
+            const bool fast = __all_sync(0xffffffffu, aux_fast_path(p, row, col_base, vec_ok));  // warp-uniform: both drains load tensor memory warp-wide
             const uint16_t* ax_warp = (const uint16_t*)p.aux + (long long)b * p.aux_batch_stride + (long long)(row - lane) * p.ld_aux + col_base;
             uint4 raw[4];
-            if constexpr (reads_aux(EPI))
-                if (fast) aux_load(ax_warp, p.ld_aux, lane, raw);
+            if (fast) aux_load(ax_warp, p.ld_aux, lane, raw);
             if (!(ok = mbar_wait(&tmem_full[buf], use & 1, abort_flag))) break;
             __syncwarp();
             tc_fence_after();
@@ -631,14 +632,9 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 __syncwarp();
                 if (lane == 0) mbar_arrive_cluster(&tmem_empty[buf], 0);
             };
-            if constexpr (EPI == EPI_PARTIAL) {
-                drain_partial(p, tbase, row, col_base, b, split, stage, lane, release);
-            } else if constexpr (reads_aux(EPI)) {
-                if (fast) drain_tile_aux<EPI, DT>(p, tbase, row_off + col_base, ax_warp, raw, stage, lane, release);
-                else drain_tile<EPI, DT>(p, tbase, row, row_off, col_base, b, vec_ok, stage, lane, release);
-            } else {
-                drain_tile<EPI, DT>(p, tbase, row, row_off, col_base, b, vec_ok, stage, lane, release);
-            }
+            if (fast) drain_tile_aux(p, tbase, row_off + col_base, ax_warp, raw, stage, lane, release);
+            else if (p.splits > 1) drain_partial(p, tbase, row, col_base, b, split, stage, lane, release);
+            else drain_tile(p, tbase, row, row_off, col_base, b, vec_ok, stage, lane, release);
         }
     }
 
@@ -683,7 +679,7 @@ __global__ void __launch_bounds__(256) splitk_reduce(const float* __restrict__ p
         const long long row = i / p.N, b = p.batch > 1 ? row / p.M : 0, r = row - b * p.M, c = i - row * p.N;
         const uint16_t* aux = (const uint16_t*)p.aux + b * p.aux_batch_stride + r * p.ld_aux + c;
         __align__(8) uint16_t a16[W], out16[W];
-        if (reads_aux(p.epilogue)) {
+        if (p.epilogue >= EPI_ADD) {
             if constexpr (VEC) *(uint2*)a16 = *(const uint2*)aux;
             else a16[0] = *aux;
         }
@@ -691,9 +687,11 @@ __global__ void __launch_bounds__(256) splitk_reduce(const float* __restrict__ p
         for (int j = 0; j < W; j++) {
             float x = acc[j];
             if (p.epilogue == EPI_RELU) x = fmaxf(x, 0.0f);
-            if (reads_aux(p.epilogue)) {
-                x = p.d_bf16 ? second_primitive(p.epilogue, from16<LB_BF16>(to16<LB_BF16>(x)), from16<LB_BF16>(a16[j]))
-                             : second_primitive(p.epilogue, from16<LB_F16>(to16<LB_F16>(x)), from16<LB_F16>(a16[j]));
+            if (p.epilogue >= EPI_ADD) {
+                float prod, other;
+                if (p.d_bf16) prod = __bfloat162float(__float2bfloat16_rn(x)), other = __uint_as_float((uint32_t)a16[j] << 16);
+                else prod = __half2float(__float2half_rn(x)), other = __half2float(__ushort_as_half(a16[j]));
+                x = p.epilogue == EPI_ADD ? __fadd_rn(other, prod) : (other > 0.0f ? prod : 0.0f);
             }
             acc[j] = x;
             out16[j] = p.d_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(x)) : __half_as_ushort(__float2half_rn(x));
@@ -808,23 +806,6 @@ int gemm_small_splits(long long M, long long N, long long K, long long batch, in
     return s;
 }
 
-template <int EPI, int DT>
-static void launch_large(const GemmArgs& p, bool pairs, int grid, const CUtensorMap& map_a, const CUtensorMap& map_b, cudaStream_t s) {
-    if (pairs) {
-        if (first_use_on_device((const void*)gemm_tcgen05_pair<EPI, DT>))
-            LB_CUDA(cudaFuncSetAttribute(gemm_tcgen05_pair<EPI, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes));
-        launch_overlapped(gemm_tcgen05_pair<EPI, DT>, dim3((unsigned)grid), dim3(kThreads), kPairSmemBytes, s, 0, map_a, map_b, p);
-    } else {
-        if (first_use_on_device((const void*)gemm_tcgen05<EPI, DT>))
-            LB_CUDA(cudaFuncSetAttribute(gemm_tcgen05<EPI, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-        launch_overlapped(gemm_tcgen05<EPI, DT>, dim3((unsigned)grid), dim3(kThreads), kSmemBytes, s, 0, map_a, map_b, p);
-    }
-}
-static void launch_large(const GemmArgs& p, bool pairs, int grid, const CUtensorMap& map_a, const CUtensorMap& map_b, cudaStream_t s) {
-    if (p.splits > 1) return launch_large<EPI_PARTIAL, LB_F32>(p, pairs, grid, map_a, map_b, s);
-    with_epilogue(p.epilogue, p.d_bf16 ? LB_BF16 : p.d_f16 ? LB_F16 : LB_F32, [&](auto epi, auto dt) { launch_large<decltype(epi)::value, decltype(dt)::value>(p, pairs, grid, map_a, map_b, s); });
-}
-
 // CTA pairs of gemm_tcgen05_pair that can be resident on `dev` at once (asked of the runtime once per device).
 static int resident_pairs(const DeviceInfo& dev) {
     static std::mutex mutex;
@@ -835,9 +816,7 @@ static int resident_pairs(const DeviceInfo& dev) {
     int pairs = 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * (dev.sms / 2), 1, 1), cfg.blockDim = dim3(kThreads, 1, 1), cfg.dynamicSmemBytes = kPairSmemBytes;
-    const auto kernel = gemm_tcgen05_pair<EPI_NONE, LB_BF16>;  // all take the same threads, registers and shared memory
-    LB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes));
-    if (cudaOccupancyMaxActiveClusters(&pairs, kernel, &cfg) != cudaSuccess || pairs <= 0) {
+    if (cudaOccupancyMaxActiveClusters(&pairs, gemm_tcgen05_pair, &cfg) != cudaSuccess || pairs <= 0) {
         cudaGetLastError();
         pairs = 0;
     }
@@ -974,6 +953,10 @@ bool gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
             gemm_small(map_a, p.b_mn_major ? map_b : make_map(bt, true, BK, 64), q, (int)batch, dev.sms, s);
             return false;
         }
+        if (first_use_on_device((const void*)gemm_tcgen05_pair)) {
+            LB_CUDA(cudaFuncSetAttribute(gemm_tcgen05, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+            LB_CUDA(cudaFuncSetAttribute(gemm_tcgen05_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes));
+        }
         const int max_pairs = resident_pairs(dev);
         long long tiles = (long long)p.tiles_m * p.tiles_n * batch;
         const int sms = dev.sms;
@@ -987,10 +970,10 @@ bool gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
         if (pairs) {
             const int resident = max_pairs > 0 ? max_pairs : sms / 2;
             int grid = 2 * (int)std::min<long long>(tiles * p.splits, resident);
-            launch_large(p, true, grid, map_a, map_b, s);
+            launch_overlapped(gemm_tcgen05_pair, dim3((unsigned)grid), dim3(kThreads), kPairSmemBytes, s, 0, map_a, map_b, p);
         } else {
             int grid = (int)std::min<long long>(tiles * p.splits, sms);
-            launch_large(p, false, grid, map_a, map_b, s);
+            launch_overlapped(gemm_tcgen05, dim3((unsigned)grid), dim3(kThreads), kSmemBytes, s, 0, map_a, map_b, p);
         }
         if (p.splits > 1) {
             const size_t quad = d.dtype == LB_F32 ? 16 : 8;  // bytes of four elements

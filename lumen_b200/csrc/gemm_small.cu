@@ -35,34 +35,10 @@ __device__ __forceinline__ float4 load_cluster(uint32_t addr, uint32_t rank) {
         : "memory");
     return v;
 }
-__device__ __forceinline__ float load_cluster_one(uint32_t addr, uint32_t rank) {
-    float v;
-    asm volatile(
-        "{\n\t.reg .b32 ra;\n\t"
-        "mapa.shared::cluster.u32 ra, %1, %2;\n\t"
-        "ld.shared::cluster.f32 %0, [ra];\n\t}"
-        : "=f"(v)
-        : "r"(addr), "r"(rank)
-        : "memory");
-    return v;
-}
 // byte offset of 16-byte chunk `c` of row `r` of the partial tile: eight rows' equal chunks fall in different banks
 __device__ __forceinline__ uint32_t chunk_at(int r, int c) { return (uint32_t)(r * BN * 4 + ((c ^ (r & 7)) << 4)); }
 
-// A sum with its epilogue: with an operand the product is rounded first, as its own primitive (16-bit results only).
-template <int EPI, int DT>
-__device__ __forceinline__ float finish(float x, uint16_t aux) {
-    if constexpr (EPI == EPI_RELU) return fmaxf(x, 0.0f);
-    else if constexpr (reads_aux(EPI)) return second_primitive(EPI, from16<DT>(to16<DT>(x)), from16<DT>(aux));
-    else return x;
-}
-
-// One kernel for each epilogue EPI and type DT of the result: what a block runs after its products it runs a few times at most and fetches as
-// it goes, and the choices of the other epilogues in between, element by element, cost more than the work. So does the ragged edge when it is
-// unrolled: it goes one element at a time. us a product, back to back, before -> after, plain and with an added operand:
-// 200 x 4096 x 1024 8.4 -> 6.5, 9.6 -> 7.7; 200 x 1024 x 4096 9.2 -> 8.8, 9.6 -> 9.0; 283 x 2176 x 544 7.1 -> 5.2, 8.4 -> 6.4;
-// 4122 x 208 x 832 8.1 -> 6.1, 9.4 -> 7.4.
-template <int STAGES, int EPI, int DT>
+template <int STAGES>
 __global__ void __launch_bounds__(kThreads, 8 / STAGES)
 gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const SmallGemmArgs p) {
     extern __shared__ uint8_t smem_raw[];
@@ -152,64 +128,57 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     // this CTA's share of the rows: eight columns per thread
     if (!*abort_flag) {
         const int rows = BM / p.splits;
-#pragma unroll 1
         for (int i = threadIdx.x; i < rows * (BN / 8); i += kThreads) {
             const int r = rank * rows + i / (BN / 8), q = i % (BN / 8);
             const long long row = (long long)m_blk * BM + r;
             const int col = n_blk * BN + q * 8;
             if (row >= p.M || col >= p.N) continue;
-            const long long at = (long long)b * p.d_batch_stride + row * p.ldd + col;
-            const uint16_t* aux = (const uint16_t*)p.aux + (long long)b * p.aux_batch_stride + row * p.ld_aux + col;
-            if (p.whole && col + 8 <= p.N) {
-                uint4 a16 = make_uint4(0, 0, 0, 0);
-                if constexpr (reads_aux(EPI)) a16 = *(const uint4*)aux;
-                float x[8];
-                if (p.splits > 1) {
-                    const uint32_t at0 = smem_u32(smem) + chunk_at(r, 2 * q), at1 = smem_u32(smem) + chunk_at(r, 2 * q + 1);
-#pragma unroll
-                    for (int j = 0; j < 8; j++) x[j] = 0.0f;
-#pragma unroll 1
-                    for (int s = 0; s < p.splits; s += 2) {  // two, four or eight ranks
-                        const float4 u0 = load_cluster(at0, s), w0 = load_cluster(at1, s), u1 = load_cluster(at0, s + 1), w1 = load_cluster(at1, s + 1);
-                        x[0] += u0.x, x[1] += u0.y, x[2] += u0.z, x[3] += u0.w, x[4] += w0.x, x[5] += w0.y, x[6] += w0.z, x[7] += w0.w;
-                        x[0] += u1.x, x[1] += u1.y, x[2] += u1.z, x[3] += u1.w, x[4] += w1.x, x[5] += w1.y, x[6] += w1.z, x[7] += w1.w;
-                    }
-                } else {
-                    const float4 u = *(const float4*)(smem + chunk_at(r, 2 * q)), w = *(const float4*)(smem + chunk_at(r, 2 * q + 1));
-                    x[0] = u.x, x[1] = u.y, x[2] = u.z, x[3] = u.w, x[4] = w.x, x[5] = w.y, x[6] = w.z, x[7] = w.w;
+            float x[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+            if (p.splits > 1) {
+                const uint32_t at0 = smem_u32(smem) + chunk_at(r, 2 * q), at1 = smem_u32(smem) + chunk_at(r, 2 * q + 1);
+                for (int s = 0; s < p.splits; s++) {
+                    const float4 u = load_cluster(at0, s), w = load_cluster(at1, s);
+                    x[0] += u.x, x[1] += u.y, x[2] += u.z, x[3] += u.w, x[4] += w.x, x[5] += w.y, x[6] += w.z, x[7] += w.w;
                 }
-                const uint32_t pair[4] = {a16.x, a16.y, a16.z, a16.w};
+            } else {
+                const float4 u = *(const float4*)(smem + chunk_at(r, 2 * q)), w = *(const float4*)(smem + chunk_at(r, 2 * q + 1));
+                x[0] = u.x, x[1] = u.y, x[2] = u.z, x[3] = u.w, x[4] = w.x, x[5] = w.y, x[6] = w.z, x[7] = w.w;
+            }
+            const int live = min(8, p.N - col);
+            const uint16_t* aux = (const uint16_t*)p.aux + (long long)b * p.aux_batch_stride + row * p.ld_aux + col;
 #pragma unroll
-                for (int j = 0; j < 8; j++) x[j] = finish<EPI, DT>(x[j], (uint16_t)(j & 1 ? pair[j / 2] >> 16 : pair[j / 2] & 0xffffu));
-                if constexpr (DT == LB_F32) {
-                    float* out = (float*)p.d + at;
+            for (int j = 0; j < 8; j++) {
+                if (p.epilogue == EPI_RELU) x[j] = fmaxf(x[j], 0.0f);
+                if (p.epilogue >= EPI_ADD && j < live) {  // 16-bit outputs only; the product is rounded first, as its own primitive
+                    const uint16_t a16 = aux[j];
+                    float prod, other;
+                    if (p.d_bf16) prod = __bfloat162float(__float2bfloat16_rn(x[j])), other = __uint_as_float((uint32_t)a16 << 16);
+                    else prod = __half2float(__float2half_rn(x[j])), other = __half2float(__ushort_as_half(a16));
+                    x[j] = p.epilogue == EPI_ADD ? __fadd_rn(other, prod) : (other > 0.0f ? prod : 0.0f);
+                }
+            }
+            const long long at = (long long)b * p.d_batch_stride + row * p.ldd + col;
+            if (p.d_bf16 || p.d_f16) {
+                uint16_t h[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) h[j] = p.d_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(x[j])) : __half_as_ushort(__float2half_rn(x[j]));
+                uint16_t* out = (uint16_t*)p.d + at;
+                if (p.vec && live == 8) {
+                    *(uint4*)out = make_uint4(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16, h[4] | (uint32_t)h[5] << 16, h[6] | (uint32_t)h[7] << 16);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        if (j < live) out[j] = h[j];
+                }
+            } else {
+                float* out = (float*)p.d + at;
+                if (p.vec && live == 8) {
                     *(float4*)out = make_float4(x[0], x[1], x[2], x[3]);
                     *(float4*)(out + 4) = make_float4(x[4], x[5], x[6], x[7]);
                 } else {
-                    uint32_t w[4];
 #pragma unroll
-                    for (int j = 0; j < 4; j++) w[j] = pair16<DT>(x[2 * j], x[2 * j + 1]);
-                    *(uint4*)((uint16_t*)p.d + at) = make_uint4(w[0], w[1], w[2], w[3]);
-                }
-            } else {
-#pragma unroll 1
-                for (int j = 0; j < 8 && col + j < p.N; j++) {
-                    const uint32_t from = chunk_at(r, 2 * q + j / 4) + 4 * (j & 3);
-                    float x = 0.0f;
-                    if (p.splits > 1) {
-#pragma unroll 1
-                        for (int s = 0; s < p.splits; s++) x += load_cluster_one(smem_u32(smem) + from, s);
-                    } else {
-                        x = *(const float*)(smem + from);
-                    }
-                    uint16_t a16 = 0;
-                    if constexpr (reads_aux(EPI)) a16 = aux[j];
-                    x = finish<EPI, DT>(x, a16);
-                    if constexpr (DT == LB_F32) {
-                        ((float*)p.d)[at + j] = x;
-                    } else {
-                        ((uint16_t*)p.d)[at + j] = to16<DT>(x);
-                    }
+                    for (int j = 0; j < 8; j++)
+                        if (j < live) out[j] = x[j];
                 }
             }
         }
@@ -233,23 +202,20 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
 }  // namespace
 
-template <int STAGES, int EPI, int DT>
+template <int STAGES>
 static void launch_small(const CUtensorMap& map_a, const CUtensorMap& map_b, const SmallGemmArgs& p, int batch, cudaStream_t s) {
-    if (first_use_on_device((const void*)gemm_small_kernel<STAGES, EPI, DT>))
-        LB_CUDA(cudaFuncSetAttribute(gemm_small_kernel<STAGES, EPI, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(STAGES)));
-    launch_overlapped(gemm_small_kernel<STAGES, EPI, DT>, dim3((unsigned)((long long)p.tiles_m * p.tiles_n * batch * p.splits)), dim3(kThreads), smem_bytes(STAGES), s,
+    if (first_use_on_device((const void*)gemm_small_kernel<STAGES>))
+        LB_CUDA(cudaFuncSetAttribute(gemm_small_kernel<STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(STAGES)));
+    launch_overlapped(gemm_small_kernel<STAGES>, dim3((unsigned)((long long)p.tiles_m * p.tiles_n * batch * p.splits)), dim3(kThreads), smem_bytes(STAGES), s,
                       (unsigned)p.splits, map_a, map_b, p);
 }
+
 void gemm_small(const CUtensorMap& map_a, const CUtensorMap& map_b, SmallGemmArgs p, int batch, int sms, cudaStream_t s) {
     p.tiles_m = (p.M + BM - 1) / BM, p.tiles_n = (p.N + BN - 1) / BN;
     const int per_line = p.d_bf16 || p.d_f16 ? 8 : 4;
-    p.whole = (uintptr_t)p.d % 16 == 0 && p.ldd % per_line == 0 && p.d_batch_stride % per_line == 0 &&
-              (p.epilogue < EPI_ADD || ((uintptr_t)p.aux % 16 == 0 && p.ld_aux % 8 == 0 && p.aux_batch_stride % 8 == 0));
-    const bool one_wave = (long long)p.tiles_m * p.tiles_n * batch * p.splits <= sms;
-    with_epilogue(p.epilogue, p.d_bf16 ? LB_BF16 : p.d_f16 ? LB_F16 : LB_F32, [&](auto epi, auto dt) {
-        if (one_wave) launch_small<8, decltype(epi)::value, decltype(dt)::value>(map_a, map_b, p, batch, s);
-        else launch_small<4, decltype(epi)::value, decltype(dt)::value>(map_a, map_b, p, batch, s);
-    });
+    p.vec = (uintptr_t)p.d % 16 == 0 && p.ldd % per_line == 0 && p.d_batch_stride % per_line == 0;
+    if ((long long)p.tiles_m * p.tiles_n * batch * p.splits <= sms) launch_small<8>(map_a, map_b, p, batch, s);
+    else launch_small<4>(map_a, map_b, p, batch, s);
 }
 
 }  // namespace lb
