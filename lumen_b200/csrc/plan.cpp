@@ -109,6 +109,12 @@ lb_tensor bind(const lb_plan& p, int id, void* ws, void* const* in, void* const*
     return t;
 }
 
+size_t view_bytes(const lb_tensor& t) {
+    size_t n = 1;
+    for (int d = 0; d < t.rank; d++) n *= (size_t)t.shape[d];
+    return n * dtype_size(t.dtype);
+}
+
 std::unique_ptr<lb_plan> parse_plan(const std::string& text) {
     auto plan = std::make_unique<lb_plan>();
     std::vector<lb_fusion*> modules;
@@ -173,6 +179,9 @@ std::unique_ptr<lb_plan> parse_plan(const std::string& text) {
                 s.scratch = std::stoi(tok.at(4));
                 ints(6, std::stoul(tok.at(5)));
                 if (s.fusion->scratch_bytes && s.scratch < 0) fail(LB_ERR_INVALID, "plan: fusion " + s.label + " needs scratch");
+                // (a text written by a library whose kernels cut the same module into fewer slices)
+                if (s.scratch >= 0 && (s.scratch >= (int)plan->views.size() || view_bytes(plan->views[s.scratch].t) < s.fusion->scratch_bytes))
+                    fail(LB_ERR_INVALID, "plan: the scratch of fusion " + s.label + " is smaller than its kernel needs: lower the module again");
             } else if (kind == "multi") {  // s multi <label> <module> <n_groups> <tensor ids, group after group>
                 s.kind = MULTI;
                 int m = std::stoi(tok.at(3));
@@ -251,12 +260,6 @@ int copy_form(const lb_tensor& src, const lb_tensor& dst) {
     if (row_major(src) && row_major(dst)) return 0;
     if (src.rank == 2 && dst.rank == 2 && src.stride[1] == 1 && dst.stride[1] == 1 && src.stride[0] >= src.shape[1] && dst.stride[0] >= dst.shape[1]) return 1;
     return 2;
-}
-
-size_t view_bytes(const lb_tensor& t) {
-    size_t n = 1;
-    for (int d = 0; d < t.rank; d++) n *= (size_t)t.shape[d];
-    return n * dtype_size(t.dtype);
 }
 
 // The side stream and events of the plan's collectives, made on the first run that reaches one.

@@ -291,6 +291,28 @@ def test_row_and_column_reductions_in_one_kernel(cuda, shape, dtype):
     assert (np.abs(q - (want * want).sum(0)) <= (half + 2e-5) * (want * want).sum(0)).all()
 
 
+# where the threads of a row and the blocks of an SM change (two vectors of eight bytes for 16 bits from 1024 columns on; one vector of 16 from
+# 2^21 elements of float32 on), and more row blocks than slices
+@pytest.mark.parametrize("dtype, shape", [("float32", s) for s in ((4100, 512), (2100, 1000), (1400, 1536), (700, 3072), (600, 4096), (420, 5000))]
+                         + [("bfloat16", s) for s in ((2000, 1024), (1000, 2304), (900, 2600), (400, 5000), (300, 8192), (3000, 512))])
+def test_threads_of_rows_with_column_sums(cuda, dtype, shape):
+    """Row and column sums of one kernel against float64: `cols` terms of a row in any order, `rows` of a column, each within
+    their number's root times 2^-24 of the sum of magnitudes in practice, four times that allowed."""
+    rows, cols = shape
+    x = torch.randn(shape, generator=torch.Generator(device=cuda).manual_seed(cols), device=cuda).to(getattr(torch, dtype))
+
+    def program(a):
+        w = a.to("float32")
+        r = prims.reduce_sum(w, (1,), "float32")
+        q = prims.reduce_sum(w * w, (1,), "float32")
+        return r, q, prims.reduce_sum(w * r.reshape(rows, 1), (0,), "float32"), prims.reduce_sum(w, (0,), "float32")
+
+    r, q, c, s = (to_numpy(t).astype(np.float64) for t in Fusion(tracer.trace(program, (dtype, shape)))(x))
+    x64 = x.double().cpu().numpy()
+    near = lambda got, terms, axis: (np.abs(got - terms.sum(axis)) <= 4 * terms.shape[axis] ** 0.5 * 2.0**-24 * np.abs(terms).sum(axis)).all()
+    assert near(r, x64, 1) and near(q, x64 * x64, 1) and near(c, x64 * r[:, None], 0) and near(s, x64, 0)
+
+
 # widths whose vectors are one or two elements: one thread per row up to a whole block, remainders of a thread's share
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("rows,cols", [(3, 1), (70, 15), (9, 17), (33, 257), (5, 511), (5, 514), (7, 3001), (4, 4097), (3, 8190), (2, 16383)])

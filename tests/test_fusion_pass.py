@@ -67,6 +67,20 @@ def test_small_column_and_row_reductions_do_not_share_a_kernel():
     same_values(g, fused, [np.random.default_rng(2).standard_normal((128, 64), dtype=np.float32)])
 
 
+def test_small_norms_and_their_column_sums_share_a_kernel():
+    """Two row sums and more, which the column sums' operands depend on: one kernel whatever the size."""
+    def program(x, g):
+        c = x - prims.reduce_sum(x, (1,), "float32").reshape(24, 1) * (1.0 / 832)
+        r = prims.rsqrt(prims.reduce_sum(c * c, (1,), "float32").reshape(24, 1) * (1.0 / 832) + 1e-5)
+        return c * r, prims.reduce_sum(c * r * g, (0,), "float32"), prims.reduce_sum(g, (0,), "float32")
+
+    g = tracer.trace(program, ("float32", (24, 832)), ("float32", (24, 832)))
+    fused = fuse(g)
+    assert len(fusions(fused)) == 1 and not bare(fused)
+    rng = np.random.default_rng(5)
+    same_values(g, fused, [rng.standard_normal((24, 832), dtype=np.float32) for _ in range(2)])
+
+
 def test_gemm_takes_its_elementwise_tail_as_an_epilogue():
     dims = (((1,), (0,)), ((), ()))
 

@@ -245,6 +245,23 @@ def test_weights_of_much_larger_products_are_transposed(m, n, k, copied):
     assert [label for _, label in steps] == compile_graph(g).labels == ["weight_transpose"] * copied + ["dot_general"]
 
 
+def test_a_plan_text_with_too_little_scratch_is_refused():
+    """Partial sums take what the library's kernels need now, whatever wrote the text."""
+    from lumen_b200.compiler import compile_graph
+
+    g = tracer.trace(lambda x: F.sum(x, 0), ("float32", (4096, 512)))
+    lines = compile_graph(g).text.splitlines(keepends=True)
+    (at,) = [i for i, line in enumerate(lines) if line.startswith("t ") and " uint8 " in line]
+    lib, plan = _bind(), ctypes.c_void_p()
+    _lib.check(lib.lb_plan_create("".join(lines).encode(), ctypes.byref(plan)))
+    lib.lb_plan_destroy(plan)
+    words = lines[at].split()
+    words[6] = str(int(words[6]) - 4)
+    lines[at] = " ".join(words) + "\n"
+    with pytest.raises(_lib.LumenError, match="scratch"):
+        _lib.check(lib.lb_plan_create("".join(lines).encode(), ctypes.byref(plan)))
+
+
 @pytest.mark.parametrize("shapes, chained, launches", [
     ([(64, 64, 64), (128, 32, 512)], False, 1), ([(64, 64, 64)] * 2, True, 2), ([(64, 64, 64)] * 5, False, 2), ([(64, 0, 64), (64, 64, 0)], False, 1),
     ([(1088, 1152, 64), (64, 64, 64), (64, 64, 64)], False, 2)])  # 17 x 18 tiles of 64 x 64: two for each of 148 SMs, a launch of their own
