@@ -454,9 +454,9 @@ class Lowering:
         """`b` [K, N], or a transposed copy of it. A weight whose K rows lie 8 KB or more apart (N contiguous, N >= 4096
         16-bit elements) is a slow TMA operand: every 128-byte row of a tile comes from a different DRAM page and the
         power-of-two stride camps on few L2 slices. The copy pays where the product is much larger than the weight, M from
-        32 K on; us as it is / with the copy, A with M contiguous: [131072, 4096, 1024] 793 / 728, [65536, 8192, 2048]
-        1604 / 1568, [32768, 4096, 1024] 201 / 189, but [16384, 4096, 1024] 105 / 107, [8192, 4096, 1024] 49.0 / 52.5,
-        [2048, 8192, 256] 13.8 / 17.0, [1152, 4608, 64] 6.9 / 8.5. The copy's rows are K long: the tensor cores read them
+        32 K on; us as it is / with the copy, A with M contiguous: [131072, 4096, 1024] 1029 / 930, [65536, 8192, 2048]
+        1774 / 1663, [32768, 4096, 1024] 228 / 216, but [16384, 4096, 1024] 113 / 110, [8192, 4096, 1024] 56.6 / 60.5,
+        [2048, 8192, 256] 17.9 / 21.8, [1152, 4608, 64] 10.1 / 11.7. The copy's rows are K long: the tensor cores read them
         only if K is a multiple of 8."""
         k, n = b.shape
         size = G.SIZE_OF[b.dtype]

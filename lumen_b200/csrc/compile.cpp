@@ -651,7 +651,7 @@ struct Lowering {
         if (dot->ints("rhs_contracting")[0] == 1) std::swap(b.shape[0], b.shape[1]), std::swap(b.strides[0], b.strides[1]);
         // A [K, N] weight whose K rows lie 8 KB or more apart (N contiguous, N >= 4096 16-bit elements) is a slow TMA
         // operand: every 128-byte row of a tile comes from a different DRAM page. Where the product is much larger (M from 32 K on,
-        // [131072, 4096, 1024] 793 -> 728 us; [8192, 4096, 1024] would go from 49.0 to 52.5) it is transposed first, and read
+        // [131072, 4096, 1024] 1029 -> 930 us; [8192, 4096, 1024] would go from 56.6 to 60.5) it is transposed first, and read
         // through the transposed view: rows of K elements, which the tensor cores take only if K is a multiple of 8.
         {
             const int64_t k = b.shape[0], n = b.shape[1];

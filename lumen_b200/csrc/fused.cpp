@@ -104,7 +104,9 @@ static void launch(lb_fusion* f, const lb_tensor* tensors, int n, void* scratch,
     const int64_t together = (int64_t)k.rows_per_block * k.row_period;
     int64_t row_blocks = (k.rows + together - 1) / together * k.row_period;
     int per_sm = k.per_sm ? k.per_sm : std::max(1, 2048 / k.threads);
-    int64_t grid = std::min<int64_t>(row_blocks, (int64_t)dev.sms * per_sm / k.row_period * k.row_period);
+    int64_t most = (int64_t)dev.sms * per_sm;
+    if (k.row_period > 1) most = most / k.row_period * k.row_period;
+    int64_t grid = std::min<int64_t>(row_blocks, most);
     launch_kernel(fn.function, grid, 1, k.threads, stream, params.data(), "cuLaunchKernelEx(fused_kernel)");
 }
 
