@@ -128,7 +128,7 @@ template <class T, int V, class I> __device__ __forceinline__ void ldv_shifted(c
         #pragma unroll
         for (int k = 0; k < V; k++) { const I i = at - shift + k; dst[k] = __ldg(p + (i < 0 ? 0 : i < total ? i : total - 1)); }
     } else {
-        u32 w[8];
+        __align__(16) u32 w[8];
         ldv_within<T, V, I>(p, at >= V ? at - V : at, total, (T*)w);
         ldv_within<T, V, I>(p, at, total, (T*)(w + 4));
         const int from = B - shift * (int)sizeof(T);  // first byte, in (0, 16]
