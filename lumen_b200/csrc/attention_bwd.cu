@@ -214,6 +214,8 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
                 mbar_expect_tx(&t2_full[b], kStream);
                 for (int d = 0; d < DB; d++) tma_load_4d(st2 + b * kStream + d * kTBlock, &map_t2, &t2_full[b], d * 64, t_head, row0, batch);
             }
+            ok = ok && mbar_wait_ring<S1>(t1_empty, (uint32_t)n_iter, abort_flag) && mbar_wait_ring<S2>(t2_empty, (uint32_t)n_iter, abort_flag);
+            if (!DKDV && ok) mbar_wait(z_free, (uint32_t)(n_iter - 1) & 1, abort_flag);
         }
       } else if (warp == 1) {
         if (n_iter > 0) {  // the whole warp: the operands stay in uniform registers

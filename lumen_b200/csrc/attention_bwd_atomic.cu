@@ -170,6 +170,7 @@ attention_bwd_atomic_kernel(const __grid_constant__ CUtensorMap map_k, const __g
                 tma_load_4d(sq + st * kTile, &map_q, &t_full[st], 0, head * group + hh, t * BT, batch);
                 tma_load_4d(sdo + st * kTile, &map_do, &t_full[st], 0, head * group + hh, t * BT, batch);
             }
+            if (ok && mbar_wait_ring<STAGES>(t_empty, (uint32_t)n_iter, abort_flag)) mbar_wait(pz_free, (uint32_t)(n_iter - 1) & 1, abort_flag);
         }
       } else if (warp == 1) {
         if (n_iter > 0) {  // the whole warp: the operands stay in uniform registers

@@ -310,6 +310,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 mbar_expect_tx(&v_full[st], kTile);
                 for (int d = 0; d < DB; d++) tma_load_4d(sv + st * kTile + d * kHalf, &map_v, &v_full[st], d * 64, kv_head, j * BKV, batch);
             }
+            if (ok && mbar_wait_ring<NS>(k_empty, (uint32_t)n_kv, abort_flag)) mbar_wait_ring<NS>(v_empty, (uint32_t)n_kv, abort_flag);
         }
     } else if (warp == 1) {
         if (n_kv > 0) {  // the whole warp: the operands stay in uniform registers
@@ -532,6 +533,7 @@ attention_fwd_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
                 if (!next_cta_answer(next_slot + slot * 16, next)) break;
                 w = fwd_work(p, next);
             }
+            if (ok && loads > 0 && mbar_wait(q_empty, (loads - 1) & 1, abort_flag) && mbar_wait_ring<NS>(k_empty, kv, abort_flag)) mbar_wait_ring<NS>(v_empty, kv, abort_flag);
         }
       } else if (warp == 1) {
         {  // the whole warp: the operands stay in uniform registers

@@ -361,6 +361,7 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                     }
                 }
             }
+            if (ok) mbar_wait_ring<STAGES>(empty, phase * STAGES + stage, abort_flag);
         }
     } else if (warp == 1) {
         // ---- MMA issuer: the whole warp, so that the operands stay in uniform registers ----
@@ -555,14 +556,7 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     }
                 }
             }
-            // every commit aimed at this CTA's `empty` barriers has to land before the CTA may exit
-            for (int s = 0; s < PSTAGES && ok; s++) {
-                ok = mbar_wait(&empty[stage], phase ^ 1, abort_flag);
-                if (++stage == PSTAGES) {
-                    stage = 0;
-                    phase ^= 1;
-                }
-            }
+            if (ok) mbar_wait_ring<PSTAGES>(empty, phase * PSTAGES + stage, abort_flag);
         }
     } else if (warp == 1) {
         // ---- MMA issuer (leader CTA only): the whole warp, so that the operands stay in uniform registers ----

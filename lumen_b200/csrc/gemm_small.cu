@@ -77,9 +77,10 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
     if (warp == 0) {
         if (lane == 0) {
+            bool ok = true;
             for (int i = 0; i < num_kb; i++) {
                 const int st = i % STAGES, k = (kb0 + i) * BK;
-                if (!mbar_wait(&empty[st], ((uint32_t)(i / STAGES) & 1) ^ 1, abort_flag)) break;
+                if (!(ok = mbar_wait(&empty[st], ((uint32_t)(i / STAGES) & 1) ^ 1, abort_flag))) break;
                 mbar_expect_tx(&full[st], kStageA + kStageB);
                 if (!p.a_mn_major) {
                     tma_load_3d(sa + st * kStageA, &map_a, &full[st], k, m_blk * BM, b);  // box {64 k, 128 m}
@@ -89,6 +90,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 if (!p.b_mn_major) tma_load_3d(sb + st * kStageB, &map_b, &full[st], k, n_blk * BN, b);  // box {64 k, 64 n}
                 else tma_load_3d(sb + st * kStageB, &map_b, &full[st], n_blk * BN, k, b);                 // box {64 n, 64 k}
             }
+            if (ok) mbar_wait_ring<STAGES>(empty, (uint32_t)num_kb, abort_flag);
         }
     } else if (warp == 1) {  // the whole warp: the operands stay in uniform registers
         const bool leader = elect_one();

@@ -73,6 +73,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     return false;
 }
 
+// Waits until the last commits aimed at a ring of barriers have arrived, `next` tiles having passed through it: what the producer does
+// before it leaves. A commit arrives on its own, and nothing says in which order two of them do, so that a later one's arrival (the
+// accumulator's) does not show that an earlier one will not reach shared memory that belongs to another block by then.
+template <int STAGES>
+__device__ __forceinline__ bool mbar_wait_ring(uint64_t* empty, uint32_t next, volatile int* abort_flag) {
+    for (int i = 0; i < STAGES; i++, next++)
+        if (!mbar_wait(&empty[next % STAGES], (next / STAGES & 1) ^ 1, abort_flag)) return false;
+    return true;
+}
+
 // ---- TMA --------------------------------------------------------------------------------------------------
 // Tile load into this CTA's shared memory, completion counted in bytes on `bar`. Coordinates innermost first; the
 // innermost one times the element size must be a multiple of 16 bytes (callers only pass multiples of the box).

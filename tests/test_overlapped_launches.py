@@ -87,3 +87,16 @@ def test_generated_kernels_wait_before_their_first_access(program, shapes, optio
         for pointer in reads:
             first = next(u for u in uses if re.match(rf"{pointer}\b", u))
             assert re.fullmatch(rf"{pointer} = behind_wait\((?:{pointer}|table\.ptr\[group\]\[\d+\]), tid\);", first), first
+
+
+def test_every_commit_is_waited_for():
+    """A block leaves once the last commit aimed at each of its barriers has arrived: those that say that something is there (`_full`)
+    are waited for by what reads it, the others, which hand a buffer back, by the producer behind its last tile's load."""
+    waits = {}
+    for path in CSRC.glob("*.cu"):
+        for name, _, body in kernels(re.sub(r"//[^\n]*", "", path.read_text())):
+            committed = set(re.findall(r"mma_commit(?:_pair)?\(&?(\w+)", body))
+            if committed:
+                after = body[body.rindex("tma_load") :]
+                waits[name] = {c for c in committed if not c.endswith("_full") and not re.search(rf"mbar_wait(?:_ring<\w+>\({c},|\({c}, [^;]* - 1\))", after)}
+    assert len(waits) >= 7 and not any(waits.values()), waits
