@@ -413,6 +413,24 @@ def test_rows_at_any_address(cuda, rows, cols):
     assert torch.equal(u, x * g + b) and torch.equal(v, (x - b).float())
 
 
+def test_rows_at_any_address_under_capture(cuda):
+    """A program that has run on aligned tensors is captured on others, which take another kernel, and replays them."""
+    rows, cols = 2503, 3001
+    x = torch.randn((rows, cols), generator=torch.Generator(device=cuda).manual_seed(0), device=cuda).bfloat16()
+    kernel = Fusion(tracer.trace(lambda a: F.relu(a * 0.375), ("bfloat16", (rows, cols))))
+    assert "PERIOD" in kernel.source
+    aligned, off = torch.empty_like(x), torch.cat([x.new_zeros(1), x.flatten()])[1:].reshape(rows, cols)
+    out = torch.empty(rows * cols + 1, device=cuda, dtype=torch.bfloat16)[1:].reshape(rows, cols)
+    kernel(x, out=[aligned])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        kernel(off, out=[out])
+    out.zero_()
+    graph.replay()
+    assert torch.equal(out, torch.relu(x * 0.375)) and torch.equal(out, aligned)
+
+
 def column_sums_in_slices(x):
     """float32 column sums in the order of the two-pass column reduction: slices of at least 64 rows, eight row lanes each that add every
     eighth row, eight slice lanes that add every eighth slice, lanes in order."""
