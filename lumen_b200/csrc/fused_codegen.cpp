@@ -623,6 +623,8 @@ class Generator {
                 while (p < t && p < 32) p *= 2;
                 return t > 32 ? (t + 31) / 32 * 32 : p;
             };
+            const int64_t one = threads_for(1), two = threads_for(2), in_ones = 1024 / one * one, in_twos = 1024 / two * two;
+            const bool ones = one == 32 || (one >= 128 && (in_ones > in_twos || in_ones == 1024));
             int64_t warps = 0;  // an SM, at least; otherwise up to 16, 128 registers a thread or more, down to 64 at 1024 threads
             T_ = (int)threads_for(chunks);
             if (min_size == 2 && VEC_ >= 4 && C_ >= 1024 && (C_ <= 2048 || C_ > 3072 || R_ * C_ >= 1 << 21)) {
@@ -633,12 +635,14 @@ class Generator {
                 T_ = (int)threads_for(chunks);
                 if (T_ > 288 && T_ <= 384 && C_ % (T_ * 8) != 0) T_ = (int)threads_for(3);  // (the last chunk a part: 2600 wide as fast, few rows faster)
                 else warps = 16;
-            } else if (min_size == 4 && VEC_ == 4 && nvec <= 1024 && R_ * C_ >= 1 << 21) {
+            } else if (min_size == 4 && VEC_ == 4 && nvec <= 1024 && R_ * C_ >= 1 << 21 && held_columns() <= 16 && (ones || col_reduces_.size() <= 4)) {
                 // float32 rows: one vector a thread where that makes a warp or four and more, 32 warps an SM; two where more threads fit so,
                 // or as many but not all 1024. us, two vectors and 16 warps -> so: 16384 x 512 44 -> 33, 8192 x 1024 46 -> 35, 5461 x 1536 58 -> 40,
                 // 4096 x 2048 50 -> 40, 2532 x 3312 73 -> 55, 2048 x 4096 61 -> 44; fewer than two million elements are up to 1.16 slower.
-                const int64_t one = threads_for(1), in_ones = 1024 / one * one, in_twos = 1024 / T_ * T_;
-                if (one == 32 || (one >= 128 && (in_ones > in_twos || in_ones == 1024))) T_ = (int)one;
+                // Such threads have 64 registers. 1 to 4 operands with 2 to 12 column sums and none or two operands by column, 2^23 elements, times
+                // two vectors and 16 warps: 0.51 - 1.03 within the bound above, 0.95 - 1.23 beyond it; two vectors in 64 to 72 registers (1536 and
+                // 3312 columns) 0.74 - 0.96 with up to four column sums, 0.82 - 1.12 with five, 0.82 - 1.29 with eight, 1.1 - 1.8 with more.
+                T_ = (int)(ones ? one : two);
                 if (T_ >= 128 || one == 32) warps = 32;
             } else if (T_ > 256 && T_ <= 384) {
                 // A block of 288 to 384 threads would be alone on its SM with 9 to 12 warps: twelve elements a thread instead make two of
@@ -663,6 +667,14 @@ class Generator {
             if (g_.type(v).numel() >= (1LL << 31) - 4096) wide_index_ = true;
         if (multi_) wide_index_ = true;  // a group's row count is a run-time value
         pair_ = VEC_ >= 2 && computes_bf16();
+    }
+
+    // What a thread of a mixed kernel holds for each of its columns: a sum for each column total, the operands by column, and those over the
+    // space twice (the row in flight and the one behind it)
+    int held_columns() const {
+        int held = (int)col_reduces_.size();
+        for (int v : g_.inputs) held += g_.type(v).numel() == R_ * C_ ? 2 : g_.type(v).numel() == C_;
+        return held;
     }
 
     // Whether rows of an odd width are read in whole vectors all the same. Their elements start at any address, but all tensors over
