@@ -409,7 +409,7 @@ class Lowering:
         (lc,), (rc,) = p["lhs_contracting"], p["rhs_contracting"]
         a = lhs if lc == 1 else View(lhs.buffer, lhs.offset, lhs.dtype, lhs.shape[::-1], lhs.strides[::-1])
         b = rhs if rc == 0 else View(rhs.buffer, rhs.offset, rhs.dtype, rhs.shape[::-1], rhs.strides[::-1])
-        b = self.k_major_copy(b, a.shape[0])
+        b = self.k_major_copy(b, a)
         out = self.fresh(out_value)
         nbytes = gemm_scratch_bytes(a, b)
         scratch = View(self.new_buffer(nbytes), 0, "uint8", (nbytes,), (1,)) if nbytes else None
@@ -450,17 +450,27 @@ class Lowering:
         self.views[value] = copy
         return copy
 
-    def k_major_copy(self, b: View, m: int) -> View:
+    def k_major_copy(self, b: View, a: View) -> View:
         """`b` [K, N], or a transposed copy of it. A weight whose K rows lie 8 KB or more apart (N contiguous, N >= 4096
         16-bit elements) is a slow TMA operand: every 128-byte row of a tile comes from a different DRAM page and the
-        power-of-two stride camps on few L2 slices. The copy pays where the product is much larger than the weight, M from
-        32 K on; us as it is / with the copy, A with M contiguous: [131072, 4096, 1024] 1029 / 930, [65536, 8192, 2048]
-        1774 / 1663, [32768, 4096, 1024] 228 / 216, but [16384, 4096, 1024] 113 / 110, [8192, 4096, 1024] 56.6 / 60.5,
-        [2048, 8192, 256] 17.9 / 21.8, [1152, 4608, 64] 10.1 / 11.7. The copy's rows are K long: the tensor cores read them
-        only if K is a multiple of 8."""
-        k, n = b.shape
+        power-of-two stride camps on few L2 slices. The copy pays where the product is much larger than the weight. Time with
+        the copy / without it, N of 4096 to 32768, medians of four runs in turn:
+
+            M           K = 128        256            512 to 4096    512 to 4096, M contiguous in A
+            8192                                      1.04 - 1.18    0.96 - 1.07
+            12288                                     0.96 - 1.08    0.87 - 1.05
+            16384                      0.96 - 1.04    0.91 - 1.06    0.91 - 1.05
+            24576                      0.96 - 1.02    0.88 - 1.05    0.89 - 1.03
+            32768       0.93 - 1.15    0.95 - 1.02    0.94 - 1.00    0.86 - 0.98
+
+        K of 64 and less is copied from M of 32 K on, where both are one launch more or less: [2048, 4096, 64] 10.0 / 11.5 us,
+        [16384, 4096, 64] 43 / 45, [131072, 4096, 64] 298 / 301. The copy's rows are K long: the tensor cores read them only if K is
+        a multiple of 8."""
+        (k, n), m = b.shape, a.shape[0]
         size = G.SIZE_OF[b.dtype]
-        if not (b.strides == (n, 1) and size == 2 and n * size >= 8192 and k * n * size <= (64 << 20) and k % 8 == 0 and m >= 32 * k and m * n * k >= 1 << 29):
+        if not (b.strides == (n, 1) and size == 2 and n * size >= 8192 and k * n * size <= (64 << 20) and k % 8 == 0):
+            return b
+        if not (m >= (12288 if a.strides[0] == 1 and k >= 512 else 24576) if k >= 256 else k <= 64 and m >= 32 * k and m * n * k >= 1 << 29):
             return b
         copy = View(self.new_buffer(k * n * size), 0, b.dtype, (n, k), (k, 1))
         self.touch(b)

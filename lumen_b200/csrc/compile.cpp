@@ -650,14 +650,15 @@ struct Lowering {
         if (dot->ints("lhs_contracting")[0] == 0) std::swap(a.shape[0], a.shape[1]), std::swap(a.strides[0], a.strides[1]);
         if (dot->ints("rhs_contracting")[0] == 1) std::swap(b.shape[0], b.shape[1]), std::swap(b.strides[0], b.strides[1]);
         // A [K, N] weight whose K rows lie 8 KB or more apart (N contiguous, N >= 4096 16-bit elements) is a slow TMA
-        // operand: every 128-byte row of a tile comes from a different DRAM page. Where the product is much larger (M from 32 K on,
-        // [131072, 4096, 1024] 1029 -> 930 us; [8192, 4096, 1024] would go from 56.6 to 60.5) it is transposed first, and read
-        // through the transposed view: rows of K elements, which the tensor cores take only if K is a multiple of 8.
+        // operand: every 128-byte row of a tile comes from a different DRAM page. Where the product is much larger it is transposed first,
+        // and read through the transposed view: rows of K elements, which the tensor cores take only if K is a multiple of 8. The lines are
+        // those of k_major_copy in compiler.py, which gives their figures (times the product without the copy: M = 24576 0.88 - 1.05, 8192 up to
+        // 1.18).
         {
-            const int64_t k = b.shape[0], n = b.shape[1];
+            const int64_t m = a.shape[0], k = b.shape[0], n = b.shape[1];
             const int size = dtype_size(b.dtype);
-            if (b.strides[0] == n && b.strides[1] == 1 && size == 2 && n * size >= 8192 && k * n * size <= (64LL << 20) && k % 8 == 0 && a.shape[0] >= 32 * k &&
-                a.shape[0] * n * k >= 1 << 29) {
+            const bool far_rows = b.strides[0] == n && b.strides[1] == 1 && size == 2 && n * size >= 8192 && k * n * size <= (64LL << 20) && k % 8 == 0;
+            if (far_rows && (k >= 256 ? m >= (a.strides[0] == 1 && k >= 512 ? 12288 : 24576) : k <= 64 && m >= 32 * k && m * n * k >= 1 << 29)) {
                 View copy = fresh(b.dtype, {n, k});
                 push_step("s transpose weight_transpose " + std::to_string(tid(b)) + " " + std::to_string(tid(copy)) + "\n");
                 b = copy;

@@ -8,7 +8,7 @@ import json
 
 import pytest
 
-from lumen_b200 import _lib, autograd, tracer
+from lumen_b200 import _lib, autograd, prims, tracer
 from lumen_b200 import functional as F
 from lumen_b200.attention_pass import match_attention
 from lumen_b200.fusion_pass import fuse
@@ -241,6 +241,19 @@ def test_weights_of_much_larger_products_are_transposed(m, n, k, copied):
     from lumen_b200.compiler import compile_graph
 
     g = tracer.trace(lambda x, w: F.matmul(x, w, "float32", "bfloat16"), ("bfloat16", (m, k)), ("bfloat16", (k, n)))
+    steps, _ = plan_of(fuse(clean(g)))
+    assert [label for _, label in steps] == compile_graph(g).labels == ["weight_transpose"] * copied + ["dot_general"]
+
+
+@pytest.mark.parametrize("m, n, k, across, copied", [
+    (24576, 4096, 256, False, True), (24575, 4096, 256, False, False), (24576, 4096, 248, False, False), (131072, 8192, 128, False, False), (12288, 4096, 256, True, False),
+    (12288, 4096, 512, True, True), (12280, 4096, 512, True, False), (12288, 4096, 512, False, False), (24576, 8192, 4096, False, True), (24576, 8200, 4096, False, False)])
+def test_weights_are_transposed_where_it_pays(m, n, k, across, copied):
+    """By M and K, and by which way the other operand lies."""
+    from lumen_b200.compiler import compile_graph
+
+    g = tracer.trace(lambda x, w: F.matmul(prims.transpose(x, (1, 0)) if across else x, w, "float32", "bfloat16"),
+                     ("bfloat16", (k, m) if across else (m, k)), ("bfloat16", (k, n)))
     steps, _ = plan_of(fuse(clean(g)))
     assert [label for _, label in steps] == compile_graph(g).labels == ["weight_transpose"] * copied + ["dot_general"]
 
