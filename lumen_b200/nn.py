@@ -117,41 +117,40 @@ def _ln_forward(x, w, b, eps):
 
 def layer_norm(tape: Tape, x: TracedTensor, w: TracedTensor, b: TracedTensor, eps: float = 1e-5) -> TracedTensor:
     """Pre-LayerNorm with scale and bias over the last dimension, statistics in float32; one `row` fusion that also
-    saves each row's mean and 1/std for the backward (a row fusion for dx, a column reduction for dw, db)."""
+    saves each row's mean and 1/std for the backward: one fusion for dx, dw and db, or a row fusion for dx and a column
+    reduction for dw, db."""
     rows, cols = x.shape
     y, mean, rstd = fused(lambda a, ww, bb: _ln_forward(a, ww, bb, eps), x, w, b, name="row", label="layer_norm")
 
     def vjp(dy, *_, pending=None):
-        def dx_body(g, a, ww, mu, rs, *acc):
-            gf = g.float() * ww.float()
-            xhat = (a.float() - mu.reshape(rows, 1)) * rs.reshape(rows, 1)
+        def normalised(a, mu, rs):
+            return (a.float() - mu.reshape(rows, 1)) * rs.reshape(rows, 1)
+
+        def dx_of(g, xhat, a, ww, rs, acc):
+            gf = g * ww.float()
             c1 = F.mean(gf, -1, keepdim=True)
             c2 = F.mean(gf * xhat, -1, keepdim=True)
             dx = ((gf - c1 - xhat * c2) * rs.reshape(rows, 1)).to(a.dtype)
             return acc[0] + dx if acc else dx  # the residual stream's cotangent, added as `grad_add` would
 
-        def dwb_body(g, a, mu, rs):
-            gf = g.float()
-            xhat = (a.float() - mu.reshape(rows, 1)) * rs.reshape(rows, 1)
-            return (prims.reduce_sum(gf * xhat, (0,), "float32").to(a.dtype), prims.reduce_sum(gf, (0,), "float32").to(a.dtype))
+        def dwb_of(g, xhat, a):
+            return tuple(prims.reduce_sum(t, (0,), "float32").to(a.dtype) for t in (g * xhat, g))
+
+        def body(g, a, ww, mu, rs, *acc):
+            g32, xhat = g.float(), normalised(a, mu, rs)
+            return dx_of(g32, xhat, a, ww, rs, acc), *dwb_of(g32, xhat, a)
 
         extra = [pending] if pending is not None else []
-        def body(g, a, ww, mu, rs, *acc):
-            g32 = g.float()
-            gf = g32 * ww.float()
-            xhat = (a.float() - mu.reshape(rows, 1)) * rs.reshape(rows, 1)
-            c1 = F.mean(gf, -1, keepdim=True)
-            c2 = F.mean(gf * xhat, -1, keepdim=True)
-            dx = ((gf - c1 - xhat * c2) * rs.reshape(rows, 1)).to(a.dtype)
-            dw, db = (prims.reduce_sum(t, (0,), "float32").to(a.dtype) for t in (g32 * xhat, g32))
-            return acc[0] + dx if acc else dx, dw, db
-
-        # One kernel, which reads dy and x once: a 2-layer float32 step of 512 tokens 288 -> 276 us, 6 layers of 16384 x 1024 bfloat16 13.44 ->
-        # 13.30 ms. Between, with several steps in flight, its blocks cost more than the second read (720 x 512 bfloat16 236 -> 240 us).
-        if not 1 << 17 < rows * cols < 1 << 20 and FusionPass.one_pass_pays(rows, cols, x.dtype != "float32", 2):
+        # One kernel reads dy and x once and takes two launches less. Times of a 2-layer training step with it, over the step with two, alone and
+        # with three steps in flight: float32, 128 to 1024 columns, 2^14 to 2^20 elements 0.95 - 1.00 and 0.95 - 1.00; 16 bits up to 256 columns
+        # 0.94 - 0.98 and 0.94 - 1.00; wider up to 2^17 elements 0.94 - 0.98 and 0.97 - 1.02, from 2^22 on 0.99 - 1.01 and 1.00 - 1.01; between
+        # 0.98 - 1.02 and 1.00 - 1.04, its blocks of many registers in the other steps' way: there the kernels stay apart.
+        between = x.dtype != "float32" and cols > 256 and 1 << 17 < rows * cols < 1 << 22
+        if not between and FusionPass.one_pass_pays(rows, cols, x.dtype != "float32", 2):
             return fused(body, dy, x, w, mean, rstd, *extra, name="row", label="layer_norm_backward")
-        dx = fused(dx_body, dy, x, w, mean, rstd, *extra, name="row", label="layer_norm_backward")
-        dw, db = fused(dwb_body, dy, x, mean, rstd, name="reduction", label="layer_norm_weight_grads")
+        dx = fused(lambda g, a, ww, mu, rs, *acc: dx_of(g.float(), normalised(a, mu, rs), a, ww, rs, acc), dy, x, w, mean, rstd, *extra,
+                   name="row", label="layer_norm_backward")
+        dw, db = fused(lambda g, a, mu, rs: dwb_of(g.float(), normalised(a, mu, rs), a), dy, x, mean, rstd, name="reduction", label="layer_norm_weight_grads")
         return dx, dw, db
 
     vjp.adds_into = 0

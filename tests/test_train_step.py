@@ -65,6 +65,18 @@ def test_step_lowers_to_a_plan():
     assert plan.workspace_bytes % 256 == 0
 
 
+@pytest.mark.parametrize("dtype, width, tokens, apart", [
+    ("float32", 128, 2048, False), ("float32", 512, 1024, False), ("bfloat16", 256, 2048, False), ("bfloat16", 384, 512, True), ("bfloat16", 512, 256, False),
+    ("bfloat16", 512, 8064, True), ("bfloat16", 512, 8192, False), ("bfloat16", 1024, 2048, True)])
+def test_layer_norm_gradients_in_one_kernel_or_two(dtype, width, tokens, apart):
+    """Apart where one kernel was measured slower: wide rows of 16 bits between 2^17 and 2^22 elements."""
+    cfg = T.Config(vocab=64, d_model=width, heads=width // 64, hidden=64, layers=1, seq=64, dtype=dtype, lr=1e-2)
+    g, _, _ = T.trace_train_step(cfg, tokens // 64)
+    labels = [n.params.get("label") for n in g.nodes if n.op == "fusion"]
+    norms = labels.count("layer_norm_backward")
+    assert norms >= 2 and labels.count("layer_norm_weight_grads") == norms * apart
+
+
 def test_reshape_views():
     assert reshape_view((6, 4), (12, 1), (2, 3, 2, 2)) == (36, 12, 2, 1)
     assert reshape_view((6, 4), (4, 1), (24,)) == (1,)
