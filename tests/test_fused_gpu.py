@@ -7,7 +7,7 @@ import torch
 import lumen_b200
 from lumen_b200 import functional as F
 from lumen_b200 import prims, tracer
-from lumen_b200.runtime import Fusion
+from lumen_b200.runtime import Fusion, desc
 from tests.helpers import BF16, bf16, run_oracle, to_numpy, to_torch
 
 pytestmark = pytest.mark.gpu
@@ -411,6 +411,37 @@ def test_rows_at_any_address(cuda, rows, cols):
     assert torch.equal(m, (x * r).amax(1)) and torch.equal(w, (x * r).float())
     u, v = run(bare, x, g, b)
     assert torch.equal(u, x * g + b) and torch.equal(v, (x - b).float())
+
+
+@pytest.mark.parametrize("rows,cols", [(50001, 129), (6300, 1001), (2503, 3001), (1601, 4095), (385, 16383), (97, 65533)])
+def test_odd_rows_count_their_own_elements(cuda, rows, cols):
+    """Sums of small whole numbers are exact in any order: every element of a row counts once and none of its neighbours' does, with
+    float32 operands beside the 16-bit ones (vectors of 32 bytes, a column operand moved by its elements)."""
+    gen = torch.Generator(device=cuda).manual_seed(cols)
+    x = torch.randint(0, 4, (rows, cols), generator=gen, device=cuda).bfloat16()
+    g, w = torch.randint(1, 5, (cols,), generator=gen, device=cuda).float(), torch.randint(0, 8, (rows, cols), generator=gen, device=cuda).float()
+
+    def program(x_, g_, w_):
+        z = (x_ * x_).to("float32") * g_ + w_
+        return z, prims.reduce_sum(z, (1,), "float32")
+
+    kernel = Fusion(tracer.trace(program, ("bfloat16", (rows, cols)), ("float32", (cols,)), ("float32", (rows, cols))))
+    assert "PERIOD" in kernel.source and "ldv_shifted<float, VEC, idx_t>" in kernel.source
+    z, total = kernel(x, g, w)
+    want = (x * x).float() * g + w
+    assert torch.equal(z, want) and torch.equal(total.double(), want.double().sum(1))
+
+
+@pytest.mark.parametrize("rows,cols", [(50001, 129), (2503, 3001), (1601, 4095), (97, 65533)])
+def test_odd_rows_in_place(cuda, rows, cols):
+    """The result over its operand: neighbours that a vector brings along are never written back."""
+    x = torch.randn((rows, cols), generator=torch.Generator(device=cuda).manual_seed(cols), device=cuda).bfloat16()
+    g = torch.randn((cols,), generator=torch.Generator(device=cuda).manual_seed(1), device=cuda).bfloat16()
+    kernel = Fusion("option inplace\n" + tracer.trace(lambda a, b: (a * b) * a, ("bfloat16", (rows, cols)), ("bfloat16", (cols,))).to_text())
+    assert "ldv_within_plain<u16, VEC, idx_t>" in kernel.source or cols < 1024  # (shorter rows without a sum are put together)
+    want = (x * g) * x
+    kernel.launch_raw([desc(t) for t in (x, g, x)])
+    assert torch.equal(x, want)
 
 
 def test_rows_at_any_address_under_capture(cuda):

@@ -382,6 +382,28 @@ def test_float32_products_of_one_launch_are_those_of_several(cuda, shapes):
         assert torch.equal(out, gemm(x[2 * i], x[2 * i + 1], torch.empty_like(out)))
 
 
+def test_batches_and_epilogues_of_one_launch(cuda):
+    """Batched products (one with a transposed operand) and a relu beside a plain product: each as it is alone."""
+    from lumen_b200.compiler import CompiledPlan, dense_strides
+    from lumen_b200.plan import Plan
+
+    products = [((3, 33, 65, 40), 1, False), ((1, 64, 64, 64), 0, False), ((2, 128, 17, 70), 0, True), ((5, 16, 32, 64), 1, True)]  # (batch, M, N, K), epilogue, B as [N, K]
+    lines, steps, x, outs = [], [], [], []
+    for i, ((batch, m, n, k), epilogue, across) in enumerate(products):
+        a, b = (to_torch(t, cuda) for t in operands(m, n, k, i, batch))
+        b = b.mT.contiguous().mT if across else b
+        x += [a, b]
+        outs.append(torch.full((batch, m, n), float("nan"), device=cuda))
+        for at, (t, base) in enumerate([(a, f"i{2 * i}"), (b, f"i{2 * i + 1}"), (outs[-1], f"o{i}")]):
+            lines.append(" ".join(map(str, ("t", 3 * i + at, "float32", base, 0, 3, *t.shape, *t.stride()))))
+        steps.append(f"s gemm dot_general {3 * i} {3 * i + 1} {3 * i + 2} {epilogue} -1 -1")
+    plan = Plan(CompiledPlan("\n".join([f"plan {len(x)} {len(outs)} 0", *lines, *steps, "end"]) + "\n", 0, len(x), len(outs)))
+    assert plan.lib.lb_plan_kernel_launches(plan.handle) == 1
+    plan.run(x, outs)
+    for i, (_, epilogue, _) in enumerate(products):
+        assert torch.equal(outs[i], gemm(x[2 * i], x[2 * i + 1], torch.empty_like(outs[i]), epilogue="relu" if epilogue else None))
+
+
 def test_a_float32_product_that_reads_anothers_result_comes_after_it(cuda):
     """The memory given to a run decides: here the first result lies where the second product's operand does, the third's result where
     the second reads."""

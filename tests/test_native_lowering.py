@@ -307,3 +307,16 @@ def test_long_products_that_narrow_tiles_fit_are_cut_on_large_tiles_only_where_t
     assert (lib.lb_gemm_step_scratch_bytes(m, n, k) > 0) == split
     if split:
         assert lib.lb_gemm_step_scratch_bytes(m, n, k) == lib.lb_gemm_scratch_bytes(m, n, k, 1)
+
+
+def test_products_into_donated_inputs_are_counted_where_they_lie():
+    """A product written into an input that its neighbour reads has a launch of its own, as in a run; without donation they share one."""
+    def program(x, y, z):
+        return F.matmul(z, y, "float32", "float32"), F.matmul(x, y, "float32", "float32")
+
+    g = fuse(clean(tracer.trace(program, *[("float32", (64, 64))] * 3)))
+    lib = _bind()
+    for donate, launches in (({1: 2}, 2), (None, 1)):
+        native = lower_native(g, donate=donate)
+        assert lib.lb_plan_kernel_launches(native) == launches
+        lib.lb_plan_destroy(native)
