@@ -629,8 +629,9 @@ class Generator {
             T_ = (int)threads_for(chunks);
             if (min_size == 2 && VEC_ >= 4 && C_ >= 1024 && (C_ <= 2048 || C_ > 3072 || R_ * C_ >= 1 << 21)) {
                 // Rows of 16 bits from 1024 columns on: two vectors of eight bytes a thread and as many blocks as 16 warps and more need, so
-                // that a block of 13 to 15 warps is not alone on its SM. (455 x 2304 9.9 -> 10.5: small ones of nine to twelve warps are left.) us, the sums above, one vector of 16 bytes a thread -> so: 2048 x 1024 12.9 ->
-                // 11.0, 4096 x 2048 32.6 -> 31.8, 3640 x 2304 42 -> 35, 2532 x 3312 52 -> 45, 1677 x 5000 48 -> 41, 1024 x 8192 58 -> 45.
+                // that a block of 13 to 15 warps is not alone on its SM. us, the sums above, one vector of 16 bytes a thread -> so: 2048 x 1024
+                // 12.9 -> 11.0, 4096 x 2048 32.6 -> 31.8, 3640 x 2304 42 -> 35, 2532 x 3312 52 -> 45, 1677 x 5000 48 -> 41, 1024 x 8192 58 -> 45.
+                // Few rows of 2049 to 3072 columns, whose blocks would have nine to twelve warps, are left: 455 x 2304 9.9 against 10.5.
                 VEC_ = 4, nvec = vectors(), chunks = 2;
                 T_ = (int)threads_for(chunks);
                 if (T_ > 288 && T_ <= 384 && C_ % (T_ * 8) != 0) T_ = (int)threads_for(3);  // (the last chunk a part: 2600 wide as fast, few rows faster)
@@ -1478,7 +1479,9 @@ class Generator {
     }
 
     // A thread with many narrow vectors of a row keeps four sums: one chain over 16 elements, where wider vectors or more threads make it
-    // four, had 1.35 times the error of a float32 sum over 3001. Shifted chunks, whose threads have as many elements, keep one a lane.
+    // four, had 1.35 times the error of a float32 sum over 3001. Shifted chunks, whose threads have as many elements, keep one a lane: which
+    // elements those are follows from the row's distance to an aligned address, so that equal rows at different places (modulo eight), or of a
+    // tensor that is not aligned, may differ in the last bits of a sum. The same call gives the same bits.
     int sums() const { return shifted_ ? VEC_ : VEC_ <= 2 && NCH_ > 4 ? 4 : 1; }
 
     // ---- emission ---------------------------------------------------------------------------------------

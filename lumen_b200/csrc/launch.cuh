@@ -4,7 +4,7 @@
 // has ended, before that one's memory is flushed and its end has been reported: launch, block setup (barriers, tensor memory,
 // descriptors) and the earlier kernel's last microsecond fall together. Every kernel launched this way calls `grid_wait` in
 // every thread, before it reads or writes memory that another kernel may touch and before any wait with a bound: it returns
-// once the kernels before it have completed and their writes are visible. As each of them did the same, that holds for the
+// once the kernels before it have completed and their writes are visible (and has no bound of its own). As each of them did the same, that holds for the
 // whole stream before it, and what is launched in the ordinary way afterwards is ordered as ever.
 //
 // The wait is a barrier to ordinary loads and stores, but a compiler takes what is read through `const __restrict__` parameters

@@ -1,8 +1,10 @@
 // Blackwell (sm_100a) building blocks as inline PTX: mbarriers with BOUNDED waits, TMA tile loads (each CTA fetches
 // its own tiles), tensor-memory allocation, tcgen05 MMA/commit/ld, and shared-memory matrix descriptors.
 //
-// Every wait here gives up after a bounded number of polls and reports failure instead of spinning forever: the
-// callers raise a status word the host reads (LB_ERR_TIMEOUT) and wind the kernel down.
+// Every wait on an mbarrier here gives up after a bounded number of polls and reports failure instead of spinning forever: the
+// callers raise a status word the host reads (LB_ERR_TIMEOUT) and wind the kernel down. Without a bound of their own are the waits
+// that the hardware has as one instruction: tensor-memory allocation (tmem_alloc, tmem_alloc_pair), the cluster barrier (cluster_sync),
+// block and named barriers, setmaxnreg.inc, the waits for tensor-memory loads and stores and for bulk copies.
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
