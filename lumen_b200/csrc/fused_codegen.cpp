@@ -212,10 +212,10 @@ __device__ __forceinline__ p2<float> f32x2_fma(p2<float> a, p2<float> b, p2<floa
     return r;
 }
 // Division of a chunk's elements by one divisor, the correctly rounded quotients as __fdiv_rn gives them: with y = RN(1 / b),
-// q0 = RN(a y), q1 = RN(q0 - (b q0 - a) y) is within an ulp and q2 = RN(q1 - (b q1 - a) y) is RN(a / b) (Markstein, "Computation
+// q0 = RN(a y), q1 = RN(q0 + (a - b q0) y) is within an ulp and q2 = RN(q1 + (a - b q1) y) is RN(a / b) (Markstein, "Computation
 // of elementary functions on the IBM RISC System/6000 processor", 1990, theorem 5.1: y correctly rounded, the residual exact). That holds
-// where nothing under- or overflows: 2^-40 <= b <= 2^40 and 2^-60 <= |a| <= 2^60 for every a that is not zero (a zero's products and
-// residuals are zeros, of its sign in the end); what is outside is divided as usual. 2.5 packed instructions an element in one block of
+// where nothing under- or overflows: 2^-40 <= b <= 2^40 and 2^-60 <= |a| <= 2^60 for every a that is not zero (which
+// is its own quotient); what is outside is divided as usual. 2.5 packed instructions an element in one block of
 // straight-line code, where a division each is ten and a branch that nothing is scheduled across, and a zero leaves even that one: a layer norm
 // of 8192 x 1024 bfloat16 with its gradients, which takes three quotients an element and is bound by its instructions, 33.4 -> 28.3 us;
 // relu(x) over its row's sum, 32768 x 1024, float32 67.8 -> 44.4, bfloat16 65.7 -> 34.1; a layer norm of as many elements with every other row
@@ -229,15 +229,15 @@ __device__ __forceinline__ void abs_range(p2<float> a, float& lo, float& hi) {
 }
 __device__ __forceinline__ void abs_range(float a, float& lo, float& hi) { lo = fminf(lo, fabsf(a)), hi = fmaxf(hi, fabsf(a)); }
 __device__ __forceinline__ p2<float> quotient(p2<float> a, float b, float y) {
-    const p2<float> bb = {b, b}, yy = {y, y}, my = {-y, -y}, ma = {-a.x, -a.y};
+    const p2<float> mb = {-b, -b}, yy = {y, y};
     p2<float> q = f32x2_mul(a, yy);
-    q = f32x2_fma(f32x2_fma(bb, q, ma), my, q);
-    return f32x2_fma(f32x2_fma(bb, q, ma), my, q);
+    q = f32x2_fma(f32x2_fma(mb, q, a), yy, q);
+    return f32x2_fma(f32x2_fma(mb, q, a), yy, q);
 }
 __device__ __forceinline__ float quotient(float a, float b, float y) {
     float q = __fmul_rn(a, y);
-    q = __fmaf_rn(__fmaf_rn(b, q, -a), -y, q);
-    return __fmaf_rn(__fmaf_rn(b, q, -a), -y, q);
+    q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+    return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
 }
 // Four elements of a chunk that holds zeros or what is outside the range. Not inlined: such code between that of the other chunks costs
 // those, the layer norm above 28.3 -> 29.8 us.
@@ -245,8 +245,9 @@ __device__ __noinline__ float4 quotients_any(float4 a, float b, float y) {
     float lo = 1.0f, hi = 1.0f;
     abs_range(a.x == 0.0f ? 1.0f : a.x, lo, hi), abs_range(a.y == 0.0f ? 1.0f : a.y, lo, hi);
     abs_range(a.z == 0.0f ? 1.0f : a.z, lo, hi), abs_range(a.w == 0.0f ? 1.0f : a.w, lo, hi);
-    if (y != 0.0f && lo >= LEAST_DIVIDEND && hi <= MOST_DIVIDEND)
-        return make_float4(quotient(a.x, b, y), quotient(a.y, b, y), quotient(a.z, b, y), quotient(a.w, b, y));
+    if (y != 0.0f && lo >= LEAST_DIVIDEND && hi <= MOST_DIVIDEND)  // (b > 0: a zero is its own quotient)
+        return make_float4(a.x == 0.0f ? a.x : quotient(a.x, b, y), a.y == 0.0f ? a.y : quotient(a.y, b, y), a.z == 0.0f ? a.z : quotient(a.z, b, y),
+                           a.w == 0.0f ? a.w : quotient(a.w, b, y));
     return make_float4(__fdiv_rn(a.x, b), __fdiv_rn(a.y, b), __fdiv_rn(a.z, b), __fdiv_rn(a.w, b));
 }
 __device__ __forceinline__ void divide_any(const p2<float>* a, p2<float>* q, float b, float y) {
@@ -257,17 +258,30 @@ __device__ __forceinline__ void divide_any(const float* a, float* q, float b, fl
     const float4 r = quotients_any(make_float4(a[0], a[1], a[2], a[3]), b, y);
     q[0] = r.x, q[1] = r.y, q[2] = r.z, q[3] = r.w;
 }
-template <int N, class T> __device__ __forceinline__ void divide_chunk(const T* a, T* q, float b, float y) {
-    float lo = 1.0f, hi = 1.0f;
-    #pragma unroll
-    for (int k = 0; k < N; k++) abs_range(a[k], lo, hi);
-    if (y != 0.0f && lo >= LEAST_DIVIDEND && hi <= MOST_DIVIDEND) {
+// What the magnitudes of a chunk's elements lie between. Divided, it becomes the quotients' range, or one that nothing is taken to fit.
+struct Magnitudes { float least, most; };
+template <int N, class T> __device__ __forceinline__ void divide_within(const T* a, T* q, float b, float y, Magnitudes& range) {
+    if (y != 0.0f && range.least >= LEAST_DIVIDEND && range.most <= MOST_DIVIDEND) {
         #pragma unroll
         for (int k = 0; k < N; k++) q[k] = quotient(a[k], b, y);
+        range.least *= y * 0.999f, range.most *= y * 1.001f;
     } else {
         #pragma unroll
         for (int k = 0; k < N; k += 16 / (int)sizeof(T)) divide_any(a + k, q + k, b, y);
+        range.least = 0.0f;
     }
+}
+template <int N, class T> __device__ __forceinline__ Magnitudes divide_chunk(const T* a, T* q, float b, float y) {
+    Magnitudes range = {1.0f, 1.0f};
+    #pragma unroll
+    for (int k = 0; k < N; k++) abs_range(a[k], range.least, range.most);
+    divide_within<N>(a, q, b, y, range);
+    return range;
+}
+// A chunk of quotients by `b`, which lie in `range`, divided by it again: the elements are not looked over a second time.
+template <int N, class T> __device__ __forceinline__ Magnitudes divide_again(const T* a, T* q, float b, float y, Magnitudes range) {
+    divide_within<N>(a, q, b, y, range);
+    return range;
 }
 )CUDA";
 
@@ -400,6 +414,7 @@ struct Phase {
     // reduction phases
     bool reduces = false;
     std::string acc, acc_type, init, combine_a_b;  // combine as a format with %A %B
+    int sums = 1;  // how many a thread keeps
     std::string result;
     bool chunked = true;  // false for the row epilogue (runs once per row, no column loop)
 };
@@ -1020,15 +1035,20 @@ class Generator {
         }
         ph.chunk_decls += format("%s %s[%s];\n", type, num.c_str(), count.c_str());
         ph.body += format("%s[%s] = %s;\n", num.c_str(), at, dividend.c_str());
-        ph.parts.push_back({ph.body, format("divide_chunk<%s>(%s, %s, %s, %s);\n", count.c_str(), num.c_str(), quo.c_str(), divisor.c_str(), y.c_str()), key, quo, type});
+        auto known = quotients_.find(dividend);  // of the same divisor: no other quotient's range is known here
+        const bool again = known != quotients_.end() && known->second.second == y;
+        const std::string range = again ? ", " + known->second.first + "_range" : "";
+        ph.parts.push_back({ph.body, format("%s_range = %s<%s>(%s, %s, %s, %s%s);\n", quo.c_str(), again ? "divide_again" : "divide_chunk", count.c_str(), num.c_str(), quo.c_str(), divisor.c_str(), y.c_str(), range.c_str()), key, quo, type});
         ph.body.clear();
         const std::string name = fresh("v");
         ph.body += format("const %s %s = %s[%s];\n", type, name.c_str(), quo.c_str(), at);
         ph.body_vars.push_back({type, name, ph.parts.size()});
+        quotients_[name] = {quo, y};
         if (pairs) pair_vars_[name] = LB_F32;
         else body_names_.insert(name);
         return name;
     }
+    std::map<std::string, std::pair<std::string, std::string>> quotients_;  // a chunk quotient's variable -> its array, the reciprocal
     static bool mentions(const std::string& code, const std::string& name) {
         for (size_t at = code.find(name); at != std::string::npos; at = code.find(name, at + 1))
             if ((at == 0 || !ident_char(code[at - 1])) && (at + name.size() == code.size() || !ident_char(code[at + name.size()]))) return true;
@@ -1044,13 +1064,13 @@ class Generator {
         for (Phase::Part& part : parts) {
             const std::string count = pair_ ? "VEC / 2" : "VEC";
             if (!has_reduce_ || NCH_ * VEC_ > 16) {
-                decls += format("%s %s[%s];\n", part.type.c_str(), part.array.c_str(), count.c_str());
+                decls += format("%s %s[%s];\nMagnitudes %s_range;\n", part.type.c_str(), part.array.c_str(), count.c_str(), part.array.c_str());
                 continue;
             }
             auto [kept, first] = kept_quotients_.emplace(part.key, part.array + "_row");
-            if (first) row_decls_ += format("%s %s[NCH][%s];\n", part.type.c_str(), kept->second.c_str(), count.c_str());
+            if (first) row_decls_ += format("%s %s[NCH][%s];\nMagnitudes %s_range[NCH];\n", part.type.c_str(), kept->second.c_str(), count.c_str(), kept->second.c_str());
             else part.then.clear();
-            decls += format("auto& %s = %s[ch];\n", part.array.c_str(), kept->second.c_str());
+            decls += format("auto& %s = %s[ch];\nauto& %s_range = %s_range[ch];\n", part.array.c_str(), kept->second.c_str(), part.array.c_str(), kept->second.c_str());
         }
         parts.push_back({ph.body, "", "", "", ""});
         for (const Phase::BodyVar& v : ph.body_vars) {
@@ -1080,9 +1100,20 @@ class Generator {
         if (it != pair_vars_.end() && it->second == LB_BF16 && dtype == LB_BF16) return format("*(u32*)&%s[e] = %s.v;\n", buf.c_str(), val.c_str());
         return both_lanes(format("%s[e] = %s;\n", buf.c_str(), to_memory(dtype, "LX(" + val + ")").c_str()));
     }
+    // Whether a pair's elements are added by one packed instruction: float32 sums. Half the instructions, and a chain half as long. With packed
+    // negations, one product for x * y and y * x, and what is said at divide_again, 58.5 -> 53.8 instructions an element and 28.2 -> 27.7 us for
+    // a layer norm of 8192 x 1024 bfloat16 with its gradients: chains of dependent instructions bound it more than their number.
+    bool adds_pairs(const std::string& combine, const std::string& val) const {
+        return pair_ && !shifted_ && combine == "rnd_f32(__fadd_rn(%A, %B))" && packable(val, LB_F32);
+    }
     // the statement(s) folding element e (and e + 1) of `val` into `acc`
     std::string accumulate(const std::string& acc, const std::string& combine, const std::string& val) {
         const char* counts = shifted_ ? "if (whole || in_row(c0 + e)) " : "";  // (a row's neighbours do not)
+        if (adds_pairs(combine, val)) {
+            const std::string second = lane_of(acc, 1, nullptr);
+            return format("{ const p2<float> sum = f32x2_add(p2<float>{%s, %s}, to_f32x2(%s)); %s = sum.x, %s = sum.y; }\n", acc.c_str(), second.c_str(),
+                          val.c_str(), acc.c_str(), second.c_str());
+        }
         if (!pair_) return format("%s%s = %s;\n", counts, acc.c_str(), subst(combine, acc, val).c_str());
         return both_lanes(format("%s%s = %s;\n", counts, acc.c_str(), subst(combine, acc, "LX(" + val + ")").c_str()));
     }
@@ -1239,8 +1270,10 @@ class Generator {
             std::string a = arg(0), b = arg(1), e;
             if (packed && (op == "add" || op == "sub" || op == "mul" || op == "max" || op == "min") && packable(ops[0]) && packable(ops[1]))
                 return def(ct.compute, format("bf16x2_%s(to_bf16x2(%s), to_bf16x2(%s))", op.c_str(), a.c_str(), b.c_str()), in_body, true);
-            if (pairs && t.dtype == LB_F32 && (op == "add" || op == "sub" || op == "mul") && packable(ops[0], LB_F32) && packable(ops[1], LB_F32))
+            if (pairs && t.dtype == LB_F32 && (op == "add" || op == "sub" || op == "mul") && packable(ops[0], LB_F32) && packable(ops[1], LB_F32)) {
+                if (op != "sub" && ops[1] < ops[0]) std::swap(a, b);  // x * y and y * x are one value
                 return def(ct.compute, format("f32x2_%s(to_f32x2(%s), to_f32x2(%s))", op.c_str(), a.c_str(), b.c_str()), in_body, true);
+            }
             if (op == "div" && t.dtype == LB_F32 && in_body && !may_be_tiny(n->inputs[0]) && divides_chunk(ph, pairs ? ops[0] : a, pairs ? ops[1] : b, pairs))
                 return chunk_quotient(ph, key_of(v, idx), pairs ? ops[0] : a, pairs ? ops[1] : b, pairs);
             if (flt) {
@@ -1281,6 +1314,7 @@ class Generator {
         if (op == "neg") {
             std::string a = arg(0);
             if (packed && packable(ops[0])) return def(ct.compute, "bf16x2_neg(to_bf16x2(" + a + "))", in_body, true);
+            if (pairs && t.dtype == LB_F32 && packable(ops[0], LB_F32)) return def(ct.compute, "f32x2_mul(to_f32x2(" + a + "), to_f32x2(-1.0f))", in_body, true);
             return def(ct.compute, flt ? "-" + a : format("(%s)((%s)RT_ZERO - (%s)%s)", ct.compute, ct.unsigned_t, ct.unsigned_t, a.c_str()), in_body);
         }
         if (op == "abs" || op == "sign" || op == "not") {
@@ -1471,7 +1505,8 @@ class Generator {
             }
         }
         std::string val = gen(n.inputs[0], src, ph);
-        ph.body += accumulate(ph.acc + (sums() == 1 ? "" : shifted_ ? "[e]" : "[ch & 3]"), ph.combine_a_b, val);
+        ph.sums = adds_pairs(ph.combine_a_b, val) ? 2 : sums();
+        ph.body += accumulate(ph.acc + (ph.sums == 1 ? "" : shifted_ ? "[e]" : ph.sums == 2 ? "[e & 1]" : "[ch & 3]"), ph.combine_a_b, val);
         row_decls_ += format("%s %s;\n", ct.compute, ph.result.c_str());
         phases_.push_back(ph);
         reduce_memo_[key] = ph.result;
@@ -1638,9 +1673,9 @@ class Generator {
         for (size_t at = 0; at < phases_.size(); at++) {
             const Phase& ph = phases_[at];
             s << "        {\n";
-            if (ph.reduces && sums() > 1) {
-                s << "            " << ph.acc_type << " " << ph.acc << "[" << sums() << "] = {" << ph.init;
-                for (int n = 1; n < sums(); n++) s << ", " << ph.init;
+            if (ph.reduces && ph.sums > 1) {
+                s << "            " << ph.acc_type << " " << ph.acc << "[" << ph.sums << "] = {" << ph.init;
+                for (int n = 1; n < ph.sums; n++) s << ", " << ph.init;
                 s << "};\n";
             } else if (ph.reduces) s << "            " << ph.acc_type << " " << ph.acc << " = " << ph.init << ";\n";
             if (ph.chunked) {
@@ -1655,7 +1690,7 @@ class Generator {
             if (ph.reduces) {
                 std::string sum = ph.acc;
                 std::vector<std::string> tree;
-                for (int n = 0; sums() > 1 && n < sums(); n++) tree.push_back(format("%s[%d]", ph.acc.c_str(), n));
+                for (int n = 0; ph.sums > 1 && n < ph.sums; n++) tree.push_back(format("%s[%d]", ph.acc.c_str(), n));
                 for (; tree.size() > 1; tree.resize(tree.size() / 2))
                     for (size_t n = 0; n < tree.size() / 2; n++) tree[n] = subst(ph.combine_a_b, tree[2 * n], tree[2 * n + 1]);
                 if (!tree.empty()) sum = tree[0];
