@@ -168,6 +168,15 @@ int lb_attention_fwd_kernel(const lb_attn_desc* desc, const lb_tensor* q, const 
 int lb_attention_bwd(const lb_attn_desc* desc, const lb_tensor* q, const lb_tensor* k, const lb_tensor* v,
                      const lb_tensor* o, const lb_tensor* d_o, const lb_tensor* lse, const lb_tensor* delta,
                      const lb_tensor* dq, const lb_tensor* dk, const lb_tensor* dv, void* stream);
+/* lb_attention_bwd with caller-provided scratch for dS = P (dP - delta) scale, bfloat16 as its products read it: at head dim 128 the
+ * dK/dV kernel leaves it there and dQ = dS K reads it back, instead of computing it a second time. lb_attention_bwd_scratch_bytes
+ * says how much (0 where dS is not handed on; at most 4.5 GiB, with which larger problems take several rounds of heads); `scratch` is
+ * 16-byte aligned, and less than one key head's, or NULL, is lb_attention_bwd. Bit-identical from run to run, whatever the scratch. */
+size_t lb_attention_bwd_scratch_bytes(const lb_attn_desc* desc, const lb_tensor* q, const lb_tensor* k);
+int lb_attention_bwd_scratch(const lb_attn_desc* desc, const lb_tensor* q, const lb_tensor* k, const lb_tensor* v,
+                             const lb_tensor* o, const lb_tensor* d_o, const lb_tensor* lse, const lb_tensor* delta,
+                             const lb_tensor* dq, const lb_tensor* dk, const lb_tensor* dv, void* scratch, size_t scratch_bytes,
+                             void* stream);
 /* lb_attention_bwd in the mode the reference's backend runs unless its `deterministic` option is set: ONE kernel
  * that computes dK and dV per key block and adds each key block's dS K into a float32 dQ atomically, in no fixed
  * order (lumen/codegen/attention/triton/mod.rs:176-180,458-466; kernel.py:108-200 with ADD_DQ). `dq_accum` is

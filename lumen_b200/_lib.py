@@ -110,6 +110,9 @@ def lib():
         _lib.lb_attention_fwd.argtypes = [ctypes.POINTER(LbAttnDesc), T, T, T, T, T, ctypes.c_void_p]
         _lib.lb_attention_fwd_kernel.argtypes = [ctypes.POINTER(LbAttnDesc), T, T, T, ctypes.POINTER(ctypes.c_int32)]
         _lib.lb_attention_bwd.argtypes = [ctypes.POINTER(LbAttnDesc)] + [T] * 10 + [ctypes.c_void_p]
+        _lib.lb_attention_bwd_scratch.argtypes = [ctypes.POINTER(LbAttnDesc)] + [T] * 10 + [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]
+        _lib.lb_attention_bwd_scratch_bytes.argtypes = [ctypes.POINTER(LbAttnDesc), T, T]
+        _lib.lb_attention_bwd_scratch_bytes.restype = ctypes.c_size_t
         _lib.lb_attention_bwd_atomic.argtypes = [ctypes.POINTER(LbAttnDesc)] + [T] * 11 + [ctypes.c_void_p]
         _lib.lb_attention_bwd_static.argtypes = [ctypes.POINTER(LbAttnDesc)] + [T] * 9 + [ctypes.c_void_p]
     return _lib

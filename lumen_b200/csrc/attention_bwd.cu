@@ -14,11 +14,19 @@
 //   dK/dV mode: CTA = (key tile, kv head, batch); R = (K, V), T = (Q, dO) over every query head of the group and
 //               every query tile that sees the keys; acc_a = dK += Z Q, acc_b = dV += P dO.
 //   dQ mode:    CTA = (query tile, head, batch); R = (Q, dO), T = (K, V) over the visible key tiles; acc_a = dQ += Z K.
-// No atomics and no scratch: every output element is produced by one CTA in a fixed order (bit-reproducible run to
+// No atomics: every output element is produced by one CTA in a fixed order (bit-reproducible run to
 // run, as the reference's deterministic mode requires, tests/functional/test_attention.py:403-407).
+//
+// Head dim 128, with scratch for it: dK/dV mode leaves dS in memory and attention_dq.cu takes dQ from it, in place of dQ mode, which
+// computes it again (every bit the same). us of the kernels at batch 8, 32 heads, sequence 4096, causal: 1750 + 1365 -> 2020 + 725, the
+// whole backward 3140 -> 2900; 4 x 32 heads on 8, 512 tokens 70.6 -> 58.7; 2 x 16, 1024 63.8 -> 54.5; 1 x 8, 256 17.1 -> 14.1; over 44
+// shapes of 128 to 8192 tokens 0.80 - 1.02 of the time.
+#include <algorithm>
+#include <cstdlib>
 #include <mutex>
 #include <type_traits>
 
+#include "attention_dq.h"
 #include "device.h"
 #include "launch.cuh"
 #include "sm100.cuh"
@@ -67,6 +75,9 @@ struct BwdArgs {
     long long a_sb, a_ss, a_sn;
     void* out_b;         // dV (dkdv mode)
     long long b_sb, b_ss, b_sn;
+    int batch0, head0;   // the launch's first batch entry and first head (kv head in dkdv mode)
+    uint8_t* scores;     // dkdv mode, head dim 128: where dS is left for attention_dq, or null
+    DsLayout ds;
     int* status;
 };
 
@@ -123,7 +134,8 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform for the compiler too
     const int tile = DKDV ? (int)blockIdx.x : (int)(gridDim.x - 1 - blockIdx.x);
-    const int head = blockIdx.y, batch = blockIdx.z;  // kv head in dkdv mode, query head in dq mode
+    const int head = p.head0 + (int)blockIdx.y, batch = p.batch0 + (int)blockIdx.z;  // kv head in dkdv mode, query head in dq mode
+    constexpr bool kHands = D == 128 && DKDV && BT == 128;  // may leave dS
     const int group = p.N / p.Nkv;
     const int r0 = tile * BR;
 
@@ -318,6 +330,17 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
             }
         };
         if (DKDV && n_iter > 0) fetch_stats(0);
+        uint8_t* scores = nullptr;  // dS of this thread's key and its warpgroup's first block of queries
+        if constexpr (kHands) {
+            if (p.scores)
+                scores = p.scores + ((long long)blockIdx.z * gridDim.y + blockIdx.y) * group * p.ds.head_bytes() + p.ds.at(tile, row_in_tile / 64, stream0 / 64) +
+                         wg * kDsHalfBytes + row_in_tile % 64 * 16;
+        }
+        // A tile's dS leaves between the next one's exponentials, a store for every eight of them: in a row, right behind the hand-over of P and
+        // Z, the stores hold up those (the backward of 1 x 8 heads x 4096 157 -> 135 us, of 8 x 32 x 4096 2990 -> 2900).
+        uint32_t left[kHands ? COLS / 2 : 1];
+        uint8_t* left_to = nullptr;
+        auto leave = [&](int c) { *(uint4*)(left_to + c * 1024) = make_uint4(left[4 * c], left[4 * c + 1], left[4 * c + 2], left[4 * c + 3]); };
         float* stat_lse = col_stats + (warp - C::kFirst) * 2 * COLS;
         float* stat_delta = stat_lse + COLS;
         bool ok = true;
@@ -343,6 +366,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
             if (DKDV) {
                 col_lo = p.causal ? row - p.causal_offset : 0;
                 col_hi = p.Sq;
+                if (kHands && scores && row >= p.Sk) col_hi = 0;  // what is left for these is multiplied by zeros and must be finite
             } else {
                 col_lo = 0;
                 col_hi = p.causal ? min((long long)p.Sk, row + p.causal_offset + 1) : (long long)p.Sk;
@@ -371,6 +395,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
                     const float2 u = __ffma2_rn(make_float2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])), s2, make_float2(l4.x, l4.y));
                     const float2 v = __ffma2_rn(make_float2(__uint_as_float(x[i + 2]), __uint_as_float(x[i + 3])), s2, make_float2(l4.z, l4.w));
                     pr[i] = fast_exp2(u.x), pr[i + 1] = fast_exp2(u.y), pr[i + 2] = fast_exp2(v.x), pr[i + 3] = fast_exp2(v.y);
+                    if (kHands && scores && it > 0 && i % 8 == 4) leave(i / 8);
                 }
                 if (masked_tile) {
 #pragma unroll
@@ -422,7 +447,16 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
             tmem_st_wait();
             tc_fence_before();
             mbar_arrive(pz_ready);
+            if constexpr (kHands) {
+                left_to = scores + hh * p.ds.head_bytes() + (long long)(it - hh * per_head) * (2 * kDsHalfBytes);
+#pragma unroll
+                for (int c = 0; c < COLS / 2; c++) left[c] = pz[kZ + c];
+            }
         }
+        if constexpr (kHands)
+            if (scores && n_iter > 0 && ok)
+#pragma unroll
+                for (int c = 0; c < 8; c++) leave(c);
         // ---- epilogue: accumulators -> bf16 rows ----
         if (n_iter > 0) ok = ok && mbar_wait(acc_full, 0, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
@@ -562,15 +596,50 @@ void launch_bwd_kernel(const CUtensorMap& r1, const CUtensorMap& r2, const CUten
     launch_overlapped(attention_bwd_kernel<D, DKDV, BT>, grid, dim3(C::kThreads), C::kBytes, s, 0, r1, r2, t1, t2, p);
 }
 
+// Of the dS that is left in memory at a time, and the fewest dK/dV CTAs of each of several rounds, whose ends leave SMs idle: batch 8, 32
+// heads, sequence 4096, causal, us, dS computed twice 3230, in rounds of 1000 CTAs 3590, of 2000 3400, of 4000 3080, at once 3030; batch 4, 32
+// heads, 8192 in two rounds of 4096 0.93 of the time, not causal in four of 2048 1.00.
+constexpr size_t kMostScores = (size_t)4608 << 20;
+constexpr long long kLeastRound = 3000;
+
+// Whether 128-row tiles are streamed at head dim 128 (see launch_bwd_pair)
+bool tall_tiles(long long streamed) { return (streamed + 63) / 64 % 2 == 0 || streamed > 5 * 64; }
+
+// Whether the backward may take dQ from the dS that its dK/dV kernel leaves, and how that lies: head dim 128 with 128-row tiles of queries
+// that all start at a multiple of 128.
+bool hands_scores(const lb_attn_desc& desc, long long Sq, long long Sk, long long D, DsLayout& ds) {
+    if (D != 128 || Sq <= 0 || Sk <= 0 || !tall_tiles(Sq) || Sq > (1 << 24) || Sk > (1 << 24)) return false;
+    if (desc.causal && (desc.causal_offset % 128 != 0 || std::abs(desc.causal_offset) > (1 << 24))) return false;
+    ds.query_blocks = (int)((Sq + 127) / 128) * 2, ds.key_tiles = (int)((Sk + 127) / 128);
+    ds.causal = desc.causal != 0, ds.offset = desc.causal ? (int)(desc.causal_offset / 64) : 0;
+    return ds.head_bytes() > 0;
+}
+
+// The heads a launch of both kernels takes at once: batch entries whole, or (0) kv heads of one entry; nothing where the rounds would be small.
+struct HandedHeads {
+    long long batches = 0, kv_heads = 0;
+    size_t bytes = 0;
+};
+HandedHeads handed_heads(const DsLayout& ds, long long B, long long N, long long Nkv, size_t most) {
+    const long long kv_head = N / Nkv * ds.head_bytes(), entry = Nkv * kv_head;
+    auto even = [](long long all, long long at_once) { return (all + (all + at_once - 1) / at_once - 1) / ((all + at_once - 1) / at_once); };
+    HandedHeads h;
+    if (entry <= (long long)most) h.batches = even(B, std::min<long long>(B, (long long)most / entry)), h.kv_heads = Nkv, h.bytes = (size_t)(h.batches * entry);
+    else if (kv_head <= (long long)most) h.kv_heads = even(Nkv, (long long)most / kv_head), h.bytes = (size_t)(h.kv_heads * kv_head);
+    const bool rounds = h.batches < B || h.kv_heads < Nkv;
+    return rounds && std::max<long long>(1, h.batches) * h.kv_heads * ds.key_tiles < kLeastRound ? HandedHeads{} : h;
+}
+
 // The two kernels; `rows` makes the map of an operand's tiles, 128 or 64 rows high. Head dim 64 streams 64 rows a tile. Head dim 128
 // streams 128, but 64 where the streamed rows are one, three or five blocks of 64: the last 128-row tile would be half empty, which
 // shows while tiles are few. Measured (us, 128 rows a tile -> 64 for dK/dV and dQ together), 64 x 4 heads: 16 rows 23.4 -> 17.4 and,
 // one head to a key head, 16.9 -> 13.7; 160 rows 32.8 -> 28.9, 21.3 -> 19.0; 320 rows 49.0 -> 45.6; two and four blocks are as fast or
 // faster with 128 (128 rows 21.6 -> 22.0, 256 30.7 -> 33.5). The 64-row form also stands in where the compiler did not assign the
 // registers that the budgets of the 128-row form (setmaxnreg) are drawn from.
+// With `scratch` for the dS of some heads (handed_heads), dK/dV leaves it there and attention_dq takes dQ from it, those heads at a time.
 template <int D, class Rows>
 void launch_bwd_pair(const Rows& rows, const lb_tensor& q, const lb_tensor& d_o, const lb_tensor& k, const lb_tensor& v, const BwdArgs& dkdv,
-                     const BwdArgs& dq, cudaStream_t s) {
+                     const BwdArgs& dq, void* scratch, const DsLayout& ds, const HandedHeads& handed, cudaStream_t s) {
     const CUtensorMap mq = rows(q, "query", 128), mdo = rows(d_o, "dO", 128), mk = rows(k, "key", 128), mv = rows(v, "value", 128);
     const dim3 grid_kv((unsigned)((dkdv.Sk + BR - 1) / BR), (unsigned)dkdv.Nkv, (unsigned)dkdv.B);
     const dim3 grid_q((unsigned)((dq.Sq + BR - 1) / BR), (unsigned)dq.N, (unsigned)dq.B);
@@ -578,8 +647,25 @@ void launch_bwd_pair(const Rows& rows, const lb_tensor& q, const lb_tensor& d_o,
     if constexpr (D == 128) {
         static const bool budgets = launch_regs((const void*)attention_bwd_kernel<128, true, 128>) >= BwdConfig<128, true, 128>::kLaunchRegs &&
                                     launch_regs((const void*)attention_bwd_kernel<128, false, 128>) >= BwdConfig<128, false, 128>::kLaunchRegs;
-        auto tall = [&](int streamed) { return budgets && ((streamed + 63) / 64 % 2 == 0 || streamed > 5 * 64); };
-        tall_kv = tall(dkdv.Sq), tall_q = tall(dq.Sk);
+        tall_kv = budgets && tall_tiles(dkdv.Sq), tall_q = budgets && tall_tiles(dq.Sk);
+        if (tall_kv && scratch && handed.kv_heads) {
+            const CUtensorMap keys = rows(k, "key", 64);
+            const int group = dq.N / dq.Nkv;
+            BwdArgs a = dkdv;
+            a.scores = (uint8_t*)scratch, a.ds = ds;
+            DqArgs d{};
+            d.ds = ds, d.scores = a.scores, d.N = dq.N, d.Nkv = dq.Nkv, d.Sq = dq.Sq, d.Sk = dq.Sk;
+            d.dq = dq.out_a, d.sb = dq.a_sb, d.ss = dq.a_ss, d.sn = dq.a_sn, d.status = dq.status;
+            const int batches = (int)std::max<long long>(1, handed.batches), heads = (int)handed.kv_heads;
+            for (int b = 0; b < dkdv.B; b += batches)
+                for (int h = 0; h < dkdv.Nkv; h += heads) {
+                    const int nb = std::min(batches, dkdv.B - b), nh = std::min(heads, dkdv.Nkv - h);
+                    a.batch0 = d.batch0 = b, a.head0 = h, d.head0 = h * group, d.heads = nh * group;
+                    launch_bwd_kernel<128, true, 128>(mk, mv, mq, mdo, dim3(grid_kv.x, (unsigned)nh, (unsigned)nb), a, s);
+                    attention_dq_launch(keys, nb, d, s);
+                }
+            return;
+        }
         if (tall_kv) launch_bwd_kernel<128, true, 128>(mk, mv, mq, mdo, grid_kv, dkdv, s);
     }
     if (!tall_kv) launch_bwd_kernel<D, true, 64>(mk, mv, rows(q, "query", 64), rows(d_o, "dO", 64), grid_kv, dkdv, s);
@@ -589,9 +675,9 @@ void launch_bwd_pair(const Rows& rows, const lb_tensor& q, const lb_tensor& d_o,
 }
 template <class Rows>
 void launch_bwd(long long D, const Rows& rows, const lb_tensor& q, const lb_tensor& d_o, const lb_tensor& k, const lb_tensor& v, const BwdArgs& dkdv,
-                const BwdArgs& dq, cudaStream_t s) {
-    if (D == 128) launch_bwd_pair<128>(rows, q, d_o, k, v, dkdv, dq, s);
-    else launch_bwd_pair<64>(rows, q, d_o, k, v, dkdv, dq, s);
+                const BwdArgs& dq, cudaStream_t s, void* scratch = nullptr, const DsLayout& ds = {}, const HandedHeads& handed = {}) {
+    if (D == 128) launch_bwd_pair<128>(rows, q, d_o, k, v, dkdv, dq, scratch, ds, handed, s);
+    else launch_bwd_pair<64>(rows, q, d_o, k, v, dkdv, dq, nullptr, ds, handed, s);
 }
 
 }  // namespace
@@ -601,7 +687,7 @@ void launch_bwd(long long D, const Rows& rows, const lb_tensor& q, const lb_tens
 // unless `deterministic` (lumen/codegen/attention/triton/mod.rs:458-466) - and rounded to dq afterwards.
 void attention_bwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o,
                    const lb_tensor& d_o, const lb_tensor& lse, const lb_tensor& delta, const lb_tensor& dq, const lb_tensor& dk,
-                   const lb_tensor& dv, void* stream, const lb_tensor* dq_acc = nullptr) {
+                   const lb_tensor& dv, void* stream, const lb_tensor* dq_acc, void* scratch, size_t scratch_bytes) {
     const long long B = q.shape[0], Sq = q.shape[1], N = q.shape[2], D = q.shape[3];
     if (q.rank != 4 || k.rank != 4 || v.rank != 4) fail(LB_ERR_INVALID, "attention backward: operands must be [B, S, N, H] tensors");
     const long long Sk = k.shape[1], Nkv = k.shape[2];
@@ -648,7 +734,20 @@ void attention_bwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor
                                     attention_map_rows(q, "query", 128), attention_map_rows(d_o, "dO", 128), q, k, a.lse, a.delta, (float*)dq_acc->ptr, dq, dk, dv, s);
         return;
     }
-    launch_bwd(D, attention_map_rows, q, d_o, k, v, kv, qq, s);
+    // dQ rows leave in whole lines there
+    DsLayout ds;
+    HandedHeads handed;
+    const bool aligned = dq.stride[0] % 8 == 0 && dq.stride[1] % 8 == 0 && dq.stride[2] % 8 == 0 && ((uintptr_t)dq.ptr & 15) == 0;
+    if (scratch && ((uintptr_t)scratch & 15) == 0 && aligned && hands_scores(desc, Sq, Sk, D, ds)) handed = handed_heads(ds, B, N, Nkv, scratch_bytes);
+    launch_bwd(D, attention_map_rows, q, d_o, k, v, kv, qq, s, scratch, ds, handed);
+}
+
+// Scratch with which the backward hands dS on: that of as many heads as kMostScores holds, 0 where it does not.
+size_t attention_bwd_scratch_bytes(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k) {
+    DsLayout ds;
+    if (q.rank != 4 || k.rank != 4 || q.dtype != LB_BF16 || q.shape[0] <= 0 || k.shape[2] <= 0 || q.shape[2] < k.shape[2] || q.shape[2] % k.shape[2]) return 0;
+    if (!hands_scores(desc, q.shape[1], k.shape[1], q.shape[3], ds)) return 0;
+    return handed_heads(ds, q.shape[0], q.shape[2], k.shape[2], kMostScores).bytes;
 }
 
 }  // namespace lb
@@ -660,10 +759,10 @@ void attention_simt_bwd(const lb_attn_desc& desc, const lb_tensor& q, const lb_t
                         const lb_tensor& dv, void* stream);
 void attention_backward(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o,
                         const lb_tensor& d_o, const lb_tensor& lse, const lb_tensor& delta, const lb_tensor& dq, const lb_tensor& dk,
-                        const lb_tensor& dv, void* stream, const lb_tensor* dq_acc) {
+                        const lb_tensor& dv, void* stream, const lb_tensor* dq_acc, void* scratch, size_t scratch_bytes) {
     if (attention_on_tensor_cores(q, k, v) && attention_on_tensor_cores(d_o, k, v) && attention_on_tensor_cores(o, k, v) && q.shape[1] > 0 &&
         k.shape[1] > 0)
-        attention_bwd(desc, q, k, v, o, d_o, lse, delta, dq, dk, dv, stream, dq_acc);
+        attention_bwd(desc, q, k, v, o, d_o, lse, delta, dq, dk, dv, stream, dq_acc, scratch, scratch_bytes);
     else
         attention_simt_bwd(desc, q, k, v, o, d_o, lse, delta, dq, dk, dv, stream);
 }
@@ -675,7 +774,22 @@ extern "C" int lb_attention_bwd(const lb_attn_desc* desc, const lb_tensor* q, co
     return lb::guarded([&] {
         if (!desc || !q || !k || !v || !o || !d_o || !lse || !delta || !dq || !dk || !dv)
             lb::fail(LB_ERR_INVALID, "lb_attention_bwd: null argument");
-        lb::attention_backward(*desc, *q, *k, *v, *o, *d_o, *lse, *delta, *dq, *dk, *dv, stream, nullptr);
+        lb::attention_backward(*desc, *q, *k, *v, *o, *d_o, *lse, *delta, *dq, *dk, *dv, stream, nullptr, nullptr, 0);
+    });
+}
+
+// lb_attention_bwd with scratch for the dS of some of the heads (lb_attention_bwd_scratch_bytes, 16-byte aligned), where it is faster for it
+// (attention_dq.cu); without, or with less than one kv head's, lb_attention_bwd.
+extern "C" size_t lb_attention_bwd_scratch_bytes(const lb_attn_desc* desc, const lb_tensor* q, const lb_tensor* k) {
+    return desc && q && k ? lb::attention_bwd_scratch_bytes(*desc, *q, *k) : 0;
+}
+extern "C" int lb_attention_bwd_scratch(const lb_attn_desc* desc, const lb_tensor* q, const lb_tensor* k, const lb_tensor* v, const lb_tensor* o,
+                                        const lb_tensor* d_o, const lb_tensor* lse, const lb_tensor* delta, const lb_tensor* dq, const lb_tensor* dk,
+                                        const lb_tensor* dv, void* scratch, size_t scratch_bytes, void* stream) {
+    return lb::guarded([&] {
+        if (!desc || !q || !k || !v || !o || !d_o || !lse || !delta || !dq || !dk || !dv)
+            lb::fail(LB_ERR_INVALID, "lb_attention_bwd_scratch: null argument");
+        lb::attention_backward(*desc, *q, *k, *v, *o, *d_o, *lse, *delta, *dq, *dk, *dv, stream, nullptr, scratch, scratch_bytes);
     });
 }
 
@@ -688,7 +802,7 @@ extern "C" int lb_attention_bwd_atomic(const lb_attn_desc* desc, const lb_tensor
     return lb::guarded([&] {
         if (!desc || !q || !k || !v || !o || !d_o || !lse || !delta || !dq_accum || !dq || !dk || !dv)
             lb::fail(LB_ERR_INVALID, "lb_attention_bwd_atomic: null argument");
-        lb::attention_backward(*desc, *q, *k, *v, *o, *d_o, *lse, *delta, *dq, *dk, *dv, stream, dq_accum);
+        lb::attention_backward(*desc, *q, *k, *v, *o, *d_o, *lse, *delta, *dq, *dk, *dv, stream, dq_accum, nullptr, 0);
     });
 }
 

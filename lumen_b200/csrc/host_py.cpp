@@ -149,20 +149,30 @@ PyObject* attention_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return finish(rc);
 }
 
-// attention_bwd(scale, causal, offset, q, k, v, o, dO, lse, delta, dq_accum or None, dq, dk, dv, stream)
+// attention_bwd_scratch_bytes(scale, causal, offset, q, k)
+PyObject* attention_bwd_scratch_bytes(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    lb_attn_desc d;
+    lb_tensor q, k;
+    if (!wants(n, 5) || !attn_desc(a, &d) || !describe(a[3], &q) || !describe(a[4], &k)) return nullptr;
+    return PyLong_FromSize_t(lb_attention_bwd_scratch_bytes(&d, &q, &k));
+}
+
+// attention_bwd(scale, causal, offset, q, k, v, o, dO, lse, delta, dq_accum or None, dq, dk, dv, scratch pointer, scratch bytes, stream)
 PyObject* attention_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     lb_attn_desc d;
     lb_tensor t[11];
-    if (!wants(n, 15) || !attn_desc(a, &d)) return nullptr;
+    if (!wants(n, 17) || !attn_desc(a, &d)) return nullptr;
     const bool atomic = a[10] != Py_None;
     for (int k = 0; k < 11; k++)
         if ((k != 7 || atomic) && !describe(a[3 + k], &t[k])) return nullptr;
-    void* stream = PyLong_AsVoidPtr(a[14]);
+    void* scratch = PyLong_AsVoidPtr(a[14]);
+    const size_t bytes = PyLong_AsSize_t(a[15]);
+    void* stream = PyLong_AsVoidPtr(a[16]);
     if (PyErr_Occurred()) return nullptr;
     int rc;
     Py_BEGIN_ALLOW_THREADS
     rc = atomic ? lb_attention_bwd_atomic(&d, &t[0], &t[1], &t[2], &t[3], &t[4], &t[5], &t[6], &t[7], &t[8], &t[9], &t[10], stream)
-                : lb_attention_bwd(&d, &t[0], &t[1], &t[2], &t[3], &t[4], &t[5], &t[6], &t[8], &t[9], &t[10], stream);
+                : lb_attention_bwd_scratch(&d, &t[0], &t[1], &t[2], &t[3], &t[4], &t[5], &t[6], &t[8], &t[9], &t[10], scratch, bytes, stream);
     Py_END_ALLOW_THREADS
     return finish(rc);
 }
@@ -443,7 +453,8 @@ PyTypeObject table_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 PyMethodDef methods[] = {
     {"setup", (PyCFunction)(void (*)(void))setup, METH_FASTCALL, "dtype codes and callbacks"},
     {"attention_fwd", (PyCFunction)(void (*)(void))attention_fwd, METH_FASTCALL, "lb_attention_fwd on tensors"},
-    {"attention_bwd", (PyCFunction)(void (*)(void))attention_bwd, METH_FASTCALL, "lb_attention_bwd / lb_attention_bwd_atomic on tensors"},
+    {"attention_bwd", (PyCFunction)(void (*)(void))attention_bwd, METH_FASTCALL, "lb_attention_bwd_scratch / lb_attention_bwd_atomic on tensors"},
+    {"attention_bwd_scratch_bytes", (PyCFunction)(void (*)(void))attention_bwd_scratch_bytes, METH_FASTCALL, "lb_attention_bwd_scratch_bytes of tensors"},
     {"gemm", (PyCFunction)(void (*)(void))gemm, METH_FASTCALL, "lb_gemm on tensors"},
     {nullptr, nullptr, 0, nullptr},
 };

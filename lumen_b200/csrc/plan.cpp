@@ -41,7 +41,7 @@ void attention_forward(const lb_attn_desc& desc, const lb_tensor& q, const lb_te
                        const lb_tensor* lse, void* stream);
 void attention_backward(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o,
                         const lb_tensor& d_o, const lb_tensor& lse, const lb_tensor& delta, const lb_tensor& dq, const lb_tensor& dk,
-                        const lb_tensor& dv, void* stream, const lb_tensor* dq_acc);
+                        const lb_tensor& dv, void* stream, const lb_tensor* dq_acc, void* scratch, size_t scratch_bytes);
 void scatter_add_rows(const lb_tensor& x, const lb_tensor& ids, const lb_tensor& updates, const lb_tensor& out, void* scratch,
                       bool x_is_zero, bool deterministic, void* stream);
 size_t scatter_add_scratch_bytes(long long rows, long long width, long long tokens, bool deterministic);
@@ -363,7 +363,7 @@ void run(const lb_plan& p, void* ws, void* const* in, void* const* out, int firs
             case ATTN_BWD: {
                 lb_tensor acc{};
                 if (s.args.size() > 10) acc = T(10);
-                attention_backward(s.attn, T(0), T(1), T(2), T(3), T(4), T(5), T(6), T(7), T(8), T(9), stream, s.args.size() > 10 ? &acc : nullptr);
+                attention_backward(s.attn, T(0), T(1), T(2), T(3), T(4), T(5), T(6), T(7), T(8), T(9), stream, s.args.size() > 10 ? &acc : nullptr, nullptr, 0);
                 break;
             }
             case SCATTER_ADD: {

@@ -224,6 +224,9 @@ def attention_forward(q, k, v, scale=None, causal=False, out=None, lse=None, str
     return out, lse
 
 
+_KEPT_SCORES = 256 << 20
+
+
 def attention_backward(q, k, v, o, d_o, lse, scale=None, causal=False, delta=None, stream=None, deterministic=True):
     """Flash attention backward; returns `(dq, dk, dv)` shaped like `q`, `k`, `v`. `deterministic` (the default here)
     runs `lb_attention_bwd`, the dK/dV + dQ kernel pair that is bit-identical from run to run; without it
@@ -236,8 +239,17 @@ def attention_backward(q, k, v, o, d_o, lse, scale=None, causal=False, delta=Non
     if delta is None:
         delta = _workspace(q, (b, n, sq), "float32", stream)
     dq_accum = None if deterministic else _workspace(q, (b, sq, n, h), "float32", stream)
-    _lib.host().attention_bwd(float(scale if scale is not None else h**-0.5), bool(causal), sk - sq, q, k, v, o, d_o, lse, delta,
-                              dq_accum, dq, dk, dv, _stream(stream))
+    scale, causal = float(scale if scale is not None else h**-0.5), bool(causal)
+    scores, nbytes = None, _lib.host().attention_bwd_scratch_bytes(scale, causal, sk - sq, q, k) if h == 128 else 0
+    if nbytes > _KEPT_SCORES and not type(q).__module__.startswith("torch"):
+        nbytes = 0  # a region that is kept for the stream
+    if nbytes:
+        try:
+            scores = _workspace(q, (nbytes,), "uint8", stream)
+        except RuntimeError:  # no memory for it: it is not needed
+            nbytes = 0
+    _lib.host().attention_bwd(scale, causal, sk - sq, q, k, v, o, d_o, lse, delta, dq_accum, dq, dk, dv, scores.data_ptr() if nbytes else 0,
+                              nbytes, _stream(stream))
     return dq, dk, dv
 
 
