@@ -45,7 +45,7 @@ struct SmallGemmArgs {
     long long ld_aux, aux_batch_stride;
     int splits;  // CTAs of a cluster: 1, 2, 4 or 8, no more than the 64-wide blocks of K
     int* status;
-    int tiles_m, tiles_n, vec;  // set by gemm_small
+    int tiles_m, tiles_n, vec, aux_vec;  // set by gemm_small
 };
 
 void gemm_small(const CUtensorMap& map_a, const CUtensorMap& map_b, SmallGemmArgs p, int batch, int sms, cudaStream_t s);

@@ -372,7 +372,8 @@ __host__ __device__ constexpr uint32_t make_idesc(int m, int n, bool bf16, bool 
 // Writes 32 rows x SEGS 16-byte segments - lane l holds row l in w[0..SEGS) - through the warp's staging area in
 // shared memory, so that one store instruction covers whole rows of SEGS * 16 contiguous bytes (four 128-byte lines
 // for SEGS = 8) instead of one 16-byte piece of 32 different lines. Segments are XOR-swizzled within a row: both the
-// row-per-lane writes and the segment-per-lane reads are free of bank conflicts. Called by all lanes of the warp.
+// row-per-lane writes and the segment-per-lane reads are free of bank conflicts. Called by all lanes of the warp; the first `rows_valid`
+// rows are written, the first `segs_valid` segments of each.
 // The area is addressed in the shared window: through generic pointers each read waited for the global store before it, which might
 // have gone to the same place (64 columns of a 256 x 256 product tile took 3000 cycles, most of them such waits).
 constexpr int kStageBytesPerWarp = 4096;
@@ -385,7 +386,8 @@ __device__ __forceinline__ uint4 ld_shared(uint32_t addr) {
     return x;
 }
 template <int SEGS>
-__device__ __forceinline__ void store_rows_coalesced(uint4* stage, const uint4* w, uint8_t* out0, long long ld_bytes, int rows_valid, int lane) {
+__device__ __forceinline__ void store_rows_coalesced(uint4* stage, const uint4* w, uint8_t* out0, long long ld_bytes, int rows_valid, int lane,
+                                                     int segs_valid = SEGS) {
     constexpr int RP = 32 / SEGS;  // rows per store instruction
     auto swz = [](int row) { return SEGS == 8 ? (row & 7) : ((row >> 1) & 3); };
     const uint32_t area = smem_u32(stage);
@@ -400,7 +402,7 @@ __device__ __forceinline__ void store_rows_coalesced(uint4* stage, const uint4* 
     uint8_t* out = out0 + (long long)sub * ld_bytes + q * 16;
 #pragma unroll
     for (int t = 0; t < SEGS; t++, out += RP * ld_bytes)
-        if (t * RP + sub < rows_valid) *(uint4*)out = x[t];
+        if (t * RP + sub < rows_valid && q < segs_valid) *(uint4*)out = x[t];
 }
 
 }  // namespace sm100
