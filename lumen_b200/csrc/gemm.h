@@ -17,7 +17,7 @@ struct SimtArgs {
     void* d;
     int d_dtype;
     int epilogue;
-    const void* aux;  // EPI_ADD / EPI_MASK operand (16-bit, the output's dtype), rows ld_aux apart, batches aux_sb apart
+    const void* aux;  // EPI_ADD / EPI_MASK operand (the output's dtype), rows ld_aux apart, batches aux_sb apart
     long long ld_aux, aux_sb;
     int a_vec, b_vec;  // groups of four elements along the operand's contiguous axis are aligned
 };

@@ -165,10 +165,15 @@ __device__ __forceinline__ void simt_tile(const T* ab, const T* bb, const SimtAr
             float x = acc[i][j];
             if (p.epilogue == EPI_RELU) x = fmaxf(x, 0.0f);
             if (p.epilogue >= EPI_ADD) {  // the rounded product, then the second primitive on it (as the tensor-core kernels do)
-                const uint16_t a16 = ((const uint16_t*)p.aux)[(long long)bz * p.aux_sb + (long long)gm * p.ld_aux + gn];
-                float prod, other;
-                if (p.d_dtype == LB_BF16) prod = __bfloat162float(__float2bfloat16_rn(x)), other = __uint_as_float((uint32_t)a16 << 16);
-                else prod = __half2float(__float2half_rn(x)), other = __half2float(__ushort_as_half(a16));
+                const long long from = (long long)bz * p.aux_sb + (long long)gm * p.ld_aux + gn;
+                float prod = x, other;
+                if (p.d_dtype == LB_F32) {
+                    other = ((const float*)p.aux)[from];
+                } else {
+                    const uint16_t a16 = ((const uint16_t*)p.aux)[from];
+                    if (p.d_dtype == LB_BF16) prod = __bfloat162float(__float2bfloat16_rn(x)), other = __uint_as_float((uint32_t)a16 << 16);
+                    else prod = __half2float(__float2half_rn(x)), other = __half2float(__ushort_as_half(a16));
+                }
                 x = p.epilogue == EPI_ADD ? __fadd_rn(other, prod) : (other > 0.0f ? prod : 0.0f);
             }
             long long at = (long long)bz * p.d_sb + (long long)gm * p.ldd + gn;

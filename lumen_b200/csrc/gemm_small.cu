@@ -7,9 +7,10 @@
 // shared memory, added in rank order (no scratch memory, no second kernel, the same bits every run), each CTA of the
 // cluster writing its share of the rows in whole 128-byte lines.
 //
-// A block runs its last part once, so that part is kept short: one conversion of eight columns for each type, the operand of an epilogue
-// fetched in one piece before the ranks' sums, which are fetched four ranks at a time. us a product, before -> so: 200 x 4096 K 1024 8.13 ->
-// 6.6 (with a mask 9.43 -> 7.8), 64^3 4.3 -> 3.5, 128 x 8192 K 1024 8.5 -> 7.0, 1024^3 8.5 -> 7.3.
+// A block runs its last part once, and its instructions come from the L2, so that part is kept short: one conversion of eight columns for each
+// type, the operand of an epilogue fetched in one piece before the ranks' sums, which are fetched four ranks at a time, and a kernel without
+// clusters where no K range is cut. us a product, before -> so: 200 x 4096 K 1024 8.1 -> 5.9 (with a mask 9.4 -> 7.3), 64^3 4.3 -> 3.1,
+// 128 x 8192 K 1024 8.5 -> 6.3, 1024^3 8.5 -> 6.2; with ranges 704 x 1024 K 4096 16.8 -> 14.6, 200 x 1024 K 4096 9.1 -> 9.0.
 #include <cuda_fp16.h>
 
 #include "gemm.h"
@@ -42,7 +43,8 @@ __device__ __forceinline__ float4 load_cluster(uint32_t addr, uint32_t rank) {
 // byte offset of 16-byte chunk `c` of row `r` of the partial tile: eight rows' equal chunks fall in different banks
 __device__ __forceinline__ uint32_t chunk_at(int r, int c) { return (uint32_t)(r * BN * 4 + ((c ^ (r & 7)) << 4)); }
 
-template <int STAGES>
+// RANKS: a tile's K range is cut over a cluster
+template <int STAGES, bool RANKS>
 __global__ void __launch_bounds__(kThreads, 8 / STAGES)
 gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const SmallGemmArgs p) {
     extern __shared__ uint8_t smem_raw[];
@@ -55,10 +57,10 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform for the compiler too
-    const int rank = p.splits > 1 ? (int)cluster_ctarank() : 0, unit = blockIdx.x / p.splits;
+    const int splits = RANKS ? p.splits : 1, rank = RANKS ? (int)cluster_ctarank() : 0, unit = blockIdx.x / splits;
     const int n_blk = unit % p.tiles_n, m_blk = unit / p.tiles_n % p.tiles_m, b = unit / (p.tiles_n * p.tiles_m);
     const int total_kb = (p.K + BK - 1) / BK;
-    const int kb0 = total_kb * rank / p.splits, num_kb = total_kb * (rank + 1) / p.splits - kb0;
+    const int kb0 = total_kb * rank / splits, num_kb = total_kb * (rank + 1) / splits - kb0;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
@@ -77,15 +79,15 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    grid_wait();
 
     // Where ranks add up their sums, the warps that wait for the accumulator go through the last part once before, on whatever shared memory
     // holds and without loads or stores of global memory: a block runs it once, and its instructions are then there when they are needed. us:
-    // 200 x 1024 K 4096 (four ranks) 9.40 -> 8.99, 512^3 (eight) 7.3 -> 6.8. One rank's is short enough not to (200 x 4096 K 1024 6.6 -> 7.1).
+    // 200 x 1024 K 4096 (four ranks) 9.40 -> 8.99, 512^3 (eight) 7.3 -> 6.8.
 #pragma unroll 1
-    for (int pass = warp >= 2 && STAGES == 8 && p.splits > 1 ? 0 : 1; pass < 2; pass++) {
+    for (int pass = warp >= 2 && STAGES == 8 && RANKS ? 0 : 1; pass < 2; pass++) {
         const bool dry = pass == 0;
         if (!dry) {
-            grid_wait();
             if (warp == 0) {
                 if (lane == 0) {
                     bool ok = true;
@@ -135,12 +137,12 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 }
             }
             __syncwarp();
-            if (p.splits > 1) cluster_sync();
+            if (RANKS) cluster_sync();
             else __syncthreads();
         }
 
         // this CTA's share of the rows: eight columns per thread
-        const int rows = BM / p.splits;
+        const int rows = BM / splits;
         const bool good = !dry && !*abort_flag;
         for (int i = dry ? threadIdx.x % 128 : (int)threadIdx.x; i < rows * (BN / 8); i += kThreads) {
             const int r = rank * rows + i / (BN / 8), q = i % (BN / 8);
@@ -163,15 +165,15 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
             const uint32_t at0 = smem_u32(smem) + chunk_at(r, 2 * q), at1 = smem_u32(smem) + chunk_at(r, 2 * q + 1);
             float x[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-            if (p.splits > 1) {
-                for (int s0 = 0; s0 < p.splits; s0 += 4) {  // up to four ranks' at once
+            if (RANKS) {
+                for (int s0 = 0; s0 < splits; s0 += 4) {  // up to four ranks' at once
                     float4 u[4], w[4];
 #pragma unroll
                     for (int s = 0; s < 4; s++)
-                        if (s0 + s < p.splits) u[s] = load_cluster(at0, dry ? rank : s0 + s), w[s] = load_cluster(at1, dry ? rank : s0 + s);
+                        if (s0 + s < splits) u[s] = load_cluster(at0, dry ? rank : s0 + s), w[s] = load_cluster(at1, dry ? rank : s0 + s);
 #pragma unroll
                     for (int s = 0; s < 4; s++)
-                        if (s0 + s < p.splits) {
+                        if (s0 + s < splits) {
                             x[0] += u[s].x, x[1] += u[s].y, x[2] += u[s].z, x[3] += u[s].w;
                             x[4] += w[s].x, x[5] += w[s].y, x[6] += w[s].z, x[7] += w[s].w;
                         }
@@ -239,7 +241,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         }
     }
     __syncwarp();
-    if (p.splits > 1) cluster_sync();  // no CTA leaves while another reads its partial tile
+    if (RANKS) cluster_sync();  // no CTA leaves while another reads its partial tile
     else __syncthreads();
     if (warp == 1) {
         tc_fence_after();
@@ -249,11 +251,11 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
 }  // namespace
 
-template <int STAGES>
+template <int STAGES, bool RANKS>
 static void launch_small(const CUtensorMap& map_a, const CUtensorMap& map_b, const SmallGemmArgs& p, int batch, cudaStream_t s) {
-    if (first_use_on_device((const void*)gemm_small_kernel<STAGES>))
-        LB_CUDA(cudaFuncSetAttribute(gemm_small_kernel<STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(STAGES)));
-    launch_overlapped(gemm_small_kernel<STAGES>, dim3((unsigned)((long long)p.tiles_m * p.tiles_n * batch * p.splits)), dim3(kThreads), smem_bytes(STAGES), s,
+    if (first_use_on_device((const void*)gemm_small_kernel<STAGES, RANKS>))
+        LB_CUDA(cudaFuncSetAttribute(gemm_small_kernel<STAGES, RANKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(STAGES)));
+    launch_overlapped(gemm_small_kernel<STAGES, RANKS>, dim3((unsigned)((long long)p.tiles_m * p.tiles_n * batch * p.splits)), dim3(kThreads), smem_bytes(STAGES), s,
                       (unsigned)p.splits, map_a, map_b, p);
 }
 
@@ -262,8 +264,9 @@ void gemm_small(const CUtensorMap& map_a, const CUtensorMap& map_b, SmallGemmArg
     const int per_line = p.d_bf16 || p.d_f16 ? 8 : 4;
     p.aux_vec = (uintptr_t)p.aux % 16 == 0 && p.ld_aux % 8 == 0 && p.aux_batch_stride % 8 == 0;
     p.vec = (uintptr_t)p.d % 16 == 0 && p.ldd % per_line == 0 && p.d_batch_stride % per_line == 0;
-    if ((long long)p.tiles_m * p.tiles_n * batch * p.splits <= sms) launch_small<8>(map_a, map_b, p, batch, s);
-    else launch_small<4>(map_a, map_b, p, batch, s);
+    if ((long long)p.tiles_m * p.tiles_n * batch * p.splits > sms) launch_small<4, true>(map_a, map_b, p, batch, s);
+    else if (p.splits > 1) launch_small<8, true>(map_a, map_b, p, batch, s);
+    else launch_small<8, false>(map_a, map_b, p, batch, s);
 }
 
 }  // namespace lb

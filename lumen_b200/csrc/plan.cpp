@@ -291,17 +291,18 @@ struct Products {
     std::vector<SimtProblem> held;
     std::vector<Bytes> read, written;
     static bool takes(const Step& s, const lb_tensor& a) { return s.kind == GEMM && a.dtype == LB_F32; }
-    bool independent(const lb_tensor& a, const lb_tensor& b, const lb_tensor& d) const {
-        const Bytes x(a), y(b), z(d);
+    bool independent(const lb_tensor& a, const lb_tensor& b, const lb_tensor& d, const lb_tensor* aux) const {
+        const Bytes x(a), y(b), z(d), u(aux ? *aux : a);
         for (const Bytes& w : written)
-            if (w.meets(x) || w.meets(y) || w.meets(z)) return false;
+            if (w.meets(x) || w.meets(y) || w.meets(z) || w.meets(u)) return false;
         for (const Bytes& r : read)
             if (r.meets(z)) return false;
         return true;
     }
-    void add(const lb_tensor& a, const lb_tensor& b, const lb_tensor& d, const SimtProblem& q) {
+    void add(const lb_tensor& a, const lb_tensor& b, const lb_tensor& d, const lb_tensor* aux, const SimtProblem& q) {
         held.push_back(q);
         read.emplace_back(a), read.emplace_back(b), written.emplace_back(d);
+        if (aux) read.emplace_back(*aux);
     }
     int queue(int sms, bool launch, cudaStream_t s) {
         if (held.empty()) return 0;
@@ -322,10 +323,11 @@ void run(const lb_plan& p, void* ws, void* const* in, void* const* out, int firs
         const Step& s = p.steps[k];
         auto T = [&](int i) { return bind(p, s.args.at(i), ws, in, out); };
         if (s.kind == GEMM && Products::takes(s, T(0))) {
-            const lb_tensor a = T(0), b = T(1), d = T(2);
-            if (!products.independent(a, b, d)) queue();
+            const lb_tensor a = T(0), b = T(1), d = T(2), other = s.aux >= 0 ? bind(p, s.aux, ws, in, out) : lb_tensor{};
+            const lb_tensor* aux = s.aux >= 0 ? &other : nullptr;
+            if (!products.independent(a, b, d, aux)) queue();
             SimtProblem q{};
-            if (gemm(a, b, d, s.epilogue, s.tuned_kernel, stream, nullptr, 0, nullptr, &s.tuning, &q)) products.add(a, b, d, q);
+            if (gemm(a, b, d, s.epilogue, s.tuned_kernel, stream, nullptr, 0, aux, &s.tuning, &q)) products.add(a, b, d, aux, q);
             continue;
         }
         queue();
@@ -604,18 +606,20 @@ int lb_plan_kernel_launches(const lb_plan* plan) {
         lb::Products products;  // told apart by where they lie in the workspace, which input and which output they are
         const int sms = lb::sm_count_hint();
         for (const lb::Step& s : plan->steps) {
-            auto place = [&](int i) {
-                const lb::View& v = plan->views.at((size_t)s.args.at(i));
+            auto placed = [&](int id) {
+                const lb::View& v = plan->views.at((size_t)id);
                 lb_tensor t = v.t;
                 const uintptr_t base = v.base_kind == 'w' ? 1 : 2 + 2 * (uintptr_t)v.base_index + (v.base_kind == 'o');
                 t.ptr = (void*)((base << 44) + v.offset);
                 return t;
             };
+            auto place = [&](int i) { return placed(s.args.at(i)); };
             if (s.kind == lb::GEMM && lb::Products::takes(s, place(0))) {
-                const lb_tensor a = place(0), b = place(1), d = place(2);
-                if (!products.independent(a, b, d)) n += products.queue(sms, false, nullptr);
+                const lb_tensor a = place(0), b = place(1), d = place(2), other = s.aux >= 0 ? placed(s.aux) : lb_tensor{};
+                const lb_tensor* aux = s.aux >= 0 ? &other : nullptr;
+                if (!products.independent(a, b, d, aux)) n += products.queue(sms, false, nullptr);
                 lb::SimtProblem q{};
-                if (lb::gemm_held(a, b, q)) products.add(a, b, d, q);
+                if (lb::gemm_held(a, b, q)) products.add(a, b, d, aux, q);
                 continue;
             }
             n += products.queue(sms, false, nullptr);

@@ -163,11 +163,11 @@ def linear(tape: Tape, x: TracedTensor, w: TracedTensor, output_dtype: str | Non
     """`x @ w.t()` for `x` `[rows, in]` and `w` `[out, in]`, accumulated in float32, written as `output_dtype`
     (the operands' by default): `F.matmul(x, w.t(), "float32", dtype)` (examples/transformer.py:116-121). A
     `dot_general` fusion carries an elementwise tail into the GEMM's epilogue, as the reference's fusion pass does
-    (lumen/codegen/fusion/triton.rs:56-74): `relu`, and `residual + product` for 16-bit models. In the backward of a
-    16-bit model, the product that yields the cotangent of a relu output is masked by that output in its epilogue
+    (lumen/codegen/fusion/triton.rs:56-74): `relu`, and `residual + product` where the product has the operands' dtype. In the
+    backward, the product that yields the cotangent of a relu output is masked by that output in its epilogue
     (the relu's own backward), instead of in a separate pass over the activations."""
     out_dtype = output_dtype or x.dtype
-    if residual is not None and out_dtype == "float32":
+    if residual is not None and out_dtype == "float32" != x.dtype:
         return add(tape, residual, linear(tape, x, w, output_dtype, relu))
     dims = (((1,), (1,)), ((), ()))
 
@@ -191,7 +191,7 @@ def linear(tape: Tape, x: TracedTensor, w: TracedTensor, output_dtype: str | Non
             dy = fused(lambda g: g.to(x.dtype), dy, label="narrow_cotangent")
         acc = "float32"
         dx_dims = (((1,), (0,)), ((), ()))
-        if getattr(x, "relu_output", False) and x.dtype != "float32":
+        if getattr(x, "relu_output", False):
             # x = relu(..): its cotangent passes where x > 0. Fused into this product's epilogue.
             dx = fused(lambda g, ww, out: F.where(F.gt(out, 0), prims.dot_general(g, ww, dx_dims, acc, x.dtype), 0), dy, w, x,
                        name="dot_general", label="linear_backward_relu")
