@@ -78,113 +78,86 @@ __device__ __forceinline__ int tile_coords(const GemmArgs& p, int unit, int& b, 
     return split;
 }
 
+// The cold paths of what follows lie behind the others: a block of one tile runs its way out once, and its instructions come from the L2.
+#define LB_RARELY(x) __builtin_expect(!!(x), 0)
+
 // Drains 128 accumulator columns (this warp's half of a 256-wide tile) of the thread's row from tensor memory and
 // stores them with the epilogue and one rounding to the output dtype. `release` hands the accumulator back to the MMA warp, once its
-// last columns are in registers.
+// last columns are in registers. Rows leave through the staging area, 128 contiguous bytes of each or, at the end of rows whose length is a
+// multiple of 16 bytes, as many 16-byte pieces as there are; other rows by the element.
 template <class Release>
 __device__ __forceinline__ void drain_tile(const GemmArgs& p, uint32_t tbase, int row, long long row_off, int col_base, int b,
                                            bool vec_ok, uint4* stage, int lane, Release release) {
+    const int rows = p.M - (row - lane);
 #pragma unroll 1
     for (int c2 = 0; c2 < BN / 2 / 64; c2++) {
-        // warp-uniform: 16-bit rows leave through the staging area, 128 contiguous bytes per row or, at the end of rows whose length is a multiple
-        // of eight, as many 16-byte pieces as there are
-        const int span = p.N - (col_base + c2 * 64);
-        const bool coalesced = vec_ok && (p.d_bf16 || p.d_f16) && (span >= 64 || (p.N % 8 == 0 && span > 0));
-        uint4 packed[8];
-        uint32_t vv[64];
-        tmem_ld_32x32(tbase + c2 * 64, vv);  // two loads in flight, one wait
-        tmem_ld_32x32(tbase + c2 * 64 + 32, vv + 32);
+        const int col0 = col_base + c2 * 64, span = p.N - col0;  // warp-uniform
+        uint32_t v[64];
+        tmem_ld_32x32(tbase + c2 * 64, v);  // two loads in flight, one wait
+        tmem_ld_32x32(tbase + c2 * 64 + 32, v + 32);
         tmem_ld_wait();
         if (c2 == BN / 2 / 64 - 1) release();
+        if (LB_RARELY(span <= 0)) continue;
+        if (p.epilogue == EPI_RELU) {
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            uint32_t* v = vv + h * 32;
-            const int col0 = col_base + c2 * 64 + h * 32;
-            // warp-uniform: a float32 row piece of 32 whole columns is one 128-byte line and leaves through the staging area too
-            const bool staged32 = vec_ok && !(p.d_bf16 || p.d_f16) && (col0 + 32 <= p.N || (p.N % 4 == 0 && col0 < p.N));
-            if (row < p.M && col0 < p.N) {
-                if (p.epilogue == EPI_RELU) {
+            for (int j = 0; j < 64; j++) v[j] = __float_as_uint(fmaxf(__uint_as_float(v[j]), 0.0f));
+        }
+        if (p.d_bf16 || p.d_f16) {
+            uint4 packed[8];
+            uint32_t* w = (uint32_t*)packed;
+            if (LB_RARELY(p.d_f16)) {
 #pragma unroll
-                    for (int j = 0; j < 32; j++) v[j] = __float_as_uint(fmaxf(__uint_as_float(v[j]), 0.0f));
+                for (int j = 0; j < 32; j++) {
+                    const __half2 h = __floats2half2_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+                    w[j] = *(const uint32_t*)&h;
                 }
-                const bool full_chunk = col0 + 32 <= p.N;
-                if (p.epilogue >= EPI_ADD) {
-                    // 16-bit outputs only (checked by the host). The product is rounded first, as its own primitive.
-                    const uint16_t* ax = (const uint16_t*)p.aux + (long long)b * p.aux_batch_stride + (long long)row * p.ld_aux + col0;
-                    uint32_t aw[16];
-                    if ((full_chunk || p.N % 8 == 0) && p.ld_aux % 8 == 0 && p.aux_batch_stride % 8 == 0 && ((uintptr_t)p.aux & 15) == 0) {
+            } else {
 #pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            const uint4 t = col0 + 8 * j < p.N ? *(const uint4*)(ax + 8 * j) : make_uint4(0u, 0u, 0u, 0u);
-                            aw[4 * j] = t.x, aw[4 * j + 1] = t.y, aw[4 * j + 2] = t.z, aw[4 * j + 3] = t.w;
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; j++) {
-                            const uint32_t lo = col0 + 2 * j < p.N ? ax[2 * j] : 0u, hi = col0 + 2 * j + 1 < p.N ? ax[2 * j + 1] : 0u;
-                            aw[j] = lo | (hi << 16);
-                        }
-                    }
-#pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        const uint16_t a16 = (uint16_t)(j & 1 ? aw[j / 2] >> 16 : aw[j / 2] & 0xffffu);
-                        const float acc = __uint_as_float(v[j]);
-                        float prod, other;
-                        if (p.d_bf16) prod = __bfloat162float(__float2bfloat16_rn(acc)), other = __uint_as_float((uint32_t)a16 << 16);
-                        else prod = __half2float(__float2half_rn(acc)), other = __half2float(__ushort_as_half(a16));
-                        v[j] = __float_as_uint(p.epilogue == EPI_ADD ? __fadd_rn(other, prod) : (other > 0.0f ? prod : 0.0f));
-                    }
-                }
-                if (p.d_bf16 || p.d_f16) {
-                    uint16_t* out = (uint16_t*)p.d + row_off + col0;
-                    if (coalesced || (full_chunk && vec_ok)) {
-#pragma unroll
-                        for (int j = 0; j < 32; j += 8) {
-                            uint32_t w[4];
-#pragma unroll
-                            for (int q = 0; q < 4; q++) {
-                                float lo = __uint_as_float(v[j + 2 * q]), hi = __uint_as_float(v[j + 2 * q + 1]);
-                                if (p.d_bf16) {
-                                    __nv_bfloat162 hh = __floats2bfloat162_rn(lo, hi);
-                                    w[q] = *(uint32_t*)&hh;
-                                } else {
-                                    __half2 hh = __floats2half2_rn(lo, hi);
-                                    w[q] = *(uint32_t*)&hh;
-                                }
-                            }
-                            if (coalesced) packed[h * 4 + j / 8] = make_uint4(w[0], w[1], w[2], w[3]);
-                            else *(uint4*)(out + j) = make_uint4(w[0], w[1], w[2], w[3]);
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; j++) {  // unrolled with a predicate: keeps the fragment in registers
-                            float x = __uint_as_float(v[j]);
-                            if (col0 + j < p.N)
-                                out[j] = p.d_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(x)) : __half_as_ushort(__float2half_rn(x));
-                        }
-                    }
-                } else {
-                    float* out = (float*)p.d + row_off + col0;
-                    if (staged32) {
-#pragma unroll
-                        for (int j = 0; j < 32; j += 4) packed[j / 4] = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                    } else if (full_chunk && vec_ok) {
-#pragma unroll
-                        for (int j = 0; j < 32; j += 4) *(uint4*)(out + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; j++)
-                            if (col0 + j < p.N) out[j] = __uint_as_float(v[j]);
-                    }
+                for (int j = 0; j < 32; j++) {
+                    const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+                    w[j] = *(const uint32_t*)&h;
                 }
             }
-            if (staged32)
-                store_rows_coalesced<8>(stage, packed, (uint8_t*)((float*)p.d + (row_off - (long long)lane * p.ldd) + col0), p.ldd * 4,
-                                        p.M - (row - lane), lane, (p.N - col0) / 4);
+            if (LB_RARELY(p.epilogue >= EPI_ADD && row < p.M)) {
+                // 16-bit outputs only (checked by the host). The product is rounded first, as its own primitive.
+                const uint16_t* ax = (const uint16_t*)p.aux + (long long)b * p.aux_batch_stride + (long long)row * p.ld_aux + col0;
+                const bool whole = (span >= 64 || p.N % 8 == 0) && p.ld_aux % 8 == 0 && p.aux_batch_stride % 8 == 0 && ((uintptr_t)p.aux & 15) == 0;
+#pragma unroll
+                for (int j0 = 0; j0 < 64; j0 += 8) {
+                    uint32_t aw[4] = {0u, 0u, 0u, 0u};
+                    if (whole && j0 < span) {
+                        const uint4 t = *(const uint4*)(ax + j0);
+                        aw[0] = t.x, aw[1] = t.y, aw[2] = t.z, aw[3] = t.w;
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; j++)
+                            if (j0 + j < span) aw[j / 2] |= (uint32_t)ax[j0 + j] << (j % 2 * 16);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; j++) w[j0 / 2 + j] = tail_pair(w[j0 / 2 + j], aw[j], p.epilogue == EPI_ADD, p.d_bf16);
+                }
+            }
+            uint16_t* out = (uint16_t*)p.d + row_off + col0;
+            if (LB_RARELY(!vec_ok || (span < 64 && p.N % 8 != 0))) {
+#pragma unroll
+                for (int j = 0; j < 64; j++)  // unrolled with a predicate: keeps the fragment in registers
+                    if (row < p.M && j < span) out[j] = (uint16_t)(w[j / 2] >> (j % 2 * 16));
+            } else {
+                store_rows_coalesced<8>(stage, packed, (uint8_t*)(out - (long long)lane * p.ldd), p.ldd * 2, rows, lane, span / 8);
+            }
+        } else {
+            float* out = (float*)p.d + row_off + col0;
+            if (LB_RARELY(!vec_ok || (span < 64 && p.N % 4 != 0))) {
+#pragma unroll
+                for (int j = 0; j < 64; j++)
+                    if (row < p.M && j < span) out[j] = __uint_as_float(v[j]);
+            } else {
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    store_rows_coalesced<8>(stage, (const uint4*)(v + h * 32), (uint8_t*)(out - (long long)lane * p.ldd + h * 32), p.ldd * 4, rows, lane,
+                                            (span - h * 32) / 4);
+            }
         }
-        if (coalesced)  // rows past M hold nothing and are not written
-            store_rows_coalesced<8>(stage, packed, (uint8_t*)((uint16_t*)p.d + (row_off - (long long)lane * p.ldd) + col_base + c2 * 64),
-                                    p.ldd * 2, p.M - (row - lane), lane, span / 8);
     }
 }
 
@@ -259,31 +232,19 @@ __device__ __forceinline__ void drain_tile_aux(const GemmArgs& p, uint32_t tbase
         tmem_ld_wait();
         if (c == BN / 2 / 32 - 1) release();
         uint4 packed[4];
+        uint32_t* w = (uint32_t*)packed;
+        if (LB_RARELY(p.d_f16)) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 8) {
-            uint32_t w[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                float r[2];
-#pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    const uint32_t pair = aw[(j + 2 * q) / 2];
-                    const uint16_t a16 = (uint16_t)(u ? pair >> 16 : pair & 0xffffu);
-                    const float acc = __uint_as_float(v[j + 2 * q + u]);
-                    float prod, other;
-                    if (p.d_bf16) prod = __bfloat162float(__float2bfloat16_rn(acc)), other = __uint_as_float((uint32_t)a16 << 16);
-                    else prod = __half2float(__float2half_rn(acc)), other = __half2float(__ushort_as_half(a16));
-                    r[u] = p.epilogue == EPI_ADD ? __fadd_rn(other, prod) : (other > 0.0f ? prod : 0.0f);
-                }
-                if (p.d_bf16) {
-                    __nv_bfloat162 hh = __floats2bfloat162_rn(r[0], r[1]);
-                    w[q] = *(uint32_t*)&hh;
-                } else {
-                    __half2 hh = __floats2half2_rn(r[0], r[1]);
-                    w[q] = *(uint32_t*)&hh;
-                }
+            for (int j = 0; j < 16; j++) {
+                const __half2 h = __floats2half2_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+                w[j] = tail_pair(*(const uint32_t*)&h, aw[j], p.epilogue == EPI_ADD, false);
             }
-            packed[j / 8] = make_uint4(w[0], w[1], w[2], w[3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+                w[j] = tail_pair(*(const uint32_t*)&h, aw[j], p.epilogue == EPI_ADD, true);
+            }
         }
         store_rows_coalesced<4>(stage, packed, out0 + c * 64, p.ldd * 2, 32, lane);
     }
@@ -438,7 +399,7 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                 if (lane == 0) mbar_arrive(&tmem_empty[buf]);
             };
             if (fast) drain_tile_aux(p, tbase, row_off + col_base, ax_warp, raw, stage, lane, release);
-            else if (p.splits > 1) drain_partial(p, tbase, row, col_base, b, split, stage, lane, release);
+            else if (LB_RARELY(p.splits > 1)) drain_partial(p, tbase, row, col_base, b, split, stage, lane, release);
             else drain_tile(p, tbase, row, row_off, col_base, b, vec_ok, stage, lane, release);
         }
     }
@@ -475,9 +436,10 @@ gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
 // divisions; the staging area is addressed as shared memory; and products are issued warp-wide. Together, us a product, bfloat16:
 // 16384 x 4096 with K = 64 92 -> 45, K = 512 108 -> 74, K = 1024 142 -> 119; 16384 x 32768 x 1024 1100 -> 920; 6442 x 1120 x 280
 // 17.8 -> 12.9; 3000 x 3000 x 600 23.8 -> 18.8; 16384 x 1024 x 4096 121 -> 117; 8192^3 885 -> 858.
-// Row pieces at the end of rows leave through the staging area like whole ones, where one store an element of a thread's row stood in line
-// (1000 x 3000 K 704 12.2 -> 9.8, 6442 x 1120 x 280 12.4 -> 10.6); without that code the kernel has no spills, and every product is about a
-// microsecond faster: 1024 x 4096 K 200 8.3 -> 7.3, 704 x 3072 K 1024 11.9 -> 10.8, 2048^3 17.5 -> 16.4, 16384 x 4096 K 1024 98.9 -> 96.
+// What a block runs once comes from the L2 instruction by instruction, and most products are a tile or two to a block: the way out is
+// kept short and its cold paths behind the others, row pieces at the end of rows leave through the staging area like whole ones (one store an
+// element of a thread's row stood in line for them), and the add and mask tails are packed. us a product: 1024 x 4096 K 200 8.3 -> 6.4, 704 x 3072
+// K 1024 11.8 -> 9.8, 2048^3 17.4 -> 15.2, 4096 x 4096 K 1024 with a mask 32.8 -> 31.2, 1000 x 3000 K 704 12.2 -> 9.7, 6442 x 1120 x 280 12.4 -> 9.4.
 constexpr int PSTAGES = 6;
 constexpr int kPairStageBytesA = BM * BK * 2, kPairStageBytesB = (BN / 2) * BK * 2;
 constexpr int kPairSmemBytes = PSTAGES * (kPairStageBytesA + kPairStageBytesB) + 1024 + 256 + kEpilogueStageBytes;
@@ -632,7 +594,7 @@ gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 if (lane == 0) mbar_arrive_cluster(&tmem_empty[buf], 0);
             };
             if (fast) drain_tile_aux(p, tbase, row_off + col_base, ax_warp, raw, stage, lane, release);
-            else if (p.splits > 1) drain_partial(p, tbase, row, col_base, b, split, stage, lane, release);
+            else if (LB_RARELY(p.splits > 1)) drain_partial(p, tbase, row, col_base, b, split, stage, lane, release);
             else drain_tile(p, tbase, row, row_off, col_base, b, vec_ok, stage, lane, release);
         }
     }

@@ -1,6 +1,10 @@
 // What the GEMM kernels' files share.
 #pragma once
 #include <cuda.h>
+#ifdef __CUDACC__
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#endif
 
 #include "device.h"
 
@@ -9,6 +13,22 @@ namespace lb {
 // EPI_ADD: out = round(round(acc) + aux); EPI_MASK: out = aux > 0 ? round(acc) : 0 - each exactly the two primitives
 // of the traced program (a rounded product followed by an add / a select), with `aux` a tensor shaped like the output
 enum Epilogue : int { EPI_NONE = 0, EPI_RELU = 1, EPI_ADD = 2, EPI_MASK = 3 };
+
+#ifdef __CUDACC__
+// Two products rounded to 16 bits and the tail's operand beside them: their sums, or the products where the operand is positive. The packed
+// add rounds the exact sum once; a float32 add and a rounding to 16 bits give the same, since what float32 drops lies 2^-24 below the larger
+// term, and no 16-bit rounding boundary is as near to a 16-bit value.
+__device__ __forceinline__ uint32_t tail_pair(uint32_t product, uint32_t other, bool adds, bool bf16) {
+    if (bf16) {
+        const __nv_bfloat162 x = *(const __nv_bfloat162*)&other, y = *(const __nv_bfloat162*)&product;
+        const __nv_bfloat162 sum = __hadd2_rn(x, y);
+        return adds ? *(const uint32_t*)&sum : product & __hgt2_mask(x, __floats2bfloat162_rn(0.0f, 0.0f));
+    }
+    const __half2 x = *(const __half2*)&other, y = *(const __half2*)&product;
+    const __half2 sum = __hadd2_rn(x, y);
+    return adds ? *(const uint32_t*)&sum : product & __hgt2_mask(x, __floats2half2_rn(0.0f, 0.0f));
+}
+#endif
 
 // The CUDA-core GEMM (gemm_simt.cu): any strides, element strides of the M, N and K axes.
 struct SimtArgs {

@@ -9,7 +9,7 @@
 //
 // A block runs its last part once, and its instructions come from the L2, so that part is kept short: one conversion of eight columns for each
 // type, the operand of an epilogue fetched in one piece before the ranks' sums, which are fetched four ranks at a time, and a kernel without
-// clusters where no K range is cut. us a product, before -> so: 200 x 4096 K 1024 8.1 -> 5.9 (with a mask 9.4 -> 7.3), 64^3 4.3 -> 3.1,
+// clusters where no K range is cut. us a product, before -> so: 200 x 4096 K 1024 8.1 -> 5.9 (with a mask 9.4 -> 6.8), 64^3 4.3 -> 3.1,
 // 128 x 8192 K 1024 8.5 -> 6.3, 1024^3 8.5 -> 6.2; with ranges 704 x 1024 K 4096 16.8 -> 14.6, 200 x 1024 K 4096 9.1 -> 9.0.
 #include <cuda_fp16.h>
 
@@ -186,29 +186,26 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             if (p.epilogue == EPI_RELU) {
 #pragma unroll
                 for (int j = 0; j < 8; j++) x[j] = fmaxf(x[j], 0.0f);
-            } else if (p.epilogue >= EPI_ADD) {  // 16-bit outputs only; the product is rounded first, as its own primitive
-                if (p.d_bf16) {
-#pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        const float prod = __bfloat162float(__float2bfloat16_rn(x[j])), other = __uint_as_float(j % 2 ? a[j / 2] & 0xffff0000u : a[j / 2] << 16);
-                        x[j] = p.epilogue == EPI_ADD ? __fadd_rn(other, prod) : (other > 0.0f ? prod : 0.0f);
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        const float prod = __half2float(__float2half_rn(x[j])), other = __half2float(__ushort_as_half((unsigned short)(a[j / 2] >> (j % 2 * 16))));
-                        x[j] = p.epilogue == EPI_ADD ? __fadd_rn(other, prod) : (other > 0.0f ? prod : 0.0f);
-                    }
-                }
             }
             const long long at = (long long)b * p.d_batch_stride + row * p.ldd + col;
             if (p.d_bf16 || p.d_f16) {
                 uint32_t h[4];
+                if (p.d_bf16) {
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const __nv_bfloat162 hb = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
-                    const __half2 hf = __floats2half2_rn(x[2 * j], x[2 * j + 1]);
-                    h[j] = p.d_bf16 ? *(const uint32_t*)&hb : *(const uint32_t*)&hf;
+                    for (int j = 0; j < 4; j++) {
+                        const __nv_bfloat162 t = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
+                        h[j] = *(const uint32_t*)&t;
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const __half2 t = __floats2half2_rn(x[2 * j], x[2 * j + 1]);
+                        h[j] = *(const uint32_t*)&t;
+                    }
+                }
+                if (p.epilogue >= EPI_ADD) {  // 16-bit outputs only; the product is rounded first, as its own primitive
+#pragma unroll
+                    for (int j = 0; j < 4; j++) h[j] = tail_pair(h[j], a[j], p.epilogue == EPI_ADD, p.d_bf16);
                 }
                 uint16_t* out = (uint16_t*)p.d + at;
                 if (whole) {
