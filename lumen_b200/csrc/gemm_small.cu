@@ -229,6 +229,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             if (dry) break;
         }
     }
+    __syncwarp();
+    if (RANKS) cluster_arrive_done();
     __syncthreads();
     if (*abort_flag) {
         if (threadIdx.x == 0) atomicExch(p.status, LB_ERR_TIMEOUT);
@@ -238,7 +240,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         }
     }
     __syncwarp();
-    if (RANKS) cluster_sync();  // no CTA leaves while another reads its partial tile
+    if (RANKS) cluster_wait_done();  // no CTA leaves while another reads its partial tile
     else __syncthreads();
     if (warp == 1) {
         tc_fence_after();

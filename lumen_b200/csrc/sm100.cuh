@@ -264,6 +264,10 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same in two halves, for the end of what other CTAs of the cluster read from this one's shared memory: it orders no memory (a release
+// would wait, about a microsecond, for the thread's global stores), but a thread has what it has used of another CTA's when it arrives.
+__device__ __forceinline__ void cluster_arrive_done() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_done() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
 // Shared-memory addresses in the cluster window carry the CTA rank from bit 24 up; clearing bit 24 of this CTA's
 // barrier address names the barrier at the same offset in the pair's even CTA.
 constexpr uint32_t kLeaderMask = 0xFEFFFFFFu;
