@@ -670,6 +670,7 @@ class Generator {
             const int64_t threads = T_ * RPB_;
             resident_ = (int)std::max<int64_t>(1, warps ? std::min((warps * 32 + threads - 1) / threads, 1024 / threads) : 512 / threads);
         }
+        if (!mixed_ && !shifted_ && !multi_ && has_reduce_ && VEC_ * min_size == 16) row_residency(nvec);
         NCH_ = (int)((nvec + T_ - 1) / T_);
         if (shifted_) {
             period_ = VEC_;  // (the width is odd)
@@ -683,6 +684,51 @@ class Generator {
             if (g_.type(v).numel() >= (1LL << 31) - 4096) wide_index_ = true;
         if (multi_) wide_index_ = true;  // a group's row count is a run-time value
         pair_ = VEC_ >= 2 && computes_bf16();
+    }
+
+    // Threads of a row and blocks an SM of kernels that go over a row more than once, where the compiler's own choice of registers leaves an SM
+    // with one block of 256 threads, or rows of many vectors are summed over more threads than those sums are worth (each warp of a row takes
+    // part in every total: ten shuffles of 1024 threads' second stage). us, as it was -> so, 2^24 elements (2^25 from 4096 columns on, 2^27 of
+    // 32768), bfloat16 where nothing else is said, float16 alike:
+    //   norms - rows written by what their sums say and by operands of the columns, no exponential on the way - are built for 512 threads an SM,
+    //   768 where a thread has 16 elements: layer norm of 512 columns 23.2 -> 14.0, 1024 23.5 -> 14.3, 1536 16.2 -> 13.7, 4096 32.5 -> 26.7,
+    //   float32 25.6 -> 22.1, 24.1 -> 22.8, (12 elements: left, 22.2 -> 24.7 at 3072,) 4096 50.5 -> 43.3; rms norm (one sum) 9.8 -> 8.1, 9.8 -> 8.1, but
+    //   4096 22.4 -> 23.5;
+    //   ... of which 512 threads and more walked 16-bit rows: eleven vectors a thread, 1024 threads an SM. 9872 columns 42.1 -> 32.0 (rms 30.0 ->
+    //   21.1), 32768 148 -> 127 (96.9 -> 95.1);
+    //   rows that are summed several times and not written (cross entropy), 16 bits, 512 threads and more: eleven vectors a thread too. 9872
+    //   columns 21.7 -> 15.0, 16384 33.9 -> 28.2, 32768 76.8 -> 53.8, but 50304 (608 threads) 59.7 -> 63.7;
+    //   float32 rows of several sums, no operands of columns, of which a power of two of threads leaves some idle: 9872 columns, softmax 52.9 ->
+    //   45.6, cross entropy 41.0 -> 30.6 (layer norm of 6000 columns 31.5 -> 33.4).
+    // Others are left: softmax, whose exponentials are taken again for its result, 0.8 - 1.3 of the time on any other threads, log softmax and
+    // centred rows 1.0 - 1.4.
+    int per_sm_ = 0;
+    void row_residency(int64_t nvec) {
+        int sums = 0, behind = 0;
+        std::map<int, int> seen;  // of a value: 1 behind a row's sum, 2 from an exponential of the space
+        for (const Node& n : g_.nodes) {
+            const bool reduce = n.op == "reduce_sum" || n.op == "reduce_max";
+            sums += reduce;
+            int has = reduce ? 1 : n.op == "exp" ? 2 : 0;
+            for (int v : n.inputs)
+                if (auto it = seen.find(v); it != seen.end()) has |= reduce ? it->second & 1 : it->second;
+            seen[n.output] = has;
+        }
+        bool written = false, columns = false;
+        for (int v : g_.outputs)
+            if (g_.type(v).numel() == R_ * C_) written = true, behind |= seen[v];
+        for (int v : g_.inputs) columns |= g_.type(v).numel() == C_ && R_ > 1;
+        const bool norm = written && behind == 1 && columns, summed = !written && sums > 1;
+        const int64_t eleven = (nvec * 3 / 32 + 31) / 32 * 32, four = (nvec + 127) / 128 * 32;
+        if (T_ >= 512 && narrow_) {
+            if (norm && eleven <= 1024) T_ = (int)eleven, per_sm_ = std::max(1, 1024 / T_);
+            else if (summed && eleven <= 512) T_ = (int)eleven, per_sm_ = (T_ > 256 ? 1536 : 1024) / T_;
+        } else if (T_ >= 512) {
+            if (sums > 1 && !columns && 8 * four <= 7 * (int64_t)T_) T_ = (int)four;
+        } else if (T_ <= 256 && norm && (sums > 1 || T_ <= 64)) {
+            const int64_t elements = (nvec + T_ - 1) / T_ * VEC_;
+            if (elements >= 16) per_sm_ = std::max(1, (elements > 16 ? 512 : 768) / (T_ * RPB_));
+        }
     }
 
     // What a thread of a mixed kernel holds for each of its columns: a sum for each column total, the operands by column, and those over the
@@ -1611,6 +1657,7 @@ class Generator {
         } else {
             s << "extern \"C\" __global__ void __launch_bounds__(" << T_ * RPB_;
             if (mixed_ || shifted_) s << ", " << resident_;
+            else if (per_sm_) s << ", " << per_sm_;
             s << ") fused_kernel(";
             for (size_t i = 0; i < g_.inputs.size(); i++) s << (i ? ", " : "") << "const void*" << restrict_kw << " in" << i;
             for (size_t i = 0; i < g_.outputs.size(); i++)
@@ -1752,6 +1799,7 @@ class Generator {
         k.rows_per_block = RPB_;
         k.row_period = period_;
         if (shifted_) k.per_sm = resident_;
+        else k.per_sm = per_sm_;
         k.n_inputs = (int)g_.inputs.size();
         k.n_outputs = (int)g_.outputs.size();
         for (int v : g_.inputs) k.types.push_back(g_.type(v));
