@@ -5,7 +5,7 @@
 //    (count, starts, place, sort, rows) adds a row's updates in update order, rounding to the operand's dtype after
 //    every add exactly like the interpreter: bit-identical to it and from run to run. The ATOMIC form adds in float32
 //    atomics in arrival order and rounds once: results vary in the last bits when a row is hit more than once.
-//  * attention_simt_fwd / attention_simt_bwd: float32 or bfloat16, any head dim up to 256, one warp per query row,
+//  * attention_simt_fwd / attention_simt_bwd: float32 or bfloat16, any head dim up to 256, one or two query rows a warp,
 //    scores and sums in float32. Used for float32 graphs (no hidden narrowing to bf16 tensor cores)
 //    and head dims other than 64/128.
 #include "launch.cuh"
@@ -242,30 +242,30 @@ struct AttnShape {
     int tile_rows;  // CUDA-core attention: rows of the streamed tiles in shared memory (launch_attn)
 };
 
-// CUDA-core attention: one warp per row (a query of the forward and dQ kernels, a key of the dK/dV kernel), eight
+// CUDA-core attention: a warp for one row or two (queries of the forward and dQ kernels, keys of the dK/dV kernel), eight warps of
 // neighbouring rows of one head per CTA. The rows they attend to stream through shared memory 32 at a time, as float32.
 // Within a chunk a lane first owns one streamed row (its dot products run over the head dimension without any exchange
 // between lanes), then head-dim elements l, l + 32, ... (the weighted sum over the chunk). A warp-wide sum per streamed
 // row, as one row at a time would need, is a chain of five shuffles: at 64 keys of 32 elements those chains were nine
 // tenths of the 48 us that the forward took.
-constexpr int kAttnRows = 8, kChunk = 32;
+constexpr int kAttnWarps = 8, kChunk = 32;
 
 // DU: head-dim elements per lane. Row pitch: a multiple of four floats whose 16-byte groups fall in different banks for
 // eight neighbouring rows. The streamed tiles have as many rows as there are to stream, at most a chunk: with full tiles of
 // zeros, which left room for two blocks an SM, 1024 heads of one query and one key of 256 elements took 34 us (now 12; one row at a time,
 // without shared memory, 3.6: seven of a block's eight warps idle there), of eight 43 us (now 26), of 16 89 us (now 62).
-template <int DU>
+template <int DU, int RW = 1>
 struct AttnSmem {
-    static constexpr int kD = DU * 32, kPitch = kD + 4;
-    float (*weight)[kAttnRows][kChunk];  // [2]
-    float* own[2];                       // the warps' rows, kD apart
-    float* tile[2];                      // streamed rows, kPitch apart
+    static constexpr int kD = DU * 32, kPitch = kD + 4, kRows = kAttnWarps * RW;
+    float (*weight)[kRows][kChunk];  // [2]
+    float* own[2];                   // the warps' rows, kD apart
+    float* tile[2];                  // streamed rows, kPitch apart
     __device__ __forceinline__ AttnSmem(uint8_t* raw, int tile_rows) {
-        weight = (float(*)[kAttnRows][kChunk])raw;
-        own[0] = (float*)raw + 2 * kAttnRows * kChunk, own[1] = own[0] + kAttnRows * kD;
-        tile[0] = own[1] + kAttnRows * kD, tile[1] = tile[0] + tile_rows * kPitch;
+        weight = (float(*)[kRows][kChunk])raw;
+        own[0] = (float*)raw + 2 * kRows * kChunk, own[1] = own[0] + kRows * kD;
+        tile[0] = own[1] + kRows * kD, tile[1] = tile[0] + tile_rows * kPitch;
     }
-    static int bytes(int tile_rows) { return (2 * kAttnRows * (kChunk + kD) + 2 * tile_rows * kPitch) * (int)sizeof(float); }
+    static int bytes(int tile_rows) { return (2 * kRows * (kChunk + kD) + 2 * tile_rows * kPitch) * (int)sizeof(float); }
 };
 
 // Rows [row0, row0 + kChunk) of those before `end`; nothing is stored for the others, which no lane may then read. Unrolled to eight
@@ -280,10 +280,10 @@ __device__ __forceinline__ void load_chunk(float* dst, const T* base, long long 
     };
     if (end - row0 >= kChunk) {
 #pragma unroll (DU > 2 ? 8 : 4 * DU)
-        for (int i = threadIdx.x; i < kChunk * kD; i += kAttnRows * 32) element(i);
+        for (int i = threadIdx.x; i < kChunk * kD; i += kAttnWarps * 32) element(i);
     } else {
 #pragma unroll 2
-        for (int i = threadIdx.x; i < (int)(end - row0) * kD; i += kAttnRows * 32) element(i);
+        for (int i = threadIdx.x; i < (int)(end - row0) * kD; i += kAttnWarps * 32) element(i);
     }
 }
 template <class T, int DU>
@@ -291,31 +291,35 @@ __device__ __forceinline__ void load_own(float* dst, const T* row, bool live, in
 #pragma unroll
     for (int u = 0; u < DU; u++) dst[lane + 32 * u] = live && lane + 32 * u < D ? to_f(row[lane + 32 * u]) : 0.0f;
 }
-// The warp's own row times the chunk row this lane owns: 64 elements at a time (32 at head dims up to 64) in sixteen (eight)
+// The warp's own rows times the chunk row this lane owns: 64 elements at a time (32 at head dims up to 64) in sixteen (eight)
 // sums that are added as a tree. The error of a score then is that of a warp-wide sum - a lane's few terms, then a tree of
 // five - which one row at a time had, or a little below; in two running sums it is 1.2 times that at 32 elements and 2.5 times at 256.
-template <int DU>
-__device__ __forceinline__ float dot_row(const float* own, const float* tile, int lane) {
+template <int DU, int RW>
+__device__ __forceinline__ void dot_rows(float* total, const float* own, const float* tile, int lane) {
     constexpr int kBlock = DU <= 2 ? 32 : 64, kSums = kBlock / 4;
-    const float4* a = (const float4*)own;
     const float4* b = (const float4*)(tile + lane * AttnSmem<DU>::kPitch);
-    float total = 0.0f;
 #pragma unroll (DU > 2 ? 1 : 2)
     for (int d0 = 0; d0 < DU * 32; d0 += kBlock) {
-        float s[kSums] = {};
+        float s[RW][kSums] = {};
 #pragma unroll
         for (int d = 0; d < kBlock; d += 4) {
-            const float4 x = a[(d0 + d) / 4], y = b[(d0 + d) / 4];
-            float* t = s + d % kSums;
-            t[0] = fmaf(x.x, y.x, t[0]), t[1] = fmaf(x.y, y.y, t[1]), t[2] = fmaf(x.z, y.z, t[2]), t[3] = fmaf(x.w, y.w, t[3]);
+            const float4 y = b[(d0 + d) / 4];
+#pragma unroll
+            for (int r = 0; r < RW; r++) {
+                const float4 x = ((const float4*)(own + r * AttnSmem<DU>::kD))[(d0 + d) / 4];
+                float* t = s[r] + d % kSums;
+                t[0] = fmaf(x.x, y.x, t[0]), t[1] = fmaf(x.y, y.y, t[1]), t[2] = fmaf(x.z, y.z, t[2]), t[3] = fmaf(x.w, y.w, t[3]);
+            }
         }
 #pragma unroll
-        for (int h = kSums / 2; h >= 1; h /= 2)
+        for (int r = 0; r < RW; r++) {
 #pragma unroll
-            for (int i = 0; i < h; i++) s[i] += s[i + h];
-        total = d0 ? total + s[0] : s[0];
+            for (int h = kSums / 2; h >= 1; h /= 2)
+#pragma unroll
+                for (int i = 0; i < h; i++) s[r][i] += s[r][i + h];
+            total[r] = d0 ? total[r] + s[r][0] : s[r][0];
+        }
     }
-    return total;
 }
 // acc[u] += sum over the chunk's rows [lo, hi) of weight[row] * tile[row][lane + 32 u], in row order. The other rows are not
 // read: their weights are 0, but a value behind the mask may be infinite or NaN, and 0 times that is NaN.
@@ -349,125 +353,203 @@ __device__ __forceinline__ void add_weighted(float* acc, const float* weight, co
         }
     }
 }
-// the CTA's rows: kAttnRows neighbours of one (batch, head)
+// The same for the warp's RW rows, weights kChunk apart, whose ranges are [lo[r], hi[r]): a streamed element is fetched once for all of
+// them where they see the whole chunk.
+template <int DU, int RW>
+__device__ __forceinline__ void add_weighted_rows(float (*acc)[DU], const float* weight, const float* tile, int lane, const int* lo, const int* hi) {
+    bool whole = true;  // warp-uniform
+#pragma unroll
+    for (int r = 0; r < RW; r++) whole &= lo[r] <= 0 && hi[r] >= kChunk;
+    if (RW == 1 || !whole) {
+#pragma unroll
+        for (int r = 0; r < RW; r++) add_weighted<DU>(acc[r], weight + r * kChunk, tile, lane, lo[r], hi[r]);
+        return;
+    }
+#pragma unroll (DU > 2 ? 1 : 2)
+    for (int j = 0; j < kChunk; j += 4) {
+        float4 w[RW];
+#pragma unroll
+        for (int r = 0; r < RW; r++) w[r] = *(const float4*)(weight + r * kChunk + j);
+#pragma unroll
+        for (int u = 0; u < DU; u++) {
+            const float* t = tile + j * AttnSmem<DU>::kPitch + lane + 32 * u;
+            const float t0 = t[0], t1 = t[AttnSmem<DU>::kPitch], t2 = t[2 * AttnSmem<DU>::kPitch], t3 = t[3 * AttnSmem<DU>::kPitch];
+#pragma unroll
+            for (int r = 0; r < RW; r++) {
+                acc[r][u] = fmaf(w[r].x, t0, acc[r][u]);
+                acc[r][u] = fmaf(w[r].y, t1, acc[r][u]);
+                acc[r][u] = fmaf(w[r].z, t2, acc[r][u]);
+                acc[r][u] = fmaf(w[r].w, t3, acc[r][u]);
+            }
+        }
+    }
+}
+// the CTA's rows: kAttnWarps * RW neighbours of one (batch, head)
+template <int RW>
 __device__ __forceinline__ void block_rows(int rows, int heads, int& r0, int& n, int& b) {
-    const int per = (rows + kAttnRows - 1) / kAttnRows;
-    r0 = (int)(blockIdx.x % per) * kAttnRows, n = (int)(blockIdx.x / per % heads), b = (int)(blockIdx.x / per / heads);
+    constexpr int kRows = kAttnWarps * RW;
+    const int per = (rows + kRows - 1) / kRows;
+    r0 = (int)(blockIdx.x % per) * kRows, n = (int)(blockIdx.x / per % heads), b = (int)(blockIdx.x / per / heads);
 }
 
-template <class T, int DU>
-__global__ void __launch_bounds__(kAttnRows * 32)
+template <class T, int DU, int RW>
+__global__ void __launch_bounds__(kAttnWarps * 32)
 attention_simt_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ o,
                           float* __restrict__ lse, AttnShape s) {
     extern __shared__ __align__(16) uint8_t raw[];
-    AttnSmem<DU> sm(raw, s.tile_rows);
+    AttnSmem<DU, RW> sm(raw, s.tile_rows);
     grid_wait(q, k, v);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int i0, n, b;
-    block_rows(s.Sq, s.N, i0, n, b);
-    const int i = i0 + warp, nk = n / (s.N / s.Nkv);
-    const bool live = i < s.Sq;
-    float* own = sm.own[0] + warp * AttnSmem<DU>::kD;
-    load_own<T, DU>(own, q + b * s.q_s[0] + (long long)i * s.q_s[1] + n * s.q_s[2], live, s.D, lane);
-    const long long last = !live ? -1 : s.causal ? min((long long)s.Sk - 1, (long long)i + s.offset) : (long long)s.Sk - 1;
-    const long long end = s.causal ? min((long long)s.Sk, (long long)i0 + kAttnRows + s.offset) : (long long)s.Sk;  // past the CTA's last key
-    float acc[DU] = {}, m = -INFINITY, l = 0.0f;
+    block_rows<RW>(s.Sq, s.N, i0, n, b);
+    const int i = i0 + warp * RW, nk = n / (s.N / s.Nkv);  // the warp's first row
+    float* own = sm.own[0] + warp * RW * AttnSmem<DU>::kD;
+    long long last[RW];  // a row's last key, -1: none
+#pragma unroll
+    for (int r = 0; r < RW; r++) {
+        const bool live = i + r < s.Sq;
+        load_own<T, DU>(own + r * AttnSmem<DU>::kD, q + b * s.q_s[0] + (long long)(i + r) * s.q_s[1] + n * s.q_s[2], live, s.D, lane);
+        last[r] = !live ? -1 : s.causal ? min((long long)s.Sk - 1, (long long)i + r + s.offset) : (long long)s.Sk - 1;
+    }
+    const long long end = s.causal ? min((long long)s.Sk, (long long)i0 + kAttnWarps * RW + s.offset) : (long long)s.Sk;  // past the CTA's last key
+    float acc[RW][DU] = {}, m[RW], l[RW];
+#pragma unroll
+    for (int r = 0; r < RW; r++) m[r] = -INFINITY, l[r] = 0.0f;
     for (long long j0 = 0; j0 < end; j0 += kChunk) {
         __syncthreads();
         load_chunk<T, DU>(sm.tile[0], k + b * s.k_s[0] + nk * s.k_s[2], s.k_s[1], j0, end, s.D);
         load_chunk<T, DU>(sm.tile[1], v + b * s.v_s[0] + nk * s.v_s[2], s.v_s[1], j0, end, s.D);
         __syncthreads();
-        if (j0 > last) continue;  // warp-uniform: this row sees nothing of the chunk
-        const float sc = j0 + lane <= last ? dot_row<DU>(own, sm.tile[0], lane) * s.scale : -INFINITY;
-        float top = sc;
+        bool any = false;  // warp-uniform: rows that see something of the chunk
+        int hi[RW], lo[RW];
 #pragma unroll
-        for (int x = 16; x >= 1; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
-        const float m_new = fmaxf(m, top);
-        const float alpha = __expf(m - m_new), p = j0 + lane <= last ? __expf(sc - m_new) : 0.0f;
-        sm.weight[0][warp][lane] = p;
-        float sum = p;
+        for (int r = 0; r < RW; r++) lo[r] = 0, hi[r] = (int)max(0LL, min((long long)kChunk, last[r] + 1 - j0)), any |= hi[r] > 0;
+        if (!any) continue;
+        float dots[RW];
+        bool seen = false;
 #pragma unroll
-        for (int x = 16; x >= 1; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
-        l = l * alpha + sum;
+        for (int r = 0; r < RW; r++) seen |= lane < hi[r];
+        if (seen) dot_rows<DU, RW>(dots, own, sm.tile[0], lane);
 #pragma unroll
-        for (int u = 0; u < DU; u++) acc[u] *= alpha;
+        for (int r = 0; r < RW; r++) {
+            if (hi[r] == 0) continue;
+            const float sc = lane < hi[r] ? dots[r] * s.scale : -INFINITY;
+            float top = sc;
+#pragma unroll
+            for (int x = 16; x >= 1; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
+            const float m_new = fmaxf(m[r], top);
+            const float alpha = __expf(m[r] - m_new), p = lane < hi[r] ? __expf(sc - m_new) : 0.0f;
+            sm.weight[0][warp * RW + r][lane] = p;
+            float sum = p;
+#pragma unroll
+            for (int x = 16; x >= 1; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
+            l[r] = l[r] * alpha + sum;
+#pragma unroll
+            for (int u = 0; u < DU; u++) acc[r][u] *= alpha;
+            m[r] = m_new;
+        }
         __syncwarp();
         // the normaliser is applied at the end
-        add_weighted<DU>(acc, sm.weight[0][warp], sm.tile[1], lane, 0, (int)min((long long)kChunk, last + 1 - j0));
+        add_weighted_rows<DU, RW>(acc, sm.weight[0][warp * RW], sm.tile[1], lane, lo, hi);
         __syncwarp();
-        m = m_new;
     }
-    if (!live) return;
-    T* op = o + b * s.o_s[0] + (long long)i * s.o_s[1] + n * s.o_s[2];
 #pragma unroll
-    for (int u = 0; u < DU; u++)
-        if (lane + 32 * u < s.D) op[lane + 32 * u] = from_f<T>(acc[u] / l);
-    if (lse && lane == 0) lse[((long long)b * s.N + n) * s.Sq + i] = m + logf(l);
+    for (int r = 0; r < RW; r++) {
+        if (i + r >= s.Sq) break;
+        T* op = o + b * s.o_s[0] + (long long)(i + r) * s.o_s[1] + n * s.o_s[2];
+#pragma unroll
+        for (int u = 0; u < DU; u++)
+            if (lane + 32 * u < s.D) op[lane + 32 * u] = from_f<T>(acc[r][u] / l[r]);
+        if (lse && lane == 0) lse[((long long)b * s.N + n) * s.Sq + i + r] = m[r] + logf(l[r]);
+    }
 }
 
-// dQ: one warp per query row.
-template <class T, int DU>
-__global__ void __launch_bounds__(kAttnRows * 32)
+// dQ: RW query rows a warp.
+template <class T, int DU, int RW>
+__global__ void __launch_bounds__(kAttnWarps * 32)
 attention_simt_dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ g,
                          const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dq, AttnShape s) {
     extern __shared__ __align__(16) uint8_t raw[];
-    AttnSmem<DU> sm(raw, s.tile_rows);
+    AttnSmem<DU, RW> sm(raw, s.tile_rows);
     grid_wait(q, k, v, g, lse, delta);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int i0, n, b;
-    block_rows(s.Sq, s.N, i0, n, b);
-    const int i = i0 + warp, nk = n / (s.N / s.Nkv);
-    const bool live = i < s.Sq;
-    float *own_q = sm.own[0] + warp * AttnSmem<DU>::kD, *own_g = sm.own[1] + warp * AttnSmem<DU>::kD;
-    load_own<T, DU>(own_q, q + b * s.q_s[0] + (long long)i * s.q_s[1] + n * s.q_s[2], live, s.D, lane);
-    load_own<T, DU>(own_g, g + b * s.g_s[0] + (long long)i * s.g_s[1] + n * s.g_s[2], live, s.D, lane);
-    const long long at = ((long long)b * s.N + n) * s.Sq + i;
-    const float L = live ? lse[at] : 0.0f, dl = live ? delta[at] : 0.0f;
-    const long long last = !live ? -1 : s.causal ? min((long long)s.Sk - 1, (long long)i + s.offset) : (long long)s.Sk - 1;
-    const long long end = s.causal ? min((long long)s.Sk, (long long)i0 + kAttnRows + s.offset) : (long long)s.Sk;
-    float acc[DU] = {};
+    block_rows<RW>(s.Sq, s.N, i0, n, b);
+    const int i = i0 + warp * RW, nk = n / (s.N / s.Nkv);
+    float *own_q = sm.own[0] + warp * RW * AttnSmem<DU>::kD, *own_g = sm.own[1] + warp * RW * AttnSmem<DU>::kD;
+    long long last[RW];
+    float L[RW], dl[RW];
+#pragma unroll
+    for (int r = 0; r < RW; r++) {
+        const bool live = i + r < s.Sq;
+        load_own<T, DU>(own_q + r * AttnSmem<DU>::kD, q + b * s.q_s[0] + (long long)(i + r) * s.q_s[1] + n * s.q_s[2], live, s.D, lane);
+        load_own<T, DU>(own_g + r * AttnSmem<DU>::kD, g + b * s.g_s[0] + (long long)(i + r) * s.g_s[1] + n * s.g_s[2], live, s.D, lane);
+        const long long at = ((long long)b * s.N + n) * s.Sq + i + r;
+        L[r] = live ? lse[at] : 0.0f, dl[r] = live ? delta[at] : 0.0f;
+        last[r] = !live ? -1 : s.causal ? min((long long)s.Sk - 1, (long long)i + r + s.offset) : (long long)s.Sk - 1;
+    }
+    const long long end = s.causal ? min((long long)s.Sk, (long long)i0 + kAttnWarps * RW + s.offset) : (long long)s.Sk;
+    float acc[RW][DU] = {};
     for (long long j0 = 0; j0 < end; j0 += kChunk) {
         __syncthreads();
         load_chunk<T, DU>(sm.tile[0], k + b * s.k_s[0] + nk * s.k_s[2], s.k_s[1], j0, end, s.D);
         load_chunk<T, DU>(sm.tile[1], v + b * s.v_s[0] + nk * s.v_s[2], s.v_s[1], j0, end, s.D);
         __syncthreads();
-        if (j0 > last) continue;
-        float ds = 0.0f;
-        if (j0 + lane <= last) {
-            const float p = __expf(dot_row<DU>(own_q, sm.tile[0], lane) * s.scale - L);
-            ds = to_f(from_f<T>(p * (dot_row<DU>(own_g, sm.tile[1], lane) - dl) * s.scale));  // dS is rounded to the operands' dtype (flash.py:71)
+        bool any = false, seen = false;
+        int hi[RW], lo[RW];
+#pragma unroll
+        for (int r = 0; r < RW; r++) lo[r] = 0, hi[r] = (int)max(0LL, min((long long)kChunk, last[r] + 1 - j0)), any |= hi[r] > 0, seen |= lane < hi[r];
+        if (!any) continue;
+        float ds[RW] = {};
+        if (seen) {
+            float dots[RW], dp[RW];
+            dot_rows<DU, RW>(dots, own_q, sm.tile[0], lane);
+            dot_rows<DU, RW>(dp, own_g, sm.tile[1], lane);
+#pragma unroll
+            for (int r = 0; r < RW; r++) {
+                const float p = __expf(dots[r] * s.scale - L[r]);
+                if (lane < hi[r]) ds[r] = to_f(from_f<T>(p * (dp[r] - dl[r]) * s.scale));  // dS is rounded to the operands' dtype (flash.py:71)
+            }
         }
-        sm.weight[0][warp][lane] = ds;
+#pragma unroll
+        for (int r = 0; r < RW; r++) sm.weight[0][warp * RW + r][lane] = ds[r];
         __syncwarp();
-        add_weighted<DU>(acc, sm.weight[0][warp], sm.tile[0], lane, 0, (int)min((long long)kChunk, last + 1 - j0));
+        add_weighted_rows<DU, RW>(acc, sm.weight[0][warp * RW], sm.tile[0], lane, lo, hi);
         __syncwarp();
     }
-    if (!live) return;
-    T* out = dq + b * s.dq_s[0] + (long long)i * s.dq_s[1] + n * s.dq_s[2];
 #pragma unroll
-    for (int u = 0; u < DU; u++)
-        if (lane + 32 * u < s.D) out[lane + 32 * u] = from_f<T>(acc[u]);
+    for (int r = 0; r < RW; r++) {
+        if (i + r >= s.Sq) break;
+        T* out = dq + b * s.dq_s[0] + (long long)(i + r) * s.dq_s[1] + n * s.dq_s[2];
+#pragma unroll
+        for (int u = 0; u < DU; u++)
+            if (lane + 32 * u < s.D) out[lane + 32 * u] = from_f<T>(acc[r][u]);
+    }
 }
 
-// dK/dV: one warp per (b, kv head, key j), looping over the group's heads and the queries that see j.
-template <class T, int DU>
-__global__ void __launch_bounds__(kAttnRows * 32)
+// dK/dV: RW keys of a (batch, kv head) a warp, looping over the group's heads and the queries that see them.
+template <class T, int DU, int RW>
+__global__ void __launch_bounds__(kAttnWarps * 32)
 attention_simt_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ g,
                            const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dk, T* __restrict__ dv, AttnShape s) {
     extern __shared__ __align__(16) uint8_t raw[];
-    AttnSmem<DU> sm(raw, s.tile_rows);
+    AttnSmem<DU, RW> sm(raw, s.tile_rows);
     grid_wait(q, k, v, g, lse, delta);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int k0, nk, b;
-    block_rows(s.Sk, s.Nkv, k0, nk, b);
-    const int j = k0 + warp, group = s.N / s.Nkv;
-    const bool live = j < s.Sk;
-    float *own_k = sm.own[0] + warp * AttnSmem<DU>::kD, *own_v = sm.own[1] + warp * AttnSmem<DU>::kD;
-    load_own<T, DU>(own_k, k + b * s.k_s[0] + (long long)j * s.k_s[1] + nk * s.k_s[2], live, s.D, lane);
-    load_own<T, DU>(own_v, v + b * s.v_s[0] + (long long)j * s.v_s[1] + nk * s.v_s[2], live, s.D, lane);
-    float ak[DU] = {}, av[DU] = {};
-    const long long first = s.causal ? max(0LL, (long long)j - s.offset) : 0LL;       // the first query that sees this key
-    const long long begin = s.causal ? max(0LL, (long long)k0 - s.offset) : 0LL;      // ... that sees the CTA's first key
+    block_rows<RW>(s.Sk, s.Nkv, k0, nk, b);
+    const int j = k0 + warp * RW, group = s.N / s.Nkv;
+    float *own_k = sm.own[0] + warp * RW * AttnSmem<DU>::kD, *own_v = sm.own[1] + warp * RW * AttnSmem<DU>::kD;
+    long long first[RW];  // the first query that sees the key
+#pragma unroll
+    for (int r = 0; r < RW; r++) {
+        const bool live = j + r < s.Sk;
+        load_own<T, DU>(own_k + r * AttnSmem<DU>::kD, k + b * s.k_s[0] + (long long)(j + r) * s.k_s[1] + nk * s.k_s[2], live, s.D, lane);
+        load_own<T, DU>(own_v + r * AttnSmem<DU>::kD, v + b * s.v_s[0] + (long long)(j + r) * s.v_s[1] + nk * s.v_s[2], live, s.D, lane);
+        first[r] = !live ? (long long)s.Sq : s.causal ? max(0LL, (long long)j + r - s.offset) : 0LL;
+    }
+    float ak[RW][DU] = {}, av[RW][DU] = {};
+    const long long begin = s.causal ? max(0LL, (long long)k0 - s.offset) : 0LL;  // the first query that sees the CTA's first key
     for (int h = 0; h < group; h++) {
         const int n = nk * group + h;
         for (long long i0 = begin; i0 < s.Sq; i0 += kChunk) {
@@ -475,29 +557,43 @@ attention_simt_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, con
             load_chunk<T, DU>(sm.tile[0], q + b * s.q_s[0] + n * s.q_s[2], s.q_s[1], i0, s.Sq, s.D);
             load_chunk<T, DU>(sm.tile[1], g + b * s.g_s[0] + n * s.g_s[2], s.g_s[1], i0, s.Sq, s.D);
             __syncthreads();
-            if (!live || i0 + kChunk <= first) continue;
-            const long long i = i0 + lane;
-            float ds = 0.0f, pr = 0.0f;
-            if (i >= first && i < s.Sq) {
-                const long long at = ((long long)b * s.N + n) * s.Sq + i;
-                const float p = __expf(dot_row<DU>(own_k, sm.tile[0], lane) * s.scale - lse[at]);
-                ds = to_f(from_f<T>(p * (dot_row<DU>(own_v, sm.tile[1], lane) - delta[at]) * s.scale));
-                pr = to_f(from_f<T>(p));
+            const int rows = (int)min((long long)kChunk, s.Sq - i0);
+            bool any = false, seen = false;
+            int hi[RW], lo[RW];
+#pragma unroll
+            for (int r = 0; r < RW; r++)
+                lo[r] = (int)max(0LL, min((long long)kChunk, first[r] - i0)), hi[r] = lo[r] < rows ? rows : 0, any |= hi[r] > 0, seen |= lane >= lo[r] && lane < hi[r];
+            if (!any) continue;
+            float ds[RW] = {}, pr[RW] = {};
+            if (seen) {
+                const long long at = ((long long)b * s.N + n) * s.Sq + i0 + lane;
+                const float L = lse[at], dl = delta[at];
+                float dots[RW], dp[RW];
+                dot_rows<DU, RW>(dots, own_k, sm.tile[0], lane);
+                dot_rows<DU, RW>(dp, own_v, sm.tile[1], lane);
+#pragma unroll
+                for (int r = 0; r < RW; r++) {
+                    const float p = __expf(dots[r] * s.scale - L);
+                    if (lane >= lo[r] && lane < hi[r]) ds[r] = to_f(from_f<T>(p * (dp[r] - dl) * s.scale)), pr[r] = to_f(from_f<T>(p));
+                }
             }
-            sm.weight[0][warp][lane] = ds, sm.weight[1][warp][lane] = pr;
+#pragma unroll
+            for (int r = 0; r < RW; r++) sm.weight[0][warp * RW + r][lane] = ds[r], sm.weight[1][warp * RW + r][lane] = pr[r];
             __syncwarp();
-            const int lo = (int)max(0LL, first - i0), hi = (int)min((long long)kChunk, s.Sq - i0);
-            add_weighted<DU>(ak, sm.weight[0][warp], sm.tile[0], lane, lo, hi);
-            add_weighted<DU>(av, sm.weight[1][warp], sm.tile[1], lane, lo, hi);
+            add_weighted_rows<DU, RW>(ak, sm.weight[0][warp * RW], sm.tile[0], lane, lo, hi);
+            add_weighted_rows<DU, RW>(av, sm.weight[1][warp * RW], sm.tile[1], lane, lo, hi);
             __syncwarp();
         }
     }
-    if (!live) return;
-    T* ok = dk + b * s.dk_s[0] + (long long)j * s.dk_s[1] + nk * s.dk_s[2];
-    T* ov = dv + b * s.dv_s[0] + (long long)j * s.dv_s[1] + nk * s.dv_s[2];
 #pragma unroll
-    for (int u = 0; u < DU; u++)
-        if (lane + 32 * u < s.D) ok[lane + 32 * u] = from_f<T>(ak[u]), ov[lane + 32 * u] = from_f<T>(av[u]);
+    for (int r = 0; r < RW; r++) {
+        if (j + r >= s.Sk) break;
+        T* ok = dk + b * s.dk_s[0] + (long long)(j + r) * s.dk_s[1] + nk * s.dk_s[2];
+        T* ov = dv + b * s.dv_s[0] + (long long)(j + r) * s.dv_s[1] + nk * s.dv_s[2];
+#pragma unroll
+        for (int u = 0; u < DU; u++)
+            if (lane + 32 * u < s.D) ok[lane + 32 * u] = from_f<T>(ak[r][u]), ov[lane + 32 * u] = from_f<T>(av[r][u]);
+    }
 }
 
 template <class T>
@@ -791,19 +887,29 @@ void strided_copy(const lb_tensor& in, const lb_tensor& out, void* stream) {
 }
 
 namespace {
-// CTAs of kAttnRows rows over `rows` rows of every (batch, head)
-unsigned attn_blocks(long long batch, long long heads, long long rows) {
-    const long long blocks = batch * heads * ((rows + kAttnRows - 1) / kAttnRows);
+// CTAs of kAttnWarps * RW rows over `rows` rows of every (batch, head)
+unsigned attn_blocks(long long batch, long long heads, long long rows, int rw) {
+    const long long blocks = batch * heads * ((rows + kAttnWarps * rw - 1) / (kAttnWarps * rw));
     if (blocks > INT32_MAX) fail(LB_ERR_UNSUPPORTED, "attention: too many rows for the CUDA-core kernels' grid");
     return (unsigned)blocks;
 }
 // `streamed`: the rows that the kernel walks per head
-template <int DU, class Kernel, class... Args>
+template <int DU, int RW, class Kernel, class... Args>
 void launch_attn(Kernel kernel, unsigned blocks, int streamed, cudaStream_t st, AttnShape s, Args... args) {
-    if (AttnSmem<DU>::bytes(kChunk) > 48 * 1024 && first_use_on_device((const void*)kernel))
-        LB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnSmem<DU>::bytes(kChunk)));
+    if (AttnSmem<DU, RW>::bytes(kChunk) > 48 * 1024 && first_use_on_device((const void*)kernel))
+        LB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnSmem<DU, RW>::bytes(kChunk)));
     s.tile_rows = std::min(kChunk, (std::max(streamed, 1) + 3) / 4 * 4);
-    launch_overlapped(kernel, dim3(blocks), dim3(kAttnRows * 32), AttnSmem<DU>::bytes(s.tile_rows), st, 0, args..., s);
+    launch_overlapped(kernel, dim3(blocks), dim3(kAttnWarps * 32), AttnSmem<DU, RW>::bytes(s.tile_rows), st, 0, args..., s);
+}
+// Two rows a warp fetch a streamed element for both (every bit the same): from 512 blocks of one row a warp on, which is where they win. us,
+// one row -> two, forward, backward: 4 x 8 heads x 256 x 64 float32 48.9 -> 43.5, 140 -> 118; 2 x 4 x 1000 x 32 111 -> 92, 288 -> 291; 2 x 8 x 300 x
+// 128 109 -> 104, 317 -> 270; 2 x 4 x 500 x 256 202 -> 166, 567 -> 492; bfloat16 16 x 704 x 64 of one batch entry 160 -> 138; but fewer blocks 8 x 4 x
+// 64 x 32 6.1 -> 6.3, 2 x 140 x 32 9.4 -> 11.0. Four rows: 0.68 - 1.6 of the time.
+bool two_rows(long long batch, long long heads, long long rows) { return batch * heads * ((rows + kAttnWarps - 1) / kAttnWarps) >= 512; }
+template <class F>
+void with_rows(bool two, F&& f) {
+    if (two) f(std::integral_constant<int, 2>());
+    else f(std::integral_constant<int, 1>());
 }
 // calls `f` with the head-dim elements per lane as a compile-time number: 1, 2, 4 or 8
 template <class F>
@@ -816,7 +922,10 @@ void with_dims_per_lane(int D, F&& f) {
 template <class T>
 void simt_fwd(const AttnShape& s, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o, float* lse, cudaStream_t st) {
     with_dims_per_lane(s.D, [&](auto du) {
-        launch_attn<du>(attention_simt_fwd_kernel<T, du>, attn_blocks(s.B, s.N, s.Sq), s.Sk, st, s, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr, (T*)o.ptr, lse);
+        with_rows(two_rows(s.B, s.N, s.Sq), [&](auto rw) {
+            launch_attn<du, rw>(attention_simt_fwd_kernel<T, du, rw>, attn_blocks(s.B, s.N, s.Sq, rw), s.Sk, st, s, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr,
+                                (T*)o.ptr, lse);
+        });
     });
 }
 template <class T>
@@ -825,10 +934,14 @@ void simt_bwd(const AttnShape& s, const lb_tensor& q, const lb_tensor& k, const 
     const long long warps = (long long)s.B * s.N * s.Sq;
     launch_overlapped(attention_delta_simt<T>, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256), 0, st, 0, (const T*)o.ptr, (const T*)g.ptr, delta, s);
     with_dims_per_lane(s.D, [&](auto du) {
-        launch_attn<du>(attention_simt_dq_kernel<T, du>, attn_blocks(s.B, s.N, s.Sq), s.Sk, st, s, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr,
-                        (const T*)g.ptr, lse, (const float*)delta, (T*)dq.ptr);
-        launch_attn<du>(attention_simt_dkdv_kernel<T, du>, attn_blocks(s.B, s.Nkv, s.Sk), s.Sq, st, s, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr,
-                        (const T*)g.ptr, lse, (const float*)delta, (T*)dk.ptr, (T*)dv.ptr);
+        with_rows(two_rows(s.B, s.N, s.Sq), [&](auto rw) {
+            launch_attn<du, rw>(attention_simt_dq_kernel<T, du, rw>, attn_blocks(s.B, s.N, s.Sq, rw), s.Sk, st, s, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr,
+                                (const T*)g.ptr, lse, (const float*)delta, (T*)dq.ptr);
+        });
+        with_rows(two_rows(s.B, s.Nkv, s.Sk), [&](auto rw) {
+            launch_attn<du, rw>(attention_simt_dkdv_kernel<T, du, rw>, attn_blocks(s.B, s.Nkv, s.Sk, rw), s.Sq, st, s, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr,
+                                (const T*)g.ptr, lse, (const float*)delta, (T*)dk.ptr, (T*)dv.ptr);
+        });
     });
 }
 }  // namespace
