@@ -208,6 +208,32 @@ def device_status() -> None:
     _lib.check(_lib.lib().lb_device_status())
 
 
+class _Torch:
+    """What calls on plain torch tensors take from torch, looked up once: the lookups on the way to `_empty_like_input`, `_workspace` and
+    `_stream` cost the host a microsecond a tensor, in front of kernels that take three."""
+
+    tensor = None  # torch.Tensor, once such a tensor has been met
+
+    @classmethod
+    def takes(cls, t, stream) -> bool:
+        """Whether `t` is a plain torch tensor and the call is for torch's current stream."""
+        if cls.tensor is None and type(t).__module__.startswith("torch"):
+            torch = sys.modules["torch"]
+            if not hasattr(torch._C, "_cuda_getCurrentRawStream"):
+                return False
+            cls.empty_like, cls.dense, cls.float32 = torch.empty_like, torch.contiguous_format, torch.float32
+            cls.raw_stream, cls.device, cls.tensor = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice, torch.Tensor
+        return type(t) is cls.tensor and stream is None and _current[0] == 0 and t.is_cuda
+
+    @classmethod
+    def like(cls, t):
+        return cls.empty_like(t, memory_format=cls.dense)
+
+    @classmethod
+    def stream(cls) -> int:
+        return cls.raw_stream(cls.device())
+
+
 def attention_forward(q, k, v, scale=None, causal=False, out=None, lse=None, stream=None):
     """Flash attention forward through `lb_attention_fwd`: `q` [B, Sq, N, H], `k`/`v` [B, Sk, Nkv, H] bfloat16 views;
     returns `(o, lse)` with `o` [B, Sq, N, H] bfloat16 and `lse` [B, N, Sq] float32. Bit-identical from call to call; the
@@ -216,11 +242,15 @@ def attention_forward(q, k, v, scale=None, causal=False, out=None, lse=None, str
     require_cuda()
     b, sq, n, h = q.shape
     sk = k.shape[1]
-    if out is None:
-        out = _empty_like_input(q, (b, sq, n, h), dtype_name(q.dtype))
-    if lse is None:
-        lse = _empty_like_input(q, (b, n, sq), "float32")
-    _lib.host().attention_fwd(float(scale if scale is not None else h**-0.5), bool(causal), sk - sq, q, k, v, out, lse, _stream(stream))
+    if out is None and lse is None and _Torch.takes(q, stream):
+        out, lse, handle = _Torch.like(q), q.new_empty((b, n, sq), dtype=_Torch.float32), _Torch.stream()
+    else:
+        if out is None:
+            out = _empty_like_input(q, tuple(q.shape), dtype_name(q.dtype))
+        if lse is None:
+            lse = _empty_like_input(q, (b, n, sq), "float32")
+        handle = _stream(stream)
+    _lib.host().attention_fwd(float(scale if scale is not None else h**-0.5), bool(causal), sk - sq, q, k, v, out, lse, handle)
     return out, lse
 
 
@@ -229,16 +259,23 @@ _KEPT_SCORES = 256 << 20
 
 def attention_backward(q, k, v, o, d_o, lse, scale=None, causal=False, delta=None, stream=None, deterministic=True):
     """Flash attention backward; returns `(dq, dk, dv)` shaped like `q`, `k`, `v`. `deterministic` (the default here)
-    runs `lb_attention_bwd`, the dK/dV + dQ kernel pair that is bit-identical from run to run; without it
+    runs `lb_attention_bwd_scratch`, the dK/dV + dQ kernel pair that is bit-identical from run to run; without it
     `lb_attention_bwd_atomic` runs the reference backend's default mode, one kernel adding dQ atomically into a float32
-    accumulator."""
+    accumulator, at head dim 64, and the same pair elsewhere."""
     require_cuda()
     b, sq, n, h = q.shape
     sk = k.shape[1]
-    dq, dk, dv = (_empty_like_input(t, tuple(t.shape), dtype_name(t.dtype)) for t in (q, k, v))
-    if delta is None:
-        delta = _workspace(q, (b, n, sq), "float32", stream)
-    dq_accum = None if deterministic else _workspace(q, (b, sq, n, h), "float32", stream)
+    plain = _Torch.takes(q, stream) and type(k) is type(v) is _Torch.tensor
+    if plain:
+        dq, dk, dv, handle = _Torch.like(q), _Torch.like(k), _Torch.like(v), _Torch.stream()
+        if delta is None:
+            delta = q.new_empty((b, n, sq), dtype=_Torch.float32)
+    else:
+        dq, dk, dv = (_empty_like_input(t, tuple(t.shape), dtype_name(t.dtype)) for t in (q, k, v))
+        if delta is None:
+            delta = _workspace(q, (b, n, sq), "float32", stream)
+        handle = _stream(stream)
+    dq_accum = _workspace(q, (b, sq, n, h), "float32", stream) if h == 64 and not deterministic else None
     scale, causal = float(scale if scale is not None else h**-0.5), bool(causal)
     scores, nbytes = None, _lib.host().attention_bwd_scratch_bytes(scale, causal, sk - sq, q, k) if h == 128 else 0
     if nbytes > _KEPT_SCORES and not type(q).__module__.startswith("torch"):
@@ -249,7 +286,7 @@ def attention_backward(q, k, v, o, d_o, lse, scale=None, causal=False, delta=Non
         except RuntimeError:  # no memory for it: it is not needed
             nbytes = 0
     _lib.host().attention_bwd(scale, causal, sk - sq, q, k, v, o, d_o, lse, delta, dq_accum, dq, dk, dv, scores.data_ptr() if nbytes else 0,
-                              nbytes, _stream(stream))
+                              nbytes, handle)
     return dq, dk, dv
 
 
