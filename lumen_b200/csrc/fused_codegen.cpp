@@ -644,13 +644,24 @@ class Generator {
             T_ = (int)threads_for(chunks);
             if (min_size == 2 && VEC_ >= 4 && C_ >= 1024 && (C_ <= 2048 || C_ > 3072 || R_ * C_ >= 1 << 21)) {
                 // Rows of 16 bits from 1024 columns on: two vectors of eight bytes a thread and as many blocks as 16 warps and more need, so
-                // that a block of 13 to 15 warps is not alone on its SM. us, the sums above, one vector of 16 bytes a thread -> so: 2048 x 1024
+                // that a block of 13 to 15 warps is not alone on its SM, 24 where every thread has both vectors whole and few sums to keep (84
+                // registers do: a layer norm's gradients 16384 x 1024 39.0 -> 32.0, 21845 x 1536 68 -> 61, 16384 x 2048 71 -> 60, the same at
+                // 2^22 elements 1.05 - 1.12, with four row sums 1.2, 512 threads 1.06, a last vector that some lack 1.03 - 1.1). us, the sums above, one vector of 16 bytes a thread -> so: 2048 x 1024
                 // 12.9 -> 11.0, 4096 x 2048 32.6 -> 31.8, 3640 x 2304 42 -> 35, 2532 x 3312 52 -> 45, 1677 x 5000 48 -> 41, 1024 x 8192 58 -> 45.
                 // Few rows of 2049 to 3072 columns, whose blocks would have nine to twelve warps, are left: 455 x 2304 9.9 against 10.5.
                 VEC_ = 4, nvec = vectors(), chunks = 2;
                 T_ = (int)threads_for(chunks);
                 if (T_ > 288 && T_ <= 384 && C_ % (T_ * 8) != 0) T_ = (int)threads_for(3);  // (the last chunk a part: 2600 wide as fast, few rows faster)
-                else warps = 16;
+                else warps = few_sums() && T_ <= 256 && C_ == T_ * VEC_ * 2 && R_ * C_ >= 1 << 23 ? 24 : 16;
+            } else if (min_size == 2 && VEC_ == 8 && C_ > 256 && C_ <= 768 && R_ * C_ > 1 << 21 && held_columns() <= 9 && (C_ < 768 || few_sums())) {
+                // Narrow rows of 16 bits: a warp to a row, so that row sums need no barrier between warps, two or three vectors of 16 bytes a
+                // thread. us, bfloat16, 2^22 to 2^25 elements, vectors a thread by the rule above -> so: a layer norm's gradients 31775 x 264
+                // 33.8 -> 23.6, 16384 x 512 20.8 -> 17.4, 13107 x 640 25.3 -> 23.3, 10922 x 768 20.1 -> 18.7; RMS norm with its gradients
+                // 16384 x 512 17.1 -> 11.7, 21845 x 768 36.7 -> 28.1; layer norm with its gradients (four sums) 31775 x 264 37.1 -> 25.2,
+                // 26214 x 640 47.9 -> 40.4, at 768 columns 0.85 - 1.04 and softmax with its gradient 0.94 - 1.13, so those keep the wider
+                // block. Left as they were: two million elements (0.9 - 1.13), 896 and 1000 columns in four vectors (0.82 - 1.4),
+                // and kernels that hold more for a column (five operands and three column sums: 0.71 - 1.26).
+                T_ = 32, warps = C_ <= 512 ? 16 : 12;
             } else if (min_size == 4 && VEC_ == 4 && nvec <= 1024 && R_ * C_ >= 1 << 21 && held_columns() <= 16 && (ones || col_reduces_.size() <= 4)) {
                 // float32 rows: one vector a thread where that makes a warp or four and more, 32 warps an SM; two where more threads fit so,
                 // or as many but not all 1024. us, two vectors and 16 warps -> so: 16384 x 512 44 -> 33, 8192 x 1024 46 -> 35, 5461 x 1536 58 -> 40,
@@ -729,6 +740,13 @@ class Generator {
             const int64_t elements = (nvec + T_ - 1) / T_ * VEC_;
             if (elements >= 16) per_sm_ = std::max(1, (elements > 16 ? 512 : 768) / (T_ * RPB_));
         }
+    }
+
+    // Whether a mixed kernel keeps little for a column and for a row
+    bool few_sums() const {
+        int sums = -(int)col_reduces_.size();
+        for (const Node& n : g_.nodes) sums += n.op == "reduce_sum" || n.op == "reduce_max";
+        return sums <= 2 && held_columns() <= 9;
     }
 
     // What a thread of a mixed kernel holds for each of its columns: a sum for each column total, the operands by column, and those over the
