@@ -742,12 +742,13 @@ class Generator {
         }
     }
 
-    // Whether a mixed kernel keeps little for a column and for a row
-    bool few_sums() const {
+    int row_sums() const {
         int sums = -(int)col_reduces_.size();
         for (const Node& n : g_.nodes) sums += n.op == "reduce_sum" || n.op == "reduce_max";
-        return sums <= 2 && held_columns() <= 9;
+        return sums;
     }
+    // Whether a mixed kernel keeps little for a column and for a row
+    bool few_sums() const { return row_sums() <= 2 && held_columns() <= 9; }
 
     // What a thread of a mixed kernel holds for each of its columns: a sum for each column total, the operands by column, and those over the
     // space twice (the row in flight and the one behind it)
@@ -1166,9 +1167,13 @@ class Generator {
     }
     // Whether a pair's elements are added by one packed instruction: float32 sums. Half the instructions, and a chain half as long. With packed
     // negations, one product for x * y and y * x, and what is said at divide_again, 58.5 -> 53.8 instructions an element and 28.2 -> 27.7 us for
-    // a layer norm of 8192 x 1024 bfloat16 with its gradients: chains of dependent instructions bound it more than their number.
+    // a layer norm of 8192 x 1024 bfloat16 with its gradients: chains of dependent instructions bound it more than their number. That kernel
+    // sums a row four times and its columns twice, and measures the same without packed sums: kernels that sum columns and, three times and
+    // more, rows keep a sum an element. 31 sizes from 8065 x 520 to 8192 x 2048, us, packed -> so: layer norm with its gradients 0.95 - 1.02 (21845 x 768
+    // 37.2 -> 35.6, 5461 x 1536 20.2 -> 19.6), softmax with its gradient 0.97 - 1.01 (16384 x 1024 32.4 -> 31.7), but RMS norm, which
+    // sums a row twice, 0.99 - 1.03.
     bool adds_pairs(const std::string& combine, const std::string& val) const {
-        return pair_ && !shifted_ && combine == "rnd_f32(__fadd_rn(%A, %B))" && packable(val, LB_F32);
+        return pair_ && !shifted_ && !(mixed_ && row_sums() > 2) && combine == "rnd_f32(__fadd_rn(%A, %B))" && packable(val, LB_F32);
     }
     // the statement(s) folding element e (and e + 1) of `val` into `acc`
     std::string accumulate(const std::string& acc, const std::string& combine, const std::string& val) {
