@@ -709,12 +709,12 @@ CUtensorMap make_map(const View3& v, bool contiguous_is_cols, int box_inner, int
 
 }  // namespace
 
-// Number of K ranges for a GEMM with few output tiles and a long K (weight gradients). 1 = no split. A cost model
-// picks it: waves of (tile, range) units times the k-blocks of a range, at the measured 4 x 171 cycles per k-block of
-// a 128 x 256 tile, plus the float32 partial tiles written by the GEMM and re-read by the reduction kernel at HBM
-// speed and that kernel's launch. A split has to win by a tenth to be taken; each range keeps at least 16 k-blocks.
+// Number of K ranges for a GEMM with few output tiles and a long K (weight gradients), with one CTA to a 128 x 256 tile. 1 = no split. A cost
+// model picks it: waves of (tile, range) units times the k-blocks of a range, at the measured 4 x 171 cycles per k-block, plus the float32
+// partial tiles written by the GEMM and re-read by the reduction kernel at HBM speed and that kernel's launch. A split has to win by a tenth
+// to be taken; each range keeps at least 16 k-blocks.
 size_t gemm_scratch_bytes(long long M, long long N, long long K, long long batch);
-int gemm_splits(long long M, long long N, long long K, long long batch, int sms) {
+static int gemm_tile_splits(long long M, long long N, long long K, long long batch, int sms) {
     const long long tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * batch, total_kb = (K + BK - 1) / BK;
     if (tiles >= 4LL * sms || total_kb < 32) return 1;
     const double us_per_kb = 0.36, bytes_per_us = 5.0e6, launch_us = 6.0;
@@ -723,6 +723,29 @@ int gemm_splits(long long M, long long N, long long K, long long batch, int sms)
         double us = (double)waves * (double)kb * us_per_kb;
         if (s > 1) us += ((2.0 * s * 4 + 2) * (double)(batch * M * N)) / bytes_per_us + launch_us;
         return us;
+    };
+    int best = 1;
+    double best_us = cost(1) * 0.9;
+    for (int s = 2; s <= 32 && total_kb / s >= 16; s++)
+        if (cost(s) < best_us) best = s, best_us = cost(s);
+    return best;
+}
+
+// The same for what runs: CTA pairs take 256 x 256 tiles of more than 128 rows. us: 3 a product, 0.3 a k-block and 2 a unit of each wave, 0.1 a
+// k-block shared by all pairs (the L2's part and the power's), 3.5 for the reduction and, a million elements of the result, 0.45 a range and 0.6:
+// a fit to 714 shapes of 129 to 9000 rows and columns and K of 500 to 30000 under 1 to 8 ranges (half of them within 6 %). Against the
+// model above, on those and 404 other shapes: 55 are cut otherwise and take 0.69 - 1.08 of the time, 0.84 in the mean, three of them more than
+// 1.03; 1500 x 1024 K 4096 24.2 -> 18.4, 1530 x 1536 K 6144 0.83, 768 x 3072 K 4096 26.4 -> 23.4, 357 x 4096 K 4096 0.86. Which products stay on narrow
+// tiles is left to the model above, which that line was measured with.
+int gemm_splits(long long M, long long N, long long K, long long batch, int sms) {
+    if (M <= BM) return gemm_tile_splits(M, N, K, batch, sms);
+    const int pairs = sms / 2;
+    const long long tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) * batch, total_kb = (K + BK - 1) / BK;
+    if (tiles >= 4LL * pairs || total_kb < 32) return 1;
+    const double millions = (double)(batch * M * N) * 1e-6;
+    auto cost = [&](int s) {
+        const double kb = (double)((total_kb + s - 1) / s), waves = (double)((tiles * s + pairs - 1) / pairs);
+        return 3.0 + waves * (0.3 * kb + 2.0) + 0.1 * kb * (double)(tiles * s) / pairs + (s > 1 ? 3.5 + millions * (0.45 * s + 0.6) : 0.0);
     };
     int best = 1;
     double best_us = cost(1) * 0.9;
@@ -794,7 +817,7 @@ size_t gemm_scratch_bytes(long long M, long long N, long long K, long long batch
 // Scratch a plan's product step takes: none where the narrow tiles run.
 static size_t gemm_step_scratch_bytes(long long M, long long N, long long K, long long batch) {
     const int sms = sm_count_hint(), split = gemm_splits(M, N, K, batch, sms);
-    return gemm_small_splits(M, N, K, batch, sms, split) ? 0 : gemm_scratch_bytes(M, N, K, batch);
+    return gemm_small_splits(M, N, K, batch, sms, split > 1 ? gemm_tile_splits(M, N, K, batch, sms) : 1) ? 0 : gemm_scratch_bytes(M, N, K, batch);
 }
 
 // Where a product of 16-bit operands runs: on narrow tiles with `ranges` CTAs a cluster, or (ranges 0) on large tiles with K cut into
@@ -803,12 +826,14 @@ struct GemmRoute {
     int ranges, splits, kb_per_split;
 };
 static GemmRoute gemm_route(long long M, long long N, long long K, long long batch, int sms, int kernel_choice, size_t scratch_bytes, const GemmTuning* tuning) {
-    const int split = scratch_bytes ? gemm_splits(M, N, K, batch, sms) : 1;
+    const int model = scratch_bytes ? gemm_splits(M, N, K, batch, sms) : 1;
     auto holds = [&](int s) { return s > 1 && scratch_bytes >= (size_t)s * batch * M * N * 4; };
     // no kernel asked for and no split or raster tuned: narrow tiles where they fit
     if (kernel_choice == 0 && !(tuning && (tuning->splits > 0 || tuning->group_m > 0)))
-        if (const int ranges = gemm_small_splits(M, N, K, batch, sms, holds(split) ? split : 1)) return {ranges, 1, 0};
-    const int want = tuning && tuning->splits > 0 ? tuning->splits : split;  // a tuned split count, if the scratch holds it
+        if (const int ranges = gemm_small_splits(M, N, K, batch, sms, holds(model) ? gemm_tile_splits(M, N, K, batch, sms) : 1)) return {ranges, 1, 0};
+    // no more ranges than the scratch holds (a saved plan's is what another model asked for), or as many as were tuned if it holds those
+    const int split = (int)std::min<size_t>(model, scratch_bytes / ((size_t)batch * M * N * 4));
+    const int want = tuning && tuning->splits > 0 ? tuning->splits : split;
     const int total_kb = (int)((K + BK - 1) / BK), kb = holds(want) ? (total_kb + want - 1) / want : total_kb;
     return {0, (total_kb + kb - 1) / kb, kb};
 }
