@@ -529,6 +529,7 @@ class Generator {
     std::set<int> behind_columns_;
     std::vector<int> column_outputs_;
     int resident_ = 1;  // CTAs per SM a kernel with column sums is built for and launched with
+    bool sixteen_warps_ = false;  // no kernel with column sums has more on an SM (and more slices), as before some had
     bool shifts_ = true, shifted_ = false;  // may start, starts a row's chunks at aligned addresses before its first element
     bool narrow_ = false;                   // 16-bit tensors
     int period_ = 1;                        // ... rows that far apart at the same distance
@@ -652,7 +653,7 @@ class Generator {
                 VEC_ = 4, nvec = vectors(), chunks = 2;
                 T_ = (int)threads_for(chunks);
                 if (T_ > 288 && T_ <= 384 && C_ % (T_ * 8) != 0) T_ = (int)threads_for(3);  // (the last chunk a part: 2600 wide as fast, few rows faster)
-                else warps = few_sums() && T_ <= 256 && C_ == T_ * VEC_ * 2 && R_ * C_ >= 1 << 23 ? 24 : 16;
+                else warps = !sixteen_warps_ && few_sums() && T_ <= 256 && C_ == T_ * VEC_ * 2 && R_ * C_ >= 1 << 23 ? 24 : 16;
             } else if (min_size == 2 && VEC_ == 8 && C_ > 256 && C_ <= 768 && R_ * C_ > 1 << 21 && held_columns() <= 9 && (C_ < 768 || few_sums())) {
                 // Narrow rows of 16 bits: a warp to a row, so that row sums need no barrier between warps, two or three vectors of 16 bytes a
                 // thread. us, bfloat16, 2^22 to 2^25 elements, vectors a thread by the rule above -> so: a layer norm's gradients 31775 x 264
@@ -2114,6 +2115,7 @@ class Generator {
     void set_multi(bool v) { multi_ = v; }
     void set_mixed(bool v) { mixed_ = v; }
     void set_shifts(bool v) { shifts_ = v; }
+    void set_sixteen_warps(bool v) { sixteen_warps_ = v; }
 
 };
 
@@ -2127,6 +2129,7 @@ static FusedKernel generate(const Module& module, bool shifts) {
     Generator gen(module, g);
     gen.set_inplace(module.options.count("inplace") != 0);
     gen.set_multi(module.options.count("multi") != 0);
+    gen.set_sixteen_warps(module.options.count("sixteen_warps") != 0);
     if (module.options.count("multi") && (reduces || Generator::wants_columns(g)))
         fail(LB_ERR_UNSUPPORTED, "option multi: a horizontally fused kernel cannot hold a reduction");
     if (Generator::wants_columns(g) && !Generator::leaves_rows(g)) return gen.run_columns();

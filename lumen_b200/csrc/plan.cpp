@@ -118,6 +118,7 @@ size_t view_bytes(const lb_tensor& t) {
 std::unique_ptr<lb_plan> parse_plan(const std::string& text) {
     auto plan = std::make_unique<lb_plan>();
     std::vector<lb_fusion*> modules;
+    std::vector<std::string> module_texts;
     std::istringstream lines(text);
     std::string line, module_text;
     bool in_module = false, seen_plan = false, ended = false;
@@ -126,7 +127,7 @@ std::unique_ptr<lb_plan> parse_plan(const std::string& text) {
     while (std::getline(lines, line)) {
         if (in_module) {
             if (line == "endmodule") {
-                modules.push_back(compile_fusion(module_text));
+                modules.push_back(compile_fusion(module_text)), module_texts.push_back(module_text);
                 in_module = false;
             } else {
                 module_text += line + "\n";
@@ -179,8 +180,10 @@ std::unique_ptr<lb_plan> parse_plan(const std::string& text) {
                 s.scratch = std::stoi(tok.at(4));
                 ints(6, std::stoul(tok.at(5)));
                 if (s.fusion->scratch_bytes && s.scratch < 0) fail(LB_ERR_INVALID, "plan: fusion " + s.label + " needs scratch");
-                // (a text written by a library whose kernels cut the same module into fewer slices)
-                if (s.scratch >= 0 && (s.scratch >= (int)plan->views.size() || view_bytes(plan->views[s.scratch].t) < s.fusion->scratch_bytes))
+                // (a text written by a library whose kernels cut the same module into fewer slices: those of at most sixteen warps an SM still can)
+                auto too_little = [&] { return s.scratch >= 0 && (s.scratch >= (int)plan->views.size() || view_bytes(plan->views[s.scratch].t) < s.fusion->scratch_bytes); };
+                if (too_little()) s.fusion = compile_fusion("option sixteen_warps\n" + module_texts[m]);
+                if (too_little())
                     fail(LB_ERR_INVALID, "plan: the scratch of fusion " + s.label + " is smaller than its kernel needs: lower the module again");
             } else if (kind == "multi") {  // s multi <label> <module> <n_groups> <tensor ids, group after group>
                 s.kind = MULTI;
