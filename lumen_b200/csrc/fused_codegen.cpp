@@ -647,8 +647,9 @@ class Generator {
                 // Rows of 16 bits from 1024 columns on: two vectors of eight bytes a thread and as many blocks as 16 warps and more need, so
                 // that a block of 13 to 15 warps is not alone on its SM, 24 where every thread has both vectors whole and few sums to keep (84
                 // registers do: a layer norm's gradients 16384 x 1024 39.0 -> 32.0, 21845 x 1536 68 -> 61, 16384 x 2048 71 -> 60, the same at
-                // 2^22 elements 1.05 - 1.12, with four row sums 1.2, 512 threads 1.06, a last vector that some lack 1.03 - 1.1). us, the sums above, one vector of 16 bytes a thread -> so: 2048 x 1024
-                // 12.9 -> 11.0, 4096 x 2048 32.6 -> 31.8, 3640 x 2304 42 -> 35, 2532 x 3312 52 -> 45, 1677 x 5000 48 -> 41, 1024 x 8192 58 -> 45.
+                // 2^22 elements 1.05 - 1.12, with four row sums 1.2, 512 threads 1.06, a last vector that some lack 1.03 - 1.1). us, the sums
+                // above, one vector of 16 bytes a thread -> so: 2048 x 1024 12.9 -> 11.0, 4096 x 2048 32.6 -> 31.8, 3640 x 2304 42 -> 35,
+                // 2532 x 3312 52 -> 45, 1677 x 5000 48 -> 41, 1024 x 8192 58 -> 45.
                 // Few rows of 2049 to 3072 columns, whose blocks would have nine to twelve warps, are left: 455 x 2304 9.9 against 10.5.
                 VEC_ = 4, nvec = vectors(), chunks = 2;
                 T_ = (int)threads_for(chunks);
