@@ -529,7 +529,7 @@ class Generator {
     std::set<int> behind_columns_;
     std::vector<int> column_outputs_;
     int resident_ = 1;  // CTAs per SM a kernel with column sums is built for and launched with
-    bool sixteen_warps_ = false;  // no kernel with column sums has more on an SM (and more slices), as before some had
+    bool sixteen_warps_ = false;  // no kernel of row and column sums has more on an SM, and more slices than it once had
     bool shifts_ = true, shifted_ = false;  // may start, starts a row's chunks at aligned addresses before its first element
     bool narrow_ = false;                   // 16-bit tensors
     int period_ = 1;                        // ... rows that far apart at the same distance
@@ -655,15 +655,22 @@ class Generator {
                 T_ = (int)threads_for(chunks);
                 if (T_ > 288 && T_ <= 384 && C_ % (T_ * 8) != 0) T_ = (int)threads_for(3);  // (the last chunk a part: 2600 wide as fast, few rows faster)
                 else warps = !sixteen_warps_ && few_sums() && T_ <= 256 && C_ == T_ * VEC_ * 2 && R_ * C_ >= 1 << 23 ? 24 : 16;
-            } else if (min_size == 2 && VEC_ == 8 && C_ > 256 && C_ <= 768 && R_ * C_ > 1 << 21 && held_columns() <= 9 && (C_ < 768 || few_sums())) {
-                // Narrow rows of 16 bits: a warp to a row, so that row sums need no barrier between warps, two or three vectors of 16 bytes a
-                // thread. us, bfloat16, 2^22 to 2^25 elements, vectors a thread by the rule above -> so: a layer norm's gradients 31775 x 264
-                // 33.8 -> 23.6, 16384 x 512 20.8 -> 17.4, 13107 x 640 25.3 -> 23.3, 10922 x 768 20.1 -> 18.7; RMS norm with its gradients
-                // 16384 x 512 17.1 -> 11.7, 21845 x 768 36.7 -> 28.1; layer norm with its gradients (four sums) 31775 x 264 37.1 -> 25.2,
-                // 26214 x 640 47.9 -> 40.4, at 768 columns 0.85 - 1.04 and softmax with its gradient 0.94 - 1.13, so those keep the wider
-                // block. Left as they were: two million elements (0.9 - 1.13), 896 and 1000 columns in four vectors (0.82 - 1.4),
-                // and kernels that hold more for a column (five operands and three column sums: 0.71 - 1.26).
-                T_ = 32, warps = C_ <= 512 ? 16 : 12;
+            } else if (min_size == 2 && VEC_ == 8 && C_ > 256 && C_ < 1024 && R_ * C_ >= 1 << 20 && !sixteen_warps_) {
+                // Rows of 264 to 1016 columns of 16 bits. Up to 384 columns a warp to a row, so that row sums need no barrier between warps, with three
+                // vectors of eight bytes a thread and 20 warps an SM; from there two of them a thread and 24 warps, but a warp to a row with two
+                // or three vectors of 16 bytes where threads hold little (at 768 columns: have few row sums) from 2^21 elements on, beyond 512
+                // columns up to 2^23: there the others take 0.92 - 1.24 of its time, at more elements 0.79 - 1.07. Times a vector of 16 bytes a thread
+                // and 16 warps, gradients of a layer norm, layer and RMS norm and softmax with theirs, softmax with column sums, five operands
+                // with three column sums, 2^20 to 2^25 elements: 0.39 - 0.98 up to 384 columns, 0.61 - 0.97 up to 768, 0.52 - 1.08 beyond (1.08:
+                // 6 us), float16 0.38 - 1.02. us, bfloat16: RMS norm with its gradients 16384 x 512 17.1 -> 11.7, 63550 x 264 47.8 -> 30.3, 18724 x 896
+                // 33.7 -> 29.6, layer norm with its gradients 26214 x 640 47.9 -> 35.0, 4128 x 1016 16.9 -> 12.5, softmax with its gradient
+                // 43690 x 384 67.9 -> 26.3.
+                if (C_ > 384 && C_ <= 768 && R_ * C_ > 1 << 21 && (C_ <= 512 || C_ == 768 || R_ * C_ < 1 << 23) && held_columns() <= 9 && (C_ < 768 || few_sums())) {
+                    T_ = 32, warps = C_ <= 512 ? 16 : 12;
+                } else {
+                    VEC_ = 4, nvec = vectors(), chunks = C_ <= 384 ? 3 : 2;
+                    T_ = (int)threads_for(chunks), warps = C_ <= 384 ? 20 : 24;
+                }
             } else if (min_size == 4 && VEC_ == 4 && nvec <= 1024 && R_ * C_ >= 1 << 21 && held_columns() <= 16 && (ones || col_reduces_.size() <= 4)) {
                 // float32 rows: one vector a thread where that makes a warp or four and more, 32 warps an SM; two where more threads fit so,
                 // or as many but not all 1024. us, two vectors and 16 warps -> so: 16384 x 512 44 -> 33, 8192 x 1024 46 -> 35, 5461 x 1536 58 -> 40,

@@ -10,6 +10,7 @@ from lumen_b200 import prims
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(8192, 256), (7944, 264), (7945, 264), (5001, 504), (4096, 512), (4097, 512), (8200, 512), (4035, 520), (3001, 760), (2732, 768),
+          (3971, 264), (3972, 264), (63550, 264), (5462, 384), (5400, 392), (2048, 512), (1638, 640), (16200, 640), (11000, 768), (1352, 776), (4200, 1000), (1033, 1016),
           (8191, 1024), (8192, 1024), (9001, 1024), (5462, 1536), (4096, 2048), (4097, 2048), (8193, 1028)]
 
 
