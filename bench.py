@@ -576,7 +576,8 @@ def secondary_measurements(device, peaks, steps=6, warmup=3):
         out[w.name] = {"value": total, "unit": "TFLOP/s", "ms": w.fwd_ms + w.bwd_ms, "frac": total / peaks["bf16_tflops"],
                        "peak": peaks["bf16_tflops"], "forward": {"value": fwd, "ms": w.fwd_ms, "frac": fwd / peaks["bf16_tflops"]},
                        "backward": {"value": bwd, "ms": w.bwd_ms, "frac": bwd / peaks["bf16_tflops"]},
-                       "kernels": "attention_fwd_kernel, attention_delta, attention_bwd_kernel x2"}
+                       "kernels": "attention_fwd_kernel, attention_delta, "
+                                  + ("attention_bwd_kernel, attention_dq_kernel" if shape[3] == 128 else "attention_bwd_kernel x2")}
         del w
         torch.cuda.empty_cache()
     return out
