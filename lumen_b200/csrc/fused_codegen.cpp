@@ -665,6 +665,7 @@ class Generator {
                 // 6 us), float16 0.38 - 1.02. us, bfloat16: RMS norm with its gradients 16384 x 512 17.1 -> 11.7, 63550 x 264 47.8 -> 30.3, 18724 x 896
                 // 33.7 -> 29.6, layer norm with its gradients 26214 x 640 47.9 -> 35.0, 4128 x 1016 16.9 -> 12.5, softmax with its gradient
                 // 43690 x 384 67.9 -> 26.3.
+                chain_ = VEC_;
                 if (C_ > 384 && C_ <= 768 && R_ * C_ > 1 << 21 && (C_ <= 512 || C_ == 768 || R_ * C_ < 1 << 23) && held_columns() <= 9 && (C_ < 768 || few_sums())) {
                     T_ = 32, warps = C_ <= 512 ? 16 : 12;
                 } else {
@@ -740,6 +741,7 @@ class Generator {
         for (int v : g_.inputs) columns |= g_.type(v).numel() == C_ && R_ > 1;
         const bool norm = written && behind == 1 && columns, summed = !written && sums > 1;
         const int64_t eleven = (nvec * 3 / 32 + 31) / 32 * 32, four = (nvec + 127) / 128 * 32;
+        const int former = T_;
         if (T_ >= 512 && narrow_) {
             if (norm && eleven <= 1024) T_ = (int)eleven, per_sm_ = std::max(1, 1024 / T_);
             else if (summed && eleven <= 512) T_ = (int)eleven, per_sm_ = (T_ > 256 ? 1536 : 1024) / T_;
@@ -749,6 +751,7 @@ class Generator {
             const int64_t elements = (nvec + T_ - 1) / T_ * VEC_;
             if (elements >= 16) per_sm_ = std::max(1, (elements > 16 ? 512 : 768) / (T_ * RPB_));
         }
+        if (T_ < former) chain_ = (int)std::max<int64_t>(VEC_, nvec * VEC_ / former);
     }
 
     int row_sums() const {
@@ -1583,8 +1586,10 @@ class Generator {
             }
         }
         std::string val = gen(n.inputs[0], src, ph);
-        ph.sums = adds_pairs(ph.combine_a_b, val) ? 2 : sums();
-        ph.body += accumulate(ph.acc + (ph.sums == 1 ? "" : shifted_ ? "[e]" : ph.sums == 2 ? "[e & 1]" : "[ch & 3]"), ph.combine_a_b, val);
+        const bool pairs = adds_pairs(ph.combine_a_b, val);
+        ph.sums = std::max(sums(sum && flt), pairs ? 2 : 1);
+        const std::string which = shifted_ ? "e" : VEC_ > 2 || ph.sums == 2 ? format("e & %d", ph.sums - 1) : pairs ? "(ch & 1) * 2 + (e & 1)" : "ch & 3";
+        ph.body += accumulate(ph.sums == 1 ? ph.acc : ph.acc + "[" + which + "]", ph.combine_a_b, val);
         row_decls_ += format("%s %s;\n", ct.compute, ph.result.c_str());
         phases_.push_back(ph);
         reduce_memo_[key] = ph.result;
@@ -1595,7 +1600,16 @@ class Generator {
     // four, had 1.35 times the error of a float32 sum over 3001. Shifted chunks, whose threads have as many elements, keep one a lane: which
     // elements those are follows from the row's distance to an aligned address, so that equal rows at different places (modulo eight), or of a
     // tensor that is not aligned, may differ in the last bits of a sum. The same call gives the same bits.
-    int sums() const { return shifted_ ? VEC_ : VEC_ <= 2 && NCH_ > 4 ? 4 : 1; }
+    // Where fewer threads walk a row than its sums were once dealt to, a thread's elements are dealt to as many sums as keep each no longer than
+    // those threads' were in the mean (chain_): 88 elements of a float16 row of 8200 in one chain had 1.6 times the error of 16.
+    int chain_ = 0;
+    int sums(bool adds) const {
+        if (shifted_) return VEC_;
+        if (VEC_ <= 2) return NCH_ > 4 ? 4 : 1;
+        int n = 1;
+        while (adds && chain_ && n < VEC_ && NCH_ * VEC_ > n * chain_) n *= 2;
+        return n;
+    }
 
     // ---- emission ---------------------------------------------------------------------------------------
     std::string indent(const std::string& code, int n) {
