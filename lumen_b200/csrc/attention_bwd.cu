@@ -769,9 +769,15 @@ static lb_tensor any_unit_strides(lb_tensor t) {
 void attention_backward(const lb_attn_desc& desc, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o,
                         const lb_tensor& d_o, const lb_tensor& lse, const lb_tensor& delta, const lb_tensor& dq, const lb_tensor& dk,
                         const lb_tensor& dv, void* stream, const lb_tensor* dq_acc, void* scratch, size_t scratch_bytes) {
+    auto on_tensor_cores = [&](const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o, const lb_tensor& g) {
+        return attention_on_tensor_cores(q, k, v) && attention_on_tensor_cores(g, k, v) && attention_on_tensor_cores(o, k, v) && q.shape[1] > 0 && k.shape[1] > 0;
+    };
     const lb_tensor tq = any_unit_strides(q), tk = any_unit_strides(k), tv = any_unit_strides(v), to = any_unit_strides(o), tg = any_unit_strides(d_o);
-    if (attention_on_tensor_cores(tq, tk, tv) && attention_on_tensor_cores(tg, tk, tv) && attention_on_tensor_cores(to, tk, tv) && q.shape[1] > 0 &&
-        k.shape[1] > 0)
+    if (on_tensor_cores(q, k, v, o, d_o))
+        attention_bwd(desc, q, k, v, o, d_o, lse, delta, dq, dk, dv, stream, dq_acc, scratch, scratch_bytes);
+    // (what attention_bwd refuses stays on the CUDA cores with such strides: scales that are not positive, accumulators that are not aligned,
+    // more entries or heads than a grid's second and third axes take)
+    else if (desc.scale > 0.0f && (!dq_acc || ((uintptr_t)dq_acc->ptr & 15) == 0) && tq.shape[0] <= 65535 && tq.shape[2] <= 65535 && on_tensor_cores(tq, tk, tv, to, tg))
         attention_bwd(desc, tq, tk, tv, to, tg, lse, delta, any_unit_strides(dq), any_unit_strides(dk), any_unit_strides(dv), stream, dq_acc, scratch, scratch_bytes);
     else
         attention_simt_bwd(desc, q, k, v, o, d_o, lse, delta, dq, dk, dv, stream);
