@@ -76,13 +76,18 @@ struct BwdArgs {
     void* out_b;         // dV (dkdv mode)
     long long b_sb, b_ss, b_sn;
     int batch0, head0;   // the launch's first batch entry and first head (kv head in dkdv mode)
-    uint8_t* scores;     // dkdv mode, head dim 128: where dS is left for attention_dq, or null
+    uint8_t* scores;     // with kHands: where dS is left for attention_dq
     DsLayout ds;
     int* status;
 };
 
-template <int D, bool DKDV, int BT>
+// TILE: the streamed rows of a tile, BT, and kHands where dK/dV mode leaves dS. Chosen at run time, the 32 registers and the stores of dS cost
+// the kernel of plans and of calls without scratch up to 7 % (the whole backward, us, 4 x 32 heads on 8 x 512 69.7 -> 74.8, 1 x 8 x 8192 404 ->
+// 431, 8 x 32 x 4096 3234 -> 3285).
+constexpr int kHands = 1;
+template <int D, bool DKDV, int TILE>
 struct BwdConfig {
+    static constexpr int BT = TILE & ~kHands;
     static constexpr int kCtas = D == 64 ? 2 : 1;        // per SM
     static constexpr int kFirst = BT == 64 ? 2 : 4;      // first compute warp (register budgets are set per aligned group of four warps)
     static constexpr int kThreads = 32 * kFirst + 256;
@@ -99,12 +104,14 @@ struct BwdConfig {
     static_assert(2 * BT + 2 * D <= kTmemCols && (2 * (S1 + S2) + 9) * 8 + 8 <= 256, "tensor memory / barrier space");
 };
 
-template <int D, bool DKDV, int BT>
-__global__ void __launch_bounds__(BwdConfig<D, DKDV, BT>::kThreads, BwdConfig<D, DKDV, BT>::kCtas)
+template <int D, bool DKDV, int TILE>
+__global__ void __launch_bounds__(BwdConfig<D, DKDV, TILE>::kThreads, BwdConfig<D, DKDV, TILE>::kCtas)
 attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_constant__ CUtensorMap map_r2,
                      const __grid_constant__ CUtensorMap map_t1, const __grid_constant__ CUtensorMap map_t2, const BwdArgs p) {
-    using C = BwdConfig<D, DKDV, BT>;
-    constexpr int kResident = C::kResident, kStream = C::kStream, S1 = C::S1, S2 = C::S2, kTmemCols = C::kTmemCols, COLS = C::kCols;
+    using C = BwdConfig<D, DKDV, TILE>;
+    constexpr bool HANDS = (TILE & kHands) != 0;
+    static_assert(!HANDS || (D == 128 && DKDV && C::BT == 128), "what attention_dq reads");
+    constexpr int BT = C::BT, kResident = C::kResident, kStream = C::kStream, S1 = C::S1, S2 = C::S2, kTmemCols = C::kTmemCols, COLS = C::kCols;
     constexpr int kRBlock = BR * 128, kTBlock = BT * 128;  // bytes of one 64-wide head-dim block of a tile
     constexpr int DB = D / 64;
     extern __shared__ uint8_t smem_raw[];
@@ -135,7 +142,6 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform for the compiler too
     const int tile = DKDV ? (int)blockIdx.x : (int)(gridDim.x - 1 - blockIdx.x);
     const int head = p.head0 + (int)blockIdx.y, batch = p.batch0 + (int)blockIdx.z;  // kv head in dkdv mode, query head in dq mode
-    constexpr bool kHands = D == 128 && DKDV && BT == 128;  // may leave dS
     const int group = p.N / p.Nkv;
     const int r0 = tile * BR;
 
@@ -331,14 +337,12 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
         };
         if (DKDV && n_iter > 0) fetch_stats(0);
         uint8_t* scores = nullptr;  // dS of this thread's key and its warpgroup's first block of queries
-        if constexpr (kHands) {
-            if (p.scores)
-                scores = p.scores + ((long long)blockIdx.z * gridDim.y + blockIdx.y) * group * p.ds.head_bytes() + p.ds.at(tile, row_in_tile / 64, stream0 / 64) +
-                         wg * kDsHalfBytes + row_in_tile % 64 * 16;
-        }
+        if constexpr (HANDS)
+            scores = p.scores + ((long long)blockIdx.z * gridDim.y + blockIdx.y) * group * p.ds.head_bytes() + p.ds.at(tile, row_in_tile / 64, stream0 / 64) +
+                     wg * kDsHalfBytes + row_in_tile % 64 * 16;
         // A tile's dS leaves between the next one's exponentials, a store for every eight of them: in a row, right behind the hand-over of P and
         // Z, the stores hold up those (the backward of 1 x 8 heads x 4096 157 -> 135 us, of 8 x 32 x 4096 2990 -> 2900).
-        uint32_t left[kHands ? COLS / 2 : 1];
+        uint32_t left[HANDS ? COLS / 2 : 1];
         uint8_t* left_to = nullptr;
         auto leave = [&](int c) { *(uint4*)(left_to + c * 1024) = make_uint4(left[4 * c], left[4 * c + 1], left[4 * c + 2], left[4 * c + 3]); };
         float* stat_lse = col_stats + (warp - C::kFirst) * 2 * COLS;
@@ -366,7 +370,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
             if (DKDV) {
                 col_lo = p.causal ? row - p.causal_offset : 0;
                 col_hi = p.Sq;
-                if (kHands && scores && row >= p.Sk) col_hi = 0;  // what is left for these is multiplied by zeros and must be finite
+                if (HANDS && row >= p.Sk) col_hi = 0;  // what is left for these is multiplied by zeros and must be finite
             } else {
                 col_lo = 0;
                 col_hi = p.causal ? min((long long)p.Sk, row + p.causal_offset + 1) : (long long)p.Sk;
@@ -395,7 +399,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
                     const float2 u = __ffma2_rn(make_float2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])), s2, make_float2(l4.x, l4.y));
                     const float2 v = __ffma2_rn(make_float2(__uint_as_float(x[i + 2]), __uint_as_float(x[i + 3])), s2, make_float2(l4.z, l4.w));
                     pr[i] = fast_exp2(u.x), pr[i + 1] = fast_exp2(u.y), pr[i + 2] = fast_exp2(v.x), pr[i + 3] = fast_exp2(v.y);
-                    if (kHands && scores && it > 0 && i % 8 == 4) leave(i / 8);
+                    if (HANDS && it > 0 && i % 8 == 4) leave(i / 8);
                 }
                 if (masked_tile) {
 #pragma unroll
@@ -447,16 +451,16 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_r1, const __grid_co
             tmem_st_wait();
             tc_fence_before();
             mbar_arrive(pz_ready);
-            if constexpr (kHands) {
+            if constexpr (HANDS) {
                 left_to = scores + hh * p.ds.head_bytes() + (long long)(it - hh * per_head) * (2 * kDsHalfBytes);
 #pragma unroll
                 for (int c = 0; c < COLS / 2; c++) left[c] = pz[kZ + c];
             }
         }
-        if constexpr (kHands)
-            if (scores && n_iter > 0 && ok)
+        if (HANDS && n_iter > 0 && ok) {
 #pragma unroll
-                for (int c = 0; c < 8; c++) leave(c);
+            for (int c = 0; c < 8; c++) leave(c);
+        }
         // ---- epilogue: accumulators -> bf16 rows ----
         if (n_iter > 0) ok = ok && mbar_wait(acc_full, 0, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
@@ -587,13 +591,13 @@ void launch_delta(const lb_tensor& o, const lb_tensor& d_o, float* delta, float*
                       (int)S, (int)N, (int)D, n_shift, o.stride[0], o.stride[1], o.stride[2], d_o.stride[0], d_o.stride[1], d_o.stride[2]);
 }
 
-template <int D, bool DKDV, int BT>
+template <int D, bool DKDV, int TILE>
 void launch_bwd_kernel(const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap& t1, const CUtensorMap& t2, dim3 grid, const BwdArgs& p,
                        cudaStream_t s) {
-    using C = BwdConfig<D, DKDV, BT>;
-    if (first_use_on_device((const void*)attention_bwd_kernel<D, DKDV, BT>))
-        LB_CUDA(cudaFuncSetAttribute(attention_bwd_kernel<D, DKDV, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kBytes));
-    launch_overlapped(attention_bwd_kernel<D, DKDV, BT>, grid, dim3(C::kThreads), C::kBytes, s, 0, r1, r2, t1, t2, p);
+    using C = BwdConfig<D, DKDV, TILE>;
+    if (first_use_on_device((const void*)attention_bwd_kernel<D, DKDV, TILE>))
+        LB_CUDA(cudaFuncSetAttribute(attention_bwd_kernel<D, DKDV, TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kBytes));
+    launch_overlapped(attention_bwd_kernel<D, DKDV, TILE>, grid, dim3(C::kThreads), C::kBytes, s, 0, r1, r2, t1, t2, p);
 }
 
 // Of the dS that is left in memory at a time, and the fewest dK/dV CTAs of each of several rounds, whose ends leave SMs idle: batch 8, 32
@@ -647,8 +651,9 @@ void launch_bwd_pair(const Rows& rows, const lb_tensor& q, const lb_tensor& d_o,
     if constexpr (D == 128) {
         static const bool budgets = launch_regs((const void*)attention_bwd_kernel<128, true, 128>) >= BwdConfig<128, true, 128>::kLaunchRegs &&
                                     launch_regs((const void*)attention_bwd_kernel<128, false, 128>) >= BwdConfig<128, false, 128>::kLaunchRegs;
+        static const bool hands = launch_regs((const void*)attention_bwd_kernel<128, true, 128 + kHands>) >= BwdConfig<128, true, 128 + kHands>::kLaunchRegs;
         tall_kv = budgets && tall_tiles(dkdv.Sq), tall_q = budgets && tall_tiles(dq.Sk);
-        if (tall_kv && scratch && handed.kv_heads) {
+        if (hands && tall_kv && scratch && handed.kv_heads) {
             const CUtensorMap keys = rows(k, "key", 64);
             const int group = dq.N / dq.Nkv;
             BwdArgs a = dkdv;
@@ -661,7 +666,7 @@ void launch_bwd_pair(const Rows& rows, const lb_tensor& q, const lb_tensor& d_o,
                 for (int h = 0; h < dkdv.Nkv; h += heads) {
                     const int nb = std::min(batches, dkdv.B - b), nh = std::min(heads, dkdv.Nkv - h);
                     a.batch0 = d.batch0 = b, a.head0 = h, d.head0 = h * group, d.heads = nh * group;
-                    launch_bwd_kernel<128, true, 128>(mk, mv, mq, mdo, dim3(grid_kv.x, (unsigned)nh, (unsigned)nb), a, s);
+                    launch_bwd_kernel<128, true, 128 + kHands>(mk, mv, mq, mdo, dim3(grid_kv.x, (unsigned)nh, (unsigned)nb), a, s);
                     attention_dq_launch(keys, nb, d, s);
                 }
             return;
