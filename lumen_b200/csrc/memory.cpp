@@ -131,6 +131,7 @@ int lb_region_alloc(lb_region* region, size_t bytes, size_t alignment, void** ou
             if (dev != region->device) cudaSetDevice(dev);
             if (err != cudaSuccess) {
                 region->base = nullptr;
+                cudaGetLastError();  // or the next check of a launch reports it
                 lb::fail(LB_ERR_CUDA, lb::format("region: reserving %zu bytes on device %d failed: %s", region->capacity, region->device,
                                                  cudaGetErrorString(err)));
             }

@@ -178,12 +178,16 @@ def _workspace(like, shape, dtype: str, stream):
             _workspaces.move_to_end(key)
             try:
                 return _workspaces[key].empty(shape, dtype)
-            except _lib.LumenError:  # too small, or in use by other threads' calls: a region of its own takes its place
-                del _workspaces[key]
-        region = _workspaces[key] = Region(max(math.prod(shape) * ITEMSIZE[dtype] + 4096, 32 << 20))
+            except _lib.LumenError:  # too small, or in use by other threads' calls: one that holds all of it takes its place
+                live = _workspaces[key].stats()["live_bytes"]
+        else:
+            live = 0
+        region = Region(max(live + math.prod(shape) * ITEMSIZE[dtype] + 4096, 32 << 20))
+        work = region.empty(shape, dtype)  # (reserves the memory: a region that cannot be had takes no place)
+        _workspaces[key] = region
         while len(_workspaces) > _WORKSPACE_STREAMS:
             _workspaces.popitem(last=False)
-        return region.empty(shape, dtype)
+        return work
 
 
 GEMM_KERNELS = {"auto": 0, "tcgen05": 1, "simt": 2, "tcgen05_1cta": 3}
@@ -254,14 +258,48 @@ def attention_forward(q, k, v, scale=None, causal=False, out=None, lse=None, str
     return out, lse
 
 
-_KEPT_SCORES = 256 << 20
+# What the backward takes for dS whatever memory there is, and at most from a region, which is kept for its stream.
+_SMALL_SCORES, _KEPT_SCORES = 64 << 20, 256 << 20
 
 
-def attention_backward(q, k, v, o, d_o, lse, scale=None, causal=False, delta=None, stream=None, deterministic=True):
+def _out_of_memory(error: RuntimeError) -> bool:
+    if isinstance(error, _lib.LumenError):
+        return "out of memory" in str(error)
+    torch = sys.modules.get("torch")
+    return torch is not None and isinstance(error, torch.OutOfMemoryError)
+
+
+def _memory_is_short(t) -> bool:
+    """Whether a request to torch's allocator for memory of `t`'s device has failed before: another one that does not fit would wait for the
+    GPU and empty the allocator's cache once more. (10 us.)"""
+    try:
+        stats = sys.modules["torch"].cuda.memory_stats_as_nested_dict(t.device)
+    except RuntimeError:  # an allocator that does not count
+        return True
+    return stats.get("num_alloc_retries", 0) + stats.get("num_ooms", 0) > 0
+
+
+def _scores(q, nbytes: int, stream):
+    """Memory for the dS that the backward hands on, or None where that may cost more than it gives."""
+    if type(q).__module__.startswith("torch"):
+        if nbytes > _SMALL_SCORES and _memory_is_short(q):
+            return None
+    elif nbytes > _KEPT_SCORES:
+        return None
+    try:
+        return _workspace(q, (nbytes,), "uint8", stream)
+    except RuntimeError as error:
+        if not _out_of_memory(error):
+            raise
+        return None
+
+
+def attention_backward(q, k, v, o, d_o, lse, scale=None, causal=False, delta=None, stream=None, deterministic=True, max_scratch=None):
     """Flash attention backward; returns `(dq, dk, dv)` shaped like `q`, `k`, `v`. `deterministic` (the default here)
     runs `lb_attention_bwd_scratch`, the dK/dV + dQ kernel pair that is bit-identical from run to run; without it
     `lb_attention_bwd_atomic` runs the reference backend's default mode, one kernel adding dQ atomically into a float32
-    accumulator, at head dim 64, and the same pair elsewhere."""
+    accumulator, at head dim 64, and the same pair elsewhere. At head dim 128 the pair hands dS on in memory of the call's, up to 4.5 GiB
+    or `max_scratch` bytes (0: none), where there is such memory; the results are the same either way."""
     require_cuda()
     b, sq, n, h = q.shape
     sk = k.shape[1]
@@ -277,16 +315,12 @@ def attention_backward(q, k, v, o, d_o, lse, scale=None, causal=False, delta=Non
         handle = _stream(stream)
     dq_accum = _workspace(q, (b, sq, n, h), "float32", stream) if h == 64 and not deterministic else None
     scale, causal = float(scale if scale is not None else h**-0.5), bool(causal)
-    scores, nbytes = None, _lib.host().attention_bwd_scratch_bytes(scale, causal, sk - sq, q, k) if h == 128 else 0
-    if nbytes > _KEPT_SCORES and not type(q).__module__.startswith("torch"):
-        nbytes = 0  # a region that is kept for the stream
-    if nbytes:
-        try:
-            scores = _workspace(q, (nbytes,), "uint8", stream)
-        except RuntimeError:  # no memory for it: it is not needed
-            nbytes = 0
-    _lib.host().attention_bwd(scale, causal, sk - sq, q, k, v, o, d_o, lse, delta, dq_accum, dq, dk, dv, scores.data_ptr() if nbytes else 0,
-                              nbytes, handle)
+    nbytes = _lib.host().attention_bwd_scratch_bytes(scale, causal, sk - sq, q, k) if h == 128 else 0
+    if max_scratch is not None:
+        nbytes = max(0, min(nbytes, max_scratch))
+    scores = _scores(q, nbytes, stream) if nbytes else None
+    pointer, nbytes = (0, 0) if scores is None else (scores.data_ptr(), nbytes)
+    _lib.host().attention_bwd(scale, causal, sk - sq, q, k, v, o, d_o, lse, delta, dq_accum, dq, dk, dv, pointer, nbytes, handle)
     return dq, dk, dv
 
 
