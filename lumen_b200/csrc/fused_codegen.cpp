@@ -709,21 +709,33 @@ class Generator {
 
     // Threads of a row and blocks an SM of kernels that go over a row more than once, where the compiler's own choice of registers leaves an SM
     // with one block of 256 threads, or rows of many vectors are summed over more threads than those sums are worth (each warp of a row takes
-    // part in every total: ten shuffles of 1024 threads' second stage). us, as it was -> so, 2^24 elements (2^25 from 4096 columns on, 2^27 of
-    // 32768), bfloat16 where nothing else is said, float16 alike:
+    // part in every total: ten shuffles of 1024 threads' second stage). What decides is what a thread holds of a row: a rule that looked at the
+    // width alone made cross entropy of two operands up to 3.1 times as slow, norms of float32 rows beside 16-bit operands up to 2.6. us, as it
+    // was -> so, 2^24 elements, bfloat16 where nothing else is said:
     //   norms - rows written by what their sums say and by operands of the columns, no exponential on the way - are built for 512 threads an SM,
-    //   768 where a thread has 16 elements: layer norm of 512 columns 23.2 -> 14.0, 1024 23.5 -> 14.3, 1536 16.2 -> 13.7, 4096 32.5 -> 26.7,
-    //   float32 25.6 -> 22.1, 24.1 -> 22.8, (12 elements: left, 22.2 -> 24.7 at 3072,) 4096 50.5 -> 43.3; rms norm (one sum) 9.8 -> 8.1, 9.8 -> 8.1, but
-    //   4096 22.4 -> 23.5;
-    //   ... of which 512 threads and more walked 16-bit rows: eleven vectors a thread, 1024 threads an SM. 9872 columns 42.1 -> 32.0 (rms 30.0 ->
-    //   21.1), 32768 148 -> 127 (96.9 -> 95.1);
-    //   rows that are summed several times and not written (cross entropy), 16 bits, 512 threads and more: eleven vectors a thread too. 9872
-    //   columns 21.7 -> 15.0, 16384 33.9 -> 28.2, 32768 76.8 -> 53.8, but 50304 (608 threads) 59.7 -> 63.7;
-    //   float32 rows of several sums, no operands of columns, of which a power of two of threads leaves some idle: 9872 columns, softmax 52.9 ->
-    //   45.6, cross entropy 41.0 -> 30.6 (layer norm of 6000 columns 31.5 -> 33.4).
+    //   768 where a thread has 16 elements. One operand over the space: layer norm of 512 columns 11.3 -> 9.5, 1024 11.4 -> 9.6, 1536 11.8 -> 10.3, 4096
+    //   12.7 -> 11.0, float32 21.5 -> 20.3, 22.2 -> 20.7, float32 of three vectors a thread left; rms norm (one sum) up to 1024 columns 10.0 -> 8.6, at
+    //   2048 9.2 -> 8.6, but three vectors a thread 8.9 -> 9.6. Several operands: residual + layer norm of 1024 columns 34.8 -> 31.2, 8192 49.5 ->
+    //   35.6; left at 64 threads a row and with three vectors a thread (0.92 - 1.11; float32 beside 16 bits with three gains 0.90 - 0.97), at
+    //   float32 whose operands and results are four (42.0 -> 45.4: bandwidth), and rows of 16 bits with four vectors a thread, weights of float32 and
+    //   32 threads a row (19.8 -> 21.7);
+    //   ... of which 512 threads and more walked 16-bit rows: eleven vectors a thread, 1024 threads an SM. Layer norm of 9872 columns 19.9 -> 14.0,
+    //   32768 28.5 -> 15.5, rms norm 14.6 -> 9.4, 15.8 -> 10.4. Two operands of 16 bits fit from where threads had four vectors and more: residual +
+    //   rms norm of 33000 columns 37.9 -> 27.6, 16384 28.0 -> 26.9 and 9872 24.2 -> 27.8 left; + layer norm 50304 47.8 -> 41.4, 36000 42.2 -> 47.3;
+    //   rows that are summed several times and not written (cross entropy), one operand of 16 bits: eleven vectors too, up to 512 threads. 9872
+    //   columns 11.8 -> 7.4, 32768 11.2 -> 8.7, but 50304 (608 threads) 9.9 -> 10.6; two operands of 32768 columns 19.1 -> 59.2;
+    //   float32 rows of several sums, one operand and none of columns, of which a power of two of threads leaves some idle: four vectors a
+    //   thread, two blocks an SM. 8200 columns, softmax 31.2 -> 25.5, cross entropy 24.4 -> 15.2; two operands 25.2 -> 31.0.
     // Others are left: softmax, whose exponentials are taken again for its result, 0.8 - 1.3 of the time on any other threads, log softmax and
     // centred rows 1.0 - 1.4.
     int per_sm_ = 0;
+    // Whether an operand is read otherwise than by a gather (cross entropy's logits are, once more)
+    bool read_in_rows(int v) const {
+        for (const Node& n : g_.nodes)
+            for (size_t k = 0; k < n.inputs.size(); k++)
+                if (n.inputs[k] == v && !(n.op == "gather" && k == 0)) return true;
+        return false;
+    }
     void row_residency(int64_t nvec) {
         int sums = 0, behind = 0;
         std::map<int, int> seen;  // of a value: 1 behind a row's sum, 2 from an exponential of the space
@@ -735,21 +747,32 @@ class Generator {
                 if (auto it = seen.find(v); it != seen.end()) has |= reduce ? it->second & 1 : it->second;
             seen[n.output] = has;
         }
-        bool written = false, columns = false;
+        bool written = false, columns = false, wide_columns = false;
+        int row_bytes = 0, bytes = 0;  // of an element: of the operands that span the space, of results too
         for (int v : g_.outputs)
-            if (g_.type(v).numel() == R_ * C_) written = true, behind |= seen[v];
-        for (int v : g_.inputs) columns |= g_.type(v).numel() == C_ && R_ > 1;
-        const bool norm = written && behind == 1 && columns, summed = !written && sums > 1;
-        const int64_t eleven = (nvec * 3 / 32 + 31) / 32 * 32, four = (nvec + 127) / 128 * 32;
+            if (g_.type(v).numel() == R_ * C_) written = true, behind |= seen[v], bytes += dtype_size(g_.type(v).dtype);
+        for (int v : g_.inputs) {
+            const int64_t n = g_.type(v).numel();
+            const int size = dtype_size(g_.type(v).dtype);
+            if (n == R_ * C_ && read_in_rows(v)) row_bytes += size, bytes += size;
+            else if (n == C_ && R_ > 1) columns = true, wide_columns |= size * VEC_ > 16;
+        }
+        const bool norm = written && behind == 1 && columns, summed = !written && sums > 1, one = row_bytes * VEC_ == 16;
+        const int64_t eleven = (nvec * 3 / 32 + 31) / 32 * 32, four = (nvec + 127) / 128 * 32, elements = (nvec + T_ - 1) / T_ * VEC_;
         const int former = T_;
-        if (T_ >= 512 && narrow_) {
+        const bool two = norm && !wide_operands() && row_bytes == 4 && nvec >= (sums == 1 ? 4096 : 5120);
+        if (T_ >= 512 && !one && !two) {
+        } else if (T_ >= 512 && narrow_) {
             if (norm && eleven <= 1024) T_ = (int)eleven, per_sm_ = std::max(1, 1024 / T_);
             else if (summed && eleven <= 512) T_ = (int)eleven, per_sm_ = (T_ > 256 ? 1536 : 1024) / T_;
         } else if (T_ >= 512) {
-            if (sums > 1 && !columns && 8 * four <= 7 * (int64_t)T_) T_ = (int)four;
-        } else if (T_ <= 256 && norm && (sums > 1 || T_ <= 64)) {
-            const int64_t elements = (nvec + T_ - 1) / T_ * VEC_;
-            if (elements >= 16) per_sm_ = std::max(1, (elements > 16 ? 512 : 768) / (T_ * RPB_));
+            if (sums > 1 && !columns && 8 * four <= 7 * (int64_t)T_) T_ = (int)four, per_sm_ = T_ <= 640 ? 2 : 0;
+        } else if (T_ <= 256 && norm && elements >= 16) {
+            const bool pays = sums == 1  ? one && (T_ <= 32 || (narrow_ && elements > 24))
+                              : !narrow_ ? bytes < 16
+                              : one      ? T_ > 32 || elements <= 24 || !wide_columns
+                                         : T_ <= 32 || (elements > 24 ? T_ > 64 : row_bytes > 4);
+            if (pays) per_sm_ = std::max(1, (elements > 16 ? 512 : 768) / (T_ * RPB_));
         }
         if (T_ < former) chain_ = (int)std::max<int64_t>(VEC_, nvec * VEC_ / former);
     }
@@ -761,6 +784,13 @@ class Generator {
     }
     // Whether a mixed kernel keeps little for a column and for a row
     bool few_sums() const { return row_sums() <= 2 && held_columns() <= 9; }
+
+    // Operands over the space of more than 16 bits
+    int wide_operands() const {
+        int wide = 0;
+        for (int v : g_.inputs) wide += g_.type(v).numel() == R_ * C_ && dtype_size(g_.type(v).dtype) > 2;
+        return wide;
+    }
 
     // What a thread of a mixed kernel holds for each of its columns: a sum for each column total, the operands by column, and those over the
     // space twice (the row in flight and the one behind it)
@@ -1587,8 +1617,11 @@ class Generator {
         }
         std::string val = gen(n.inputs[0], src, ph);
         const bool pairs = adds_pairs(ph.combine_a_b, val);
-        ph.sums = std::max(sums(sum && flt), pairs ? 2 : 1);
-        const std::string which = shifted_ ? "e" : VEC_ > 2 || ph.sums == 2 ? format("e & %d", ph.sums - 1) : pairs ? "(ch & 1) * 2 + (e & 1)" : "ch & 3";
+        ph.sums = std::max(sums(sum && flt, pairs), pairs ? 2 : 1);
+        const std::string which = shifted_                                ? "e"
+                                  : !pairs                                ? format("ch & %d", ph.sums - 1)
+                                  : VEC_ > 2 || ph.sums == 2 ? format("e & %d", ph.sums - 1)
+                                                                          : "(ch & 1) * 2 + (e & 1)";
         ph.body += accumulate(ph.sums == 1 ? ph.acc : ph.acc + "[" + which + "]", ph.combine_a_b, val);
         row_decls_ += format("%s %s;\n", ct.compute, ph.result.c_str());
         phases_.push_back(ph);
@@ -1601,13 +1634,15 @@ class Generator {
     // elements those are follows from the row's distance to an aligned address, so that equal rows at different places (modulo eight), or of a
     // tensor that is not aligned, may differ in the last bits of a sum. The same call gives the same bits.
     // Where fewer threads walk a row than its sums were once dealt to, a thread's elements are dealt to as many sums as keep each no longer than
-    // those threads' were in the mean (chain_): 88 elements of a float16 row of 8200 in one chain had 1.6 times the error of 16.
+    // those threads' were in the mean (chain_): 88 elements of a float16 row of 8200 in one chain had 1.6 times the error of 16. Pairs that are
+    // added packed go by element, others vector by vector: by element, layer norm of 699 x 24000 float16 took 25.3 us instead of 17.8, softmax of
+    // 1699 x 9872 float32 27.6 instead of 25.4; packed, vector by vector, layer norm of 24000 columns 15.9 instead of 15.0.
     int chain_ = 0;
-    int sums(bool adds) const {
+    int sums(bool adds, bool pairs) const {
         if (shifted_) return VEC_;
         if (VEC_ <= 2) return NCH_ > 4 ? 4 : 1;
         int n = 1;
-        while (adds && chain_ && n < VEC_ && NCH_ * VEC_ > n * chain_) n *= 2;
+        while (adds && chain_ && n < VEC_ && (pairs ? NCH_ * VEC_ > n * chain_ : (NCH_ + n - 1) / n * VEC_ > chain_)) n *= 2;
         return n;
     }
 
