@@ -647,14 +647,15 @@ class Generator {
                 // Rows of 16 bits from 1024 columns on: two vectors of eight bytes a thread and as many blocks as 16 warps and more need, so
                 // that a block of 13 to 15 warps is not alone on its SM, 24 where every thread has both vectors whole and few sums to keep (84
                 // registers do: a layer norm's gradients 16384 x 1024 39.0 -> 32.0, 21845 x 1536 68 -> 61, 16384 x 2048 71 -> 60, the same at
-                // 2^22 elements 1.05 - 1.12, with four row sums 1.2, 512 threads 1.06, a last vector that some lack 1.03 - 1.1). us, the sums
+                // 2^22 elements 1.05 - 1.12, with four row sums 1.2, 512 threads 1.06, a last vector that some lack 1.03 - 1.1; operands of
+                // float32, which hold twice as much, 0.86 - 0.98 with 128 threads a row, but beyond them 30.9 -> 34.8 at 10922 x 1536). us, the sums
                 // above, one vector of 16 bytes a thread -> so: 2048 x 1024 12.9 -> 11.0, 4096 x 2048 32.6 -> 31.8, 3640 x 2304 42 -> 35,
                 // 2532 x 3312 52 -> 45, 1677 x 5000 48 -> 41, 1024 x 8192 58 -> 45.
                 // Few rows of 2049 to 3072 columns, whose blocks would have nine to twelve warps, are left: 455 x 2304 9.9 against 10.5.
                 VEC_ = 4, nvec = vectors(), chunks = 2;
                 T_ = (int)threads_for(chunks);
                 if (T_ > 288 && T_ <= 384 && C_ % (T_ * 8) != 0) T_ = (int)threads_for(3);  // (the last chunk a part: 2600 wide as fast, few rows faster)
-                else warps = !sixteen_warps_ && few_sums() && T_ <= 256 && C_ == T_ * VEC_ * 2 && R_ * C_ >= 1 << 23 ? 24 : 16;
+                else warps = !sixteen_warps_ && few_sums() && (!wide_operands() || held_columns() + 2 * wide_operands() <= (T_ <= 128 ? 9 : 8)) && T_ <= 256 && C_ == T_ * VEC_ * 2 && R_ * C_ >= 1 << 23 ? 24 : 16;
             } else if (min_size == 2 && VEC_ == 8 && C_ > 256 && C_ < 1024 && R_ * C_ >= 1 << 20 && !sixteen_warps_) {
                 // Rows of 264 to 1016 columns of 16 bits. Up to 384 columns a warp to a row, so that row sums need no barrier between warps, with three
                 // vectors of eight bytes a thread and 20 warps an SM; from there two of them a thread and 24 warps, but a warp to a row with two

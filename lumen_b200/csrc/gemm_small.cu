@@ -245,7 +245,6 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
         }
     }
-    if (PUSH) bulk_push_wait();
     __syncwarp();
     if (RANKS) cluster_arrive_done();
     __syncthreads();
@@ -257,7 +256,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         }
     }
     __syncwarp();
-    if (RANKS) cluster_wait_done();  // no CTA leaves while another reads its partial tile
+    if (RANKS) cluster_wait_done();  // no CTA leaves while another reads its partial tile, or before what it sent has landed (each has waited for that)
     else __syncthreads();
     if (warp == 1) {
         tc_fence_after();

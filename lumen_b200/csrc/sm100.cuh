@@ -265,19 +265,17 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // `bytes` contiguous bytes of this CTA's shared memory into that of CTA `rank` of the cluster, to where `dst` lies here, counted on the barrier
-// at `bar`'s offset there. Addresses and size are multiples of 16; fence_proxy_async first by those who wrote the source.
+// at `bar`'s offset there, which alone says when it has arrived. Addresses and size are multiples of 16; fence_proxy_async first by those who
+// wrote the source. Neither CTA may leave before it has arrived.
 __device__ __forceinline__ void bulk_push(void* dst, const void* src, uint32_t bytes, uint64_t* bar, uint32_t rank) {
     asm volatile(
         "{\n\t.reg .b32 rd, rb;\n\t"
         "mapa.shared::cluster.u32 rd, %0, %4;\n\t"
         "mapa.shared::cluster.u32 rb, %3, %4;\n\t"
-        "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [rd], [%1], %2, [rb];\n\t"
-        "cp.async.bulk.commit_group;\n\t}"
+        "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [rd], [%1], %2, [rb];\n\t}"
         ::"r"(smem_u32(dst)), "r"(smem_u32(src)), "r"(bytes), "r"(smem_u32(bar)), "r"(rank)
         : "memory");
 }
-// Waits until what this thread has pushed has arrived.
-__device__ __forceinline__ void bulk_push_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // cluster_sync in two halves, for the end of what other CTAs of the cluster read from this one's shared memory: it orders no memory (a release
 // would wait, about a microsecond, for the thread's global stores), but a thread has what it has used of another CTA's when it arrives.
 __device__ __forceinline__ void cluster_arrive_done() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }

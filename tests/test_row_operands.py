@@ -6,7 +6,7 @@ import re
 import pytest
 
 from lumen_b200 import functional as F
-from lumen_b200 import tracer
+from lumen_b200 import prims, tracer
 from lumen_b200.runtime import Fusion
 
 
@@ -79,3 +79,19 @@ def test_norms_of_two_wide_operands(program, cols, dtype):
     # a rounding of the result, and float32 sums of chains of 2^6 and trees of 2^10
     bound = {"bfloat16": 2.0**-8, "float16": 2.0**-11}[dtype] * want.abs() + 2.0**-18 * (s.abs() + 1) * (d.abs() + 1)
     assert ((got - want).abs() <= bound).all()
+
+
+def gradients(g, a, w):
+    x = a.float() * F.rsqrt(F.mean(a.float() * a.float(), -1, keepdim=True) + 1e-5)
+    t = g.float() * w.float()
+    return (t - x * F.mean(t * x, -1, keepdim=True)).to(a.dtype), prims.reduce_sum(g.float() * x, (0,), "float32"), prims.reduce_sum(g.float(), (0,), "float32")
+
+
+@pytest.mark.parametrize("cols, dtypes, blocks", [(1024, (B, B, B), 6), (1536, (B, B, B), 4), (2048, (H, H, W), 3), (1024, (W, B, B), 6), (1536, (W, B, B), 3), (1536, (B, W, B), 3),
+                                                  (2048, (B, W, W), 2), (1024, (W, W, B), 4)])
+def test_warps_of_kernels_that_sum_columns(cols, dtypes, blocks):
+    """24 warps an SM for operands of 16 bits, one of float32 at 128 threads a row; sixteen for others."""
+    rows = (1 << 24) // cols
+    types = [(d, shape) for d, shape in zip(dtypes, ((rows, cols), (rows, cols), (cols,)))]
+    source = Fusion(tracer.trace(gradients, *types)).source
+    assert int(re.search(r"__launch_bounds__\(\d+, (\d+)\) fused_kernel", source)[1]) == blocks
