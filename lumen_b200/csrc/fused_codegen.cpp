@@ -658,16 +658,16 @@ class Generator {
                 else warps = !sixteen_warps_ && few_sums() && (!wide_operands() || held_columns() + 2 * wide_operands() <= (T_ <= 128 ? 9 : 8)) && T_ <= 256 && C_ == T_ * VEC_ * 2 && R_ * C_ >= 1 << 23 ? 24 : 16;
             } else if (min_size == 2 && VEC_ == 8 && C_ > 256 && C_ < 1024 && R_ * C_ >= 1 << 20 && !sixteen_warps_) {
                 // Rows of 264 to 1016 columns of 16 bits. Up to 384 columns a warp to a row, so that row sums need no barrier between warps, with three
-                // vectors of eight bytes a thread and 20 warps an SM; from there two of them a thread and 24 warps, but a warp to a row with two
-                // or three vectors of 16 bytes where threads hold little (at 768 columns: have few row sums) from 2^21 elements on, beyond 512
-                // columns up to 2^23: there the others take 0.92 - 1.24 of its time, at more elements 0.79 - 1.07. Times a vector of 16 bytes a thread
-                // and 16 warps, gradients of a layer norm, layer and RMS norm and softmax with theirs, softmax with column sums, five operands
-                // with three column sums, 2^20 to 2^25 elements: 0.39 - 0.98 up to 384 columns, 0.61 - 0.97 up to 768, 0.52 - 1.08 beyond (1.08:
-                // 6 us), float16 0.38 - 1.02. us, bfloat16: RMS norm with its gradients 16384 x 512 17.1 -> 11.7, 63550 x 264 47.8 -> 30.3, 18724 x 896
-                // 33.7 -> 29.6, layer norm with its gradients 26214 x 640 47.9 -> 35.0, 4128 x 1016 16.9 -> 12.5, softmax with its gradient
-                // 43690 x 384 67.9 -> 26.3.
+                // vectors of eight bytes a thread and 20 warps an SM; from there two of them a thread and 24 warps, but from 2^21 elements on, where
+                // threads hold little, a warp to a row with two or three vectors of 16 bytes: up to 512 columns; beyond them with few row sums where
+                // no lane lacks its last vector, and else up to five million elements. Times a vector of 16 bytes a thread and 16 warps, gradients of
+                // a layer norm, layer and RMS norm and softmax with theirs, softmax with column sums, 2^20 to 2^25 elements: 0.39 - 1.0. A warp
+                // to a row against two vectors a thread, 520, 640, 744 and 760 columns: four million elements 0.90 - 1.07, seven 0.96 - 1.09 (two
+                // softmaxes, five row sums, 1.03 - 1.26), nine and more 0.99 - 1.30; 768 columns: one or two row sums 0.89 - 1.02 at any of these
+                // sizes, more 0.95 - 1.29.
                 chain_ = VEC_;
-                if (C_ > 384 && C_ <= 768 && R_ * C_ > 1 << 21 && (C_ <= 512 || C_ == 768 || R_ * C_ < 1 << 23) && held_columns() <= 9 && (C_ < 768 || few_sums())) {
+                const bool warp_rows = C_ <= 512 || (nvec % 32 == 0 ? few_sums() : row_sums() <= 4 && R_ * C_ <= 5 << 20);
+                if (C_ > 384 && C_ <= 768 && R_ * C_ > 1 << 21 && warp_rows && held_columns() <= 9) {
                     T_ = 32, warps = C_ <= 512 ? 16 : 12;
                 } else {
                     VEC_ = 4, nvec = vectors(), chunks = C_ <= 384 ? 3 : 2;
