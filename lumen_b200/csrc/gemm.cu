@@ -885,7 +885,7 @@ bool gemm(const lb_tensor& a_t, const lb_tensor& b_t, const lb_tensor& d_t, int 
         aux = view3(*aux_t, "epilogue operand");
         if (aux.dtype != d.dtype || aux.rows != d.rows || aux.cols != d.cols || aux.batch != d.batch || (aux.sc != 1 && aux.cols > 1))
             fail(LB_ERR_INVALID, "gemm: the epilogue operand must be a row-major tensor of the output's shape and dtype");
-        if (d.dtype != LB_BF16 && d.dtype != LB_F16 && a.dtype != LB_F32)
+        if (d.dtype != LB_BF16 && d.dtype != LB_F16 && !(a.dtype == LB_F32 && held))  // float32 products take one in plans alone
             fail(LB_ERR_UNSUPPORTED, "gemm: the add / mask epilogue is built for 16-bit outputs of the tensor-core kernels");
     }
     if (a.dtype != b.dtype) fail(LB_ERR_INVALID, "gemm: operands must share a dtype (no hidden casts)");
@@ -1004,8 +1004,6 @@ extern "C" {
 int lb_gemm(const lb_tensor* a, const lb_tensor* b, const lb_gemm_out* out, const lb_gemm_cfg* cfg, void* stream) {
     return lb::guarded([&] {
         if (!a || !b || !out) lb::fail(LB_ERR_INVALID, "lb_gemm: null argument");
-        if (out->epilogue >= lb::EPI_ADD && out->epilogue <= lb::EPI_MASK && out->product.dtype == LB_F32)
-            lb::fail(LB_ERR_UNSUPPORTED, "gemm: the add / mask epilogue is built for 16-bit outputs of the tensor-core kernels");  // plans alone
         lb::GemmTuning tuning{cfg ? cfg->splits : 0, cfg ? cfg->group_m : 0};
         lb::gemm(*a, *b, out->product, out->epilogue, cfg ? cfg->kernel : 0, stream, cfg ? cfg->scratch : nullptr,
                  cfg ? cfg->scratch_bytes : 0, out->epilogue >= 2 ? &out->aux : nullptr, &tuning, nullptr);
