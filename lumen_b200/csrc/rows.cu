@@ -902,10 +902,14 @@ void launch_attn(Kernel kernel, unsigned blocks, int streamed, cudaStream_t st, 
     launch_overlapped(kernel, dim3(blocks), dim3(kAttnWarps * 32), AttnSmem<DU, RW>::bytes(s.tile_rows), st, 0, args..., s);
 }
 // Two rows a warp fetch a streamed element for both (every bit the same): from 512 blocks of one row a warp on, which is where they win. us,
-// one row -> two, forward, backward: 4 x 8 heads x 256 x 64 float32 48.9 -> 43.5, 140 -> 118; 2 x 4 x 1000 x 32 111 -> 92, 288 -> 291; 2 x 8 x 300 x
-// 128 109 -> 104, 317 -> 270; 2 x 4 x 500 x 256 202 -> 166, 567 -> 492; bfloat16 16 x 704 x 64 of one batch entry 160 -> 138; but fewer blocks 8 x 4 x
-// 64 x 32 6.1 -> 6.3, 2 x 140 x 32 9.4 -> 11.0. Four rows: 0.68 - 1.6 of the time.
-bool two_rows(long long batch, long long heads, long long rows) { return batch * heads * ((rows + kAttnWarps - 1) / kAttnWarps) >= 512; }
+// one row -> two, forward, backward: 4 x 8 heads x 256 x 64 float32 48.9 -> 43.5, 140 -> 118; 2 x 8 x 300 x 128 109 -> 104, 317 -> 270; 2 x 4 x 500 x
+// 256 202 -> 166, 567 -> 492; bfloat16 16 x 704 x 64 of one batch entry 160 -> 138; but fewer blocks 8 x 4 x 64 x 32 6.1 -> 6.3, 2 x 140 x 32 9.4 ->
+// 11.0. Where head dims up to 32 are masked the line is at 768: 2 x 4 x 520 (520 blocks) 38.5 -> 40.2, 2 x 4 x 1000 106 -> 93, 277 -> 213. Over 14
+// shapes of 512 to 4096 blocks, head dims of 32 to 256 in either type: 0.53 - 1.02 of the time; the six forms that spill up to 52 bytes 0.65 - 0.87.
+// Four rows: 0.68 - 1.6 of the time.
+bool two_rows(const AttnShape& s, long long heads, long long rows) {
+    return s.B * heads * ((rows + kAttnWarps - 1) / kAttnWarps) >= (s.causal && s.D <= 32 ? 768 : 512);
+}
 template <class F>
 void with_rows(bool two, F&& f) {
     if (two) f(std::integral_constant<int, 2>());
@@ -922,7 +926,7 @@ void with_dims_per_lane(int D, F&& f) {
 template <class T>
 void simt_fwd(const AttnShape& s, const lb_tensor& q, const lb_tensor& k, const lb_tensor& v, const lb_tensor& o, float* lse, cudaStream_t st) {
     with_dims_per_lane(s.D, [&](auto du) {
-        with_rows(two_rows(s.B, s.N, s.Sq), [&](auto rw) {
+        with_rows(two_rows(s, s.N, s.Sq), [&](auto rw) {
             launch_attn<du, rw>(attention_simt_fwd_kernel<T, du, rw>, attn_blocks(s.B, s.N, s.Sq, rw), s.Sk, st, s, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr,
                                 (T*)o.ptr, lse);
         });
@@ -934,11 +938,11 @@ void simt_bwd(const AttnShape& s, const lb_tensor& q, const lb_tensor& k, const 
     const long long warps = (long long)s.B * s.N * s.Sq;
     launch_overlapped(attention_delta_simt<T>, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256), 0, st, 0, (const T*)o.ptr, (const T*)g.ptr, delta, s);
     with_dims_per_lane(s.D, [&](auto du) {
-        with_rows(two_rows(s.B, s.N, s.Sq), [&](auto rw) {
+        with_rows(two_rows(s, s.N, s.Sq), [&](auto rw) {
             launch_attn<du, rw>(attention_simt_dq_kernel<T, du, rw>, attn_blocks(s.B, s.N, s.Sq, rw), s.Sk, st, s, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr,
                                 (const T*)g.ptr, lse, (const float*)delta, (T*)dq.ptr);
         });
-        with_rows(two_rows(s.B, s.Nkv, s.Sk), [&](auto rw) {
+        with_rows(two_rows(s, s.Nkv, s.Sk), [&](auto rw) {
             launch_attn<du, rw>(attention_simt_dkdv_kernel<T, du, rw>, attn_blocks(s.B, s.Nkv, s.Sk, rw), s.Sq, st, s, (const T*)q.ptr, (const T*)k.ptr, (const T*)v.ptr,
                                 (const T*)g.ptr, lse, (const float*)delta, (T*)dk.ptr, (T*)dv.ptr);
         });
