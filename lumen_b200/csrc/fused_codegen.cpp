@@ -1208,13 +1208,10 @@ class Generator {
         if (it != pair_vars_.end() && it->second == LB_BF16 && dtype == LB_BF16) return format("*(u32*)&%s[e] = %s.v;\n", buf.c_str(), val.c_str());
         return both_lanes(format("%s[e] = %s;\n", buf.c_str(), to_memory(dtype, "LX(" + val + ")").c_str()));
     }
-    // Whether a pair's elements are added by one packed instruction: float32 sums. Half the instructions, and a chain half as long. With packed
-    // negations, one product for x * y and y * x, and what is said at divide_again, 58.5 -> 53.8 instructions an element and 28.2 -> 27.7 us for
-    // a layer norm of 8192 x 1024 bfloat16 with its gradients: chains of dependent instructions bound it more than their number. That kernel
-    // sums a row four times and its columns twice, and measures the same without packed sums: kernels that sum columns and, three times and
-    // more, rows keep a sum an element. 31 sizes from 8065 x 520 to 8192 x 2048, us, packed -> so: layer norm with its gradients 0.95 - 1.02 (21845 x 768
-    // 37.2 -> 35.6, 5461 x 1536 20.2 -> 19.6), softmax with its gradient 0.97 - 1.01 (16384 x 1024 32.4 -> 31.7), but RMS norm, which
-    // sums a row twice, 0.99 - 1.03.
+    // Whether a pair's elements are added by one packed instruction: float32 sums. Half the instructions, and a chain half as long. Not in kernels that
+    // sum columns and, three times and more, rows: 31 sizes from 8065 x 520 to 8192 x 2048, packed -> an element each, layer norm with its gradients 0.95 - 1.02
+    // of the time (21845 x 768 37.2 -> 35.6 us, 5461 x 1536 20.2 -> 19.6, 8192 x 1024 the same), softmax with its gradient 0.97 - 1.01 (16384 x 1024 32.4 -> 31.7),
+    // but RMS norm, which sums a row twice, 0.99 - 1.03.
     bool adds_pairs(const std::string& combine, const std::string& val) const {
         return pair_ && !shifted_ && !(mixed_ && row_sums() > 2) && combine == "rnd_f32(__fadd_rn(%A, %B))" && packable(val, LB_F32);
     }
@@ -1619,10 +1616,7 @@ class Generator {
         std::string val = gen(n.inputs[0], src, ph);
         const bool pairs = adds_pairs(ph.combine_a_b, val);
         ph.sums = std::max(sums(sum && flt, pairs), pairs ? 2 : 1);
-        const std::string which = shifted_                                ? "e"
-                                  : !pairs                                ? format("ch & %d", ph.sums - 1)
-                                  : VEC_ > 2 || ph.sums == 2 ? format("e & %d", ph.sums - 1)
-                                                                          : "(ch & 1) * 2 + (e & 1)";
+        const std::string which = shifted_ ? "e" : !pairs ? format("ch & %d", ph.sums - 1) : ph.sums == 2 ? "e & 1" : "(ch & 1) * 2 + (e & 1)";
         ph.body += accumulate(ph.sums == 1 ? ph.acc : ph.acc + "[" + which + "]", ph.combine_a_b, val);
         row_decls_ += format("%s %s;\n", ct.compute, ph.result.c_str());
         phases_.push_back(ph);
@@ -1635,15 +1629,15 @@ class Generator {
     // elements those are follows from the row's distance to an aligned address, so that equal rows at different places (modulo eight), or of a
     // tensor that is not aligned, may differ in the last bits of a sum. The same call gives the same bits.
     // Where fewer threads walk a row than its sums were once dealt to, a thread's elements are dealt to as many sums as keep each no longer than
-    // those threads' were in the mean (chain_): 88 elements of a float16 row of 8200 in one chain had 1.6 times the error of 16. Pairs that are
-    // added packed go by element, others vector by vector: by element, layer norm of 699 x 24000 float16 took 25.3 us instead of 17.8, softmax of
-    // 1699 x 9872 float32 27.6 instead of 25.4; packed, vector by vector, layer norm of 24000 columns 15.9 instead of 15.0.
+    // those threads' were in the mean (chain_), vector by vector: 88 elements of a float16 row of 8200 in one chain had 1.6 times the error of 16.
+    // (Element by element, layer norm of 699 x 24000 float16 took 25.3 us instead of 17.8, softmax of 1699 x 9872 float32 27.6 instead of 25.4.) Pairs
+    // that are added packed are two sums, of up to 44 elements: 2.9e-8 -> 3.3e-8 of a sum of 16384 exponentials, half a unit in its last place either way.
     int chain_ = 0;
     int sums(bool adds, bool pairs) const {
         if (shifted_) return VEC_;
         if (VEC_ <= 2) return NCH_ > 4 ? 4 : 1;
         int n = 1;
-        while (adds && chain_ && n < VEC_ && (pairs ? NCH_ * VEC_ > n * chain_ : (NCH_ + n - 1) / n * VEC_ > chain_)) n *= 2;
+        while (adds && !pairs && chain_ && n < VEC_ && (NCH_ + n - 1) / n * VEC_ > chain_) n *= 2;
         return n;
     }
 
