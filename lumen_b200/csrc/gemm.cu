@@ -733,14 +733,14 @@ static int gemm_tile_splits(long long M, long long N, long long K, long long bat
 
 // The same for what runs: CTA pairs take 256 x 256 tiles of more than 128 rows. us: 3 a product, 0.3 a k-block and 2 a unit of each wave, 0.1 a
 // k-block shared by all pairs (the L2's part and the power's), 3.5 for the reduction and, a million elements of the result, 0.45 a range and 0.6:
-// a fit to 714 shapes of 129 to 9000 rows and columns and K of 500 to 30000 under 1 to 8 ranges (half of them within 6 %). Another number than
-// the model's above has to win by a tenth of that: of 30 shapes, among those and 404 others, that the two would cut otherwise, five are within
-// it and took up to 1.07 of the time (1576 x 536 K 19752, 1.00 by the model), the others 0.69 - 1.06, 0.82 in the mean; 1500 x 1024 K 4096
-// 24.2 -> 18.4, 1530 x 1536 K 6144 0.83, 768 x 3072 K 4096 26.4 -> 23.4, 357 x 4096 K 4096 0.86. Which products stay on narrow tiles is left to
-// the model above, which that line was measured with.
+// a fit to 714 shapes of 129 to 9000 rows and columns and K of 500 to 30000 under 1 to 8 ranges (half of them within 6 %). Against the
+// model above, on those and 404 other shapes: 55 are cut otherwise and take 0.69 - 1.08 of the time, 0.84 in the mean, three of them more than
+// 1.03; 1500 x 1024 K 4096 24.2 -> 18.4, 1530 x 1536 K 6144 0.83, 768 x 3072 K 4096 26.4 -> 23.4, 357 x 4096 K 4096 0.86. (The former number where
+// this model puts another less than a tenth below it is no better line: 64 such shapes, every operand major, 0.84 - 1.14 of these counts' time for a product alone,
+// 1.007 in the mean, and 0.84 - 1.37, 0.99, one after another under the power cap.) Which products stay on narrow tiles is left to the model above, which
+// that line was measured with.
 int gemm_splits(long long M, long long N, long long K, long long batch, int sms) {
-    int best = gemm_tile_splits(M, N, K, batch, sms);
-    if (M <= BM) return best;
+    if (M <= BM) return gemm_tile_splits(M, N, K, batch, sms);
     const int pairs = sms / 2;
     const long long tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) * batch, total_kb = (K + BK - 1) / BK;
     if (tiles >= 4LL * pairs || total_kb < 32) return 1;
@@ -749,8 +749,9 @@ int gemm_splits(long long M, long long N, long long K, long long batch, int sms)
         const double kb = (double)((total_kb + s - 1) / s), waves = (double)((tiles * s + pairs - 1) / pairs);
         return 3.0 + waves * (0.3 * kb + 2.0) + 0.1 * kb * (double)(tiles * s) / pairs + (s > 1 ? 3.5 + millions * (0.45 * s + 0.6) : 0.0);
     };
-    double best_us = cost(best) * 0.9;
-    for (int s = 1; s <= 32 && (s == 1 || total_kb / s >= 16); s++)
+    int best = 1;
+    double best_us = cost(1) * 0.9;
+    for (int s = 2; s <= 32 && total_kb / s >= 16; s++)
         if (cost(s) < best_us) best = s, best_us = cost(s);
     return best;
 }
