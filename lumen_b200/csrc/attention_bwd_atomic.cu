@@ -79,13 +79,6 @@ __device__ __forceinline__ void tma_reduce_add_4d(const CUtensorMap* map, const 
 }
 // Barrier `id` over `count` threads (a warpgroup): the CTA-wide barrier 0 stays free for the other roles.
 __device__ __forceinline__ void named_barrier(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
-// The same, and whether each of the threads has said yes.
-__device__ __forceinline__ bool named_barrier_all(int id, int count, bool yes) {
-    uint32_t all;
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tbar.red.and.pred q, %1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-                 : "=r"(all) : "r"(id), "r"(count), "r"((uint32_t)yes) : "memory");
-    return all != 0;
-}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
@@ -246,30 +239,33 @@ attention_bwd_atomic_kernel(const __grid_constant__ CUtensorMap map_k, const __g
         const int swz = row_in_tile & 7;
         const bool issuer = warp == 4 && lane == 0;
         bool ok = true;
-        for (int j = 0; j < n_iter && ok; j++) {
+        // The four warps go through every tile and both of its barriers, also when a wait has run out: one that left while another's wait still
+        // ended would leave that one at a barrier, which has no limit, for good.
+        for (int j = 0; j < n_iter; j++) {
             const int hh = j / per_head;
             const int q0 = (t_begin + j - hh * per_head) * BT;
-            ok = mbar_wait_warp(dq_full, (uint32_t)j & 1, abort_flag);
+            ok = ok && mbar_wait_warp(dq_full, (uint32_t)j & 1, abort_flag);
             tc_fence_after();
             if (issuer) bulk_wait_read();  // the previous reduces have read the staging tiles
-            // the four warps leave together: one that gave up while another's wait still ended would leave that one at the barrier for good
-            if (!(ok = named_barrier_all(1, 128, ok))) break;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {  // two halves of 32 columns: [128 rows x 128 bytes], swizzled as the tensor map expects
-                uint32_t v[32];
-                tmem_ld_32x32(tmem_dq + lane_addr + h * 32, v);
-                tmem_ld_wait();
-                if (h == 1) {
-                    tc_fence_before();
-                    mbar_arrive(dq_empty);
-                }
-#pragma unroll
-                for (int i = 0; i < 8; i++)
-                    *(uint4*)(stage + h * kHalf + row_in_tile * 128 + ((i ^ swz) * 16)) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-            }
-            fence_proxy_async();
             named_barrier(1, 128);
-            if (issuer) {
+            if (ok) {
+#pragma unroll
+                for (int h = 0; h < 2; h++) {  // two halves of 32 columns: [128 rows x 128 bytes], swizzled as the tensor map expects
+                    uint32_t v[32];
+                    tmem_ld_32x32(tmem_dq + lane_addr + h * 32, v);
+                    tmem_ld_wait();
+                    if (h == 1) {
+                        tc_fence_before();
+                        mbar_arrive(dq_empty);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; i++)
+                        *(uint4*)(stage + h * kHalf + row_in_tile * 128 + ((i ^ swz) * 16)) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                }
+                fence_proxy_async();
+            }
+            named_barrier(1, 128);
+            if (issuer && ok) {
                 tma_reduce_add_4d(&map_acc, stage, 0, head * group + hh, q0, batch);
                 tma_reduce_add_4d(&map_acc, stage + kHalf, 32, head * group + hh, q0, batch);
                 bulk_commit();

@@ -7,10 +7,11 @@ import re
 SOURCE = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "lumen_b200", "csrc", "attention_bwd_atomic.cu")
 
 
-def test_the_warps_leave_together():
+def test_the_warps_stay_together():
     text = re.sub(r"//[^\n]*", "", open(SOURCE).read())
-    loop = text[text.index("regs_dec<kRegsDrain>") : text.index("bulk_wait_all();")]
-    body = loop[loop.index("for (int j = 0; j < n_iter && ok; j++)") :]
-    vote = re.search(r"if \(!\(ok = named_barrier_all\(1, 128, ok\)\)\) break;", body)
-    assert vote and not re.search(r"\b(break|return|continue)\b", body[: vote.start()])
-    assert len(re.findall(r"\b(break|return|continue)\b", body)) == 1 and body.count("named_barrier(1, 128)") == 1
+    body = text[text.index("regs_dec<kRegsDrain>") : text.index("bulk_wait_all();\n    } else {")]
+    assert re.findall(r"\bfor \(int j = 0;[^)]*\)", body) == ["for (int j = 0; j < n_iter; j++)"]
+    assert not re.search(r"\b(break|return|continue)\b", body)
+    for barrier in re.finditer(r"\n( *)named_barrier\(1, 128\);", body):
+        assert barrier[1] == " " * 12  # in the loop, under no condition
+    assert body.count("named_barrier(1, 128)") == 2
